@@ -71,11 +71,39 @@ uint32_t sm_count()
   return (uint32_t)v;
 }
 
-Plan plan_for(uint32_t dim0, uint32_t C, uint32_t N, bool aligned16)
+// What planning derives from a shape alone.  A call asks for it several times and a training loop makes the
+// same few calls over and over, so each thread keeps the answers for the shapes it saw last (a fixed number of
+// entries, nothing shared between threads).  Planning on every call cost 10 - 50 us of host time, several times
+// the kernel's own time on small layers (the slice-resident kernel's planner alone searches hundreds of layouts).
+struct ShapeInfo {
+  uint32_t dim0, C, N, sms;      // key; sms == 0: empty
+  Plan plan[2];                  // tile plan: [pointers 16-byte aligned]
+  bool ring_ok[2];               // warp-specialised kernel, per direction, for aligned pointers
+  Plan ring_plan[2];
+  RingGeom ring_geom[2];
+  uint64_t tiled_bytes, part_bytes;
+};
+constexpr uint32_t kShapeCache = 64;      // entries per thread, direct mapped
+
+static void fill_shape_info(ShapeInfo &s);
+
+static const ShapeInfo &shape_info(uint32_t dim0, uint32_t C, uint32_t N)
 {
-  const Tunables &t = tunables();
-  return make_plan(dim0, C, N, aligned16, sm_count() * t.blocks_per_sm, t.tile_floats, 1);
+  thread_local std::unique_ptr<ShapeInfo[]> cache;
+  if (!cache) cache.reset(new ShapeInfo[kShapeCache]());
+  const uint32_t sms = sm_count();
+  const uint32_t h = (dim0 * 0x9e3779b1u) ^ (C * 0x85ebca6bu) ^ (N * 0xc2b2ae35u);
+  ShapeInfo &s = cache[(h >> 16) % kShapeCache];
+  if (s.dim0 != dim0 || s.C != C || s.N != N || s.sms != sms) {
+    s.sms = 0;
+    s.dim0 = dim0; s.C = C; s.N = N;
+    fill_shape_info(s);
+    s.sms = sms;
+  }
+  return s;
 }
+
+Plan plan_for(uint32_t dim0, uint32_t C, uint32_t N, bool aligned16) { return shape_info(dim0, C, N).plan[aligned16 ? 1 : 0]; }
 
 // Shared-memory layout of the warp-specialised kernel for plan `p` (see bn_ring.cuh).
 // consumer warps of direction `dir`: 8 or 16 (the two instantiations of bn_ring.cuh)
@@ -134,10 +162,9 @@ static uint64_t ring_window_bytes(const Plan &p, int dir)
 constexpr uint32_t kRingLargeSlotsBwd = 3, kRingLargeFloatsBwd = 9408;
 constexpr uint64_t kRingLargeWindowMax = 48ull << 20;     // also the part of a larger window that is marked "keep" (launch_ring)
 
-bool ring_plan_for(uint32_t dim0, uint32_t C, uint32_t N, bool aligned, int dir, Plan &p, RingGeom &g)
+static bool make_ring_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, Plan &p, RingGeom &g)
 {
   const Tunables &t = tunables();
-  if (!aligned) return false;
   if (!ring_plan_with(dim0, C, N, dir, dir == 0 ? t.ring_slots : t.ring_slots_bwd,
                       dir == 0 ? t.ring_floats_fwd : t.ring_floats_bwd, p, g)) return false;
   if (dir == 1) {
@@ -148,6 +175,15 @@ bool ring_plan_for(uint32_t dim0, uint32_t C, uint32_t N, bool aligned, int dir,
       p = pl; g = gl;
     }
   }
+  return true;
+}
+
+bool ring_plan_for(uint32_t dim0, uint32_t C, uint32_t N, bool aligned, int dir, Plan &p, RingGeom &g)
+{
+  if (!aligned) return false;
+  const ShapeInfo &s = shape_info(dim0, C, N);
+  if (!s.ring_ok[dir]) return false;
+  p = s.ring_plan[dir]; g = s.ring_geom[dir];
   return true;
 }
 
@@ -213,24 +249,28 @@ int launch_ring(FusedArgs &a, const RingGeom &g_in, int dir, cudaStream_t stream
 // direction's kernels keep state in their part from launch to launch (which partial buffer is
 // current, words waiting to be cleared), laid out by that direction's own tile plan, so forward
 // and backward launches must not share one.  The status word is the first word of the whole.
-// Bytes of a part taken by the tile-plan kernels (plain, warp-specialised, cluster); the records of the
-// slice-resident kernel follow behind them.
-static uint64_t tiled_part_bytes(uint32_t dim0, uint32_t C, uint32_t N)
+static void fill_shape_info(ShapeInfo &s)
 {
-  // the plan depends on pointer alignment, which is not known yet: cover both cases
-  const Plan a = plan_for(dim0, C, N, true), b = plan_for(dim0, C, N, false);
-  uint64_t need = a.ws_bytes > b.ws_bytes ? a.ws_bytes : b.ws_bytes;
-  for (int dir = 0; dir < 2; ++dir) {
-    Plan rp; RingGeom g;
-    if (ring_plan_for(dim0, C, N, true, dir, rp, g) && rp.ws_bytes > need) need = rp.ws_bytes;
+  const Tunables &t = tunables();
+  // the plan depends on pointer alignment, which is not known when a workspace is sized: cover both cases
+  uint64_t need = 0;
+  for (int al = 0; al < 2; ++al) {
+    s.plan[al] = make_plan(s.dim0, s.C, s.N, al != 0, sm_count() * t.blocks_per_sm, t.tile_floats, 1);
+    if (s.plan[al].ws_bytes > need) need = s.plan[al].ws_bytes;
   }
-  return align_up_u64(need, 256);
+  for (int dir = 0; dir < 2; ++dir) {
+    s.ring_ok[dir] = make_ring_plan(s.dim0, s.C, s.N, dir, s.ring_plan[dir], s.ring_geom[dir]);
+    if (s.ring_ok[dir] && s.ring_plan[dir].ws_bytes > need) need = s.ring_plan[dir].ws_bytes;
+  }
+  s.tiled_bytes = align_up_u64(need, 256);
+  s.part_bytes = align_up_u64(s.tiled_bytes + resident_ws_bytes(s.dim0, s.C, s.N), 256);
 }
 
-uint64_t workspace_part_bytes(uint32_t dim0, uint32_t C, uint32_t N)
-{
-  return align_up_u64(tiled_part_bytes(dim0, C, N) + resident_ws_bytes(dim0, C, N), 256);
-}
+// Bytes of a part taken by the tile-plan kernels (plain, warp-specialised, cluster); the records of the
+// slice-resident kernel follow behind them.
+static uint64_t tiled_part_bytes(uint32_t dim0, uint32_t C, uint32_t N) { return shape_info(dim0, C, N).tiled_bytes; }
+
+uint64_t workspace_part_bytes(uint32_t dim0, uint32_t C, uint32_t N) { return shape_info(dim0, C, N).part_bytes; }
 
 // Bytes at the start of a workspace that hold progress counters, flags and records, i.e. what has
 // to be zero when a launch begins (the per-tile partials behind them are written before they are read).
