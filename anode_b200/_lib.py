@@ -126,6 +126,32 @@ def load():
     return lib
 
 
+_native = None
+_addresses = {}
+
+
+def address(name):
+    """Address of a function of the loaded library."""
+    a = _addresses.get(name)
+    if a is None:
+        a = _addresses[name] = ctypes.cast(getattr(load(), name), ctypes.c_void_p).value
+    return a
+
+
+def native():
+    """The extension module with the hot entry points' Python side (csrc/bn_py.cpp), bound to the loaded library."""
+    global _native
+    if _native is None:
+        load()
+        try:
+            from . import _native as module
+        except ImportError as e:
+            raise ImportError("anode_b200/_native.so is not built: run `python -m anode_b200.build` (%s)" % e)
+        module.bind({name: address(name) for name in SIGNATURES})
+        _native = module
+    return _native
+
+
 ERRORS = {
     -1: "ANODE_E_NULL: a required pointer is NULL",
     -2: "ANODE_E_DIMS: a dimension is 0 or the tensor has 2^32 or more elements",

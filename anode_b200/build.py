@@ -1,4 +1,5 @@
-"""Builds libanode_routines_gpu.so in-tree with plain nvcc (sm_100a only).
+"""Builds libanode_routines_gpu.so in-tree with plain nvcc (sm_100a only), and _native.so, the Python side of the hot
+entry points, with the host compiler.
 
 The flags follow the reference's own recipe where they matter for numerics
 (build.rs:47-48: -prec-div=true -prec-sqrt=true); the architecture list is replaced by the
@@ -11,6 +12,8 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libanode_routines_gpu.so")
+NATIVE = os.path.join(HERE, "_native.so")
+NATIVE_SOURCE = os.path.join(CSRC, "bn_py.cpp")
 SOURCES = ["bn_fused.cu", "bn_legacy.cu", "bn_sync.cu", "bn_static.cu", "bn_hoststep.cu", "bn_segres.cu", "bn_infer.cu", "bn_resident.cu", "bn_resident_diag.cpp"]
 HEADERS = ["bn_plan.h", "bn_device.cuh", "bn_fused.cuh", "bn_ring.cuh", "bn_resident_plan.h", "bn_host.h", "bn_sync.h",
            os.path.join("..", "..", "include", "anode_routines_gpu.h")]
@@ -48,7 +51,28 @@ def _stale():
     return any(os.path.exists(d) and os.path.getmtime(d) > t for d in deps)
 
 
+def build_native(force=False):
+    """The CPython module anode_b200._native: compiled against this interpreter's and torch's headers, linked against
+    torch only (the C ABI is handed to it as addresses at run time)."""
+    if not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) > os.path.getmtime(NATIVE_SOURCE):
+        return NATIVE
+    import sysconfig
+    import torch
+    root = os.path.dirname(torch.__file__)
+    tmp = NATIVE + ".tmp%d" % os.getpid()
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
+           "-I", os.path.join(root, "include"), "-I", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           "-I", os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include"), "-I", sysconfig.get_paths()["include"],
+           NATIVE_SOURCE, "-o", tmp, "-L", os.path.join(root, "lib"),
+           "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    subprocess.check_call(cmd)
+    os.replace(tmp, NATIVE)
+    return NATIVE
+
+
 def build_library(force=False, verbose=False):
+    build_native(force)
     if not force and not _stale():
         return LIB
     nvcc = os.environ.get("NVCC", "nvcc")

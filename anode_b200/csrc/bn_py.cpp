@@ -1,0 +1,284 @@
+// Python side of the hot entry points: argument checks, tensor -> pointer, current stream and the C call in one
+// native step.  A layer call through ctypes spent 12 - 20 us in the interpreter (one Python-level check per tensor,
+// a stream object, twenty boxed arguments), several times the duration of the kernel on small layers; the same work
+// here takes well under a microsecond.  The functions of the C ABI come in as addresses (bind), so this module is
+// linked against nothing but Python and torch, and a library chosen at run time is honoured.
+//
+// Arguments mirror anode_b200/ops.py, which keeps the public signatures, defaults and error types.
+#include <torch/csrc/autograd/python_variable.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <stdint.h>
+
+namespace {
+
+struct KernelConfig { uint32_t block_sz, max_block_ct; };
+
+// addresses of the C ABI, in the order of kNames
+enum { F_FWD, F_FWD_ACT, F_FWD_ADD, F_BWD, F_BWD_ACT, F_BWD_ADD, F_INFER, F_COUNT };
+const char *const kNames[F_COUNT] = {
+    "anode_gpu_batch_norm_relu_fused_fwd_3d1_packed_f32", "anode_gpu_batch_norm_act_fused_fwd_3d1_packed_f32",
+    "anode_gpu_batch_norm_add_act_fused_fwd_3d1_packed_f32", "anode_gpu_batch_norm_relu_fused_bwd_3d1_packed_f32",
+    "anode_gpu_batch_norm_act_fused_bwd_3d1_packed_f32", "anode_gpu_batch_norm_add_act_fused_bwd_3d1_packed_f32",
+    "anode_gpu_batch_norm_act_infer_3d1_packed_f32"};
+void *g_fn[F_COUNT] = {};
+
+typedef const float *In;
+typedef float *Out;
+typedef int (*FwdFn)(uint32_t, uint32_t, uint32_t, float, float, int, In, In, In, Out, Out, Out, Out, Out, void *, size_t, const KernelConfig *, void *);
+typedef int (*FwdActFn)(uint32_t, uint32_t, uint32_t, float, float, float, In, In, In, Out, Out, Out, Out, Out, void *, size_t, const KernelConfig *, void *);
+typedef int (*FwdAddFn)(uint32_t, uint32_t, uint32_t, float, float, float, In, In, In, In, Out, Out, Out, Out, Out, void *, size_t, const KernelConfig *, void *);
+typedef int (*BwdFn)(uint32_t, uint32_t, uint32_t, int, int, In, In, In, In, In, In, Out, Out, Out, void *, size_t, const KernelConfig *, void *);
+typedef int (*BwdActFn)(uint32_t, uint32_t, uint32_t, float, int, In, In, In, In, In, In, Out, Out, Out, void *, size_t, const KernelConfig *, void *);
+typedef int (*BwdAddFn)(uint32_t, uint32_t, uint32_t, float, int, In, In, In, In, In, In, In, Out, Out, Out, Out, void *, size_t, const KernelConfig *, void *);
+typedef int (*InferFn)(uint32_t, uint32_t, uint32_t, float, In, In, In, In, In, Out, const KernelConfig *, void *);
+
+// One call's arguments: the first failure sets the Python error and every later access is harmless.
+struct Args {
+  PyObject *const *v;
+  bool ok = true;
+
+  const at::Tensor *tensor(int i, bool null_ok)
+  {
+    if (v[i] == Py_None && null_ok) return nullptr;
+    if (!THPVariable_Check(v[i])) {
+      if (ok) PyErr_SetString(PyExc_ValueError, "expected a contiguous float32 CUDA tensor");
+      ok = false;
+      return nullptr;
+    }
+    return &THPVariable_Unpack(v[i]);
+  }
+  // device pointer of a packed f32 array (the reference only implements packed arrays too, src/ops_gpu.rs:3777-3779)
+  Out ptr(int i, bool null_ok = true)
+  {
+    const at::Tensor *t = tensor(i, null_ok);
+    if (!t) return nullptr;
+    if (!(t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous())) {
+      if (ok) PyErr_SetString(PyExc_ValueError, "expected a contiguous float32 CUDA tensor");
+      ok = false;
+      return nullptr;
+    }
+    return static_cast<float *>(t->data_ptr());
+  }
+  float f(int i)
+  {
+    const double d = PyFloat_AsDouble(v[i]);
+    if (d == -1.0 && PyErr_Occurred()) ok = false;
+    return (float)d;
+  }
+  int truth(int i)
+  {
+    const int r = PyObject_IsTrue(v[i]);
+    if (r < 0) ok = false;
+    return r > 0;
+  }
+  size_t size(int i)
+  {
+    const size_t r = PyLong_AsSize_t(v[i]);
+    if (r == (size_t)-1 && PyErr_Occurred()) ok = false;
+    return r;
+  }
+  void *raw(int i)
+  {
+    const at::Tensor *t = tensor(i, true);
+    return t ? t->data_ptr() : nullptr;
+  }
+  // a torch stream, or None for the current one
+  void *stream(int i)
+  {
+    if (v[i] == Py_None) return c10::cuda::getCurrentCUDAStream().stream();
+    PyObject *h = PyObject_GetAttrString(v[i], "cuda_stream");
+    if (!h) { ok = false; return nullptr; }
+    void *p = PyLong_AsVoidPtr(h);
+    Py_DECREF(h);
+    if (PyErr_Occurred()) ok = false;
+    return p;
+  }
+  // [N, C, *spatial] -> (dim0, dim1, dim2) as the apply closures compute them (src/ops_gpu.rs:3764-3766, :4911-4913);
+  // `axes` (None: not checked) must be the positions of the spatial dimensions (src/ops_gpu.rs:3736)
+  void dims(int axes, int i, uint32_t d[3])
+  {
+    const at::Tensor *t = tensor(i, false);
+    if (!t) return;
+    const int64_t nd = t->dim();
+    if (axes >= 0 && v[axes] != Py_None) {
+      bool same = true;
+      const Py_ssize_t n = PySequence_Size(v[axes]);
+      if (n < 0) { ok = false; return; }
+      same = n == (nd > 2 ? nd - 2 : 0);
+      for (Py_ssize_t k = 0; same && k < n; ++k) {
+        PyObject *e = PySequence_GetItem(v[axes], k);
+        if (!e) { ok = false; return; }
+        same = PyLong_AsLong(e) == (long)k;
+        Py_DECREF(e);
+        if (PyErr_Occurred()) PyErr_Clear();
+      }
+      if (!same) {
+        PyObject *want = PyList_New(0);
+        for (int64_t k = 0; k + 2 < nd; ++k) { PyObject *e = PyLong_FromLongLong(k); PyList_Append(want, e); Py_DECREF(e); }
+        if (ok) PyErr_Format(PyExc_ValueError, "axes must be %R for a %d-D batch array", want, (int)(nd - 2));
+        Py_DECREF(want);
+        ok = false;
+        return;
+      }
+    }
+    if (nd < 2) { if (ok) PyErr_SetString(PyExc_IndexError, "expected an array [N, C, *spatial]"); ok = false; return; }
+    uint64_t d0 = 1;
+    for (int64_t k = 2; k < nd; ++k) d0 *= (uint64_t)t->size(k);
+    d[0] = (uint32_t)d0; d[1] = (uint32_t)t->size(1); d[2] = (uint32_t)t->size(0);
+  }
+};
+
+bool want_args(Py_ssize_t n, Py_ssize_t want)
+{
+  if (n == want) return true;
+  PyErr_Format(PyExc_TypeError, "expected %zd arguments, got %zd", want, n);
+  return false;
+}
+bool bound(int which)
+{
+  if (g_fn[which]) return true;
+  PyErr_SetString(PyExc_ImportError, "the CUDA library is not loaded");
+  return false;
+}
+const KernelConfig kDefaultCfg = {1024, 148 * 32};     // ops.py's default launch hint (the kernels choose their own shapes)
+
+// fwd(axes, epsilon, avg_rate, x, residual, y, mean, var, avg_mean, avg_var, gamma, beta, relu, neg_slope | None, ws, ws_bytes, stream)
+PyObject *py_fwd(PyObject *, PyObject *const *v, Py_ssize_t n)
+{
+  if (!want_args(n, 17)) return nullptr;
+  Args a{v};
+  uint32_t d[3] = {0, 0, 0};
+  a.dims(0, 3, d);
+  const float eps = a.f(1), rate = a.f(2);
+  const bool add = v[4] != Py_None, act = add || v[13] != Py_None;
+  In x = a.ptr(3), res = a.ptr(4), gamma = a.ptr(10), beta = a.ptr(11);
+  Out y = a.ptr(5), mean = a.ptr(6), var = a.ptr(7), rm = a.ptr(8), rv = a.ptr(9);
+  const float slope = v[13] != Py_None ? a.f(13) : 0.f;
+  const int relu = a.truth(12);
+  void *ws = a.raw(14);
+  const size_t bytes = a.size(15);
+  void *s = a.stream(16);
+  if (!a.ok) return nullptr;
+  const int which = add ? F_FWD_ADD : act ? F_FWD_ACT : F_FWD;
+  if (!bound(which)) return nullptr;
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  if (add) rc = ((FwdAddFn)g_fn[which])(d[0], d[1], d[2], eps, rate, slope, x, res, gamma, beta, y, mean, var, rm, rv, ws, bytes, &kDefaultCfg, s);
+  else if (act) rc = ((FwdActFn)g_fn[which])(d[0], d[1], d[2], eps, rate, slope, x, gamma, beta, y, mean, var, rm, rv, ws, bytes, &kDefaultCfg, s);
+  else rc = ((FwdFn)g_fn[which])(d[0], d[1], d[2], eps, rate, relu, x, gamma, beta, y, mean, var, rm, rv, ws, bytes, &kDefaultCfg, s);
+  Py_END_ALLOW_THREADS
+  return PyLong_FromLong(rc);
+}
+
+// bwd(axes, dy, x, y | None, mean, var, dx, dresidual, gamma, beta, dgamma, dbeta, relu, neg_slope | None, accumulate, ws, ws_bytes, stream)
+PyObject *py_bwd(PyObject *, PyObject *const *v, Py_ssize_t n)
+{
+  if (!want_args(n, 18)) return nullptr;
+  Args a{v};
+  uint32_t d[3] = {0, 0, 0};
+  a.dims(0, 2, d);
+  const bool add = v[3] != Py_None, act = add || v[13] != Py_None;
+  In dy = a.ptr(1), x = a.ptr(2), y = a.ptr(3), mean = a.ptr(4), var = a.ptr(5), gamma = a.ptr(8), beta = a.ptr(9);
+  Out dx = a.ptr(6), dres = a.ptr(7), dg = a.ptr(10), db = a.ptr(11);
+  const float slope = v[13] != Py_None ? a.f(13) : 0.f;
+  const int relu = a.truth(12), acc = a.truth(14);
+  void *ws = a.raw(15);
+  const size_t bytes = a.size(16);
+  void *s = a.stream(17);
+  if (!a.ok) return nullptr;
+  const int which = add ? F_BWD_ADD : act ? F_BWD_ACT : F_BWD;
+  if (!bound(which)) return nullptr;
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  if (add) rc = ((BwdAddFn)g_fn[which])(d[0], d[1], d[2], slope, acc, dy, x, y, mean, var, gamma, beta, dx, dres, dg, db, ws, bytes, &kDefaultCfg, s);
+  else if (act) rc = ((BwdActFn)g_fn[which])(d[0], d[1], d[2], slope, acc, dy, x, mean, var, gamma, beta, dx, dg, db, ws, bytes, &kDefaultCfg, s);
+  else rc = ((BwdFn)g_fn[which])(d[0], d[1], d[2], relu, acc, dy, x, mean, var, gamma, beta, dx, dg, db, ws, bytes, &kDefaultCfg, s);
+  Py_END_ALLOW_THREADS
+  return PyLong_FromLong(rc);
+}
+
+// infer(axes, x, mean, var, y, gamma, beta, neg_slope, stream)
+PyObject *py_infer(PyObject *, PyObject *const *v, Py_ssize_t n)
+{
+  if (!want_args(n, 9)) return nullptr;
+  Args a{v};
+  uint32_t d[3] = {0, 0, 0};
+  a.dims(0, 1, d);
+  In x = a.ptr(1), mean = a.ptr(2), var = a.ptr(3), gamma = a.ptr(5), beta = a.ptr(6);
+  Out y = a.ptr(4);
+  const float slope = a.f(7);
+  void *s = a.stream(8);
+  if (!a.ok || !bound(F_INFER)) return nullptr;
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = ((InferFn)g_fn[F_INFER])(d[0], d[1], d[2], slope, x, mean, var, gamma, beta, y, &kDefaultCfg, s);
+  Py_END_ALLOW_THREADS
+  return PyLong_FromLong(rc);
+}
+
+// packed(address, axes, like, tensors, epsilon | None, stream): one of the reference's own entry points.  `like` gives
+// (dim0, dim1, dim2) when axes is not False, else the element count; tensors are the pointers in the order of the C call.
+PyObject *py_packed(PyObject *, PyObject *const *v, Py_ssize_t n)
+{
+  if (!want_args(n, 6)) return nullptr;
+  void *fn = PyLong_AsVoidPtr(v[0]);
+  if (PyErr_Occurred()) return nullptr;
+  Args a{v};
+  if (!PyTuple_Check(v[3])) { PyErr_SetString(PyExc_TypeError, "tensors: a tuple"); return nullptr; }
+  const Py_ssize_t k = PyTuple_GET_SIZE(v[3]);
+  if (k < 2 || k > 5 || !fn) { PyErr_SetString(PyExc_TypeError, "2 to 5 tensors"); return nullptr; }
+  PyObject *items[5];
+  for (Py_ssize_t i = 0; i < k; ++i) items[i] = PyTuple_GET_ITEM(v[3], i);
+  Args t{items};
+  void *p[5] = {};
+  for (Py_ssize_t i = 0; i < k; ++i) p[i] = t.ptr((int)i);
+  void *s = a.stream(5);
+  if (!t.ok) return nullptr;
+  const KernelConfig *cfg = &kDefaultCfg;
+  const bool flat = v[1] == Py_False, with_eps = v[4] != Py_None;
+  uint32_t d[3] = {0, 0, 0};
+  if (flat) { const at::Tensor *x = a.tensor(2, false); if (x) d[0] = (uint32_t)x->numel(); }
+  else a.dims(1, 2, d);
+  const float eps = with_eps ? a.f(4) : 0.f;
+  if (!a.ok) return nullptr;
+  if ((flat && k > 3) || (with_eps && k != 3)) { PyErr_SetString(PyExc_TypeError, "no entry point takes these arguments"); return nullptr; }
+  typedef void *P;
+  typedef const KernelConfig *K;
+  Py_BEGIN_ALLOW_THREADS
+  if (flat && k == 2) ((void (*)(uint32_t, P, P, K, P))fn)(d[0], p[0], p[1], cfg, s);
+  else if (flat) ((void (*)(uint32_t, P, P, P, K, P))fn)(d[0], p[0], p[1], p[2], cfg, s);
+  else if (with_eps) ((void (*)(uint32_t, uint32_t, uint32_t, float, P, P, P, K, P))fn)(d[0], d[1], d[2], eps, p[0], p[1], p[2], cfg, s);
+  else if (k == 2) ((void (*)(uint32_t, uint32_t, uint32_t, P, P, K, P))fn)(d[0], d[1], d[2], p[0], p[1], cfg, s);
+  else if (k == 3) ((void (*)(uint32_t, uint32_t, uint32_t, P, P, P, K, P))fn)(d[0], d[1], d[2], p[0], p[1], p[2], cfg, s);
+  else if (k == 4) ((void (*)(uint32_t, uint32_t, uint32_t, P, P, P, P, K, P))fn)(d[0], d[1], d[2], p[0], p[1], p[2], p[3], cfg, s);
+  else ((void (*)(uint32_t, uint32_t, uint32_t, P, P, P, P, P, K, P))fn)(d[0], d[1], d[2], p[0], p[1], p[2], p[3], p[4], cfg, s);
+  Py_END_ALLOW_THREADS
+  Py_RETURN_NONE;
+}
+
+// bind({name: address}): the C ABI's functions
+PyObject *py_bind(PyObject *, PyObject *const *v, Py_ssize_t n)
+{
+  if (!want_args(n, 1)) return nullptr;
+  for (int i = 0; i < F_COUNT; ++i) {
+    PyObject *e = PyDict_GetItemString(v[0], kNames[i]);
+    if (!e) { PyErr_Format(PyExc_KeyError, "%s", kNames[i]); return nullptr; }
+    g_fn[i] = PyLong_AsVoidPtr(e);
+    if (PyErr_Occurred()) return nullptr;
+  }
+  Py_RETURN_NONE;
+}
+
+PyMethodDef kMethods[] = {
+    {"bind", (PyCFunction)(void *)py_bind, METH_FASTCALL, nullptr},
+    {"fwd", (PyCFunction)(void *)py_fwd, METH_FASTCALL, nullptr},
+    {"bwd", (PyCFunction)(void *)py_bwd, METH_FASTCALL, nullptr},
+    {"infer", (PyCFunction)(void *)py_infer, METH_FASTCALL, nullptr},
+    {"packed", (PyCFunction)(void *)py_packed, METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", "Fast paths of anode_b200.ops into the C ABI.", -1, kMethods};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__native(void) { return PyModule_Create(&kModule); }

@@ -16,7 +16,7 @@ import enum
 import torch
 
 from . import _lib
-from ._lib import AnodeError, KernelConfig, check  # noqa: F401  (re-exported)
+from ._lib import AnodeError, KernelConfig, check, native  # noqa: F401  (re-exported)
 
 
 class WriteCap(enum.Enum):
@@ -26,10 +26,11 @@ class WriteCap(enum.Enum):
 
 
 _DEFAULT_CFG = KernelConfig(1024, 148 * 32)
+_DEFAULT_CFG_REF = ctypes.byref(_DEFAULT_CFG)
 
 
 def _cfg(cfg):
-    return ctypes.byref(cfg if cfg is not None else _DEFAULT_CFG)
+    return ctypes.byref(cfg) if cfg is not None else _DEFAULT_CFG_REF
 
 
 def _stream(stream):
@@ -64,13 +65,10 @@ def dims_of(x, axes=None):
     return d0, int(x.shape[1]), int(x.shape[0])
 
 
-def _call(name, *args):
-    getattr(_lib.load(), name)(*args)
-
-
-def _dims(x):
-    d0, c, n = dims_of(x)
-    return ctypes.c_uint32(d0), ctypes.c_uint32(c), ctypes.c_uint32(n)
+def _packed(name, axes, x, tensors, stream, epsilon=None):
+    """One of the reference's entry points on [N, C, *spatial] arrays (axes False: on flat arrays).  The launch hint
+    (`cfg` of the ops) is not passed on: the kernels choose their own launch shapes."""
+    native().packed(_lib.address(name), axes, x, tensors, epsilon, stream)
 
 
 # --------------------------------------------------------------------------------------------
@@ -82,10 +80,9 @@ class BatchMean2dOp:
     """src/ops_gpu.rs:3690-3800.  Accumulate is `unimplemented!()` there and rejected here."""
     @staticmethod
     def apply(axes, x, mean, cap=WriteCap.Assign, cfg=None, stream=None):
-        dims_of(x, axes)
         if cap is not WriteCap.Assign:
             raise NotImplementedError("BatchMean2dOp: Accumulate (unimplemented in the reference)")
-        _call("anode_gpu_batch_mean_3d1_packed_f32", *_dims(x), _p(x), _p(mean), _cfg(cfg), _stream(stream))
+        _packed("anode_gpu_batch_mean_3d1_packed_f32", axes, x, (x, mean), stream)
         return mean
 
 
@@ -93,10 +90,9 @@ class BatchMean2dBwdOp:
     """src/ops_gpu.rs:3803-3911."""
     @staticmethod
     def apply(axes, dmean, x, dx, cap=WriteCap.Assign, cfg=None, stream=None):
-        dims_of(x, axes)
         name = "anode_gpu_batch_mean_bwd_3d1_packed_f32" if cap is WriteCap.Assign else \
             "anode_gpu_batch_mean_bwd_3d1_packed_accumulate_f32"
-        _call(name, *_dims(x), _p(dmean), _p(dx), _cfg(cfg), _stream(stream))
+        _packed(name, axes, x, (dmean, dx), stream)
         return dx
 
 
@@ -104,11 +100,9 @@ class BatchVariance2dOp:
     """src/ops_gpu.rs:3913-4010.  The stored variance includes epsilon."""
     @staticmethod
     def apply(axes, epsilon, x, mean, var, cap=WriteCap.Assign, cfg=None, stream=None):
-        dims_of(x, axes)
         if cap is not WriteCap.Assign:
             raise NotImplementedError("BatchVariance2dOp: Accumulate (unimplemented in the reference)")
-        _call("anode_gpu_batch_var_3d1_packed_f32", *_dims(x), ctypes.c_float(epsilon), _p(x), _p(mean),
-              _p(var), _cfg(cfg), _stream(stream))
+        _packed("anode_gpu_batch_var_3d1_packed_f32", axes, x, (x, mean, var), stream, epsilon)
         return var
 
 
@@ -116,10 +110,9 @@ class BatchVariance2dBwdOp:
     """src/ops_gpu.rs:4012-4130."""
     @staticmethod
     def apply(axes, dvar, x, mean, dx, cap=WriteCap.Assign, cfg=None, stream=None):
-        dims_of(x, axes)
         name = "anode_gpu_batch_var_bwd_3d1_packed_f32" if cap is WriteCap.Assign else \
             "anode_gpu_batch_var_bwd_3d1_packed_accumulate_f32"
-        _call(name, *_dims(x), _p(dvar), _p(x), _p(mean), _p(dx), _cfg(cfg), _stream(stream))
+        _packed(name, axes, x, (dvar, x, mean, dx), stream)
         return dx
 
 
@@ -127,10 +120,9 @@ class BatchVariance2dBwdMeanOp:
     """src/ops_gpu.rs:4132-4247."""
     @staticmethod
     def apply(axes, dvar, x, mean, dmean, cap=WriteCap.Assign, cfg=None, stream=None):
-        dims_of(x, axes)
         name = "anode_gpu_batch_var_bwd_mean_3d1_packed_f32" if cap is WriteCap.Assign else \
             "anode_gpu_batch_var_bwd_mean_3d1_packed_accumulate_f32"
-        _call(name, *_dims(x), _p(dvar), _p(x), _p(mean), _p(dmean), _cfg(cfg), _stream(stream))
+        _packed(name, axes, x, (dvar, x, mean, dmean), stream)
         return dmean
 
 
@@ -138,11 +130,9 @@ class BatchNormalize2dOp:
     """src/ops_gpu.rs:4249-4362."""
     @staticmethod
     def apply(axes, x, mean, var, y, cap=WriteCap.Assign, cfg=None, stream=None):
-        dims_of(x, axes)
         if cap is not WriteCap.Assign:
             raise NotImplementedError("BatchNormalize2dOp: Accumulate (unimplemented in the reference)")
-        _call("anode_gpu_batch_norm_3d1_packed_f32", *_dims(x), _p(x), _p(mean), _p(var), _p(y),
-              _cfg(cfg), _stream(stream))
+        _packed("anode_gpu_batch_norm_3d1_packed_f32", axes, x, (x, mean, var, y), stream)
         return y
 
 
@@ -150,10 +140,9 @@ class BatchNormalize2dBwdOp:
     """src/ops_gpu.rs:4364-4474."""
     @staticmethod
     def apply(axes, dy, var, dx, cap=WriteCap.Assign, cfg=None, stream=None):
-        dims_of(dy, axes)
         name = "anode_gpu_batch_norm_bwd_3d1_packed_f32" if cap is WriteCap.Assign else \
             "anode_gpu_batch_norm_bwd_3d1_packed_accumulate_f32"
-        _call(name, *_dims(dy), _p(dy), _p(var), _p(dx), _cfg(cfg), _stream(stream))
+        _packed(name, axes, dy, (dy, var, dx), stream)
         return dx
 
 
@@ -161,10 +150,9 @@ class BatchNormalize2dBwdMeanOp:
     """src/ops_gpu.rs:4476-4584."""
     @staticmethod
     def apply(axes, dy, var, dmean, cap=WriteCap.Assign, cfg=None, stream=None):
-        dims_of(dy, axes)
         name = "anode_gpu_batch_norm_bwd_mean_3d1_packed_f32" if cap is WriteCap.Assign else \
             "anode_gpu_batch_norm_bwd_mean_3d1_packed_accumulate_f32"
-        _call(name, *_dims(dy), _p(dy), _p(var), _p(dmean), _cfg(cfg), _stream(stream))
+        _packed(name, axes, dy, (dy, var, dmean), stream)
         return dmean
 
 
@@ -173,18 +161,16 @@ class BatchNormalize2dBwdVarianceOp:
     saved normalized output instead of x."""
     @staticmethod
     def apply(axes, dy, x, mean, var, dvar, cap=WriteCap.Assign, cfg=None, stream=None):
-        dims_of(x, axes)
         name = "anode_gpu_batch_norm_bwd_var_3d1_packed_f32" if cap is WriteCap.Assign else \
             "anode_gpu_batch_norm_bwd_var_3d1_packed_accumulate_f32"
-        _call(name, *_dims(x), _p(dy), _p(x), _p(mean), _p(var), _p(dvar), _cfg(cfg), _stream(stream))
+        _packed(name, axes, x, (dy, x, mean, var, dvar), stream)
         return dvar
 
     @staticmethod
     def apply_v2(axes, dy, y, var, dvar, cap=WriteCap.Assign, cfg=None, stream=None):
-        dims_of(y, axes)
         name = "anode_gpu_batch_norm_bwd_var_v2_3d1_packed_f32" if cap is WriteCap.Assign else \
             "anode_gpu_batch_norm_bwd_var_v2_3d1_packed_accumulate_f32"
-        _call(name, *_dims(y), _p(dy), _p(y), _p(var), _p(dvar), _cfg(cfg), _stream(stream))
+        _packed(name, axes, y, (dy, y, var, dvar), stream)
         return dvar
 
 
@@ -211,8 +197,7 @@ class PositiveClipOp:
     is the in-place form of PositiveClipClobberOp (:8584-8671)."""
     @staticmethod
     def apply(x, y, cfg=None, stream=None):
-        _call("anode_gpu_positive_clip_flat_map_f32", ctypes.c_uint32(x.numel()), _p(x), _p(y),
-              _cfg(cfg), _stream(stream))
+        _packed("anode_gpu_positive_clip_flat_map_f32", False, x, (x, y), stream)
         return y
 
 
@@ -220,8 +205,7 @@ class PositiveClipBwdOp:
     """src/ops_gpu.rs:8499-8582: dx = dy * (y > 0); `dx is dy` is the clobber form (:8673-8755)."""
     @staticmethod
     def apply(dy, y, dx, cfg=None, stream=None):
-        _call("anode_gpu_positive_clip_flat_map_bwd_f32", ctypes.c_uint32(dy.numel()), _p(dy), _p(y), _p(dx),
-              _cfg(cfg), _stream(stream))
+        _packed("anode_gpu_positive_clip_flat_map_bwd_f32", False, dy, (dy, y, dx), stream)
         return dx
 
 
@@ -229,8 +213,7 @@ class FlatJoinOp:
     """src/ops_gpu.rs:8169-8261: y = x1 * step(x2) (routines_gpu/flat_join.cu:50-60)."""
     @staticmethod
     def apply(x1, x2, y, cfg=None, stream=None):
-        _call("anode_gpu_M1_copy_map_M2_unit_step_map_R_product_reduce_flat_join_f32",
-              ctypes.c_uint32(x1.numel()), _p(x1), _p(x2), _p(y), _cfg(cfg), _stream(stream))
+        _packed("anode_gpu_M1_copy_map_M2_unit_step_map_R_product_reduce_flat_join_f32", False, x1, (x1, x2, y), stream)
         return y
 
 
@@ -343,25 +326,21 @@ class Workspace:
               "workspace_init")
 
 
+def _scratch(workspace, x):
+    return workspace if workspace is not None else Workspace(*dims_of(x), x.device)
+
+
 class BatchNormalize2dFusedOp:
     """Forward: statistics, running averages, normalize, affine, ReLU in one launch."""
     @staticmethod
     def apply(axes, epsilon, avg_rate, x, y, mean, var, avg_mean=None, avg_var=None, gamma=None, beta=None,
               relu=True, workspace=None, cfg=None, stream=None, neg_slope=None):
-        d0, c, n = dims_of(x, axes)
-        ws = workspace if workspace is not None else Workspace(d0, c, n, x.device)
-        if neg_slope is not None:      # general activation t*(t > 0 ? 1 : neg_slope), e.g. leaky ReLU
-            check(_lib.load().anode_gpu_batch_norm_act_fused_fwd_3d1_packed_f32(
-                d0, c, n, ctypes.c_float(epsilon), ctypes.c_float(avg_rate), ctypes.c_float(neg_slope),
-                _p(x), _p(gamma), _p(beta), _p(y), _p(mean), _p(var), _p(avg_mean), _p(avg_var),
-                ws.ptr, ws.bytes, _cfg(cfg), _stream(stream)),
-                "anode_gpu_batch_norm_act_fused_fwd_3d1_packed_f32")
-            return y
-        check(_lib.load().anode_gpu_batch_norm_relu_fused_fwd_3d1_packed_f32(
-            d0, c, n, ctypes.c_float(epsilon), ctypes.c_float(avg_rate), int(bool(relu)),
-            _p(x), _p(gamma), _p(beta), _p(y), _p(mean), _p(var), _p(avg_mean), _p(avg_var),
-            ws.ptr, ws.bytes, _cfg(cfg), _stream(stream)),
-            "anode_gpu_batch_norm_relu_fused_fwd_3d1_packed_f32")
+        # neg_slope: general activation t*(t > 0 ? 1 : neg_slope), e.g. leaky ReLU
+        ws = _scratch(workspace, x)
+        rc = native().fwd(axes, epsilon, avg_rate, x, None, y, mean, var, avg_mean, avg_var, gamma, beta, relu, neg_slope,
+                          ws.buf, ws.bytes, stream)
+        if rc:
+            check(rc, "anode_gpu_batch_norm_%s_fused_fwd_3d1_packed_f32" % ("relu" if neg_slope is None else "act"))
         return y
 
 
@@ -370,20 +349,11 @@ class BatchNormalize2dBwdFusedOp:
     @staticmethod
     def apply(axes, dy, x, mean, var, dx, gamma=None, beta=None, dgamma=None, dbeta=None, relu=True,
               cap=WriteCap.Assign, workspace=None, cfg=None, stream=None, neg_slope=None):
-        d0, c, n = dims_of(x, axes)
-        ws = workspace if workspace is not None else Workspace(d0, c, n, x.device)
-        if neg_slope is not None:
-            check(_lib.load().anode_gpu_batch_norm_act_fused_bwd_3d1_packed_f32(
-                d0, c, n, ctypes.c_float(neg_slope), int(cap is WriteCap.Accumulate),
-                _p(dy), _p(x), _p(mean), _p(var), _p(gamma), _p(beta), _p(dx), _p(dgamma), _p(dbeta),
-                ws.ptr, ws.bytes, _cfg(cfg), _stream(stream)),
-                "anode_gpu_batch_norm_act_fused_bwd_3d1_packed_f32")
-            return dx
-        check(_lib.load().anode_gpu_batch_norm_relu_fused_bwd_3d1_packed_f32(
-            d0, c, n, int(bool(relu)), int(cap is WriteCap.Accumulate),
-            _p(dy), _p(x), _p(mean), _p(var), _p(gamma), _p(beta), _p(dx), _p(dgamma), _p(dbeta),
-            ws.ptr, ws.bytes, _cfg(cfg), _stream(stream)),
-            "anode_gpu_batch_norm_relu_fused_bwd_3d1_packed_f32")
+        ws = _scratch(workspace, x)
+        rc = native().bwd(axes, dy, x, None, mean, var, dx, None, gamma, beta, dgamma, dbeta, relu, neg_slope,
+                          cap is WriteCap.Accumulate, ws.buf, ws.bytes, stream)
+        if rc:
+            check(rc, "anode_gpu_batch_norm_%s_fused_bwd_3d1_packed_f32" % ("relu" if neg_slope is None else "act"))
         return dx
 
 
@@ -393,23 +363,25 @@ class BatchNormalize2dAddActFusedOp:
     @staticmethod
     def apply(axes, epsilon, avg_rate, x, residual, y, mean, var, avg_mean=None, avg_var=None, gamma=None, beta=None,
               neg_slope=0.0, workspace=None, cfg=None, stream=None):
-        d0, c, n = dims_of(x, axes)
-        ws = workspace if workspace is not None else Workspace(d0, c, n, x.device)
-        check(_lib.load().anode_gpu_batch_norm_add_act_fused_fwd_3d1_packed_f32(
-            d0, c, n, ctypes.c_float(epsilon), ctypes.c_float(avg_rate), ctypes.c_float(neg_slope),
-            _p(x), _p(residual), _p(gamma), _p(beta), _p(y), _p(mean), _p(var), _p(avg_mean), _p(avg_var),
-            ws.ptr, ws.bytes, _cfg(cfg), _stream(stream)), "anode_gpu_batch_norm_add_act_fused_fwd_3d1_packed_f32")
+        ws = _scratch(workspace, x)
+        if residual is None:
+            check(-1, "anode_gpu_batch_norm_add_act_fused_fwd_3d1_packed_f32")
+        rc = native().fwd(axes, epsilon, avg_rate, x, residual, y, mean, var, avg_mean, avg_var, gamma, beta, True, neg_slope,
+                          ws.buf, ws.bytes, stream)
+        if rc:
+            check(rc, "anode_gpu_batch_norm_add_act_fused_fwd_3d1_packed_f32")
         return y
 
     @staticmethod
     def adjoint(axes, dy, x, y, mean, var, dx, dresidual=None, gamma=None, beta=None, dgamma=None, dbeta=None,
                 neg_slope=0.0, cap=WriteCap.Assign, workspace=None, cfg=None, stream=None):
-        d0, c, n = dims_of(x, axes)
-        ws = workspace if workspace is not None else Workspace(d0, c, n, x.device)
-        check(_lib.load().anode_gpu_batch_norm_add_act_fused_bwd_3d1_packed_f32(
-            d0, c, n, ctypes.c_float(neg_slope), int(cap is WriteCap.Accumulate),
-            _p(dy), _p(x), _p(y), _p(mean), _p(var), _p(gamma), _p(beta), _p(dx), _p(dresidual), _p(dgamma), _p(dbeta),
-            ws.ptr, ws.bytes, _cfg(cfg), _stream(stream)), "anode_gpu_batch_norm_add_act_fused_bwd_3d1_packed_f32")
+        ws = _scratch(workspace, x)
+        if y is None:
+            check(-1, "anode_gpu_batch_norm_add_act_fused_bwd_3d1_packed_f32")
+        rc = native().bwd(axes, dy, x, y, mean, var, dx, dresidual, gamma, beta, dgamma, dbeta, True, neg_slope,
+                          cap is WriteCap.Accumulate, ws.buf, ws.bytes, stream)
+        if rc:
+            check(rc, "anode_gpu_batch_norm_add_act_fused_bwd_3d1_packed_f32")
         return dx, dresidual
 
 
@@ -421,10 +393,9 @@ class BatchNormalize2dActInferOp:
     neg_slope 0 = ReLU (positive_clip), 1 = none, c = leaky ReLU (flat_map.cu:44-52)."""
     @staticmethod
     def apply(axes, x, mean, var, y, gamma=None, beta=None, neg_slope=0.0, cfg=None, stream=None):
-        d0, c, n = dims_of(x, axes)
-        check(_lib.load().anode_gpu_batch_norm_act_infer_3d1_packed_f32(
-            d0, c, n, ctypes.c_float(neg_slope), _p(x), _p(mean), _p(var), _p(gamma), _p(beta), _p(y),
-            _cfg(cfg), _stream(stream)), "anode_gpu_batch_norm_act_infer_3d1_packed_f32")
+        rc = native().infer(axes, x, mean, var, y, gamma, beta, neg_slope, stream)
+        if rc:
+            check(rc, "anode_gpu_batch_norm_act_infer_3d1_packed_f32")
         return y
 
 
@@ -447,6 +418,7 @@ class FusedBatchNormRelu:
         self.dgamma = torch.zeros(channels, device=dev) if affine else None
         self.dbeta = torch.zeros(channels, device=dev) if affine else None
         self._ws = None
+        self._ws_shape = None
         self._staging = None
         self._dev = None
         self._x = None
@@ -504,27 +476,36 @@ class FusedBatchNormRelu:
 
     def infer(self, x, out=None):
         """Evaluation mode: normalize with the running averages, then the activation."""
-        axes = list(range(x.dim() - 2))
         y = out if out is not None else torch.empty_like(x)
-        return BatchNormalize2dActInferOp.apply(axes, x, self.avg_mean, self.avg_var, y, self.gamma, self.beta,
-                                                0.0 if self.relu else 1.0)
+        rc = native().infer(None, x, self.avg_mean, self.avg_var, y, self.gamma, self.beta, 0.0 if self.relu else 1.0, None)
+        if rc:
+            check(rc, "anode_gpu_batch_norm_act_infer_3d1_packed_f32")
+        return y
 
     def forward(self, x, out=None):
-        axes = list(range(x.dim() - 2))
         y = out if out is not None else torch.empty_like(x)
-        BatchNormalize2dFusedOp.apply(axes, self.epsilon, self.avg_rate, x, y, self.mean, self.var,
-                                      self.avg_mean, self.avg_var, self.gamma, self.beta, self.relu,
-                                      self._workspace(x))
+        ws = self._ws
+        if ws is None or self._ws_shape != x.shape:
+            ws = self._workspace(x)
+            self._ws_shape = x.shape
+        rc = native().fwd(None, self.epsilon, self.avg_rate, x, None, y, self.mean, self.var, self.avg_mean, self.avg_var,
+                          self.gamma, self.beta, self.relu, None, ws.buf, ws.bytes, None)
+        if rc:
+            check(rc, "anode_gpu_batch_norm_relu_fused_fwd_3d1_packed_f32")
         self._x = x
         return y
 
     def backward(self, dy, out=None):
         x = self._x
-        axes = list(range(x.dim() - 2))
         dx = out if out is not None else torch.empty_like(x)
-        BatchNormalize2dBwdFusedOp.apply(axes, dy, x, self.mean, self.var, dx, self.gamma, self.beta,
-                                         self.dgamma, self.dbeta, self.relu, WriteCap.Assign,
-                                         self._workspace(x))
+        ws = self._ws
+        if ws is None or self._ws_shape != x.shape:
+            ws = self._workspace(x)
+            self._ws_shape = x.shape
+        rc = native().bwd(None, dy, x, None, self.mean, self.var, dx, None, self.gamma, self.beta, self.dgamma, self.dbeta,
+                          self.relu, None, False, ws.buf, ws.bytes, None)
+        if rc:
+            check(rc, "anode_gpu_batch_norm_relu_fused_bwd_3d1_packed_f32")
         return dx
 
 
