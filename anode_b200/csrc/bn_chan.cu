@@ -1,0 +1,307 @@
+// Fused batch-norm (+activation, +residual) for channels that fit the registers of a few thread blocks: small layers,
+// where a kernel's latency is its time, and any row length or alignment.
+//
+// A channel belongs to a TEAM of threads: one warp, one block, or a thread-block cluster of up to eight blocks.  Every
+// thread loads its elements of the channel into registers, all loads in flight at once, and the tensor is read once:
+//   1. warp moments (two passes over registers: mean, then squares about it), or the warp's backward sums;
+//   2. each warp pushes its record into the shared memory of every block of the cluster (one remote store per lane)
+//      and the cluster barrier follows: the only synchronisation of the kernel, and none at all in a one-warp team;
+//   3. every warp merges all records in a fixed order in double precision (bit-identical coefficients everywhere);
+//   4. y (or dx) is computed from the registers and stored.
+//
+// What bounds it: on small layers the chain launch -> load -> barrier -> store, 3 - 4 us; the plain kernel's grid-wide
+// partials, counters and flags took 6 - 15 us for the same layers (figures at chan_preferred).  Elements a team does not own to the full are predicated, so the split is by
+// the flat index inside the channel (row-major over samples): odd rows cost an add and a compare per element, no division.
+//
+// Reference kernels this replaces: routines_gpu/batch_norm.cu:24-57, 125-163, 314-336 (forward), :181-206, 240-280,
+// 354-376, 408-444, 476-515 (backward), flat_map.cu:172-194 (ReLU).
+#include "bn_device.cuh"
+#include "bn_host.h"
+
+namespace anode_b200 {
+
+constexpr uint32_t kChanThreads = 512;       // most threads of a block
+constexpr uint32_t kChanCluster = 8;         // most blocks of a team (the portable cluster size)
+constexpr uint32_t kChanWarpTeams = 4;       // one-warp teams per block
+
+struct ChanGeom {
+  uint32_t vec, floats;      // floats per load (4 or 1) and per thread (the template's F)
+  uint32_t threads, cluster; // team = cluster * threads; threads == 32: one-warp teams, kChanWarpTeams to a block
+  uint32_t d0v, total;       // vectors per row and per channel
+  uint32_t team;             // threads of a team = distance between a thread's vectors
+  uint32_t step_off, step_col, wrap;   // a step of `team` vectors: floats forward, columns forward, floats added when the column wraps
+  double inv_count;
+};
+
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// float4 into the shared memory of block `rank` of the cluster, at the address `p` has in this block
+__device__ __forceinline__ void st_cluster_f4(void *p, uint32_t rank, float4 v)
+{
+  const uint32_t local = (uint32_t)__cvta_generic_to_shared(p);
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(remote), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+
+// F: floats a thread holds per tensor
+template <int DIR, int VEC, int F, bool EXTRA>
+__global__ void __launch_bounds__(kChanThreads, 2) bn_chan_kernel(const FusedArgs a, const ChanGeom g)
+{
+  constexpr int E = F / VEC;
+  __shared__ float4 rec[kChanCluster * kChanThreads / 32];
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool solo = g.threads == 32;                      // one-warp teams
+  const uint32_t csh = (uint32_t)__ffs((int)g.cluster) - 1u;
+  const uint32_t c = solo ? blockIdx.x * kChanWarpTeams + warp : blockIdx.x >> csh;
+  const uint32_t rank = solo ? 0u : blockIdx.x & (g.cluster - 1u);
+  const uint32_t C = a.plan.C;
+  // remote shared memory may only be written once its block runs: announce this block now, collect the others' word
+  // right before the first remote store
+  if (g.cluster > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  const uint32_t t = solo ? lane : rank * g.threads + tid;
+  const uint32_t row = t / g.d0v;
+  const uint32_t col0 = t - row * g.d0v;
+  const uint32_t off0 = row * (C * a.plan.dim0) + c * a.plan.dim0 + col0 * VEC;      // below 2^32 (check_dims)
+  const uint32_t cnt = t < g.total ? (g.total - t - 1) / g.team + 1 : 0;          // this thread's vectors, <= E
+  pdl_wait();
+  pdl_trigger();
+  if (c >= C) return;                                     // (one-warp teams only: the last block may be ragged)
+
+  const float gm = a.gamma ? a.gamma[c] : 1.0f;
+  const float bt = (a.gamma && a.beta) ? a.beta[c] : 0.0f;
+  const bool owner = rank == 0 && (solo || warp == 0) && lane == 0;
+  float mean = 0.f, scale = 0.f, rstd = 0.f, rm = 0.f, rv = 0.f;
+  if (DIR == 1) { mean = a.mean_in[c]; rstd = inv_std(a.var_in[c]); scale = gm * rstd; }
+  else if (owner) { if (a.run_mean) rm = a.run_mean[c]; if (a.run_var) rv = a.run_var[c]; }
+  const float slope = a.neg_slope;      // activation: t * (t > 0 ? 1 : slope)
+
+  Pack<VEC> vx[E], ve[(DIR == 1 || EXTRA) ? E : 1];       // ve: dy, later dz (backward) or the residual (forward)
+  {
+    uint32_t off = off0, col = col0;
+    Pack<VEC> vm[(DIR == 1 && EXTRA) ? E : 1];            // the saved output, which carries the mask
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+      vx[k] = pack_fill<VEC>(0.f);
+      if (DIR == 1 || EXTRA) ve[k] = pack_fill<VEC>(0.f);
+      if (DIR == 1 && EXTRA) vm[k] = pack_fill<VEC>(0.f);
+      if (k < cnt) {
+        vx[k] = Pack<VEC>::load(a.x + off);
+        if (DIR == 1) ve[k] = Pack<VEC>::load(a.dy + off);
+        if (DIR == 0 && EXTRA) ve[k] = Pack<VEC>::load(a.res + off);
+        if (DIR == 1 && EXTRA) vm[k] = Pack<VEC>::load(a.ymask + off);
+      }
+      off += g.step_off; col += g.step_col;
+      if (col >= g.d0v) { col -= g.d0v; off += g.wrap; }
+    }
+    if (DIR == 1) {
+      // x becomes x - mean, dy becomes dz = dy * act'(y)  (routines_gpu/flat_map.cu:191-192)
+#pragma unroll
+      for (int k = 0; k < E; ++k)
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) {
+          const float d = vx[k].v[i] - mean;
+          const float yb = EXTRA ? vm[k].v[i] : fmaf(d, scale, bt);
+          vx[k].v[i] = k < cnt ? d : 0.f;
+          ve[k].v[i] *= yb > 0.0f ? 1.0f : slope;
+        }
+    }
+  }
+
+  // ---- the warp's record
+  float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (DIR == 0) {
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < E; ++k)
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) s += vx[k].v[i];
+    s = warp_sum_all(s);
+    const float n = (float)(__reduce_add_sync(0xffffffffu, cnt) * VEC);
+    const float m = n > 0.f ? __fdividef(s, n) : 0.f;
+    float q = 0.f, dev = 0.f;      // dev: what the division and the sum's rounding left in the mean
+#pragma unroll
+    for (int k = 0; k < E; ++k)
+      if (k < cnt) {
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) { const float d = vx[k].v[i] - m; dev += d; q = fmaf(d, d, q); }
+      }
+    q = warp_sum_all(q); dev = warp_sum_all(dev);
+    r = make_float4(n, m, q, dev);
+  } else {
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < E; ++k)
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) { s1 += ve[k].v[i]; s2 = fmaf(ve[k].v[i], vx[k].v[i], s2); }
+    r.x = warp_sum_all(s1); r.y = warp_sum_all(s2);
+  }
+
+  // ---- all records of the team, merged by every warp
+  double t0 = 0.0, t1 = 0.0;
+  auto add = [&](const float4 &p) {
+    if (DIR == 0) {
+      // sum and sum of squares about zero: sum(x) = n*m + dev, sum(x^2) = q + m*(n*m + 2*dev)
+      const double n = (double)p.x, m = (double)p.y, e = (double)p.w;
+      t0 += fma(n, m, e); t1 += fma(m, fma(n, m, 2.0 * e), (double)p.z);
+    } else { t0 += (double)p.x; t1 += (double)p.y; }
+  };
+  if (solo) {
+    add(r);
+  } else {
+    const uint32_t warps = g.threads >> 5;
+    if (g.cluster > 1) {
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+      if (lane < g.cluster) st_cluster_f4(&rec[rank * warps + warp], lane, r);
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else {
+      if (lane == 0) rec[warp] = r;
+      __syncthreads();
+    }
+    for (uint32_t i = lane; i < warps * g.cluster; i += 32) add(rec[i]);
+    t0 = warp_sum_all(t0); t1 = warp_sum_all(t1);
+  }
+
+  // ---- coefficients and per-channel results
+  float cB = 0.f, cC = 0.f;
+  if (DIR == 0) {
+    const double md = t0 * g.inv_count;
+    mean = (float)md;
+    const float var = (float)(fmax(t1 - t0 * md, 0.0) * g.inv_count + (double)a.epsilon);      // biased, epsilon folded in (batch_norm.cu:160)
+    scale = gm * inv_std(var);
+    if (owner) {
+      a.mean[c] = mean; a.var[c] = var;
+      if (a.run_mean) a.run_mean[c] = rm + a.avg_rate * (mean - rm);
+      if (a.run_var) a.run_var[c] = rv + a.avg_rate * (var - rv);
+    }
+  } else {
+    const double rs2 = (double)rstd * t1;                 // sum(dz * xhat)
+    const double A = (double)gm * (double)rstd;
+    cB = (float)(-A * (double)rstd * rs2 * g.inv_count);
+    cC = (float)(-A * t0 * g.inv_count);
+    if (owner) {
+      if (a.dbeta) a.dbeta[c] = (float)t0;
+      if (a.dgamma) a.dgamma[c] = (float)rs2;
+    }
+  }
+
+  // ---- apply
+  uint32_t off = off0, col = col0;
+#pragma unroll
+  for (int k = 0; k < E; ++k) {
+    if (k < cnt) {
+      Pack<VEC> o;
+      if (DIR == 1 && a.accumulate) o = Pack<VEC>::load(a.out + off);
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) {
+        if (DIR == 0) {
+          float yb = fmaf(vx[k].v[i] - mean, scale, bt);
+          if (EXTRA) yb += ve[k].v[i];
+          o.v[i] = yb * (yb > 0.0f ? 1.0f : slope);
+        } else {
+          const float dx = fmaf(scale, ve[k].v[i], fmaf(cB, vx[k].v[i], cC));
+          o.v[i] = a.accumulate ? o.v[i] + dx : dx;
+        }
+      }
+      o.put(a.out + off);
+      if (DIR == 1 && EXTRA && a.dres) ve[k].put(a.dres + off);
+    }
+    off += g.step_off; col += g.step_col;
+    if (col >= g.d0v) { col -= g.d0v; off += g.wrap; }
+  }
+}
+
+// ---- host side -------------------------------------------------------------------------------
+
+typedef void (*ChanKernel)(const FusedArgs, const ChanGeom);
+
+template <int DIR, bool EXTRA>
+static ChanKernel chan_kernel_of(uint32_t vec, uint32_t f)
+{
+  if (vec == 4) {
+    if (f == 4) return bn_chan_kernel<DIR, 4, 4, EXTRA>;
+    if (f == 8) return bn_chan_kernel<DIR, 4, 8, EXTRA>;
+    if (f == 16) return bn_chan_kernel<DIR, 4, 16, EXTRA>;
+    if constexpr (DIR == 0 && !EXTRA) return bn_chan_kernel<DIR, 4, 32, EXTRA>;
+  } else {
+    if (f == 4) return bn_chan_kernel<DIR, 1, 4, EXTRA>;
+    if (f == 8) return bn_chan_kernel<DIR, 1, 8, EXTRA>;
+    if (f == 16) return bn_chan_kernel<DIR, 1, 16, EXTRA>;
+    if constexpr (DIR == 0 && !EXTRA) return bn_chan_kernel<DIR, 1, 32, EXTRA>;
+  }
+  return nullptr;
+}
+
+static bool chan_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, bool aligned, ChanGeom &g)
+{
+  g.vec = aligned && dim0 % 4 == 0 ? 4u : 1u;
+  const uint64_t total = (uint64_t)(dim0 / g.vec) * N;
+  const uint32_t fmax = dir == 0 && !extra ? 32u : 16u;
+  if (total > (uint64_t)kChanThreads * kChanCluster * (fmax / g.vec)) return false;
+  g.d0v = dim0 / g.vec; g.total = (uint32_t)total;
+  // floats per thread: as few as leave the whole problem on the device at once (about 1024 threads per SM)
+  uint32_t f = 4;
+  while (f < fmax && ((uint64_t)C * total * g.vec > (uint64_t)f * sm_count() * 1024 ||
+                      total > (uint64_t)kChanThreads * kChanCluster * (f / g.vec))) f *= 2;
+  const uint32_t e = f / g.vec;
+  const uint32_t need = (uint32_t)((total + e - 1) / e);             // threads of the team
+  g.floats = f; g.cluster = 1;
+  if (need <= 32) {
+    g.threads = 32;
+  } else {
+    while (need > g.cluster * kChanThreads) g.cluster *= 2;
+    g.threads = (ceil_div_u32(need, g.cluster) + 31) / 32 * 32;
+  }
+  g.team = g.threads * g.cluster;
+  const uint32_t drow = g.team / g.d0v;
+  g.step_col = g.team - drow * g.d0v;
+  g.step_off = drow * (C * dim0) + g.step_col * g.vec;
+  g.wrap = C * dim0 - dim0;
+  g.inv_count = 1.0 / ((double)dim0 * (double)N);
+  return true;
+}
+
+// Where this kernel is taken: wherever a team can hold the channel, except on large layers of short unaligned rows whose
+// runs of several channels are aligned.  There the scalar walk (some 22 instructions per element) costs more than the
+// shared-memory cluster kernel's chain of phases ([1024,2048,7,7] forward 310 us here, 200 us there; [64,512,7,7] the
+// other way round).  Forward + backward at the kernels' places, before and now: [2,512,7,7] 11.5 -> 4.5 us,
+// [32,64,28,28] 20.7 -> 9.8, [1,53,39,25] 17.9 -> 5.2, [1,260,128,128] 34.0 -> 16.7, [1,1240,45,30] 60.5 -> 13.8,
+// [40,2048,146,5] 630 -> 413, residual [256,1024,14,14] 459 -> 377.
+bool chan_preferred(const FusedArgs &a, int dir, bool aligned)
+{
+  ChanGeom g;
+  const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
+  if (a.mode != MODE_FUSED || a.world > 1) return false;
+  if (!chan_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, extra, aligned, g)) return false;
+  const uint64_t elements = (uint64_t)a.plan.dim0 * a.plan.C * a.plan.N;
+  return g.vec == 4 || elements < (8u << 20) || !segres_applies(a, dir, aligned);
+}
+
+int launch_chan(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)
+{
+  ChanGeom g;
+  const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
+  if (!chan_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, extra, aligned, g)) return ANODE_E_LAUNCH;
+  ChanKernel k = dir == 0 ? (extra ? chan_kernel_of<0, true>(g.vec, g.floats) : chan_kernel_of<0, false>(g.vec, g.floats))
+                          : (extra ? chan_kernel_of<1, true>(g.vec, g.floats) : chan_kernel_of<1, false>(g.vec, g.floats));
+  if (!k) return ANODE_E_LAUNCH;
+  const bool solo = g.threads == 32;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(solo ? ceil_div_u32(a.plan.C, kChanWarpTeams) : a.plan.C * g.cluster);
+  cfg.blockDim = dim3(solo ? 32 * kChanWarpTeams : g.threads);
+  cfg.stream = stream;
+  // The launch may overlap the tail of the kernel before it on the stream; every block waits for that kernel's
+  // results (griddepcontrol.wait) before it touches memory.
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = g.cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = g.cluster > 1 ? 2 : 1;
+  if (cudaLaunchKernelEx(&cfg, k, a, g) != cudaSuccess) { (void)cudaGetLastError(); return ANODE_E_LAUNCH; }
+  return ANODE_OK;
+}
+
+}  // namespace anode_b200

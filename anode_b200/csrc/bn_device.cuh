@@ -76,6 +76,7 @@ template <> struct Pack<4> {
                  : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]) : "l"(p), "l"(pol));
     return r;
   }
+  __device__ __forceinline__ void put(float *p) const { *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]); }
   // streaming store: the written tensor is not read again by this kernel
   __device__ __forceinline__ void store_stream(float *p) const
   {
@@ -96,6 +97,7 @@ template <> struct Pack<1> {
     asm volatile("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(r.v[0]) : "l"(p), "l"(pol));
     return r;
   }
+  __device__ __forceinline__ void put(float *p) const { *p = v[0]; }
   __device__ __forceinline__ void store_stream(float *p) const { __stcs(p, v[0]); }
   __device__ __forceinline__ void store(float *p, uint64_t pol) const
   {

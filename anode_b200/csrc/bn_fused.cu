@@ -307,7 +307,9 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
     case ANODE_KERNEL_CLUSTER: if (segres_applies(a, dir, aligned)) return ANODE_KERNEL_CLUSTER; break;
     case ANODE_KERNEL_RESIDENT: if (resident_applies(a, dir, aligned)) return ANODE_KERNEL_RESIDENT; break;
     case ANODE_KERNEL_PLAIN: if (plain_ok) return ANODE_KERNEL_PLAIN; break;
-    default: break;
+    default:
+      if (chan_preferred(a, dir, aligned)) return kKernelChan;
+      break;
   }
   if (extra) {
     // short rows: the cluster kernel; otherwise the plain kernel on one GPU (measured faster there) and
@@ -329,6 +331,7 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
 int launch_best(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)
 {
   int kind = pick_kernel_kind(a, dir, aligned);
+  if (kind == kKernelChan) return launch_chan(a, dir, aligned, stream);
   if (kind == ANODE_KERNEL_CLUSTER) {
     if (launch_segres(a, dir, stream) == ANODE_OK) return ANODE_OK;
     const bool extra = a.res || a.ymask || a.dres;
@@ -609,6 +612,15 @@ extern "C" int anode_gpu_online_average_f32(uint32_t len, float rate, const floa
   return ANODE_OK;
 }
 
+// The family callers see (ANODE_KERNEL_*): the register-resident kernel counts as a cluster kernel on the shapes of
+// that family and as the any-shape, any-alignment kernel elsewhere.
+static int public_kind(const FusedArgs &a, int dir, bool aligned)
+{
+  const int k = pick_kernel_kind(a, dir, aligned);
+  if (k != kKernelChan) return k;
+  return segres_applies(a, dir, aligned) ? ANODE_KERNEL_CLUSTER : ANODE_KERNEL_PLAIN;
+}
+
 // Which kernel serves direction `dir` of a plain [dim0, dim1, dim2] call with 16-byte aligned tensors on
 // one GPU: an ANODE_KERNEL_* value.
 extern "C" int anode_gpu_batch_norm_fused_kernel_kind(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir)
@@ -618,7 +630,7 @@ extern "C" int anode_gpu_batch_norm_fused_kernel_kind(uint32_t dim0, uint32_t di
   a.plan = plan_for(dim0, dim1, dim2, true);
   a.mode = MODE_FUSED;
   a.ws_capacity = workspace_part_bytes(dim0, dim1, dim2);
-  return pick_kernel_kind(a, dir, true);
+  return public_kind(a, dir, true);
 }
 
 // The same for the residual-epilogue calls (anode_gpu_batch_norm_add_act_fused_*).
@@ -631,7 +643,7 @@ extern "C" int anode_gpu_batch_norm_add_act_fused_kernel_kind(uint32_t dim0, uin
   a.mode = MODE_FUSED;
   a.ws_capacity = workspace_part_bytes(dim0, dim1, dim2);
   if (dir == 0) a.res = &dummy; else a.ymask = &dummy;       // only their presence matters here
-  return pick_kernel_kind(a, dir, true);
+  return public_kind(a, dir, true);
 }
 
 extern "C" int anode_gpu_batch_norm_fused_set_kernel(int kernel)

@@ -49,7 +49,8 @@ static void static_need(const FusedArgs &a, bool aligned, uint64_t &need, uint64
 {
   const uint32_t dim0 = a.plan.dim0, C = a.plan.C, N = a.plan.N;
   switch (pick_kernel_kind(a, 0, aligned)) {
-    case ANODE_KERNEL_CLUSTER:        // keeps everything on chip: only the status word lives in the array
+    case kKernelChan:
+    case ANODE_KERNEL_CLUSTER:        // keep everything on chip: only the status word lives in the array
       need = clear = 256;
       break;
     case ANODE_KERNEL_PLAIN: {
