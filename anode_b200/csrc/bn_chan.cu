@@ -268,15 +268,19 @@ static bool chan_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra
 // shared-memory cluster kernel's chain of phases ([1024,2048,7,7] forward 310 us here, 200 us there; [64,512,7,7] the
 // other way round).  Forward + backward at the kernels' places, before and now: [2,512,7,7] 11.5 -> 4.5 us,
 // [32,64,28,28] 20.7 -> 9.8, [1,53,39,25] 17.9 -> 5.2, [1,260,128,128] 34.0 -> 16.7, [1,1240,45,30] 60.5 -> 13.8,
-// [40,2048,146,5] 630 -> 413, residual [256,1024,14,14] 459 -> 377.
-bool chan_preferred(const FusedArgs &a, int dir, bool aligned)
+// [40,2048,146,5] 630 -> 413, residual [256,1024,14,14] 459 -> 377.  Large layers of ragged rows go to the tiled kernel
+// (`tiled_ok`) from rows of kChanLongRow floats on: [39,255,45,45] forward 62 us here, 44 us there, [349,255,15,15] 64 and
+// 68 us, [45,33,45,45] 12.9 and 15.5 us.
+constexpr uint32_t kChanLongRow = 300;
+bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
 {
   ChanGeom g;
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
   if (a.mode != MODE_FUSED || a.world > 1) return false;
   if (!chan_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, extra, aligned, g)) return false;
   const uint64_t elements = (uint64_t)a.plan.dim0 * a.plan.C * a.plan.N;
-  return g.vec == 4 || elements < (8u << 20) || !segres_applies(a, dir, aligned);
+  if (g.vec == 4 || elements < (8u << 20)) return true;
+  return !segres_applies(a, dir, aligned) && !(tiled_ok && a.plan.dim0 >= kChanLongRow);
 }
 
 int launch_chan(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)

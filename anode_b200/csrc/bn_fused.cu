@@ -15,6 +15,15 @@
 
 namespace anode_b200 {
 
+// Ragged rows (a length that is no multiple of four floats): the shortest one the tiled kernel takes, forward and
+// backward.  A row costs the producer a bulk copy per tensor, so below some length the plain kernel's 4-byte accesses
+// are the faster form.  20 M elements, 33 channels, forward / backward in us, tiled against plain: 9 x 9 144 / 270
+// against 116 / 160, 11 x 11 105 / 195 (116 / 161), 13 x 13 82 / 150 (116 / 161), 25 x 25 45 / 79 (117 / 160),
+// 63 x 63 43 / 62 (113 / 155).
+constexpr uint32_t kRaggedMinRow[2] = {112, 160};
+// Workspace header: (exit counter, parity) of the tiled kernel's plans (words 3 and 4 are the slice-resident kernel's)
+constexpr uint32_t kRingHdr = 4, kRingHdrRagged = 32, kRingHdrExtra = 40;
+
 // ---- planner constants, from sweeps on B200 -------------------------------------------------------
 #ifndef ANODE_SLACK_STEPS
 #define ANODE_SLACK_STEPS 2
@@ -42,8 +51,6 @@ const Tunables &tunables()
       ANODE_RING_FLOATS_FWD,    // ring_floats_fwd
       ANODE_RING_FLOATS_BWD,    // ring_floats_bwd
       1,        // ring_blocks_per_sm
-      8,        // ring_warps_fwd
-      16,       // ring_warps_bwd
   };
   return t;
 }
@@ -78,10 +85,10 @@ uint32_t sm_count()
 struct ShapeInfo {
   uint32_t dim0, C, N, sms;      // key; sms == 0: empty
   Plan plan[2];                  // tile plan: [pointers 16-byte aligned]
-  bool ring_ok[2];               // warp-specialised kernel, per direction, for aligned pointers
-  Plan ring_plan[2];
-  RingGeom ring_geom[2];
-  uint64_t tiled_bytes, part_bytes;
+  bool ring_ok[2][2];            // warp-specialised kernel for aligned pointers: [direction][residual epilogue]
+  Plan ring_plan[2][2];
+  RingGeom ring_geom[2][2];
+  uint64_t tiled_bytes, static_bytes, part_bytes;      // see fill_shape_info
 };
 constexpr uint32_t kShapeCache = 64;      // entries per thread, direct mapped
 
@@ -105,25 +112,21 @@ static const ShapeInfo &shape_info(uint32_t dim0, uint32_t C, uint32_t N)
 
 Plan plan_for(uint32_t dim0, uint32_t C, uint32_t N, bool aligned16) { return shape_info(dim0, C, N).plan[aligned16 ? 1 : 0]; }
 
-// Shared-memory layout of the warp-specialised kernel for plan `p` (see bn_ring.cuh).
-// consumer warps of direction `dir`: 8 or 16 (the two instantiations of bn_ring.cuh)
-static uint32_t ring_warps(int dir)
-{
-  const Tunables &t = tunables();
-  return (dir == 0 ? t.ring_warps_fwd : t.ring_warps_bwd) >= 16 ? 16u : 8u;
-}
+// consumer warps of direction `dir` (the two instantiations of bn_ring.cuh)
+static uint32_t ring_warps(int dir) { return dir == 0 ? 8u : 16u; }
 
-static RingGeom ring_geom(const Plan &p, int dir, uint32_t slots, uint32_t slot_floats)
+// Shared-memory layout of the warp-specialised kernel for plan `p` (see bn_ring.cuh).
+static RingGeom ring_geom(const Plan &p, int dir, bool extra, uint32_t slots, uint32_t slot_floats)
 {
   RingGeom g{};
-  g.slots = slots; g.slot_floats = slot_floats;
+  g.slots = slots; g.slot_floats = slot_floats; g.hdr = kRingHdr;
   uint32_t off = kRingCtlBytes;
-  const uint32_t cwarps = ring_warps(dir);
+  const uint32_t cwarps = ring_warps(dir), planes = (dir == 1 ? 2u : 1u) + (extra ? 1u : 0u);
   g.res_stride = p.cb > cwarps ? p.cb : cwarps;   // regime R: one partial per consumer warp
   g.off_res = off;  off += (uint32_t)align_up_u64((uint64_t)kResQ * g.res_stride * 16, 128);
   g.off_coef = off; off += (uint32_t)align_up_u64((uint64_t)kCoefQ * p.cb * 32, 128);
   g.off_slots = off;
-  g.slot_stride = (uint32_t)align_up_u64((uint64_t)slot_floats * 4 * (dir == 1 ? 2 : 1) + (dir == 1 ? (uint64_t)p.cb * 16 : 0), 128);
+  g.slot_stride = (uint32_t)align_up_u64((uint64_t)slot_floats * 4 * planes + (dir == 1 ? (uint64_t)p.cb * 16 : 0), 128);
   g.smem_bytes = off + slots * g.slot_stride;
   return g;
 }
@@ -131,23 +134,33 @@ static RingGeom ring_geom(const Plan &p, int dir, uint32_t slots, uint32_t slot_
 // Plan for the warp-specialised kernel, or false when it does not apply (scalar paths, tiles that
 // do not fit a slot, too little shared memory): the caller then uses the plain kernel.
 // Plan and geometry for `slots` slots of `slot_floats` floats (per tensor); false when they do not fit.
-static bool ring_plan_with(uint32_t dim0, uint32_t C, uint32_t N, int dir, uint32_t slots, uint32_t slot_floats, Plan &p, RingGeom &g)
+static bool ring_plan_with(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, uint32_t slots, uint32_t slot_floats, Plan &p, RingGeom &g)
 {
   const Tunables &t = tunables();
   slot_floats = (slot_floats / 4) * 4;
   if (slot_floats < 1024) slot_floats = 1024;
   slots = slots < 2 ? 2 : (slots > kMaxSlots ? kMaxSlots : slots);
   uint32_t bps = t.ring_blocks_per_sm ? t.ring_blocks_per_sm : 1;
-  p = make_plan(dim0, C, N, true, sm_count() * bps, slot_floats, t.slack_steps);
+  // rows that are no multiple of four floats take up to 6 floats more in a slot (ragged_pitch)
+  const bool ragged = dim0 % 4 != 0;
+  if (ragged && dim0 < kRaggedMinRow[dir]) return false;
+  uint32_t target = slot_floats;
+  if (ragged) target = 4 * ragged_pitch(dim0) <= slot_floats ? slot_floats / (4 * ragged_pitch(dim0)) * dim0 : slot_floats - 8;
+  p = make_plan(dim0, C, N, true, sm_count() * bps, target, t.slack_steps);
   // short rows (regime S) belong to the cluster kernel or the plain kernel
-  if (p.vec != 4 || p.regime != 0) return false;
-  // a tile must fit one slot: rows * len <= slot_floats
-  const uint64_t tile_max = (uint64_t)p.rows_per_tile * p.piece_len;
+  if (p.regime != 0) return false;
+  if (ragged) {
+    const uint32_t per_row = ragged_pitch(p.piece_len < dim0 ? p.piece_len : dim0);
+    p.vec = 4;
+    p.div_mul = (uint32_t)((1ull << 32) / per_row) + 1;
+  }
+  // a tile must fit one slot
+  const uint64_t tile_max = (uint64_t)p.rows_per_tile * (ragged ? 4 * ragged_pitch(p.piece_len < dim0 ? p.piece_len : dim0) : p.piece_len);
   if (tile_max > slot_floats) return false;
   slot_floats = (uint32_t)((tile_max + 31) / 32 * 32);     // slots no larger than the largest tile
-  g = ring_geom(p, dir, slots, slot_floats);
+  g = ring_geom(p, dir, extra, slots, slot_floats);
   const uint32_t budget = 227u * 1024u;
-  while (g.smem_bytes > budget && slots > 2) { --slots; g = ring_geom(p, dir, slots, slot_floats); }
+  while (g.smem_bytes > budget && slots > 2) { --slots; g = ring_geom(p, dir, extra, slots, slot_floats); }
   return g.smem_bytes <= budget;
 }
 
@@ -162,14 +175,30 @@ static uint64_t ring_window_bytes(const Plan &p, int dir)
 constexpr uint32_t kRingLargeSlotsBwd = 3, kRingLargeFloatsBwd = 9408;
 constexpr uint64_t kRingLargeWindowMax = 48ull << 20;     // also the part of a larger window that is marked "keep" (launch_ring)
 
-static bool make_ring_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, Plan &p, RingGeom &g)
+// The residual epilogue's slots hold a third tensor (a second one in the forward pass, used by the apply visits only).
+#ifndef ANODE_RING_SLOTS_FWD_EXTRA
+#define ANODE_RING_SLOTS_FWD_EXTRA 4
+#endif
+#ifndef ANODE_RING_FLOATS_FWD_EXTRA
+#define ANODE_RING_FLOATS_FWD_EXTRA 6656
+#endif
+#ifndef ANODE_RING_SLOTS_BWD_EXTRA
+#define ANODE_RING_SLOTS_BWD_EXTRA 3
+#endif
+#ifndef ANODE_RING_FLOATS_BWD_EXTRA
+#define ANODE_RING_FLOATS_BWD_EXTRA 6272
+#endif
+static bool make_ring_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, Plan &p, RingGeom &g)
 {
   const Tunables &t = tunables();
-  if (!ring_plan_with(dim0, C, N, dir, dir == 0 ? t.ring_slots : t.ring_slots_bwd,
+  if (extra)
+    return dir == 0 ? ring_plan_with(dim0, C, N, dir, true, ANODE_RING_SLOTS_FWD_EXTRA, ANODE_RING_FLOATS_FWD_EXTRA, p, g)
+                    : ring_plan_with(dim0, C, N, dir, true, ANODE_RING_SLOTS_BWD_EXTRA, ANODE_RING_FLOATS_BWD_EXTRA, p, g);
+  if (!ring_plan_with(dim0, C, N, dir, false, dir == 0 ? t.ring_slots : t.ring_slots_bwd,
                       dir == 0 ? t.ring_floats_fwd : t.ring_floats_bwd, p, g)) return false;
   if (dir == 1) {
     Plan pl; RingGeom gl;
-    if (ring_plan_with(dim0, C, N, dir, kRingLargeSlotsBwd, kRingLargeFloatsBwd, pl, gl) && gl.slots == kRingLargeSlotsBwd &&
+    if (ring_plan_with(dim0, C, N, dir, false, kRingLargeSlotsBwd, kRingLargeFloatsBwd, pl, gl) && gl.slots == kRingLargeSlotsBwd &&
         (uint64_t)pl.rows_per_tile * pl.piece_len > (uint64_t)p.rows_per_tile * p.piece_len &&
         ring_window_bytes(pl, dir) <= kRingLargeWindowMax) {
       p = pl; g = gl;
@@ -178,34 +207,52 @@ static bool make_ring_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, Plan 
   return true;
 }
 
-bool ring_plan_for(uint32_t dim0, uint32_t C, uint32_t N, bool aligned, int dir, Plan &p, RingGeom &g)
+bool ring_plan_for(uint32_t dim0, uint32_t C, uint32_t N, bool aligned, int dir, bool extra, Plan &p, RingGeom &g)
 {
   if (!aligned) return false;
   const ShapeInfo &s = shape_info(dim0, C, N);
-  if (!s.ring_ok[dir]) return false;
-  p = s.ring_plan[dir]; g = s.ring_geom[dir];
+  if (!s.ring_ok[dir][extra]) return false;
+  p = s.ring_plan[dir][extra]; g = s.ring_geom[dir][extra];
   return true;
+}
+
+// Plan of the warp-specialised kernel for a prepared call, or false when it does not serve it.  Ragged rows and the
+// residual epilogue are one-launch, one-GPU forms.
+static bool ring_plan_of(const FusedArgs &a, int dir, bool aligned, Plan &p, RingGeom &g)
+{
+  const bool extra = a.res || a.ymask || a.dres;
+  if ((extra || a.plan.dim0 % 4 != 0) && (a.mode != MODE_FUSED || a.world > 1)) return false;
+  return ring_plan_for(a.plan.dim0, a.plan.C, a.plan.N, aligned, dir, extra, p, g) && p.ws_bytes <= a.ws_capacity;
+}
+
+// Bytes of a part up to the end of that plan's words; 0 when the kernel does not serve the call.
+uint64_t ring_ws_bytes(const FusedArgs &a, int dir, bool aligned)
+{
+  Plan p; RingGeom g;
+  return ring_plan_of(a, dir, aligned, p, g) ? p.ws_bytes : 0;
 }
 
 typedef void (*RingKernel)(const FusedArgs, const RingGeom);
 
-static RingKernel pick_ring_kernel(const Plan &p, int dir, uint32_t &threads)
+static RingKernel pick_ring_kernel(const Plan &p, int dir, bool extra, uint32_t &threads)
 {
-  // only regime R reaches this point (ring_plan_for)
-  (void)p;
-  if (ring_warps(dir) == 16) {
-    threads = ring16::kRingThreads;
-    return dir == 0 ? ring16::bn_ring_kernel<0> : ring16::bn_ring_kernel<1>;
+  const bool ragged = p.dim0 % 4 != 0;
+  threads = dir == 0 ? ring8::kRingThreads : ring16::kRingThreads;
+  if (dir == 0) {
+    if (extra) return ragged ? ring8::bn_ring_kernel<0, true, true> : ring8::bn_ring_kernel<0, true, false>;
+    return ragged ? ring8::bn_ring_kernel<0, false, true> : ring8::bn_ring_kernel<0, false, false>;
   }
-  threads = ring8::kRingThreads;
-  return dir == 0 ? ring8::bn_ring_kernel<0> : ring8::bn_ring_kernel<1>;
+  if (extra) return ragged ? ring16::bn_ring_kernel<1, true, true> : ring16::bn_ring_kernel<1, true, false>;
+  return ragged ? ring16::bn_ring_kernel<1, false, true> : ring16::bn_ring_kernel<1, false, false>;
 }
 
 int launch_ring(FusedArgs &a, const RingGeom &g_in, int dir, cudaStream_t stream)
 {
   RingGeom g = g_in;
   uint32_t threads = 0;
-  RingKernel k = pick_ring_kernel(a.plan, dir, threads);
+  RingKernel k = pick_ring_kernel(a.plan, dir, a.res || a.ymask || a.dres, threads);
+  // the reduce visits may store dres before the apply visits read x only where it is not x itself
+  a.dres_early = a.dres && a.dres != a.x ? 1u : 0u;
   static std::mutex mu;
   static std::map<std::pair<const void *, uint32_t>, int> occ;     // (kernel, smem) -> blocks per SM
   int per_sm = 0;
@@ -233,7 +280,8 @@ int launch_ring(FusedArgs &a, const RingGeom &g_in, int dir, cudaStream_t stream
   a.use_rec = a.mode == MODE_FUSED ? 1u : 0u;
   // A window larger than what L2 keeps would cycle through it whole (config 3, backward: 67 MB); marking only
   // the part that fits lets that part stay (backward 4.42 -> 4.27 ms).  Smaller windows keep everything.
-  const uint64_t window = ring_window_bytes(a.plan, dir);
+  uint64_t window = ring_window_bytes(a.plan, dir);
+  if (a.ymask && !a.dres_early) window += window / 2;      // x, dy and the saved output come twice
   g.keep_frac = window > kRingLargeWindowMax ? (float)((double)kRingLargeWindowMax / (double)window) : 1.0f;
   void *params[] = {(void *)&a, (void *)&g};
   cudaError_t e;
@@ -258,12 +306,32 @@ static void fill_shape_info(ShapeInfo &s)
     s.plan[al] = make_plan(s.dim0, s.C, s.N, al != 0, sm_count() * t.blocks_per_sm, t.tile_floats, 1);
     if (s.plan[al].ws_bytes > need) need = s.plan[al].ws_bytes;
   }
-  for (int dir = 0; dir < 2; ++dir) {
-    s.ring_ok[dir] = make_ring_plan(s.dim0, s.C, s.N, dir, s.ring_plan[dir], s.ring_geom[dir]);
-    if (s.ring_ok[dir] && s.ring_plan[dir].ws_bytes > need) need = s.ring_plan[dir].ws_bytes;
-  }
+  for (int dir = 0; dir < 2; ++dir)
+    for (int ex = 0; ex < 2; ++ex)
+      s.ring_ok[dir][ex] = make_ring_plan(s.dim0, s.C, s.N, dir, ex != 0, s.ring_plan[dir][ex], s.ring_geom[dir][ex]);
+  const bool ragged = s.dim0 % 4 != 0;
+  if (!ragged)
+    for (int dir = 0; dir < 2; ++dir)
+      if (s.ring_ok[dir][0] && s.ring_plan[dir][0].ws_bytes > need) need = s.ring_plan[dir][0].ws_bytes;
   s.tiled_bytes = align_up_u64(need, 256);
-  s.part_bytes = align_up_u64(s.tiled_bytes + resident_ws_bytes(s.dim0, s.C, s.N), 256);
+  s.static_bytes = align_up_u64(s.tiled_bytes + resident_ws_bytes(s.dim0, s.C, s.N), 256);
+  // The tiled kernel keeps tagged words from launch to launch, laid out by its plan.  Ragged rows and the residual
+  // epilogue have plans of their own beside the plain kernel's and the ordinary call's on the same workspace, so their
+  // words (and their two header words) lie apart, behind everything else.
+  s.part_bytes = s.static_bytes;
+  for (int dir = 0; dir < 2; ++dir)
+    for (int ex = 0; ex < 2; ++ex) {
+      if (!s.ring_ok[dir][ex] || (!ex && !ragged)) continue;
+      Plan &p = s.ring_plan[dir][ex];
+      // the fused form of this kernel uses the tagged words only
+      uint64_t off = s.static_bytes;
+      if (ex && ragged && s.ring_ok[dir][0]) off = align_up_u64(s.ring_plan[dir][0].ws_bytes, 256);
+      const uint64_t end = align_up_u64(off + 16ull * p.total_tiles * p.cb, 256);
+      if (end > 0xffffffffull) { s.ring_ok[dir][ex] = false; continue; }
+      p.off_tag = (uint32_t)off; p.off_part = (uint32_t)end; p.ws_bytes = end;
+      s.ring_geom[dir][ex].hdr = ex ? kRingHdrExtra : kRingHdrRagged;
+      if (end > s.part_bytes) s.part_bytes = end;
+    }
 }
 
 // Bytes of a part taken by the tile-plan kernels (plain, warp-specialised, cluster); the records of the
@@ -272,6 +340,9 @@ static uint64_t tiled_part_bytes(uint32_t dim0, uint32_t C, uint32_t N) { return
 
 uint64_t workspace_part_bytes(uint32_t dim0, uint32_t C, uint32_t N) { return shape_info(dim0, C, N).part_bytes; }
 
+// Bytes of a part behind which only the ragged and the residual plans of the tiled kernel keep their words.
+uint64_t workspace_static_bytes(uint32_t dim0, uint32_t C, uint32_t N) { return shape_info(dim0, C, N).static_bytes; }
+
 // Bytes at the start of a workspace that hold progress counters, flags and records, i.e. what has
 // to be zero when a launch begins (the per-tile partials behind them are written before they are read).
 uint64_t control_region_bytes(uint32_t dim0, uint32_t C, uint32_t N, bool aligned)
@@ -279,19 +350,12 @@ uint64_t control_region_bytes(uint32_t dim0, uint32_t C, uint32_t N, bool aligne
   uint64_t n = plan_for(dim0, C, N, aligned).off_part;
   for (int dir = 0; dir < 2; ++dir) {
     Plan rp; RingGeom g;
-    if (ring_plan_for(dim0, C, N, aligned, dir, rp, g) && rp.off_part > n) n = rp.off_part;
+    if (ring_plan_for(dim0, C, N, aligned, dir, false, rp, g) && rp.off_part > n) n = rp.off_part;
   }
   // the slice-resident kernel's records validate themselves against the launch counter in the header,
   // which the clearing resets: they have to go too
-  if (aligned && resident_ws_bytes(dim0, C, N)) n = workspace_part_bytes(dim0, C, N);
+  if (aligned && resident_ws_bytes(dim0, C, N)) { const uint64_t r = workspace_static_bytes(dim0, C, N); if (r > n) n = r; }
   return n;
-}
-
-// True when the warp-specialised kernel will serve this call (the in-kernel exchange needs it).
-bool ring_applies(const FusedArgs &a, int dir, bool aligned)
-{
-  Plan rp; RingGeom g;
-  return ring_plan_for(a.plan.dim0, a.plan.C, a.plan.N, aligned, dir, rp, g) && rp.ws_bytes <= a.ws_capacity;
 }
 
 // Which kernel launch_best takes for a prepared call: ANODE_KERNEL_* (never AUTO), or -1 when none can
@@ -301,19 +365,21 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
   const bool extra = a.res || a.ymask || a.dres;        // residual epilogue
   const bool plain_ok = !(a.mode == MODE_FUSED && a.world > 1);
   Plan rp; RingGeom g;
-  const bool tiled_ok = !extra && ring_plan_for(a.plan.dim0, a.plan.C, a.plan.N, aligned, dir, rp, g) && rp.ws_bytes <= a.ws_capacity;
+  const bool tiled_ok = ring_plan_of(a, dir, aligned, rp, g);
   switch (kernel_choice()) {
     case ANODE_KERNEL_TILED: if (tiled_ok) return ANODE_KERNEL_TILED; break;
     case ANODE_KERNEL_CLUSTER: if (segres_applies(a, dir, aligned)) return ANODE_KERNEL_CLUSTER; break;
     case ANODE_KERNEL_RESIDENT: if (resident_applies(a, dir, aligned)) return ANODE_KERNEL_RESIDENT; break;
     case ANODE_KERNEL_PLAIN: if (plain_ok) return ANODE_KERNEL_PLAIN; break;
     default:
-      if (chan_preferred(a, dir, aligned)) return kKernelChan;
+      if (chan_preferred(a, dir, aligned, tiled_ok)) return kKernelChan;
       break;
   }
   if (extra) {
-    // short rows: the cluster kernel; otherwise the plain kernel on one GPU (measured faster there) and
-    // the slice-resident kernel, which has the exchange inside, in synchronized calls
+    // long rows: the tiled kernel on one GPU (forward / backward: [256,512,28,28] 263 / 452 us, cluster kernel 383 / too
+    // large for it, plain kernel 315 / 618; [256,64,56,56] 136 / 188 us, plain kernel 152 / 303); short ones the cluster
+    // kernel, and in synchronized calls what has the exchange inside
+    if (tiled_ok) return ANODE_KERNEL_TILED;
     if (segres_applies(a, dir, aligned)) return ANODE_KERNEL_CLUSTER;
     if (plain_ok) return ANODE_KERNEL_PLAIN;
     return resident_applies(a, dir, aligned) ? ANODE_KERNEL_RESIDENT : -1;
@@ -334,15 +400,14 @@ int launch_best(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)
   if (kind == kKernelChan) return launch_chan(a, dir, aligned, stream);
   if (kind == ANODE_KERNEL_CLUSTER) {
     if (launch_segres(a, dir, stream) == ANODE_OK) return ANODE_OK;
-    const bool extra = a.res || a.ymask || a.dres;
     Plan rp; RingGeom g;
-    if (!extra && ring_plan_for(a.plan.dim0, a.plan.C, a.plan.N, aligned, dir, rp, g) && rp.ws_bytes <= a.ws_capacity) kind = ANODE_KERNEL_TILED;
+    if (ring_plan_of(a, dir, aligned, rp, g)) kind = ANODE_KERNEL_TILED;
     else if (resident_applies(a, dir, aligned)) kind = ANODE_KERNEL_RESIDENT;
     else kind = (a.mode == MODE_FUSED && a.world > 1) ? -1 : ANODE_KERNEL_PLAIN;
   }
   if (kind == ANODE_KERNEL_TILED) {
     Plan rp; RingGeom g;
-    if (!ring_plan_for(a.plan.dim0, a.plan.C, a.plan.N, aligned, dir, rp, g)) return ANODE_E_LAUNCH;
+    if (!ring_plan_of(a, dir, aligned, rp, g)) return ANODE_E_LAUNCH;
     a.plan = rp;
     return launch_ring(a, g, dir, stream);
   }
@@ -663,7 +728,7 @@ extern "C" int anode_gpu_batch_norm_tiled_geometry(uint32_t dim0, uint32_t dim1,
   if (!out || (dir != 0 && dir != 1) || check_dims(dim0, dim1, dim2)) return ANODE_E_DIMS;
   Plan p; RingGeom g;
   for (int i = 0; i < 12; ++i) out[i] = 0;
-  if (!ring_plan_for(dim0, dim1, dim2, true, dir, p, g)) return ANODE_OK;
+  if (!ring_plan_for(dim0, dim1, dim2, true, dir, false, p, g)) return ANODE_OK;
   const uint64_t window = ring_window_bytes(p, dir);
   out[0] = 1; out[1] = p.rows_per_tile; out[2] = p.piece_len; out[3] = p.tiles_per_unit; out[4] = g.slots;
   out[5] = g.slot_stride; out[6] = g.smem_bytes; out[7] = (uint32_t)(window >> 10);

@@ -32,10 +32,11 @@ struct FusedArgs {
   const float *dy;         // backward only
   const float *gamma, *beta;
   const float *mean_in, *var_in;   // backward only
-  // residual epilogue (plain kernel only): forward y = act(bn(x) + res); backward takes the mask
+  // residual epilogue: forward y = act(bn(x) + res); backward takes the mask
   // from the saved output ymask and also writes dres = dy*mask
   const float *res, *ymask;
   float *dres;
+  uint32_t dres_early;     // tiled kernel: dres is written by the reduce visits and read back by the apply visits
   float *out;              // y (forward) or dx (backward)
   float *mean, *var, *run_mean, *run_var;   // forward outputs
   float *dgamma, *dbeta;   // backward outputs
@@ -720,8 +721,11 @@ constexpr uint32_t kResQ = 4;          // partial mailbox depth
 constexpr uint32_t kCoefQ = 4;         // coefficient mailbox depth
 constexpr uint32_t kMaxSlots = 8;
 constexpr uint32_t kRingCtlBytes = 1024;   // room reserved for the kernel's barrier block (RingCtl)
+// 16-byte vectors a row of `len` floats can touch when it starts anywhere within one (tiled kernel, ragged rows)
+ANODE_HD uint32_t ragged_pitch(uint32_t len) { return (len + 6) / 4; }
 struct RingGeom {
   uint32_t slots, slot_floats, slot_stride, res_stride, off_res, off_coef, off_slots, smem_bytes;
+  uint32_t hdr;            // byte offset of this plan's exit counter and parity word in the workspace header
   float keep_frac;         // fused mode: fraction of the reduce visits' lines loaded with the L2 "keep" priority
 };
 

@@ -24,8 +24,6 @@ struct Tunables {
   uint32_t ring_floats_fwd; // floats per slot (forward: x)
   uint32_t ring_floats_bwd; // floats per tensor per slot (backward: x and dy)
   uint32_t ring_blocks_per_sm;
-  uint32_t ring_warps_fwd;  // consumer warps of the forward kernel (8 or 16)
-  uint32_t ring_warps_bwd;  // consumer warps of the backward kernel (8 or 16)
 };
 const Tunables &tunables();
 
@@ -46,16 +44,17 @@ int launch_pipeline(FusedArgs &a, int dir, cudaStream_t stream);
 int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned);
 int launch_best(FusedArgs &a, int dir, bool aligned, cudaStream_t stream);
 int kernel_choice();
-bool ring_applies(const FusedArgs &a, int dir, bool aligned);
 // the cluster kernel for short rows (bn_segres.cu)
 bool segres_applies(const FusedArgs &a, int dir, bool aligned);
 bool segres_preferred(const FusedArgs &a, int dir, bool aligned);      // take it even where the tiled kernel applies
 int launch_segres(FusedArgs &a, int dir, cudaStream_t stream);
 // the register-resident kernel (bn_chan.cu); one GPU, any alignment
 constexpr int kKernelChan = 5;            // its number inside the library (callers see the family, see public_kind)
-bool chan_preferred(const FusedArgs &a, int dir, bool aligned);
+bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok);
 int launch_chan(FusedArgs &a, int dir, bool aligned, cudaStream_t stream);
 uint64_t workspace_part_bytes(uint32_t dim0, uint32_t C, uint32_t N);
+uint64_t workspace_static_bytes(uint32_t dim0, uint32_t C, uint32_t N);
+uint64_t ring_ws_bytes(const FusedArgs &a, int dir, bool aligned);
 // the slice-resident kernel (bn_resident.cu)
 bool resident_applies(const FusedArgs &a, int dir, bool aligned);
 uint64_t resident_ws_bytes(uint32_t dim0, uint32_t C, uint32_t N);

@@ -32,9 +32,6 @@
 #if !defined(ANODE_RING_NS) || !defined(ANODE_RING_CONSUMERS)
 #error "define ANODE_RING_NS and ANODE_RING_CONSUMERS before including bn_ring.cuh"
 #endif
-#ifndef ANODE_RING_STORE
-#define ANODE_RING_STORE 1      // 0: store with an L2 evict-first hint, 1: st.global.cs, 2: plain store
-#endif
 #ifndef ANODE_RING_BACKOFF_NS
 #define ANODE_RING_BACKOFF_NS 100
 #endif
@@ -181,10 +178,11 @@ struct Sched {
 
 // dynamic shared memory accessors
 __device__ __forceinline__ float *slot_x(unsigned char *sm, const RingGeom &g, uint32_t slot) { return reinterpret_cast<float *>(sm + g.off_slots + (size_t)slot * g.slot_stride); }
-template <int DIR> __device__ __forceinline__ float *slot_dy(unsigned char *sm, const RingGeom &g, uint32_t slot) { return slot_x(sm, g, slot) + g.slot_floats; }
-template <int DIR> __device__ __forceinline__ float4 *slot_side(unsigned char *sm, const RingGeom &g, uint32_t slot)
+// a slot holds kPlanes tensors side by side: x, then dy (backward), then the residual (forward) / saved output (backward)
+template <int DIR, bool EXTRA> constexpr uint32_t kPlanes = (DIR == 1 ? 2u : 1u) + (EXTRA ? 1u : 0u);
+template <int DIR, bool EXTRA> __device__ __forceinline__ float4 *slot_side(unsigned char *sm, const RingGeom &g, uint32_t slot)
 {
-  return reinterpret_cast<float4 *>(slot_x(sm, g, slot) + (DIR == 1 ? 2 : 1) * g.slot_floats);
+  return reinterpret_cast<float4 *>(slot_x(sm, g, slot) + kPlanes<DIR, EXTRA> * g.slot_floats);
 }
 __device__ __forceinline__ float4 *res_box(unsigned char *sm, const RingGeom &g, uint32_t q) { return reinterpret_cast<float4 *>(sm + g.off_res) + (size_t)q * g.res_stride; }
 __device__ __forceinline__ float4 *coef_box(unsigned char *sm, const RingGeom &g, uint32_t cb, uint32_t q) { return reinterpret_cast<float4 *>(sm + g.off_coef) + (size_t)q * cb * 2; }
@@ -206,7 +204,36 @@ __device__ __forceinline__ Pack<4> lds128(uint32_t saddr)
 }
 constexpr uint32_t kVecStride = kConsumers * 16;     // bytes between consecutive vectors of one thread
 
-template <int DIR>
+// Backward pass of the residual epilogue: dres = dz leaves during the reduce visit and the apply visit reads it back
+// (from L2) in the place of dy and the saved output, unless there is no dres or it is x itself (FusedArgs::dres_early).
+// The read is a bulk copy, hence the fence between the two proxies before the slot is given back.
+__device__ __forceinline__ void fence_global_to_bulk() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
+
+// Places, in global memory, of the vectors tid, tid + kConsumers, ... of a tile whose rows lie back to back in the slot,
+// per_row vectors each: a step is an add and a compare, without a division or a 64-bit product per vector.
+struct RowWalk {
+  uint32_t row, col;              // float offset of the row's first float (below 2^32, check_dims); vector within the row
+  uint32_t step_row, step_col, rs, per_row;
+  __device__ __forceinline__ void init(const FusedArgs &a, const TileRange &tr, uint32_t per_row_)
+  {
+    const uint32_t tid = threadIdx.x;
+    per_row = per_row_; rs = a.plan.C * a.plan.dim0;
+    uint32_t r = 0, sr = 0;
+    // several rows: always whole ones, whose vectors plan.div_mul divides by; one row: never wraps
+    if (tr.rows > 1) { r = fast_div(tid, a.plan.div_mul); sr = fast_div(kConsumers, a.plan.div_mul); }
+    col = tid - r * per_row; row = (uint32_t)tr.base + r * rs;
+    step_col = kConsumers - sr * per_row; step_row = sr * rs;
+  }
+  __device__ __forceinline__ void advance()
+  {
+    row += step_row; col += step_col;
+    if (col >= per_row) { col -= per_row; row += rs; }
+  }
+  __device__ __forceinline__ uint32_t at() const { return (row & ~3u) + 4 * col; }            // float offset of the vector
+  __device__ __forceinline__ int first() const { return (int)(4 * col) - (int)(row & 3u); }   // its first float's place in the row
+};
+
+template <int DIR, bool EXTRA>
 __device__ __forceinline__ void warp_reduce_R(const FusedArgs &a, const RingGeom &g, unsigned char *sm, RingCtl *ctl,
                                               const TileRange &tr, uint32_t slot, float4 *res)
 {
@@ -260,22 +287,30 @@ __device__ __forceinline__ void warp_reduce_R(const FusedArgs &a, const RingGeom
     }
   } else {
     uint32_t ad = ax + g.slot_floats * 4;
-    const float4 cf = slot_side<1>(sm, g, slot)[0];
+    const float4 cf = slot_side<1, EXTRA>(sm, g, slot)[0];
     const float mean = cf.x, scale = cf.y, beta = cf.z;
     const float slope = a.neg_slope;      // activation: t * (t > 0 ? 1 : slope)
     float s1 = 0.f, s2 = 0.f;
+    RowWalk w;
+    float *dres = nullptr;
+    if constexpr (EXTRA) { if (a.dres_early) { dres = a.dres; w.init(a, tr, tr.len / 4); } }
     // (one vector per tensor at a time: with two in flight the sixteen warps of this pass were measured slower)
     for (uint32_t i = 0; i < cnt; ++i, ax += kVecStride, ad += kVecStride) {
       const Pack<4> x0 = lds128(ax), g0 = lds128(ad);
+      Pack<4> m0 = x0, z;
+      if constexpr (EXTRA) m0 = lds128(ad + g.slot_floats * 4);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float d0 = x0.v[e] - mean;
-        const float y0 = fmaf(d0, scale, beta);
+        const float y0 = EXTRA ? m0.v[e] : fmaf(d0, scale, beta);      // residual epilogue: the saved output carries the mask
         // dz = dy * (float)(y > 0)  (routines_gpu/flat_map.cu:191-192)
         const float z0 = g0.v[e] * (y0 > 0.0f ? 1.0f : slope);
         s1 += z0; s2 = fmaf(z0, d0, s2);
+        z.v[e] = z0;
       }
+      if constexpr (EXTRA) { if (dres) { z.put(dres + w.row + 4 * w.col); w.advance(); } }
     }
+    if constexpr (EXTRA) { if (dres) fence_global_to_bulk(); }
     __syncwarp();
     if (lane == 0) mbar_arrive(&ctl->empty[slot]);
     s1 = warp_sum(s1); s2 = warp_sum(s2);
@@ -283,16 +318,17 @@ __device__ __forceinline__ void warp_reduce_R(const FusedArgs &a, const RingGeom
   }
 }
 
-template <int DIR>
+template <int DIR, bool EXTRA>
 __device__ __forceinline__ void warp_apply_R(const FusedArgs &a, const RingGeom &g, unsigned char *sm, RingCtl *ctl,
                                              const TileRange &tr, uint32_t slot, const float4 *coef, uint32_t coef_q)
 {
   const uint32_t tid = threadIdx.x, lane = tid & 31;
   const float slope = a.neg_slope;      // activation: t * (t > 0 ? 1 : slope)
   const bool acc = a.accumulate != 0;
-  const uint64_t drop = policy_drop();
+  const bool early = EXTRA && DIR == 1 && a.dres_early;      // plane 1 holds dz (see fence_global_to_bulk)
   const uint64_t rs = (uint64_t)a.plan.C * a.plan.dim0;
   float *out = a.out + tr.base;
+  float *dres = EXTRA && DIR == 1 && !early ? a.dres : nullptr;
   const float4 c0 = coef[0], c1 = coef[1];
   const float mean = c0.x, scale = c0.y, beta = c0.z, cB = c1.x, cC = c1.y;
   const uint32_t per_row = tr.len / 4, nvec = per_row * tr.rows;
@@ -313,36 +349,187 @@ __device__ __forceinline__ void warp_apply_R(const FusedArgs &a, const RingGeom 
     if (col >= per_row) { col -= per_row; dst += wrap_ptr; }
   };
   // one vector: o = activation(bn(x)) or the input gradient
-  auto one = [&](const Pack<4> &vx, const Pack<4> &vd, float *p) {
-    Pack<4> o;
+  auto one = [&](const Pack<4> &vx, const Pack<4> &vd, const Pack<4> &ve, float *p) {
+    Pack<4> o, z;
     if constexpr (DIR == 0) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) { const float yb = fmaf(vx.v[e] - mean, scale, beta); o.v[e] = yb * (yb > 0.0f ? 1.0f : slope); }
+      for (int e = 0; e < 4; ++e) {
+        float yb = fmaf(vx.v[e] - mean, scale, beta);
+        if constexpr (EXTRA) yb += ve.v[e];
+        o.v[e] = yb * (yb > 0.0f ? 1.0f : slope);
+      }
     } else {
       if (acc) o = Pack<4>::load(p);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float d = vx.v[e] - mean;
-        const float yb = fmaf(d, scale, beta);
-        const float dz = vd.v[e] * (yb > 0.0f ? 1.0f : slope);
+        const float yb = EXTRA ? ve.v[e] : fmaf(d, scale, beta);
+        const float dz = vd.v[e] * (early || yb > 0.0f ? 1.0f : slope);
         const float dx = fmaf(scale, dz, fmaf(cB, d, cC));
         o.v[e] = acc ? o.v[e] + dx : dx;
+        z.v[e] = dz;
       }
     }
-#if ANODE_RING_STORE == 1
     o.store_stream(p);
-#elif ANODE_RING_STORE == 2
-    *reinterpret_cast<float4 *>(p) = make_float4(o.v[0], o.v[1], o.v[2], o.v[3]);
-#else
-    o.store(p, drop);
-#endif
+    if constexpr (EXTRA && DIR == 1) { if (dres) z.store_stream(dres + (p - a.out)); }
   };
   for (uint32_t i = 0; i < cnt; ++i, ax += kVecStride, ad += kVecStride) {
     const Pack<4> x0 = lds128(ax);
-    Pack<4> d0 = x0;
+    Pack<4> d0 = x0, e0 = x0;
     if constexpr (DIR == 1) d0 = lds128(ad);
-    one(x0, d0, dst);
+    if constexpr (EXTRA) { if (!early) e0 = lds128(DIR == 1 ? ad + g.slot_floats * 4 : ad); }
+    one(x0, d0, e0, dst);
     advance();
+  }
+  __syncwarp();
+  if (lane == 0) { mbar_arrive(&ctl->empty[slot]); mbar_arrive(&ctl->coef_empty[coef_q]); }
+}
+
+// ---- rows that are not a multiple of four floats ------------------------------------------
+// A row starts h = (its offset) mod 4 floats behind a 16-byte boundary.  The producer fetches every row from the
+// boundary below its start to the one above its end, so that all tensors' vectors (and the output's) line up; a row
+// takes ragged_pitch(len) vectors of the slot and only its first and last ones hold foreign floats, which are left
+// out element by element (and written one by one).  RowWalk steps through the vectors of one thread.
+template <int DIR, bool EXTRA>
+__device__ __forceinline__ void warp_reduce_ragged(const FusedArgs &a, const RingGeom &g, unsigned char *sm, RingCtl *ctl,
+                                                   const TileRange &tr, uint32_t slot, float4 *res)
+{
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t per_row = ragged_pitch(tr.len), nvec = per_row * tr.rows;
+  const uint32_t cnt = tid < nvec ? (nvec - tid + kConsumers - 1) / kConsumers : 0;
+  const int len = (int)tr.len;
+  const float *xs = slot_x(sm, g, slot);
+  uint32_t ax = smem_u32(xs) + tid * 16;
+  RowWalk w;
+  w.init(a, tr, per_row);
+  if constexpr (DIR == 0) {
+    const float K = xs[(uint32_t)tr.base & 3u];      // shift: the tile's first element
+    float s = 0.f, q = 0.f;
+    uint32_t n = 0;
+#pragma unroll 2
+    for (uint32_t i = 0; i < cnt; ++i, ax += kVecStride) {
+      const Pack<4> v = lds128(ax);
+      const int i0 = w.first();
+      if (i0 >= 0 && i0 + 4 <= len) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { const float d = v.v[e] - K; s += d; q = fmaf(d, d, q); }
+        n += 4;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if ((uint32_t)(i0 + e) < (uint32_t)len) { const float d = v.v[e] - K; s += d; q = fmaf(d, d, q); ++n; }
+      }
+      w.advance();
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&ctl->empty[slot]);
+    s = warp_sum(s); q = warp_sum(q);
+    const uint32_t nw = __reduce_add_sync(0xffffffffu, n);
+    if (lane == 0) {
+      Moments m{0.f, 0.f, 0.f};
+      if (nw) {
+        m.n = (float)nw;
+        const float inv = __fdividef(1.0f, m.n);
+        m.mean = fmaf(s, inv, K);
+        m.m2 = fmaxf(q - s * s * inv, 0.f);
+      }
+      res[warp] = make_float4(m.n, m.mean, m.m2, 0.f);
+    }
+  } else {
+    uint32_t ad = ax + g.slot_floats * 4;
+    const float4 cf = slot_side<1, EXTRA>(sm, g, slot)[0];
+    const float mean = cf.x, scale = cf.y, beta = cf.z;
+    const float slope = a.neg_slope;
+    float *dres = EXTRA && a.dres_early ? a.dres : nullptr;
+    float s1 = 0.f, s2 = 0.f;
+    for (uint32_t i = 0; i < cnt; ++i, ax += kVecStride, ad += kVecStride) {
+      const Pack<4> x0 = lds128(ax), g0 = lds128(ad);
+      Pack<4> m0 = x0, z, d;
+      if constexpr (EXTRA) m0 = lds128(ad + g.slot_floats * 4);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        d.v[e] = x0.v[e] - mean;
+        const float y0 = EXTRA ? m0.v[e] : fmaf(d.v[e], scale, beta);
+        z.v[e] = g0.v[e] * (y0 > 0.0f ? 1.0f : slope);
+      }
+      const int i0 = w.first();
+      if (i0 >= 0 && i0 + 4 <= len) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { s1 += z.v[e]; s2 = fmaf(z.v[e], d.v[e], s2); }
+        if constexpr (EXTRA) { if (dres) z.put(dres + w.at()); }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if ((uint32_t)(i0 + e) < (uint32_t)len) {
+            s1 += z.v[e]; s2 = fmaf(z.v[e], d.v[e], s2);
+            if constexpr (EXTRA) { if (dres) dres[w.at() + e] = z.v[e]; }
+          }
+      }
+      w.advance();
+    }
+    if constexpr (EXTRA) { if (dres) fence_global_to_bulk(); }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&ctl->empty[slot]);
+    s1 = warp_sum(s1); s2 = warp_sum(s2);
+    if (lane == 0) res[warp] = make_float4(s1, s2, 0.f, 0.f);
+  }
+}
+
+template <int DIR, bool EXTRA>
+__device__ __forceinline__ void warp_apply_ragged(const FusedArgs &a, const RingGeom &g, unsigned char *sm, RingCtl *ctl,
+                                                  const TileRange &tr, uint32_t slot, const float4 *coef, uint32_t coef_q)
+{
+  const uint32_t tid = threadIdx.x, lane = tid & 31;
+  const float slope = a.neg_slope;
+  const bool acc = a.accumulate != 0;
+  const bool early = EXTRA && DIR == 1 && a.dres_early;
+  float *dres = EXTRA && DIR == 1 && !early ? a.dres : nullptr;
+  const float4 c0 = coef[0], c1 = coef[1];
+  const float mean = c0.x, scale = c0.y, beta = c0.z, cB = c1.x, cC = c1.y;
+  const uint32_t per_row = ragged_pitch(tr.len), nvec = per_row * tr.rows;
+  const uint32_t cnt = tid < nvec ? (nvec - tid + kConsumers - 1) / kConsumers : 0;
+  const int len = (int)tr.len;
+  uint32_t ax = smem_u32(slot_x(sm, g, slot)) + tid * 16;
+  uint32_t ad = ax + g.slot_floats * 4;
+  RowWalk w;
+  w.init(a, tr, per_row);
+  for (uint32_t i = 0; i < cnt; ++i, ax += kVecStride, ad += kVecStride) {
+    const Pack<4> x0 = lds128(ax);
+    Pack<4> d0 = x0, e0 = x0, o, z;
+    if constexpr (DIR == 1) d0 = lds128(ad);
+    if constexpr (EXTRA) { if (!early) e0 = lds128(DIR == 1 ? ad + g.slot_floats * 4 : ad); }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float d = x0.v[e] - mean;
+      if constexpr (DIR == 0) {
+        float yb = fmaf(d, scale, beta);
+        if constexpr (EXTRA) yb += e0.v[e];
+        o.v[e] = yb * (yb > 0.0f ? 1.0f : slope);
+      } else {
+        const float yb = EXTRA ? e0.v[e] : fmaf(d, scale, beta);
+        z.v[e] = d0.v[e] * (early || yb > 0.0f ? 1.0f : slope);
+        o.v[e] = fmaf(scale, z.v[e], fmaf(cB, d, cC));
+      }
+    }
+    const int i0 = w.first();
+    float *p = a.out + w.at();
+    if (i0 >= 0 && i0 + 4 <= len) {
+      if (DIR == 1 && acc) {
+        const Pack<4> old = Pack<4>::load(p);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o.v[e] = old.v[e] + o.v[e];
+      }
+      o.store_stream(p);
+      if constexpr (EXTRA && DIR == 1) { if (dres) z.store_stream(dres + w.at()); }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if ((uint32_t)(i0 + e) < (uint32_t)len) {
+          p[e] = DIR == 1 && acc ? p[e] + o.v[e] : o.v[e];
+          if constexpr (EXTRA && DIR == 1) { if (dres) dres[w.at() + e] = z.v[e]; }
+        }
+    }
+    w.advance();
   }
   __syncwarp();
   if (lane == 0) { mbar_arrive(&ctl->empty[slot]); mbar_arrive(&ctl->coef_empty[coef_q]); }
@@ -625,7 +812,8 @@ __device__ __forceinline__ bool pull_merge_unit(const FusedArgs &a, RingCtl *ctl
 // ======================================================================================
 // Whole-row tiles only (one channel per unit): short-row shapes are served by the cluster kernel
 // (bn_segres.cu) and the plain kernel.
-template <int DIR>
+// EXTRA: residual epilogue; RAGGED: rows that are not a multiple of four floats.
+template <int DIR, bool EXTRA, bool RAGGED>
 __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArgs a, const RingGeom g)
 {
   extern __shared__ __align__(128) unsigned char sm[];
@@ -633,7 +821,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
   const Plan &P = a.plan;
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint32_t *status = a.status;
-  uint32_t *exit_ctr = ws_u32(a, 4);
+  uint32_t *exit_ctr = ws_u32(a, g.hdr);
   uint32_t *done = ws_u32(a, P.off_done);
 
   if (tid == 0) {
@@ -641,7 +829,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
     for (uint32_t i = 0; i < kResQ; ++i) { mbar_init(&ctl->res_full[i], kCWarps); mbar_init(&ctl->res_empty[i], 1); }
     for (uint32_t i = 0; i < kCoefQ; ++i) { mbar_init(&ctl->coef_full[i], 1); mbar_init(&ctl->coef_empty[i], kCWarps); }
     ctl->abort = 0; ctl->last_block = 0;
-    ctl->parity = *ws_u32(a, 8) & 1u;
+    ctl->parity = *ws_u32(a, g.hdr + 4) & 1u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -663,14 +851,16 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
         bool ok = warp_wait(&ctl->res_empty[q], qpar ^ 1u, ctl, status, ANODE_ST_WAIT_STATS);
         ok = ok && warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS);
         if (!ok) break;                                 // warps are independent: no barrier to honour
-        warp_reduce_R<DIR>(a, g, sm, ctl, tr, slot, res_box(sm, g, q));
+        if constexpr (RAGGED) warp_reduce_ragged<DIR, EXTRA>(a, g, sm, ctl, tr, slot, res_box(sm, g, q));
+        else warp_reduce_R<DIR, EXTRA>(a, g, sm, ctl, tr, slot, res_box(sm, g, q));
         if (lane == 0) mbar_arrive(&ctl->res_full[q]);
       } else {
         const uint32_t q = ncoef % kCoefQ, qpar = (ncoef / kCoefQ) & 1u; ++ncoef;
         bool ok = warp_wait(&ctl->coef_full[q], qpar, ctl, status, ANODE_ST_WAIT_STATS);
         ok = ok && warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS);
         if (!ok) break;
-        warp_apply_R<DIR>(a, g, sm, ctl, tr, slot, coef_box(sm, g, P.cb, q), q);
+        if constexpr (RAGGED) warp_apply_ragged<DIR, EXTRA>(a, g, sm, ctl, tr, slot, coef_box(sm, g, P.cb, q), q);
+        else warp_apply_R<DIR, EXTRA>(a, g, sm, ctl, tr, slot, coef_box(sm, g, P.cb, q), q);
       }
     }
   } else if (warp == kConsumers / 32) {
@@ -678,7 +868,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
     // where the window between the two visits exceeds what L2 keeps, only the fraction that fits is marked "keep"
     const uint64_t keep = g.keep_frac < 1.0f ? policy_keep_fraction(g.keep_frac) : policy_keep(), drop = policy_drop();
     const uint64_t rs = (uint64_t)P.C * P.dim0;
-    uint32_t k = 0;
+    uint32_t k = 0, applied = 0;
     uint32_t slot = g.slots - 1, par = 1;
     bool ok = true;
     TileRange tr;
@@ -703,6 +893,16 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
       // visits exceeds what L2 keeps, and hardly faster elsewhere)
       uint32_t okw = 1;
       if (lane == 0) okw = mbar_wait(&ctl->empty[slot], par ^ 1u, ctl, status, ANODE_ST_WAIT_STATS) ? 1u : 0u;
+      if constexpr (DIR == 1 && EXTRA) {
+        // the dz this visit reads back was stored by visit kr, which must have been given back: implied by the wait
+        // above unless fewer than `slots` visits lie in between (blocks with a few tiles)
+        if (kind == 1) {
+          const uint32_t kr = applied + (applied > sc.look ? applied - sc.look : 0u);
+          if (lane == 0 && okw && a.dres_early && k - 1 - kr < g.slots)
+            okw = mbar_wait(&ctl->empty[kr % g.slots], (kr / g.slots) & 1u, ctl, status, ANODE_ST_WAIT_STATS) ? 1u : 0u;
+          ++applied;
+        }
+      }
       ok = __shfl_sync(0xffffffffu, okw, 0) != 0;     // one lane decides for the warp
       if (!ok) { --k; break; }
       float *xs = slot_x(sm, g, slot);
@@ -717,23 +917,77 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
           next_c = tr.c0 + 1 < P.C ? tr.c0 + 1 : tr.c0;
           next_raw = load_side_raw(next_c); next_pending = true; next_age = 0;
         }
-        if (lane == 0) slot_side<1>(sm, g, slot)[0] = side_v;
+        if (lane == 0) slot_side<1, EXTRA>(sm, g, slot)[0] = side_v;
       }
       __syncwarp();
-      const uint32_t row_bytes = tr.len * 4u;
-      if (lane == 0) mbar_arrive_expect_tx(&ctl->full[slot], row_bytes * tr.rows * (DIR == 1 ? 2u : 1u));
-      __syncwarp();
       const uint64_t pol = (kind == 0 && a.mode == MODE_FUSED) ? keep : drop;
+      // the visit's tensors: x; dy, or the dz that the reduce visit stored; residual or saved output where it is needed
+      const float *p1 = nullptr, *p2 = nullptr;
+      uint64_t pol1 = pol;
+      if constexpr (DIR == 1) {
+        p1 = a.dy;
+        if constexpr (EXTRA) {
+          if (!a.dres_early) p2 = a.ymask;
+          else if (kind == 0) { p2 = a.ymask; pol1 = drop; }      // dy and the saved output are not read again
+          else p1 = a.dres;
+        }
+      } else if constexpr (EXTRA) {
+        if (kind == 1) p1 = a.res;
+      }
+      const uint32_t planes = 1u + (p1 ? 1u : 0u) + (p2 ? 1u : 0u);
       // every row is fetched as several bulk copies (one per lane at a time), so that a tile made of
       // one long row still has many copies in flight
-      const uint32_t per_row = (row_bytes + kCopyBytes - 1) / kCopyBytes, ncopies = per_row * tr.rows;
-      for (uint32_t c = lane; c < ncopies; c += 32) {
-        const uint32_t r = c / per_row, o = (c - r * per_row) * kCopyBytes;
-        const uint32_t nb = row_bytes - o < kCopyBytes ? row_bytes - o : kCopyBytes;
-        const size_t goff = (size_t)tr.base + (size_t)r * rs + o / 4;
-        float *dst = xs + (size_t)r * tr.len + o / 4;
-        bulk_g2s(dst, a.x + goff, nb, &ctl->full[slot], pol);
-        if (DIR == 1) bulk_g2s(dst + g.slot_floats, a.dy + goff, nb, &ctl->full[slot], pol);
+      if constexpr (!RAGGED) {
+        const uint32_t row_bytes = tr.len * 4u;
+        if (lane == 0) mbar_arrive_expect_tx(&ctl->full[slot], row_bytes * tr.rows * planes);
+        __syncwarp();
+        const uint32_t per_row = (row_bytes + kCopyBytes - 1) / kCopyBytes, ncopies = per_row * tr.rows;
+        for (uint32_t c = lane; c < ncopies; c += 32) {
+          const uint32_t r = c / per_row, o = (c - r * per_row) * kCopyBytes;
+          const uint32_t nb = row_bytes - o < kCopyBytes ? row_bytes - o : kCopyBytes;
+          const size_t goff = (size_t)tr.base + (size_t)r * rs + o / 4;
+          float *dst = xs + (size_t)r * tr.len + o / 4;
+          bulk_g2s(dst, a.x + goff, nb, &ctl->full[slot], pol);
+          if (p1) bulk_g2s(dst + g.slot_floats, p1 + goff, nb, &ctl->full[slot], pol1);
+          if (p2) bulk_g2s(dst + 2 * g.slot_floats, p2 + goff, nb, &ctl->full[slot], pol1);
+        }
+      } else {
+        // from the boundary below each row's start to the one above its end, but never past the tensor's own end:
+        // the last floats of a tensor whose size is no multiple of four are stored by three lanes instead
+        const uint32_t per_row = ragged_pitch(tr.len);
+        const uint64_t total = rs * P.N;
+        auto span = [&](uint32_t r, uint64_t &start) {      // bytes of row r, and the float it is fetched from
+          const uint64_t first = tr.base + r * rs, whole = total & ~3ull;
+          start = first & ~3ull;
+          uint64_t end = (first + tr.len + 3) & ~3ull;
+          if (end > whole) end = whole;
+          return (uint32_t)(end - start) * 4u;
+        };
+        uint32_t bytes = 0;
+        for (uint32_t r = lane; r < tr.rows; r += 32) { uint64_t start; bytes += span(r, start); }
+        bytes = __reduce_add_sync(0xffffffffu, bytes) * planes;
+        const uint64_t last = tr.base + (tr.rows - 1) * rs, tail = total & 3ull;
+        if (tail && last + tr.len == total && lane < tail) {
+          const uint64_t src = (total & ~3ull) + lane;
+          float *dst = xs + 4 * (size_t)per_row * (tr.rows - 1) + (src - (last & ~3ull));
+          *dst = __ldcg(a.x + src);
+          if (p1) dst[g.slot_floats] = __ldcg(p1 + src);
+          if (p2) dst[2 * g.slot_floats] = __ldcg(p2 + src);
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // (before a later copy into this slot)
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive_expect_tx(&ctl->full[slot], bytes);
+        __syncwarp();
+        for (uint32_t r = lane; r < tr.rows; r += 32) {
+          uint64_t start;
+          const uint32_t nb = span(r, start);
+          float *dst = xs + 4 * (size_t)per_row * r;
+          if (nb) {
+            bulk_g2s(dst, a.x + start, nb, &ctl->full[slot], pol);
+            if (p1) bulk_g2s(dst + g.slot_floats, p1 + start, nb, &ctl->full[slot], pol1);
+            if (p2) bulk_g2s(dst + 2 * g.slot_floats, p2 + start, nb, &ctl->full[slot], pol1);
+          }
+        }
       }
       // the values fetched ahead are turned into coefficients one visit later, when they have arrived
       if (DIR == 1 && next_pending && next_age++ >= 1) { next_v = finish_side(next_raw); next_pending = false; }
@@ -876,7 +1130,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
     }
     __syncthreads();
     if (ctl->last_block && tid == 0) {
-      *ws_u32(a, 8) = ctl->parity ^ 1u;       // the next launch uses the other partial buffer
+      *ws_u32(a, g.hdr + 4) = ctl->parity ^ 1u;       // the next launch uses the other partial buffer
       *exit_ctr = 0;
     }
   }

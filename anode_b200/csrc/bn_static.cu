@@ -59,7 +59,7 @@ static void static_need(const FusedArgs &a, bool aligned, uint64_t &need, uint64
       break;
     }
     default:                          // tiled and slice-resident kernels: their share of a workspace part
-      need = workspace_part_bytes(dim0, C, N);
+      need = dim0 % 4 == 0 ? workspace_static_bytes(dim0, C, N) : ring_ws_bytes(a, 0, aligned);
       clear = control_region_bytes(dim0, C, N, aligned);
       break;
   }

@@ -244,3 +244,59 @@ def test_tiled_schedule_cannot_wait_in_a_cycle():
     # the exact bound; the planner asks for one step more, and for the slack on top)
     assert not simulate_tiled_schedule(tiles=8 * 40, per_unit=40, grid=8, look=3)
     assert simulate_tiled_schedule(tiles=8 * 40, per_unit=40, grid=8, look=4)
+
+
+def ragged_walk(tid, threads, base, rows, length, rs):
+    """The vectors of one thread in a ragged tile: (slot vector, float offset in the tensor, its first float's place in the row)."""
+    pitch = (length + 6) // 4
+    r, sr = (tid // pitch, threads // pitch) if rows > 1 else (0, 0)
+    col, row = tid - r * pitch, base + r * rs
+    for v in range(tid, pitch * rows, threads):
+        yield v, (row & ~3) + 4 * col, 4 * col - (row & 3)
+        row += sr * rs
+        col += threads - sr * pitch
+        if col >= pitch:
+            col -= pitch
+            row += rs
+
+
+def test_ragged_tiles_cover_every_float_once():
+    """Rows of a length that is no multiple of four: the tiled kernel fetches each from the 16-byte boundary below its
+    start to the one above its end (not past the tensor's end) and its threads walk the vectors.  For the planner's
+    geometries: tiles fit their slots, no copy leaves the slot or the tensor, and the walks of a tile's threads take
+    every float of its rows exactly once, from the place in the slot where the copy put it."""
+    for d0, c, n in [(161, 3, 7), (167, 5, 1), (225, 7, 64), (1023, 1, 33), (3025, 5, 9), (8191, 3, 3), (16781, 3, 2),
+                     (65543, 3, 1), (16705, 13, 2), (3026, 3, 5), (3027, 3, 5)]:
+        rs, total = d0 * c, d0 * c * n
+        for direction in (0, 1):
+            g = tiled_geometry(d0, c, n, direction)
+            assert g["applies"] == 1 and g["smem"] <= 227 * 1024
+            planes, threads = (2, 512) if direction else (1, 256)
+            slot_floats = g["slot_bytes"] // 4 // planes
+            pieces = -(-d0 // g["piece"])
+            assert g["tiles_per_unit"] == pieces * -(-n // g["rows"]) and g["lookahead"] * g["grid"] >= g["tiles_per_unit"]
+            for ch in {0, c - 1}:
+                for k in {0, 1, g["tiles_per_unit"] // 2, g["tiles_per_unit"] - 1}:
+                    if k >= g["tiles_per_unit"]:
+                        continue
+                    sb, piece = divmod(k, pieces)
+                    rows, length = min(g["rows"], n - sb * g["rows"]), min(g["piece"], d0 - piece * g["piece"])
+                    assert rows == 1 or pieces == 1
+                    base = (sb * g["rows"] * c + ch) * d0 + piece * g["piece"]
+                    pitch = (length + 6) // 4
+                    assert 4 * pitch * rows <= slot_floats
+                    slot = {}
+                    for r in range(rows):
+                        first = base + r * rs
+                        lo, hi = first & ~3, min((first + length + 3) & ~3, total & ~3)
+                        assert hi - lo <= 4 * pitch
+                        for f in range(lo, max(hi, min(first + length, total))):     # the copy, and the lanes' tail
+                            slot[4 * pitch * r + f - lo] = f
+                    seen = []
+                    for tid in range(threads):
+                        for v, at, i0 in ragged_walk(tid, threads, base, rows, length, rs):
+                            for e in range(4):
+                                if 0 <= i0 + e < length:
+                                    assert slot[4 * v + e] == at + e
+                                    seen.append(at + e)
+                    assert sorted(seen) == sorted(base + r * rs + i for r in range(rows) for i in range(length)), (d0, c, n, k)
