@@ -33,9 +33,6 @@ struct ChanGeom {
   double inv_count;
 };
 
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // float4 into the shared memory of block `rank` of the cluster, at the address `p` has in this block
 __device__ __forceinline__ void st_cluster_f4(void *p, uint32_t rank, float4 v)
 {
@@ -263,14 +260,17 @@ static bool chan_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra
   return true;
 }
 
-// Where this kernel is taken: wherever a team can hold the channel, except on large layers of short unaligned rows whose
-// runs of several channels are aligned.  There the scalar walk (some 22 instructions per element) costs more than the
-// shared-memory cluster kernel's chain of phases ([1024,2048,7,7] forward 310 us here, 200 us there; [64,512,7,7] the
-// other way round).  Forward + backward at the kernels' places, before and now: [2,512,7,7] 11.5 -> 4.5 us,
-// [32,64,28,28] 20.7 -> 9.8, [1,53,39,25] 17.9 -> 5.2, [1,260,128,128] 34.0 -> 16.7, [1,1240,45,30] 60.5 -> 13.8,
-// [40,2048,146,5] 630 -> 413, residual [256,1024,14,14] 459 -> 377.  Large layers of ragged rows go to the tiled kernel
-// (`tiled_ok`) from rows of kChanLongRow floats on: [39,255,45,45] forward 62 us here, 44 us there, [349,255,15,15] 64 and
-// 68 us, [45,33,45,45] 12.9 and 15.5 us.
+// Where this kernel is taken: wherever a team can hold the channel, except on large layers where the team would be of
+// more than half the largest size (its load, exchange and store then follow one another on most of the device) and
+// where the elements would be fetched one by one although aligned runs of several channels, or long ragged rows, can be
+// had (the scalar walk costs some 22 instructions per element).
+// Forward + backward at the places of other kernels, there and here: [2,512,7,7] 11.5 -> 4.5 us, [32,64,28,28] 20.7 ->
+// 9.8, [1,53,39,25] 17.9 -> 5.2, [1,260,128,128] 34.0 -> 16.7, [1,1240,45,30] 60.5 -> 13.8, [40,2048,146,5] 630 -> 413.
+// The other way round, us here and there: streaming kernel, forward [512,1024,14,14] 213 and 185, backward
+// [256,1024,14,14] 164 and 147, residual epilogue 156 / 222 and 137 / 209; [64,2048,7,7] 19.0 / 25.5 and 15.0 / 20.4,
+// but [300,100,7,7] 5.9 / 8.6 and 6.7 / 8.3.  Tiled kernel, forward [128,512,28,28] 105 and 87, [39,255,45,45] 62 and
+// 44, but [349,255,15,15] 64 and 68, [45,33,45,45] 12.9 and 15.5.
+constexpr uint64_t kChanLarge = 8u << 20, kChanLargeScalar = 3u << 20;      // elements from which on the others are asked
 constexpr uint32_t kChanLongRow = 300;
 bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
 {
@@ -278,9 +278,15 @@ bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
   if (a.mode != MODE_FUSED || a.world > 1) return false;
   if (!chan_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, extra, aligned, g)) return false;
-  const uint64_t elements = (uint64_t)a.plan.dim0 * a.plan.C * a.plan.N;
-  if (g.vec == 4 || elements < (8u << 20)) return true;
-  return !segres_applies(a, dir, aligned) && !(tiled_ok && a.plan.dim0 >= kChanLongRow);
+  const uint64_t channel = (uint64_t)a.plan.dim0 * a.plan.N, elements = channel * a.plan.C;
+  const uint32_t most = dir == 0 && !extra ? 32u : 16u;
+  if (g.vec == 4) {
+    if (elements < kChanLarge || channel <= (uint64_t)kChanThreads * kChanCluster * most / 2) return true;
+    return !stream_preferred(a, dir, aligned, tiled_ok) && !(dir == 0 && !extra && tiled_ok);
+  }
+  if (elements < kChanLargeScalar) return true;
+  if (stream_preferred(a, dir, aligned, tiled_ok)) return false;
+  return elements < kChanLarge || !(segres_applies(a, dir, aligned) || (tiled_ok && a.plan.dim0 >= kChanLongRow));
 }
 
 int launch_chan(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)

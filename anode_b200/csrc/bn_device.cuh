@@ -36,6 +36,10 @@ __device__ __forceinline__ void st_release_sys(uint32_t *p, uint32_t v)
   asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+// ---- programmatic dependent launch: wait for the kernel before this one on the stream; let the next one be scheduled
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- L2 eviction policies ----------------------------------------------------------------
 // keep: data that will be read a second time (the reduce pass of a tile);
 // drop: data that is dead after this access (the apply pass's re-read, and every output).

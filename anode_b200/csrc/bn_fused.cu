@@ -373,6 +373,7 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
     case ANODE_KERNEL_PLAIN: if (plain_ok) return ANODE_KERNEL_PLAIN; break;
     default:
       if (chan_preferred(a, dir, aligned, tiled_ok)) return kKernelChan;
+      if (stream_preferred(a, dir, aligned, tiled_ok)) return kKernelStream;
       break;
   }
   if (extra) {
@@ -384,8 +385,10 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
     if (plain_ok) return ANODE_KERNEL_PLAIN;
     return resident_applies(a, dir, aligned) ? ANODE_KERNEL_RESIDENT : -1;
   }
-  // short rows, and channels small enough to sit in a few blocks' shared memory: the cluster kernel
-  if (segres_preferred(a, dir, aligned)) return ANODE_KERNEL_CLUSTER;
+  // short rows, and in synchronized calls channels small enough to sit in a few blocks' shared memory: the cluster
+  // kernel (on one GPU the register-resident kernel has those, and of large layers the tiled kernel is the faster one:
+  // [128,512,28,28] forward 87 us, 105 us on the cluster kernel)
+  if (segres_preferred(a, dir, aligned) && !(tiled_ok && a.world <= 1 && kernel_choice() == ANODE_KERNEL_AUTO)) return ANODE_KERNEL_CLUSTER;
   if (tiled_ok) return ANODE_KERNEL_TILED;
   if (segres_applies(a, dir, aligned)) return ANODE_KERNEL_CLUSTER;
   if (plain_ok) return ANODE_KERNEL_PLAIN;
@@ -398,6 +401,10 @@ int launch_best(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)
 {
   int kind = pick_kernel_kind(a, dir, aligned);
   if (kind == kKernelChan) return launch_chan(a, dir, aligned, stream);
+  if (kind == kKernelStream) {
+    if (launch_stream(a, dir, stream) == ANODE_OK) return ANODE_OK;
+    kind = segres_applies(a, dir, aligned) ? ANODE_KERNEL_CLUSTER : ANODE_KERNEL_PLAIN;
+  }
   if (kind == ANODE_KERNEL_CLUSTER) {
     if (launch_segres(a, dir, stream) == ANODE_OK) return ANODE_OK;
     Plan rp; RingGeom g;
@@ -677,12 +684,14 @@ extern "C" int anode_gpu_online_average_f32(uint32_t len, float rate, const floa
   return ANODE_OK;
 }
 
-// The family callers see (ANODE_KERNEL_*): the register-resident kernel counts as a cluster kernel on the shapes of
-// that family and as the any-shape, any-alignment kernel elsewhere.
+// The family callers see (ANODE_KERNEL_*), by the shapes it stands for: the register-resident and the streaming kernel
+// count as cluster kernels on the shapes of that family and as the any-shape, any-alignment family elsewhere, and so do
+// the tiled kernel's ragged rows.
 static int public_kind(const FusedArgs &a, int dir, bool aligned)
 {
   const int k = pick_kernel_kind(a, dir, aligned);
-  if (k != kKernelChan) return k;
+  if (k == ANODE_KERNEL_TILED && a.plan.dim0 % 4 != 0) return ANODE_KERNEL_PLAIN;
+  if (k != kKernelChan && k != kKernelStream) return k;
   return segres_applies(a, dir, aligned) ? ANODE_KERNEL_CLUSTER : ANODE_KERNEL_PLAIN;
 }
 

@@ -36,7 +36,7 @@ struct FusedArgs {
   // from the saved output ymask and also writes dres = dy*mask
   const float *res, *ymask;
   float *dres;
-  uint32_t dres_early;     // tiled kernel: dres is written by the reduce visits and read back by the apply visits
+  uint32_t dres_early;     // tiled and streaming kernels: dres is written with the sums and read back when dx is made
   float *out;              // y (forward) or dx (backward)
   float *mean, *var, *run_mean, *run_var;   // forward outputs
   float *dgamma, *dbeta;   // backward outputs

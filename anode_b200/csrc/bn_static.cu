@@ -49,15 +49,16 @@ static void static_need(const FusedArgs &a, bool aligned, uint64_t &need, uint64
 {
   const uint32_t dim0 = a.plan.dim0, C = a.plan.C, N = a.plan.N;
   switch (pick_kernel_kind(a, 0, aligned)) {
+    case kKernelStream:               // (where the device refuses its cluster, the plain kernel may have to serve the call)
+    case ANODE_KERNEL_PLAIN: {
+      const Plan p = plan_for(dim0, C, N, aligned);
+      need = p.ws_bytes; clear = p.off_part;
+      if (pick_kernel_kind(a, 0, aligned) == ANODE_KERNEL_PLAIN || !segres_applies(a, 0, aligned)) break;
+    }                                 // fall through
     case kKernelChan:
     case ANODE_KERNEL_CLUSTER:        // keep everything on chip: only the status word lives in the array
       need = clear = 256;
       break;
-    case ANODE_KERNEL_PLAIN: {
-      const Plan p = plan_for(dim0, C, N, aligned);
-      need = p.ws_bytes; clear = p.off_part;
-      break;
-    }
     default:                          // tiled and slice-resident kernels: their share of a workspace part
       need = dim0 % 4 == 0 ? workspace_static_bytes(dim0, C, N) : ring_ws_bytes(a, 0, aligned);
       clear = control_region_bytes(dim0, C, N, aligned);

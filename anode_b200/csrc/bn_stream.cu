@@ -1,0 +1,389 @@
+// Fused batch-norm (+activation, +residual) for large layers of short rows, e.g. [1024, 2048, 7, 7]: a channel's data is
+// thousands of short runs far apart, too many to hold on chip.
+//
+// A unit is a block of cb channels, i.e. per sample one contiguous, 16-byte aligned run of cb*dim0 floats.  A
+// thread-block CLUSTER owns one unit and splits its samples; a thread keeps one float4 column of the run and walks down
+// the samples twice:
+//   1. statistics: kBatch 128-bit loads in flight per thread, shifted sums (or the backward sums) per column in registers,
+//      folded over the block's threads in a fixed order in double precision;
+//   2. each block pushes its channel sums into every block of the cluster (remote shared memory), one cluster barrier;
+//   3. every block merges them in rank order (bit-identical coefficients) and walks its samples again, last batch first:
+//      that one is still in registers, the others come from L2.  The cluster size keeps what all resident blocks have
+//      between their two walks within reach of L2 (kStreamWindow).
+//
+// What bounds it: HBM and the loads in flight.  Nothing is staged in shared memory, so the blocks per SM are limited by
+// registers only and some stream while others fold and wait; the kernel that holds the slices in shared memory
+// (bn_segres.cu) runs its load, six dependent phases and store one after the other.
+// Forward / backward: [1024,2048,7,7] 203 / 436 us there, 179 / 298 us here (0.70 / 0.63 of the copy bandwidth),
+// [256,1024,14,14] backward 164 -> 147; where a unit does not fit sixteen blocks' shared memory and the plain kernel
+// served the layer, [4096,512,7,7] 490 / 797 -> 206 / 338, [1024,64,15,15] 87 / 178 -> 31 / 54, residual
+// [1024,2048,7,7] 383 / 1151 -> 248 / 420.
+//
+// Reference kernels this replaces: routines_gpu/batch_norm.cu:24-57, 125-163, 314-336 (forward), :181-206, 240-280,
+// 354-376, 408-444, 476-515 (backward), flat_map.cu:172-194 (ReLU).
+#include "bn_device.cuh"
+#include "bn_host.h"
+
+namespace anode_b200 {
+
+// Most threads of a block, and blocks per SM.  [1024,2048,7,7] forward / backward: three of 256 threads (80 registers)
+// 180 / 298 us, two of 448 (72) 193 / 319, two of 352 (88) 190 / 304, four of 256 (64) 251 / 392.
+constexpr uint32_t kStreamThreads = 256, kStreamBlocks = 3;
+constexpr uint32_t kStreamRecords = 1024;    // most channels * blocks of a unit
+constexpr uint32_t kStreamChannels = 128;    // most channels of a unit
+
+struct StreamGeom {
+  uint32_t cb, units;        // channels per unit
+  uint32_t cluster, rows;    // blocks per unit, samples per block
+  uint32_t groups, threads;  // sample groups of a block: thread = group * vectors per run + vector
+  double inv_count;
+};
+
+// two doubles into the shared memory of block `rank` of the cluster, at the address `p` has in this block
+__device__ __forceinline__ void st_cluster_d2(void *p, uint32_t rank, double x, double y)
+{
+  const uint32_t local = (uint32_t)__cvta_generic_to_shared(p);
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(remote), "d"(x), "d"(y) : "memory");
+}
+
+template <int DIR, bool EXTRA>
+__global__ void __launch_bounds__(kStreamThreads, kStreamBlocks) bn_stream_kernel(const FusedArgs a, const StreamGeom g)
+{
+  constexpr int kBatch = DIR == 0 && !EXTRA ? 8 : 4;     // samples in flight per thread (more of them spill)
+  __shared__ double2 part[2][kStreamThreads];            // per thread: its sums for the one or two channels of its column
+  __shared__ double2 rec[kStreamRecords];                // [channel][block of the cluster]
+  __shared__ float4 coef0[kStreamChannels];              // mean, gamma/std, beta, -
+  __shared__ float2 coef1[kStreamChannels];              // backward: factor of x - mean, constant
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = (blockDim.x + 31) >> 5;
+  const uint32_t csh = (uint32_t)__ffs((int)g.cluster) - 1u;
+  const uint32_t u = blockIdx.x >> csh, rank = blockIdx.x & (g.cluster - 1u);
+  const uint32_t dim0 = a.plan.dim0, C = a.plan.C, N = a.plan.N;
+  // remote shared memory may only be written once its block runs (collected right before the first remote store)
+  if (g.cluster > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  const uint32_t c0 = u * g.cb, cw = C - c0 < g.cb ? C - c0 : g.cb;
+  const uint32_t L4 = cw * dim0 / 4, rs = C * dim0;
+  const uint32_t grp = tid / L4, v = tid - grp * L4;
+  const uint32_t n0 = rank * g.rows, rows = n0 < N ? (N - n0 < g.rows ? N - n0 : g.rows) : 0;
+  const uint32_t nk = grp < g.groups && grp < rows ? (rows - grp - 1) / g.groups + 1 : 0;      // this thread's samples
+  const uint32_t step = g.groups * rs;                   // float offsets are below 2^32 (check_dims) wherever k < nk
+  const uint32_t off0 = (n0 + grp) * rs + c0 * dim0 + 4 * v;
+  // the column's four floats lie in channel chA up to float eB, in the next one from there on
+  const uint32_t chA = grp < g.groups ? 4 * v / dim0 : 0;
+  const uint32_t eB = (chA + 1) * dim0 - 4 * v;
+  const uint32_t chB = eB < 4 && chA + 1 < cw ? chA + 1 : chA;
+  const float slope = a.neg_slope;                       // activation: t * (t > 0 ? 1 : slope)
+  const bool early = DIR == 1 && EXTRA && a.dres_early;  // dz is stored in the first walk and read back in the second
+  const uint64_t keep = policy_keep(), drop = policy_drop();
+  pdl_wait();
+  pdl_trigger();
+
+  float mean[4], scale[4], beta[4];
+  if (DIR == 1) {
+    const float mA = a.mean_in[c0 + chA], mB = a.mean_in[c0 + chB];
+    const float sA = (a.gamma ? a.gamma[c0 + chA] : 1.0f) * inv_std(a.var_in[c0 + chA]);
+    const float sB = (a.gamma ? a.gamma[c0 + chB] : 1.0f) * inv_std(a.var_in[c0 + chB]);
+    const float bA = a.gamma && a.beta ? a.beta[c0 + chA] : 0.f, bB = a.gamma && a.beta ? a.beta[c0 + chB] : 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) { const bool b = (uint32_t)e >= eB; mean[e] = b ? mB : mA; scale[e] = b ? sB : sA; beta[e] = b ? bB : bA; }
+  }
+
+  // ---- first walk
+  Pack<4> vx[kBatch], vd[DIR == 1 ? kBatch : 1];         // after the walk: the last batch (vd: its dz)
+  float s[4] = {0.f, 0.f, 0.f, 0.f}, q[4] = {0.f, 0.f, 0.f, 0.f}, K[4] = {0.f, 0.f, 0.f, 0.f};
+  uint32_t kb = 0;
+  for (uint32_t k = 0; k < nk; k += kBatch) {
+    kb = k;
+    Pack<4> vm[DIR == 1 && EXTRA ? kBatch : 1];
+#pragma unroll
+    for (int i = 0; i < kBatch; ++i) {
+      const uint32_t off = off0 + (k + i) * step;
+      vx[i] = pack_fill<4>(0.f);
+      if (k + i < nk) {
+        vx[i] = Pack<4>::load(a.x + off, keep);
+        if (DIR == 1) vd[i] = Pack<4>::load(a.dy + off, early ? drop : keep);
+        if (DIR == 1 && EXTRA) vm[i] = Pack<4>::load(a.ymask + off, early ? drop : keep);
+      }
+    }
+    if (DIR == 0) {
+      if (k == 0) {
+        // shift of the sums: the mean of the column's first batch
+        const float inv = __fdividef(1.0f, (float)(nk < kBatch ? nk : kBatch));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float t = 0.f;
+#pragma unroll
+          for (int i = 0; i < kBatch; ++i) t += vx[i].v[e];
+          K[e] = t * inv;
+        }
+      }
+      // batch by batch, so that a long column's sums are rounded once per batch
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float bs = 0.f, bq = 0.f;
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+          const float d = k + i < nk ? vx[i].v[e] - K[e] : 0.f;
+          bs += d; bq = fmaf(d, d, bq);
+        }
+        s[e] += bs; q[e] += bq;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i)
+        if (k + i < nk) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float d = vx[i].v[e] - mean[e];
+            const float yb = EXTRA ? vm[i].v[e] : fmaf(d, scale[e], beta[e]);
+            vd[i].v[e] *= yb > 0.0f ? 1.0f : slope;      // dz = dy * act'(y)  (routines_gpu/flat_map.cu:191-192)
+            s[e] += vd[i].v[e]; q[e] = fmaf(vd[i].v[e], d, q[e]);
+          }
+          if (EXTRA && early) vd[i].put(a.dres + (off0 + (k + i) * step));
+        }
+    }
+  }
+
+  // ---- the thread's sums for its channels: of x and x^2 about zero (from the shifted sums, in double precision: nothing
+  // that the f32 sums hold is lost), or the backward sums
+  {
+    double2 p[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      double t1 = (double)s[e], t2 = (double)q[e];
+      if (DIR == 0) {
+        const double n = (double)nk, k = (double)K[e];
+        t2 = fma(k, fma(n, k, 2.0 * t1), t2); t1 = fma(n, k, t1);
+      }
+      const bool b = (uint32_t)e >= eB;
+      p[0].x += b ? 0.0 : t1; p[0].y += b ? 0.0 : t2;
+      p[1].x += b ? t1 : 0.0; p[1].y += b ? t2 : 0.0;
+    }
+    part[0][tid] = p[0]; part[1][tid] = p[1];
+  }
+  __syncthreads();
+
+  // ---- the block's sums: one warp per channel over the threads whose column touches it, in a fixed order
+  if (g.cluster > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  for (uint32_t ci = warp; ci < cw; ci += warps) {
+    const uint32_t v0 = ci * dim0 / 4, nv = (ci * dim0 + dim0 - 1) / 4 - v0 + 1;
+    double t1 = 0.0, t2 = 0.0;
+    for (uint32_t i = lane; i < nv * g.groups; i += 32) {
+      const uint32_t gi = i / nv, vi = v0 + i - gi * nv;
+      const double2 p = part[4 * vi < ci * dim0 ? 1 : 0][gi * L4 + vi];     // (a column that starts in the channel before)
+      t1 += p.x; t2 += p.y;
+    }
+    t1 = warp_sum_all(t1); t2 = warp_sum_all(t2);
+    if (g.cluster > 1) { if (lane < g.cluster) st_cluster_d2(&rec[ci * g.cluster + rank], lane, t1, t2); }
+    else if (lane == 0) rec[ci] = make_double2(t1, t2);
+  }
+  if (g.cluster > 1) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  } else {
+    __syncthreads();
+  }
+
+  // ---- merged in rank order by every block; block 0 writes the channel's results
+  for (uint32_t ci = tid; ci < cw; ci += blockDim.x) {
+    const uint32_t c = c0 + ci;
+    double t1 = 0.0, t2 = 0.0;
+    for (uint32_t r = 0; r < g.cluster; ++r) { const double2 p = rec[ci * g.cluster + r]; t1 += p.x; t2 += p.y; }
+    const float gm = a.gamma ? a.gamma[c] : 1.0f;
+    const float bt = (a.gamma && a.beta) ? a.beta[c] : 0.0f;
+    if (DIR == 0) {
+      const double md = t1 * g.inv_count;
+      const float mf = (float)md;
+      const float vf = (float)(fmax(t2 - t1 * md, 0.0) * g.inv_count + (double)a.epsilon);      // biased, epsilon folded in (batch_norm.cu:160)
+      coef0[ci] = make_float4(mf, gm * inv_std(vf), bt, 0.f);
+      if (rank == 0) {
+        a.mean[c] = mf; a.var[c] = vf;
+        if (a.run_mean) { const float o = a.run_mean[c]; a.run_mean[c] = o + a.avg_rate * (mf - o); }
+        if (a.run_var) { const float o = a.run_var[c]; a.run_var[c] = o + a.avg_rate * (vf - o); }
+      }
+    } else {
+      const float rstd = inv_std(a.var_in[c]);
+      const double rs2 = (double)rstd * t2;              // sum(dz * xhat)
+      const double A = (double)gm * (double)rstd;
+      coef1[ci] = make_float2((float)(-A * (double)rstd * rs2 * g.inv_count), (float)(-A * t1 * g.inv_count));
+      if (rank == 0) {
+        if (a.dbeta) a.dbeta[c] = (float)t1;
+        if (a.dgamma) a.dgamma[c] = (float)rs2;
+      }
+    }
+  }
+  __syncthreads();
+  if (!nk) return;
+
+  // ---- second walk, last batch first
+  float cB[4], cC[4];
+  if (DIR == 0) {
+    const float4 cA = coef0[chA], cBf = coef0[chB];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) { const bool b = (uint32_t)e >= eB; mean[e] = b ? cBf.x : cA.x; scale[e] = b ? cBf.y : cA.y; beta[e] = b ? cBf.z : cA.z; }
+  } else {
+    const float2 cA = coef1[chA], cBf = coef1[chB];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) { const bool b = (uint32_t)e >= eB; cB[e] = b ? cBf.x : cA.x; cC[e] = b ? cBf.y : cA.y; }
+  }
+  for (uint32_t k = kb;; k -= kBatch) {
+    if (DIR == 0) {
+      if (k != kb) {
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) vx[i] = Pack<4>::load(a.x + (off0 + (k + i) * step), drop);      // (only the last batch is short)
+      }
+#pragma unroll
+      for (int h = 0; h < kBatch; h += 4) {
+        Pack<4> ve[EXTRA ? 4 : 1];
+        if (EXTRA) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) if (k + h + i < nk) ve[i] = Pack<4>::load(a.res + (off0 + (k + h + i) * step), drop);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (k + h + i < nk) {
+            Pack<4> o;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              float yb = fmaf(vx[h + i].v[e] - mean[e], scale[e], beta[e]);
+              if (EXTRA) yb += ve[i].v[e];
+              o.v[e] = yb * (yb > 0.0f ? 1.0f : slope);
+            }
+            o.store_stream(a.out + (off0 + (k + h + i) * step));
+          }
+      }
+    } else {
+      if (k != kb) {
+        const float *second = early ? a.dres : a.dy;
+        Pack<4> vm[EXTRA ? kBatch : 1];
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+          const uint32_t off = off0 + (k + i) * step;
+          vx[i] = Pack<4>::load(a.x + off, drop);
+          vd[i] = Pack<4>::load(second + off, drop);
+          if (EXTRA && !early) vm[i] = Pack<4>::load(a.ymask + off, drop);
+        }
+        if (!early) {
+#pragma unroll
+          for (int i = 0; i < kBatch; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float yb = EXTRA ? vm[i].v[e] : fmaf(vx[i].v[e] - mean[e], scale[e], beta[e]);
+              vd[i].v[e] *= yb > 0.0f ? 1.0f : slope;
+            }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i)
+        if (k + i < nk) {
+          const uint32_t off = off0 + (k + i) * step;
+          Pack<4> o;
+          if (a.accumulate) o = Pack<4>::load(a.out + off);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float dx = fmaf(scale[e], vd[i].v[e], fmaf(cB[e], vx[i].v[e] - mean[e], cC[e]));
+            o.v[e] = a.accumulate ? o.v[e] + dx : dx;
+          }
+          o.store_stream(a.out + off);
+          if (EXTRA && !early && a.dres) vd[i].store_stream(a.dres + off);
+        }
+    }
+    if (k == 0) break;
+  }
+}
+
+// ---- host side -------------------------------------------------------------------------------
+
+// Bytes that the resident blocks may have between their two walks.  It wants to fit L2, but a large cluster waits longer
+// for its slowest block and leaves more SMs without a place for a whole cluster: [1024,2048,7,7] takes 199 / 343 us
+// with 64 MB (clusters of 8 / 16), 180 / 298 with 96 MB (4 / 8) and the same with 128 MB.
+constexpr uint64_t kStreamWindow = 96ull << 20;
+
+static bool stream_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, StreamGeom &g)
+{
+  if (dim0 < 4 || (uint64_t)C * dim0 % 4 != 0) return false;
+  uint32_t q = 4; if (dim0 % 2 == 0) q = 2; if (dim0 % 4 == 0) q = 1;      // cb*dim0 must be a multiple of 4
+  // runs of at least 512 bytes, then the channel count that leaves the fewest of the block's threads without a column
+  uint32_t best = 0, best_used = 0;
+  for (uint32_t cb = q; cb <= C && cb <= kStreamChannels && (uint64_t)cb * dim0 <= 4 * kStreamThreads; cb += q) {
+    const uint32_t L4 = cb * dim0 / 4, used = kStreamThreads / L4 * L4;
+    if (best * dim0 >= 128 && used * 16 <= best_used * 17) continue;
+    best = cb; best_used = used;
+  }
+  if (!best) return false;
+  const uint32_t L4 = best * dim0 / 4;
+  g.cb = best; g.units = ceil_div_u32(C, best);
+  g.groups = kStreamThreads / L4; if (g.groups > N) g.groups = N;
+  const uint64_t unit_bytes = 16ull * L4 * N * (dir == 1 ? 2 : 1);
+  uint32_t cl = 1;
+  while (cl < 16 && cl * 2 * g.cb <= kStreamRecords &&
+         ((uint64_t)kStreamBlocks * sm_count() * unit_bytes / cl > kStreamWindow ||
+          (g.units * cl < 2 * kStreamBlocks * sm_count() && N / (cl * 2) >= g.groups * 4))) cl *= 2;
+  g.cluster = cl;
+  g.rows = ceil_div_u32(N, cl);
+  if (g.groups > g.rows) g.groups = g.rows;
+  g.threads = (g.groups * L4 + 31) / 32 * 32;
+  g.inv_count = 1.0 / ((double)dim0 * (double)N);
+  return true;
+}
+
+// Where this kernel is taken (after the register-resident kernel): all rows that the tiled kernel does not serve, and of
+// those it does serve (`tiled_ok`) the short ones and the medium ones of channels that are not too large.  Forward /
+// backward in us, here and on the tiled kernel: [4096,64,16,16] 131 / 225 and 168 / 336, [2048,64,20,20] 111 / 192 and
+// 107 / 202, [256,128,24,24] 35 / 55 and 39 / 68, [1024,64,24,24] 78 / 136 and 68 / 128, [128,256,32,32] 60 / 98 and
+// 56 / 101, [256,256,28,28] 97 / 162 and 84 / 158; residual [256,256,28,28] 138 / 221 and 135 / 232, [1024,64,28,28]
+// 162 / 249 and 132 / 218.
+constexpr uint32_t kStreamShortRow = 512, kStreamMediumRow = 600, kStreamLongRow = 1024;
+bool stream_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
+{
+  StreamGeom g;
+  const uint32_t dim0 = a.plan.dim0;
+  if (!aligned || a.mode != MODE_FUSED || a.world > 1 || !stream_geom(dim0, a.plan.C, a.plan.N, dir, g)) return false;
+  if (!tiled_ok || dim0 <= kStreamShortRow) return true;
+  const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
+  const uint64_t most = (extra ? 1u << 18 : dir == 1 ? 1u << 17 : 1u << 16) * (dim0 <= kStreamMediumRow ? 4ull : 1ull);
+  return dim0 <= kStreamLongRow && (uint64_t)dim0 * a.plan.N <= most;
+}
+
+// ANODE_E_LAUNCH when the device refuses the cluster shape (the caller takes the next kernel that applies).
+int launch_stream(FusedArgs &a, int dir, cudaStream_t stream)
+{
+  StreamGeom g;
+  if (!stream_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, g)) return ANODE_E_LAUNCH;
+  const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
+  // dres may be stored before x is read again only where it is not x itself
+  a.dres_early = a.dres && a.dres != a.x ? 1u : 0u;
+  auto kernel = dir == 0 ? (extra ? bn_stream_kernel<0, true> : bn_stream_kernel<0, false>)
+                         : (extra ? bn_stream_kernel<1, true> : bn_stream_kernel<1, false>);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(g.units * g.cluster);
+  cfg.blockDim = dim3(g.threads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // (as launch_chan)
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = g.cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = g.cluster > 1 ? 2 : 1;
+  if (g.cluster > 8) {
+    // larger than the portable size: asked for once per kernel and device
+    static std::mutex mu;
+    static std::map<std::pair<const void *, int>, bool> allowed;
+    int dev = 0;
+    (void)cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    const auto key = std::make_pair((const void *)kernel, dev);
+    auto it = allowed.find(key);
+    if (it == allowed.end()) {
+      const bool ok = cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+      if (!ok) (void)cudaGetLastError();
+      it = allowed.emplace(key, ok).first;
+    }
+    if (!it->second) return ANODE_E_LAUNCH;
+  }
+  if (cudaLaunchKernelEx(&cfg, kernel, a, g) != cudaSuccess) { (void)cudaGetLastError(); return ANODE_E_LAUNCH; }
+  return ANODE_OK;
+}
+
+}  // namespace anode_b200

@@ -50,7 +50,10 @@ def test_residual_epilogue(tiled, shape, slope):
 def test_outputs_over_inputs(tiled, shape, form):
     """Every output that may take an input's place, and the accumulating write, as the plain kernel does it; a residual
     call between ordinary calls of the same layer on one workspace leaves both right."""
-    ops = tiled
+    outputs_over_inputs(tiled, shape, form, "tiled")
+
+
+def outputs_over_inputs(ops, shape, form, kernel_name):
     d = make_inputs(shape, seed=3, loc=0.5, scale=2.0)
     y_h = np.maximum(np.random.default_rng(4).standard_normal(shape), 0).astype(np.float32)
     c = shape[1]
@@ -71,10 +74,13 @@ def test_outputs_over_inputs(tiled, shape, form):
         assert ws.status() == 0
         return [host(t) for t in (dx, dres, dg, db) if t is not None], ws
 
-    want, _ = call("plain")
-    for _ in range(3):
-        got, ws = call("tiled")
-        for g, w in zip(got, want):
-            assert np.allclose(g, w, rtol=1e-4, atol=1e-5 + 1e-4 * float(np.sqrt(np.mean(w.astype(np.float64) ** 2))))
-        run, _ = run_fused(ops, d, ws=ws)
-        check_layer_own_mask(d, run, "%r between residual calls " % (shape,))
+    try:
+        want, _ = call("plain")
+        for _ in range(3):
+            got, ws = call(kernel_name)
+            for g, w in zip(got, want):
+                assert np.allclose(g, w, rtol=1e-4, atol=1e-5 + 1e-4 * float(np.sqrt(np.mean(w.astype(np.float64) ** 2))))
+            run, _ = run_fused(ops, d, ws=ws)
+            check_layer_own_mask(d, run, "%r between residual calls " % (shape,))
+    finally:
+        ops.set_kernel("auto")
