@@ -7,10 +7,15 @@
 //   elementwise kernels      128-bit grid-stride loops; the channel of a vector comes from one
 //                            division per four elements instead of two per element
 //
+// What bounds them on layers of a few 10 MB: L2 and the gaps between launches.  The composition of thirteen of them on
+// [64,128,28,28] took 134 us with a 64-bit division per vector, two loads in flight in the reductions and ordinary
+// launches, 115 us with none (32-bit ones in the maps), four, and launches that overlap the tail of the one before.
+//
 // Expressions are kept term for term as the reference writes them (e.g. rsqrtf, the
 // "* 2.0f / norm" order), so results differ from its kernels only by summation order.
 #include <cooperative_groups.h>
 
+#include "bn_device.cuh"
 #include "bn_host.h"
 
 namespace cg = cooperative_groups;
@@ -51,6 +56,8 @@ __global__ void __launch_bounds__(kRedThreads) legacy_reduce_kernel(const RedArg
   const uint32_t c = blockIdx.x / cs;
   __shared__ double gather[kClusterMax];
   __shared__ double warp_part[kRedThreads / 32];
+  pdl_wait();
+  pdl_trigger();
 
   float m = 0.f, t = 0.f;
   if (KIND == 1 || KIND == 2 || KIND == 4) m = g.p_mean[c];
@@ -64,24 +71,38 @@ __global__ void __launch_bounds__(kRedThreads) legacy_reduce_kernel(const RedArg
   const uint64_t rs = (uint64_t)g.C * g.dim0;
   const float *pa = g.a + (size_t)c * g.dim0;
   const float *pb = (KIND >= 4) ? g.b + (size_t)c * g.dim0 : nullptr;
-  float acc[2] = {0.f, 0.f};
-  const uint64_t stride = (uint64_t)cs * kRedThreads;
-  for (uint64_t j = (uint64_t)rank * kRedThreads + threadIdx.x; j < total; j += 2 * stride) {
+  // The thread's vectors are j0, j0 + stride, ...; their places are found by walking (row, column) along, without a
+  // division per vector, and kLoads of them are in flight.
+  constexpr int kLoads = KIND >= 4 ? 2 : 4;
+  const uint64_t stride = (uint64_t)cs * kRedThreads, j0 = (uint64_t)rank * kRedThreads + threadIdx.x;
+  const uint64_t row0 = j0 / per_row, drow = stride / per_row;
+  uint32_t col = (uint32_t)(j0 - row0 * per_row);
+  const uint32_t dcol = (uint32_t)(stride - drow * per_row);
+  size_t off = (size_t)row0 * rs + (size_t)col * VEC;
+  const size_t step = (size_t)drow * rs + (size_t)dcol * VEC, wrap = rs - (uint64_t)per_row * VEC;
+  const uint64_t cnt = j0 < total ? (total - j0 - 1) / stride + 1 : 0;
+  float acc[kLoads] = {};
+  for (uint64_t k = 0; k < cnt; k += kLoads) {
+    Pack<VEC> va[kLoads], vb[KIND >= 4 ? kLoads : 1];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const uint64_t jj = j + u * stride;
-      if (jj < total) {
-        const uint32_t row = (uint32_t)(jj / per_row), col = (uint32_t)(jj - (uint64_t)row * per_row);
-        const size_t off = (size_t)row * rs + (size_t)col * VEC;
-        const Pack<VEC> va = Pack<VEC>::load(pa + off);
-        Pack<VEC> vb = va;
-        if (KIND >= 4) vb = Pack<VEC>::load(pb + off);
-#pragma unroll
-        for (int i = 0; i < VEC; ++i) acc[u] += red_term<KIND>(va.v[i], vb.v[i], m, t);
+    for (int u = 0; u < kLoads; ++u) {
+      if (k + u < cnt) {
+        va[u] = Pack<VEC>::load(pa + off);
+        if (KIND >= 4) vb[u] = Pack<VEC>::load(pb + off);
       }
+      off += step; col += dcol;
+      if (col >= per_row) { col -= per_row; off += wrap; }
     }
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u)
+      if (k + u < cnt) {
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) acc[u] += red_term<KIND>(va[u].v[i], KIND >= 4 ? vb[KIND >= 4 ? u : 0].v[i] : 0.f, m, t);
+      }
   }
-  double s = (double)acc[0] + (double)acc[1];
+  double s = 0.0;
+#pragma unroll
+  for (int u = 0; u < kLoads; ++u) s += (double)acc[u];
   s = warp_sum(s);
   if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = s;
   __syncthreads();
@@ -123,10 +144,14 @@ static void launch_reduce(const RedArgs &g, cudaStream_t stream)
   cfg.blockDim = dim3(kRedThreads);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  // The launch may overlap the tail of the kernel before it (every block waits for that kernel's results before it
+  // touches memory): the ops of a composition are a dozen dependent launches of a few microseconds each.
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = cs; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = 2;
   if (vec) (void)cudaLaunchKernelEx(&cfg, legacy_reduce_kernel<KIND, 4, Write>, g);
   else (void)cudaLaunchKernelEx(&cfg, legacy_reduce_kernel<KIND, 1, Write>, g);
 }
@@ -145,13 +170,16 @@ struct MapArgs {
 template <int OP, int VEC, typename Write>
 __global__ void __launch_bounds__(256) legacy_map_kernel(const MapArgs g)
 {
+  pdl_wait();
+  pdl_trigger();
   const uint64_t nvec = g.len / VEC;
+  const bool small = g.len <= 0xffffffffull;      // 32-bit divisions below
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < nvec; j += stride) {
     const size_t off = (size_t)j * VEC;
     float k0 = 0.f, k1 = 0.f;
     if (OP <= 3) {
-      const uint32_t c = (uint32_t)((off / g.dim0) % g.C);    // Index3::Unpack (common.cuh:96-105)
+      const uint32_t c = small ? ((uint32_t)off / g.dim0) % g.C : (uint32_t)((off / g.dim0) % g.C);    // Index3::Unpack (common.cuh:96-105)
       if (OP == 0) k0 = g.p0[c] / g.norm;                     // dmean[c] / norm1   (batch_norm.cu:92)
       if (OP == 1) { k0 = g.p0[c]; k1 = g.p1[c]; }            // dvar[c], mean[c]   (batch_norm.cu:203)
       if (OP == 2) { k0 = g.p0[c]; k1 = rsqrtf(g.p1[c]); }    // mean[c], rsqrt(var[c]) (batch_norm.cu:333)
@@ -187,8 +215,16 @@ static void launch_map(const MapArgs &g, cudaStream_t stream)
   const uint64_t want = (nvec + 255) / 256;
   const uint32_t cap = sm_count() * 16;
   const uint32_t blocks = (uint32_t)(want < cap ? want : cap);
-  if (vec) legacy_map_kernel<OP, 4, Write><<<blocks, 256, 0, stream>>>(g);
-  else legacy_map_kernel<OP, 1, Write><<<blocks, 256, 0, stream>>>(g);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // (as in launch_reduce)
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  if (vec) (void)cudaLaunchKernelEx(&cfg, legacy_map_kernel<OP, 4, Write>, g);
+  else (void)cudaLaunchKernelEx(&cfg, legacy_map_kernel<OP, 1, Write>, g);
 }
 
 static void check_cfg(const KernelConfig *cfg)
