@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kChanThreads, 2) bn_chan_kernel(const FusedArg
   if (DIR == 0) {
     const double md = t0 * g.inv_count;
     mean = (float)md;
-    const float var = (float)(fmax(t1 - t0 * md, 0.0) * g.inv_count + (double)a.epsilon);      // biased, epsilon folded in (batch_norm.cu:160)
+    const float var = (float)(not_below_zero(t1 - t0 * md) * g.inv_count + (double)a.epsilon);      // biased, epsilon folded in (batch_norm.cu:160)
     scale = gm * inv_std(var);
     if (owner) {
       a.mean[c] = mean; a.var[c] = var;

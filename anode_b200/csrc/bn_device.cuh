@@ -120,6 +120,10 @@ template <int VEC> __device__ __forceinline__ Pack<VEC> pack_fill(float f)
 // Negative inputs give -0, NaN stays NaN, -inf gives NaN.
 __device__ __forceinline__ float positive_clip(float x) { return x * (x > 0.0f ? 1.0f : 0.0f); }
 
+// A sum of squared deviations that rounding may have taken below zero.  A NaN stays one (fmax would return the zero):
+// a channel that holds a NaN or an infinity has no variance, and its running average must show it.
+__device__ __forceinline__ double not_below_zero(double v) { return v < 0.0 ? 0.0 : v; }
+
 // ---- reductions ------------------------------------------------------------------------
 struct Moments { float n, mean, m2; };
 

@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kSegThreads) bn_segres_kernel(const FusedArgs 
           t1 = fma(n, m, t1); t2 += (double)colB[gi * Lw + col] + n * m * m;
         }
         const double mean = t1 * inv_rows;
-        colA[col] = (float)mean; colB[col] = (float)fmax(t2 - t1 * mean, 0.0);
+        colA[col] = (float)mean; colB[col] = (float)not_below_zero(t2 - t1 * mean);
       } else {
         double t1 = 0.0, t2 = 0.0;
         for (uint32_t gi = 0; gi < Gr; ++gi) { t1 += (double)colA[gi * Lw + col]; t2 += (double)colB[gi * Lw + col]; }
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(kSegThreads) bn_segres_kernel(const FusedArgs 
       if (lane == 0) {
         if (DIR == 0) {
           const double n = (double)rows * (double)dim0, mean = t1 / (double)dim0;      // equal counts per column
-          part[ci] = make_float4((float)n, (float)mean, (float)fmax(t2 - (double)rows * t1 * mean, 0.0), 0.f);
+          part[ci] = make_float4((float)n, (float)mean, (float)not_below_zero(t2 - (double)rows * t1 * mean), 0.f);
         } else {
           part[ci] = make_float4((float)t1, (float)t2, 0.f, 0.f);
         }
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(kSegThreads) bn_segres_kernel(const FusedArgs 
         if (rank == 0) {
           // word 0 of a forward record is the element count as an exact integer
           uint32_t w0, w1, w2;
-          if (DIR == 0) { const double mean = t1 / t0; w0 = (uint32_t)t0; w1 = __float_as_uint((float)mean); w2 = __float_as_uint((float)fmax(t2 - t1 * mean, 0.0)); }
+          if (DIR == 0) { const double mean = t1 / t0; w0 = (uint32_t)t0; w1 = __float_as_uint((float)mean); w2 = __float_as_uint((float)not_below_zero(t2 - t1 * mean)); }
           else { w0 = __float_as_uint((float)t1); w1 = __float_as_uint((float)t2); w2 = 0u; }
           const unsigned long long e = (unsigned long long)a.epoch << 32;
           for (uint32_t r = 0; r < a.world; ++r) {
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kSegThreads) bn_segres_kernel(const FusedArgs 
         }
       }
       if (DIR == 0) {
-        const double mean = t1 / t0, m2 = fmax(t2 - t1 * mean, 0.0);
+        const double mean = t1 / t0, m2 = not_below_zero(t2 - t1 * mean);
         const float mf = (float)mean;
         const float vf = (float)(m2 / t0 + (double)a.epsilon);        // biased, epsilon folded in (batch_norm.cu:160)
         coef[8 * ci + 0] = mf; coef[8 * ci + 1] = gm * inv_std(vf); coef[8 * ci + 2] = bt;

@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamBlocks) bn_stream_kerne
     if (DIR == 0) {
       const double md = t1 * g.inv_count;
       const float mf = (float)md;
-      const float vf = (float)(fmax(t2 - t1 * md, 0.0) * g.inv_count + (double)a.epsilon);      // biased, epsilon folded in (batch_norm.cu:160)
+      const float vf = (float)(not_below_zero(t2 - t1 * md) * g.inv_count + (double)a.epsilon);      // biased, epsilon folded in (batch_norm.cu:160)
       coef0[ci] = make_float4(mf, gm * inv_std(vf), bt, 0.f);
       if (rank == 0) {
         a.mean[c] = mf; a.var[c] = vf;
