@@ -5,6 +5,10 @@
 // linked against nothing but Python and torch, and a library chosen at run time is honoured.
 //
 // Arguments mirror anode_b200/ops.py, which keeps the public signatures, defaults and error types.
+// torch reports some conditions by C++ exceptions (no driver, a tensor without storage inside a function transform, a
+// sparse one): every function turns them into Python errors (HANDLE_TH_ERRORS), and nothing is asked of torch or CUDA once
+// an argument was refused.
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -33,16 +37,22 @@ typedef int (*BwdActFn)(uint32_t, uint32_t, uint32_t, float, int, In, In, In, In
 typedef int (*BwdAddFn)(uint32_t, uint32_t, uint32_t, float, int, In, In, In, In, In, In, In, Out, Out, Out, Out, void *, size_t, const KernelConfig *, void *);
 typedef int (*InferFn)(uint32_t, uint32_t, uint32_t, float, In, In, In, In, In, Out, const KernelConfig *, void *);
 
-// One call's arguments: the first failure sets the Python error and every later access is harmless.
+// The interpreter's lock is given back while this lives (exceptions included).
+struct Unlocked {
+  PyThreadState *state = PyEval_SaveThread();
+  ~Unlocked() { PyEval_RestoreThread(state); }
+};
+
+// One call's arguments: the first failure sets the Python error and every later access does nothing.
 struct Args {
   PyObject *const *v;
   bool ok = true;
 
   const at::Tensor *tensor(int i, bool null_ok)
   {
-    if (v[i] == Py_None && null_ok) return nullptr;
+    if (!ok || (v[i] == Py_None && null_ok)) return nullptr;
     if (!THPVariable_Check(v[i])) {
-      if (ok) PyErr_SetString(PyExc_ValueError, "expected a contiguous float32 CUDA tensor");
+      PyErr_SetString(PyExc_ValueError, "expected a contiguous float32 CUDA tensor");
       ok = false;
       return nullptr;
     }
@@ -54,7 +64,7 @@ struct Args {
     const at::Tensor *t = tensor(i, null_ok);
     if (!t) return nullptr;
     if (!(t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous())) {
-      if (ok) PyErr_SetString(PyExc_ValueError, "expected a contiguous float32 CUDA tensor");
+      PyErr_SetString(PyExc_ValueError, "expected a contiguous float32 CUDA tensor");
       ok = false;
       return nullptr;
     }
@@ -62,18 +72,21 @@ struct Args {
   }
   float f(int i)
   {
+    if (!ok) return 0.f;
     const double d = PyFloat_AsDouble(v[i]);
     if (d == -1.0 && PyErr_Occurred()) ok = false;
     return (float)d;
   }
   int truth(int i)
   {
+    if (!ok) return 0;
     const int r = PyObject_IsTrue(v[i]);
     if (r < 0) ok = false;
     return r > 0;
   }
   size_t size(int i)
   {
+    if (!ok) return 0;
     const size_t r = PyLong_AsSize_t(v[i]);
     if (r == (size_t)-1 && PyErr_Occurred()) ok = false;
     return r;
@@ -86,6 +99,7 @@ struct Args {
   // a torch stream, or None for the current one
   void *stream(int i)
   {
+    if (!ok) return nullptr;
     if (v[i] == Py_None) return c10::cuda::getCurrentCUDAStream().stream();
     PyObject *h = PyObject_GetAttrString(v[i], "cuda_stream");
     if (!h) { ok = false; return nullptr; }
@@ -116,13 +130,13 @@ struct Args {
       if (!same) {
         PyObject *want = PyList_New(0);
         for (int64_t k = 0; k + 2 < nd; ++k) { PyObject *e = PyLong_FromLongLong(k); PyList_Append(want, e); Py_DECREF(e); }
-        if (ok) PyErr_Format(PyExc_ValueError, "axes must be %R for a %d-D batch array", want, (int)(nd - 2));
+        PyErr_Format(PyExc_ValueError, "axes must be %R for a %d-D batch array", want, (int)(nd - 2));
         Py_DECREF(want);
         ok = false;
         return;
       }
     }
-    if (nd < 2) { if (ok) PyErr_SetString(PyExc_IndexError, "expected an array [N, C, *spatial]"); ok = false; return; }
+    if (nd < 2) { PyErr_SetString(PyExc_IndexError, "expected an array [N, C, *spatial]"); ok = false; return; }
     uint64_t d0 = 1;
     for (int64_t k = 2; k < nd; ++k) d0 *= (uint64_t)t->size(k);
     d[0] = (uint32_t)d0; d[1] = (uint32_t)t->size(1); d[2] = (uint32_t)t->size(0);
@@ -146,6 +160,7 @@ const KernelConfig kDefaultCfg = {1024, 148 * 32};     // ops.py's default launc
 // fwd(axes, epsilon, avg_rate, x, residual, y, mean, var, avg_mean, avg_var, gamma, beta, relu, neg_slope | None, ws, ws_bytes, stream)
 PyObject *py_fwd(PyObject *, PyObject *const *v, Py_ssize_t n)
 {
+  HANDLE_TH_ERRORS
   if (!want_args(n, 17)) return nullptr;
   Args a{v};
   uint32_t d[3] = {0, 0, 0};
@@ -163,17 +178,20 @@ PyObject *py_fwd(PyObject *, PyObject *const *v, Py_ssize_t n)
   const int which = add ? F_FWD_ADD : act ? F_FWD_ACT : F_FWD;
   if (!bound(which)) return nullptr;
   int rc;
-  Py_BEGIN_ALLOW_THREADS
-  if (add) rc = ((FwdAddFn)g_fn[which])(d[0], d[1], d[2], eps, rate, slope, x, res, gamma, beta, y, mean, var, rm, rv, ws, bytes, &kDefaultCfg, s);
-  else if (act) rc = ((FwdActFn)g_fn[which])(d[0], d[1], d[2], eps, rate, slope, x, gamma, beta, y, mean, var, rm, rv, ws, bytes, &kDefaultCfg, s);
-  else rc = ((FwdFn)g_fn[which])(d[0], d[1], d[2], eps, rate, relu, x, gamma, beta, y, mean, var, rm, rv, ws, bytes, &kDefaultCfg, s);
-  Py_END_ALLOW_THREADS
+  {
+    Unlocked unlocked;
+    if (add) rc = ((FwdAddFn)g_fn[which])(d[0], d[1], d[2], eps, rate, slope, x, res, gamma, beta, y, mean, var, rm, rv, ws, bytes, &kDefaultCfg, s);
+    else if (act) rc = ((FwdActFn)g_fn[which])(d[0], d[1], d[2], eps, rate, slope, x, gamma, beta, y, mean, var, rm, rv, ws, bytes, &kDefaultCfg, s);
+    else rc = ((FwdFn)g_fn[which])(d[0], d[1], d[2], eps, rate, relu, x, gamma, beta, y, mean, var, rm, rv, ws, bytes, &kDefaultCfg, s);
+  }
   return PyLong_FromLong(rc);
+  END_HANDLE_TH_ERRORS
 }
 
 // bwd(axes, dy, x, y | None, mean, var, dx, dresidual, gamma, beta, dgamma, dbeta, relu, neg_slope | None, accumulate, ws, ws_bytes, stream)
 PyObject *py_bwd(PyObject *, PyObject *const *v, Py_ssize_t n)
 {
+  HANDLE_TH_ERRORS
   if (!want_args(n, 18)) return nullptr;
   Args a{v};
   uint32_t d[3] = {0, 0, 0};
@@ -190,17 +208,20 @@ PyObject *py_bwd(PyObject *, PyObject *const *v, Py_ssize_t n)
   const int which = add ? F_BWD_ADD : act ? F_BWD_ACT : F_BWD;
   if (!bound(which)) return nullptr;
   int rc;
-  Py_BEGIN_ALLOW_THREADS
-  if (add) rc = ((BwdAddFn)g_fn[which])(d[0], d[1], d[2], slope, acc, dy, x, y, mean, var, gamma, beta, dx, dres, dg, db, ws, bytes, &kDefaultCfg, s);
-  else if (act) rc = ((BwdActFn)g_fn[which])(d[0], d[1], d[2], slope, acc, dy, x, mean, var, gamma, beta, dx, dg, db, ws, bytes, &kDefaultCfg, s);
-  else rc = ((BwdFn)g_fn[which])(d[0], d[1], d[2], relu, acc, dy, x, mean, var, gamma, beta, dx, dg, db, ws, bytes, &kDefaultCfg, s);
-  Py_END_ALLOW_THREADS
+  {
+    Unlocked unlocked;
+    if (add) rc = ((BwdAddFn)g_fn[which])(d[0], d[1], d[2], slope, acc, dy, x, y, mean, var, gamma, beta, dx, dres, dg, db, ws, bytes, &kDefaultCfg, s);
+    else if (act) rc = ((BwdActFn)g_fn[which])(d[0], d[1], d[2], slope, acc, dy, x, mean, var, gamma, beta, dx, dg, db, ws, bytes, &kDefaultCfg, s);
+    else rc = ((BwdFn)g_fn[which])(d[0], d[1], d[2], relu, acc, dy, x, mean, var, gamma, beta, dx, dg, db, ws, bytes, &kDefaultCfg, s);
+  }
   return PyLong_FromLong(rc);
+  END_HANDLE_TH_ERRORS
 }
 
 // infer(axes, x, mean, var, y, gamma, beta, neg_slope, stream)
 PyObject *py_infer(PyObject *, PyObject *const *v, Py_ssize_t n)
 {
+  HANDLE_TH_ERRORS
   if (!want_args(n, 9)) return nullptr;
   Args a{v};
   uint32_t d[3] = {0, 0, 0};
@@ -211,16 +232,19 @@ PyObject *py_infer(PyObject *, PyObject *const *v, Py_ssize_t n)
   void *s = a.stream(8);
   if (!a.ok || !bound(F_INFER)) return nullptr;
   int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = ((InferFn)g_fn[F_INFER])(d[0], d[1], d[2], slope, x, mean, var, gamma, beta, y, &kDefaultCfg, s);
-  Py_END_ALLOW_THREADS
+  {
+    Unlocked unlocked;
+    rc = ((InferFn)g_fn[F_INFER])(d[0], d[1], d[2], slope, x, mean, var, gamma, beta, y, &kDefaultCfg, s);
+  }
   return PyLong_FromLong(rc);
+  END_HANDLE_TH_ERRORS
 }
 
 // packed(address, axes, like, tensors, epsilon | None, stream): one of the reference's own entry points.  `like` gives
 // (dim0, dim1, dim2) when axes is not False, else the element count; tensors are the pointers in the order of the C call.
 PyObject *py_packed(PyObject *, PyObject *const *v, Py_ssize_t n)
 {
+  HANDLE_TH_ERRORS
   if (!want_args(n, 6)) return nullptr;
   void *fn = PyLong_AsVoidPtr(v[0]);
   if (PyErr_Occurred()) return nullptr;
@@ -233,8 +257,8 @@ PyObject *py_packed(PyObject *, PyObject *const *v, Py_ssize_t n)
   Args t{items};
   void *p[5] = {};
   for (Py_ssize_t i = 0; i < k; ++i) p[i] = t.ptr((int)i);
-  void *s = a.stream(5);
   if (!t.ok) return nullptr;
+  void *s = a.stream(5);
   const KernelConfig *cfg = &kDefaultCfg;
   const bool flat = v[1] == Py_False, with_eps = v[4] != Py_None;
   uint32_t d[3] = {0, 0, 0};
@@ -245,21 +269,24 @@ PyObject *py_packed(PyObject *, PyObject *const *v, Py_ssize_t n)
   if ((flat && k > 3) || (with_eps && k != 3)) { PyErr_SetString(PyExc_TypeError, "no entry point takes these arguments"); return nullptr; }
   typedef void *P;
   typedef const KernelConfig *K;
-  Py_BEGIN_ALLOW_THREADS
-  if (flat && k == 2) ((void (*)(uint32_t, P, P, K, P))fn)(d[0], p[0], p[1], cfg, s);
-  else if (flat) ((void (*)(uint32_t, P, P, P, K, P))fn)(d[0], p[0], p[1], p[2], cfg, s);
-  else if (with_eps) ((void (*)(uint32_t, uint32_t, uint32_t, float, P, P, P, K, P))fn)(d[0], d[1], d[2], eps, p[0], p[1], p[2], cfg, s);
-  else if (k == 2) ((void (*)(uint32_t, uint32_t, uint32_t, P, P, K, P))fn)(d[0], d[1], d[2], p[0], p[1], cfg, s);
-  else if (k == 3) ((void (*)(uint32_t, uint32_t, uint32_t, P, P, P, K, P))fn)(d[0], d[1], d[2], p[0], p[1], p[2], cfg, s);
-  else if (k == 4) ((void (*)(uint32_t, uint32_t, uint32_t, P, P, P, P, K, P))fn)(d[0], d[1], d[2], p[0], p[1], p[2], p[3], cfg, s);
-  else ((void (*)(uint32_t, uint32_t, uint32_t, P, P, P, P, P, K, P))fn)(d[0], d[1], d[2], p[0], p[1], p[2], p[3], p[4], cfg, s);
-  Py_END_ALLOW_THREADS
+  {
+    Unlocked unlocked;
+    if (flat && k == 2) ((void (*)(uint32_t, P, P, K, P))fn)(d[0], p[0], p[1], cfg, s);
+    else if (flat) ((void (*)(uint32_t, P, P, P, K, P))fn)(d[0], p[0], p[1], p[2], cfg, s);
+    else if (with_eps) ((void (*)(uint32_t, uint32_t, uint32_t, float, P, P, P, K, P))fn)(d[0], d[1], d[2], eps, p[0], p[1], p[2], cfg, s);
+    else if (k == 2) ((void (*)(uint32_t, uint32_t, uint32_t, P, P, K, P))fn)(d[0], d[1], d[2], p[0], p[1], cfg, s);
+    else if (k == 3) ((void (*)(uint32_t, uint32_t, uint32_t, P, P, P, K, P))fn)(d[0], d[1], d[2], p[0], p[1], p[2], cfg, s);
+    else if (k == 4) ((void (*)(uint32_t, uint32_t, uint32_t, P, P, P, P, K, P))fn)(d[0], d[1], d[2], p[0], p[1], p[2], p[3], cfg, s);
+    else ((void (*)(uint32_t, uint32_t, uint32_t, P, P, P, P, P, K, P))fn)(d[0], d[1], d[2], p[0], p[1], p[2], p[3], p[4], cfg, s);
+  }
   Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
 }
 
 // bind({name: address}): the C ABI's functions
 PyObject *py_bind(PyObject *, PyObject *const *v, Py_ssize_t n)
 {
+  HANDLE_TH_ERRORS
   if (!want_args(n, 1)) return nullptr;
   for (int i = 0; i < F_COUNT; ++i) {
     PyObject *e = PyDict_GetItemString(v[0], kNames[i]);
@@ -268,6 +295,7 @@ PyObject *py_bind(PyObject *, PyObject *const *v, Py_ssize_t n)
     if (PyErr_Occurred()) return nullptr;
   }
   Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
 }
 
 PyMethodDef kMethods[] = {

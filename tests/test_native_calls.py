@@ -1,0 +1,67 @@
+"""The native call module (csrc/bn_py.cpp) refuses what it cannot take with a Python error, on any machine: nothing of a
+refused call reaches CUDA, and no C++ exception leaves the module."""
+import pytest
+import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+
+from anode_b200 import ops
+
+
+class Scratch:
+    """Stands in for ops.Workspace, whose constructor needs a device."""
+    def __init__(self):
+        self.buf, self.bytes = torch.empty(256, dtype=torch.uint8), 256
+
+
+def calls(x, v):
+    """Every op that goes through the module, on activations x and per-channel vectors v."""
+    ax, f, b, r = [0, 1], ops.BatchNormalize2dFusedOp.apply, ops.BatchNormalize2dBwdFusedOp.apply, ops.BatchNormalize2dAddActFusedOp
+    ws = Scratch()
+    return {
+        "fwd": lambda: f(ax, 1e-5, 0.1, x, x, v, v, workspace=ws),
+        "fwd leaky": lambda: f(ax, 1e-5, 0.1, x, x, v, v, workspace=ws, neg_slope=0.1),
+        "bwd": lambda: b(ax, x, x, v, v, x, workspace=ws),
+        "residual fwd": lambda: r.apply(ax, 1e-5, 0.1, x, x, x, v, v, workspace=ws),
+        "residual bwd": lambda: r.adjoint(ax, x, x, x, v, v, x, workspace=ws),
+        "infer": lambda: ops.BatchNormalize2dActInferOp.apply(ax, x, v, v, x),
+        "mean": lambda: ops.BatchMean2dOp.apply(ax, x, v),
+        "mean bwd": lambda: ops.BatchMean2dBwdOp.apply(ax, v, x, x),
+        "var": lambda: ops.BatchVariance2dOp.apply(ax, 1e-5, x, v, v),
+        "var bwd": lambda: ops.BatchVariance2dBwdOp.apply(ax, v, x, v, x),
+        "var bwd mean": lambda: ops.BatchVariance2dBwdMeanOp.apply(ax, v, x, v, v),
+        "norm": lambda: ops.BatchNormalize2dOp.apply(ax, x, v, v, x),
+        "norm bwd": lambda: ops.BatchNormalize2dBwdOp.apply(ax, x, v, x),
+        "norm bwd var": lambda: ops.BatchNormalize2dBwdVarianceOp.apply(ax, x, x, v, v, v),
+        "clip": lambda: ops.PositiveClipOp.apply(x, x),
+        "clip bwd": lambda: ops.PositiveClipBwdOp.apply(x, x, x),
+        "join": lambda: ops.FlatJoinOp.apply(x, x, x),
+    }
+
+
+NAMES = sorted(calls(None, None))
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_host_tensors_are_refused_before_anything_is_asked_of_cuda(name):
+    with pytest.raises(ValueError, match="contiguous float32 CUDA tensor"):
+        calls(torch.zeros(2, 3, 4, 4), torch.zeros(3))[name]()
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_tensors_without_storage_raise(name):
+    with FakeTensorMode():
+        x, v = torch.empty(5, 2, 3, 4, 4, device="cuda"), torch.empty(5, 3, device="cuda")
+
+        def one(x, v):
+            return calls(x, v)[name]()
+        with pytest.raises(RuntimeError):
+            torch.func.vmap(one)(x, v)
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="needs a machine without a driver")
+@pytest.mark.filterwarnings("ignore:Accessing the data pointer of FakeTensor")
+def test_no_driver_is_an_error_not_an_abort():
+    with FakeTensorMode():
+        x, v = torch.empty(2, 3, 4, 4, device="cuda"), torch.empty(3, device="cuda")
+    with pytest.raises(RuntimeError):
+        ops.BatchNormalize2dActInferOp.apply([0, 1], x, v, v, x)      # asks for the current stream
