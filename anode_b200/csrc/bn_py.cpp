@@ -240,44 +240,101 @@ PyObject *py_infer(PyObject *, PyObject *const *v, Py_ssize_t n)
   END_HANDLE_TH_ERRORS
 }
 
-// packed(address, axes, like, tensors, epsilon | None, stream): one of the reference's own entry points.  `like` gives
-// (dim0, dim1, dim2) when axes is not False, else the element count; tensors are the pointers in the order of the C call.
+// The tensors of one of the reference's own entry points: `lo` to `hi` of them, all required (these entry points have no
+// status, and their kernels read and write what they are given).
+struct Pointers {
+  void *p[5] = {};
+  Py_ssize_t k = 0;
+
+  bool take(PyObject *tuple, Py_ssize_t lo, Py_ssize_t hi)
+  {
+    if (!PyTuple_Check(tuple)) { PyErr_SetString(PyExc_TypeError, "tensors: a tuple"); return false; }
+    k = PyTuple_GET_SIZE(tuple);
+    if (k < lo || k > hi) { PyErr_Format(PyExc_TypeError, "%zd to %zd tensors", lo, hi); return false; }
+    PyObject *items[5];
+    for (Py_ssize_t i = 0; i < k; ++i) items[i] = PyTuple_GET_ITEM(tuple, i);
+    Args t{items};
+    for (Py_ssize_t i = 0; i < k; ++i) {
+      p[i] = t.ptr((int)i, false);
+      if (t.ok && !p[i] && THPVariable_Unpack(items[i]).numel() != 0) {
+        PyErr_SetString(PyExc_RuntimeError, "a tensor has no storage");
+        t.ok = false;
+      }
+    }
+    return t.ok;
+  }
+};
+typedef void *P;
+typedef const KernelConfig *K;
+
+// The form of the C call is the function's, never read off the arguments' values.
+// flat(address, tensors, stream): element count (of the first tensor) and 2 or 3 arrays
+PyObject *py_flat(PyObject *, PyObject *const *v, Py_ssize_t n)
+{
+  HANDLE_TH_ERRORS
+  if (!want_args(n, 3)) return nullptr;
+  void *fn = PyLong_AsVoidPtr(v[0]);
+  if (PyErr_Occurred()) return nullptr;
+  Args a{v};
+  Pointers q;
+  if (!q.take(v[1], 2, 3)) return nullptr;
+  const uint32_t len = (uint32_t)THPVariable_Unpack(PyTuple_GET_ITEM(v[1], 0)).numel();
+  void *s = a.stream(2);
+  if (!a.ok) return nullptr;
+  const KernelConfig *cfg = &kDefaultCfg;
+  {
+    Unlocked unlocked;
+    if (q.k == 2) ((void (*)(uint32_t, P, P, K, P))fn)(len, q.p[0], q.p[1], cfg, s);
+    else ((void (*)(uint32_t, P, P, P, K, P))fn)(len, q.p[0], q.p[1], q.p[2], cfg, s);
+  }
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+// packed(address, axes, like, tensors, stream): the dimensions of `like` and 2 to 5 arrays
 PyObject *py_packed(PyObject *, PyObject *const *v, Py_ssize_t n)
+{
+  HANDLE_TH_ERRORS
+  if (!want_args(n, 5)) return nullptr;
+  void *fn = PyLong_AsVoidPtr(v[0]);
+  if (PyErr_Occurred()) return nullptr;
+  Args a{v};
+  uint32_t d[3] = {0, 0, 0};
+  a.dims(1, 2, d);
+  Pointers q;
+  if (!a.ok || !q.take(v[3], 2, 5)) return nullptr;
+  void *s = a.stream(4);
+  if (!a.ok) return nullptr;
+  const KernelConfig *cfg = &kDefaultCfg;
+  {
+    Unlocked unlocked;
+    if (q.k == 2) ((void (*)(uint32_t, uint32_t, uint32_t, P, P, K, P))fn)(d[0], d[1], d[2], q.p[0], q.p[1], cfg, s);
+    else if (q.k == 3) ((void (*)(uint32_t, uint32_t, uint32_t, P, P, P, K, P))fn)(d[0], d[1], d[2], q.p[0], q.p[1], q.p[2], cfg, s);
+    else if (q.k == 4) ((void (*)(uint32_t, uint32_t, uint32_t, P, P, P, P, K, P))fn)(d[0], d[1], d[2], q.p[0], q.p[1], q.p[2], q.p[3], cfg, s);
+    else ((void (*)(uint32_t, uint32_t, uint32_t, P, P, P, P, P, K, P))fn)(d[0], d[1], d[2], q.p[0], q.p[1], q.p[2], q.p[3], q.p[4], cfg, s);
+  }
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+// packed_eps(address, axes, like, tensors, epsilon, stream): the dimensions of `like`, epsilon and 3 arrays
+PyObject *py_packed_eps(PyObject *, PyObject *const *v, Py_ssize_t n)
 {
   HANDLE_TH_ERRORS
   if (!want_args(n, 6)) return nullptr;
   void *fn = PyLong_AsVoidPtr(v[0]);
   if (PyErr_Occurred()) return nullptr;
   Args a{v};
-  if (!PyTuple_Check(v[3])) { PyErr_SetString(PyExc_TypeError, "tensors: a tuple"); return nullptr; }
-  const Py_ssize_t k = PyTuple_GET_SIZE(v[3]);
-  if (k < 2 || k > 5 || !fn) { PyErr_SetString(PyExc_TypeError, "2 to 5 tensors"); return nullptr; }
-  PyObject *items[5];
-  for (Py_ssize_t i = 0; i < k; ++i) items[i] = PyTuple_GET_ITEM(v[3], i);
-  Args t{items};
-  void *p[5] = {};
-  for (Py_ssize_t i = 0; i < k; ++i) p[i] = t.ptr((int)i);
-  if (!t.ok) return nullptr;
-  void *s = a.stream(5);
-  const KernelConfig *cfg = &kDefaultCfg;
-  const bool flat = v[1] == Py_False, with_eps = v[4] != Py_None;
   uint32_t d[3] = {0, 0, 0};
-  if (flat) { const at::Tensor *x = a.tensor(2, false); if (x) d[0] = (uint32_t)x->numel(); }
-  else a.dims(1, 2, d);
-  const float eps = with_eps ? a.f(4) : 0.f;
+  a.dims(1, 2, d);
+  const float eps = a.f(4);
+  Pointers q;
+  if (!a.ok || !q.take(v[3], 3, 3)) return nullptr;
+  void *s = a.stream(5);
   if (!a.ok) return nullptr;
-  if ((flat && k > 3) || (with_eps && k != 3)) { PyErr_SetString(PyExc_TypeError, "no entry point takes these arguments"); return nullptr; }
-  typedef void *P;
-  typedef const KernelConfig *K;
   {
     Unlocked unlocked;
-    if (flat && k == 2) ((void (*)(uint32_t, P, P, K, P))fn)(d[0], p[0], p[1], cfg, s);
-    else if (flat) ((void (*)(uint32_t, P, P, P, K, P))fn)(d[0], p[0], p[1], p[2], cfg, s);
-    else if (with_eps) ((void (*)(uint32_t, uint32_t, uint32_t, float, P, P, P, K, P))fn)(d[0], d[1], d[2], eps, p[0], p[1], p[2], cfg, s);
-    else if (k == 2) ((void (*)(uint32_t, uint32_t, uint32_t, P, P, K, P))fn)(d[0], d[1], d[2], p[0], p[1], cfg, s);
-    else if (k == 3) ((void (*)(uint32_t, uint32_t, uint32_t, P, P, P, K, P))fn)(d[0], d[1], d[2], p[0], p[1], p[2], cfg, s);
-    else if (k == 4) ((void (*)(uint32_t, uint32_t, uint32_t, P, P, P, P, K, P))fn)(d[0], d[1], d[2], p[0], p[1], p[2], p[3], cfg, s);
-    else ((void (*)(uint32_t, uint32_t, uint32_t, P, P, P, P, P, K, P))fn)(d[0], d[1], d[2], p[0], p[1], p[2], p[3], p[4], cfg, s);
+    ((void (*)(uint32_t, uint32_t, uint32_t, float, P, P, P, K, P))fn)(d[0], d[1], d[2], eps, q.p[0], q.p[1], q.p[2], &kDefaultCfg, s);
   }
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
@@ -303,7 +360,9 @@ PyMethodDef kMethods[] = {
     {"fwd", (PyCFunction)(void *)py_fwd, METH_FASTCALL, nullptr},
     {"bwd", (PyCFunction)(void *)py_bwd, METH_FASTCALL, nullptr},
     {"infer", (PyCFunction)(void *)py_infer, METH_FASTCALL, nullptr},
+    {"flat", (PyCFunction)(void *)py_flat, METH_FASTCALL, nullptr},
     {"packed", (PyCFunction)(void *)py_packed, METH_FASTCALL, nullptr},
+    {"packed_eps", (PyCFunction)(void *)py_packed_eps, METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", "Fast paths of anode_b200.ops into the C ABI.", -1, kMethods};
 

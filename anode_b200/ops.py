@@ -65,10 +65,20 @@ def dims_of(x, axes=None):
     return d0, int(x.shape[1]), int(x.shape[0])
 
 
-def _packed(name, axes, x, tensors, stream, epsilon=None):
-    """One of the reference's entry points on [N, C, *spatial] arrays (axes False: on flat arrays).  The launch hint
-    (`cfg` of the ops) is not passed on: the kernels choose their own launch shapes."""
-    native().packed(_lib.address(name), axes, x, tensors, epsilon, stream)
+def _packed(name, axes, x, tensors, stream):
+    """One of the reference's entry points on [N, C, *spatial] arrays.  The launch hint (`cfg` of the ops) is not passed
+    on: the kernels choose their own launch shapes."""
+    native().packed(_lib.address(name), axes, x, tensors, stream)
+
+
+def _packed_eps(name, axes, x, tensors, epsilon, stream):
+    """The same with an epsilon between dimensions and arrays."""
+    native().packed_eps(_lib.address(name), axes, x, tensors, epsilon, stream)
+
+
+def _flat(name, tensors, stream):
+    """The same on flat arrays of the first one's length."""
+    native().flat(_lib.address(name), tensors, stream)
 
 
 # --------------------------------------------------------------------------------------------
@@ -102,7 +112,7 @@ class BatchVariance2dOp:
     def apply(axes, epsilon, x, mean, var, cap=WriteCap.Assign, cfg=None, stream=None):
         if cap is not WriteCap.Assign:
             raise NotImplementedError("BatchVariance2dOp: Accumulate (unimplemented in the reference)")
-        _packed("anode_gpu_batch_var_3d1_packed_f32", axes, x, (x, mean, var), stream, epsilon)
+        _packed_eps("anode_gpu_batch_var_3d1_packed_f32", axes, x, (x, mean, var), epsilon, stream)
         return var
 
 
@@ -197,7 +207,7 @@ class PositiveClipOp:
     is the in-place form of PositiveClipClobberOp (:8584-8671)."""
     @staticmethod
     def apply(x, y, cfg=None, stream=None):
-        _packed("anode_gpu_positive_clip_flat_map_f32", False, x, (x, y), stream)
+        _flat("anode_gpu_positive_clip_flat_map_f32", (x, y), stream)
         return y
 
 
@@ -205,7 +215,7 @@ class PositiveClipBwdOp:
     """src/ops_gpu.rs:8499-8582: dx = dy * (y > 0); `dx is dy` is the clobber form (:8673-8755)."""
     @staticmethod
     def apply(dy, y, dx, cfg=None, stream=None):
-        _packed("anode_gpu_positive_clip_flat_map_bwd_f32", False, dy, (dy, y, dx), stream)
+        _flat("anode_gpu_positive_clip_flat_map_bwd_f32", (dy, y, dx), stream)
         return dx
 
 
@@ -213,7 +223,7 @@ class FlatJoinOp:
     """src/ops_gpu.rs:8169-8261: y = x1 * step(x2) (routines_gpu/flat_join.cu:50-60)."""
     @staticmethod
     def apply(x1, x2, y, cfg=None, stream=None):
-        _packed("anode_gpu_M1_copy_map_M2_unit_step_map_R_product_reduce_flat_join_f32", False, x1, (x1, x2, y), stream)
+        _flat("anode_gpu_M1_copy_map_M2_unit_step_map_R_product_reduce_flat_join_f32", (x1, x2, y), stream)
         return y
 
 

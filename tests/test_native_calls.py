@@ -65,3 +65,22 @@ def test_no_driver_is_an_error_not_an_abort():
         x, v = torch.empty(2, 3, 4, 4, device="cuda"), torch.empty(3, device="cuda")
     with pytest.raises(RuntimeError):
         ops.BatchNormalize2dActInferOp.apply([0, 1], x, v, v, x)      # asks for the current stream
+
+
+def test_the_form_of_a_call_never_depends_on_its_arguments():
+    """Values that once chose between the C calls' forms are refused like any other wrong ones."""
+    x, v = torch.zeros(2, 3, 4, 4), torch.zeros(3)
+    with pytest.raises(TypeError):
+        ops.BatchVariance2dOp.apply([0, 1], None, x, v, v)             # no epsilon
+    with pytest.raises(TypeError):
+        ops.BatchMean2dOp.apply(False, x, v)                          # no axes: not the flat form
+    with pytest.raises(TypeError):
+        ops.BatchNormalize2dBwdOp.apply(False, x, v, x)
+
+
+@pytest.mark.parametrize("call", [lambda x, v: ops.BatchMean2dOp.apply([0, 1], x, None), lambda x, v: ops.PositiveClipOp.apply(None, x),
+                                  lambda x, v: ops.BatchNormalize2dOp.apply([0, 1], x, None, v, x)])
+def test_the_references_entry_points_take_no_missing_array(call):
+    """They have no status to answer with: a missing array would be read."""
+    with pytest.raises((ValueError, AttributeError)):
+        call(torch.zeros(2, 3, 4, 4), torch.zeros(3))
