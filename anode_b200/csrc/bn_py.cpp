@@ -116,25 +116,18 @@ struct Args {
     if (!t) return;
     const int64_t nd = t->dim();
     if (axes >= 0 && v[axes] != Py_None) {
-      bool same = true;
-      const Py_ssize_t n = PySequence_Size(v[axes]);
-      if (n < 0) { ok = false; return; }
-      same = n == (nd > 2 ? nd - 2 : 0);
-      for (Py_ssize_t k = 0; same && k < n; ++k) {
-        PyObject *e = PySequence_GetItem(v[axes], k);
-        if (!e) { ok = false; return; }
-        same = PyLong_AsLong(e) == (long)k;
-        Py_DECREF(e);
-        if (PyErr_Occurred()) PyErr_Clear();
+      // any iterable whose items equal 0, 1, ...
+      PyObject *got = PySequence_List(v[axes]), *want = got ? PyList_New(0) : nullptr;
+      int same = want ? 1 : -1;
+      for (int64_t k = 0; same > 0 && k + 2 < nd; ++k) {
+        PyObject *e = PyLong_FromLongLong(k);
+        if (!e || PyList_Append(want, e)) same = -1;
+        Py_XDECREF(e);
       }
-      if (!same) {
-        PyObject *want = PyList_New(0);
-        for (int64_t k = 0; k + 2 < nd; ++k) { PyObject *e = PyLong_FromLongLong(k); PyList_Append(want, e); Py_DECREF(e); }
-        PyErr_Format(PyExc_ValueError, "axes must be %R for a %d-D batch array", want, (int)(nd - 2));
-        Py_DECREF(want);
-        ok = false;
-        return;
-      }
+      if (same > 0) same = PyObject_RichCompareBool(got, want, Py_EQ);
+      if (same == 0) PyErr_Format(PyExc_ValueError, "axes must be %R for a %d-D batch array", want, (int)(nd - 2));
+      Py_XDECREF(got); Py_XDECREF(want);
+      if (same <= 0) { ok = false; return; }
     }
     if (nd < 2) { PyErr_SetString(PyExc_IndexError, "expected an array [N, C, *spatial]"); ok = false; return; }
     uint64_t d0 = 1;
@@ -167,9 +160,9 @@ PyObject *py_fwd(PyObject *, PyObject *const *v, Py_ssize_t n)
   a.dims(0, 3, d);
   const float eps = a.f(1), rate = a.f(2);
   const bool add = v[4] != Py_None, act = add || v[13] != Py_None;
+  const float slope = act ? a.f(13) : 0.f;      // (the residual epilogue always has one: None is refused)
   In x = a.ptr(3), res = a.ptr(4), gamma = a.ptr(10), beta = a.ptr(11);
   Out y = a.ptr(5), mean = a.ptr(6), var = a.ptr(7), rm = a.ptr(8), rv = a.ptr(9);
-  const float slope = v[13] != Py_None ? a.f(13) : 0.f;
   const int relu = a.truth(12);
   void *ws = a.raw(14);
   const size_t bytes = a.size(15);
@@ -197,9 +190,9 @@ PyObject *py_bwd(PyObject *, PyObject *const *v, Py_ssize_t n)
   uint32_t d[3] = {0, 0, 0};
   a.dims(0, 2, d);
   const bool add = v[3] != Py_None, act = add || v[13] != Py_None;
+  const float slope = act ? a.f(13) : 0.f;      // (the residual epilogue always has one: None is refused)
   In dy = a.ptr(1), x = a.ptr(2), y = a.ptr(3), mean = a.ptr(4), var = a.ptr(5), gamma = a.ptr(8), beta = a.ptr(9);
   Out dx = a.ptr(6), dres = a.ptr(7), dg = a.ptr(10), db = a.ptr(11);
-  const float slope = v[13] != Py_None ? a.f(13) : 0.f;
   const int relu = a.truth(12), acc = a.truth(14);
   void *ws = a.raw(15);
   const size_t bytes = a.size(16);
@@ -226,9 +219,9 @@ PyObject *py_infer(PyObject *, PyObject *const *v, Py_ssize_t n)
   Args a{v};
   uint32_t d[3] = {0, 0, 0};
   a.dims(0, 1, d);
+  const float slope = a.f(7);
   In x = a.ptr(1), mean = a.ptr(2), var = a.ptr(3), gamma = a.ptr(5), beta = a.ptr(6);
   Out y = a.ptr(4);
-  const float slope = a.f(7);
   void *s = a.stream(8);
   if (!a.ok || !bound(F_INFER)) return nullptr;
   int rc;

@@ -65,19 +65,28 @@ def dims_of(x, axes=None):
     return d0, int(x.shape[1]), int(x.shape[0])
 
 
-def _packed(name, axes, x, tensors, stream):
-    """One of the reference's entry points on [N, C, *spatial] arrays.  The launch hint (`cfg` of the ops) is not passed
-    on: the kernels choose their own launch shapes."""
+def _hint(cfg):
+    """The ops' launch hint: a KernelConfig or None.  It is looked at here and not passed on: the kernels choose their own
+    launch shapes."""
+    if cfg is not None:
+        ctypes.byref(cfg)
+
+
+def _packed(name, axes, x, tensors, stream, cfg):
+    """One of the reference's entry points on [N, C, *spatial] arrays."""
+    _hint(cfg)
     native().packed(_lib.address(name), axes, x, tensors, stream)
 
 
-def _packed_eps(name, axes, x, tensors, epsilon, stream):
+def _packed_eps(name, axes, x, tensors, epsilon, stream, cfg):
     """The same with an epsilon between dimensions and arrays."""
+    _hint(cfg)
     native().packed_eps(_lib.address(name), axes, x, tensors, epsilon, stream)
 
 
-def _flat(name, tensors, stream):
+def _flat(name, tensors, stream, cfg):
     """The same on flat arrays of the first one's length."""
+    _hint(cfg)
     native().flat(_lib.address(name), tensors, stream)
 
 
@@ -92,7 +101,7 @@ class BatchMean2dOp:
     def apply(axes, x, mean, cap=WriteCap.Assign, cfg=None, stream=None):
         if cap is not WriteCap.Assign:
             raise NotImplementedError("BatchMean2dOp: Accumulate (unimplemented in the reference)")
-        _packed("anode_gpu_batch_mean_3d1_packed_f32", axes, x, (x, mean), stream)
+        _packed("anode_gpu_batch_mean_3d1_packed_f32", axes, x, (x, mean), stream, cfg)
         return mean
 
 
@@ -102,7 +111,7 @@ class BatchMean2dBwdOp:
     def apply(axes, dmean, x, dx, cap=WriteCap.Assign, cfg=None, stream=None):
         name = "anode_gpu_batch_mean_bwd_3d1_packed_f32" if cap is WriteCap.Assign else \
             "anode_gpu_batch_mean_bwd_3d1_packed_accumulate_f32"
-        _packed(name, axes, x, (dmean, dx), stream)
+        _packed(name, axes, x, (dmean, dx), stream, cfg)
         return dx
 
 
@@ -112,7 +121,7 @@ class BatchVariance2dOp:
     def apply(axes, epsilon, x, mean, var, cap=WriteCap.Assign, cfg=None, stream=None):
         if cap is not WriteCap.Assign:
             raise NotImplementedError("BatchVariance2dOp: Accumulate (unimplemented in the reference)")
-        _packed_eps("anode_gpu_batch_var_3d1_packed_f32", axes, x, (x, mean, var), epsilon, stream)
+        _packed_eps("anode_gpu_batch_var_3d1_packed_f32", axes, x, (x, mean, var), epsilon, stream, cfg)
         return var
 
 
@@ -122,7 +131,7 @@ class BatchVariance2dBwdOp:
     def apply(axes, dvar, x, mean, dx, cap=WriteCap.Assign, cfg=None, stream=None):
         name = "anode_gpu_batch_var_bwd_3d1_packed_f32" if cap is WriteCap.Assign else \
             "anode_gpu_batch_var_bwd_3d1_packed_accumulate_f32"
-        _packed(name, axes, x, (dvar, x, mean, dx), stream)
+        _packed(name, axes, x, (dvar, x, mean, dx), stream, cfg)
         return dx
 
 
@@ -132,7 +141,7 @@ class BatchVariance2dBwdMeanOp:
     def apply(axes, dvar, x, mean, dmean, cap=WriteCap.Assign, cfg=None, stream=None):
         name = "anode_gpu_batch_var_bwd_mean_3d1_packed_f32" if cap is WriteCap.Assign else \
             "anode_gpu_batch_var_bwd_mean_3d1_packed_accumulate_f32"
-        _packed(name, axes, x, (dvar, x, mean, dmean), stream)
+        _packed(name, axes, x, (dvar, x, mean, dmean), stream, cfg)
         return dmean
 
 
@@ -142,7 +151,7 @@ class BatchNormalize2dOp:
     def apply(axes, x, mean, var, y, cap=WriteCap.Assign, cfg=None, stream=None):
         if cap is not WriteCap.Assign:
             raise NotImplementedError("BatchNormalize2dOp: Accumulate (unimplemented in the reference)")
-        _packed("anode_gpu_batch_norm_3d1_packed_f32", axes, x, (x, mean, var, y), stream)
+        _packed("anode_gpu_batch_norm_3d1_packed_f32", axes, x, (x, mean, var, y), stream, cfg)
         return y
 
 
@@ -152,7 +161,7 @@ class BatchNormalize2dBwdOp:
     def apply(axes, dy, var, dx, cap=WriteCap.Assign, cfg=None, stream=None):
         name = "anode_gpu_batch_norm_bwd_3d1_packed_f32" if cap is WriteCap.Assign else \
             "anode_gpu_batch_norm_bwd_3d1_packed_accumulate_f32"
-        _packed(name, axes, dy, (dy, var, dx), stream)
+        _packed(name, axes, dy, (dy, var, dx), stream, cfg)
         return dx
 
 
@@ -162,7 +171,7 @@ class BatchNormalize2dBwdMeanOp:
     def apply(axes, dy, var, dmean, cap=WriteCap.Assign, cfg=None, stream=None):
         name = "anode_gpu_batch_norm_bwd_mean_3d1_packed_f32" if cap is WriteCap.Assign else \
             "anode_gpu_batch_norm_bwd_mean_3d1_packed_accumulate_f32"
-        _packed(name, axes, dy, (dy, var, dmean), stream)
+        _packed(name, axes, dy, (dy, var, dmean), stream, cfg)
         return dmean
 
 
@@ -173,14 +182,14 @@ class BatchNormalize2dBwdVarianceOp:
     def apply(axes, dy, x, mean, var, dvar, cap=WriteCap.Assign, cfg=None, stream=None):
         name = "anode_gpu_batch_norm_bwd_var_3d1_packed_f32" if cap is WriteCap.Assign else \
             "anode_gpu_batch_norm_bwd_var_3d1_packed_accumulate_f32"
-        _packed(name, axes, x, (dy, x, mean, var, dvar), stream)
+        _packed(name, axes, x, (dy, x, mean, var, dvar), stream, cfg)
         return dvar
 
     @staticmethod
     def apply_v2(axes, dy, y, var, dvar, cap=WriteCap.Assign, cfg=None, stream=None):
         name = "anode_gpu_batch_norm_bwd_var_v2_3d1_packed_f32" if cap is WriteCap.Assign else \
             "anode_gpu_batch_norm_bwd_var_v2_3d1_packed_accumulate_f32"
-        _packed(name, axes, y, (dy, y, var, dvar), stream)
+        _packed(name, axes, y, (dy, y, var, dvar), stream, cfg)
         return dvar
 
 
@@ -207,7 +216,7 @@ class PositiveClipOp:
     is the in-place form of PositiveClipClobberOp (:8584-8671)."""
     @staticmethod
     def apply(x, y, cfg=None, stream=None):
-        _flat("anode_gpu_positive_clip_flat_map_f32", (x, y), stream)
+        _flat("anode_gpu_positive_clip_flat_map_f32", (x, y), stream, cfg)
         return y
 
 
@@ -215,7 +224,7 @@ class PositiveClipBwdOp:
     """src/ops_gpu.rs:8499-8582: dx = dy * (y > 0); `dx is dy` is the clobber form (:8673-8755)."""
     @staticmethod
     def apply(dy, y, dx, cfg=None, stream=None):
-        _flat("anode_gpu_positive_clip_flat_map_bwd_f32", (dy, y, dx), stream)
+        _flat("anode_gpu_positive_clip_flat_map_bwd_f32", (dy, y, dx), stream, cfg)
         return dx
 
 
@@ -223,7 +232,7 @@ class FlatJoinOp:
     """src/ops_gpu.rs:8169-8261: y = x1 * step(x2) (routines_gpu/flat_join.cu:50-60)."""
     @staticmethod
     def apply(x1, x2, y, cfg=None, stream=None):
-        _flat("anode_gpu_M1_copy_map_M2_unit_step_map_R_product_reduce_flat_join_f32", (x1, x2, y), stream)
+        _flat("anode_gpu_M1_copy_map_M2_unit_step_map_R_product_reduce_flat_join_f32", (x1, x2, y), stream, cfg)
         return y
 
 
@@ -336,8 +345,12 @@ class Workspace:
               "workspace_init")
 
 
-def _scratch(workspace, x):
-    return workspace if workspace is not None else Workspace(*dims_of(x), x.device)
+def _scratch(workspace, x, axes):
+    """The call's workspace and axes: a caller without a workspace has the axes checked before one is made."""
+    if workspace is not None:
+        return workspace, axes
+    axes = None if axes is None else list(axes)
+    return Workspace(*dims_of(x, axes), x.device), axes
 
 
 class BatchNormalize2dFusedOp:
@@ -345,8 +358,9 @@ class BatchNormalize2dFusedOp:
     @staticmethod
     def apply(axes, epsilon, avg_rate, x, y, mean, var, avg_mean=None, avg_var=None, gamma=None, beta=None,
               relu=True, workspace=None, cfg=None, stream=None, neg_slope=None):
+        _hint(cfg)
         # neg_slope: general activation t*(t > 0 ? 1 : neg_slope), e.g. leaky ReLU
-        ws = _scratch(workspace, x)
+        ws, axes = _scratch(workspace, x, axes)
         rc = native().fwd(axes, epsilon, avg_rate, x, None, y, mean, var, avg_mean, avg_var, gamma, beta, relu, neg_slope,
                           ws.buf, ws.bytes, stream)
         if rc:
@@ -359,7 +373,8 @@ class BatchNormalize2dBwdFusedOp:
     @staticmethod
     def apply(axes, dy, x, mean, var, dx, gamma=None, beta=None, dgamma=None, dbeta=None, relu=True,
               cap=WriteCap.Assign, workspace=None, cfg=None, stream=None, neg_slope=None):
-        ws = _scratch(workspace, x)
+        _hint(cfg)
+        ws, axes = _scratch(workspace, x, axes)
         rc = native().bwd(axes, dy, x, None, mean, var, dx, None, gamma, beta, dgamma, dbeta, relu, neg_slope,
                           cap is WriteCap.Accumulate, ws.buf, ws.bytes, stream)
         if rc:
@@ -373,7 +388,8 @@ class BatchNormalize2dAddActFusedOp:
     @staticmethod
     def apply(axes, epsilon, avg_rate, x, residual, y, mean, var, avg_mean=None, avg_var=None, gamma=None, beta=None,
               neg_slope=0.0, workspace=None, cfg=None, stream=None):
-        ws = _scratch(workspace, x)
+        _hint(cfg)
+        ws, axes = _scratch(workspace, x, axes)
         if residual is None:
             check(-1, "anode_gpu_batch_norm_add_act_fused_fwd_3d1_packed_f32")
         rc = native().fwd(axes, epsilon, avg_rate, x, residual, y, mean, var, avg_mean, avg_var, gamma, beta, True, neg_slope,
@@ -385,7 +401,8 @@ class BatchNormalize2dAddActFusedOp:
     @staticmethod
     def adjoint(axes, dy, x, y, mean, var, dx, dresidual=None, gamma=None, beta=None, dgamma=None, dbeta=None,
                 neg_slope=0.0, cap=WriteCap.Assign, workspace=None, cfg=None, stream=None):
-        ws = _scratch(workspace, x)
+        _hint(cfg)
+        ws, axes = _scratch(workspace, x, axes)
         if y is None:
             check(-1, "anode_gpu_batch_norm_add_act_fused_bwd_3d1_packed_f32")
         rc = native().bwd(axes, dy, x, y, mean, var, dx, dresidual, gamma, beta, dgamma, dbeta, True, neg_slope,
@@ -403,6 +420,7 @@ class BatchNormalize2dActInferOp:
     neg_slope 0 = ReLU (positive_clip), 1 = none, c = leaky ReLU (flat_map.cu:44-52)."""
     @staticmethod
     def apply(axes, x, mean, var, y, gamma=None, beta=None, neg_slope=0.0, cfg=None, stream=None):
+        _hint(cfg)
         rc = native().infer(axes, x, mean, var, y, gamma, beta, neg_slope, stream)
         if rc:
             check(rc, "anode_gpu_batch_norm_act_infer_3d1_packed_f32")

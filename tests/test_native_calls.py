@@ -1,5 +1,6 @@
 """The native call module (csrc/bn_py.cpp) refuses what it cannot take with a Python error, on any machine: nothing of a
 refused call reaches CUDA, and no C++ exception leaves the module."""
+import numpy as np
 import pytest
 import torch
 from torch._subclasses.fake_tensor import FakeTensorMode
@@ -84,3 +85,54 @@ def test_the_references_entry_points_take_no_missing_array(call):
     """They have no status to answer with: a missing array would be read."""
     with pytest.raises((ValueError, AttributeError)):
         call(torch.zeros(2, 3, 4, 4), torch.zeros(3))
+
+
+def entries(axes, **kw):
+    """One op of each kind with these axes, on host tensors, with a workspace where one is taken."""
+    x, v = torch.zeros(2, 3, 4, 4), torch.zeros(3)
+    fused = dict(kw, workspace=Scratch())
+    return [lambda: ops.BatchMean2dOp.apply(axes(), x, v, **kw), lambda: ops.BatchVariance2dOp.apply(axes(), 1e-5, x, v, v, **kw),
+            lambda: ops.BatchNormalize2dActInferOp.apply(axes(), x, v, v, x, **kw),
+            lambda: ops.BatchNormalize2dFusedOp.apply(axes(), 1e-5, 0.1, x, x, v, v, **fused),
+            lambda: ops.BatchNormalize2dBwdFusedOp.apply(axes(), x, x, v, v, x, **fused),
+            lambda: ops.BatchNormalize2dAddActFusedOp.apply(axes(), 1e-5, 0.1, x, x, x, v, v, **fused),
+            lambda: ops.BatchNormalize2dAddActFusedOp.adjoint(axes(), x, x, x, v, v, x, **fused)]
+
+
+@pytest.mark.parametrize("axes", [lambda: [0, 1], lambda: (0, 1), lambda: range(2), lambda: iter([0, 1]), lambda: {0: 0, 1: 0},
+                                  lambda: np.arange(2), lambda: torch.arange(2), lambda: [0.0, 1.0], lambda: None],
+                         ids=["list", "tuple", "range", "iterator", "keys", "numpy", "torch", "floats", "unchecked"])
+def test_axes_are_any_iterable_of_the_positions(axes):
+    for call in entries(axes):
+        with pytest.raises(ValueError, match="contiguous float32 CUDA tensor"):      # the axes were taken
+            call()
+
+
+@pytest.mark.parametrize("axes", [[1, 0], [0], [0, 1, 2], [], "ab"])
+def test_other_axes_are_refused(axes):
+    for call in entries(lambda: axes):
+        with pytest.raises(ValueError, match="axes must be"):
+            call()
+    x, v = torch.zeros(2, 3, 4, 4), torch.zeros(3)
+    with pytest.raises(ValueError, match="axes must be"):          # and before a workspace is made
+        ops.BatchNormalize2dFusedOp.apply(axes, 1e-5, 0.1, x, x, v, v)
+    with pytest.raises(TypeError):
+        ops.BatchMean2dOp.apply(7, x, v)
+
+
+def test_a_launch_hint_is_one():
+    x = torch.zeros(2, 3, 4, 4)
+    for call in entries(lambda: [0, 1], cfg="1024") + [lambda: ops.PositiveClipOp.apply(x, x, cfg=1024)]:
+        with pytest.raises(TypeError):
+            call()
+    for call in entries(lambda: [0, 1], cfg=ops.KernelConfig(256, 148)):
+        with pytest.raises(ValueError, match="contiguous float32 CUDA tensor"):
+            call()
+
+
+def test_the_residual_epilogue_has_a_slope():
+    x, v = torch.zeros(2, 3, 4, 4), torch.zeros(3)
+    with pytest.raises(TypeError):
+        ops.BatchNormalize2dAddActFusedOp.apply([0, 1], 1e-5, 0.1, x, x, x, v, v, neg_slope=None, workspace=Scratch())
+    with pytest.raises(TypeError):
+        ops.BatchNormalize2dAddActFusedOp.adjoint([0, 1], x, x, x, v, v, x, neg_slope=None, workspace=Scratch())
