@@ -18,11 +18,13 @@ namespace anode_b200 {
 
 constexpr uint32_t kInferThreads = 256;
 
+// The inputs carry no __restrict__: it would let the compiler treat their loads as reads of memory that nothing writes while
+// the kernel runs and move them above pdl_wait(), where the kernel before this one may still be writing them (the running
+// averages of a training step, the activations of the layer below).
 template <int VEC>
 __global__ void __launch_bounds__(kInferThreads) bn_infer_kernel(uint32_t dim0, uint32_t C, uint32_t N, float neg_slope,
-                                                                 const float *__restrict__ x, const float *__restrict__ mean,
-                                                                 const float *__restrict__ var, const float *__restrict__ gamma,
-                                                                 const float *__restrict__ beta, float *y)
+                                                                 const float *x, const float *mean, const float *var,
+                                                                 const float *gamma, const float *beta, float *y)
 {
   const uint64_t per_sample = (uint64_t)C * dim0;                 // floats
   const uint64_t col = ((uint64_t)blockIdx.x * kInferThreads + threadIdx.x) * VEC;
