@@ -45,6 +45,23 @@ def test_residual_epilogue(tiled, shape, slope):
     check_layer_own_mask(d, got, "%r slope %g " % (shape, slope), residual=res, slope=slope)
 
 
+@pytest.mark.parametrize("at", [0.0, 30.0, 100.0])
+@pytest.mark.parametrize("shape,residual", [((64, 12, 55, 55), False), ((64, 12, 55, 55), True), ((9, 5, 31, 33), False),
+                                            ((64, 8, 56, 56), False), ((64, 8, 56, 56), True), ((6, 3, 160, 121), False)])
+def test_rows_that_begin_far_from_the_mean(tiled, shape, residual, at):
+    """The first element of every row (the corner of the image) lies at many standard deviations.  A thread adds up at most
+    16384 / 256 = 64 squares one after another, about a shift that is within two deviations of the mean, so the variance is
+    off by at most 64 roundings of 2^-24 on 1 + 2^2 times its size, and typically by far less."""
+    d = make_inputs(shape, seed=sum(shape), loc=0.0, scale=1.0)
+    d["x"][:, :, 0, 0] = at
+    x = d["x"].astype(np.float64)
+    want = x.var(axis=(0, 2, 3)) + 1e-5
+    got = run_add_act(tiled, d, np.zeros(shape, np.float32), 0.0) if residual else run_fused(tiled, d)[0]
+    err = float(np.max(np.abs(got["var"] - want) / want))
+    print("%r residual %d first element %g: relative error of the variance %.1e" % (shape, residual, at, err))
+    assert err < 5 * 64 * 2.0 ** -24, err
+
+
 @pytest.mark.parametrize("shape", [(7, 3, 13, 13), (64, 7, 15, 15), (700, 3, 33, 31), (40, 24, 56, 56), (2, 3, 160, 120)])
 @pytest.mark.parametrize("form", ["separate", "dres is dy", "dres is y", "dres is x", "no dres", "dx is dy", "dx is x", "accumulate"])
 def test_outputs_over_inputs(tiled, shape, form):
