@@ -260,6 +260,13 @@ static bool chan_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra
   return true;
 }
 
+bool chan_applies(const FusedArgs &a, int dir, bool aligned)
+{
+  ChanGeom g;
+  const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
+  return a.mode == MODE_FUSED && a.world <= 1 && chan_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, extra, aligned, g);
+}
+
 // Where this kernel is taken: wherever a team can hold the channel, except on large layers where the team would be of
 // more than half the largest size (its load, exchange and store then follow one another on most of the device) and
 // where the elements would be fetched one by one although aligned runs of several channels, or long ragged rows, can be

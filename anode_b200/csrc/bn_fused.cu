@@ -371,9 +371,11 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
     case ANODE_KERNEL_CLUSTER: if (segres_applies(a, dir, aligned)) return ANODE_KERNEL_CLUSTER; break;
     case ANODE_KERNEL_RESIDENT: if (resident_applies(a, dir, aligned)) return ANODE_KERNEL_RESIDENT; break;
     case ANODE_KERNEL_PLAIN: if (plain_ok) return ANODE_KERNEL_PLAIN; break;
+    case ANODE_KERNEL_REGISTER: if (chan_applies(a, dir, aligned)) return ANODE_KERNEL_REGISTER; break;
+    case ANODE_KERNEL_STREAM: if (stream_applies(a, dir, aligned)) return ANODE_KERNEL_STREAM; break;
     default:
-      if (chan_preferred(a, dir, aligned, tiled_ok)) return kKernelChan;
-      if (stream_preferred(a, dir, aligned, tiled_ok)) return kKernelStream;
+      if (chan_preferred(a, dir, aligned, tiled_ok)) return ANODE_KERNEL_REGISTER;
+      if (stream_preferred(a, dir, aligned, tiled_ok)) return ANODE_KERNEL_STREAM;
       break;
   }
   if (extra) {
@@ -400,8 +402,8 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
 int launch_best(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)
 {
   int kind = pick_kernel_kind(a, dir, aligned);
-  if (kind == kKernelChan) return launch_chan(a, dir, aligned, stream);
-  if (kind == kKernelStream) {
+  if (kind == ANODE_KERNEL_REGISTER) return launch_chan(a, dir, aligned, stream);
+  if (kind == ANODE_KERNEL_STREAM) {
     if (launch_stream(a, dir, stream) == ANODE_OK) return ANODE_OK;
     kind = segres_applies(a, dir, aligned) ? ANODE_KERNEL_CLUSTER : ANODE_KERNEL_PLAIN;
   }
@@ -684,45 +686,55 @@ extern "C" int anode_gpu_online_average_f32(uint32_t len, float rate, const floa
   return ANODE_OK;
 }
 
-// The family callers see (ANODE_KERNEL_*), by the shapes it stands for: the register-resident and the streaming kernel
-// count as cluster kernels on the shapes of that family and as the any-shape, any-alignment family elsewhere, and so do
-// the tiled kernel's ragged rows.
-static int public_kind(const FusedArgs &a, int dir, bool aligned)
+// A call of this form with a workspace of the full size, as far as the choice of the kernel looks at it.
+static FusedArgs probe_call(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool residual, bool aligned, int world)
 {
-  const int k = pick_kernel_kind(a, dir, aligned);
-  if (k == ANODE_KERNEL_TILED && a.plan.dim0 % 4 != 0) return ANODE_KERNEL_PLAIN;
-  if (k != kKernelChan && k != kKernelStream) return k;
-  return segres_applies(a, dir, aligned) ? ANODE_KERNEL_CLUSTER : ANODE_KERNEL_PLAIN;
+  static const float dummy = 0.f;
+  FusedArgs a{};
+  a.plan = plan_for(dim0, C, N, aligned);
+  a.mode = MODE_FUSED;
+  a.world = world > 1 ? (uint32_t)world : 0u;
+  a.ws_capacity = workspace_part_bytes(dim0, C, N);
+  if (residual) (dir == 0 ? a.res : a.ymask) = &dummy;       // only their presence matters here
+  return a;
 }
 
-// Which kernel serves direction `dir` of a plain [dim0, dim1, dim2] call with 16-byte aligned tensors on
-// one GPU: an ANODE_KERNEL_* value.
+extern "C" int anode_gpu_batch_norm_fused_serving_kernel(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual,
+                                                         int aligned, int world)
+{
+  if (check_dims(dim0, dim1, dim2) || (dir != 0 && dir != 1)) return ANODE_E_DIMS;
+  const int k = pick_kernel_kind(probe_call(dim0, dim1, dim2, dir, residual != 0, aligned != 0, world), dir, aligned != 0);
+  return k < 0 ? ANODE_KERNEL_AUTO : k;
+}
+
+// The family, among the first four kernels, of the shape of a one-GPU call on aligned tensors.
+static int family(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool residual)
+{
+  if (check_dims(dim0, C, N)) return ANODE_E_DIMS;
+  const FusedArgs a = probe_call(dim0, C, N, dir, residual, true, 1);
+  const int k = pick_kernel_kind(a, dir, true);
+  if (k == ANODE_KERNEL_TILED && dim0 % 4 != 0) return ANODE_KERNEL_PLAIN;
+  if (k != ANODE_KERNEL_REGISTER && k != ANODE_KERNEL_STREAM) return k;
+  if (segres_preferred(a, dir, true)) return ANODE_KERNEL_CLUSTER;
+  Plan p; RingGeom g;
+  if (dim0 % 4 == 0 && ring_plan_of(a, dir, true, p, g)) return ANODE_KERNEL_TILED;
+  return segres_applies(a, dir, true) ? ANODE_KERNEL_CLUSTER : ANODE_KERNEL_PLAIN;
+}
+
 extern "C" int anode_gpu_batch_norm_fused_kernel_kind(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir)
 {
-  if (check_dims(dim0, dim1, dim2)) return ANODE_E_DIMS;
-  FusedArgs a{};
-  a.plan = plan_for(dim0, dim1, dim2, true);
-  a.mode = MODE_FUSED;
-  a.ws_capacity = workspace_part_bytes(dim0, dim1, dim2);
-  return public_kind(a, dir, true);
+  return family(dim0, dim1, dim2, dir, false);
 }
 
 // The same for the residual-epilogue calls (anode_gpu_batch_norm_add_act_fused_*).
 extern "C" int anode_gpu_batch_norm_add_act_fused_kernel_kind(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir)
 {
-  if (check_dims(dim0, dim1, dim2)) return ANODE_E_DIMS;
-  static const float dummy = 0.f;
-  FusedArgs a{};
-  a.plan = plan_for(dim0, dim1, dim2, true);
-  a.mode = MODE_FUSED;
-  a.ws_capacity = workspace_part_bytes(dim0, dim1, dim2);
-  if (dir == 0) a.res = &dummy; else a.ymask = &dummy;       // only their presence matters here
-  return public_kind(a, dir, true);
+  return family(dim0, dim1, dim2, dir, true);
 }
 
 extern "C" int anode_gpu_batch_norm_fused_set_kernel(int kernel)
 {
-  if (kernel < ANODE_KERNEL_AUTO || kernel > ANODE_KERNEL_PLAIN) return ANODE_E_DIMS;
+  if (kernel < ANODE_KERNEL_AUTO || kernel > ANODE_KERNEL_STREAM) return ANODE_E_DIMS;
   g_kernel_choice.store(kernel, std::memory_order_relaxed);
   return ANODE_OK;
 }

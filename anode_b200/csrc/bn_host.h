@@ -49,11 +49,11 @@ bool segres_applies(const FusedArgs &a, int dir, bool aligned);
 bool segres_preferred(const FusedArgs &a, int dir, bool aligned);      // take it even where the tiled kernel applies
 int launch_segres(FusedArgs &a, int dir, cudaStream_t stream);
 // the register-resident kernel (bn_chan.cu); one GPU, any alignment
-constexpr int kKernelChan = 5;            // its number inside the library (callers see the family, see public_kind)
+bool chan_applies(const FusedArgs &a, int dir, bool aligned);
 bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok);
 int launch_chan(FusedArgs &a, int dir, bool aligned, cudaStream_t stream);
 // the streaming cluster kernel for large layers of short rows (bn_stream.cu); one GPU
-constexpr int kKernelStream = 6;          // its number inside the library (callers see the cluster family)
+bool stream_applies(const FusedArgs &a, int dir, bool aligned);
 bool stream_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok);
 int launch_stream(FusedArgs &a, int dir, cudaStream_t stream);
 uint64_t workspace_part_bytes(uint32_t dim0, uint32_t C, uint32_t N);

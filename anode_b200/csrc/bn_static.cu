@@ -49,13 +49,13 @@ static void static_need(const FusedArgs &a, bool aligned, uint64_t &need, uint64
 {
   const uint32_t dim0 = a.plan.dim0, C = a.plan.C, N = a.plan.N;
   switch (pick_kernel_kind(a, 0, aligned)) {
-    case kKernelStream:               // (where the device refuses its cluster, the plain kernel may have to serve the call)
+    case ANODE_KERNEL_STREAM:             // (where the device refuses its cluster, the plain kernel may have to serve the call)
     case ANODE_KERNEL_PLAIN: {
       const Plan p = plan_for(dim0, C, N, aligned);
       need = p.ws_bytes; clear = p.off_part;
       if (pick_kernel_kind(a, 0, aligned) == ANODE_KERNEL_PLAIN || !segres_applies(a, 0, aligned)) break;
     }                                 // fall through
-    case kKernelChan:
+    case ANODE_KERNEL_REGISTER:
     case ANODE_KERNEL_CLUSTER:        // keep everything on chip: only the status word lives in the array
       need = clear = 256;
       break;

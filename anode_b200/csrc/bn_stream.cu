@@ -328,6 +328,12 @@ static bool stream_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, StreamGe
   return true;
 }
 
+bool stream_applies(const FusedArgs &a, int dir, bool aligned)
+{
+  StreamGeom g;
+  return aligned && a.mode == MODE_FUSED && a.world <= 1 && stream_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, g);
+}
+
 // Where this kernel is taken (after the register-resident kernel): all rows that the tiled kernel does not serve, and of
 // those it does serve (`tiled_ok`) the short ones and the medium ones of channels that are not too large.  Forward /
 // backward in us, here and on the tiled kernel: [4096,64,16,16] 131 / 225 and 168 / 336, [2048,64,20,20] 111 / 192 and
@@ -337,9 +343,8 @@ static bool stream_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, StreamGe
 constexpr uint32_t kStreamShortRow = 512, kStreamMediumRow = 600, kStreamLongRow = 1024;
 bool stream_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
 {
-  StreamGeom g;
   const uint32_t dim0 = a.plan.dim0;
-  if (!aligned || a.mode != MODE_FUSED || a.world > 1 || !stream_geom(dim0, a.plan.C, a.plan.N, dir, g)) return false;
+  if (!stream_applies(a, dir, aligned)) return false;
   if (!tiled_ok || dim0 <= kStreamShortRow) return true;
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
   const uint64_t most = (extra ? 1u << 18 : dir == 1 ? 1u << 17 : 1u << 16) * (dim0 <= kStreamMediumRow ? 4ull : 1ull);

@@ -303,13 +303,25 @@ def relu(x, inplace=False, cfg=None, stream=None):
 # built by the reference (src/ops.rs:105-106).  One kernel per direction.
 # --------------------------------------------------------------------------------------------
 
-KERNELS = {"auto": 0, "tiled": 1, "cluster": 2, "resident": 3, "plain": 4}
+KERNELS = {"auto": 0, "tiled": 1, "cluster": 2, "resident": 3, "plain": 4, "register": 5, "stream": 6}
 
 
 def set_kernel(name):
     """Process-wide kernel preference of the fused calls (anode_gpu_batch_norm_fused_set_kernel):
-    'auto', 'tiled', 'cluster', 'resident' or 'plain'.  For tests and measurements."""
+    a name of KERNELS.  For tests and measurements."""
     check(_lib.load().anode_gpu_batch_norm_fused_set_kernel(KERNELS[name]), "anode_gpu_batch_norm_fused_set_kernel")
+
+
+def serving_kernel(shape, dir, residual=False, aligned=True, world=1):
+    """Name, in KERNELS, of the kernel that a fused call on a [N, C, *spatial] shape launches
+    (anode_gpu_batch_norm_fused_serving_kernel); None where a synchronized call takes three."""
+    d0 = 1
+    for s in shape[2:]:
+        d0 *= int(s)
+    k = _lib.load().anode_gpu_batch_norm_fused_serving_kernel(d0, int(shape[1]), int(shape[0]), dir, int(residual), int(aligned), world)
+    if k < 0:
+        raise AnodeError(k, "anode_gpu_batch_norm_fused_serving_kernel")
+    return {v: n for n, v in KERNELS.items()}[k] if k else None
 
 
 def set_wait_limit_ms(ms):
@@ -565,9 +577,7 @@ class SyncBatchNormRelu(FusedBatchNormRelu):
             return 6
         if self._x is None:
             return 2
-        d0, c, n = dims_of(self._x)
-        kind = _lib.load().anode_gpu_batch_norm_fused_kernel_kind
-        return sum(1 if kind(d0, c, n, d) != 4 else 3 for d in (0, 1))      # 4: the plain kernel (ANODE_KERNEL_PLAIN)
+        return sum(3 if serving_kernel(self._x.shape, d, world=self.comm.world) is None else 1 for d in (0, 1))
 
     def step_from_host(self, hx, hdy, hy, hdx, chunk_channels=0):
         """This rank's shard in (page-locked) host memory, through ONE C-ABI call: channel blocks copied in

@@ -185,14 +185,20 @@ void anode_gpu_positive_clip_flat_map_bwd_f32(
  *   CLUSTER   thread-block clusters keeping a unit's slice in shared memory (short rows, small channels);
  *   RESIDENT  slices resident in shared memory, all global traffic by bulk copies; takes the residual
  *             epilogue on long rows, also in synchronized calls;
- *   PLAIN     plain loads and stores (any shape, any alignment; one GPU).
- * anode_gpu_batch_norm_fused_set_kernel makes another choice process-wide: that kernel is used wherever
- * it applies, the automatic choice elsewhere.  Meant for tests and measurements. */
+ *   PLAIN     plain loads and stores (any shape, any alignment; one GPU);
+ *   REGISTER  channels held in the registers of a warp, a block or a cluster (small layers, any alignment;
+ *             one GPU);
+ *   STREAM    clusters that walk a block of channels twice (large layers of short rows; one GPU).
+ * anode_gpu_batch_norm_fused_set_kernel makes another choice process-wide: that kernel is used wherever it
+ * applies, elsewhere one of the first four by the shape.  Meant for tests and measurements; which kernel a
+ * call launches is answered by anode_gpu_batch_norm_fused_serving_kernel (anode_routines_gpu_diag.h). */
 #define ANODE_KERNEL_AUTO      0
 #define ANODE_KERNEL_TILED     1
 #define ANODE_KERNEL_CLUSTER   2
 #define ANODE_KERNEL_RESIDENT  3
 #define ANODE_KERNEL_PLAIN     4
+#define ANODE_KERNEL_REGISTER  5
+#define ANODE_KERNEL_STREAM    6
 int anode_gpu_batch_norm_fused_set_kernel(int kernel);
 
 /* Bound of every wait inside the kernels (for a channel's statistics, for another GPU's records), in

@@ -12,8 +12,17 @@
 extern "C" {
 #endif
 
-/* Kernel that serves direction `dir` (0 forward, 1 backward) of a plain fused call on 16-byte
- * aligned tensors on one GPU: an ANODE_KERNEL_* value of anode_routines_gpu.h. */
+/* Kernel that direction `dir` (0 forward, 1 backward) of a fused call launches, with a workspace of the full size:
+ * an ANODE_KERNEL_* value of anode_routines_gpu.h.  residual: the residual-epilogue calls; aligned: every tensor on a
+ * 16-byte boundary; world: ranks of a synchronized call whose communicator has an exchange buffer (1: a call on one
+ * GPU).  ANODE_KERNEL_AUTO (0): a synchronized call that no kernel with the exchange inside serves (a reduce, an
+ * exchange and an apply kernel are launched). */
+int anode_gpu_batch_norm_fused_serving_kernel(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual,
+                                              int aligned, int world);
+
+/* Family, among the first four ANODE_KERNEL_* values, that the shape of a plain fused call on 16-byte aligned tensors
+ * belongs to.  (The REGISTER and STREAM kernels and the TILED kernel's ragged rows count as the family whose shapes they
+ * take over on one GPU; for the kernel that is launched ask anode_gpu_batch_norm_fused_serving_kernel.) */
 int anode_gpu_batch_norm_fused_kernel_kind(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir);
 
 /* The same for the residual-epilogue calls (anode_gpu_batch_norm_add_act_fused_*). */

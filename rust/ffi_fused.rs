@@ -35,6 +35,8 @@ pub const ANODE_KERNEL_TILED: c_int = 1;
 pub const ANODE_KERNEL_CLUSTER: c_int = 2;
 pub const ANODE_KERNEL_RESIDENT: c_int = 3;
 pub const ANODE_KERNEL_PLAIN: c_int = 4;
+pub const ANODE_KERNEL_REGISTER: c_int = 5;
+pub const ANODE_KERNEL_STREAM: c_int = 6;
 pub const ANODE_STATIC_SCRATCH_BYTES: usize = 4 << 20;
 
 #[link(name = "anode_routines_gpu")]
