@@ -389,7 +389,8 @@ def bench_workload(ops, name, rank, world, steps, warmup, dist, device, sample_c
     n_global = n_local * world
     ms = total / steps
     res = {"ms_per_step": ms, "fwd_ms": fwd, "bwd_ms": bwd, "elements_local": n_local, "elements_global": n_global,
-           "value": n_global / (ms * 1e-3), "clocks": clocks, "launches_per_step": layer.launches_per_step, "parity": parity}
+           "value": n_global / (ms * 1e-3), "clocks": clocks, "launches_per_step": layer.launches_per_step, "parity": parity,
+           "exchange": world == 1 or getattr(layer.comm, "_exchange", None) is not None}
     if with_e2e:
         res["e2e"] = bench_e2e(ops, layer, x, dy, y, dx, dist, device, min(steps, 3))     # first: it compares with y, dx of the timed steps
         res["infer"] = bench_infer(layer, x, y, steps, warmup)
@@ -427,12 +428,18 @@ def bench_residual(ops, layer, x, dy, y, dx, steps, warmup):
     peak, kind = hbm_peak()
     gbs = 32.0 * x.numel() / (ms * 1e-3) / 1e9
     del res, dres
-    from anode_b200 import _lib
-    names = {1: "bn_ring_kernel", 2: "bn_segres_kernel", 3: "bn_resident_kernel", 4: "bn_pipeline_kernel"}
-    d0, c, n = ops.dims_of(x)
-    kk = [names.get(_lib.load().anode_gpu_batch_norm_add_act_fused_kernel_kind(d0, c, n, d), "?") for d in (0, 1)]
+    kk = [KERNEL_NAMES[ops.serving_kernel(x.shape, d, residual=True)][0] for d in (0, 1)]
     return {"kernel": "%s (forward), %s (backward), residual epilogue" % tuple(kk), "ms_per_step": ms,
             "elements_per_s": x.numel() / (ms * 1e-3), "achieved_gbs": gbs, "frac_of_hbm_peak": gbs / peak, "peak_kind": kind}
+
+
+#: kernel family -> (its CUDA kernel, how it works)
+KERNEL_NAMES = {"tiled": ("bn_ring_kernel", "fused reduce+apply, tiled"),
+                "cluster": ("bn_segres_kernel", "fused reduce+apply, clusters"),
+                "resident": ("bn_resident_kernel", "fused reduce+apply, slices resident in shared memory"),
+                "plain": ("bn_pipeline_kernel", "fused reduce+apply, plain"),
+                "register": ("bn_chan_kernel", "fused reduce+apply, channels in registers"),
+                "stream": ("bn_stream_kernel", "fused reduce+apply, streaming clusters")}
 
 
 def bench_infer(layer, x, y, steps, warmup):
@@ -545,7 +552,7 @@ def main():
     ap.add_argument("--shape", default=None, help="custom global shape N,C,spatial... (N(0,1) data, sharded on axis 0); "
                     "used for small profiler captures")
     ap.add_argument("--no-extras", action="store_true", help="skip cpu_baseline, e2e and other_workloads")
-    ap.add_argument("--kernel", default="auto", choices=["auto", "tiled", "cluster", "resident", "plain"],
+    ap.add_argument("--kernel", default="auto", choices=["auto"] + sorted(KERNEL_NAMES),
                     help="kernel preference of the fused calls (anode_gpu_batch_norm_fused_set_kernel); for profiler captures")
     args = ap.parse_args()
     args.warmup = max(args.warmup, 3)
@@ -586,18 +593,12 @@ def main():
 
     w = WORKLOADS[args.workload]
     def kernel_name(direction):
-        if main_res["launches_per_step"] != 2:
+        if not main_res["exchange"]:
             return "reduce kernel + all-gather + merge kernel + apply kernel (%s)" % direction
-        from anode_b200 import _lib
-        shp = local_shape(w, rank, world)
-        d0 = 1
-        for v in shp[2:]:
-            d0 *= int(v)
-        c, n = int(shp[1]), int(shp[0])
-        kind = _lib.load().anode_gpu_batch_norm_fused_kernel_kind(d0, c, n, 0 if direction == "fwd" else 1)
-        return {3: "bn_resident_kernel<%s> (fused reduce+apply, slices resident in shared memory)",
-                1: "bn_ring_kernel<%s> (fused reduce+apply, tiled)", 2: "bn_segres_kernel<%s> (fused reduce+apply, clusters)",
-                4: "bn_pipeline_kernel<%s> (fused reduce+apply, plain)"}.get(kind, "?%s") % direction
+        kind = ops.serving_kernel(local_shape(w, rank, world), 0 if direction == "fwd" else 1, world=world)
+        if kind is None:
+            return "reduce kernel + exchange kernel + apply kernel (%s)" % direction
+        return "%s<%s> (%s)" % (KERNEL_NAMES[kind][0], direction, KERNEL_NAMES[kind][1])
     line = {
         "metric": "bn_relu_fwd_bwd_elements_per_s", "value": main_res["value"], "unit": "elements/s",
         "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": main_res["ms_per_step"],
@@ -606,7 +607,9 @@ def main():
                    "sharded_axis": w["axis"], "layout": "NCHW f32, eps=1e-5, avg_rate=0.1, gamma/beta, ReLU",
                    "l2": "inputs larger than L2 (no flush needed)" if main_res["elements_local"] * 4 > 512e6 else "inputs near L2 size",
                    "parallelism": "syncbn_dp%d" % world,
-                   "exchange": "none" if world == 1 else ("in-kernel peer stores" if main_res["launches_per_step"] == 2 else "nccl all-gather")},
+                   "exchange": "none" if world == 1 else ("nccl all-gather" if not main_res["exchange"] else
+                                                          "in-kernel peer stores" if main_res["launches_per_step"] == 2 else
+                                                          "peer stores (in the kernel, or in a kernel of their own)")},
         "per_gpu_value": main_res["value"] / world,
         "fwd_ms": main_res["fwd_ms"], "bwd_ms": main_res["bwd_ms"],
         "roofline": dict(roof(BYTES_BWD, main_res["bwd_ms"]), kernel=kernel_name("bwd")),
