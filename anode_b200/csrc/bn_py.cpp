@@ -6,13 +6,28 @@
 //
 // Arguments mirror anode_b200/ops.py, which keeps the public signatures, defaults and error types.
 // torch reports some conditions by C++ exceptions (no driver, a tensor without storage inside a function transform, a
-// sparse one): every function turns them into Python errors (HANDLE_TH_ERRORS), and nothing is asked of torch or CUDA once
+// sparse one): every function turns them into Python errors (GUARDED), and nothing is asked of torch or CUDA once
 // an argument was refused.
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <c10/cuda/CUDAStream.h>
 
 #include <stdint.h>
+
+#include <exception>
+
+// Exceptions become Python errors by torch's own translation, which runs only when there is one: HANDLE_TH_ERRORS around
+// every call would set up a buffer for C++ warnings each time.
+namespace {
+PyObject *translated(std::exception_ptr e)
+{
+  HANDLE_TH_ERRORS
+  std::rethrow_exception(e);
+  END_HANDLE_TH_ERRORS
+}
+}  // namespace
+#define GUARDED try {
+#define END_GUARDED } catch (...) { return translated(std::current_exception()); }
 
 namespace {
 
@@ -116,15 +131,21 @@ struct Args {
     if (!t) return;
     const int64_t nd = t->dim();
     if (axes >= 0 && v[axes] != Py_None) {
-      // any iterable whose items equal 0, 1, ...
-      PyObject *got = PySequence_List(v[axes]), *want = got ? PyList_New(0) : nullptr;
-      int same = want ? 1 : -1;
-      for (int64_t k = 0; same > 0 && k + 2 < nd; ++k) {
+      // any iterable whose items equal 0, 1, ...; the usual list of integers without making another one
+      bool usual = PyList_CheckExact(v[axes]) && PyList_GET_SIZE(v[axes]) == (nd > 2 ? nd - 2 : 0);
+      for (Py_ssize_t k = 0; usual && k + 2 < nd; ++k) {
+        PyObject *e = PyList_GET_ITEM(v[axes], k);
+        usual = PyLong_CheckExact(e) && PyLong_AsLong(e) == (long)k;
+        if (PyErr_Occurred()) PyErr_Clear();      // (an integer beyond a long)
+      }
+      PyObject *got = usual ? nullptr : PySequence_List(v[axes]), *want = got ? PyList_New(0) : nullptr;
+      int same = usual ? 2 : want ? 1 : -1;
+      for (int64_t k = 0; same == 1 && k + 2 < nd; ++k) {
         PyObject *e = PyLong_FromLongLong(k);
         if (!e || PyList_Append(want, e)) same = -1;
         Py_XDECREF(e);
       }
-      if (same > 0) same = PyObject_RichCompareBool(got, want, Py_EQ);
+      if (same == 1) same = PyObject_RichCompareBool(got, want, Py_EQ);
       if (same == 0) PyErr_Format(PyExc_ValueError, "axes must be %R for a %d-D batch array", want, (int)(nd - 2));
       Py_XDECREF(got); Py_XDECREF(want);
       if (same <= 0) { ok = false; return; }
@@ -153,7 +174,7 @@ const KernelConfig kDefaultCfg = {1024, 148 * 32};     // ops.py's default launc
 // fwd(axes, epsilon, avg_rate, x, residual, y, mean, var, avg_mean, avg_var, gamma, beta, relu, neg_slope | None, ws, ws_bytes, stream)
 PyObject *py_fwd(PyObject *, PyObject *const *v, Py_ssize_t n)
 {
-  HANDLE_TH_ERRORS
+  GUARDED
   if (!want_args(n, 17)) return nullptr;
   Args a{v};
   uint32_t d[3] = {0, 0, 0};
@@ -178,13 +199,13 @@ PyObject *py_fwd(PyObject *, PyObject *const *v, Py_ssize_t n)
     else rc = ((FwdFn)g_fn[which])(d[0], d[1], d[2], eps, rate, relu, x, gamma, beta, y, mean, var, rm, rv, ws, bytes, &kDefaultCfg, s);
   }
   return PyLong_FromLong(rc);
-  END_HANDLE_TH_ERRORS
+  END_GUARDED
 }
 
 // bwd(axes, dy, x, y | None, mean, var, dx, dresidual, gamma, beta, dgamma, dbeta, relu, neg_slope | None, accumulate, ws, ws_bytes, stream)
 PyObject *py_bwd(PyObject *, PyObject *const *v, Py_ssize_t n)
 {
-  HANDLE_TH_ERRORS
+  GUARDED
   if (!want_args(n, 18)) return nullptr;
   Args a{v};
   uint32_t d[3] = {0, 0, 0};
@@ -208,13 +229,13 @@ PyObject *py_bwd(PyObject *, PyObject *const *v, Py_ssize_t n)
     else rc = ((BwdFn)g_fn[which])(d[0], d[1], d[2], relu, acc, dy, x, mean, var, gamma, beta, dx, dg, db, ws, bytes, &kDefaultCfg, s);
   }
   return PyLong_FromLong(rc);
-  END_HANDLE_TH_ERRORS
+  END_GUARDED
 }
 
 // infer(axes, x, mean, var, y, gamma, beta, neg_slope, stream)
 PyObject *py_infer(PyObject *, PyObject *const *v, Py_ssize_t n)
 {
-  HANDLE_TH_ERRORS
+  GUARDED
   if (!want_args(n, 9)) return nullptr;
   Args a{v};
   uint32_t d[3] = {0, 0, 0};
@@ -230,7 +251,7 @@ PyObject *py_infer(PyObject *, PyObject *const *v, Py_ssize_t n)
     rc = ((InferFn)g_fn[F_INFER])(d[0], d[1], d[2], slope, x, mean, var, gamma, beta, y, &kDefaultCfg, s);
   }
   return PyLong_FromLong(rc);
-  END_HANDLE_TH_ERRORS
+  END_GUARDED
 }
 
 // The tensors of one of the reference's own entry points: `lo` to `hi` of them, all required (these entry points have no
@@ -264,7 +285,7 @@ typedef const KernelConfig *K;
 // flat(address, tensors, stream): element count (of the first tensor) and 2 or 3 arrays
 PyObject *py_flat(PyObject *, PyObject *const *v, Py_ssize_t n)
 {
-  HANDLE_TH_ERRORS
+  GUARDED
   if (!want_args(n, 3)) return nullptr;
   void *fn = PyLong_AsVoidPtr(v[0]);
   if (PyErr_Occurred()) return nullptr;
@@ -281,13 +302,13 @@ PyObject *py_flat(PyObject *, PyObject *const *v, Py_ssize_t n)
     else ((void (*)(uint32_t, P, P, P, K, P))fn)(len, q.p[0], q.p[1], q.p[2], cfg, s);
   }
   Py_RETURN_NONE;
-  END_HANDLE_TH_ERRORS
+  END_GUARDED
 }
 
 // packed(address, axes, like, tensors, stream): the dimensions of `like` and 2 to 5 arrays
 PyObject *py_packed(PyObject *, PyObject *const *v, Py_ssize_t n)
 {
-  HANDLE_TH_ERRORS
+  GUARDED
   if (!want_args(n, 5)) return nullptr;
   void *fn = PyLong_AsVoidPtr(v[0]);
   if (PyErr_Occurred()) return nullptr;
@@ -307,13 +328,13 @@ PyObject *py_packed(PyObject *, PyObject *const *v, Py_ssize_t n)
     else ((void (*)(uint32_t, uint32_t, uint32_t, P, P, P, P, P, K, P))fn)(d[0], d[1], d[2], q.p[0], q.p[1], q.p[2], q.p[3], q.p[4], cfg, s);
   }
   Py_RETURN_NONE;
-  END_HANDLE_TH_ERRORS
+  END_GUARDED
 }
 
 // packed_eps(address, axes, like, tensors, epsilon, stream): the dimensions of `like`, epsilon and 3 arrays
 PyObject *py_packed_eps(PyObject *, PyObject *const *v, Py_ssize_t n)
 {
-  HANDLE_TH_ERRORS
+  GUARDED
   if (!want_args(n, 6)) return nullptr;
   void *fn = PyLong_AsVoidPtr(v[0]);
   if (PyErr_Occurred()) return nullptr;
@@ -330,13 +351,13 @@ PyObject *py_packed_eps(PyObject *, PyObject *const *v, Py_ssize_t n)
     ((void (*)(uint32_t, uint32_t, uint32_t, float, P, P, P, K, P))fn)(d[0], d[1], d[2], eps, q.p[0], q.p[1], q.p[2], &kDefaultCfg, s);
   }
   Py_RETURN_NONE;
-  END_HANDLE_TH_ERRORS
+  END_GUARDED
 }
 
 // bind({name: address}): the C ABI's functions
 PyObject *py_bind(PyObject *, PyObject *const *v, Py_ssize_t n)
 {
-  HANDLE_TH_ERRORS
+  GUARDED
   if (!want_args(n, 1)) return nullptr;
   for (int i = 0; i < F_COUNT; ++i) {
     PyObject *e = PyDict_GetItemString(v[0], kNames[i]);
@@ -345,7 +366,7 @@ PyObject *py_bind(PyObject *, PyObject *const *v, Py_ssize_t n)
     if (PyErr_Occurred()) return nullptr;
   }
   Py_RETURN_NONE;
-  END_HANDLE_TH_ERRORS
+  END_GUARDED
 }
 
 PyMethodDef kMethods[] = {
