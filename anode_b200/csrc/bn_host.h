@@ -46,6 +46,7 @@ int launch_best(FusedArgs &a, int dir, bool aligned, cudaStream_t stream);
 int kernel_choice();
 // the cluster kernel for short rows (bn_segres.cu)
 bool segres_applies(const FusedArgs &a, int dir, bool aligned);
+uint32_t segres_blocks(const FusedArgs &a, int dir, bool aligned);     // blocks of its launch, 0 where it does not apply
 bool segres_preferred(const FusedArgs &a, int dir, bool aligned);      // take it even where the tiled kernel applies
 int launch_segres(FusedArgs &a, int dir, cudaStream_t stream);
 // the register-resident kernel (bn_chan.cu); one GPU, any alignment
@@ -54,6 +55,7 @@ bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok);
 int launch_chan(FusedArgs &a, int dir, bool aligned, cudaStream_t stream);
 // the streaming cluster kernel for large layers of short rows (bn_stream.cu); one GPU
 bool stream_applies(const FusedArgs &a, int dir, bool aligned);
+uint32_t stream_cluster(const FusedArgs &a, int dir, bool aligned);
 bool stream_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok);
 int launch_stream(FusedArgs &a, int dir, cudaStream_t stream);
 uint64_t workspace_part_bytes(uint32_t dim0, uint32_t C, uint32_t N);

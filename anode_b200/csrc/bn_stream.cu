@@ -299,16 +299,21 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamBlocks) bn_stream_kerne
 // for its slowest block and leaves more SMs without a place for a whole cluster: [1024,2048,7,7] takes 199 / 343 us
 // with 64 MB (clusters of 8 / 16), 180 / 298 with 96 MB (4 / 8) and the same with 128 MB.
 constexpr uint64_t kStreamWindow = 96ull << 20;
+constexpr uint64_t kStreamSplit = 72ull << 20;
 
 static bool stream_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, StreamGeom &g)
 {
   if (dim0 < 4 || (uint64_t)C * dim0 % 4 != 0) return false;
   uint32_t q = 4; if (dim0 % 2 == 0) q = 2; if (dim0 % 4 == 0) q = 1;      // cb*dim0 must be a multiple of 4
-  // runs of at least 512 bytes, then the channel count that leaves the fewest of the block's threads without a column
+  // runs of at least 512 bytes, then the channel count that leaves the fewest of a block's threads without a column, as
+  // long as there are units for a block at every place of the device (of runs up to a kilobyte, for some 64 blocks)
+  // (forward / backward, us, with the fewest idle threads alone and now: [6688,120,11] 32 and 160 blocks, 151 / 350 and
+  // 22 / 37; [724,524,11] 96 and 352, 24 / 41 and 10 / 14)
   uint32_t best = 0, best_used = 0;
   for (uint32_t cb = q; cb <= C && cb <= kStreamChannels && (uint64_t)cb * dim0 <= 4 * kStreamThreads; cb += q) {
     const uint32_t L4 = cb * dim0 / 4, used = kStreamThreads / L4 * L4;
-    if (best * dim0 >= 128 && used * 16 <= best_used * 17) continue;
+    if (best * dim0 >= 128 && (used * 16 <= best_used * 17 ||
+                               ceil_div_u32(C, cb) * 16 < (cb * dim0 <= 256 ? 64u : kStreamBlocks * sm_count()))) continue;
     best = cb; best_used = used;
   }
   if (!best) return false;
@@ -316,16 +321,29 @@ static bool stream_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, StreamGe
   g.cb = best; g.units = ceil_div_u32(C, best);
   g.groups = kStreamThreads / L4; if (g.groups > N) g.groups = N;
   const uint64_t unit_bytes = 16ull * L4 * N * (dir == 1 ? 2 : 1);
+  // Large layers: clusters that keep to the window.  Small ones: as many blocks as are resident at once, a few more at
+  // most, and four samples per thread at least; a second wave only repeats each block's fixed steps: [43,832,183] 1664
+  // blocks and 416, 19.3 / 25.7 us and 12.7 / 18.2; [995,1892,6] 1264 and 316, 38 / 54 and 21 / 41.  (Backward passes over
+  // more than 72 MB gain by what a second or third wave takes out of L2's way: [264,968,37] one wave 34.7 us, two 31.8.)
+  const uint32_t wave = kStreamBlocks * sm_count();
+  const bool split = dir == 1 && unit_bytes * g.units > kStreamSplit;
+  const uint32_t most = split ? 3 * wave : wave * 8 / 7, least = split ? 9 : 4;
   uint32_t cl = 1;
   while (cl < 16 && cl * 2 * g.cb <= kStreamRecords &&
-         ((uint64_t)kStreamBlocks * sm_count() * unit_bytes / cl > kStreamWindow ||
-          (g.units * cl < 2 * kStreamBlocks * sm_count() && N / (cl * 2) >= g.groups * 4))) cl *= 2;
+         (wave * unit_bytes / cl > kStreamWindow || (g.units * cl * 2 <= most && N / (cl * 2) >= g.groups * least))) cl *= 2;
   g.cluster = cl;
   g.rows = ceil_div_u32(N, cl);
   if (g.groups > g.rows) g.groups = g.rows;
   g.threads = (g.groups * L4 + 31) / 32 * 32;
   g.inv_count = 1.0 / ((double)dim0 * (double)N);
   return true;
+}
+
+// Blocks of a cluster for this call; 0 where the kernel does not apply.
+uint32_t stream_cluster(const FusedArgs &a, int dir, bool aligned)
+{
+  StreamGeom g;
+  return stream_applies(a, dir, aligned) && stream_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, g) ? g.cluster : 0u;
 }
 
 bool stream_applies(const FusedArgs &a, int dir, bool aligned)
@@ -341,12 +359,23 @@ bool stream_applies(const FusedArgs &a, int dir, bool aligned)
 // 56 / 101, [256,256,28,28] 97 / 162 and 84 / 158; residual [256,256,28,28] 138 / 221 and 135 / 232, [1024,64,28,28]
 // 162 / 249 and 132 / 218.
 constexpr uint32_t kStreamShortRow = 512, kStreamMediumRow = 600, kStreamLongRow = 1024;
+// Layers of few channels leave the device to a few clusters whose threads walk hundreds of samples.  With rows that the
+// tiled kernel serves it is the faster one there, forward / backward, here and there: [7663,4,412] 47 / 119 and 31 / 54,
+// [5111,9,420] 54 / 102 and 43 / 77, but [4976,11,260] 43 / 76 and 43 / 78 (104 samples a thread), [295,122,588] 39 / 66
+// and 42 / 77 (74).  For odd rows below that the plain kernel is, in the residual epilogue's forward pass only:
+// [45953,8,21] 162 and 121, [17770,12,27] 94 and 72, [11845,12,73] 94 and 75, but [18431,12,37] 70 and 90 (192 samples),
+// [129340,8,10] 224 and 330, [57124,7,32] 167 and 189.
+constexpr uint32_t kStreamLongWalk = 112, kStreamFewBlocks = 48;
 bool stream_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
 {
   const uint32_t dim0 = a.plan.dim0;
-  if (!stream_applies(a, dir, aligned)) return false;
-  if (!tiled_ok || dim0 <= kStreamShortRow) return true;
+  StreamGeom g;
+  if (!stream_applies(a, dir, aligned) || !stream_geom(dim0, a.plan.C, a.plan.N, dir, g)) return false;
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
+  const uint32_t walk = ceil_div_u32(g.rows, g.groups), blocks = g.units * g.cluster;
+  if (tiled_ok && walk >= kStreamLongWalk) return false;
+  if (!tiled_ok && extra && dir == 0 && dim0 > 16 && dim0 % 4 != 0 && blocks <= kStreamFewBlocks && walk >= 2 * kStreamLongWalk) return false;
+  if (!tiled_ok || dim0 <= kStreamShortRow) return true;
   const uint64_t most = (extra ? 1u << 18 : dir == 1 ? 1u << 17 : 1u << 16) * (dim0 <= kStreamMediumRow ? 4ull : 1ull);
   return dim0 <= kStreamLongRow && (uint64_t)dim0 * a.plan.N <= most;
 }
@@ -392,3 +421,15 @@ int launch_stream(FusedArgs &a, int dir, cudaStream_t stream)
 }
 
 }  // namespace anode_b200
+
+// ---- diagnostics: geometry of the streaming kernel for a shape (no GPU needed) -----------------
+extern "C" int anode_gpu_batch_norm_stream_geometry(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, uint32_t *out)
+{
+  using namespace anode_b200;
+  if (!out || (dir != 0 && dir != 1) || check_dims(dim0, dim1, dim2)) return ANODE_E_DIMS;
+  StreamGeom g{};
+  const bool ok = stream_geom(dim0, dim1, dim2, dir, g);
+  const uint32_t v[7] = {ok ? 1u : 0u, g.cb, g.units, g.cluster, g.rows, g.groups, g.threads};
+  for (int i = 0; i < 7; ++i) out[i] = v[i];
+  return ANODE_OK;
+}

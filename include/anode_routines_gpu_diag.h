@@ -47,6 +47,10 @@ int anode_gpu_batch_norm_fused_plan_walk(uint32_t dim0, uint32_t dim1, uint32_t 
  * per block, units, shared-memory bytes. */
 int anode_gpu_batch_norm_segres_geometry(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, uint32_t *out);
 
+/* Geometry of the streaming kernel.  out (7 values): applies, channels per unit, units, blocks per cluster, samples per
+ * block, sample groups of a block, threads. */
+int anode_gpu_batch_norm_stream_geometry(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, uint32_t *out);
+
 /* Geometry of the tiled kernel (bn_ring.cuh) for direction `dir` of a fused call on 16-byte aligned tensors.
  * out (12 values): applies, rows per tile, floats per row piece, tiles per unit, slots, bytes per slot, dynamic
  * shared memory bytes, KiB between a tile's two visits (what L2 has to hold), the fraction (in 1/1000) of

@@ -1,4 +1,6 @@
 """Which kernel serves a call, and how many launches a synchronized step takes (no GPU needed)."""
+import ctypes
+
 import pytest
 import torch
 
@@ -63,3 +65,59 @@ def test_launches_of_a_synchronized_step(shape, launches):
     assert layer.launches_per_step == 6
     layer.comm = Comm(1, None)
     assert layer.launches_per_step == 2
+
+
+def routes(shape):
+    """Kernels of the plain forward and backward and of the residual epilogue's, on one GPU."""
+    return tuple(ops.serving_kernel(shape, d, residual=r) for r in (False, True) for d in (0, 1))
+
+
+STREAM_FIELDS = ["applies", "cb", "units", "cluster", "rows", "groups", "threads"]
+
+
+def stream_geometry(shape, direction):
+    d0, c, n = ops.dims_of(torch.empty(shape, device="meta"))
+    out = (ctypes.c_uint32 * 7)()
+    assert _lib.load().anode_gpu_batch_norm_stream_geometry(d0, c, n, direction, out) == 0
+    return dict(zip(STREAM_FIELDS, list(out)))
+
+
+@pytest.mark.parametrize("shape", [(1411, 128, 7, 7), (1500, 4, 7, 9), (4099, 16, 2, 2), (1025, 512, 4, 4), (40001, 8, 1, 5),
+                                   (6688, 120, 1, 11), (724, 524, 1, 11), (7663, 4, 1, 412), (333, 257, 12, 12), (3, 4, 3, 3),
+                                   (1, 4, 16, 16), (5, 128, 1, 4), (2048, 2048, 7, 7), (43, 832, 1, 183), (596, 1860, 1, 9)])
+def test_streaming_geometry(shape):
+    """Units of 16-byte aligned runs, clusters whose blocks cover the samples, records and columns that fit the block's."""
+    d0, c, n = ops.dims_of(torch.empty(shape, device="meta"))
+    for direction in (0, 1):
+        g = stream_geometry(shape, direction)
+        assert g["applies"] == 1
+        vectors = g["cb"] * d0 // 4
+        assert g["cb"] * d0 % 4 == 0 and g["cb"] <= 128 and g["cb"] * g["cluster"] <= 1024
+        assert g["units"] == -(-c // g["cb"])
+        assert g["cluster"] in (1, 2, 4, 8, 16) and g["cluster"] * g["rows"] >= n and g["rows"] <= n
+        assert 1 <= g["groups"] <= g["rows"] and g["groups"] * vectors <= g["threads"] <= 256
+    assert stream_geometry((9, 4, 1, 3), 0)["applies"] == 0            # rows of less than four floats
+    assert stream_geometry((9, 3, 1, 7), 0)["applies"] == 0            # no aligned run
+
+
+@pytest.mark.parametrize("shape,blocks", [((6688, 120, 1, 11), 160), ((3067, 108, 1, 22), 288), ((724, 524, 1, 11), 300), ((5879, 15, 1, 76), 100)])
+def test_layers_of_few_channels_are_split_into_enough_units(shape, blocks):
+    for direction in (0, 1):
+        g = stream_geometry(shape, direction)
+        assert g["units"] * g["cluster"] >= blocks, g
+
+
+@pytest.mark.parametrize("shape", [(43, 832, 1, 183), (230, 568, 1, 46), (454, 304, 1, 35), (995, 1892, 1, 6)])
+def test_small_layers_take_one_wave_of_blocks(shape):
+    g = stream_geometry(shape, 0)
+    assert g["units"] * g["cluster"] <= 3 * 148 * 8 // 7, g
+
+
+def test_routes_of_layers_that_the_streaming_kernel_leaves_to_others():
+    # few channels, hundreds of samples a thread: the tiled kernel where it can, for odd rows the plain one in one pass
+    assert routes((7663, 4, 1, 412)) == ("tiled",) * 4
+    assert routes((5111, 9, 1, 420)) == ("tiled",) * 4
+    assert routes((4976, 11, 1, 260)) == ("stream",) * 4
+    assert routes((17770, 12, 1, 27)) == ("stream", "stream", "plain", "stream")
+    assert routes((18431, 12, 1, 37)) == ("stream",) * 4
+    assert routes((57124, 7, 1, 32)) == ("stream",) * 4
