@@ -274,10 +274,20 @@ bool chan_applies(const FusedArgs &a, int dir, bool aligned)
 // Forward + backward at the places of other kernels, there and here: [2,512,7,7] 11.5 -> 4.5 us, [32,64,28,28] 20.7 ->
 // 9.8, [1,53,39,25] 17.9 -> 5.2, [1,260,128,128] 34.0 -> 16.7, [1,1240,45,30] 60.5 -> 13.8, [40,2048,146,5] 630 -> 413.
 // The other way round, us here and there: streaming kernel, forward [512,1024,14,14] 213 and 185, backward
-// [256,1024,14,14] 164 and 147, residual epilogue 156 / 222 and 137 / 209; [64,2048,7,7] 19.0 / 25.5 and 15.0 / 20.4,
+// [256,1024,14,14] 164 and 147, residual epilogue 156 / 222 and 137 / 209; [64,2048,7,7] 19.0 / 25.5 and 13.4 / 20.2,
 // but [300,100,7,7] 5.9 / 8.6 and 6.7 / 8.3.  Tiled kernel, forward [128,512,28,28] 105 and 87, [39,255,45,45] 62 and
 // 44, but [349,255,15,15] 64 and 68, [45,33,45,45] 12.9 and 15.5.
-constexpr uint64_t kChanLarge = 8u << 20, kChanLargeScalar = 3u << 20;      // elements from which on the others are asked
+// Elements from which on the others are asked (rows without aligned runs of several channels, residual backward, on the
+// tiled kernel: [26,551,431], 6.2 M, 57 and 47; [15,528,631], 5.0 M, 39 and 41).  Scalar rows with such runs go earlier where
+// the teams take more than one wave of blocks, so that their load, exchange and store come twice: backward passes and the
+// residual epilogue, us here and on the streaming kernel: residual backward [103,304,53] 15.2 and 8.8, residual forward
+// [115,704,29] 11.8 and 7.4, backward [230,384,31] 13.7 and 8.8; but one wave, backward [19,728,145] 8.0 and 9.4, few
+// samples, [15,1516,130] 10.8 and 12.5, clusters of sixteen, [336,212,29] 8.7 and 12.9.  Rows of 1 - 3 floats, which the
+// threads fetch from far apart, on the shared-memory kernel: [1024,512,3] residual backward 25.8 and 18.5, [1540,632,2]
+// backward 24.4 and 18.7, [1457,828,1] residual forward 23.6 and 20.6.
+constexpr uint64_t kChanLarge = 8u << 20, kChanLargeScalar = 3u << 20, kChanLargeExtra = 5u << 20;
+constexpr uint64_t kChanWaves = 1500000, kChanShortest = 1200000;
+constexpr uint32_t kChanFewSamples = 32;
 constexpr uint32_t kChanLongRow = 300;
 bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
 {
@@ -291,9 +301,20 @@ bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
     if (elements < kChanLarge || channel <= (uint64_t)kChanThreads * kChanCluster * most / 2) return true;
     return !stream_preferred(a, dir, aligned, tiled_ok) && !(dir == 0 && !extra && tiled_ok);
   }
-  if (elements < kChanLargeScalar) return true;
+  if (elements < kChanLargeScalar) {
+    if ((dir == 0 && !extra) || elements < kChanShortest) return true;
+    if (a.plan.dim0 < 4) {
+      const uint32_t blocks = segres_blocks(a, dir, aligned);
+      return blocks == 0 || blocks > 2 * sm_count();
+    }
+    const uint64_t places = (uint64_t)sm_count() * (2 * kChanThreads / g.threads);
+    if (elements < kChanWaves || a.plan.N < kChanFewSamples || (uint64_t)a.plan.C * g.cluster <= places) return true;
+    const uint32_t cluster = stream_cluster(a, dir, aligned);
+    return cluster == 0 || cluster > 8;
+  }
   if (stream_preferred(a, dir, aligned, tiled_ok)) return false;
-  return elements < kChanLarge || !(segres_applies(a, dir, aligned) || (tiled_ok && a.plan.dim0 >= kChanLongRow));
+  if (elements >= kChanLarge && segres_applies(a, dir, aligned)) return false;
+  return elements < (extra && dir == 1 ? kChanLargeExtra : kChanLarge) || !(tiled_ok && a.plan.dim0 >= kChanLongRow);
 }
 
 int launch_chan(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)

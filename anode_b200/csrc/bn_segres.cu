@@ -448,6 +448,13 @@ bool segres_applies(const FusedArgs &a, int dir, bool aligned)
   return aligned && a.mode == MODE_FUSED && seg_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, extra, g);
 }
 
+uint32_t segres_blocks(const FusedArgs &a, int dir, bool aligned)
+{
+  SegGeom g;
+  const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
+  return segres_applies(a, dir, aligned) && seg_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, extra, g) ? g.units * g.cluster : 0u;
+}
+
 // Launches the segments kernel for a prepared call.  ANODE_E_LAUNCH when the device refuses the
 // cluster shape (the caller falls back to the plain kernel).
 int launch_segres(FusedArgs &a, int dir, cudaStream_t stream)

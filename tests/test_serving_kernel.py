@@ -121,3 +121,22 @@ def test_routes_of_layers_that_the_streaming_kernel_leaves_to_others():
     assert routes((17770, 12, 1, 27)) == ("stream", "stream", "plain", "stream")
     assert routes((18431, 12, 1, 37)) == ("stream",) * 4
     assert routes((57124, 7, 1, 32)) == ("stream",) * 4
+
+
+def test_routes_of_scalar_rows_between_the_register_resident_kernel_and_the_others():
+    reg = "register"
+    # teams of more than one wave of blocks: backward passes and the residual epilogue go to the streaming kernel
+    assert routes((103, 304, 1, 53)) == (reg, "stream", "stream", "stream")
+    assert routes((115, 704, 1, 29)) == (reg, "stream", "stream", "stream")
+    # one wave, few samples, or clusters of sixteen there: they stay
+    assert routes((19, 728, 1, 145)) == (reg,) * 4
+    assert routes((15, 1516, 1, 130)) == (reg,) * 4
+    assert routes((336, 212, 1, 29)) == (reg,) * 4
+    # rows of 1 - 3 floats: the shared-memory kernel where its blocks are resident at once
+    assert routes((1024, 512, 1, 3))[0] == reg and routes((1024, 512, 1, 3))[2] == "cluster"
+    assert routes((256, 1000, 1, 1)) == (reg,) * 4
+    # rows without an aligned run: the residual epilogue's backward pass goes to the tiled kernel earlier
+    assert routes((26, 551, 1, 431)) == (reg, reg, reg, "tiled")
+    # small layers
+    for shape in ((2, 512, 7, 7), (32, 64, 28, 28), (1, 53, 39, 25), (1, 260, 128, 128)):
+        assert routes(shape) == (reg,) * 4
