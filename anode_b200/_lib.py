@@ -145,10 +145,14 @@ def native():
     global _native
     if _native is None:
         load()
+        from .build import native_built_for
         try:
             from . import _native as module
         except ImportError as e:
-            raise ImportError("anode_b200/_native.so is not built: run `python -m anode_b200.build` (%s)" % e)
+            raise ImportError("anode_b200/_native.so is missing or not loadable: run `python -m anode_b200.build` (%s)" % e)
+        if module.built_for != native_built_for():
+            raise ImportError("anode_b200/_native.so was %s, this is %s: run `python -m anode_b200.build`"
+                              % (module.built_for, native_built_for()))
         module.bind({name: address(name) for name in SIGNATURES})
         _native = module
     return _native

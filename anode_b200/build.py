@@ -51,17 +51,34 @@ def _stale():
     return any(os.path.exists(d) and os.path.getmtime(d) > t for d in deps)
 
 
-def build_native(force=False):
-    """The CPython module anode_b200._native: compiled against this interpreter's and torch's headers, linked against
-    torch only (the C ABI is handed to it as addresses at run time)."""
-    if not force and os.path.exists(NATIVE) and os.path.getmtime(NATIVE) > os.path.getmtime(NATIVE_SOURCE):
-        return NATIVE
+def native_built_for():
+    """What a build of the native module is bound to: this interpreter's ABI and this torch."""
     import sysconfig
     import torch
+    return "built for %s, torch %s" % (sysconfig.get_config_var("SOABI"), torch.__version__)
+
+
+def native_is_current(path, source, built_for):
+    """Whether the module at `path` is newer than its source and this file, and was built for `built_for` (the text is
+    compiled into it)."""
+    if not os.path.exists(path) or any(os.path.getmtime(path) <= os.path.getmtime(f) for f in (source, os.path.abspath(__file__))):
+        return False
+    with open(path, "rb") as f:
+        return built_for.encode() + b"\0" in f.read()
+
+
+def build_native(force=False):
+    """The CPython module anode_b200._native: compiled against this interpreter's and torch's headers, linked against
+    torch only (the C ABI is handed to it as addresses at run time).  Built again after a change of either."""
+    import sysconfig
+    import torch
+    built_for = native_built_for()
+    if not force and native_is_current(NATIVE, NATIVE_SOURCE, built_for):
+        return NATIVE
     root = os.path.dirname(torch.__file__)
     tmp = NATIVE + ".tmp%d" % os.getpid()
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
-           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI), '-DANODE_BUILT_FOR="%s"' % built_for,
            "-I", os.path.join(root, "include"), "-I", os.path.join(root, "include", "torch", "csrc", "api", "include"),
            "-I", os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include"), "-I", sysconfig.get_paths()["include"],
            NATIVE_SOURCE, "-o", tmp, "-L", os.path.join(root, "lib"),

@@ -382,4 +382,9 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", "Fast paths of anode_b2
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__native(void) { return PyModule_Create(&kModule); }
+PyMODINIT_FUNC PyInit__native(void)
+{
+  PyObject *m = PyModule_Create(&kModule);
+  if (m && PyModule_AddStringConstant(m, "built_for", ANODE_BUILT_FOR) < 0) { Py_DECREF(m); return nullptr; }
+  return m;
+}

@@ -5,7 +5,7 @@ import pytest
 import torch
 from torch._subclasses.fake_tensor import FakeTensorMode
 
-from anode_b200 import ops
+from anode_b200 import _lib, build, ops
 
 
 class Scratch:
@@ -136,3 +136,14 @@ def test_the_residual_epilogue_has_a_slope():
         ops.BatchNormalize2dAddActFusedOp.apply([0, 1], 1e-5, 0.1, x, x, x, v, v, neg_slope=None, workspace=Scratch())
     with pytest.raises(TypeError):
         ops.BatchNormalize2dAddActFusedOp.adjoint([0, 1], x, x, x, v, v, x, neg_slope=None, workspace=Scratch())
+
+
+def test_the_module_is_bound_to_this_interpreter_and_torch(tmp_path, monkeypatch):
+    assert _lib.native().built_for == build.native_built_for()
+    assert build.native_is_current(build.NATIVE, build.NATIVE_SOURCE, build.native_built_for())
+    assert not build.native_is_current(build.NATIVE, build.NATIVE_SOURCE, "built for cpython-311, torch 2.0")     # built again
+    assert not build.native_is_current(str(tmp_path / "missing.so"), build.NATIVE_SOURCE, build.native_built_for())
+    monkeypatch.setattr(build, "native_built_for", lambda: "built for cpython-311, torch 2.0")
+    monkeypatch.setattr(_lib, "_native", None)
+    with pytest.raises(ImportError, match="built for cpython-311"):        # and not used in the meantime
+        _lib.native()
