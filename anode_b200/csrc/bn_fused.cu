@@ -15,7 +15,7 @@
 
 namespace anode_b200 {
 
-// Ragged rows (a length that is no multiple of four floats): the shortest one the tiled kernel takes, forward and
+// Ragged rows (a length that is no multiple of four floats): the shortest one the tiled kernel can take, forward and
 // backward.  A row costs the producer a bulk copy per tensor, so below some length the plain kernel's 4-byte accesses
 // are the faster form.  20 M elements, 33 channels, forward / backward in us, tiled against plain: 9 x 9 144 / 270
 // against 116 / 160, 11 x 11 105 / 195 (116 / 161), 13 x 13 82 / 150 (116 / 161), 25 x 25 45 / 79 (117 / 160),
@@ -150,6 +150,7 @@ static bool ring_plan_with(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool 
   // short rows (regime S) belong to the cluster kernel or the plain kernel
   if (p.regime != 0) return false;
   if (ragged) {
+    p.rows_per_tile = ceil_div_u32(N, p.sample_blocks);      // (equal tiles: the last one would hold what is left over)
     const uint32_t per_row = ragged_pitch(p.piece_len < dim0 ? p.piece_len : dim0);
     p.vec = 4;
     p.div_mul = (uint32_t)((1ull << 32) / per_row) + 1;
@@ -230,6 +231,18 @@ uint64_t ring_ws_bytes(const FusedArgs &a, int dir, bool aligned)
 {
   Plan p; RingGeom g;
   return ring_plan_of(a, dir, aligned, p, g) ? p.ws_bytes : 0;
+}
+
+// Whether the tiled kernel, which can serve the call, is the faster form.  Not for the residual epilogue on ragged rows below
+// these lengths (forward, backward), us here and on the plain kernel: forward [2123,21,139] 51 and 48, but [998,17,145] 25
+// and 36; backward [1841,15,165] 60 and 47, [177,77,183] 39 and 36, but [966,13,191] 31 and 35.
+// (On large layers of long aligned rows that leave much of a slot empty the plain kernel would be the faster form of the
+// residual forward pass, [118,100,3516] 190 and 141, but its partials lie over the tagged words that an ordinary call of the
+// tiled kernel keeps in the same workspace.  A ragged plan's words lie apart.)
+constexpr uint32_t kRaggedMinRowExtra[2] = {144, 184};
+static bool tiled_preferred(const FusedArgs &a, int dir)
+{
+  return !(a.res || a.ymask || a.dres) || a.plan.dim0 % 4 == 0 || a.plan.dim0 >= kRaggedMinRowExtra[dir];
 }
 
 typedef void (*RingKernel)(const FusedArgs, const RingGeom);
@@ -365,7 +378,7 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
   const bool extra = a.res || a.ymask || a.dres;        // residual epilogue
   const bool plain_ok = !(a.mode == MODE_FUSED && a.world > 1);
   Plan rp; RingGeom g;
-  const bool tiled_ok = ring_plan_of(a, dir, aligned, rp, g);
+  const bool tiled_ok = ring_plan_of(a, dir, aligned, rp, g) && (kernel_choice() != ANODE_KERNEL_AUTO || tiled_preferred(a, dir));
   switch (kernel_choice()) {
     case ANODE_KERNEL_TILED: if (tiled_ok) return ANODE_KERNEL_TILED; break;
     case ANODE_KERNEL_CLUSTER: if (segres_applies(a, dir, aligned)) return ANODE_KERNEL_CLUSTER; break;

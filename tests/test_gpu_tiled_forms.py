@@ -70,6 +70,14 @@ def test_outputs_over_inputs(tiled, shape, form):
     outputs_over_inputs(tiled, shape, form, "tiled")
 
 
+@pytest.mark.parametrize("shape", [(1841, 15, 1, 165), (2123, 21, 1, 139)])
+def test_plain_and_tiled_calls_share_a_workspace(shape):
+    """Ragged rows whose residual epilogue goes to the plain kernel while the ordinary calls are the tiled one's."""
+    from anode_b200 import ops
+    assert [ops.serving_kernel(shape, 1, residual=r) for r in (False, True)] == [("tiled" if shape[3] > 160 else "plain"), "plain"]
+    outputs_over_inputs(ops, shape, "separate", "auto")
+
+
 def outputs_over_inputs(ops, shape, form, kernel_name):
     d = make_inputs(shape, seed=3, loc=0.5, scale=2.0)
     y_h = np.maximum(np.random.default_rng(4).standard_normal(shape), 0).astype(np.float32)

@@ -140,3 +140,23 @@ def test_routes_of_scalar_rows_between_the_register_resident_kernel_and_the_othe
     # small layers
     for shape in ((2, 512, 7, 7), (32, 64, 28, 28), (1, 53, 39, 25), (1, 260, 128, 128)):
         assert routes(shape) == (reg,) * 4
+
+
+def test_routes_of_the_residual_epilogue_on_long_rows():
+    for shape in ((256, 256, 56, 56), (331, 19, 1, 4392), (126, 16, 1, 3776), (256, 64, 56, 56)):
+        assert routes(shape)[2:] == ("tiled", "tiled"), shape
+    # ragged rows below which the plain kernel is the faster form
+    assert routes((2123, 21, 1, 139))[2:] == ("plain", "plain")
+    assert routes((1841, 15, 1, 165)) == ("tiled", "tiled", "tiled", "plain")
+    assert routes((966, 13, 1, 191)) == ("tiled",) * 4
+
+
+def test_ragged_tiles_hold_equally_many_rows():
+    lib = _lib.load()
+    for d0, c, n in ((131, 106, 846), (135, 210, 371), (3025, 95, 64), (1001, 7, 50)):
+        for direction in (0, 1):
+            out = (ctypes.c_uint32 * 12)()
+            assert lib.anode_gpu_batch_norm_tiled_geometry(d0, c, n, direction, out) == 0
+            if out[0] and out[2] >= d0:
+                tiles = -(-n // out[1])
+                assert out[3] == tiles and n - (tiles - 1) * out[1] > out[1] - tiles, (d0, c, n, list(out))
