@@ -7,8 +7,8 @@
 //   elementwise kernels      128-bit grid-stride loops; the channel of a vector comes from one
 //                            division per four elements instead of two per element
 //
-// What bounds them on layers of a few 10 MB: L2 and the gaps between launches.  The composition of thirteen of them on
-// [64,128,28,28] took 134 us with a 64-bit division per vector, two loads in flight in the reductions and ordinary
+// What bounds them on layers of a few 10 MB: L2 and the gaps between launches.  The composition of eleven of them (and two
+// running averages and four fills) on [64,128,28,28] took 134 us with a 64-bit division per vector, two loads in flight in the reductions and ordinary
 // launches, 115 us with none (32-bit ones in the maps), four, and launches that overlap the tail of the one before.
 //
 // Expressions are kept term for term as the reference writes them (e.g. rsqrtf, the

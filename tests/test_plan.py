@@ -122,9 +122,9 @@ def test_cluster_kernel_geometry_invariants():
             ok, cb, cluster, rows, units, smem = list(out)
             kind = lib.anode_gpu_batch_norm_fused_kernel_kind(d0, c, n, direction)
             if not ok:
-                assert kind in (1, 4)       # ANODE_KERNEL_TILED, ANODE_KERNEL_PLAIN
+                assert kind in (1, 4)       # the shape's family: ANODE_KERNEL_TILED, ANODE_KERNEL_PLAIN
                 continue
-            assert kind == 2                # ANODE_KERNEL_CLUSTER
+            assert kind == 2                # ANODE_KERNEL_CLUSTER (what is launched: tests/test_serving_kernel.py)
             assert (cb * d0) % 4 == 0 or cb == c
             assert cb * d0 <= 1024 and 1 <= cb <= max(c, 1)
             assert units == -(-c // cb)

@@ -1,10 +1,10 @@
 """The forward entry point that brings its own scratch (a fixed array inside the library, for
 callers that cannot allocate: anode's fixed op argument list has no workspace slot, and code
-inside a memory-pool transaction must not call cudaMalloc).  It is called through the C ABI on
-shapes served by kernels that really keep state in the array (the tiled and the plain kernel; the
-cluster kernel needs none), back to back and alternating, so that every call finds the leftovers of
-a different problem; each result is compared with the workspace-taking entry point on the same
-inputs and with the float64 oracle."""
+inside a memory-pool transaction must not call cudaMalloc).  It is called through the C ABI with every
+kernel forced that keeps state in the array (the tiled kernel with several plans, ragged rows among
+them, and the plain kernel in both its forms) and with the others in between, back to back and
+alternating, so that every call finds the leftovers of a different problem; each result is compared
+with the workspace-taking entry point on the same inputs and with the float64 oracle."""
 import ctypes
 
 import numpy as np
@@ -49,20 +49,27 @@ def run_both(lib, ops, d, eps, rate):
     return out
 
 
-def test_static_scratch_forward_matches_workspace_forward_and_oracle():
+def test_static_scratch_forward_matches_workspace_forward_and_oracle(request):
     from anode_b200 import _lib, ops
     lib = _lib.load()
     kind = lib.anode_gpu_batch_norm_fused_kernel_kind
     # tiled kernel, plain kernel, cluster kernel, and two more tiled problems with other tile plans
     shapes = [(16, 8, 56, 56), (5, 3, 7, 7), (16, 8, 28, 28), (64, 8, 56, 56), (8, 6, 112, 112)]
     served = {kind(*ops.dims_of(torch.empty(s, device="meta")), 0) for s in shapes}
-    assert {1, 2, 4} <= served, served          # ANODE_KERNEL_TILED, _CLUSTER, _PLAIN: two of them use the array
+    assert {1, 2, 4} <= served, served          # the families of these shapes; what runs is forced below
+    kernels = {(16, 8, 56, 56): "tiled", (5, 3, 7, 7): "plain", (16, 8, 28, 28): "cluster", (64, 8, 56, 56): "tiled",
+               (8, 6, 112, 112): "tiled", (9, 5, 55, 55): "tiled", (64, 96, 7, 7): "plain", (3, 512, 7, 7): "register",
+               (64, 16, 7, 7): "stream", (64, 8, 48, 48): "auto"}
+    shapes = list(kernels)
     data = {s: make_inputs(s, seed=51 + i, loc=0.5, scale=2.0) for i, s in enumerate(shapes)}
     truth = {s: o.bn_relu_fwd_bwd_f64(d["x"], d["dy"], 1e-5, 0.1, d["run_mean"], d["run_var"], d["gamma"], d["beta"])
              for s, d in data.items()}
     # each problem twice in a row, then all of them again: every call finds another plan's leftovers
+    request.addfinalizer(lambda: ops.set_kernel("auto"))
     for shape in shapes + shapes[::-1]:
         d = data[shape]
+        ops.set_kernel(kernels[shape])
+        assert kernels[shape] in ("auto", ops.serving_kernel(shape, 0)), shape
         for _ in range(2):
             out = run_both(lib, ops, d, 1e-5, 0.1)
             skip = borderline(truth[shape], d["x"], d["gamma"], d["beta"])
@@ -75,10 +82,11 @@ def test_static_scratch_forward_matches_workspace_forward_and_oracle():
 def test_static_scratch_rejects_problems_beyond_its_size():
     from anode_b200 import _lib
     lib = _lib.load()
-    # 4.2e9 elements in 256000 odd rows: the plain kernel serves it and keeps 32 bytes per tile in its
-    # scratch, twice the built-in 4 MiB (checked on the host first: the call must be refused, not run)
+    # 4.2e9 elements in 256000 odd rows: the tiled kernel serves them with a workspace, and neither its words nor
+    # the plain kernel's (32 bytes per tile, twice the built-in 4 MiB) fit the array (checked on the host first:
+    # the call must be refused, not run)
     d0, c, n = 16385, 256, 1000
-    assert lib.anode_gpu_batch_norm_fused_kernel_kind(d0, c, n, 0) == 4      # ANODE_KERNEL_PLAIN
+    assert lib.anode_gpu_batch_norm_fused_kernel_kind(d0, c, n, 0) == 4      # the family of ragged rows
     plan = (ctypes.c_uint32 * 15)()
     assert lib.anode_gpu_batch_norm_fused_plan(d0, c, n, 1, 0, 0, 0, plan, 15) == 0
     assert plan[13] + (plan[14] << 32) > (4 << 20)
