@@ -150,7 +150,9 @@ static bool ring_plan_with(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool 
   // short rows (regime S) belong to the cluster kernel or the plain kernel
   if (p.regime != 0) return false;
   if (ragged) {
-    p.rows_per_tile = ceil_div_u32(N, p.sample_blocks);      // (equal tiles: the last one would hold what is left over)
+    // Equal tiles: the last of a channel would hold what is left over and cost a step all the same.  Forward, before and
+    // now: [846,106,131] 67.8 and 61.8 us, [371,210,135] 65.8 and 55.5, [64,95,55,55] 41.9 and 42.0.
+    p.rows_per_tile = ceil_div_u32(N, p.sample_blocks);
     const uint32_t per_row = ragged_pitch(p.piece_len < dim0 ? p.piece_len : dim0);
     p.vec = 4;
     p.div_mul = (uint32_t)((1ull << 32) / per_row) + 1;
