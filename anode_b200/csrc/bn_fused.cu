@@ -112,8 +112,24 @@ static const ShapeInfo &shape_info(uint32_t dim0, uint32_t C, uint32_t N)
 
 Plan plan_for(uint32_t dim0, uint32_t C, uint32_t N, bool aligned16) { return shape_info(dim0, C, N).plan[aligned16 ? 1 : 0]; }
 
+constexpr uint32_t kRingSmemBudget = 227u * 1024u;      // a block's most
+
+// vectors that a row takes in a slot, and those of the largest tile
+static uint32_t ring_pitch(const Plan &p)
+{
+  const uint32_t len = p.piece_len < p.dim0 ? p.piece_len : p.dim0;
+  return p.dim0 % 4 != 0 ? ragged_pitch(len) : len / 4;
+}
+static uint32_t ring_tile_vecs(const Plan &p) { return p.rows_per_tile * ring_pitch(p); }
+
 // consumer warps of direction `dir` (the two instantiations of bn_ring.cuh)
 static uint32_t ring_warps(int dir) { return dir == 0 ? 8u : 16u; }
+
+// Fused mode: the tiles that stay in tensor memory.
+static void ring_keep(const Plan &p, int dir, RingGeom &g)
+{
+  plan_keep(g, ring_tile_vecs(p), dir == 1 ? 2u : 1u, ring_warps(dir), p.lookahead_steps);
+}
 
 // Shared-memory layout of the warp-specialised kernel for plan `p` (see bn_ring.cuh).
 static RingGeom ring_geom(const Plan &p, int dir, bool extra, uint32_t slots, uint32_t slot_floats)
@@ -124,9 +140,9 @@ static RingGeom ring_geom(const Plan &p, int dir, bool extra, uint32_t slots, ui
   const uint32_t cwarps = ring_warps(dir), planes = (dir == 1 ? 2u : 1u) + (extra ? 1u : 0u);
   g.res_stride = p.cb > cwarps ? p.cb : cwarps;   // regime R: one partial per consumer warp
   g.off_res = off;  off += (uint32_t)align_up_u64((uint64_t)kResQ * g.res_stride * 16, 128);
-  g.off_coef = off; off += (uint32_t)align_up_u64((uint64_t)kCoefQ * p.cb * 32, 128);
+  g.off_coef = off; off += (uint32_t)align_up_u64((uint64_t)kCoefQ * kCoefBox * 16, 128);
   g.off_slots = off;
-  g.slot_stride = (uint32_t)align_up_u64((uint64_t)slot_floats * 4 * planes + (dir == 1 ? (uint64_t)p.cb * 16 : 0), 128);
+  g.slot_stride = (uint32_t)align_up_u64((uint64_t)slot_floats * 4 * planes + 32, 128);
   g.smem_bytes = off + slots * g.slot_stride;
   return g;
 }
@@ -153,18 +169,15 @@ static bool ring_plan_with(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool 
     // Equal tiles: the last of a channel would hold what is left over and cost a step all the same.  Forward, before and
     // now: [846,106,131] 67.8 and 61.8 us, [371,210,135] 65.8 and 55.5, [64,95,55,55] 41.9 and 42.0.
     p.rows_per_tile = ceil_div_u32(N, p.sample_blocks);
-    const uint32_t per_row = ragged_pitch(p.piece_len < dim0 ? p.piece_len : dim0);
     p.vec = 4;
-    p.div_mul = (uint32_t)((1ull << 32) / per_row) + 1;
   }
   // a tile must fit one slot
-  const uint64_t tile_max = (uint64_t)p.rows_per_tile * (ragged ? 4 * ragged_pitch(p.piece_len < dim0 ? p.piece_len : dim0) : p.piece_len);
+  const uint64_t tile_max = 4ull * ring_tile_vecs(p);
   if (tile_max > slot_floats) return false;
   slot_floats = (uint32_t)((tile_max + 31) / 32 * 32);     // slots no larger than the largest tile
   g = ring_geom(p, dir, extra, slots, slot_floats);
-  const uint32_t budget = 227u * 1024u;
-  while (g.smem_bytes > budget && slots > 2) { --slots; g = ring_geom(p, dir, extra, slots, slot_floats); }
-  return g.smem_bytes <= budget;
+  while (g.smem_bytes > kRingSmemBudget && slots > 2) { --slots; g = ring_geom(p, dir, extra, slots, slot_floats); }
+  return g.smem_bytes <= kRingSmemBudget;
 }
 
 // Bytes between the two visits of a tile: what L2 has to hold for the apply visit to find its tile there.
@@ -271,13 +284,16 @@ int launch_ring(FusedArgs &a, const RingGeom &g_in, int dir, cudaStream_t stream
   static std::mutex mu;
   static std::map<std::pair<const void *, uint32_t>, int> occ;     // (kernel, smem) -> blocks per SM
   int per_sm = 0;
+  // Blocks that use tensor memory take the SM's whole shared memory: a block of another kernel beside them could hold columns
+  // they need, or wait for theirs, and blocks that wait for one another across SMs must not also wait for columns.
+  const uint32_t smem = a.mode == MODE_FUSED ? kRingSmemBudget : g.smem_bytes;
   {
     std::lock_guard<std::mutex> lock(mu);
-    const auto key = std::make_pair((const void *)k, g.smem_bytes);
+    const auto key = std::make_pair((const void *)k, smem);
     auto it = occ.find(key);
     if (it == occ.end()) {
-      if (cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024)) != cudaSuccess ||
-          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, (int)threads, g.smem_bytes) != cudaSuccess) {
+      if (cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRingSmemBudget) != cudaSuccess ||
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, (int)threads, smem) != cudaSuccess) {
         (void)cudaGetLastError();
         per_sm = 0;
       }
@@ -293,17 +309,20 @@ int launch_ring(FusedArgs &a, const RingGeom &g_in, int dir, cudaStream_t stream
     a.plan.lookahead_steps = ceil_div_u32(a.plan.tiles_per_unit, a.plan.grid) + tunables().slack_steps;
   }
   a.use_rec = a.mode == MODE_FUSED ? 1u : 0u;
+  plan_walk(g, a.plan, ring_pitch(a.plan), ring_warps(dir) * 32);
+  g.keep_slots = 0; g.keep_period = 1;
+  if (a.mode == MODE_FUSED) ring_keep(a.plan, dir, g);
   // A window larger than what L2 keeps would cycle through it whole (config 3, backward: 67 MB); marking only
   // the part that fits lets that part stay (backward 4.42 -> 4.27 ms).  Smaller windows keep everything.
-  uint64_t window = ring_window_bytes(a.plan, dir);
+  uint64_t window = ring_window_bytes(a.plan, dir) * (g.keep_period - g.keep_slots) / g.keep_period;
   if (a.ymask && !a.dres_early) window += window / 2;      // x, dy and the saved output come twice
   g.keep_frac = window > kRingLargeWindowMax ? (float)((double)kRingLargeWindowMax / (double)window) : 1.0f;
   void *params[] = {(void *)&a, (void *)&g};
   cudaError_t e;
   if (a.mode == MODE_FUSED)
-    e = cudaLaunchCooperativeKernel((const void *)k, dim3(a.plan.grid), dim3(threads), params, g.smem_bytes, stream);
+    e = cudaLaunchCooperativeKernel((const void *)k, dim3(a.plan.grid), dim3(threads), params, smem, stream);
   else
-    e = cudaLaunchKernel((const void *)k, dim3(a.plan.grid), dim3(threads), params, g.smem_bytes, stream);
+    e = cudaLaunchKernel((const void *)k, dim3(a.plan.grid), dim3(threads), params, smem, stream);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return ANODE_E_LAUNCH; }
   return ANODE_OK;
 }
@@ -770,6 +789,26 @@ extern "C" int anode_gpu_batch_norm_tiled_geometry(uint32_t dim0, uint32_t dim1,
   out[5] = g.slot_stride; out[6] = g.smem_bytes; out[7] = (uint32_t)(window >> 10);
   out[8] = window > kRingLargeWindowMax ? (uint32_t)(1000.0 * (double)kRingLargeWindowMax / (double)window) : 1000u;
   out[9] = p.grid; out[10] = p.lookahead_steps; out[11] = p.total_tiles;
+  return ANODE_OK;
+}
+
+// ---- diagnostics: what of a block's tiles stays in tensor memory (no GPU needed) ------------------
+// out (10 values): kept at all, tile number `tile` of a block kept, place, the dealt number of consumer warp `warp`, its first
+// column, kept tiles before, vectors of the largest tile, consumer warps, columns per set, steps between a tile's two visits
+extern "C" int anode_gpu_batch_norm_tiled_keep(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual,
+                                               uint32_t tile, uint32_t warp, uint32_t *out)
+{
+  using namespace anode_b200;
+  if (!out || (dir != 0 && dir != 1) || check_dims(dim0, dim1, dim2) || warp >= ring_warps(dir)) return ANODE_E_DIMS;
+  Plan p; RingGeom g;
+  for (int i = 0; i < 10; ++i) out[i] = 0;
+  if (!ring_plan_for(dim0, dim1, dim2, true, dir, residual != 0, p, g)) return ANODE_OK;
+  ring_keep(p, dir, g);
+  KeepIter it; it.init(g);
+  for (uint32_t t = 0; t < tile; ++t) it.advance();
+  out[0] = g.keep_slots; out[1] = it.kept() ? 1u : 0u; out[2] = it.slot;
+  keep_place(g, it.slot, warp, ring_warps(dir), out[3], out[4]);
+  out[5] = kept_before(g, tile); out[6] = ring_tile_vecs(p); out[7] = ring_warps(dir); out[8] = g.keep_set; out[9] = p.lookahead_steps;
   return ANODE_OK;
 }
 

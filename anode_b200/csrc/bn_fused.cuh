@@ -719,6 +719,7 @@ __global__ void __launch_bounds__(kThreads) bn_pipeline_kernel(const FusedArgs a
 // ---- shared by the instantiations of the warp-specialised kernel (bn_ring.cuh) and the host ----
 constexpr uint32_t kResQ = 4;          // partial mailbox depth
 constexpr uint32_t kCoefQ = 4;         // coefficient mailbox depth
+constexpr uint32_t kCoefBox = 3;       // 16-byte words of its entries
 constexpr uint32_t kMaxSlots = 8;
 constexpr uint32_t kRingCtlBytes = 1024;   // room reserved for the kernel's barrier block (RingCtl)
 // 16-byte vectors a row of `len` floats can touch when it starts anywhere within one (tiled kernel, ragged rows)
@@ -727,6 +728,64 @@ struct RingGeom {
   uint32_t slots, slot_floats, slot_stride, res_stride, off_res, off_coef, off_slots, smem_bytes;
   uint32_t hdr;            // byte offset of this plan's exit counter and parity word in the workspace header
   float keep_frac;         // fused mode: fraction of the reduce visits' lines loaded with the L2 "keep" priority
+  // Fused mode: of every keep_period tiles of a block, keep_slots stay in tensor memory between their two visits.  A tile's
+  // vectors make keep_base sets of one vector per consumer thread and keep_extra warps' worth beyond; a warp's share of a
+  // set takes keep_set columns.
+  uint32_t keep_slots, keep_period, keep_base, keep_extra, keep_set;
+  // From one vector of a consumer thread to the next: floats on, columns (vectors) on within rows of walk_per vectors, and
+  // floats on top where that passes a row's end; walk_mul divides by walk_per (tiles of one piece of a row: never passes).
+  uint32_t walk_mul, walk_per, walk_col, walk_step, walk_wrap;
 };
+constexpr uint32_t kMaxKeepTurns = 64;      // keep_slots * keep_extra is at most this many turns of the warps
+
+// The tiles of a block one after another: evenly spread, keep_slots out of keep_period stay.  `slot` is where.
+struct KeepIter {
+  uint32_t acc, slot, slots, period;
+  ANODE_HD void init(const RingGeom &g) { acc = 0; slot = 0; slots = g.keep_slots; period = g.keep_period; }
+  ANODE_HD bool kept() const { return acc < slots; }
+  ANODE_HD void advance()
+  {
+    acc += slots;
+    if (acc >= period) { acc -= period; if (++slot >= slots) slot = 0; }
+  }
+};
+// Place `slot` as consumer warp `warp` of `warps` sees it: the warp's number in the dealing of the tile's vectors (which
+// starts with another warp for each place, so that the sets beyond whole turns fall on every warp in turn), and its first
+// column among those of its group of four warps.
+ANODE_HD void keep_place(const RingGeom &g, uint32_t slot, uint32_t warp, uint32_t warps, uint32_t &dealt, uint32_t &column)
+{
+  const uint32_t extra = slot * g.keep_extra;      // sets dealt before, beyond whole turns
+  dealt = (warp + warps * kMaxKeepTurns - extra) % warps;
+  column = (slot * g.keep_base + (extra + warps - 1 - warp) / warps) * g.keep_set;
+}
+// How many of a block's first n tiles stay.
+ANODE_HD uint32_t kept_before(const RingGeom &g, uint32_t n)
+{
+  if (!g.keep_slots) return 0;
+  const uint32_t q = n / g.keep_period, r = n - q * g.keep_period;
+  return q * g.keep_slots + (r ? (r - 1) * g.keep_slots / g.keep_period + 1 : 0);
+}
+// The walk of one of `threads` consumer threads through tiles of plan `p` whose rows take `pitch` vectors of a slot.
+inline void plan_walk(RingGeom &g, const Plan &p, uint32_t pitch, uint32_t threads)
+{
+  const uint32_t rs = p.C * p.dim0;
+  g.walk_mul = 0; g.walk_per = 1u << 30; g.walk_col = threads; g.walk_step = 4 * threads; g.walk_wrap = 0;
+  if (p.pieces != 1) return;
+  const uint32_t rows = threads / pitch;
+  g.walk_mul = (uint32_t)((1ull << 32) / pitch) + 1; g.walk_per = pitch; g.walk_col = threads - rows * pitch;
+  g.walk_step = rows * rs + 4 * g.walk_col; g.walk_wrap = rs - 4 * pitch;
+}
+// Places for tiles of `vecs` vectors of `planes` tensors in the tensor memory of a block with `warps` consumer warps (four
+// of them share 512 columns of 32 lanes), for tiles that a block applies `look` steps after it has reduced them.
+inline void plan_keep(RingGeom &g, uint32_t vecs, uint32_t planes, uint32_t warps, uint32_t look)
+{
+  const uint32_t sets = (vecs + 31) / 32;                     // per warp and vector
+  g.keep_base = sets / warps; g.keep_extra = sets % warps; g.keep_set = 4 * planes;
+  g.keep_period = look + 1;      // a step's reduce visit comes before its apply visit
+  const uint32_t room = 512 / (warps / 4) / g.keep_set;       // vectors per warp
+  uint32_t k = 0;
+  while (k < g.keep_period && (k + 1) * g.keep_base + ((k + 1) * g.keep_extra + warps - 1) / warps <= room) ++k;
+  g.keep_slots = k;
+}
 
 }  // namespace anode_b200

@@ -7,20 +7,30 @@
 //                    slots with bulk asynchronous copies (cp.async.bulk + mbarrier), tagged
 //                    with L2 eviction hints: "keep" for the reduce visit, "drop" for the
 //                    apply visit.  The ring keeps HBM requests in flight while everything
-//                    else happens.
-//   consumer warps   (8) read slots with 128-bit shared loads, accumulate / normalise, write
+//                    else happens.  Each slot carries a description of its visit.
+//   consumer warps   (8 or 16) read slots with 128-bit shared loads, accumulate / normalise, write
 //                    results with 128-bit streaming stores, and hand partials to the delivery
-//                    warp through a shared-memory mailbox.  In regime R every warp works on its
-//                    own share of a tile and never synchronises with the other warps.
+//                    warp through a shared-memory mailbox.  Every warp works on its
+//                    own share of a tile and never synchronises with the other warps.  Of most
+//                    tiles the reduce visit leaves what it read in TENSOR MEMORY (256 KB per SM,
+//                    37 MB on the device), from where the apply visit takes it: no second trip
+//                    through L2 and no slot.
 //   delivery warp    merges the consumer warps' partials of a tile and stores them as ONE tagged
 //                    8-byte word per tile in the workspace (no counter, no fence, no atomic).
 //   coefficient warp polls, for each upcoming apply visit, the partial words of the visit's
 //                    channel until none is zero, merges them in a fixed order in double
 //                    precision (every block obtains bit-identical coefficients; with several
 //                    GPUs the owner block exchanges per-GPU records with the peers here) and
-//                    stages the visit's coefficients in a second mailbox.
+//                    stages the visit's coefficients and description in a second mailbox.
 //                    (In the three-launch form of the synchronized calls the reduce launch still counts
 //                    partials per unit and the apply launch reads prepared coefficients.)
+//
+// What bounds it: the first visits' loads and the stores where all of a window stays in tensor memory, and on the way there
+// the instructions of the consumers and the merge of a channel's partials.  Forward / backward in us, with every second visit
+// from L2, with tensor memory, with descriptions and pairs on top, with the shorter merge on top: [256,64,112,112] 301 / 495,
+// 370 / 595, 281 / 436, 276 / 420; [2048,256,56,56] 2555 / 4362, 2446 / 4371, 2197 / 3763, 2134 / 3347;
+// [4,32,128,128,128] 454 / 737, 389 / 634, 372 / 621, 350 / 598.  (Tensor memory alone was no gain: its stores and loads
+// came on top of 23 / 55 instructions per element, where 10 / 16 are arithmetic.)
 //
 // Every wait is bounded: a wait that runs out sets a status bit, raises the block's abort flag
 // and all three roles drain and leave.
@@ -55,6 +65,7 @@ struct RingCtl {
   volatile uint32_t abort;
   uint32_t last_block;
   uint32_t parity;       // which of the two tagged-partial buffers this launch uses
+  uint32_t tmem;         // base address of the block's tensor memory (g.keep_slots > 0)
 };
 static_assert(sizeof(RingCtl) <= kRingCtlBytes, "RingCtl outgrew the room reserved for it");
 
@@ -126,6 +137,26 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
                ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy) : "memory");
 }
+// ---- tensor memory as a store for tiles ---------------------------------------------------------
+// The SM's 256 KB of tensor memory hold what the reduce visits of `keep_slots` out of every keep_period tiles have read
+// (forward: x; backward: x - mean and dz), so that their apply visits need neither L2 nor a slot of the ring.  A warp
+// reaches the 32 lanes of its place in its group of four warps; the groups divide the 512 columns among them.
+// Every instruction here is the whole warp's.
+constexpr uint32_t kTmemCols = 512;
+__device__ __forceinline__ void tmem_alloc(uint32_t *dst)
+{
+  // never waits: the launch takes the SM's whole shared memory, so that no other block holds columns (launch_ring)
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)), "n"(kTmemCols) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_free(uint32_t base)
+{
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "n"(kTmemCols) : "memory");
+}
+__device__ __forceinline__ void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
 // ---- the block's schedule --------------------------------------------------------------------
 // Operation k of a block: steps s = 0, 1, ...; at step s first REDUCE tile s (if any is left), then
 // APPLY tile s - look (if s >= look).  Every role walks this same sequence with its own cursor.
@@ -134,8 +165,11 @@ struct Sched {
   bool do_reduce, do_apply;
   uint32_t s, phase;     // phase 0: reduce of step s pending; 1: apply of step s pending
   TileIter it_reduce, it_apply;     // the reduce visits and the apply visits both walk b, b+G, ...
-  __device__ __forceinline__ void init(const FusedArgs &a)
+  KeepIter keep_reduce, keep_apply;
+  KeepIter keep;                    // of the visit handed out last
+  __device__ __forceinline__ void init(const FusedArgs &a, const RingGeom &g)
   {
+    keep_reduce.init(g); keep_apply.init(g); keep = keep_reduce;
     b = blockIdx.x; G = gridDim.x;
     my_tiles = (b < a.plan.total_tiles) ? (a.plan.total_tiles - b + G - 1) / G : 0;
     look = (a.mode == MODE_FUSED) ? a.plan.lookahead_steps : 0;
@@ -143,33 +177,18 @@ struct Sched {
     s = 0; phase = 0;
     it_reduce.init(a.plan, b, G); it_apply.init(a.plan, b, G);
   }
-  // Same walk, but hands out the tile's range without any per-tile division.
+  // Advances to the next operation; returns false at the end.  kind: 0 reduce, 1 apply.
   __device__ __forceinline__ bool next_range(const Plan &P, uint32_t &kind, TileRange &tr)
   {
     for (;;) {
       if (s >= my_tiles + look) return false;
       if (phase == 0) {
         phase = 1;
-        if (do_reduce && s < my_tiles) { kind = 0; tr = it_reduce.range(P); it_reduce.advance(P); return true; }
+        if (do_reduce && s < my_tiles) { kind = 0; tr = it_reduce.range(P); it_reduce.advance(P); keep = keep_reduce; keep_reduce.advance(); return true; }
       } else {
         phase = 0;
         const uint32_t ss = s++;
-        if (do_apply && ss >= look) { kind = 1; tr = it_apply.range(P); it_apply.advance(P); return true; }
-      }
-    }
-  }
-  // Advances to the next operation; returns false at the end.  kind: 0 reduce, 1 apply.
-  __device__ __forceinline__ bool next(uint32_t &kind, uint32_t &tile)
-  {
-    for (;;) {
-      if (s >= my_tiles + look) return false;
-      if (phase == 0) {
-        phase = 1;
-        if (do_reduce && s < my_tiles) { kind = 0; tile = b + s * G; return true; }
-      } else {
-        phase = 0;
-        const uint32_t ss = s++;
-        if (do_apply && ss >= look) { kind = 1; tile = b + (ss - look) * G; return true; }
+        if (do_apply && ss >= look) { kind = 1; tr = it_apply.range(P); it_apply.advance(P); keep = keep_apply; keep_apply.advance(); return true; }
       }
     }
   }
@@ -180,29 +199,98 @@ struct Sched {
 __device__ __forceinline__ float *slot_x(unsigned char *sm, const RingGeom &g, uint32_t slot) { return reinterpret_cast<float *>(sm + g.off_slots + (size_t)slot * g.slot_stride); }
 // a slot holds kPlanes tensors side by side: x, then dy (backward), then the residual (forward) / saved output (backward)
 template <int DIR, bool EXTRA> constexpr uint32_t kPlanes = (DIR == 1 ? 2u : 1u) + (EXTRA ? 1u : 0u);
+// an apply visit from tensor memory needs a slot only for the residual
+template <int DIR, bool EXTRA> constexpr bool kSlotAlways = DIR == 0 && EXTRA;
+// behind the planes: the visit (reduce visits only) and, in the backward pass, (mean, scale, beta) of its channel
 template <int DIR, bool EXTRA> __device__ __forceinline__ float4 *slot_side(unsigned char *sm, const RingGeom &g, uint32_t slot)
 {
   return reinterpret_cast<float4 *>(slot_x(sm, g, slot) + kPlanes<DIR, EXTRA> * g.slot_floats);
 }
 __device__ __forceinline__ float4 *res_box(unsigned char *sm, const RingGeom &g, uint32_t q) { return reinterpret_cast<float4 *>(sm + g.off_res) + (size_t)q * g.res_stride; }
-__device__ __forceinline__ float4 *coef_box(unsigned char *sm, const RingGeom &g, uint32_t cb, uint32_t q) { return reinterpret_cast<float4 *>(sm + g.off_coef) + (size_t)q * cb * 2; }
+// a mailbox entry of the coefficient warp: (mean, scale, beta, cB), (cC, -, -, -), the visit
+__device__ __forceinline__ float4 *coef_box(unsigned char *sm, const RingGeom &g, uint32_t q) { return reinterpret_cast<float4 *>(sm + g.off_coef) + q * kCoefBox; }
 
 // ======================================================================================
 // consumer side
 // ======================================================================================
-// ---- each consumer warp handles vectors warp*32 + lane + i*256 of the tile ----------
+// What bounds the consumers is the instructions they issue: a visit is three or four vectors per thread in the backward
+// pass, so whatever is done once per visit weighs as much as the arithmetic.  Hence the visit's range comes ready-made from
+// the service warps (one 16-byte word), arithmetic is two floats per instruction, and places are found by adding up.
+// Instructions per element, [256,16,112,112]: forward 23, backward 55 when every warp walked the schedule by itself.
 constexpr uint32_t kCWarps = kConsumers / 32;
-constexpr uint32_t kPerTurn = 32 / kCWarps;      // mailbox entries the delivery warp merges per turn
+constexpr uint32_t kVecStride = kConsumers * 16;     // bytes between consecutive vectors of one thread
 
-// 128-bit shared load by 32-bit shared address (keeps the address arithmetic in 32 bits)
-__device__ __forceinline__ Pack<4> lds128(uint32_t saddr)
+// ---- pairs of floats: one instruction for two, each rounded as its scalar form
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair(float lo, float hi) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
+__device__ __forceinline__ f32x2 pair(float v) { return pair(v, v); }
+__device__ __forceinline__ float2 split(f32x2 v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ f32x2 slopes(f32x2 y, float slope)      // act'(y)
 {
-  Pack<4> r;
-  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]) : "r"(saddr) : "memory");
+  const float2 t = split(y);
+  return pair(t.x > 0.0f ? 1.0f : slope, t.y > 0.0f ? 1.0f : slope);
+}
+struct Quad { f32x2 a, b; };     // a 16-byte vector
+__device__ __forceinline__ Quad quad(float v) { const f32x2 p = pair(v); return Quad{p, p}; }
+__device__ __forceinline__ float4 floats(const Quad &q) { const float2 a = split(q.a), b = split(q.b); return make_float4(a.x, a.y, b.x, b.y); }
+__device__ __forceinline__ Quad lds_quad(uint32_t saddr)
+{
+  Quad r;
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(r.a), "=l"(r.b) : "r"(saddr) : "memory");
   return r;
 }
-constexpr uint32_t kVecStride = kConsumers * 16;     // bytes between consecutive vectors of one thread
+__device__ __forceinline__ Quad ldg_quad(const float *p)
+{
+  Quad r;
+  asm volatile("ld.global.v2.b64 {%0, %1}, [%2];" : "=l"(r.a), "=l"(r.b) : "l"(p) : "memory");
+  return r;
+}
+__device__ __forceinline__ void stg_quad(float *p, const Quad &q) { asm volatile("st.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(q.a), "l"(q.b) : "memory"); }
+__device__ __forceinline__ void stg_stream(float *p, const Quad &q) { asm volatile("st.global.cs.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(q.a), "l"(q.b) : "memory"); }
+
+// ---- tensor memory, a vector per thread and four columns (the whole warp)
+#define ANODE_T16 "{t0, t1, t2, t3, t4, t5, t6, t7, t8, t9, t10, t11, t12, t13, t14, t15}"
+__device__ __forceinline__ void tmem_st(uint32_t at, const Quad &a)
+{
+  asm volatile("{\n\t.reg .b32 t<4>;\n\tmov.b64 {t0, t1}, %1;\n\tmov.b64 {t2, t3}, %2;\n\t"
+               "tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {t0, t1, t2, t3};\n\t}" ::"r"(at), "l"(a.a), "l"(a.b) : "memory");
+}
+__device__ __forceinline__ void tmem_st(uint32_t at, const Quad &a, const Quad &b)
+{
+  asm volatile("{\n\t.reg .b32 t<8>;\n\tmov.b64 {t0, t1}, %1;\n\tmov.b64 {t2, t3}, %2;\n\tmov.b64 {t4, t5}, %3;\n\tmov.b64 {t6, t7}, %4;\n\t"
+               "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {t0, t1, t2, t3, t4, t5, t6, t7};\n\t}"
+               ::"r"(at), "l"(a.a), "l"(a.b), "l"(b.a), "l"(b.b) : "memory");
+}
+__device__ __forceinline__ void tmem_st(uint32_t at, const Quad &a, const Quad &b, const Quad &c, const Quad &d)
+{
+  asm volatile("{\n\t.reg .b32 t<16>;\n\tmov.b64 {t0, t1}, %1;\n\tmov.b64 {t2, t3}, %2;\n\tmov.b64 {t4, t5}, %3;\n\tmov.b64 {t6, t7}, %4;\n\t"
+               "mov.b64 {t8, t9}, %5;\n\tmov.b64 {t10, t11}, %6;\n\tmov.b64 {t12, t13}, %7;\n\tmov.b64 {t14, t15}, %8;\n\t"
+               "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], " ANODE_T16 ";\n\t}"
+               ::"r"(at), "l"(a.a), "l"(a.b), "l"(b.a), "l"(b.b), "l"(c.a), "l"(c.b), "l"(d.a), "l"(d.b) : "memory");
+}
+// (the wait stands in the same statement as the load, so that nothing can use a register before it has arrived)
+__device__ __forceinline__ void tmem_ld(uint32_t at, Quad &a)
+{
+  asm volatile("{\n\t.reg .b32 t<4>;\n\ttcgen05.ld.sync.aligned.32x32b.x4.b32 {t0, t1, t2, t3}, [%2];\n\ttcgen05.wait::ld.sync.aligned;\n\t"
+               "mov.b64 %0, {t0, t1};\n\tmov.b64 %1, {t2, t3};\n\t}" : "=l"(a.a), "=l"(a.b) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void tmem_ld(uint32_t at, Quad &a, Quad &b)
+{
+  asm volatile("{\n\t.reg .b32 t<8>;\n\ttcgen05.ld.sync.aligned.32x32b.x8.b32 {t0, t1, t2, t3, t4, t5, t6, t7}, [%4];\n\ttcgen05.wait::ld.sync.aligned;\n\t"
+               "mov.b64 %0, {t0, t1};\n\tmov.b64 %1, {t2, t3};\n\tmov.b64 %2, {t4, t5};\n\tmov.b64 %3, {t6, t7};\n\t}"
+               : "=l"(a.a), "=l"(a.b), "=l"(b.a), "=l"(b.b) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void tmem_ld(uint32_t at, Quad &a, Quad &b, Quad &c, Quad &d)
+{
+  asm volatile("{\n\t.reg .b32 t<16>;\n\ttcgen05.ld.sync.aligned.32x32b.x16.b32 " ANODE_T16 ", [%8];\n\ttcgen05.wait::ld.sync.aligned;\n\t"
+               "mov.b64 %0, {t0, t1};\n\tmov.b64 %1, {t2, t3};\n\tmov.b64 %2, {t4, t5};\n\tmov.b64 %3, {t6, t7};\n\t"
+               "mov.b64 %4, {t8, t9};\n\tmov.b64 %5, {t10, t11};\n\tmov.b64 %6, {t12, t13};\n\tmov.b64 %7, {t14, t15};\n\t}"
+               : "=l"(a.a), "=l"(a.b), "=l"(b.a), "=l"(b.b), "=l"(c.a), "=l"(c.b), "=l"(d.a), "=l"(d.b) : "r"(at) : "memory");
+}
+#undef ANODE_T16
 
 // Shift of the sums: the median of three elements.  A single one is no shift to rely on: the first of an image is the corner
 // that a zero-padded convolution makes, and far from the mean it costs the variance its digits.  Relative error of the
@@ -218,332 +306,298 @@ __device__ __forceinline__ float median3(float a, float b, float c) { return fma
 // The read is a bulk copy, hence the fence between the two proxies before the slot is given back.
 __device__ __forceinline__ void fence_global_to_bulk() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
-// Places, in global memory, of the vectors tid, tid + kConsumers, ... of a tile whose rows lie back to back in the slot,
-// per_row vectors each: a step is an add and a compare, without a division or a 64-bit product per vector.
-struct RowWalk {
-  uint32_t row, col;              // float offset of the row's first float (below 2^32, check_dims); vector within the row
-  uint32_t step_row, step_col, rs, per_row;
-  __device__ __forceinline__ void init(const FusedArgs &a, const TileRange &tr, uint32_t per_row_)
+// A visit, as the service warps describe it to the consumers (16 bytes): its vectors, its place in tensor memory + 1 (0:
+// none), the float offset of its first element (below 2^32, check_dims), floats per row, rows.
+__device__ __forceinline__ uint4 describe(const TileRange &tr, bool ragged, const KeepIter &keep)
+{
+  const uint32_t nvec = (ragged ? ragged_pitch(tr.len) : tr.len / 4) * tr.rows;
+  return make_uint4(nvec | (keep.kept() ? keep.slot + 1u : 0u) << 16, (uint32_t)tr.base, tr.len, tr.rows);
+}
+
+// The visit as one thread sees it: its vectors are tid, tid + kConsumers, ... of the tile's rows laid back to back (`cnt` of
+// them; the warp's lane with the most has `steps`), kept in tensor memory from column `tm` on.
+template <bool KEEP>
+struct Mine {
+  uint32_t tid, cnt, steps, tm;
+  __device__ __forceinline__ Mine(const RingGeom &g, const RingCtl *ctl, const uint4 &d)
   {
-    const uint32_t tid = threadIdx.x;
-    per_row = per_row_; rs = a.plan.C * a.plan.dim0;
-    uint32_t r = 0, sr = 0;
-    // several rows: always whole ones, whose vectors plan.div_mul divides by; one row: never wraps
-    if (tr.rows > 1) { r = fast_div(tid, a.plan.div_mul); sr = fast_div(kConsumers, a.plan.div_mul); }
-    col = tid - r * per_row; row = (uint32_t)tr.base + r * rs;
-    step_col = kConsumers - sr * per_row; step_row = sr * rs;
+    tid = threadIdx.x; tm = 0;
+    const uint32_t nvec = d.x & 0xffffu;
+    if constexpr (KEEP) {
+      const uint32_t warp = tid >> 5;
+      uint32_t dealt, column;
+      keep_place(g, (d.x >> 16) - 1, warp, kCWarps, dealt, column);
+      tid = dealt * 32 + (tid & 31);
+      tm = ctl->tmem + ((warp & 3u) << 21) + (warp >> 2) * (kTmemCols * 4 / kCWarps) + column;
+    }
+    cnt = (nvec + kConsumers - 1 - tid) / kConsumers;
+    steps = (nvec + kConsumers - 1 - (tid & ~31u)) / kConsumers;
   }
-  __device__ __forceinline__ void advance()
-  {
-    row += step_row; col += step_col;
-    if (col >= per_row) { col -= per_row; row += rs; }
-  }
-  __device__ __forceinline__ uint32_t at() const { return (row & ~3u) + 4 * col; }            // float offset of the vector
-  __device__ __forceinline__ int first() const { return (int)(4 * col) - (int)(row & 3u); }   // its first float's place in the row
 };
 
-template <int DIR, bool EXTRA>
-__device__ __forceinline__ void warp_reduce_R(const FusedArgs &a, const RingGeom &g, unsigned char *sm, RingCtl *ctl,
-                                              const TileRange &tr, uint32_t slot, float4 *res)
-{
-  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t nvec = (tr.len / 4) * tr.rows;        // the slot holds the tile's rows back to back
-  const uint32_t cnt = tid < nvec ? (nvec - tid + kConsumers - 1) / kConsumers : 0;   // this thread's vectors
-  uint32_t ax = smem_u32(slot_x(sm, g, slot)) + tid * 16;
-  if constexpr (DIR == 0) {
-    // shifted sums (see bn_fused.cuh), two accumulator pairs
-    // K: from the warp's first vector (lane 0 has the lowest vector index, so it has a vector whenever any lane has one).
-    // One shift per warp makes s and q plain sums over lanes.
-    const Pack<4> v0 = cnt ? lds128(ax) : pack_fill<4>(0.f);
-    const float K = __shfl_sync(0xffffffffu, median3(v0.v[0], v0.v[1], v0.v[2]), 0);
-    float s0 = 0.f, q0 = 0.f, s1 = 0.f, q1 = 0.f;
-    uint32_t i = 0;
-    for (; i + 4 <= cnt; i += 4, ax += 4 * kVecStride) {
-      const Pack<4> v0 = lds128(ax), v1 = lds128(ax + kVecStride), v2 = lds128(ax + 2 * kVecStride), v3 = lds128(ax + 3 * kVecStride);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float d0 = v0.v[e] - K, d1 = v1.v[e] - K, d2 = v2.v[e] - K, d3 = v3.v[e] - K;
-        s0 += d0; q0 = fmaf(d0, d0, q0); s1 += d1; q1 = fmaf(d1, d1, q1);
-        s0 += d2; q0 = fmaf(d2, d2, q0); s1 += d3; q1 = fmaf(d3, d3, q1);
-      }
-    }
-    for (; i + 2 <= cnt; i += 2, ax += 2 * kVecStride) {
-      const Pack<4> v0 = lds128(ax), v1 = lds128(ax + kVecStride);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float d0 = v0.v[e] - K, d1 = v1.v[e] - K;
-        s0 += d0; q0 = fmaf(d0, d0, q0); s1 += d1; q1 = fmaf(d1, d1, q1);
-      }
-    }
-    if (i < cnt) {
-      const Pack<4> v0 = lds128(ax);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) { const float d0 = v0.v[e] - K; s0 += d0; q0 = fmaf(d0, d0, q0); }
-    }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&ctl->empty[slot]);
-    const float s = warp_sum(s0 + s1), q = warp_sum(q0 + q1);
-    const uint32_t nw = __reduce_add_sync(0xffffffffu, cnt * 4);
-    if (lane == 0) {
-      Moments m{0.f, 0.f, 0.f};
-      if (nw) {
-        m.n = (float)nw;
-        const float inv = __fdividef(1.0f, m.n);
-        m.mean = fmaf(s, inv, K);
-        m.m2 = fmaxf(q - s * s * inv, 0.f);
-      }
-      res[warp] = make_float4(m.n, m.mean, m.m2, 0.f);
-    }
-  } else {
-    uint32_t ad = ax + g.slot_floats * 4;
-    const float4 cf = slot_side<1, EXTRA>(sm, g, slot)[0];
-    const float mean = cf.x, scale = cf.y, beta = cf.z;
-    const float slope = a.neg_slope;      // activation: t * (t > 0 ? 1 : slope)
-    float s1 = 0.f, s2 = 0.f;
-    RowWalk w;
-    float *dres = nullptr;
-    if constexpr (EXTRA) { if (a.dres_early) { dres = a.dres; w.init(a, tr, tr.len / 4); } }
-    // (one vector per tensor at a time: with two in flight the sixteen warps of this pass were measured slower)
-    for (uint32_t i = 0; i < cnt; ++i, ax += kVecStride, ad += kVecStride) {
-      const Pack<4> x0 = lds128(ax), g0 = lds128(ad);
-      Pack<4> m0 = x0, z;
-      if constexpr (EXTRA) m0 = lds128(ad + g.slot_floats * 4);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float d0 = x0.v[e] - mean;
-        const float y0 = EXTRA ? m0.v[e] : fmaf(d0, scale, beta);      // residual epilogue: the saved output carries the mask
-        // dz = dy * (float)(y > 0)  (routines_gpu/flat_map.cu:191-192)
-        const float z0 = g0.v[e] * (y0 > 0.0f ? 1.0f : slope);
-        s1 += z0; s2 = fmaf(z0, d0, s2);
-        z.v[e] = z0;
-      }
-      if constexpr (EXTRA) { if (dres) { z.put(dres + w.row + 4 * w.col); w.advance(); } }
-    }
-    if constexpr (EXTRA) { if (dres) fence_global_to_bulk(); }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&ctl->empty[slot]);
-    s1 = warp_sum(s1); s2 = warp_sum(s2);
-    if (lane == 0) res[warp] = make_float4(s1, s2, 0.f, 0.f);
+// Places of a thread's vectors in global memory: a step is an add and a compare, without a division or a 64-bit product.
+// (Ragged rows: `at` is the row's first float plus 4 * col, whose last two bits say how far into a vector the row starts.)
+struct Walk {
+  uint32_t at, col;
+  __device__ __forceinline__ Walk(const FusedArgs &a, const RingGeom &g, uint32_t base, uint32_t tid)
+  {
+    const uint32_t r = __umulhi(tid, g.walk_mul);
+    col = tid - r * g.walk_per; at = base + r * (a.plan.C * a.plan.dim0) + 4 * col;
   }
-}
-
-template <int DIR, bool EXTRA>
-__device__ __forceinline__ void warp_apply_R(const FusedArgs &a, const RingGeom &g, unsigned char *sm, RingCtl *ctl,
-                                             const TileRange &tr, uint32_t slot, const float4 *coef, uint32_t coef_q)
-{
-  const uint32_t tid = threadIdx.x, lane = tid & 31;
-  const float slope = a.neg_slope;      // activation: t * (t > 0 ? 1 : slope)
-  const bool acc = a.accumulate != 0;
-  const bool early = EXTRA && DIR == 1 && a.dres_early;      // plane 1 holds dz (see fence_global_to_bulk)
-  const uint64_t rs = (uint64_t)a.plan.C * a.plan.dim0;
-  float *out = a.out + tr.base;
-  float *dres = EXTRA && DIR == 1 && !early ? a.dres : nullptr;
-  const float4 c0 = coef[0], c1 = coef[1];
-  const float mean = c0.x, scale = c0.y, beta = c0.z, cB = c1.x, cC = c1.y;
-  const uint32_t per_row = tr.len / 4, nvec = per_row * tr.rows;
-  const uint32_t cnt = tid < nvec ? (nvec - tid + kConsumers - 1) / kConsumers : 0;
-  uint32_t ax = smem_u32(slot_x(sm, g, slot)) + tid * 16;
-  uint32_t ad = ax + g.slot_floats * 4;
-  // The thread's vectors are tid, tid + kConsumers, ... of the tile's rows laid back to back; their places in
-  // global memory are found by walking (column, row) along, without a division or a 64-bit product per vector.
-  uint32_t col = tid, row = 0;
-  if (tr.rows > 1) { row = fast_div(tid, a.plan.div_mul); col = tid - row * per_row; }   // rows > 1 only occurs with whole rows, where per_row matches div_mul
-  float *dst = out + (size_t)row * rs + 4 * (size_t)col;
-  const uint32_t step_rows = tr.rows > 1 ? fast_div(kConsumers, a.plan.div_mul) : 0;     // kConsumers = step_rows * per_row + step_cols
-  const uint32_t step_cols = kConsumers - step_rows * per_row;
-  const size_t step_ptr = (size_t)step_rows * rs + 4 * (size_t)step_cols;               // floats from one vector of the thread to the next
-  const size_t wrap_ptr = rs - 4 * (size_t)per_row;                                      // on top of that when the column wraps into the next row
-  auto advance = [&]() {
-    dst += step_ptr; col += step_cols;
-    if (col >= per_row) { col -= per_row; dst += wrap_ptr; }
-  };
-  // one vector: o = activation(bn(x)) or the input gradient
-  auto one = [&](const Pack<4> &vx, const Pack<4> &vd, const Pack<4> &ve, float *p) {
-    Pack<4> o, z;
-    if constexpr (DIR == 0) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float yb = fmaf(vx.v[e] - mean, scale, beta);
-        if constexpr (EXTRA) yb += ve.v[e];
-        o.v[e] = yb * (yb > 0.0f ? 1.0f : slope);
-      }
-    } else {
-      if (acc) o = Pack<4>::load(p);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float d = vx.v[e] - mean;
-        const float yb = EXTRA ? ve.v[e] : fmaf(d, scale, beta);
-        const float dz = vd.v[e] * (early || yb > 0.0f ? 1.0f : slope);
-        const float dx = fmaf(scale, dz, fmaf(cB, d, cC));
-        o.v[e] = acc ? o.v[e] + dx : dx;
-        z.v[e] = dz;
-      }
-    }
-    o.store_stream(p);
-    if constexpr (EXTRA && DIR == 1) { if (dres) z.store_stream(dres + (p - a.out)); }
-  };
-  for (uint32_t i = 0; i < cnt; ++i, ax += kVecStride, ad += kVecStride) {
-    const Pack<4> x0 = lds128(ax);
-    Pack<4> d0 = x0, e0 = x0;
-    if constexpr (DIR == 1) d0 = lds128(ad);
-    if constexpr (EXTRA) { if (!early) e0 = lds128(DIR == 1 ? ad + g.slot_floats * 4 : ad); }
-    one(x0, d0, e0, dst);
-    advance();
+  __device__ __forceinline__ void advance(const RingGeom &g)
+  {
+    at += g.walk_step; col += g.walk_col;
+    if (col >= g.walk_per) { col -= g.walk_per; at += g.walk_wrap; }
   }
-  __syncwarp();
-  if (lane == 0) { mbar_arrive(&ctl->empty[slot]); mbar_arrive(&ctl->coef_empty[coef_q]); }
-}
+  __device__ __forceinline__ uint32_t vector() const { return at & ~3u; }                         // ragged rows: the vector
+  __device__ __forceinline__ int first() const { return (int)(4 * col) - (int)(at & 3u); }        // and its first float's place in the row
+};
 
-// ---- rows that are not a multiple of four floats ------------------------------------------
-// A row starts h = (its offset) mod 4 floats behind a 16-byte boundary.  The producer fetches every row from the
-// boundary below its start to the one above its end, so that all tensors' vectors (and the output's) line up; a row
-// takes ragged_pitch(len) vectors of the slot and only its first and last ones hold foreign floats, which are left
-// out element by element (and written one by one).  RowWalk steps through the vectors of one thread.
-template <int DIR, bool EXTRA>
-__device__ __forceinline__ void warp_reduce_ragged(const FusedArgs &a, const RingGeom &g, unsigned char *sm, RingCtl *ctl,
-                                                   const TileRange &tr, uint32_t slot, float4 *res)
+template <int DIR, bool EXTRA, bool RAGGED, bool KEEP>
+__device__ __forceinline__ void visit_reduce(const FusedArgs &a, const RingGeom &g, unsigned char *sm, RingCtl *ctl,
+                                             const uint4 &d, uint32_t slot, float4 *res)
 {
-  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t per_row = ragged_pitch(tr.len), nvec = per_row * tr.rows;
-  const uint32_t cnt = tid < nvec ? (nvec - tid + kConsumers - 1) / kConsumers : 0;
-  const int len = (int)tr.len;
+  const uint32_t lane = threadIdx.x & 31;
+  const Mine<KEEP> mine(g, ctl, d);
+  const uint32_t cnt = mine.cnt, steps = mine.steps;
   const float *xs = slot_x(sm, g, slot);
-  uint32_t ax = smem_u32(xs) + tid * 16;
-  RowWalk w;
-  w.init(a, tr, per_row);
+  uint32_t ax = smem_u32(xs) + mine.tid * 16, tm = mine.tm;
+  const int len = (int)d.z;
+  float4 out;
   if constexpr (DIR == 0) {
-    const uint32_t first = (uint32_t)tr.base, rs = a.plan.C * a.plan.dim0, rm = tr.rows / 2, rl = tr.rows - 1;
-    const float K = median3(xs[(first & 3u) + tr.len / 6], xs[4 * per_row * rm + ((first + rm * rs) & 3u) + tr.len / 2],
-                            xs[4 * per_row * rl + ((first + rl * rs) & 3u) + tr.len - 1 - tr.len / 6]);
-    float s = 0.f, q = 0.f;
+    // shifted sums (see bn_fused.cuh); one shift per warp makes them plain sums over lanes
+    float K = 0.f;
     uint32_t n = 0;
-#pragma unroll 2
-    for (uint32_t i = 0; i < cnt; ++i, ax += kVecStride) {
-      const Pack<4> v = lds128(ax);
-      const int i0 = w.first();
-      if (i0 >= 0 && i0 + 4 <= len) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { const float d = v.v[e] - K; s += d; q = fmaf(d, d, q); }
-        n += 4;
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if ((uint32_t)(i0 + e) < (uint32_t)len) { const float d = v.v[e] - K; s += d; q = fmaf(d, d, q); ++n; }
+    f32x2 sa = 0, sb = 0, qa = 0, qb = 0;
+    if constexpr (!RAGGED) {
+      if (steps) { const float4 v0 = floats(lds_quad(ax - lane * 16)); K = median3(v0.x, v0.y, v0.z); }
+      const f32x2 nK = pair(-K);
+      auto take = [&](const Quad &v) {
+        const f32x2 da = add2(v.a, nK), db = add2(v.b, nK);
+        sa = add2(sa, da); qa = fma2(da, da, qa); sb = add2(sb, db); qb = fma2(db, db, qb);
+      };
+      uint32_t i = 0;
+      for (; i + 4 <= steps; i += 4, ax += 4 * kVecStride, tm += 16) {
+        // (the lanes differ in their last vector only; a missing one is K)
+        const Quad v0 = lds_quad(ax), v1 = lds_quad(ax + kVecStride), v2 = lds_quad(ax + 2 * kVecStride);
+        Quad v3 = quad(K);
+        if (i + 3 < cnt) v3 = lds_quad(ax + 3 * kVecStride);
+        if constexpr (KEEP) { __syncwarp(); tmem_st(tm, v0, v1, v2, v3); }
+        take(v0); take(v1); take(v2); take(v3);
       }
-      w.advance();
+      for (; i < steps; ++i, ax += kVecStride, tm += 4) {
+        Quad v0 = quad(K);
+        if (i < cnt) v0 = lds_quad(ax);
+        if constexpr (KEEP) { __syncwarp(); tmem_st(tm, v0); }
+        take(v0);
+      }
+      // the warp's vectors: whole steps, and what the last one has
+      if (steps) { const uint32_t left = (d.x & 0xffffu) - (mine.tid & ~31u) - (steps - 1) * kConsumers; n = 128 * (steps - 1) + 4 * (left < 32 ? left : 32); }
+    } else {
+      const uint32_t per_row = ragged_pitch(d.z), first = d.y, rs = a.plan.C * a.plan.dim0, rm = d.w / 2, rl = d.w - 1;
+      K = median3(xs[(first & 3u) + d.z / 6], xs[4 * per_row * rm + ((first + rm * rs) & 3u) + d.z / 2],
+                  xs[4 * per_row * rl + ((first + rl * rs) & 3u) + d.z - 1 - d.z / 6]);
+      const f32x2 nK = pair(-K);
+      Walk w(a, g, first, mine.tid);
+#pragma unroll 2
+      for (uint32_t i = 0; i < steps; ++i, ax += kVecStride, tm += 4) {
+        Quad v = quad(K);
+        if (i < cnt) v = lds_quad(ax);
+        if constexpr (KEEP) { __syncwarp(); tmem_st(tm, v); }
+        const int i0 = i < cnt ? w.first() : len;
+        Quad e{add2(v.a, nK), add2(v.b, nK)};
+        if (i0 >= 0 && i0 + 4 <= len) {
+          n += 4;
+        } else {      // foreign floats at a row's ends count nothing
+          const float4 t = floats(e);
+          auto own = [&](float f, int k) { const bool in = (uint32_t)(i0 + k) < (uint32_t)len; n += in; return in ? f : 0.f; };
+          e.a = pair(own(t.x, 0), own(t.y, 1)); e.b = pair(own(t.z, 2), own(t.w, 3));
+        }
+        sa = add2(sa, e.a); qa = fma2(e.a, e.a, qa); sb = add2(sb, e.b); qb = fma2(e.b, e.b, qb);
+        w.advance(g);
+      }
+      n = __reduce_add_sync(0xffffffffu, n);
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(&ctl->empty[slot]);
-    s = warp_sum(s); q = warp_sum(q);
-    const uint32_t nw = __reduce_add_sync(0xffffffffu, n);
-    if (lane == 0) {
-      Moments m{0.f, 0.f, 0.f};
-      if (nw) {
-        m.n = (float)nw;
-        const float inv = __fdividef(1.0f, m.n);
-        m.mean = fmaf(s, inv, K);
-        m.m2 = fmaxf(q - s * s * inv, 0.f);
-      }
-      res[warp] = make_float4(m.n, m.mean, m.m2, 0.f);
+    const float2 st = split(add2(sa, sb)), qt = split(add2(qa, qb));
+    const float s = warp_sum(st.x + st.y), q = warp_sum(qt.x + qt.y);
+    out = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (n) {
+      out.x = (float)n;
+      const float inv = __fdividef(1.0f, out.x);
+      out.y = fmaf(s, inv, K);
+      out.z = fmaxf(q - s * s * inv, 0.f);
     }
   } else {
     uint32_t ad = ax + g.slot_floats * 4;
-    const float4 cf = slot_side<1, EXTRA>(sm, g, slot)[0];
-    const float mean = cf.x, scale = cf.y, beta = cf.z;
-    const float slope = a.neg_slope;
+    const float4 cf = slot_side<1, EXTRA>(sm, g, slot)[1];
+    const f32x2 nmean = pair(-cf.x), scale = pair(cf.y), beta = pair(cf.z);
+    const float slope = a.neg_slope;      // activation: t * (t > 0 ? 1 : slope)
     float *dres = EXTRA && a.dres_early ? a.dres : nullptr;
-    float s1 = 0.f, s2 = 0.f;
-    for (uint32_t i = 0; i < cnt; ++i, ax += kVecStride, ad += kVecStride) {
-      const Pack<4> x0 = lds128(ax), g0 = lds128(ad);
-      Pack<4> m0 = x0, z, d;
-      if constexpr (EXTRA) m0 = lds128(ad + g.slot_floats * 4);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        d.v[e] = x0.v[e] - mean;
-        const float y0 = EXTRA ? m0.v[e] : fmaf(d.v[e], scale, beta);
-        z.v[e] = g0.v[e] * (y0 > 0.0f ? 1.0f : slope);
+    Walk w(a, g, d.y, mine.tid);          // (unused in the ordinary aligned form)
+    f32x2 s1a = 0, s1b = 0, s2a = 0, s2b = 0;
+    // (one vector per tensor at a time: with two in flight the sixteen warps of this pass were measured slower)
+    for (uint32_t i = 0; i < (KEEP ? steps : cnt); ++i, ax += kVecStride, ad += kVecStride) {
+      Quad e{0, 0}, z{0, 0};
+      const bool live = !KEEP || i < cnt;
+      if (live) {
+        const Quad x = lds_quad(ax), gy = lds_quad(ad);
+        e.a = add2(x.a, nmean); e.b = add2(x.b, nmean);
+        Quad y;
+        if constexpr (EXTRA) y = lds_quad(ad + g.slot_floats * 4);      // residual epilogue: the saved output carries the mask
+        else { y.a = fma2(e.a, scale, beta); y.b = fma2(e.b, scale, beta); }
+        // dz = dy * (float)(y > 0)  (routines_gpu/flat_map.cu:191-192)
+        z.a = mul2(gy.a, slopes(y.a, slope)); z.b = mul2(gy.b, slopes(y.b, slope));
       }
-      const int i0 = w.first();
-      if (i0 >= 0 && i0 + 4 <= len) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) { s1 += z.v[e]; s2 = fmaf(z.v[e], d.v[e], s2); }
-        if constexpr (EXTRA) { if (dres) z.put(dres + w.at()); }
+      if constexpr (KEEP) { __syncwarp(); tmem_st(tm, e, z); tm += 8; }
+      if constexpr (!RAGGED) {
+        if constexpr (EXTRA) { if (dres && live) stg_quad(dres + w.at, z); }
       } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if ((uint32_t)(i0 + e) < (uint32_t)len) {
-            s1 += z.v[e]; s2 = fmaf(z.v[e], d.v[e], s2);
-            if constexpr (EXTRA) { if (dres) dres[w.at() + e] = z.v[e]; }
+        const int i0 = live ? w.first() : len;
+        if (i0 >= 0 && i0 + 4 <= len) {
+          if constexpr (EXTRA) { if (dres) stg_quad(dres + w.vector(), z); }
+        } else {      // (foreign floats may be anything, an infinity or a NaN too)
+          const float4 t = floats(z), u = floats(e);
+          auto in = [&](int k) { return (uint32_t)(i0 + k) < (uint32_t)len; };
+          if constexpr (EXTRA) {
+            if (dres) {
+              float *p = dres + w.vector();
+              if (in(0)) p[0] = t.x;
+              if (in(1)) p[1] = t.y;
+              if (in(2)) p[2] = t.z;
+              if (in(3)) p[3] = t.w;
+            }
           }
+          z.a = pair(in(0) ? t.x : 0.f, in(1) ? t.y : 0.f); z.b = pair(in(2) ? t.z : 0.f, in(3) ? t.w : 0.f);
+          e.a = pair(in(0) ? u.x : 0.f, in(1) ? u.y : 0.f); e.b = pair(in(2) ? u.z : 0.f, in(3) ? u.w : 0.f);
+        }
       }
-      w.advance();
+      s1a = add2(s1a, z.a); s2a = fma2(z.a, e.a, s2a); s1b = add2(s1b, z.b); s2b = fma2(z.b, e.b, s2b);
+      if constexpr (EXTRA || RAGGED) w.advance(g);
     }
     if constexpr (EXTRA) { if (dres) fence_global_to_bulk(); }
     __syncwarp();
     if (lane == 0) mbar_arrive(&ctl->empty[slot]);
-    s1 = warp_sum(s1); s2 = warp_sum(s2);
-    if (lane == 0) res[warp] = make_float4(s1, s2, 0.f, 0.f);
+    const float2 u = split(add2(s1a, s1b)), v = split(add2(s2a, s2b));
+    out = make_float4(warp_sum(u.x + u.y), warp_sum(v.x + v.y), 0.f, 0.f);
   }
+  if (lane == 0) res[threadIdx.x >> 5] = out;
 }
 
-template <int DIR, bool EXTRA>
-__device__ __forceinline__ void warp_apply_ragged(const FusedArgs &a, const RingGeom &g, unsigned char *sm, RingCtl *ctl,
-                                                  const TileRange &tr, uint32_t slot, const float4 *coef, uint32_t coef_q)
+template <int DIR, bool EXTRA, bool RAGGED, bool KEEP>
+__device__ __forceinline__ void visit_apply(const FusedArgs &a, const RingGeom &g, unsigned char *sm, RingCtl *ctl,
+                                            const uint4 &d, uint32_t slot, const float4 *coef, uint32_t coef_q)
 {
-  const uint32_t tid = threadIdx.x, lane = tid & 31;
-  const float slope = a.neg_slope;
-  const bool acc = a.accumulate != 0;
-  const bool early = EXTRA && DIR == 1 && a.dres_early;
+  const uint32_t lane = threadIdx.x & 31;
+  const Mine<KEEP> mine(g, ctl, d);
+  const uint32_t cnt = mine.cnt, steps = mine.steps;
+  const float slope = a.neg_slope;      // activation: t * (t > 0 ? 1 : slope)
+  const bool acc = DIR == 1 && a.accumulate != 0;
+  const bool early = EXTRA && DIR == 1 && a.dres_early;      // plane 1 holds dz (see fence_global_to_bulk)
   float *dres = EXTRA && DIR == 1 && !early ? a.dres : nullptr;
-  const float4 c0 = coef[0], c1 = coef[1];
-  const float mean = c0.x, scale = c0.y, beta = c0.z, cB = c1.x, cC = c1.y;
-  const uint32_t per_row = ragged_pitch(tr.len), nvec = per_row * tr.rows;
-  const uint32_t cnt = tid < nvec ? (nvec - tid + kConsumers - 1) / kConsumers : 0;
-  const int len = (int)tr.len;
-  uint32_t ax = smem_u32(slot_x(sm, g, slot)) + tid * 16;
+  const float4 c0 = coef[0];
+  const f32x2 nmean = pair(-c0.x), scale = pair(c0.y), beta = pair(c0.z), cB = pair(c0.w), cC = pair(coef[1].x);
+  const int len = (int)d.z;
+  uint32_t ax = smem_u32(slot_x(sm, g, slot)) + mine.tid * 16, tm = mine.tm;
   uint32_t ad = ax + g.slot_floats * 4;
-  RowWalk w;
-  w.init(a, tr, per_row);
-  for (uint32_t i = 0; i < cnt; ++i, ax += kVecStride, ad += kVecStride) {
-    const Pack<4> x0 = lds128(ax);
-    Pack<4> d0 = x0, e0 = x0, o, z;
-    if constexpr (DIR == 1) d0 = lds128(ad);
-    if constexpr (EXTRA) { if (!early) e0 = lds128(DIR == 1 ? ad + g.slot_floats * 4 : ad); }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float d = x0.v[e] - mean;
-      if constexpr (DIR == 0) {
-        float yb = fmaf(d, scale, beta);
-        if constexpr (EXTRA) yb += e0.v[e];
-        o.v[e] = yb * (yb > 0.0f ? 1.0f : slope);
-      } else {
-        const float yb = EXTRA ? e0.v[e] : fmaf(d, scale, beta);
-        z.v[e] = d0.v[e] * (early || yb > 0.0f ? 1.0f : slope);
-        o.v[e] = fmaf(scale, z.v[e], fmaf(cB, d, cC));
-      }
-    }
-    const int i0 = w.first();
-    float *p = a.out + w.at();
-    if (i0 >= 0 && i0 + 4 <= len) {
-      if (DIR == 1 && acc) {
-        const Pack<4> old = Pack<4>::load(p);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) o.v[e] = old.v[e] + o.v[e];
-      }
-      o.store_stream(p);
-      if constexpr (EXTRA && DIR == 1) { if (dres) z.store_stream(dres + w.at()); }
+  Walk w(a, g, d.y, mine.tid);
+  // one vector: activation(bn(x)) or the input gradient.  x: the input (KEEP and backward: x - mean); gy: dy or dz;
+  // e: residual or saved output
+  auto one = [&](const Quad &x, const Quad &gy, const Quad &e) {
+    Quad o, z;
+    const Quad u = KEEP && DIR == 1 ? x : Quad{add2(x.a, nmean), add2(x.b, nmean)};
+    if constexpr (DIR == 0) {
+      o.a = fma2(u.a, scale, beta); o.b = fma2(u.b, scale, beta);
+      if constexpr (EXTRA) { o.a = add2(o.a, e.a); o.b = add2(o.b, e.b); }
+      o.a = mul2(o.a, slopes(o.a, slope)); o.b = mul2(o.b, slopes(o.b, slope));
     } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if ((uint32_t)(i0 + e) < (uint32_t)len) {
-          p[e] = DIR == 1 && acc ? p[e] + o.v[e] : o.v[e];
-          if constexpr (EXTRA && DIR == 1) { if (dres) dres[w.at() + e] = z.v[e]; }
-        }
+      z = gy;
+      if (!KEEP && !early) {
+        const Quad y = EXTRA ? e : Quad{fma2(u.a, scale, beta), fma2(u.b, scale, beta)};
+        z.a = mul2(gy.a, slopes(y.a, slope)); z.b = mul2(gy.b, slopes(y.b, slope));
+      }
+      o.a = fma2(scale, z.a, fma2(cB, u.a, cC)); o.b = fma2(scale, z.b, fma2(cB, u.b, cC));
     }
-    w.advance();
+    float *p = a.out + (RAGGED ? w.vector() : w.at);
+    const int i0 = RAGGED ? w.first() : 0;
+    if (!RAGGED || (i0 >= 0 && i0 + 4 <= len)) {
+      if (acc) { const Quad old = ldg_quad(p); o.a = add2(old.a, o.a); o.b = add2(old.b, o.b); }
+      stg_stream(p, o);
+      if constexpr (EXTRA && DIR == 1) { if (dres) stg_stream(dres + (p - a.out), z); }
+    } else {
+      const float4 t = floats(o), s = floats(z);
+      auto put = [&](int k, float f, float r) {
+        if ((uint32_t)(i0 + k) < (uint32_t)len) {
+          p[k] = acc ? p[k] + f : f;
+          if constexpr (EXTRA && DIR == 1) { if (dres) dres[(p - a.out) + k] = r; }
+        }
+      };
+      put(0, t.x, s.x); put(1, t.y, s.y); put(2, t.z, s.z); put(3, t.w, s.w);
+    }
+    w.advance(g);
+  };
+  if constexpr (KEEP) {
+    tmem_wait_st();      // what this warp stored in the reduce visits
+    uint32_t i = 0;
+    if constexpr (DIR == 0) {
+      auto put = [&](const Quad &x, uint32_t j) {
+        if (j >= cnt) return;
+        Quad e = x;
+        if constexpr (EXTRA) { e = lds_quad(ad); ad += kVecStride; }
+        one(x, x, e);
+      };
+      if constexpr (!RAGGED) {
+        for (; i + 4 <= steps; i += 4, tm += 16) {
+          Quad x0, x1, x2, x3;
+          tmem_ld(tm, x0, x1, x2, x3);
+          put(x0, i); put(x1, i + 1); put(x2, i + 2); put(x3, i + 3);
+          __syncwarp();
+        }
+      }
+      if constexpr (!RAGGED) {
+        if (i + 2 <= steps) {
+          Quad x0, x1;
+          tmem_ld(tm, x0, x1);
+          put(x0, i); put(x1, i + 1);
+          __syncwarp();
+          i += 2; tm += 8;
+        }
+      }
+      for (; i < steps; ++i, tm += 4) {
+        Quad x0;
+        tmem_ld(tm, x0);
+        put(x0, i);
+        __syncwarp();
+      }
+    } else {
+      if constexpr (!RAGGED) {
+        for (; i + 2 <= steps; i += 2, tm += 16) {
+          Quad d0, z0, d1, z1;
+          tmem_ld(tm, d0, z0, d1, z1);
+          one(d0, z0, d0);
+          if (i + 1 < cnt) one(d1, z1, d1);
+          __syncwarp();
+        }
+      }
+      for (; i < steps; ++i, tm += 8) {
+        Quad d0, z0;
+        tmem_ld(tm, d0, z0);
+        if (i < cnt) one(d0, z0, d0);
+        __syncwarp();
+      }
+    }
+  } else {
+    for (uint32_t i = 0; i < cnt; ++i, ax += kVecStride, ad += kVecStride) {
+      const Quad x = lds_quad(ax);
+      Quad gy = x, e = x;
+      if constexpr (DIR == 1) gy = lds_quad(ad);
+      if constexpr (EXTRA) { if (!early) e = lds_quad(DIR == 1 ? ad + g.slot_floats * 4 : ad); }
+      one(x, gy, e);
+    }
   }
   __syncwarp();
-  if (lane == 0) { mbar_arrive(&ctl->empty[slot]); mbar_arrive(&ctl->coef_empty[coef_q]); }
+  if (lane == 0) { if (!KEEP || kSlotAlways<DIR, EXTRA>) mbar_arrive(&ctl->empty[slot]); mbar_arrive(&ctl->coef_empty[coef_q]); }
 }
 
 // ======================================================================================
@@ -654,15 +708,22 @@ __device__ __forceinline__ void st_relaxed_sys_u64(unsigned long long *p, unsign
 {
   asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-// partial words per lane per round of pull_merge_unit: the backward pass has four times the tiles per unit of the
-// forward pass (smaller tiles), and a round costs a trip to L2; the forward merge does more arithmetic per word
-constexpr int kPullRegsFwd = 8, kPullRegsBwd = 16;
+// Partial words per lane per round of pull_merge_unit.  Rounds are short, so that most words are merged while the last ones
+// are still on their way: [2048,256,56,56] backward with 2 / 3 / 4 / 5 / 8 words 3504 / 3441 / 3493 / 3554 / 3567 us,
+// [256,64,112,112] forward 284 / 275 / 273 / 270 / 313.  (One word per block and unit instead of one per tile makes the merge
+// shorter still, but all blocks then poll a few lines while all blocks write them: 4026 us, and 3673 with the words 32 bytes
+// apart.)
+constexpr int kPullRegsFwd = 4, kPullRegsBwd = 3;
 
 // Whole warp.  Returns false when the wait ran out (abort raised).  On success c0 / c1 hold the
 // unit's coefficients in every lane; `owner` makes lane 0 write the per-channel outputs.
+// The merge runs in every block for every unit, on the way from the last delivery to the first apply: sums about one shift
+// in a single pass, no double precision division (inv_local and inv_total: reciprocals of this GPU's and of all GPUs' elements
+// per channel).  With two passes and three divisions a merge took 2800 cycles after its last word had come, in the forward
+// pass a third of the kernel's time.
 template <int DIR>
-__device__ __forceinline__ bool pull_merge_unit(const FusedArgs &a, RingCtl *ctl, uint32_t *status, uint32_t u, bool owner,
-                                                float4 &c0, float4 &c1)
+__device__ __forceinline__ bool pull_merge_unit(const FusedArgs &a, RingCtl *ctl, uint32_t *status,
+                                                uint32_t u, bool owner, double inv_local, double inv_total, float4 &c0, float4 &c1)
 {
   constexpr int kPullRegs = DIR == 0 ? kPullRegsFwd : kPullRegsBwd;
   const Plan &P = a.plan;
@@ -674,13 +735,26 @@ __device__ __forceinline__ bool pull_merge_unit(const FusedArgs &a, RingCtl *ctl
   float mean_in = 0.f, var_in = 1.f;
   if constexpr (DIR == 1) { mean_in = a.mean_in[u]; var_in = a.var_in[u]; }
   Moments64 tot{0.0, 0.0, 0.0};
-  double s1 = 0.0, s2 = 0.0;
+  double s1 = 0.0, s2 = 0.0, K = 0.0;      // forward: sums about K, the mean of the first partial
   const long long t0 = clock64();
   // With several GPUs only the unit's owner block needs the local merge (it ships the result to
   // every rank); all other blocks go straight to the exchanged records.
   const bool local = (a.world <= 1) || owner;
   for (uint32_t k0 = 0; local && k0 < T; k0 += 32u * kPullRegs) {
     unsigned long long r[kPullRegs];
+    uint32_t nk[kPullRegs];
+    if constexpr (DIR == 0) {
+#pragma unroll
+      for (int i = 0; i < kPullRegs; ++i) {
+        const uint32_t k = k0 + lane + 32u * i;
+        uint32_t sb = k, piece = 0;
+        if (P.pieces != 1) { sb = k / P.pieces; piece = k - sb * P.pieces; }
+        const uint32_t n0 = sb * P.rows_per_tile, col0 = piece * P.piece_len;
+        const uint32_t rows = (P.N - n0 < P.rows_per_tile) ? (P.N - n0) : P.rows_per_tile;
+        const uint32_t len = (P.dim0 - col0 < P.piece_len) ? (P.dim0 - col0) : P.piece_len;
+        nk[i] = k < T ? rows * len : 0u;
+      }
+    }
     for (;;) {
       bool all = true;
 #pragma unroll
@@ -699,36 +773,14 @@ __device__ __forceinline__ bool pull_merge_unit(const FusedArgs &a, RingCtl *ctl
       if (__shfl_sync(0xffffffffu, stop, 0)) return false;
     }
     if constexpr (DIR == 0) {
-      // element count of partial k, from the tile geometry (no division when rows are not split)
-      auto count_of = [&](uint32_t k) -> float {
-        if (k >= T) return 0.f;
-        uint32_t sb = k, piece = 0;
-        if (P.pieces != 1) { sb = k / P.pieces; piece = k - sb * P.pieces; }
-        const uint32_t n0 = sb * P.rows_per_tile, col0 = piece * P.piece_len;
-        const uint32_t rows = (P.N - n0 < P.rows_per_tile) ? (P.N - n0) : P.rows_per_tile;
-        const uint32_t len = (P.dim0 - col0 < P.piece_len) ? (P.dim0 - col0) : P.piece_len;
-        return (float)(rows * len);
-      };
-      float nk[kPullRegs];
-      double sn = 0.0, sm = 0.0;
+      if (k0 == 0) K = (double)__shfl_sync(0xffffffffu, __uint_as_float((uint32_t)r[0]), 0);
 #pragma unroll
       for (int i = 0; i < kPullRegs; ++i) {
-        nk[i] = count_of(k0 + lane + 32u * i);
-        const double mk = (double)__uint_as_float((uint32_t)(r[i] & 0xffffffffull));
-        sn += (double)nk[i]; sm = fma((double)nk[i], mk, sm);
+        if (nk[i]) {
+          const double n = (double)nk[i], d = (double)__uint_as_float((uint32_t)r[i]) - K;
+          s1 = fma(n, d, s1); s2 += fma(n * d, d, (double)__uint_as_float((uint32_t)(r[i] >> 32)));
+        }
       }
-      sn = warp_sum_all(sn); sm = warp_sum_all(sm);
-      const double mean = sm / sn;
-      double sq = 0.0;
-#pragma unroll
-      for (int i = 0; i < kPullRegs; ++i) {
-        const double mk = (double)__uint_as_float((uint32_t)(r[i] & 0xffffffffull));
-        const double m2 = (double)__uint_as_float((uint32_t)(r[i] >> 32));
-        const double d = mk - mean;
-        if (nk[i] > 0.f) sq += m2 + (double)nk[i] * d * d;
-      }
-      sq = warp_sum_all(sq);
-      tot = merge64(tot, Moments64{sn, mean, sq});
     } else {
 #pragma unroll
       for (int i = 0; i < kPullRegs; ++i) {
@@ -740,7 +792,13 @@ __device__ __forceinline__ bool pull_merge_unit(const FusedArgs &a, RingCtl *ctl
       }
     }
   }
-  if constexpr (DIR == 1) { if (local) { s1 = warp_sum_all(s1); s2 = warp_sum_all(s2); } }
+  if (local) {
+    s1 = warp_sum_all(s1); s2 = warp_sum_all(s2);
+    if constexpr (DIR == 0) {
+      const double m = s1 * inv_local;
+      tot = Moments64{(double)a.plan.dim0 * (double)a.plan.N, K + m, not_below_zero(s2 - s1 * m)};
+    }
+  }
   if (a.world > 1) {
     // ---- exchange between GPUs.  A record is three 8-byte words (value in the low half, the
     // call's epoch in the high half): every word validates itself, so plain peer stores suffice
@@ -795,7 +853,7 @@ __device__ __forceinline__ bool pull_merge_unit(const FusedArgs &a, RingCtl *ctl
   }
   if constexpr (DIR == 0) {
     const float mf = (float)tot.mean;
-    const float vf = (float)(tot.m2 / tot.n + (double)a.epsilon);     // biased, epsilon folded in (batch_norm.cu:160)
+    const float vf = (float)(tot.m2 * inv_total + (double)a.epsilon);     // biased, epsilon folded in (batch_norm.cu:160)
     c0 = make_float4(mf, gm * inv_std(vf), bt, 0.f);
     c1 = make_float4(0.f, 0.f, 0.f, 0.f);
     if (owner && lane == 0) {
@@ -807,9 +865,8 @@ __device__ __forceinline__ bool pull_merge_unit(const FusedArgs &a, RingCtl *ctl
     const float r = inv_std(var_in);
     const double rs2 = (double)r * s2;                       // sum(dz * xhat)
     const double A = (double)gm * (double)r;
-    const double invM = 1.0 / a.count_total;
     c0 = make_float4(mean_in, gm * r, bt, 0.f);
-    c1 = make_float4((float)(-A * (double)r * rs2 * invM), (float)(-A * s1 * invM), 0.f, 0.f);
+    c1 = make_float4((float)(-A * (double)r * rs2 * inv_total), (float)(-A * s1 * inv_total), 0.f, 0.f);
     if (owner && lane == 0) {
       if (a.dbeta) a.dbeta[u] = (float)s1;
       if (a.dgamma) a.dgamma[u] = (float)rs2;
@@ -844,34 +901,45 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  if (g.keep_slots && warp == 0) { __syncwarp(); tmem_alloc(&ctl->tmem); tmem_fence_before(); }
   __syncthreads();
+  if (g.keep_slots) tmem_fence_after();
 
-  Sched sc; sc.init(a);
+  Sched sc; sc.init(a, g);
   uint32_t kind;
 
   if (warp < kConsumers / 32) {
     // ------------------------------------------------------------------ consumers
-    uint32_t nres = 0, ncoef = 0;             // reduce count, apply count
     uint32_t slot = g.slots - 1, par = 1;     // ring position, stepped without divisions
-    TileRange tr;
-    while (sc.next_range(P, kind, tr)) {
-      if (++slot == g.slots) { slot = 0; par ^= 1u; }
-      if (kind == 0) {
-        const uint32_t q = nres % kResQ, qpar = (nres / kResQ) & 1u; ++nres;
+    uint32_t qres = 0, rpar = 1, qcoef = 0, cpar = 0;      // mailbox positions
+    const uint32_t look = sc.look, steps = sc.my_tiles + look;
+    const uint32_t n_red = sc.do_reduce ? sc.my_tiles : 0, first_app = sc.do_apply ? look : steps;
+    for (uint32_t s = 0; s < steps; ++s) {
+      if (s < n_red) {
+        if (++slot == g.slots) { slot = 0; par ^= 1u; }
         // the partial mailbox entry must have been emptied by the delivery warp (first pass: free)
-        bool ok = warp_wait(&ctl->res_empty[q], qpar ^ 1u, ctl, status, ANODE_ST_WAIT_STATS);
+        bool ok = warp_wait(&ctl->res_empty[qres], rpar, ctl, status, ANODE_ST_WAIT_STATS);
         ok = ok && warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS);
         if (!ok) break;                                 // warps are independent: no barrier to honour
-        if constexpr (RAGGED) warp_reduce_ragged<DIR, EXTRA>(a, g, sm, ctl, tr, slot, res_box(sm, g, q));
-        else warp_reduce_R<DIR, EXTRA>(a, g, sm, ctl, tr, slot, res_box(sm, g, q));
-        if (lane == 0) mbar_arrive(&ctl->res_full[q]);
-      } else {
-        const uint32_t q = ncoef % kCoefQ, qpar = (ncoef / kCoefQ) & 1u; ++ncoef;
-        bool ok = warp_wait(&ctl->coef_full[q], qpar, ctl, status, ANODE_ST_WAIT_STATS);
-        ok = ok && warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS);
-        if (!ok) break;
-        if constexpr (RAGGED) warp_apply_ragged<DIR, EXTRA>(a, g, sm, ctl, tr, slot, coef_box(sm, g, P.cb, q), q);
-        else warp_apply_R<DIR, EXTRA>(a, g, sm, ctl, tr, slot, coef_box(sm, g, P.cb, q), q);
+        const uint4 d = *reinterpret_cast<const uint4 *>(slot_side<DIR, EXTRA>(sm, g, slot));
+        float4 *res = res_box(sm, g, qres);
+        if (d.x >> 16) visit_reduce<DIR, EXTRA, RAGGED, true>(a, g, sm, ctl, d, slot, res);
+        else visit_reduce<DIR, EXTRA, RAGGED, false>(a, g, sm, ctl, d, slot, res);
+        if (lane == 0) mbar_arrive(&ctl->res_full[qres]);
+        if (++qres == kResQ) { qres = 0; rpar ^= 1u; }
+      }
+      if (s >= first_app) {
+        if (!warp_wait(&ctl->coef_full[qcoef], cpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
+        const float4 *coef = coef_box(sm, g, qcoef);
+        const uint4 d = *reinterpret_cast<const uint4 *>(coef + 2);
+        const bool kept = (d.x >> 16) != 0;
+        if (!kept || kSlotAlways<DIR, EXTRA>) {
+          if (++slot == g.slots) { slot = 0; par ^= 1u; }
+          if (!warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS)) break;
+        }
+        if (kept) visit_apply<DIR, EXTRA, RAGGED, true>(a, g, sm, ctl, d, slot, coef, qcoef);
+        else visit_apply<DIR, EXTRA, RAGGED, false>(a, g, sm, ctl, d, slot, coef, qcoef);
+        if (++qcoef == kCoefQ) { qcoef = 0; cpar ^= 1u; }
       }
     }
   } else if (warp == kConsumers / 32) {
@@ -898,6 +966,11 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
     };
     auto finish_side = [&](const float4 &r) { return make_float4(r.x, r.z * inv_std(r.y), r.w, 0.f); };
     while (ok && sc.next_range(P, kind, tr)) {
+      const bool kept = sc.keep.kept();
+      if (kind == 1) {
+        ++applied;
+        if (kept && !kSlotAlways<DIR, EXTRA>) continue;      // from tensor memory
+      }
       ++k;
       if (++slot == g.slots) { slot = 0; par ^= 1u; }
       // (one lane polls here: a producer that reacts sooner was measured slower where the window between the two
@@ -905,13 +978,13 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
       uint32_t okw = 1;
       if (lane == 0) okw = mbar_wait(&ctl->empty[slot], par ^ 1u, ctl, status, ANODE_ST_WAIT_STATS) ? 1u : 0u;
       if constexpr (DIR == 1 && EXTRA) {
-        // the dz this visit reads back was stored by visit kr, which must have been given back: implied by the wait
-        // above unless fewer than `slots` visits lie in between (blocks with a few tiles)
-        if (kind == 1) {
-          const uint32_t kr = applied + (applied > sc.look ? applied - sc.look : 0u);
-          if (lane == 0 && okw && a.dres_early && k - 1 - kr < g.slots)
+        // the dz this visit reads back was stored by visit kr (counting those that use a slot), which must have been
+        // given back: implied by the wait above unless fewer than `slots` visits lie in between
+        if (kind == 1 && lane == 0 && okw && a.dres_early) {
+          const uint32_t j = applied - 1, before = j > sc.look ? j - sc.look : 0u;
+          const uint32_t kr = j + before - kept_before(g, before);
+          if (k - 1 - kr < g.slots)
             okw = mbar_wait(&ctl->empty[kr % g.slots], (kr / g.slots) & 1u, ctl, status, ANODE_ST_WAIT_STATS) ? 1u : 0u;
-          ++applied;
         }
       }
       ok = __shfl_sync(0xffffffffu, okw, 0) != 0;     // one lane decides for the warp
@@ -928,10 +1001,11 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
           next_c = tr.c0 + 1 < P.C ? tr.c0 + 1 : tr.c0;
           next_raw = load_side_raw(next_c); next_pending = true; next_age = 0;
         }
-        if (lane == 0) slot_side<1, EXTRA>(sm, g, slot)[0] = side_v;
+        if (lane == 0) slot_side<1, EXTRA>(sm, g, slot)[1] = side_v;
       }
+      if (kind == 0 && lane == 0) *reinterpret_cast<uint4 *>(slot_side<DIR, EXTRA>(sm, g, slot)) = describe(tr, RAGGED, sc.keep);
       __syncwarp();
-      const uint64_t pol = (kind == 0 && a.mode == MODE_FUSED) ? keep : drop;
+      const uint64_t pol = (kind == 0 && a.mode == MODE_FUSED && !kept) ? keep : drop;
       // the visit's tensors: x; dy, or the dz that the reduce visit stored; residual or saved output where it is needed
       const float *p1 = nullptr, *p2 = nullptr;
       uint64_t pol1 = pol;
@@ -945,7 +1019,8 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
       } else if constexpr (EXTRA) {
         if (kind == 1) p1 = a.res;
       }
-      const uint32_t planes = 1u + (p1 ? 1u : 0u) + (p2 ? 1u : 0u);
+      const bool p0 = !kSlotAlways<DIR, EXTRA> || kind == 0 || !kept;
+      const uint32_t planes = (p0 ? 1u : 0u) + (p1 ? 1u : 0u) + (p2 ? 1u : 0u);
       // every row is fetched as several bulk copies (one per lane at a time), so that a tile made of
       // one long row still has many copies in flight
       if constexpr (!RAGGED) {
@@ -958,7 +1033,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
           const uint32_t nb = row_bytes - o < kCopyBytes ? row_bytes - o : kCopyBytes;
           const size_t goff = (size_t)tr.base + (size_t)r * rs + o / 4;
           float *dst = xs + (size_t)r * tr.len + o / 4;
-          bulk_g2s(dst, a.x + goff, nb, &ctl->full[slot], pol);
+          if (p0) bulk_g2s(dst, a.x + goff, nb, &ctl->full[slot], pol);
           if (p1) bulk_g2s(dst + g.slot_floats, p1 + goff, nb, &ctl->full[slot], pol1);
           if (p2) bulk_g2s(dst + 2 * g.slot_floats, p2 + goff, nb, &ctl->full[slot], pol1);
         }
@@ -981,7 +1056,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
         if (tail && last + tr.len == total && lane < tail) {
           const uint64_t src = (total & ~3ull) + lane;
           float *dst = xs + 4 * (size_t)per_row * (tr.rows - 1) + (src - (last & ~3ull));
-          *dst = __ldcg(a.x + src);
+          if (p0) *dst = __ldcg(a.x + src);
           if (p1) dst[g.slot_floats] = __ldcg(p1 + src);
           if (p2) dst[2 * g.slot_floats] = __ldcg(p2 + src);
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // (before a later copy into this slot)
@@ -994,7 +1069,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
           const uint32_t nb = span(r, start);
           float *dst = xs + 4 * (size_t)per_row * r;
           if (nb) {
-            bulk_g2s(dst, a.x + start, nb, &ctl->full[slot], pol);
+            if (p0) bulk_g2s(dst, a.x + start, nb, &ctl->full[slot], pol);
             if (p1) bulk_g2s(dst + g.slot_floats, p1 + start, nb, &ctl->full[slot], pol1);
             if (p2) bulk_g2s(dst + 2 * g.slot_floats, p2 + start, nb, &ctl->full[slot], pol1);
           }
@@ -1013,123 +1088,101 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
     }
   } else if (warp == kConsumers / 32 + 1) {
     // ------------------------------------------------------------------ delivery warp
-    // Reduce visit j of this block is tile b + j*G.  Each turn serves every partial that waits,
-    // one lane per partial, so the fences and atomics of several tiles overlap.
+    // Reduce visit j of this block is tile b + j*G.  The consumer warps' partials of a tile are merged in a fixed order.
     const uint32_t n_red = sc.do_reduce ? sc.my_tiles : 0;
-    uint32_t nres = 0;
-    while (nres < n_red) {
-      // sleep on the next entry's barrier (no polling loop competing with the consumers for issue
-      // slots), then take along whatever else has arrived in the meantime
-      if (!warp_wait(&ctl->res_full[nres % kResQ], (nres / kResQ) & 1u, ctl, status, ANODE_ST_WAIT_STATS)) break;
-      const uint32_t jd = nres + lane;
-      const bool d_ok = lane < kResQ && jd < n_red && mbar_test(&ctl->res_full[jd % kResQ], (jd / kResQ) & 1u);
-      const uint32_t d_mask = __ballot_sync(0xffffffffu, d_ok);
-      uint32_t nd = __ffs(~d_mask) - 1;                               // in order: leading run of ones
-      if (nd > kPerTurn) nd = kPerTurn;
-      if (nd) {
-        {
-          // entry e is served by lanes 8e .. 8e+7: one warp partial each, merged in a fixed order
-          const uint32_t e = lane / kCWarps, w = lane % kCWarps;
-          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (e < nd) v = res_box(sm, g, (nres + e) % kResQ)[w];
-          if constexpr (DIR == 0) {
-            Moments m{v.x, v.y, v.z};
+    uint32_t q = 0, qpar = 0, tile = sc.b;
+    for (uint32_t j = 0; j < n_red; ++j) {
+      if (!warp_wait(&ctl->res_full[q], qpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
+      float4 v = lane < kCWarps ? res_box(sm, g, q)[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+      if constexpr (DIR == 0) {
+        Moments m{v.x, v.y, v.z};
 #pragma unroll
-            for (int o = (int)kCWarps / 2; o > 0; o >>= 1) {
-              Moments c;
-              c.n = __shfl_down_sync(0xffffffffu, m.n, o, kCWarps);
-              c.mean = __shfl_down_sync(0xffffffffu, m.mean, o, kCWarps);
-              c.m2 = __shfl_down_sync(0xffffffffu, m.m2, o, kCWarps);
-              m = merge(m, c);
-            }
-            v = make_float4(m.n, m.mean, m.m2, 0.f);
-          } else {
+        for (int o = (int)kCWarps / 2; o > 0; o >>= 1) {
+          Moments c;
+          c.n = __shfl_down_sync(0xffffffffu, m.n, o, kCWarps);
+          c.mean = __shfl_down_sync(0xffffffffu, m.mean, o, kCWarps);
+          c.m2 = __shfl_down_sync(0xffffffffu, m.m2, o, kCWarps);
+          m = merge(m, c);
+        }
+        v = make_float4(m.n, m.mean, m.m2, 0.f);
+      } else {
 #pragma unroll
-            for (int o = (int)kCWarps / 2; o > 0; o >>= 1) {
-              v.x += __shfl_down_sync(0xffffffffu, v.x, o, kCWarps);
-              v.y += __shfl_down_sync(0xffffffffu, v.y, o, kCWarps);
-            }
-          }
-          if (a.mode == MODE_FUSED) {
-            // one tagged 8-byte word per tile; nothing else to do for a delivery
-            if (e < nd && w == 0) {
-              const size_t t = (size_t)(sc.b + (nres + e) * sc.G);
-              const float lo = DIR == 0 ? v.y : v.x, hi = DIR == 0 ? v.z : v.y;
-              st_relaxed_gpu_u64(tag_buf(a, ctl->parity) + t, pack_rec(lo, __uint_as_float(__float_as_uint(hi) | 1u)));
-              tag_buf(a, ctl->parity ^ 1u)[t] = 0ull;
-            }
-            __syncwarp();
-            if (lane < nd) mbar_arrive(&ctl->res_empty[(nres + lane) % kResQ]);
-            nres += nd;
-            continue;
-          }
-          if (e < nd && w == 0) __stcg(ws_f4(a, P.off_part) + (size_t)(sc.b + (nres + e) * sc.G), v);
+        for (int o = (int)kCWarps / 2; o > 0; o >>= 1) {
+          v.x += __shfl_down_sync(0xffffffffu, v.x, o, kCWarps);
+          v.y += __shfl_down_sync(0xffffffffu, v.y, o, kCWarps);
         }
-        __syncwarp();
-        uint32_t last = 0, unit = 0;
-        if (lane < nd) {
-          const uint32_t j = nres + lane;
-          unit = (sc.b + j * sc.G) / P.tiles_per_unit;
-          mbar_arrive(&ctl->res_empty[j % kResQ]);
-          // release: the partial stored above is visible before the count; acquire: whoever sees the
-          // full count also sees every partial counted before
-          uint32_t old;
-          asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(done + unit) : "memory");
-          last = (old + 1 == P.tiles_per_unit) ? 1u : 0u;
-        }
-        uint32_t lmask = __ballot_sync(0xffffffffu, last != 0);
-        while (lmask) {
-          const uint32_t src = __ffs(lmask) - 1; lmask &= lmask - 1;
-          const uint32_t u = __shfl_sync(0xffffffffu, unit, src);
-          warp_finish_unit_R<DIR>(a, u);
-          if (lane == 0) done[u] = 0;
-        }
-        nres += nd;
       }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl->res_empty[q]);
+      if (++q == kResQ) { q = 0; qpar ^= 1u; }
+      if (a.mode == MODE_FUSED) {
+        // one tagged 8-byte word per tile; nothing else to do for a delivery
+        if (lane == 0) {
+          const float lo = DIR == 0 ? v.y : v.x, hi = DIR == 0 ? v.z : v.y;
+          st_relaxed_gpu_u64(tag_buf(a, ctl->parity) + tile, pack_rec(lo, __uint_as_float(__float_as_uint(hi) | 1u)));
+          tag_buf(a, ctl->parity ^ 1u)[tile] = 0ull;
+        }
+        tile += sc.G;
+        continue;
+      }
+      const uint32_t unit = tile / P.tiles_per_unit;
+      uint32_t last = 0;
+      if (lane == 0) {
+        __stcg(ws_f4(a, P.off_part) + tile, v);
+        // release: the partial stored above is visible before the count; acquire: whoever sees the
+        // full count also sees every partial counted before
+        uint32_t old;
+        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(old) : "l"(done + unit) : "memory");
+        last = (old + 1 == P.tiles_per_unit) ? 1u : 0u;
+      }
+      if (__shfl_sync(0xffffffffu, last, 0)) {
+        warp_finish_unit_R<DIR>(a, unit);
+        if (lane == 0) done[unit] = 0;
+      }
+      tile += sc.G;
     }
   } else {
     // ------------------------------------------------------------------ coefficient warp
     // Apply visit j of this block is tile b + j*G (one channel per unit).
     const uint32_t n_app = sc.do_apply ? sc.my_tiles : 0;
-    uint32_t ncoef = 0;
-    if (a.mode == MODE_FUSED) {
-      // merge each unit's partials here (see pull_merge_unit); consecutive visits of the same unit reuse
-      // the result
-      uint32_t have = 0xffffffffu;
-      float4 c0 = make_float4(0.f, 0.f, 0.f, 0.f), c1 = c0;
-      while (ncoef < n_app) {
-        if (!warp_wait(&ctl->coef_empty[ncoef % kCoefQ], ((ncoef / kCoefQ) & 1u) ^ 1u, ctl, status, ANODE_ST_WAIT_STATS)) break;
-        const uint32_t t = sc.b + ncoef * sc.G, u = t / P.tiles_per_unit;
-        if (u != have) {
+    const double inv_local = 1.0 / ((double)P.dim0 * (double)P.N), inv_total = 1.0 / a.count_total;
+    uint32_t q = 0, qpar = 1;
+    // fused mode: each unit's partials are merged here (see pull_merge_unit), and consecutive visits of the same unit reuse
+    // the result.  Apply pass of the three-launch form: the coefficients were prepared by the exchange / merge kernel.
+    uint32_t have = 0xffffffffu;
+    float4 c0 = make_float4(0.f, 0.f, 0.f, 0.f), c1 = c0;
+    for (uint32_t n = 0; n < n_app; ++n) {
+      if (!warp_wait(&ctl->coef_empty[q], qpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
+      const TileRange tr = sc.it_apply.range(P);
+      const uint32_t u = tr.unit;
+      if (u != have) {
+        if (a.mode == MODE_FUSED) {
           // the block that owns the unit's first tile also writes the per-channel outputs
-          if (!pull_merge_unit<DIR>(a, ctl, status, u, t == u * P.tiles_per_unit, c0, c1)) break;
-          have = u;
+          if (!pull_merge_unit<DIR>(a, ctl, status, u, sc.it_apply.tile() == u * P.tiles_per_unit, inv_local, inv_total, c0, c1)) break;
+        } else {
+          const float4 *coef = ws_f4(a, P.off_coef) + 2 * (size_t)u;
+          c0 = __ldcg(coef); c1 = __ldcg(coef + 1);
         }
-        if (lane == 0) {
-          float4 *box = coef_box(sm, g, P.cb, ncoef % kCoefQ);
-          box[0] = c0; box[1] = c1;
-          mbar_arrive(&ctl->coef_full[ncoef % kCoefQ]);
-        }
-        ++ncoef;
+        have = u;
       }
-    } else {
-      // apply pass of the three-launch form: the coefficients were prepared by the exchange / merge kernel
-      while (ncoef < n_app) {
-        if (!warp_wait(&ctl->coef_empty[ncoef % kCoefQ], ((ncoef / kCoefQ) & 1u) ^ 1u, ctl, status, ANODE_ST_WAIT_STATS)) break;
-        const uint32_t c = (sc.b + ncoef * sc.G) / P.tiles_per_unit;
-        if (lane == 0) {
-          const float4 *coef = ws_f4(a, P.off_coef) + 2 * (size_t)c;
-          float4 *box = coef_box(sm, g, P.cb, ncoef % kCoefQ);
-          box[0] = __ldcg(coef); box[1] = __ldcg(coef + 1);
-          mbar_arrive(&ctl->coef_full[ncoef % kCoefQ]);
-        }
-        ++ncoef;
+      if (lane == 0) {
+        float4 *box = coef_box(sm, g, q);
+        box[0] = make_float4(c0.x, c0.y, c0.z, c1.x); box[1] = make_float4(c1.y, 0.f, 0.f, 0.f);
+        *reinterpret_cast<uint4 *>(box + 2) = describe(tr, RAGGED, sc.keep_apply);
+        mbar_arrive(&ctl->coef_full[q]);
       }
+      sc.it_apply.advance(P); sc.keep_apply.advance();
+      if (++q == kCoefQ) { q = 0; qpar ^= 1u; }
     }
   }
 
   // ---- leave: the last block out lowers the ready flags so that the workspace is clean again
+  if (g.keep_slots) {
+    if (warp < kCWarps) { __syncwarp(); tmem_wait_st(); }
+    tmem_fence_before();
+  }
   __syncthreads();
+  if (g.keep_slots && warp == 0) { tmem_fence_after(); tmem_free(ctl->tmem); }
   if (ctl->abort) {
     if (tid == 0) atomicOr(status, ANODE_ST_ABORTED);
     return;

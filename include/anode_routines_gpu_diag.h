@@ -57,6 +57,13 @@ int anode_gpu_batch_norm_stream_geometry(uint32_t dim0, uint32_t dim1, uint32_t 
  * that window loaded with the "keep" priority, thread blocks, steps between a tile's two visits, tiles. */
 int anode_gpu_batch_norm_tiled_geometry(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, uint32_t *out);
 
+/* Which of a block's tiles stay in tensor memory between their two visits (tiled kernel, one launch per direction).
+ * out (10 values): tiles kept at a time (0: none), whether tile number `tile` of a block is kept, its place, the number
+ * under which consumer warp `warp` is dealt vectors of that place, the warp's first column, kept tiles before this one,
+ * vectors of the largest tile, consumer warps, columns per set of one vector per lane, steps between a tile's two visits. */
+int anode_gpu_batch_norm_tiled_keep(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual,
+                                    uint32_t tile, uint32_t warp, uint32_t *out);
+
 /* Plan of the slice-resident kernel for `planes` tensors per shared-memory slot.  out (16 values): applies,
  * rows per piece, parts per row, floats per part, pieces per channel, blocks per team, teams, grid, pieces
  * per block and channel, slot bytes, slots, resident-ring slots, streaming-ring slots, resident pieces per
