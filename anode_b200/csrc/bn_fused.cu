@@ -310,6 +310,7 @@ int launch_ring(FusedArgs &a, const RingGeom &g_in, int dir, cudaStream_t stream
   }
   a.use_rec = a.mode == MODE_FUSED ? 1u : 0u;
   plan_walk(g, a.plan, ring_pitch(a.plan), ring_warps(dir) * 32);
+  g.copies = ceil_div_u32(16 * ring_pitch(a.plan), kRingCopyBytes);
   g.keep_slots = 0; g.keep_period = 1;
   if (a.mode == MODE_FUSED) ring_keep(a.plan, dir, g);
   // A window larger than what L2 keeps would cycle through it whole (config 3, backward: 67 MB); marking only
@@ -804,10 +805,9 @@ extern "C" int anode_gpu_batch_norm_tiled_keep(uint32_t dim0, uint32_t dim1, uin
   for (int i = 0; i < 10; ++i) out[i] = 0;
   if (!ring_plan_for(dim0, dim1, dim2, true, dir, residual != 0, p, g)) return ANODE_OK;
   ring_keep(p, dir, g);
-  KeepIter it; it.init(g);
-  for (uint32_t t = 0; t < tile; ++t) it.advance();
-  out[0] = g.keep_slots; out[1] = it.kept() ? 1u : 0u; out[2] = it.slot;
-  keep_place(g, it.slot, warp, ring_warps(dir), out[3], out[4]);
+  const Keep k = keep_at(g, tile);
+  out[0] = g.keep_slots; out[1] = k.kept ? 1u : 0u; out[2] = k.slot;
+  keep_place(g, k.slot, warp, ring_warps(dir), out[3], out[4]);
   out[5] = kept_before(g, tile); out[6] = ring_tile_vecs(p); out[7] = ring_warps(dir); out[8] = g.keep_set; out[9] = p.lookahead_steps;
   return ANODE_OK;
 }

@@ -720,6 +720,7 @@ __global__ void __launch_bounds__(kThreads) bn_pipeline_kernel(const FusedArgs a
 constexpr uint32_t kResQ = 4;          // partial mailbox depth
 constexpr uint32_t kCoefQ = 4;         // coefficient mailbox depth
 constexpr uint32_t kCoefBox = 3;       // 16-byte words of its entries
+constexpr uint32_t kRingCopyBytes = 32768;      // largest bulk copy (a tile of several rows has none longer)
 constexpr uint32_t kMaxSlots = 8;
 constexpr uint32_t kRingCtlBytes = 1024;   // room reserved for the kernel's barrier block (RingCtl)
 // 16-byte vectors a row of `len` floats can touch when it starts anywhere within one (tiled kernel, ragged rows)
@@ -735,20 +736,17 @@ struct RingGeom {
   // From one vector of a consumer thread to the next: floats on, columns (vectors) on within rows of walk_per vectors, and
   // floats on top where that passes a row's end; walk_mul divides by walk_per (tiles of one piece of a row: never passes).
   uint32_t walk_mul, walk_per, walk_col, walk_step, walk_wrap;
+  uint32_t copies;         // bulk copies per row of a tile
 };
 constexpr uint32_t kMaxKeepTurns = 64;      // keep_slots * keep_extra is at most this many turns of the warps
 
-// The tiles of a block one after another: evenly spread, keep_slots out of keep_period stay.  `slot` is where.
-struct KeepIter {
-  uint32_t acc, slot, slots, period;
-  ANODE_HD void init(const RingGeom &g) { acc = 0; slot = 0; slots = g.keep_slots; period = g.keep_period; }
-  ANODE_HD bool kept() const { return acc < slots; }
-  ANODE_HD void advance()
-  {
-    acc += slots;
-    if (acc >= period) { acc -= period; if (++slot >= slots) slot = 0; }
-  }
-};
+// A block's tile number n: whether it stays (evenly spread, keep_slots out of keep_period do), and where.
+struct Keep { bool kept; uint32_t slot; };
+ANODE_HD Keep keep_at(const RingGeom &g, uint32_t n)
+{
+  const uint32_t x = n % g.keep_period * g.keep_slots;
+  return Keep{x % g.keep_period < g.keep_slots, x / g.keep_period};
+}
 // Place `slot` as consumer warp `warp` of `warps` sees it: the warp's number in the dealing of the tile's vectors (which
 // starts with another warp for each place, so that the sets beyond whole turns fall on every warp in turn), and its first
 // column among those of its group of four warps.

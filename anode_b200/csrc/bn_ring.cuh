@@ -45,16 +45,12 @@
 #ifndef ANODE_RING_BACKOFF_NS
 #define ANODE_RING_BACKOFF_NS 100
 #endif
-#ifndef ANODE_RING_COPY_BYTES
-#define ANODE_RING_COPY_BYTES 32768
-#endif
 
 namespace anode_b200 {
 namespace ANODE_RING_NS {
 
 constexpr uint32_t kConsumers = ANODE_RING_CONSUMERS;   // consumer threads (a power of two, 256..1024)
 constexpr uint32_t kRingThreads = kConsumers + 96;   // + producer, delivery and coefficient warps
-constexpr uint32_t kCopyBytes = ANODE_RING_COPY_BYTES;   // size of one bulk copy (a multiple of 16)
 constexpr long long kWaitCycles = 3000000000ll;      // about 1.5 s at 2 GHz
 
 struct RingCtl {
@@ -80,9 +76,9 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long *bar)
 {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_expect_tx(unsigned long long *bar, uint32_t bytes)
+__device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, uint32_t bytes)
 {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ bool mbar_test(unsigned long long *bar, uint32_t parity)
 {
@@ -158,42 +154,22 @@ __device__ __forceinline__ void tmem_fence_after() { asm volatile("tcgen05.fence
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // ---- the block's schedule --------------------------------------------------------------------
-// Operation k of a block: steps s = 0, 1, ...; at step s first REDUCE tile s (if any is left), then
-// APPLY tile s - look (if s >= look).  Every role walks this same sequence with its own cursor.
+// The visits of a block: steps s = 0, 1, ...; at step s first REDUCE its tile number s (if any is left), then APPLY number
+// s - look (if s >= look).  Tile number n of the block is tile b + n*G.  Every role walks this same sequence by itself.
 struct Sched {
   uint32_t my_tiles, look, b, G;
-  bool do_reduce, do_apply;
-  uint32_t s, phase;     // phase 0: reduce of step s pending; 1: apply of step s pending
-  TileIter it_reduce, it_apply;     // the reduce visits and the apply visits both walk b, b+G, ...
-  KeepIter keep_reduce, keep_apply;
-  KeepIter keep;                    // of the visit handed out last
-  __device__ __forceinline__ void init(const FusedArgs &a, const RingGeom &g)
+  uint32_t steps, reduces, applies;       // steps, reduce visits, apply visits
+  __device__ __forceinline__ void init(const FusedArgs &a)
   {
-    keep_reduce.init(g); keep_apply.init(g); keep = keep_reduce;
     b = blockIdx.x; G = gridDim.x;
     my_tiles = (b < a.plan.total_tiles) ? (a.plan.total_tiles - b + G - 1) / G : 0;
     look = (a.mode == MODE_FUSED) ? a.plan.lookahead_steps : 0;
-    do_reduce = a.mode != MODE_APPLY; do_apply = a.mode != MODE_STATS;
-    s = 0; phase = 0;
-    it_reduce.init(a.plan, b, G); it_apply.init(a.plan, b, G);
+    steps = my_tiles + look;
+    reduces = a.mode != MODE_APPLY ? my_tiles : 0; applies = a.mode != MODE_STATS ? my_tiles : 0;
   }
-  // Advances to the next operation; returns false at the end.  kind: 0 reduce, 1 apply.
-  __device__ __forceinline__ bool next_range(const Plan &P, uint32_t &kind, TileRange &tr)
-  {
-    for (;;) {
-      if (s >= my_tiles + look) return false;
-      if (phase == 0) {
-        phase = 1;
-        if (do_reduce && s < my_tiles) { kind = 0; tr = it_reduce.range(P); it_reduce.advance(P); keep = keep_reduce; keep_reduce.advance(); return true; }
-      } else {
-        phase = 0;
-        const uint32_t ss = s++;
-        if (do_apply && ss >= look) { kind = 1; tr = it_apply.range(P); it_apply.advance(P); keep = keep_apply; keep_apply.advance(); return true; }
-      }
-    }
-  }
+  __device__ __forceinline__ bool reduce_at(uint32_t s) const { return s < reduces; }
+  __device__ __forceinline__ bool apply_at(uint32_t s) const { return s >= look && s - look < applies; }
 };
-
 
 // dynamic shared memory accessors
 __device__ __forceinline__ float *slot_x(unsigned char *sm, const RingGeom &g, uint32_t slot) { return reinterpret_cast<float *>(sm + g.off_slots + (size_t)slot * g.slot_stride); }
@@ -308,10 +284,17 @@ __device__ __forceinline__ void fence_global_to_bulk() { asm volatile("fence.pro
 
 // A visit, as the service warps describe it to the consumers (16 bytes): its vectors, its place in tensor memory + 1 (0:
 // none), the float offset of its first element (below 2^32, check_dims), floats per row, rows.
-__device__ __forceinline__ uint4 describe(const TileRange &tr, bool ragged, const KeepIter &keep)
+// The service warps work 32 of them out at a time, one per lane: one after another they took the producer a microsecond
+// each, more than its copies, and bounded tiles of less than 32 KB.
+__device__ __forceinline__ uint4 describe(const TileRange &tr, bool ragged, const Keep &keep)
 {
   const uint32_t nvec = (ragged ? ragged_pitch(tr.len) : tr.len / 4) * tr.rows;
-  return make_uint4(nvec | (keep.kept() ? keep.slot + 1u : 0u) << 16, (uint32_t)tr.base, tr.len, tr.rows);
+  return make_uint4(nvec | (keep.kept ? keep.slot + 1u : 0u) << 16, (uint32_t)tr.base, tr.len, tr.rows);
+}
+__device__ __forceinline__ uint4 shfl4(const uint4 &v, uint32_t lane)
+{
+  return make_uint4(__shfl_sync(0xffffffffu, v.x, lane), __shfl_sync(0xffffffffu, v.y, lane), __shfl_sync(0xffffffffu, v.z, lane),
+                    __shfl_sync(0xffffffffu, v.w, lane));
 }
 
 // The visit as one thread sees it: its vectors are tid, tid + kConsumers, ... of the tile's rows laid back to back (`cnt` of
@@ -723,17 +706,13 @@ constexpr int kPullRegsFwd = 4, kPullRegsBwd = 3;
 // pass a third of the kernel's time.
 template <int DIR>
 __device__ __forceinline__ bool pull_merge_unit(const FusedArgs &a, RingCtl *ctl, uint32_t *status,
-                                                uint32_t u, bool owner, double inv_local, double inv_total, float4 &c0, float4 &c1)
+                                                uint32_t u, bool owner, const float4 &in, double inv_local, double inv_total, float4 &c0, float4 &c1)
 {
   constexpr int kPullRegs = DIR == 0 ? kPullRegsFwd : kPullRegsBwd;
   const Plan &P = a.plan;
   const uint32_t lane = threadIdx.x & 31, T = P.tiles_per_unit;
   const unsigned long long *buf = tag_buf(a, ctl->parity) + (size_t)u * T;
-  // inputs that do not depend on the partials: fetch them while waiting
-  const float gm = a.gamma ? a.gamma[u] : 1.0f;
-  const float bt = (a.gamma && a.beta) ? a.beta[u] : 0.0f;
-  float mean_in = 0.f, var_in = 1.f;
-  if constexpr (DIR == 1) { mean_in = a.mean_in[u]; var_in = a.var_in[u]; }
+  const float gm = in.x, bt = in.y;      // gamma, beta; backward: mean, 1 / std
   Moments64 tot{0.0, 0.0, 0.0};
   double s1 = 0.0, s2 = 0.0, K = 0.0;      // forward: sums about K, the mean of the first partial
   const long long t0 = clock64();
@@ -862,10 +841,10 @@ __device__ __forceinline__ bool pull_merge_unit(const FusedArgs &a, RingCtl *ctl
       if (a.run_var) { const float o = a.run_var[u]; a.run_var[u] = o + a.avg_rate * (vf - o); }
     }
   } else {
-    const float r = inv_std(var_in);
+    const float r = in.w;
     const double rs2 = (double)r * s2;                       // sum(dz * xhat)
     const double A = (double)gm * (double)r;
-    c0 = make_float4(mean_in, gm * r, bt, 0.f);
+    c0 = make_float4(in.z, gm * r, bt, 0.f);
     c1 = make_float4((float)(-A * (double)r * rs2 * inv_total), (float)(-A * s1 * inv_total), 0.f, 0.f);
     if (owner && lane == 0) {
       if (a.dbeta) a.dbeta[u] = (float)s1;
@@ -905,17 +884,14 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
   __syncthreads();
   if (g.keep_slots) tmem_fence_after();
 
-  Sched sc; sc.init(a, g);
-  uint32_t kind;
+  Sched sc; sc.init(a);
 
   if (warp < kConsumers / 32) {
     // ------------------------------------------------------------------ consumers
     uint32_t slot = g.slots - 1, par = 1;     // ring position, stepped without divisions
     uint32_t qres = 0, rpar = 1, qcoef = 0, cpar = 0;      // mailbox positions
-    const uint32_t look = sc.look, steps = sc.my_tiles + look;
-    const uint32_t n_red = sc.do_reduce ? sc.my_tiles : 0, first_app = sc.do_apply ? look : steps;
-    for (uint32_t s = 0; s < steps; ++s) {
-      if (s < n_red) {
+    for (uint32_t s = 0; s < sc.steps; ++s) {
+      if (sc.reduce_at(s)) {
         if (++slot == g.slots) { slot = 0; par ^= 1u; }
         // the partial mailbox entry must have been emptied by the delivery warp (first pass: free)
         bool ok = warp_wait(&ctl->res_empty[qres], rpar, ctl, status, ANODE_ST_WAIT_STATS);
@@ -928,7 +904,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
         if (lane == 0) mbar_arrive(&ctl->res_full[qres]);
         if (++qres == kResQ) { qres = 0; rpar ^= 1u; }
       }
-      if (s >= first_app) {
+      if (sc.apply_at(s)) {
         if (!warp_wait(&ctl->coef_full[qcoef], cpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
         const float4 *coef = coef_box(sm, g, qcoef);
         const uint4 d = *reinterpret_cast<const uint4 *>(coef + 2);
@@ -946,31 +922,37 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
     // ------------------------------------------------------------------ producer
     // where the window between the two visits exceeds what L2 keeps, only the fraction that fits is marked "keep"
     const uint64_t keep = g.keep_frac < 1.0f ? policy_keep_fraction(g.keep_frac) : policy_keep(), drop = policy_drop();
-    const uint64_t rs = (uint64_t)P.C * P.dim0;
-    uint32_t k = 0, applied = 0;
+    const uint32_t rs = P.C * P.dim0;                  // float offsets are below 2^32 (check_dims)
+    const uint32_t row0 = lane / g.copies, off0 = (lane - row0 * g.copies) * kRingCopyBytes;      // the lane's copy of a tile
+    uint32_t k = 0;
     uint32_t slot = g.slots - 1, par = 1;
     bool ok = true;
-    TileRange tr;
-    // backward pass: (mean, gamma / std, beta) of the current channel and, fetched ahead, of the next one
-    uint32_t side_c = 0xffffffffu, next_c = 0xffffffffu, next_age = 0;
-    float4 side_v = make_float4(0.f, 0.f, 0.f, 0.f), next_v = side_v, next_raw = side_v;
-    bool next_pending = false;
-    auto load_side_raw = [&](uint32_t c) {      // the loads only; the arithmetic waits until the values are used
-      float4 r = make_float4(0.f, 1.f, 1.f, 0.f);
-      if constexpr (DIR == 1) {
-        r.x = a.mean_in[c]; r.y = a.var_in[c];
-        r.z = a.gamma ? a.gamma[c] : 1.0f;
-        r.w = (a.gamma && a.beta) ? a.beta[c] : 0.0f;
+    // lane l: the visits of tiles n + l, n a multiple of 32; and, backward, (mean, gamma / std, beta) of the tile's channel
+    uint4 red = make_uint4(0, 0, 0, 0), app = red;
+    float4 side = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t v = 0; ok && v < 2 * sc.steps; ++v) {
+      const uint32_t s = v >> 1, kind = v & 1u;
+      if (kind == 0 ? !sc.reduce_at(s) : !sc.apply_at(s)) continue;
+      if (kind == 1 && !kSlotAlways<DIR, EXTRA> && g.keep_slots == g.keep_period) continue;      // all from tensor memory
+      const uint32_t n = kind == 0 ? s : s - sc.look;
+      float4 raw = make_float4(0.f, 1.f, 1.f, 0.f);
+      const bool fresh = (n & 31u) == 0u;
+      if (fresh) {
+        uint4 d = make_uint4(0, 0, 0, 0);
+        if (n + lane < sc.my_tiles) {
+          const TileRange tr = tile_range(P, sc.b + (n + lane) * sc.G);
+          d = describe(tr, RAGGED, keep_at(g, n + lane));
+          if (DIR == 1 && kind == 0) {
+            raw.x = a.mean_in[tr.c0]; raw.y = a.var_in[tr.c0];
+            if (a.gamma) raw.z = a.gamma[tr.c0];
+            if (a.gamma && a.beta) raw.w = a.beta[tr.c0];
+          }
+        }
+        if (kind == 0) red = d; else app = d;
       }
-      return r;
-    };
-    auto finish_side = [&](const float4 &r) { return make_float4(r.x, r.z * inv_std(r.y), r.w, 0.f); };
-    while (ok && sc.next_range(P, kind, tr)) {
-      const bool kept = sc.keep.kept();
-      if (kind == 1) {
-        ++applied;
-        if (kept && !kSlotAlways<DIR, EXTRA>) continue;      // from tensor memory
-      }
+      const uint4 d = shfl4(kind == 0 ? red : app, n & 31u);
+      const bool kept = (d.x >> 16) != 0;
+      if (kind == 1 && kept && !kSlotAlways<DIR, EXTRA>) continue;
       ++k;
       if (++slot == g.slots) { slot = 0; par ^= 1u; }
       // (one lane polls here: a producer that reacts sooner was measured slower where the window between the two
@@ -981,8 +963,8 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
         // the dz this visit reads back was stored by visit kr (counting those that use a slot), which must have been
         // given back: implied by the wait above unless fewer than `slots` visits lie in between
         if (kind == 1 && lane == 0 && okw && a.dres_early) {
-          const uint32_t j = applied - 1, before = j > sc.look ? j - sc.look : 0u;
-          const uint32_t kr = j + before - kept_before(g, before);
+          const uint32_t before = n > sc.look ? n - sc.look : 0u;
+          const uint32_t kr = n + before - kept_before(g, before);
           if (k - 1 - kr < g.slots)
             okw = mbar_wait(&ctl->empty[kr % g.slots], (kr / g.slots) & 1u, ctl, status, ANODE_ST_WAIT_STATS) ? 1u : 0u;
         }
@@ -990,21 +972,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
       ok = __shfl_sync(0xffffffffu, okw, 0) != 0;     // one lane decides for the warp
       if (!ok) { --k; break; }
       float *xs = slot_x(sm, g, slot);
-      if (DIR == 1 && kind == 0) {
-        // coefficients of the reduce visit's ReLU mask (one channel per unit here).  They change only when the
-        // block moves on to another channel, and the next channel's are fetched ahead of time: a visit's issue
-        // must not wait for global memory, or the slot stays empty for that long.
-        if (tr.c0 != side_c) {
-          if (tr.c0 == next_c) side_v = next_pending ? finish_side(next_raw) : next_v;
-          else side_v = finish_side(load_side_raw(tr.c0));
-          side_c = tr.c0;
-          next_c = tr.c0 + 1 < P.C ? tr.c0 + 1 : tr.c0;
-          next_raw = load_side_raw(next_c); next_pending = true; next_age = 0;
-        }
-        if (lane == 0) slot_side<1, EXTRA>(sm, g, slot)[1] = side_v;
-      }
-      if (kind == 0 && lane == 0) *reinterpret_cast<uint4 *>(slot_side<DIR, EXTRA>(sm, g, slot)) = describe(tr, RAGGED, sc.keep);
-      __syncwarp();
+      const uint32_t base = d.y, len = d.z, rows = d.w;
       const uint64_t pol = (kind == 0 && a.mode == MODE_FUSED && !kept) ? keep : drop;
       // the visit's tensors: x; dy, or the dz that the reduce visit stored; residual or saved output where it is needed
       const float *p1 = nullptr, *p2 = nullptr;
@@ -1021,62 +989,61 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
       }
       const bool p0 = !kSlotAlways<DIR, EXTRA> || kind == 0 || !kept;
       const uint32_t planes = (p0 ? 1u : 0u) + (p1 ? 1u : 0u) + (p2 ? 1u : 0u);
-      // every row is fetched as several bulk copies (one per lane at a time), so that a tile made of
-      // one long row still has many copies in flight
+      auto fetch = [&](float *dst, uint32_t src, uint32_t bytes) {
+        if (p0) bulk_g2s(dst, a.x + src, bytes, &ctl->full[slot], pol);
+        if (p1) bulk_g2s(dst + g.slot_floats, p1 + src, bytes, &ctl->full[slot], pol1);
+        if (p2) bulk_g2s(dst + 2 * g.slot_floats, p2 + src, bytes, &ctl->full[slot], pol1);
+      };
+      // the copies go out first; the visit's description and the arrival that completes the barrier's count follow
       if constexpr (!RAGGED) {
-        const uint32_t row_bytes = tr.len * 4u;
-        if (lane == 0) mbar_arrive_expect_tx(&ctl->full[slot], row_bytes * tr.rows * planes);
+        // a long row is fetched as several bulk copies (one per lane), so that many are in flight
+        const uint32_t row_bytes = len * 4u;
+        if (lane == 0) mbar_expect_tx(&ctl->full[slot], row_bytes * rows * planes);
         __syncwarp();
-        const uint32_t per_row = (row_bytes + kCopyBytes - 1) / kCopyBytes, ncopies = per_row * tr.rows;
-        for (uint32_t c = lane; c < ncopies; c += 32) {
-          const uint32_t r = c / per_row, o = (c - r * per_row) * kCopyBytes;
-          const uint32_t nb = row_bytes - o < kCopyBytes ? row_bytes - o : kCopyBytes;
-          const size_t goff = (size_t)tr.base + (size_t)r * rs + o / 4;
-          float *dst = xs + (size_t)r * tr.len + o / 4;
-          if (p0) bulk_g2s(dst, a.x + goff, nb, &ctl->full[slot], pol);
-          if (p1) bulk_g2s(dst + g.slot_floats, p1 + goff, nb, &ctl->full[slot], pol1);
-          if (p2) bulk_g2s(dst + 2 * g.slot_floats, p2 + goff, nb, &ctl->full[slot], pol1);
+        if (off0 < row_bytes) {
+          const uint32_t nb = row_bytes - off0 < kRingCopyBytes ? row_bytes - off0 : kRingCopyBytes;
+          for (uint32_t r = row0; r < rows; r += 32) fetch(xs + r * len + off0 / 4, base + r * rs + off0 / 4, nb);
         }
       } else {
         // from the boundary below each row's start to the one above its end, but never past the tensor's own end:
         // the last floats of a tensor whose size is no multiple of four are stored by three lanes instead
-        const uint32_t per_row = ragged_pitch(tr.len);
-        const uint64_t total = rs * P.N;
-        auto span = [&](uint32_t r, uint64_t &start) {      // bytes of row r, and the float it is fetched from
-          const uint64_t first = tr.base + r * rs, whole = total & ~3ull;
-          start = first & ~3ull;
-          uint64_t end = (first + tr.len + 3) & ~3ull;
-          if (end > whole) end = whole;
-          return (uint32_t)(end - start) * 4u;
+        const uint32_t per_row = ragged_pitch(len), total = rs * P.N, whole = total & ~3u;
+        auto span = [&](uint32_t r, uint32_t &start) {      // bytes of row r, and the float it is fetched from
+          const uint32_t first = base + r * rs;
+          start = first & ~3u;
+          return ((first + len >= whole ? whole : (first + len + 3) & ~3u) - start) * 4u;
         };
         uint32_t bytes = 0;
-        for (uint32_t r = lane; r < tr.rows; r += 32) { uint64_t start; bytes += span(r, start); }
+        for (uint32_t r = lane; r < rows; r += 32) { uint32_t start; bytes += span(r, start); }
         bytes = __reduce_add_sync(0xffffffffu, bytes) * planes;
-        const uint64_t last = tr.base + (tr.rows - 1) * rs, tail = total & 3ull;
-        if (tail && last + tr.len == total && lane < tail) {
-          const uint64_t src = (total & ~3ull) + lane;
-          float *dst = xs + 4 * (size_t)per_row * (tr.rows - 1) + (src - (last & ~3ull));
+        const uint32_t last = base + (rows - 1) * rs, tail = total & 3u;
+        if (tail && last + len == total && lane < tail) {
+          const uint32_t src = whole + lane;
+          float *dst = xs + 4 * per_row * (rows - 1) + (src - (last & ~3u));
           if (p0) *dst = __ldcg(a.x + src);
           if (p1) dst[g.slot_floats] = __ldcg(p1 + src);
           if (p2) dst[2 * g.slot_floats] = __ldcg(p2 + src);
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // (before a later copy into this slot)
         }
+        if (lane == 0) mbar_expect_tx(&ctl->full[slot], bytes);
         __syncwarp();
-        if (lane == 0) mbar_arrive_expect_tx(&ctl->full[slot], bytes);
-        __syncwarp();
-        for (uint32_t r = lane; r < tr.rows; r += 32) {
-          uint64_t start;
+        for (uint32_t r = lane; r < rows; r += 32) {
+          uint32_t start;
           const uint32_t nb = span(r, start);
-          float *dst = xs + 4 * (size_t)per_row * r;
-          if (nb) {
-            if (p0) bulk_g2s(dst, a.x + start, nb, &ctl->full[slot], pol);
-            if (p1) bulk_g2s(dst + g.slot_floats, p1 + start, nb, &ctl->full[slot], pol1);
-            if (p2) bulk_g2s(dst + 2 * g.slot_floats, p2 + start, nb, &ctl->full[slot], pol1);
-          }
+          if (nb) fetch(xs + 4 * per_row * r, start, nb);
         }
       }
-      // the values fetched ahead are turned into coefficients one visit later, when they have arrived
-      if (DIR == 1 && next_pending && next_age++ >= 1) { next_v = finish_side(next_raw); next_pending = false; }
+      if (kind == 0) {
+        float4 *box = slot_side<DIR, EXTRA>(sm, g, slot);
+        if constexpr (DIR == 1) {
+          // coefficients of the visit's ReLU mask
+          if (fresh) side = make_float4(raw.x, raw.z * inv_std(raw.y), raw.w, 0.f);
+          if (lane == (n & 31u)) box[1] = side;
+        }
+        if (lane == (n & 31u)) *reinterpret_cast<uint4 *>(box) = d;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl->full[slot]);
     }
     // after an abort: wait (bounded) for copies that were issued but will not be consumed
     if (!ok && lane == 0) {
@@ -1089,9 +1056,8 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
   } else if (warp == kConsumers / 32 + 1) {
     // ------------------------------------------------------------------ delivery warp
     // Reduce visit j of this block is tile b + j*G.  The consumer warps' partials of a tile are merged in a fixed order.
-    const uint32_t n_red = sc.do_reduce ? sc.my_tiles : 0;
     uint32_t q = 0, qpar = 0, tile = sc.b;
-    for (uint32_t j = 0; j < n_red; ++j) {
+    for (uint32_t j = 0; j < sc.reduces; ++j) {
       if (!warp_wait(&ctl->res_full[q], qpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
       float4 v = lane < kCWarps ? res_box(sm, g, q)[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
       if constexpr (DIR == 0) {
@@ -1144,34 +1110,46 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
   } else {
     // ------------------------------------------------------------------ coefficient warp
     // Apply visit j of this block is tile b + j*G (one channel per unit).
-    const uint32_t n_app = sc.do_apply ? sc.my_tiles : 0;
     const double inv_local = 1.0 / ((double)P.dim0 * (double)P.N), inv_total = 1.0 / a.count_total;
     uint32_t q = 0, qpar = 1;
     // fused mode: each unit's partials are merged here (see pull_merge_unit), and consecutive visits of the same unit reuse
     // the result.  Apply pass of the three-launch form: the coefficients were prepared by the exchange / merge kernel.
     uint32_t have = 0xffffffffu;
     float4 c0 = make_float4(0.f, 0.f, 0.f, 0.f), c1 = c0;
-    for (uint32_t n = 0; n < n_app; ++n) {
+    // lane l: the visits of tiles n + l, n a multiple of 32, their channels and these channels' parameters
+    uint4 visit = make_uint4(0, 0, 0, 0);
+    uint32_t unit = 0;
+    float4 in = c0;
+    for (uint32_t n = 0; n < sc.applies; ++n) {
+      const uint32_t at = n & 31u;
+      if (at == 0 && n + lane < sc.my_tiles) {
+        const TileRange tr = tile_range(P, sc.b + (n + lane) * sc.G);
+        visit = describe(tr, RAGGED, keep_at(g, n + lane)); unit = tr.unit;
+        if (a.mode == MODE_FUSED) {
+          in.x = a.gamma ? a.gamma[unit] : 1.0f;
+          in.y = (a.gamma && a.beta) ? a.beta[unit] : 0.0f;
+          if constexpr (DIR == 1) { in.z = a.mean_in[unit]; in.w = inv_std(a.var_in[unit]); }
+        }
+      }
       if (!warp_wait(&ctl->coef_empty[q], qpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
-      const TileRange tr = sc.it_apply.range(P);
-      const uint32_t u = tr.unit;
+      const uint32_t u = __shfl_sync(0xffffffffu, unit, at);
       if (u != have) {
         if (a.mode == MODE_FUSED) {
+          const float4 v = make_float4(__shfl_sync(0xffffffffu, in.x, at), __shfl_sync(0xffffffffu, in.y, at),
+                                       __shfl_sync(0xffffffffu, in.z, at), __shfl_sync(0xffffffffu, in.w, at));
           // the block that owns the unit's first tile also writes the per-channel outputs
-          if (!pull_merge_unit<DIR>(a, ctl, status, u, sc.it_apply.tile() == u * P.tiles_per_unit, inv_local, inv_total, c0, c1)) break;
+          if (!pull_merge_unit<DIR>(a, ctl, status, u, sc.b + n * sc.G == u * P.tiles_per_unit, v, inv_local, inv_total, c0, c1)) break;
         } else {
           const float4 *coef = ws_f4(a, P.off_coef) + 2 * (size_t)u;
           c0 = __ldcg(coef); c1 = __ldcg(coef + 1);
         }
         have = u;
       }
-      if (lane == 0) {
-        float4 *box = coef_box(sm, g, q);
-        box[0] = make_float4(c0.x, c0.y, c0.z, c1.x); box[1] = make_float4(c1.y, 0.f, 0.f, 0.f);
-        *reinterpret_cast<uint4 *>(box + 2) = describe(tr, RAGGED, sc.keep_apply);
-        mbar_arrive(&ctl->coef_full[q]);
-      }
-      sc.it_apply.advance(P); sc.keep_apply.advance();
+      float4 *box = coef_box(sm, g, q);
+      if (lane == at) *reinterpret_cast<uint4 *>(box + 2) = visit;
+      if (lane == 0) { box[0] = make_float4(c0.x, c0.y, c0.z, c1.x); box[1] = make_float4(c1.y, 0.f, 0.f, 0.f); }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl->coef_full[q]);
       if (++q == kCoefQ) { q = 0; qpar ^= 1u; }
     }
   }
