@@ -113,6 +113,7 @@ static const ShapeInfo &shape_info(uint32_t dim0, uint32_t C, uint32_t N)
 Plan plan_for(uint32_t dim0, uint32_t C, uint32_t N, bool aligned16) { return shape_info(dim0, C, N).plan[aligned16 ? 1 : 0]; }
 
 constexpr uint32_t kRingSmemBudget = 227u * 1024u;      // a block's most
+constexpr uint64_t kRingLargeWindowMax = 48ull << 20;     // what L2 keeps of a window between a tile's two visits
 
 // vectors that a row takes in a slot, and those of the largest tile
 static uint32_t ring_pitch(const Plan &p)
@@ -147,6 +148,26 @@ static RingGeom ring_geom(const Plan &p, int dir, bool extra, uint32_t slots, ui
   return g;
 }
 
+// Steps between a tile's two visits: the fewest, and `slack` more for a channel's statistics to come together.  Two, but
+//  - three where a channel has no more tiles than there are blocks, so that each visit waits for another channel: backward
+//    passes of many steps ([256,256,56,56] 414 - 425 -> 393 us), forward passes of few ([64,95,55,55] 41.0 -> 39.3,
+//    [128,256,32,32] 53.6 -> 50.2; at 90 steps equal);
+//  - one in backward passes whose window is over what L2 keeps even with a part of it in tensor memory
+//    ([4,32,128,128,128] 605 -> 572 us; where the window fits one step is slower: [256,64,112,112] 394 -> 450).
+static uint32_t ring_lookahead(const Plan &p, int dir)
+{
+  uint32_t slack = tunables().slack_steps;
+  const uint32_t least = ceil_div_u32(p.tiles_per_unit, p.grid), steps = ceil_div_u32(p.total_tiles, p.grid);
+  if (p.tiles_per_unit <= p.grid && (dir == 1 ? steps >= 32 : steps < 64)) ++slack;
+  if (dir == 1 && slack > 1) {
+    RingGeom g{};
+    plan_keep(g, ring_tile_vecs(p), 2, ring_warps(dir), least + slack);
+    const uint64_t window = (uint64_t)(least + slack) * p.grid * ring_tile_vecs(p) * 32;
+    if (window * (g.keep_period - g.keep_slots) / g.keep_period > kRingLargeWindowMax) slack = 1;
+  }
+  return least + slack;
+}
+
 // Plan for the warp-specialised kernel, or false when it does not apply (scalar paths, tiles that
 // do not fit a slot, too little shared memory): the caller then uses the plain kernel.
 // Plan and geometry for `slots` slots of `slot_floats` floats (per tensor); false when they do not fit.
@@ -171,6 +192,7 @@ static bool ring_plan_with(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool 
     p.rows_per_tile = ceil_div_u32(N, p.sample_blocks);
     p.vec = 4;
   }
+  p.lookahead_steps = ring_lookahead(p, dir);
   // a tile must fit one slot
   const uint64_t tile_max = 4ull * ring_tile_vecs(p);
   if (tile_max > slot_floats) return false;
@@ -189,14 +211,13 @@ static uint64_t ring_window_bytes(const Plan &p, int dir)
 // Backward pass: three slots of larger tiles are faster than four of the standard ones as long as the larger
 // window they make still fits what L2 keeps ([256,256,56,56]: 0.50 -> 0.44 ms; with a 56 MB window 10 % slower).
 constexpr uint32_t kRingLargeSlotsBwd = 3, kRingLargeFloatsBwd = 9408;
-constexpr uint64_t kRingLargeWindowMax = 48ull << 20;     // also the part of a larger window that is marked "keep" (launch_ring)
 
 // The residual epilogue's slots hold a third tensor (a second one in the forward pass, used by the apply visits only).
 #ifndef ANODE_RING_SLOTS_FWD_EXTRA
 #define ANODE_RING_SLOTS_FWD_EXTRA 4
 #endif
 #ifndef ANODE_RING_FLOATS_FWD_EXTRA
-#define ANODE_RING_FLOATS_FWD_EXTRA 6656
+#define ANODE_RING_FLOATS_FWD_EXTRA 9408
 #endif
 #ifndef ANODE_RING_SLOTS_BWD_EXTRA
 #define ANODE_RING_SLOTS_BWD_EXTRA 3
@@ -306,7 +327,7 @@ int launch_ring(FusedArgs &a, const RingGeom &g_in, int dir, cudaStream_t stream
   if (fit == 0) return ANODE_E_LAUNCH;
   if (a.plan.grid > fit) {
     a.plan.grid = fit;
-    a.plan.lookahead_steps = ceil_div_u32(a.plan.tiles_per_unit, a.plan.grid) + tunables().slack_steps;
+    a.plan.lookahead_steps = ring_lookahead(a.plan, dir);
   }
   a.use_rec = a.mode == MODE_FUSED ? 1u : 0u;
   plan_walk(g, a.plan, ring_pitch(a.plan), ring_warps(dir) * 32);

@@ -382,14 +382,10 @@ __device__ __forceinline__ void visit_reduce(const FusedArgs &a, const RingGeom 
                   xs[4 * per_row * rl + ((first + rl * rs) & 3u) + d.z - 1 - d.z / 6]);
       const f32x2 nK = pair(-K);
       Walk w(a, g, first, mine.tid);
-#pragma unroll 2
-      for (uint32_t i = 0; i < steps; ++i, ax += kVecStride, tm += 4) {
-        Quad v = quad(K);
-        if (i < cnt) v = lds_quad(ax);
-        if constexpr (KEEP) { __syncwarp(); tmem_st(tm, v); }
-        const int i0 = i < cnt ? w.first() : len;
+      auto take = [&](const Quad &v, bool live) {
+        const int i0 = live ? w.first() : len;
         Quad e{add2(v.a, nK), add2(v.b, nK)};
-        if (i0 >= 0 && i0 + 4 <= len) {
+        if ((uint32_t)i0 <= (uint32_t)(len - 4)) {
           n += 4;
         } else {      // foreign floats at a row's ends count nothing
           const float4 t = floats(e);
@@ -398,6 +394,20 @@ __device__ __forceinline__ void visit_reduce(const FusedArgs &a, const RingGeom 
         }
         sa = add2(sa, e.a); qa = fma2(e.a, e.a, qa); sb = add2(sb, e.b); qb = fma2(e.b, e.b, qb);
         w.advance(g);
+      };
+      uint32_t i = 0;
+      for (; i + 4 <= steps; i += 4, ax += 4 * kVecStride, tm += 16) {
+        const Quad v0 = lds_quad(ax), v1 = lds_quad(ax + kVecStride), v2 = lds_quad(ax + 2 * kVecStride);
+        Quad v3 = quad(K);
+        if (i + 3 < cnt) v3 = lds_quad(ax + 3 * kVecStride);
+        if constexpr (KEEP) { __syncwarp(); tmem_st(tm, v0, v1, v2, v3); }
+        take(v0, true); take(v1, true); take(v2, true); take(v3, i + 3 < cnt);
+      }
+      for (; i < steps; ++i, ax += kVecStride, tm += 4) {
+        Quad v = quad(K);
+        if (i < cnt) v = lds_quad(ax);
+        if constexpr (KEEP) { __syncwarp(); tmem_st(tm, v); }
+        take(v, i < cnt);
       }
       n = __reduce_add_sync(0xffffffffu, n);
     }
@@ -420,25 +430,28 @@ __device__ __forceinline__ void visit_reduce(const FusedArgs &a, const RingGeom 
     float *dres = EXTRA && a.dres_early ? a.dres : nullptr;
     Walk w(a, g, d.y, mine.tid);          // (unused in the ordinary aligned form)
     f32x2 s1a = 0, s1b = 0, s2a = 0, s2b = 0;
-    // (one vector per tensor at a time: with two in flight the sixteen warps of this pass were measured slower)
-    for (uint32_t i = 0; i < (KEEP ? steps : cnt); ++i, ax += kVecStride, ad += kVecStride) {
-      Quad e{0, 0}, z{0, 0};
-      const bool live = !KEEP || i < cnt;
+    // two vectors at a time; a missing one is (mean, 0), which adds nothing
+    auto load = [&](bool live, Quad &x, Quad &gy, Quad &y) {
+      x = quad(cf.x); gy = quad(0.f); y = gy;
       if (live) {
-        const Quad x = lds_quad(ax), gy = lds_quad(ad);
-        e.a = add2(x.a, nmean); e.b = add2(x.b, nmean);
-        Quad y;
-        if constexpr (EXTRA) y = lds_quad(ad + g.slot_floats * 4);      // residual epilogue: the saved output carries the mask
-        else { y.a = fma2(e.a, scale, beta); y.b = fma2(e.b, scale, beta); }
-        // dz = dy * (float)(y > 0)  (routines_gpu/flat_map.cu:191-192)
-        z.a = mul2(gy.a, slopes(y.a, slope)); z.b = mul2(gy.b, slopes(y.b, slope));
+        x = lds_quad(ax); gy = lds_quad(ad);
+        if constexpr (EXTRA) y = lds_quad(ad + g.slot_floats * 4);
       }
-      if constexpr (KEEP) { __syncwarp(); tmem_st(tm, e, z); tm += 8; }
+      ax += kVecStride; ad += kVecStride;
+    };
+    auto work = [&](const Quad &x, const Quad &gy, Quad y, Quad &e, Quad &z) {
+      e.a = add2(x.a, nmean); e.b = add2(x.b, nmean);
+      // residual epilogue: the saved output carries the mask
+      if constexpr (!EXTRA) { y.a = fma2(e.a, scale, beta); y.b = fma2(e.b, scale, beta); }
+      // dz = dy * (float)(y > 0)  (routines_gpu/flat_map.cu:191-192)
+      z.a = mul2(gy.a, slopes(y.a, slope)); z.b = mul2(gy.b, slopes(y.b, slope));
+    };
+    auto sum = [&](bool live, Quad e, Quad z) {
       if constexpr (!RAGGED) {
         if constexpr (EXTRA) { if (dres && live) stg_quad(dres + w.at, z); }
       } else {
         const int i0 = live ? w.first() : len;
-        if (i0 >= 0 && i0 + 4 <= len) {
+        if ((uint32_t)i0 <= (uint32_t)(len - 4)) {
           if constexpr (EXTRA) { if (dres) stg_quad(dres + w.vector(), z); }
         } else {      // (foreign floats may be anything, an infinity or a NaN too)
           const float4 t = floats(z), u = floats(e);
@@ -458,6 +471,17 @@ __device__ __forceinline__ void visit_reduce(const FusedArgs &a, const RingGeom 
       }
       s1a = add2(s1a, z.a); s2a = fma2(z.a, e.a, s2a); s1b = add2(s1b, z.b); s2b = fma2(z.b, e.b, s2b);
       if constexpr (EXTRA || RAGGED) w.advance(g);
+    };
+    for (uint32_t i = 0; i < steps; i += 2, tm += 16) {
+      const bool l0 = i < cnt, l1 = i + 1 < cnt;
+      Quad x0, g0, y0, x1, g1, y1, e0, z0, e1, z1;
+      load(l0, x0, g0, y0); load(l1, x1, g1, y1);
+      work(x0, g0, y0, e0, z0); work(x1, g1, y1, e1, z1);
+      if constexpr (KEEP) {
+        __syncwarp();
+        if (i + 1 < steps) tmem_st(tm, e0, z0, e1, z1); else tmem_st(tm, e0, z0);
+      }
+      sum(l0, e0, z0); sum(l1, e1, z1);
     }
     if constexpr (EXTRA) { if (dres) fence_global_to_bulk(); }
     __syncwarp();
@@ -504,7 +528,7 @@ __device__ __forceinline__ void visit_apply(const FusedArgs &a, const RingGeom &
     }
     float *p = a.out + (RAGGED ? w.vector() : w.at);
     const int i0 = RAGGED ? w.first() : 0;
-    if (!RAGGED || (i0 >= 0 && i0 + 4 <= len)) {
+    if (!RAGGED || (uint32_t)i0 <= (uint32_t)(len - 4)) {
       if (acc) { const Quad old = ldg_quad(p); o.a = add2(old.a, o.a); o.b = add2(old.b, o.b); }
       stg_stream(p, o);
       if constexpr (EXTRA && DIR == 1) { if (dres) stg_stream(dres + (p - a.out), z); }
@@ -531,6 +555,7 @@ __device__ __forceinline__ void visit_apply(const FusedArgs &a, const RingGeom &
         one(x, x, e);
       };
       if constexpr (!RAGGED) {
+        // (ragged rows: [64,95,55,55] residual 60 -> 76 us with four at a time)
         for (; i + 4 <= steps; i += 4, tm += 16) {
           Quad x0, x1, x2, x3;
           tmem_ld(tm, x0, x1, x2, x3);
