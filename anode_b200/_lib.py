@@ -67,6 +67,8 @@ SIGNATURES = {
     "anode_gpu_batch_norm_relu_fused_step_host_3d1_packed_f32":
         (c_int, _D + [f32, f32, c_int] + [vp] * 12 + [vp, size_t, u32] + _T),
     "anode_gpu_batch_norm_act_infer_3d1_packed_f32": (c_int, _D + [f32] + [vp] * 6 + _T),
+    "anode_gpu_batch_normalize_3d1_packed_f32": (c_int, _D + [f32, f32] + [vp] * 6 + _T),
+    "anode_gpu_batch_normalize_adjoint_3d1_packed_f32": (c_int, _D + [vp] * 7 + _T),
     "anode_gpu_online_average_f32": (c_int, [u32, f32, vp, vp] + _T),
     "anode_gpu_sync_unique_id_bytes": (size_t, []),
     "anode_gpu_sync_get_unique_id": (c_int, [vp]),

@@ -1,0 +1,239 @@
+// The front end's own composition (src/ops.rs:999-1014: mean, variance, two running averages, normalize) and its adjoint
+// (the seven ops that src/ops_gpu.rs:4344-4352, 3997-4003 and 3787-3791 emit), one launch each, without scratch memory.
+//
+// A thread-block cluster of up to eight blocks owns a channel and visits it two or three times, the sums of a visit going
+// through distributed shared memory before the next one begins:
+//   forward   sum x -> mean; sum (x-mean)^2 -> var, running averages; y = (x-mean) * rsqrt(var)
+//   adjoint   sums of dy*(x-mean), dy and x-mean -> dvar, dmean; dx = dy*rsqrt(var) + dvar*(x-mean)*2/norm + dmean/norm
+// Where a channel fits the cluster's registers it is read once; else the later visits find it in L2, a cluster's share being
+// small.  Forward passes that the register-resident and streaming kernels of the fused calls serve (short rows) are
+// theirs; the expressions here are the reference's op by op (rsqrtf; mean need not be the batch's in the adjoint).
+//
+// What bounds the composition, [64,128,28,28] (26 MB tensors): seventeen launches and twenty passes over L2 took 114.5 us,
+// composition and adjoint in one launch each and the two ReLU maps 52.
+#include <cooperative_groups.h>
+
+#include "bn_device.cuh"
+#include "bn_host.h"
+
+namespace cg = cooperative_groups;
+
+namespace anode_b200 {
+
+constexpr uint32_t kComposeThreads = 512, kComposeCluster = 8;
+constexpr int kComposeHold = 4;       // vectors per tensor that a thread holds (64 registers: two blocks per SM)
+
+struct ComposeArgs {
+  uint32_t dim0, C, N;
+  float epsilon, avg_rate;
+  const float *x, *dy, *mean_in, *var_in;
+  float *out, *mean, *var, *run_mean, *run_var;      // adjoint: dx, dmean, dvar
+};
+
+// Sums of K values over the threads of the cluster, in a fixed order, to every thread.
+template <int K>
+__device__ __forceinline__ void cluster_sums(cg::cluster_group &cluster, double (&v)[K], double (*part)[kComposeThreads / 32],
+                                             double (*gather)[kComposeCluster])
+{
+  const uint32_t tid = threadIdx.x, cs = cluster.num_blocks(), rank = cluster.block_rank(), warps = blockDim.x / 32;
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    v[k] = warp_sum(v[k]);
+    if ((tid & 31) == 0) part[k][tid >> 5] = v[k];
+  }
+  __syncthreads();
+  if (tid < K * cs) {
+    const uint32_t k = tid / cs, r = tid - k * cs;
+    double s = 0.0;
+    for (uint32_t w = 0; w < warps; ++w) s += part[k][w];
+    cluster.map_shared_rank(&gather[k][0], r)[rank] = s;
+  }
+  cluster.sync();
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    v[k] = 0.0;
+    for (uint32_t r = 0; r < cs; ++r) v[k] += gather[k][r];
+  }
+}
+
+// HOLD: the thread's vectors (at most kComposeHold) stay in registers
+template <int DIR, int VEC, bool HOLD>
+__global__ void __launch_bounds__(kComposeThreads, 2) bn_compose_kernel(const ComposeArgs g)
+{
+  cg::cluster_group cluster = cg::this_cluster();
+  const uint32_t cs = cluster.num_blocks(), rank = cluster.block_rank();
+  const uint32_t c = blockIdx.x / cs;
+  __shared__ double part[3][kComposeThreads / 32], gather[2][3][kComposeCluster];
+  // remote shared memory may only be written once its block runs (collected before the first sums)
+  if (cs > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+
+  // the thread's vectors are j0, j0 + stride, ... of the channel, B of them in flight; places by walking (row, column) along
+  // (float offsets are below 2^32, check_dims)
+  constexpr int B = HOLD || DIR == 0 ? kComposeHold : kComposeHold / 2;
+  const uint32_t per_row = g.dim0 / VEC, total = per_row * g.N, rs = g.C * g.dim0;
+  const uint32_t stride = cs * blockDim.x, j0 = rank * blockDim.x + threadIdx.x;
+  const uint32_t row0 = j0 / per_row, drow = stride / per_row;
+  const uint32_t col0 = j0 - row0 * per_row, dcol = stride - drow * per_row;
+  const uint32_t off0 = c * g.dim0 + row0 * rs + col0 * VEC;
+  const uint32_t step = drow * rs + dcol * VEC, wrap = rs - per_row * VEC;
+  const uint32_t cnt = j0 < total ? (total - j0 - 1) / stride + 1 : 0;
+  pdl_wait();
+  pdl_trigger();
+
+  Pack<VEC> vx[B], vd[DIR == 1 ? B : 1];
+  // visit(f): f(x, dy, offset) for every vector, B loads in flight; the first visit of a held channel loads it
+  bool loaded = false;
+  auto visit = [&](auto f) {
+    uint32_t off = off0, col = col0;
+    for (uint32_t k = 0; k < cnt; k += B) {
+      uint32_t at[B];
+#pragma unroll
+      for (int u = 0; u < B; ++u) {
+        at[u] = off;
+        if (k + u < cnt && !(HOLD && loaded)) {
+          vx[u] = Pack<VEC>::load(g.x + off);
+          if (DIR == 1) vd[u] = Pack<VEC>::load(g.dy + off);
+        }
+        off += step; col += dcol;
+        if (col >= per_row) { col -= per_row; off += wrap; }
+      }
+#pragma unroll
+      for (int u = 0; u < B; ++u)
+        if (k + u < cnt) f(vx[u], vd[DIR == 1 ? u : 0], at[u], u);
+      if (HOLD) break;
+    }
+    loaded = true;
+  };
+  const float norm = (float)g.dim0 * (float)g.N;
+
+  if constexpr (DIR == 0) {
+    float acc[B] = {};
+    visit([&](const Pack<VEC> &x, const Pack<VEC> &, uint32_t, int u) {
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) acc[u] += x.v[i];
+    });
+    double v[1] = {0.0};
+#pragma unroll
+    for (int u = 0; u < B; ++u) { v[0] += (double)acc[u]; acc[u] = 0.f; }
+    if (cs > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_sums(cluster, v, part, gather[0]);
+    const float m = (float)v[0] / norm;                               // batch_norm.cu:54
+    visit([&](const Pack<VEC> &x, const Pack<VEC> &, uint32_t, int u) {
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) { const float d = x.v[i] - m; acc[u] += d * d; }
+    });
+    v[0] = 0.0;
+#pragma unroll
+    for (int u = 0; u < B; ++u) v[0] += (double)acc[u];
+    cluster_sums(cluster, v, part, gather[1]);
+    const float var = (float)v[0] / norm + g.epsilon;                 // batch_norm.cu:160
+    if (rank == 0 && threadIdx.x == 0) {
+      g.mean[c] = m; g.var[c] = var;
+      if (g.run_mean) { const float o = g.run_mean[c]; g.run_mean[c] = o + g.avg_rate * (m - o); }
+      if (g.run_var) { const float o = g.run_var[c]; g.run_var[c] = o + g.avg_rate * (var - o); }
+    }
+    const float r = rsqrtf(var);                                      // batch_norm.cu:333
+    visit([&](const Pack<VEC> &x, const Pack<VEC> &, uint32_t at, int) {
+      Pack<VEC> o;
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) o.v[i] = (x.v[i] - m) * r;
+      o.put(g.out + at);
+    });
+  } else {
+    const float m = g.mean_in[c], va = g.var_in[c], r = rsqrtf(va);
+    float a1[B] = {}, a2[B] = {}, a3[B] = {};
+    visit([&](const Pack<VEC> &x, const Pack<VEC> &dy, uint32_t, int u) {
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) { const float d = x.v[i] - m; a1[u] = fmaf(dy.v[i], d, a1[u]); a2[u] += dy.v[i]; a3[u] += d; }
+    });
+    double v[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int u = 0; u < B; ++u) { v[0] += (double)a1[u]; v[1] += (double)a2[u]; v[2] += (double)a3[u]; }
+    if (cs > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_sums(cluster, v, part, gather[0]);
+    const float dvar = (float)((double)(-0.5f * r / va) * v[0]);                            // batch_norm.cu:492
+    const float dmean = (float)(-(double)r * v[1]) + (float)((double)(-dvar * 2.0f) * v[2]) / norm;      // :420, :255, :277
+    if (rank == 0 && threadIdx.x == 0) { g.var[c] = dvar; g.mean[c] = dmean; }
+    const float k1 = dvar * 2.0f / norm, k0 = dmean / norm;                                 // :203, :92
+    visit([&](const Pack<VEC> &x, const Pack<VEC> &dy, uint32_t at, int) {
+      Pack<VEC> o;
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) o.v[i] = fmaf(dy.v[i], r, fmaf(x.v[i] - m, k1, k0));
+      o.put(g.out + at);
+    });
+  }
+}
+
+template <int DIR>
+static int launch_compose(const ComposeArgs &g, bool aligned, cudaStream_t stream)
+{
+  const bool vec = g.dim0 % 4 == 0 && aligned;
+  const uint64_t total = (uint64_t)(vec ? g.dim0 / 4 : g.dim0) * g.N;
+  // the smallest cluster that holds the channel; else enough blocks for the device
+  uint32_t cs = 1;
+  while (cs < kComposeCluster && total > (uint64_t)cs * kComposeThreads * kComposeHold) cs *= 2;
+  const bool hold = total <= (uint64_t)cs * kComposeThreads * kComposeHold;
+  const uint64_t each = (total + cs - 1) / cs;
+  const uint32_t threads = each < kComposeThreads ? (uint32_t)(each + 31) / 32 * 32 : kComposeThreads;
+  if ((uint64_t)g.C * cs > 0x7fffffffull) return ANODE_E_DIMS;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(g.C * cs);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cs; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // (as in bn_legacy.cu)
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = 2;
+  auto kernel = vec ? (hold ? bn_compose_kernel<DIR, 4, true> : bn_compose_kernel<DIR, 4, false>)
+                    : (hold ? bn_compose_kernel<DIR, 1, true> : bn_compose_kernel<DIR, 1, false>);
+  if (cudaLaunchKernelEx(&cfg, kernel, g) != cudaSuccess) { (void)cudaGetLastError(); return ANODE_E_LAUNCH; }
+  return ANODE_OK;
+}
+
+}  // namespace anode_b200
+
+using namespace anode_b200;
+
+extern "C" int anode_gpu_batch_normalize_3d1_packed_f32(
+    uint32_t dim0, uint32_t dim1, uint32_t dim2, float epsilon, float avg_rate, const float *x, float *y, float *mean, float *var,
+    float *run_mean, float *run_var, const struct KernelConfig *cfg, struct CUstream_st *stream)
+{
+  (void)cfg;
+  const int rc = check_dims(dim0, dim1, dim2);
+  if (rc) return rc;
+  if (!x || !y || !mean || !var) return ANODE_E_NULL;
+  if (!aligned4(x) || !aligned4(y)) return ANODE_E_ALIGN;
+  const bool aligned = aligned16(x) && aligned16(y);
+  // a fused call without affine step and activation, as far as its kernel needs no scratch
+  FusedArgs a{};
+  a.plan = plan_for(dim0, dim1, dim2, aligned);
+  a.ws_capacity = workspace_part_bytes(dim0, dim1, dim2);
+  a.x = x; a.out = y; a.mean = mean; a.var = var; a.run_mean = run_mean; a.run_var = run_var;
+  a.epsilon = epsilon; a.avg_rate = avg_rate; a.neg_slope = 1.0f;
+  a.mode = MODE_FUSED;
+  a.count_total = (double)dim0 * (double)dim2;
+  const int kind = pick_kernel_kind(a, 0, aligned);
+  if (kind == ANODE_KERNEL_REGISTER && launch_chan(a, 0, aligned, stream) == ANODE_OK) return ANODE_OK;
+  if (kind == ANODE_KERNEL_STREAM && launch_stream(a, 0, stream) == ANODE_OK) return ANODE_OK;
+  ComposeArgs g{};
+  g.dim0 = dim0; g.C = dim1; g.N = dim2; g.epsilon = epsilon; g.avg_rate = avg_rate;
+  g.x = x; g.out = y; g.mean = mean; g.var = var; g.run_mean = run_mean; g.run_var = run_var;
+  return launch_compose<0>(g, aligned, stream);
+}
+
+extern "C" int anode_gpu_batch_normalize_adjoint_3d1_packed_f32(
+    uint32_t dim0, uint32_t dim1, uint32_t dim2, const float *dy, const float *x, const float *mean, const float *var,
+    float *dx, float *dmean, float *dvar, const struct KernelConfig *cfg, struct CUstream_st *stream)
+{
+  (void)cfg;
+  const int rc = check_dims(dim0, dim1, dim2);
+  if (rc) return rc;
+  if (!dy || !x || !mean || !var || !dx || !dmean || !dvar) return ANODE_E_NULL;
+  if (!aligned4(x) || !aligned4(dy) || !aligned4(dx)) return ANODE_E_ALIGN;
+  ComposeArgs g{};
+  g.dim0 = dim0; g.C = dim1; g.N = dim2;
+  g.x = x; g.dy = dy; g.mean_in = mean; g.var_in = var; g.out = dx; g.mean = dmean; g.var = dvar;
+  return launch_compose<1>(g, aligned16(x) && aligned16(dy) && aligned16(dx), stream);
+}

@@ -34,12 +34,13 @@ namespace {
 struct KernelConfig { uint32_t block_sz, max_block_ct; };
 
 // addresses of the C ABI, in the order of kNames
-enum { F_FWD, F_FWD_ACT, F_FWD_ADD, F_BWD, F_BWD_ACT, F_BWD_ADD, F_INFER, F_COUNT };
+enum { F_FWD, F_FWD_ACT, F_FWD_ADD, F_BWD, F_BWD_ACT, F_BWD_ADD, F_INFER, F_NORMALIZE, F_ADJOINT, F_COUNT };
 const char *const kNames[F_COUNT] = {
     "anode_gpu_batch_norm_relu_fused_fwd_3d1_packed_f32", "anode_gpu_batch_norm_act_fused_fwd_3d1_packed_f32",
     "anode_gpu_batch_norm_add_act_fused_fwd_3d1_packed_f32", "anode_gpu_batch_norm_relu_fused_bwd_3d1_packed_f32",
     "anode_gpu_batch_norm_act_fused_bwd_3d1_packed_f32", "anode_gpu_batch_norm_add_act_fused_bwd_3d1_packed_f32",
-    "anode_gpu_batch_norm_act_infer_3d1_packed_f32"};
+    "anode_gpu_batch_norm_act_infer_3d1_packed_f32", "anode_gpu_batch_normalize_3d1_packed_f32",
+    "anode_gpu_batch_normalize_adjoint_3d1_packed_f32"};
 void *g_fn[F_COUNT] = {};
 
 typedef const float *In;
@@ -51,6 +52,8 @@ typedef int (*BwdFn)(uint32_t, uint32_t, uint32_t, int, int, In, In, In, In, In,
 typedef int (*BwdActFn)(uint32_t, uint32_t, uint32_t, float, int, In, In, In, In, In, In, Out, Out, Out, void *, size_t, const KernelConfig *, void *);
 typedef int (*BwdAddFn)(uint32_t, uint32_t, uint32_t, float, int, In, In, In, In, In, In, In, Out, Out, Out, Out, void *, size_t, const KernelConfig *, void *);
 typedef int (*InferFn)(uint32_t, uint32_t, uint32_t, float, In, In, In, In, In, Out, const KernelConfig *, void *);
+typedef int (*NormalizeFn)(uint32_t, uint32_t, uint32_t, float, float, In, Out, Out, Out, Out, Out, const KernelConfig *, void *);
+typedef int (*AdjointFn)(uint32_t, uint32_t, uint32_t, In, In, In, In, Out, Out, Out, const KernelConfig *, void *);
 
 // The interpreter's lock is given back while this lives (exceptions included).
 struct Unlocked {
@@ -254,6 +257,49 @@ PyObject *py_infer(PyObject *, PyObject *const *v, Py_ssize_t n)
   END_GUARDED
 }
 
+// normalize(axes, epsilon, avg_rate, x, y, mean, var, avg_mean, avg_var, stream)
+PyObject *py_normalize(PyObject *, PyObject *const *v, Py_ssize_t n)
+{
+  GUARDED
+  if (!want_args(n, 10)) return nullptr;
+  Args a{v};
+  uint32_t d[3] = {0, 0, 0};
+  a.dims(0, 3, d);
+  const float eps = a.f(1), rate = a.f(2);
+  In x = a.ptr(3, false);
+  Out y = a.ptr(4, false), mean = a.ptr(5, false), var = a.ptr(6, false), rm = a.ptr(7, false), rv = a.ptr(8, false);
+  void *s = a.stream(9);
+  if (!a.ok || !bound(F_NORMALIZE)) return nullptr;
+  int rc;
+  {
+    Unlocked unlocked;
+    rc = ((NormalizeFn)g_fn[F_NORMALIZE])(d[0], d[1], d[2], eps, rate, x, y, mean, var, rm, rv, &kDefaultCfg, s);
+  }
+  return PyLong_FromLong(rc);
+  END_GUARDED
+}
+
+// adjoint(axes, dy, x, mean, var, dx, dmean, dvar, stream)
+PyObject *py_adjoint(PyObject *, PyObject *const *v, Py_ssize_t n)
+{
+  GUARDED
+  if (!want_args(n, 9)) return nullptr;
+  Args a{v};
+  uint32_t d[3] = {0, 0, 0};
+  a.dims(0, 2, d);
+  In dy = a.ptr(1, false), x = a.ptr(2, false), mean = a.ptr(3, false), var = a.ptr(4, false);
+  Out dx = a.ptr(5, false), dmean = a.ptr(6, false), dvar = a.ptr(7, false);
+  void *s = a.stream(8);
+  if (!a.ok || !bound(F_ADJOINT)) return nullptr;
+  int rc;
+  {
+    Unlocked unlocked;
+    rc = ((AdjointFn)g_fn[F_ADJOINT])(d[0], d[1], d[2], dy, x, mean, var, dx, dmean, dvar, &kDefaultCfg, s);
+  }
+  return PyLong_FromLong(rc);
+  END_GUARDED
+}
+
 // The tensors of one of the reference's own entry points: `lo` to `hi` of them, all required (these entry points have no
 // status, and their kernels read and write what they are given).
 struct Pointers {
@@ -374,6 +420,8 @@ PyMethodDef kMethods[] = {
     {"fwd", (PyCFunction)(void *)py_fwd, METH_FASTCALL, nullptr},
     {"bwd", (PyCFunction)(void *)py_bwd, METH_FASTCALL, nullptr},
     {"infer", (PyCFunction)(void *)py_infer, METH_FASTCALL, nullptr},
+    {"normalize", (PyCFunction)(void *)py_normalize, METH_FASTCALL, nullptr},
+    {"adjoint", (PyCFunction)(void *)py_adjoint, METH_FASTCALL, nullptr},
     {"flat", (PyCFunction)(void *)py_flat, METH_FASTCALL, nullptr},
     {"packed", (PyCFunction)(void *)py_packed, METH_FASTCALL, nullptr},
     {"packed_eps", (PyCFunction)(void *)py_packed_eps, METH_FASTCALL, nullptr},

@@ -237,8 +237,12 @@ class FlatJoinOp:
 
 
 # --------------------------------------------------------------------------------------------
-# Front-end compositions (src/ops.rs:983-1056) and their adjoints, kernel by kernel.
+# Front-end compositions (src/ops.rs:983-1056) and their adjoints.  The training forms are one launch each; the others, and
+# arrays without elements or beyond 32-bit indexes, go op by op.
 # --------------------------------------------------------------------------------------------
+
+_FUSED_LIMIT = 1 << 32
+
 
 def batch_normalize_2d(x, axes, online, avg_rate, epsilon, avg_mean=None, avg_var=None, cfg=None, stream=None):
     """`x.batch_normalize_2d(axes, online, avg_rate, epsilon)` of src/ops.rs:999-1014.
@@ -249,12 +253,20 @@ def batch_normalize_2d(x, axes, online, avg_rate, epsilon, avg_mean=None, avg_va
     (`switch(online, avg, batch)`, src/ops.rs:1671-1674).
     """
     c = x.shape[1]
-    mean = torch.zeros(c, device=x.device, dtype=torch.float32)
-    var = torch.zeros(c, device=x.device, dtype=torch.float32)
+    fused = online and 0 < x.numel() < _FUSED_LIMIT
+    new = torch.empty if fused else torch.zeros
+    mean = new(c, device=x.device, dtype=torch.float32)
+    var = new(c, device=x.device, dtype=torch.float32)
     if avg_mean is None:
         avg_mean = torch.zeros_like(mean)
     if avg_var is None:
         avg_var = torch.zeros_like(var)
+    if fused:
+        _hint(cfg)
+        y = torch.empty_like(x)
+        check(native().normalize(axes, epsilon, avg_rate, x, y, mean, var, avg_mean, avg_var, stream),
+              "anode_gpu_batch_normalize_3d1_packed_f32")
+        return y, mean, var, avg_mean, avg_var
     BatchMean2dOp.apply(axes, x, mean, cfg=cfg, stream=stream)
     BatchVariance2dOp.apply(axes, epsilon, x, mean, var, cfg=cfg, stream=stream)
     OnlineAverageOp.apply(avg_rate, mean, avg_mean, cfg=cfg, stream=stream)
@@ -277,8 +289,14 @@ def batch_normalize_adjoint(axes, dy_bn, x, mean, var, cfg=None, stream=None):
     evaluates it: BatchNormalize2dOp.adjoint emits (adj_x, adj_mean, adj_var)
     (src/ops_gpu.rs:4344-4352), BatchVariance2dOp.adjoint (adj_x, adj_mean) (:3997-4003),
     BatchMean2dOp.adjoint adj_x (:3787-3791); the first contribution to a variable is written
-    with Assign and later ones with Accumulate (src/lib.rs:2160-2165).  Seven kernels."""
+    with Assign and later ones with Accumulate (src/lib.rs:2160-2165).  One launch in the place of the seven ops."""
     c = x.shape[1]
+    if 0 < x.numel() < _FUSED_LIMIT:
+        _hint(cfg)
+        dvar, dmean = torch.empty(c, device=x.device, dtype=torch.float32), torch.empty(c, device=x.device, dtype=torch.float32)
+        dx = torch.empty_like(x)
+        check(native().adjoint(axes, dy_bn, x, mean, var, dx, dmean, dvar, stream), "anode_gpu_batch_normalize_adjoint_3d1_packed_f32")
+        return dx, dmean, dvar
     dvar = torch.zeros(c, device=x.device, dtype=torch.float32)
     dmean = torch.zeros(c, device=x.device, dtype=torch.float32)
     dx = torch.empty_like(x)

@@ -294,6 +294,20 @@ int anode_gpu_batch_norm_add_act_fused_bwd_3d1_packed_f32(
     void *workspace, size_t workspace_bytes,
     const struct KernelConfig *cfg, struct CUstream_st *stream);
 
+/* The front end's composition without affine step and activation, and its adjoint, one launch each and without scratch
+ * memory: what src/ops.rs:999-1014 builds of mean, variance, two running averages and normalize (run_mean, run_var may be
+ * NULL), and the seven ops of src/ops_gpu.rs:4344-4352, 3997-4003, 3787-3791 with Assign to dx, dmean and dvar.  As in
+ * those ops mean and var of the adjoint need not be the batch's. */
+int anode_gpu_batch_normalize_3d1_packed_f32(
+    uint32_t dim0, uint32_t dim1, uint32_t dim2, float epsilon, float avg_rate,
+    const float *x, float *y, float *mean, float *var, float *run_mean, float *run_var,
+    const struct KernelConfig *cfg, struct CUstream_st *stream);
+int anode_gpu_batch_normalize_adjoint_3d1_packed_f32(
+    uint32_t dim0, uint32_t dim1, uint32_t dim2,
+    const float *dy, const float *x, const float *mean, const float *var,
+    float *dx, float *dmean, float *dvar,
+    const struct KernelConfig *cfg, struct CUstream_st *stream);
+
 /* Forward pass for callers that have no scratch memory to give.  No counterpart in the
  * reference.  Same arguments and results as anode_gpu_batch_norm_relu_fused_fwd_3d1_packed_f32
  * minus the workspace: anode's op closures pass only dimensions, inputs, pre-made outputs, a

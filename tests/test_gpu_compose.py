@@ -1,0 +1,84 @@
+"""The one-launch composition and its adjoint (csrc/bn_compose.cu) against float64, op by op: channels held in registers by a
+warp, a block and clusters, channels that are not, 16- and 4-byte loads, unaligned tensors, and a mean and variance that are
+not the batch's."""
+import numpy as np
+import pytest
+import torch
+
+from anode_b200 import _lib, ops
+from tests.test_gpu_fused import dev, host
+from tests.util import assert_close, assert_sum_close, make_inputs
+
+SHAPES = [(2, 3, 1, 1), (2, 5, 3, 3), (3, 2, 16, 16), (32, 4, 28, 28), (64, 3, 28, 28), (85, 3, 28, 28), (86, 3, 28, 28),
+          (9, 5, 55, 55), (700, 3, 7, 7), (1, 2, 1, 16384), (1, 2, 1, 16385), (1, 2, 1, 65536), (1, 2, 1, 65540), (4, 3, 128, 200),
+          (2, 2, 5, 6, 7), (600, 40, 2, 2)]
+
+
+def address(name):
+    return getattr(_lib.load(), name)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("offset", [0, 1])
+def test_composition_and_adjoint(shape, offset):
+    d = make_inputs(shape, seed=sum(shape), loc=0.5, scale=2.0, affine=False)
+    c, ax = shape[1], tuple(i for i in range(len(shape)) if i != 1)
+    bs = (1, c) + (1,) * (len(shape) - 2)
+    axes = list(range(len(shape) - 2))
+
+    def place(a):
+        t = torch.empty(a.size + offset, device="cuda")[offset:].view(shape)
+        return t.copy_(torch.from_numpy(a))
+    x64, dy64 = d["x"].astype(np.float64), d["dy"].astype(np.float64)
+    m = x64.size // c
+    tx, tdy = place(d["x"]), place(d["dy"])
+    am, av = dev(d["run_mean"]), dev(d["run_var"])
+    want_mean, want_var = x64.mean(ax), x64.var(ax) + 1e-5
+    for kernel in ("auto", "plain"):           # the fused calls' kernels where they serve, and this file's own
+        ops.set_kernel(kernel)
+        try:
+            am, av = dev(d["run_mean"]), dev(d["run_var"])
+            y, mean, var, am, av = ops.batch_normalize_2d(tx, axes, True, 0.1, 1e-5, am, av)
+        finally:
+            ops.set_kernel("auto")
+        assert_close(host(mean), want_mean, "mean")
+        assert_close(host(var), want_var, "var")
+        assert_close(host(am), 0.1 * want_mean, "running mean")
+        assert_close(host(av), 0.9 + 0.1 * want_var, "running variance")
+        assert_close(host(y), (x64 - want_mean.reshape(bs)) / np.sqrt(want_var).reshape(bs), "y")
+    # the adjoint at a mean and a variance of the caller's
+    rng = np.random.default_rng(3)
+    for mean32, var32 in ((want_mean.astype(np.float32), want_var.astype(np.float32)),
+                          (rng.standard_normal(c).astype(np.float32), (rng.random(c) + 0.5).astype(np.float32))):
+        dx, dmean, dvar = ops.batch_normalize_adjoint(axes, tdy, tx, dev(mean32), dev(var32))
+        e = x64 - mean32.astype(np.float64).reshape(bs)
+        r = 1.0 / np.sqrt(var32.astype(np.float64))
+        wvar = (dy64 * e).sum(ax) * -0.5 * r / var32
+        wmean = -r * dy64.sum(ax) - 2.0 * wvar * e.sum(ax) / m
+        assert_sum_close(host(dvar), wvar, "dvar")
+        assert_sum_close(host(dmean), wmean, "dmean")
+        assert_close(host(dx), dy64 * r.reshape(bs) + (2.0 * wvar / m).reshape(bs) * e + (wmean / m).reshape(bs), "dx")
+
+
+@pytest.mark.gpu
+def test_arrays_without_elements_and_running_statistics_go_op_by_op():
+    x = torch.empty(0, 3, 4, 4, device="cuda")
+    y, mean, var, am, av = ops.batch_normalize_2d(x, [0, 1], True, 0.1, 1e-5)
+    assert y.shape == x.shape and mean.tolist() == var.tolist() == am.tolist() == av.tolist() == [0.0] * 3
+    dx, dmean, dvar = ops.batch_normalize_adjoint([0, 1], x, x, mean, var)
+    assert dx.shape == x.shape and dmean.tolist() == dvar.tolist() == [0.0] * 3
+
+
+def test_refusals():
+    x, v = torch.zeros(2, 3, 4, 4), torch.zeros(3)
+    with pytest.raises(ValueError, match="contiguous float32 CUDA tensor"):
+        ops.batch_normalize_2d(x, [0, 1], True, 0.1, 1e-5)
+    with pytest.raises(ValueError, match="contiguous float32 CUDA tensor"):
+        ops.batch_normalize_adjoint([0, 1], x, x, v, v)
+    with pytest.raises(ValueError, match="axes"):
+        ops.batch_normalize_2d(x, [1, 2], True, 0.1, 1e-5)
+    f, b = address("anode_gpu_batch_normalize_3d1_packed_f32"), address("anode_gpu_batch_normalize_adjoint_3d1_packed_f32")
+    assert f(0, 3, 2, 1e-5, 0.1, *[None] * 8) == -2 and f(65536, 65536, 1, 1e-5, 0.1, *[None] * 8) == -2
+    assert f(4, 3, 2, 1e-5, 0.1, *[None] * 8) == -1 and f(4, 3, 2, 1e-5, 0.1, 2, 16, 16, 16, None, None, None, None) == -6
+    assert b(0, 3, 2, *[None] * 9) == -2 and b(4, 3, 2, *[None] * 9) == -1 and b(4, 3, 2, 2, 16, 16, 16, 16, 16, 16, None, None) == -6
