@@ -5,7 +5,11 @@
 // examples/run_imagenet_mpi.rs:310-417).  For callers on that side of the boundary the cost of a
 // layer is the PCIe transfer, not the kernels, so this entry point overlaps the two directions of
 // the link: channels are independent in batch-norm, so the layer is cut into blocks of channels and
-// block k+1 travels to the device while block k is computed and block k-1 travels back.
+// block k+1 travels to the device while block k is computed and block k-1 travels back.  Within a block
+// the forward kernel needs x only, and y leaves while dy arrives: of the first block only x and of the
+// last only dx travel alone.  [64,64,56,56], four blocks of 12.8 MB a tensor: 2740 us with all copies
+// before and behind both kernels, 2510 so.  More and smaller blocks are slower, their rows being shorter
+// pieces of the host tensor's (8 blocks 2640, 16 blocks 2970).
 //
 // Streams: the kernels run on the caller's stream; host->device and device->host copies run on two
 // streams owned by the library (created on first use, one pair per device), ordered against the
@@ -21,7 +25,8 @@ constexpr int kStageBufs = 3;
 
 struct HostPipe {
   cudaStream_t in = nullptr, out = nullptr;
-  cudaEvent_t start = nullptr, in_done[kStageBufs] = {}, k_done[kStageBufs] = {}, out_done[kStageBufs] = {};
+  cudaEvent_t start = nullptr, x_done[kStageBufs] = {}, in_done[kStageBufs] = {}, f_done[kStageBufs] = {}, k_done[kStageBufs] = {},
+              out_done[kStageBufs] = {};
   bool ok = false;
 };
 
@@ -39,7 +44,9 @@ static HostPipe *host_pipe()
               cudaStreamCreateWithFlags(&p.out, cudaStreamNonBlocking) == cudaSuccess &&
               cudaEventCreateWithFlags(&p.start, cudaEventDisableTiming) == cudaSuccess;
   for (int i = 0; good && i < kStageBufs; ++i)
-    good = cudaEventCreateWithFlags(&p.in_done[i], cudaEventDisableTiming) == cudaSuccess &&
+    good = cudaEventCreateWithFlags(&p.x_done[i], cudaEventDisableTiming) == cudaSuccess &&
+           cudaEventCreateWithFlags(&p.f_done[i], cudaEventDisableTiming) == cudaSuccess &&
+           cudaEventCreateWithFlags(&p.in_done[i], cudaEventDisableTiming) == cudaSuccess &&
            cudaEventCreateWithFlags(&p.k_done[i], cudaEventDisableTiming) == cudaSuccess &&
            cudaEventCreateWithFlags(&p.out_done[i], cudaEventDisableTiming) == cudaSuccess;
   if (!good) { (void)cudaGetLastError(); return nullptr; }
@@ -167,6 +174,9 @@ static int host_step(uint32_t dim0, uint32_t dim1, uint32_t dim2, uint64_t globa
   ANODE_TRY(cudaStreamWaitEvent(P->out, P->start, 0));
 
   const uint32_t nchunks = ceil_div_u32(dim1, L.chunk);
+  // y may take dy's place in host memory: then it leaves only when dy has been read
+  const uint64_t floats = (uint64_t)dim0 * dim1 * dim2;
+  const bool y_over_dy = host_y < host_dy + floats && host_dy < host_y + floats;
   uint32_t prev_cc = 0;
   for (uint32_t k = 0; k < nchunks; ++k) {
     const int b = (int)(k % kStageBufs);
@@ -175,10 +185,11 @@ static int host_step(uint32_t dim0, uint32_t dim1, uint32_t dim2, uint64_t globa
     // host -> device, once the buffer's previous contents have left
     if (k >= (uint32_t)kStageBufs) ANODE_TRY(cudaStreamWaitEvent(P->in, P->out_done[b], 0));
     ANODE_TRY(copy_block(tensor(b, 0), const_cast<float *>(host_x), dim0, dim1, dim2, c0, cc, true, P->in));
+    ANODE_TRY(cudaEventRecord(P->x_done[b], P->in));
     ANODE_TRY(copy_block(dx_, const_cast<float *>(host_dy), dim0, dim1, dim2, c0, cc, true, P->in));
     ANODE_TRY(cudaEventRecord(P->in_done[b], P->in));
-    // both kernels on the caller's stream
-    ANODE_TRY(cudaStreamWaitEvent(stream, P->in_done[b], 0));
+    // both kernels on the caller's stream, device -> host behind each
+    ANODE_TRY(cudaStreamWaitEvent(stream, P->x_done[b], 0));
     if (prev_cc != 0 && cc != prev_cc)   // the last block is tiled differently: start from a clean workspace
       ANODE_TRY(cudaMemsetAsync(ws + 256, 0, L.ws_bytes - 256, stream));
     prev_cc = cc;
@@ -190,6 +201,11 @@ static int host_step(uint32_t dim0, uint32_t dim1, uint32_t dim2, uint64_t globa
     if (rc) return rc;
     rc = comm ? sync_launch(a, 0, true, comm, fused, stream) : launch_best(a, 0, true, stream);
     if (rc) return rc;
+    ANODE_TRY(cudaEventRecord(P->f_done[b], stream));
+    ANODE_TRY(cudaStreamWaitEvent(P->out, P->f_done[b], 0));
+    if (y_over_dy) ANODE_TRY(cudaStreamWaitEvent(P->out, P->in_done[b], 0));
+    ANODE_TRY(copy_block(tensor(b, 2), host_y, dim0, dim1, dim2, c0, cc, false, P->out));
+    ANODE_TRY(cudaStreamWaitEvent(stream, P->in_done[b], 0));
     rc = prepare_bwd(a, dim0, cc, dim2, relu, 0, dx_, tensor(b, 0), mean + c0, var + c0, gamma ? gamma + c0 : nullptr,
                      (gamma && beta) ? beta + c0 : nullptr, dx_, dgamma ? dgamma + c0 : nullptr,
                      dbeta ? dbeta + c0 : nullptr, ws, fused);
@@ -198,9 +214,7 @@ static int host_step(uint32_t dim0, uint32_t dim1, uint32_t dim2, uint64_t globa
     rc = comm ? sync_launch(a, 1, true, comm, fused, stream) : launch_best(a, 1, true, stream);
     if (rc) return rc;
     ANODE_TRY(cudaEventRecord(P->k_done[b], stream));
-    // device -> host
     ANODE_TRY(cudaStreamWaitEvent(P->out, P->k_done[b], 0));
-    ANODE_TRY(copy_block(tensor(b, 2), host_y, dim0, dim1, dim2, c0, cc, false, P->out));
     ANODE_TRY(copy_block(dx_, host_dx, dim0, dim1, dim2, c0, cc, false, P->out));
     ANODE_TRY(cudaEventRecord(P->out_done[b], P->out));
   }

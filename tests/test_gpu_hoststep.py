@@ -80,3 +80,20 @@ def test_host_step_argument_errors():
         layer.step_from_host(good.cuda(), good, good, good)
     with pytest.raises(ValueError):
         layer.step_from_host(good[:, :2], good, good, good)
+
+
+@pytest.mark.parametrize("form", ["y over dy", "dx over x", "both crosswise"])
+def test_outputs_may_take_either_inputs_place(form):
+    """Blocks whose dy is still on its way when y is ready: y must not overtake it where the two share host memory."""
+    from anode_b200 import ops
+    shape = (64, 16, 56, 56)
+    d = make_inputs(shape, seed=41, loc=0.5, scale=2.0)
+    want, _, _ = run_host_step(d, 4)
+    layer = ops.FusedBatchNormRelu(shape[1], epsilon=1e-5, avg_rate=0.1)
+    layer.gamma.copy_(torch.from_numpy(d["gamma"])); layer.beta.copy_(torch.from_numpy(d["beta"]))
+    hx, hdy = pinned(d["x"]), pinned(d["dy"])
+    hy = hdy if form != "dx over x" else torch.empty_like(hx).pin_memory()
+    hdx = hx if form != "y over dy" else torch.empty_like(hx).pin_memory()
+    layer.step_from_host(hx, hdy, hy, hdx, chunk_channels=4)
+    assert layer.host_step_status() == 0
+    assert np.array_equal(hy.numpy(), want["y"]) and np.array_equal(hdx.numpy(), want["dx"])
