@@ -285,6 +285,12 @@ bool chan_applies(const FusedArgs &a, int dir, bool aligned)
 // samples, [15,1516,130] 10.8 and 12.5, clusters of sixteen, [336,212,29] 8.7 and 12.9.  Rows of 1 - 3 floats, which the
 // threads fetch from far apart, on the shared-memory kernel: [1024,512,3] residual backward 25.8 and 18.5, [1540,632,2]
 // backward 24.4 and 18.7, [1457,828,1] residual forward 23.6 and 20.6.
+// Backward passes and the residual epilogue of large layers of medium and long aligned rows go to the tiled kernel although a
+// team holds the channel, unless a channel is but a tile or two there.  Us here and there: backward [8,1024,56,56] 74 and 59,
+// [16,512,56,56] 82 and 59, [35,512,28,28] 42 and 36, but [64,1024,18,18] 69 and 71, [1,2048,100,100] 51 and 54; residual
+// [16,512,56,56] 80 / 109 and 62 / 96, [8,1024,56,56] 68 / 100 and 61 / 98, but [2,512,128,128] 41 / 61 and 44 / 65,
+// [25,1024,28,28] 51 / 76 and 57 / 80.  (Forward passes: [64,512,28,28] 52 and 52, [25,1024,28,28] 36 and 47.)
+constexpr uint64_t kChanTiled = 16u << 20, kChanTiledExtra = 18u << 20, kChanTiledChannel = 24u << 10;
 constexpr uint64_t kChanLarge = 8u << 20, kChanLargeScalar = 3u << 20, kChanLargeExtra = 5u << 20;
 constexpr uint64_t kChanWaves = 1500000, kChanShortest = 1200000;
 constexpr uint32_t kChanFewSamples = 32;
@@ -298,8 +304,11 @@ bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
   const uint64_t channel = (uint64_t)a.plan.dim0 * a.plan.N, elements = channel * a.plan.C;
   const uint32_t most = dir == 0 && !extra ? 32u : 16u;
   if (g.vec == 4) {
+    if (tiled_ok && (dir == 1 || extra) && channel >= kChanTiledChannel && elements >= (extra ? kChanTiledExtra : kChanTiled) &&
+        tiled_takes(a.plan.dim0, elements, dir, extra)) return false;
     if (elements < kChanLarge || channel <= (uint64_t)kChanThreads * kChanCluster * most / 2) return true;
-    return !stream_preferred(a, dir, aligned, tiled_ok) && !(dir == 0 && !extra && tiled_ok);
+    return !stream_preferred(a, dir, aligned, tiled_ok) &&
+           !(tiled_ok && ((dir == 0 && !extra) || tiled_takes(a.plan.dim0, elements, dir, extra)));
   }
   if (elements < kChanLargeScalar) {
     if ((dir == 0 && !extra) || elements < kChanShortest) return true;

@@ -281,6 +281,24 @@ static bool tiled_preferred(const FusedArgs &a, int dir)
   return !(a.res || a.ymask || a.dres) || a.plan.dim0 % 4 == 0 || a.plan.dim0 >= kRaggedMinRowExtra[dir];
 }
 
+// Layers of 16-byte aligned rows from which on the tiled kernel is faster than the streaming kernel: it reads a layer once,
+// the other one twice, but a tile costs it some 2 us whatever its size.  Forward / backward in us, tiled and streaming:
+//   rows of 256   24 M elements 46 / 84 and 49 / 83, 67 M [4096,64,16,16] 107 / 229 and 131 / 228, [512,512,16,16] 105 / 231, 104 / 177
+//   rows of 324   10 M 25 / 36 and 21 / 35, 14 M 31 / 48 and 29 / 50, 24 M 45 / 75 and 56 / 78
+//   rows of 576   10 M 22 / 30 and 18 / 30, 14 M 26 / 38 and 26 / 43, 24 M 40 / 60 and 43 / 73
+//   rows of 784    7 M 19 / 23 and 17 / 24, 10 M 21 / 28 and 22 / 37, 24 M 40 / 56 and 57 / 80
+// residual epilogue
+//   rows of 256   24 M 76 / 106 and 72 / 99;  324  10 M 32 / 46 and 27 / 46, 14 M 42 / 60 and 40 / 65, 24 M 63 / 94 and 76 / 108
+//   rows of 784   10 M 25 / 39 and 29 / 47, 14 M 34 / 53 and 43 / 65
+constexpr uint32_t kTiledRow = 320;
+constexpr uint64_t kTiledFwd = 18u << 20, kTiledBwd = 12u << 20, kTiledFwdExtra = 12u << 20, kTiledBwdExtra = 11u << 20;
+bool tiled_takes(uint32_t dim0, uint64_t elements, int dir, bool extra)
+{
+  if (dim0 % 4 != 0) return false;
+  if (dim0 < kTiledRow) return dir == 0 && !extra && elements >= kTiledFwd + kTiledFwd / 4;
+  return elements >= (dir == 0 ? (extra ? kTiledFwdExtra : kTiledFwd) : extra ? kTiledBwdExtra : kTiledBwd);
+}
+
 typedef void (*RingKernel)(const FusedArgs, const RingGeom);
 
 static RingKernel pick_ring_kernel(const Plan &p, int dir, bool extra, uint32_t &threads)
@@ -797,8 +815,8 @@ extern "C" int anode_gpu_batch_norm_fused_set_kernel(int kernel)
 
 // ---- diagnostics: geometry of the tiled kernel for a shape (no GPU needed) ----------------------
 // out (12 values): applies, rows per tile, floats per row piece, tiles per unit, slots, bytes per slot, dynamic
-// shared memory bytes, KiB between a tile's two visits, the fraction (in 1/1000) of that window loaded with the
-// "keep" priority, blocks, steps between a tile's two visits, tiles
+// shared memory bytes, KiB between a tile's two visits, the fraction (in 1/1000) of such a window that L2 keeps by
+// itself, blocks, steps between a tile's two visits, tiles
 extern "C" int anode_gpu_batch_norm_tiled_geometry(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, uint32_t *out)
 {
   using namespace anode_b200;

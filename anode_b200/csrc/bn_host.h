@@ -44,6 +44,8 @@ int launch_pipeline(FusedArgs &a, int dir, cudaStream_t stream);
 int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned);
 int launch_best(FusedArgs &a, int dir, bool aligned, cudaStream_t stream);
 int kernel_choice();
+// large layers of aligned rows that the tiled kernel serves faster than the streaming kernel
+bool tiled_takes(uint32_t dim0, uint64_t elements, int dir, bool extra);
 // the cluster kernel for short rows (bn_segres.cu)
 bool segres_applies(const FusedArgs &a, int dir, bool aligned);
 uint32_t segres_blocks(const FusedArgs &a, int dir, bool aligned);     // blocks of its launch, 0 where it does not apply

@@ -353,11 +353,8 @@ bool stream_applies(const FusedArgs &a, int dir, bool aligned)
 }
 
 // Where this kernel is taken (after the register-resident kernel): all rows that the tiled kernel does not serve, and of
-// those it does serve (`tiled_ok`) the short ones and the medium ones of channels that are not too large.  Forward /
-// backward in us, here and on the tiled kernel: [4096,64,16,16] 131 / 225 and 168 / 336, [2048,64,20,20] 111 / 192 and
-// 107 / 202, [256,128,24,24] 35 / 55 and 39 / 68, [1024,64,24,24] 78 / 136 and 68 / 128, [128,256,32,32] 60 / 98 and
-// 56 / 101, [256,256,28,28] 97 / 162 and 84 / 158; residual [256,256,28,28] 138 / 221 and 135 / 232, [1024,64,28,28]
-// 162 / 249 and 132 / 218.
+// those it does serve (`tiled_ok`) the short ones and the medium ones of layers and channels that are not too large
+// (tiled_takes; beyond that line by the channel's size, as measured when the tiled kernel read every tile twice).
 constexpr uint32_t kStreamShortRow = 512, kStreamMediumRow = 600, kStreamLongRow = 1024;
 // Layers of few channels leave the device to a few clusters whose threads walk hundreds of samples.  With rows that the
 // tiled kernel serves it is the faster one there, forward / backward, here and there: [7663,4,412] 47 / 119 and 31 / 54,
@@ -375,6 +372,7 @@ bool stream_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
   const uint32_t walk = ceil_div_u32(g.rows, g.groups), blocks = g.units * g.cluster;
   if (tiled_ok && walk >= kStreamLongWalk) return false;
   if (!tiled_ok && extra && dir == 0 && dim0 > 16 && dim0 % 4 != 0 && blocks <= kStreamFewBlocks && walk >= 2 * kStreamLongWalk) return false;
+  if (tiled_ok && tiled_takes(dim0, (uint64_t)dim0 * a.plan.C * a.plan.N, dir, extra)) return false;
   if (!tiled_ok || dim0 <= kStreamShortRow) return true;
   const uint64_t most = (extra ? 1u << 18 : dir == 1 ? 1u << 17 : 1u << 16) * (dim0 <= kStreamMediumRow ? 4ull : 1ull);
   return dim0 <= kStreamLongRow && (uint64_t)dim0 * a.plan.N <= most;

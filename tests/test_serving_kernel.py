@@ -160,3 +160,18 @@ def test_ragged_tiles_hold_equally_many_rows():
             if out[0] and out[2] >= d0:
                 tiles = -(-n // out[1])
                 assert out[3] == tiles and n - (tiles - 1) * out[1] > out[1] - tiles, (d0, c, n, list(out))
+
+
+@pytest.mark.parametrize("shape,one,residual", [
+    # medium rows: the tiled kernel takes the large layers, backward passes and the residual epilogue earlier
+    ((256, 256, 20, 20), ("tiled", "tiled"), ("tiled", "tiled")), ((128, 512, 28, 28), ("tiled", "tiled"), ("tiled", "tiled")),
+    ((256, 256, 24, 24), ("tiled", "tiled"), ("tiled", "tiled")),
+    ((140, 128, 28, 28), ("tiled", "tiled"), ("tiled", "tiled")), ((100, 300, 24, 24), ("register", "tiled"), ("tiled", "tiled")),
+    # not the ordinary layers, nor rows of less than 320 floats beyond the forward pass
+    ((279, 32, 28, 28), ("tiled", "tiled"), ("stream", "stream")), ((4096, 64, 16, 16), ("tiled", "stream"), ("stream", "stream")),
+    ((549, 32, 16, 16), ("stream", "stream"), ("stream", "stream")),
+    # channels that a team holds: backward passes and the residual epilogue, where a channel is more than a tile or two
+    ((16, 512, 56, 56), ("register", "tiled"), ("tiled", "tiled")), ((1, 2048, 100, 100), ("register", "register"), ("register", "register")),
+    ((25, 1024, 28, 28), ("register", "register"), ("register", "register"))])
+def test_routes_between_the_streaming_the_register_resident_and_the_tiled_kernel(shape, one, residual):
+    assert routes(shape) == one + residual
