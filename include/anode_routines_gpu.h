@@ -180,7 +180,7 @@ void anode_gpu_positive_clip_flat_map_bwd_f32(
 #define ANODE_ST_ABORTED      4u  /* some block saw the bits above and skipped work */
 
 /* Kernels behind the fused calls.  ANODE_KERNEL_AUTO (the default) picks by shape:
- *   TILED     persistent kernel streaming tiles through a shared-memory ring, re-reading them from L2
+ *   TILED     persistent kernel streaming tiles through a shared-memory ring and keeping them in tensor memory or L2
  *             (long 16-byte aligned rows);
  *   CLUSTER   thread-block clusters keeping a unit's slice in shared memory (short rows, small channels);
  *   RESIDENT  slices resident in shared memory, all global traffic by bulk copies; takes the residual

@@ -53,8 +53,8 @@ int anode_gpu_batch_norm_stream_geometry(uint32_t dim0, uint32_t dim1, uint32_t 
 
 /* Geometry of the tiled kernel (bn_ring.cuh) for direction `dir` of a fused call on 16-byte aligned tensors.
  * out (12 values): applies, rows per tile, floats per row piece, tiles per unit, slots, bytes per slot, dynamic
- * shared memory bytes, KiB between a tile's two visits (what L2 has to hold), the fraction (in 1/1000) of
- * that window loaded with the "keep" priority, thread blocks, steps between a tile's two visits, tiles. */
+ * shared memory bytes of the layout (the one-launch forms take the SM's whole), KiB between a tile's two visits, the
+ * fraction (in 1/1000) of such a window that L2 would keep by itself (anode_gpu_batch_norm_tiled_keep: what tensor memory takes off it), thread blocks, steps between a tile's two visits, tiles. */
 int anode_gpu_batch_norm_tiled_geometry(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, uint32_t *out);
 
 /* Which of a block's tiles stay in tensor memory between their two visits (tiled kernel, one launch per direction).
