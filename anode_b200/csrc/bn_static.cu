@@ -61,6 +61,9 @@ static void static_need(const FusedArgs &a, bool aligned, uint64_t &need, uint64
       break;
     default:                          // tiled and slice-resident kernels: their share of a workspace part
       need = dim0 % 4 == 0 ? workspace_static_bytes(dim0, C, N) : ring_ws_bytes(a, 0, aligned);
+      // (large layers of medium rows, which the streaming kernel could serve with less: the forward plan's own need, or some of
+      // them would be refused)
+      if (dim0 % 4 == 0 && stream_applies(a, 0, aligned) && pick_kernel_kind(a, 0, aligned) == ANODE_KERNEL_TILED) need = ring_ws_bytes(a, 0, aligned);
       clear = control_region_bytes(dim0, C, N, aligned);
       break;
   }
