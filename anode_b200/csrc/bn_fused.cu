@@ -851,6 +851,9 @@ extern "C" int anode_gpu_batch_norm_tiled_keep(uint32_t dim0, uint32_t dim1, uin
   return ANODE_OK;
 }
 
+// ---- diagnostics: the tiled kernel's test for the inner vectors of a ragged row piece (no GPU needed) ----
+extern "C" int anode_gpu_batch_norm_ragged_whole(int first, uint32_t len) { return anode_b200::ragged_whole(first, len) ? 1 : 0; }
+
 // ---- diagnostics: the tile plan, for tests of the index arithmetic (no GPU needed) ----------
 extern "C" int anode_gpu_batch_norm_fused_plan(uint32_t dim0, uint32_t dim1, uint32_t dim2, int aligned,
                                                uint32_t resident_blocks, uint32_t tile_floats,

@@ -385,7 +385,7 @@ __device__ __forceinline__ void visit_reduce(const FusedArgs &a, const RingGeom 
       auto take = [&](const Quad &v, bool live) {
         const int i0 = live ? w.first() : len;
         Quad e{add2(v.a, nK), add2(v.b, nK)};
-        if ((uint32_t)i0 <= (uint32_t)(len - 4)) {
+        if (ragged_whole(i0, d.z)) {
           n += 4;
         } else {      // foreign floats at a row's ends count nothing
           const float4 t = floats(e);
@@ -451,7 +451,7 @@ __device__ __forceinline__ void visit_reduce(const FusedArgs &a, const RingGeom 
         if constexpr (EXTRA) { if (dres && live) stg_quad(dres + w.at, z); }
       } else {
         const int i0 = live ? w.first() : len;
-        if ((uint32_t)i0 <= (uint32_t)(len - 4)) {
+        if (ragged_whole(i0, d.z)) {
           if constexpr (EXTRA) { if (dres) stg_quad(dres + w.vector(), z); }
         } else {      // (foreign floats may be anything, an infinity or a NaN too)
           const float4 t = floats(z), u = floats(e);
@@ -528,7 +528,7 @@ __device__ __forceinline__ void visit_apply(const FusedArgs &a, const RingGeom &
     }
     float *p = a.out + (RAGGED ? w.vector() : w.at);
     const int i0 = RAGGED ? w.first() : 0;
-    if (!RAGGED || (uint32_t)i0 <= (uint32_t)(len - 4)) {
+    if (!RAGGED || ragged_whole(i0, d.z)) {
       if (acc) { const Quad old = ldg_quad(p); o.a = add2(old.a, o.a); o.b = add2(old.b, o.b); }
       stg_stream(p, o);
       if constexpr (EXTRA && DIR == 1) { if (dres) stg_stream(dres + (p - a.out), z); }

@@ -64,6 +64,10 @@ int anode_gpu_batch_norm_tiled_geometry(uint32_t dim0, uint32_t dim1, uint32_t d
 int anode_gpu_batch_norm_tiled_keep(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual,
                                     uint32_t tile, uint32_t warp, uint32_t *out);
 
+/* Whether the tiled kernel takes the 16-byte vector that begins with float number `first` (below 0: before it) of a ragged
+ * row piece of `len` floats for one that lies wholly within the piece (1 or 0). */
+int anode_gpu_batch_norm_ragged_whole(int first, uint32_t len);
+
 /* Plan of the slice-resident kernel for `planes` tensors per shared-memory slot.  out (16 values): applies,
  * rows per piece, parts per row, floats per part, pieces per channel, blocks per team, teams, grid, pieces
  * per block and channel, slot bytes, slots, resident-ring slots, streaming-ring slots, resident pieces per
