@@ -1031,7 +1031,8 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
         }
       } else {
         // from the boundary below each row's start to the one above its end, but never past the tensor's own end:
-        // the last floats of a tensor whose size is no multiple of four are stored by three lanes instead
+        // the last floats of a tensor whose size is no multiple of four are stored by three lanes instead (they may
+        // belong to two pieces of the last row: the last one may hold a single float)
         const uint32_t per_row = ragged_pitch(len), total = rs * P.N, whole = total & ~3u;
         auto span = [&](uint32_t r, uint32_t &start) {      // bytes of row r, and the float it is fetched from
           const uint32_t first = base + r * rs;
@@ -1042,7 +1043,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
         for (uint32_t r = lane; r < rows; r += 32) { uint32_t start; bytes += span(r, start); }
         bytes = __reduce_add_sync(0xffffffffu, bytes) * planes;
         const uint32_t last = base + (rows - 1) * rs, tail = total & 3u;
-        if (tail && last + len == total && lane < tail) {
+        if (last + len > whole && lane < tail) {
           const uint32_t src = whole + lane;
           float *dst = xs + 4 * per_row * (rows - 1) + (src - (last & ~3u));
           if (p0) *dst = __ldcg(a.x + src);
