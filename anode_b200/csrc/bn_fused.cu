@@ -219,6 +219,12 @@ constexpr uint32_t kRingLargeSlotsBwd = 3, kRingLargeFloatsBwd = 9408;
 #ifndef ANODE_RING_FLOATS_FWD_EXTRA
 #define ANODE_RING_FLOATS_FWD_EXTRA 9408
 #endif
+// (Forward, small layers: where the planner halves that for want of tiles and ends below what it makes of this.  Residual
+// forward pass with the one and with the other, us: [149,5,2888] 19.9 and 15.3, [94,7,1197] 16.6 and 14.6, [113,15,1364]
+// 16.0 and 14.7.)
+#ifndef ANODE_RING_FLOATS_FWD_EXTRA_SMALL
+#define ANODE_RING_FLOATS_FWD_EXTRA_SMALL 6656
+#endif
 #ifndef ANODE_RING_SLOTS_BWD_EXTRA
 #define ANODE_RING_SLOTS_BWD_EXTRA 3
 #endif
@@ -228,16 +234,21 @@ constexpr uint32_t kRingLargeSlotsBwd = 3, kRingLargeFloatsBwd = 9408;
 static bool make_ring_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, Plan &p, RingGeom &g)
 {
   const Tunables &t = tunables();
-  if (extra)
-    return dir == 0 ? ring_plan_with(dim0, C, N, dir, true, ANODE_RING_SLOTS_FWD_EXTRA, ANODE_RING_FLOATS_FWD_EXTRA, p, g)
-                    : ring_plan_with(dim0, C, N, dir, true, ANODE_RING_SLOTS_BWD_EXTRA, ANODE_RING_FLOATS_BWD_EXTRA, p, g);
+  auto tile = [](const Plan &q) { return (uint64_t)q.rows_per_tile * q.piece_len; };
+  if (extra) {
+    if (dir == 1) return ring_plan_with(dim0, C, N, dir, true, ANODE_RING_SLOTS_BWD_EXTRA, ANODE_RING_FLOATS_BWD_EXTRA, p, g);
+    const bool ok = ring_plan_with(dim0, C, N, dir, true, ANODE_RING_SLOTS_FWD_EXTRA, ANODE_RING_FLOATS_FWD_EXTRA, p, g);
+    Plan ps; RingGeom gs;
+    if (ring_plan_with(dim0, C, N, dir, true, ANODE_RING_SLOTS_FWD_EXTRA, ANODE_RING_FLOATS_FWD_EXTRA_SMALL, ps, gs) &&
+        (!ok || tile(ps) > tile(p))) { p = ps; g = gs; return true; }
+    return ok;
+  }
   if (!ring_plan_with(dim0, C, N, dir, false, dir == 0 ? t.ring_slots : t.ring_slots_bwd,
                       dir == 0 ? t.ring_floats_fwd : t.ring_floats_bwd, p, g)) return false;
   if (dir == 1) {
     Plan pl; RingGeom gl;
     if (ring_plan_with(dim0, C, N, dir, false, kRingLargeSlotsBwd, kRingLargeFloatsBwd, pl, gl) && gl.slots == kRingLargeSlotsBwd &&
-        (uint64_t)pl.rows_per_tile * pl.piece_len > (uint64_t)p.rows_per_tile * p.piece_len &&
-        ring_window_bytes(pl, dir) <= kRingLargeWindowMax) {
+        tile(pl) > tile(p) && ring_window_bytes(pl, dir) <= kRingLargeWindowMax) {
       p = pl; g = gl;
     }
   }

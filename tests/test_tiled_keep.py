@@ -50,3 +50,11 @@ def test_places_of_kept_tiles(shape, direction, residual):
                     assert b <= c or d <= a, (t, u)
     # evenly spread: as many of any period's tiles as there are places
     assert sum(r is not None for r in ranges[:look + 1]) == first["slots"]
+
+
+def test_small_layers_have_no_smaller_tiles_for_a_larger_slot():
+    """Forward pass of the residual epilogue: where the planner halves the tiles for want of enough of them, what it makes of the
+    larger slots may be less than what it makes of smaller ones."""
+    for shape, vectors in (((2888, 5, 149), 1444), ((2886, 5, 149), 1446), ((1197, 7, 94), 600), ((1364, 15, 113), 1364),
+                           ((3136, 256, 256), 2352), ((3025, 95, 64), 2271)):
+        assert keep(shape, 0, 1, 0, 0)["vecs"] == vectors, shape
