@@ -126,9 +126,20 @@ static uint32_t ring_tile_vecs(const Plan &p) { return p.rows_per_tile * ring_pi
 // consumer warps of direction `dir` (the two instantiations of bn_ring.cuh)
 static uint32_t ring_warps(int dir) { return dir == 0 ? 8u : 16u; }
 
+// Forward pass of the residual epilogue on ragged rows from this length on: no tile stays in tensor memory.  The two forms of
+// a ragged visit are long, and consumers that run one of them alone are faster than tensor memory makes them; on shorter rows
+// the producer's copies, one per row and tensor, bound the kernel, and a kept tile needs one less.  Us with tensor memory, and
+// without either: 40 M elements of 131 channels, rows of 301 119 and 144, 451 107 and 116, 601 103 and 103, 713 104 and 99,
+// 1201 109 and 99; [34,123,6374] 96 and 70, [50,119,12674] 268 and 202, [200,100,5041] 357 and 273 (where every second visit
+// was one from L2, in an older form of both: 76, 238, 279).
+constexpr uint32_t kRaggedKeepMost = 640;
+static bool ring_keeps(const Plan &p, int dir, bool extra) { return !(dir == 0 && extra && p.dim0 % 4 != 0 && p.dim0 >= kRaggedKeepMost); }
+
 // Fused mode: the tiles that stay in tensor memory.
-static void ring_keep(const Plan &p, int dir, RingGeom &g)
+static void ring_keep(const Plan &p, int dir, bool extra, RingGeom &g)
 {
+  g.keep_slots = 0; g.keep_period = 1;
+  if (!ring_keeps(p, dir, extra)) return;
   plan_keep(g, ring_tile_vecs(p), dir == 1 ? 2u : 1u, ring_warps(dir), p.lookahead_steps);
 }
 
@@ -317,6 +328,7 @@ static RingKernel pick_ring_kernel(const Plan &p, int dir, bool extra, uint32_t 
   const bool ragged = p.dim0 % 4 != 0;
   threads = dir == 0 ? ring8::kRingThreads : ring16::kRingThreads;
   if (dir == 0) {
+    if (extra && !ring_keeps(p, dir, extra)) return ring8::bn_ring_kernel<0, true, true, false>;
     if (extra) return ragged ? ring8::bn_ring_kernel<0, true, true> : ring8::bn_ring_kernel<0, true, false>;
     return ragged ? ring8::bn_ring_kernel<0, false, true> : ring8::bn_ring_kernel<0, false, false>;
   }
@@ -328,15 +340,16 @@ int launch_ring(FusedArgs &a, const RingGeom &g_in, int dir, cudaStream_t stream
 {
   RingGeom g = g_in;
   uint32_t threads = 0;
-  RingKernel k = pick_ring_kernel(a.plan, dir, a.res || a.ymask || a.dres, threads);
+  const bool extra = a.res || a.ymask || a.dres;
+  RingKernel k = pick_ring_kernel(a.plan, dir, extra, threads);
   // the reduce visits may store dres before the apply visits read x only where it is not x itself
   a.dres_early = a.dres && a.dres != a.x ? 1u : 0u;
   static std::mutex mu;
   static std::map<std::pair<const void *, uint32_t>, int> occ;     // (kernel, smem) -> blocks per SM
   int per_sm = 0;
-  // Blocks that use tensor memory take the SM's whole shared memory: a block of another kernel beside them could hold columns
-  // they need, or wait for theirs, and blocks that wait for one another across SMs must not also wait for columns.
-  const uint32_t smem = a.mode == MODE_FUSED ? kRingSmemBudget : g.smem_bytes;
+  // Blocks of kernels that use tensor memory take the SM's whole shared memory: a block of another kernel beside them could
+  // hold columns they need, or wait for theirs, and blocks that wait for one another across SMs must not also wait for columns.
+  const uint32_t smem = a.mode == MODE_FUSED && ring_keeps(a.plan, dir, extra) ? kRingSmemBudget : g.smem_bytes;
   {
     std::lock_guard<std::mutex> lock(mu);
     const auto key = std::make_pair((const void *)k, smem);
@@ -362,7 +375,7 @@ int launch_ring(FusedArgs &a, const RingGeom &g_in, int dir, cudaStream_t stream
   plan_walk(g, a.plan, ring_pitch(a.plan), ring_warps(dir) * 32);
   g.copies = ceil_div_u32(16 * ring_pitch(a.plan), kRingCopyBytes);
   g.keep_slots = 0; g.keep_period = 1;
-  if (a.mode == MODE_FUSED) ring_keep(a.plan, dir, g);
+  if (a.mode == MODE_FUSED) ring_keep(a.plan, dir, extra, g);
   // A window larger than what L2 keeps would cycle through it whole (config 3, backward: 67 MB); marking only
   // the part that fits lets that part stay (backward 4.42 -> 4.27 ms).  Smaller windows keep everything.
   uint64_t window = ring_window_bytes(a.plan, dir) * (g.keep_period - g.keep_slots) / g.keep_period;
@@ -854,7 +867,7 @@ extern "C" int anode_gpu_batch_norm_tiled_keep(uint32_t dim0, uint32_t dim1, uin
   Plan p; RingGeom g;
   for (int i = 0; i < 10; ++i) out[i] = 0;
   if (!ring_plan_for(dim0, dim1, dim2, true, dir, residual != 0, p, g)) return ANODE_OK;
-  ring_keep(p, dir, g);
+  ring_keep(p, dir, residual != 0, g);
   const Keep k = keep_at(g, tile);
   out[0] = g.keep_slots; out[1] = k.kept ? 1u : 0u; out[2] = k.slot;
   keep_place(g, k.slot, warp, ring_warps(dir), out[3], out[4]);

@@ -884,8 +884,9 @@ __device__ __forceinline__ bool pull_merge_unit(const FusedArgs &a, RingCtl *ctl
 // ======================================================================================
 // Whole-row tiles only (one channel per unit): short-row shapes are served by the cluster kernel
 // (bn_segres.cu) and the plain kernel.
-// EXTRA: residual epilogue; RAGGED: rows that are not a multiple of four floats.
-template <int DIR, bool EXTRA, bool RAGGED>
+// EXTRA: residual epilogue; RAGGED: rows that are not a multiple of four floats; TMEM: some tiles may stay in tensor memory
+// (ring_keeps).
+template <int DIR, bool EXTRA, bool RAGGED, bool TMEM = true>
 __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArgs a, const RingGeom g)
 {
   extern __shared__ __align__(128) unsigned char sm[];
@@ -905,9 +906,9 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (g.keep_slots && warp == 0) { __syncwarp(); tmem_alloc(&ctl->tmem); tmem_fence_before(); }
+  if (TMEM && g.keep_slots && warp == 0) { __syncwarp(); tmem_alloc(&ctl->tmem); tmem_fence_before(); }
   __syncthreads();
-  if (g.keep_slots) tmem_fence_after();
+  if (TMEM && g.keep_slots) tmem_fence_after();
 
   Sched sc; sc.init(a);
 
@@ -924,7 +925,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
         if (!ok) break;                                 // warps are independent: no barrier to honour
         const uint4 d = *reinterpret_cast<const uint4 *>(slot_side<DIR, EXTRA>(sm, g, slot));
         float4 *res = res_box(sm, g, qres);
-        if (d.x >> 16) visit_reduce<DIR, EXTRA, RAGGED, true>(a, g, sm, ctl, d, slot, res);
+        if (TMEM && d.x >> 16) visit_reduce<DIR, EXTRA, RAGGED, true>(a, g, sm, ctl, d, slot, res);
         else visit_reduce<DIR, EXTRA, RAGGED, false>(a, g, sm, ctl, d, slot, res);
         if (lane == 0) mbar_arrive(&ctl->res_full[qres]);
         if (++qres == kResQ) { qres = 0; rpar ^= 1u; }
@@ -933,12 +934,12 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
         if (!warp_wait(&ctl->coef_full[qcoef], cpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
         const float4 *coef = coef_box(sm, g, qcoef);
         const uint4 d = *reinterpret_cast<const uint4 *>(coef + 2);
-        const bool kept = (d.x >> 16) != 0;
+        const bool kept = TMEM && (d.x >> 16) != 0;
         if (!kept || kSlotAlways<DIR, EXTRA>) {
           if (++slot == g.slots) { slot = 0; par ^= 1u; }
           if (!warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS)) break;
         }
-        if (kept) visit_apply<DIR, EXTRA, RAGGED, true>(a, g, sm, ctl, d, slot, coef, qcoef);
+        if (TMEM && kept) visit_apply<DIR, EXTRA, RAGGED, true>(a, g, sm, ctl, d, slot, coef, qcoef);
         else visit_apply<DIR, EXTRA, RAGGED, false>(a, g, sm, ctl, d, slot, coef, qcoef);
         if (++qcoef == kCoefQ) { qcoef = 0; cpar ^= 1u; }
       }
@@ -1181,12 +1182,12 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
   }
 
   // ---- leave: the last block out lowers the ready flags so that the workspace is clean again
-  if (g.keep_slots) {
+  if (TMEM && g.keep_slots) {
     if (warp < kCWarps) { __syncwarp(); tmem_wait_st(); }
     tmem_fence_before();
   }
   __syncthreads();
-  if (g.keep_slots && warp == 0) { tmem_fence_after(); tmem_free(ctl->tmem); }
+  if (TMEM && g.keep_slots && warp == 0) { tmem_fence_after(); tmem_free(ctl->tmem); }
   if (ctl->abort) {
     if (tid == 0) atomicOr(status, ANODE_ST_ABORTED);
     return;

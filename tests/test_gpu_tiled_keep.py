@@ -33,3 +33,17 @@ def test_some_tiles_stay_and_some_do_not(shape, residual):
                 assert np.array_equal(again[k], got[k]), (shape, k)
     finally:
         ops.set_kernel("auto")
+
+
+@pytest.mark.parametrize("row", [639, 640, 641, 1283])
+def test_residual_rows_on_both_sides_of_the_line_below_which_tiles_stay(row):
+    from anode_b200 import ops
+    shape = (120, 9, 1, row)
+    d = make_inputs(shape, seed=row, loc=0.5, scale=2.0)
+    res = np.random.default_rng(5).standard_normal(shape).astype(np.float32)
+    ops.set_kernel("tiled")
+    try:
+        assert bool(keep((row, 9, 120), 0, 1, 0, 0)["slots"]) == (row <= 640)
+        check_layer_own_mask(d, run_add_act(ops, d, res, 0.1), "%r " % (shape,), residual=res, slope=0.1)
+    finally:
+        ops.set_kernel("auto")

@@ -58,3 +58,10 @@ def test_small_layers_have_no_smaller_tiles_for_a_larger_slot():
     for shape, vectors in (((2888, 5, 149), 1444), ((2886, 5, 149), 1446), ((1197, 7, 94), 600), ((1364, 15, 113), 1364),
                            ((3136, 256, 256), 2352), ((3025, 95, 64), 2271)):
         assert keep(shape, 0, 1, 0, 0)["vecs"] == vectors, shape
+
+
+def test_long_ragged_rows_of_the_residual_forward_pass_keep_no_tiles():
+    for d0, forward in ((637, True), (639, True), (640, True), (641, False), (643, False), (6374, False), (6376, True)):
+        shape = (d0, 20, 300)
+        assert [bool(keep(shape, d, 1, 0, 0)["slots"]) for d in (0, 1)] == [forward, True], d0
+        assert all(keep(shape, d, 0, 0, 0)["slots"] for d in (0, 1)), d0
