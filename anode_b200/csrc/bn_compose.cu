@@ -1,5 +1,6 @@
 // The front end's own composition (src/ops.rs:999-1014: mean, variance, two running averages, normalize) and its adjoint
-// (the seven ops that src/ops_gpu.rs:4344-4352, 3997-4003 and 3787-3791 emit), one launch each, without scratch memory.
+// (the seven ops that src/ops_gpu.rs:4344-4352, 3997-4003 and 3787-3791 emit), one launch each, without scratch memory
+// (large layers of few channels: the normalization is a launch of its own, normalized_apart).
 //
 // A thread-block cluster of up to eight blocks owns a channel and visits it two or three times, the sums of a visit going
 // through distributed shared memory before the next one begins:
@@ -27,7 +28,7 @@ struct ComposeArgs {
   uint32_t dim0, C, N;
   float epsilon, avg_rate;
   const float *x, *dy, *mean_in, *var_in;
-  float *out, *mean, *var, *run_mean, *run_var;      // adjoint: dx, dmean, dvar
+  float *out, *mean, *var, *run_mean, *run_var;      // adjoint: dx, dmean, dvar; forward: no out, no third visit
 };
 
 // Sums of K values over the threads of the cluster, in a fixed order, to every thread.
@@ -132,6 +133,7 @@ __global__ void __launch_bounds__(kComposeThreads, 2) bn_compose_kernel(const Co
       if (g.run_mean) { const float o = g.run_mean[c]; g.run_mean[c] = o + g.avg_rate * (m - o); }
       if (g.run_var) { const float o = g.run_var[c]; g.run_var[c] = o + g.avg_rate * (var - o); }
     }
+    if (!g.out) return;
     const float r = rsqrtf(var);                                      // batch_norm.cu:333
     visit([&](const Pack<VEC> &x, const Pack<VEC> &, uint32_t at, int) {
       Pack<VEC> o;
@@ -162,6 +164,19 @@ __global__ void __launch_bounds__(kComposeThreads, 2) bn_compose_kernel(const Co
       o.put(g.out + at);
     });
   }
+}
+
+// Forward passes over aligned rows whose few clusters leave SMs idle: the normalization goes over the whole device in a launch
+// of its own, where the clusters of eight have a block for every SM at most and a channel is large.  Us in one launch, in two,
+// and op by op:
+//   1 channel   3 M 59, 33, 46, 25 M 702, 440, 492      3   3 M 23, 18, 27, 10 M 78, 50, 66, 50 M 544, 390, 423
+//   8 channels  10 M 29, 29, 43, 25 M 121, 101, 116     16  25 M 83, 77, 88, 50 M 160, 148, 161
+// but 12 channels 10 M 23.4, 24.5, 37, and of 36 200 M 630, 650, 598.  (Rows that threads load float by float gain little by
+// it: 8 channels, 10 M 56, 67, 136.)
+constexpr uint64_t kApartChannel = 1u << 20;
+static bool normalized_apart(uint32_t dim0, uint32_t C, uint32_t N, bool aligned)
+{
+  return dim0 % 4 == 0 && aligned && (uint64_t)dim0 * N >= kApartChannel && (uint64_t)C * kComposeCluster <= sm_count();
 }
 
 template <int DIR>
@@ -200,7 +215,6 @@ extern "C" int anode_gpu_batch_normalize_3d1_packed_f32(
     uint32_t dim0, uint32_t dim1, uint32_t dim2, float epsilon, float avg_rate, const float *x, float *y, float *mean, float *var,
     float *run_mean, float *run_var, const struct KernelConfig *cfg, struct CUstream_st *stream)
 {
-  (void)cfg;
   const int rc = check_dims(dim0, dim1, dim2);
   if (rc) return rc;
   if (!x || !y || !mean || !var) return ANODE_E_NULL;
@@ -220,7 +234,13 @@ extern "C" int anode_gpu_batch_normalize_3d1_packed_f32(
   ComposeArgs g{};
   g.dim0 = dim0; g.C = dim1; g.N = dim2; g.epsilon = epsilon; g.avg_rate = avg_rate;
   g.x = x; g.out = y; g.mean = mean; g.var = var; g.run_mean = run_mean; g.run_var = run_var;
-  return launch_compose<0>(g, aligned, stream);
+  if (!normalized_apart(dim0, dim1, dim2, aligned)) return launch_compose<0>(g, aligned, stream);
+  g.out = nullptr;
+  const int stats = launch_compose<0>(g, aligned, stream);
+  if (stats) return stats;
+  anode_gpu_batch_norm_3d1_packed_f32(dim0, dim1, dim2, x, mean, var, y, cfg, stream);
+  if (cudaGetLastError() != cudaSuccess) return ANODE_E_LAUNCH;
+  return ANODE_OK;
 }
 
 extern "C" int anode_gpu_batch_normalize_adjoint_3d1_packed_f32(

@@ -294,8 +294,9 @@ int anode_gpu_batch_norm_add_act_fused_bwd_3d1_packed_f32(
     void *workspace, size_t workspace_bytes,
     const struct KernelConfig *cfg, struct CUstream_st *stream);
 
-/* The front end's composition without affine step and activation, and its adjoint, one launch each and without scratch
- * memory: what src/ops.rs:999-1014 builds of mean, variance, two running averages and normalize (run_mean, run_var may be
+/* The front end's composition without affine step and activation, and its adjoint, one launch each (two for large
+ * layers of few channels, whose normalization goes over the whole device) and without scratch memory: what
+ * src/ops.rs:999-1014 builds of mean, variance, two running averages and normalize (run_mean, run_var may be
  * NULL), and the seven ops of src/ops_gpu.rs:4344-4352, 3997-4003, 3787-3791 with Assign to dx, dmean and dvar.  As in
  * those ops mean and var of the adjoint need not be the batch's. */
 int anode_gpu_batch_normalize_3d1_packed_f32(

@@ -82,3 +82,34 @@ def test_refusals():
     assert f(0, 3, 2, 1e-5, 0.1, *[None] * 8) == -2 and f(65536, 65536, 1, 1e-5, 0.1, *[None] * 8) == -2
     assert f(4, 3, 2, 1e-5, 0.1, *[None] * 8) == -1 and f(4, 3, 2, 1e-5, 0.1, 2, 16, 16, 16, None, None, None, None) == -6
     assert b(0, 3, 2, *[None] * 9) == -2 and b(4, 3, 2, *[None] * 9) == -1 and b(4, 3, 2, 2, 16, 16, 16, 16, 16, 16, None, None) == -6
+
+
+def compare_with_float64(shape, seed=0):
+    """Composition and adjoint of a large layer, reference computed on the device."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    x = torch.randn(shape, device="cuda", generator=g).mul_(2.0).add_(0.5)
+    dy = torch.randn(shape, device="cuda", generator=g)
+    c, ax = shape[1], (0, 2, 3)
+    am, av = torch.zeros(c, device="cuda"), torch.ones(c, device="cuda")
+    y, mean, var, am, av = ops.batch_normalize_2d(x, [0, 1], True, 0.1, 1e-5, am, av)
+    x64, bs, m = x.double(), (1, c, 1, 1), x.numel() // c
+    wm, wv = x64.mean(ax), x64.var(ax, unbiased=False) + 1e-5
+    for name, got, want in (("mean", mean, wm), ("var", var, wv), ("running mean", am, 0.1 * wm), ("running variance", av, 0.9 + 0.1 * wv),
+                            ("y", y, (x64 - wm.view(bs)) / wv.sqrt().view(bs))):
+        assert bool(((got.double() - want).abs() <= 1e-5 + 1e-4 * want.abs()).all()), (shape, name)
+    dx, dmean, dvar = ops.batch_normalize_adjoint([0, 1], dy, x, mean, var)
+    e, r, dy64 = x64 - mean.double().view(bs), var.double().rsqrt(), dy.double()
+    wvar = (dy64 * e).sum(ax) * -0.5 * r / var.double()
+    wmean = -r * dy64.sum(ax) - 2.0 * wvar * e.sum(ax) / m
+    assert_sum_close(host(dvar), host(wvar), "dvar")
+    assert_sum_close(host(dmean), host(wmean), "dmean")
+    want = dy64 * r.view(bs) + (2.0 * wvar / m).view(bs) * e + (wmean / m).view(bs)
+    assert bool(((dx.double() - want).abs() <= 1e-5 + 1e-4 * want.abs()).all()), (shape, "dx")
+
+
+# one million floats to a channel and clusters for 148 SMs: the lines of normalized_apart
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1337, 1, 28, 28), (1338, 1, 28, 28), (700, 3, 40, 40), (1338, 18, 28, 28), (1338, 19, 28, 28), (1100, 2, 31, 31)])
+def test_large_layers_of_few_channels(shape):
+    compare_with_float64(shape)
