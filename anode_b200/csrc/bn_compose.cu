@@ -22,6 +22,7 @@ namespace cg = cooperative_groups;
 namespace anode_b200 {
 
 constexpr uint32_t kComposeThreads = 512, kComposeCluster = 8;
+constexpr uint64_t kComposeSmall = 128u << 10;      // floats of a small channel (launch_compose)
 constexpr int kComposeHold = 4;       // vectors per tensor that a thread holds (64 registers: two blocks per SM)
 
 struct ComposeArgs {
@@ -184,9 +185,14 @@ static int launch_compose(const ComposeArgs &g, bool aligned, cudaStream_t strea
 {
   const bool vec = g.dim0 % 4 == 0 && aligned;
   const uint64_t total = (uint64_t)(vec ? g.dim0 / 4 : g.dim0) * g.N;
-  // the smallest cluster that holds the channel; else enough blocks for the device
+  // The smallest cluster that holds the channel; else enough blocks for the device.  Forward passes that load the floats of
+  // small channels one by one: no larger than makes eight blocks per SM, more blocks only repeat the fixed steps of a cluster
+  // for a few floats a thread.  Us with the cluster that would hold the channel, with this one, and op by op: [3,1024,55,55]
+  // 91, 48, 60, [8,2048,55,55] 395, 152, 313, [16,1024,33,33] 181, 78, 113, [6,512,55,55] 83, 49, 60, but [65,1024,55,55] 684,
+  // 798, 1251.
+  const uint64_t most = DIR == 0 && !vec && total <= kComposeSmall ? 8ull * sm_count() : ~0ull;
   uint32_t cs = 1;
-  while (cs < kComposeCluster && total > (uint64_t)cs * kComposeThreads * kComposeHold) cs *= 2;
+  while (cs < kComposeCluster && total > (uint64_t)cs * kComposeThreads * kComposeHold && (uint64_t)g.C * cs < most) cs *= 2;
   const bool hold = total <= (uint64_t)cs * kComposeThreads * kComposeHold;
   const uint64_t each = (total + cs - 1) / cs;
   const uint32_t threads = each < kComposeThreads ? (uint32_t)(each + 31) / 32 * 32 : kComposeThreads;

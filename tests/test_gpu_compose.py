@@ -113,3 +113,10 @@ def compare_with_float64(shape, seed=0):
 @pytest.mark.parametrize("shape", [(1337, 1, 28, 28), (1338, 1, 28, 28), (700, 3, 40, 40), (1338, 18, 28, 28), (1338, 19, 28, 28), (1100, 2, 31, 31)])
 def test_large_layers_of_few_channels(shape):
     compare_with_float64(shape)
+
+
+# rows that are loaded float by float, on both sides of eight blocks per SM and of 128 Ki floats to a channel
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(3, 1024, 55, 55), (8, 600, 55, 55), (2, 2048, 55, 55), (6, 295, 55, 55), (6, 297, 55, 55), (44, 300, 55, 55)])
+def test_scalar_rows_of_many_channels(shape):
+    compare_with_float64(shape)
