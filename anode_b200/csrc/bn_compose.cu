@@ -71,7 +71,10 @@ __global__ void __launch_bounds__(kComposeThreads, 2) bn_compose_kernel(const Co
 
   // the thread's vectors are j0, j0 + stride, ... of the channel, B of them in flight; places by walking (row, column) along
   // (float offsets are below 2^32, check_dims)
-  constexpr int B = HOLD || DIR == 0 ? kComposeHold : kComposeHold / 2;
+  // (H batches a turn, so that the adjoint's plain sums have four chains of additions per thread, as the ops they stand for,
+  // and that of dy * (x - mean) two: with two chains each the sum of 8 M equal dy was off by 8.0e-6, the ops' by 4.2e-6)
+  constexpr int B = HOLD || DIR == 0 ? kComposeHold : kComposeHold / 2, H = VEC == 1 ? kComposeHold / B : 1;
+  constexpr int S = kComposeHold / (B * H), D = HOLD ? kComposeHold : kComposeHold / 2;
   const uint32_t per_row = g.dim0 / VEC, total = per_row * g.N, rs = g.C * g.dim0;
   const uint32_t stride = cs * blockDim.x, j0 = rank * blockDim.x + threadIdx.x;
   const uint32_t row0 = j0 / per_row, drow = stride / per_row;
@@ -83,25 +86,29 @@ __global__ void __launch_bounds__(kComposeThreads, 2) bn_compose_kernel(const Co
   pdl_trigger();
 
   Pack<VEC> vx[B], vd[DIR == 1 ? B : 1];
-  // visit(f): f(x, dy, offset) for every vector, B loads in flight; the first visit of a held channel loads it
+  // visit(f): f(x, dy, offset, number of its chain) for every vector, B loads in flight; the first visit of a held channel loads it
   bool loaded = false;
   auto visit = [&](auto f) {
     uint32_t off = off0, col = col0;
-    for (uint32_t k = 0; k < cnt; k += B) {
-      uint32_t at[B];
+    for (uint32_t k0 = 0; k0 < cnt; k0 += B * H) {
 #pragma unroll
-      for (int u = 0; u < B; ++u) {
-        at[u] = off;
-        if (k + u < cnt && !(HOLD && loaded)) {
-          vx[u] = Pack<VEC>::load(g.x + off);
-          if (DIR == 1) vd[u] = Pack<VEC>::load(g.dy + off);
+      for (int h = 0; h < H; ++h) {
+        const uint32_t k = k0 + h * B;
+        uint32_t at[B];
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+          at[u] = off;
+          if (k + u < cnt && !(HOLD && loaded)) {
+            vx[u] = Pack<VEC>::load(g.x + off);
+            if (DIR == 1) vd[u] = Pack<VEC>::load(g.dy + off);
+          }
+          off += step; col += dcol;
+          if (col >= per_row) { col -= per_row; off += wrap; }
         }
-        off += step; col += dcol;
-        if (col >= per_row) { col -= per_row; off += wrap; }
-      }
 #pragma unroll
-      for (int u = 0; u < B; ++u)
-        if (k + u < cnt) f(vx[u], vd[DIR == 1 ? u : 0], at[u], u);
+        for (int u = 0; u < B; ++u)
+          if (k + u < cnt) f(vx[u], vd[DIR == 1 ? u : 0], at[u], u + h * B);
+      }
       if (HOLD) break;
     }
     loaded = true;
@@ -144,14 +151,16 @@ __global__ void __launch_bounds__(kComposeThreads, 2) bn_compose_kernel(const Co
     });
   } else {
     const float m = g.mean_in[c], va = g.var_in[c], r = rsqrtf(va);
-    float a1[B] = {}, a2[B] = {}, a3[B] = {};
+    float a1[D] = {}, a2[kComposeHold] = {}, a3[kComposeHold] = {};
     visit([&](const Pack<VEC> &x, const Pack<VEC> &dy, uint32_t, int u) {
 #pragma unroll
-      for (int i = 0; i < VEC; ++i) { const float d = x.v[i] - m; a1[u] = fmaf(dy.v[i], d, a1[u]); a2[u] += dy.v[i]; a3[u] += d; }
+      for (int i = 0; i < VEC; ++i) { const float d = x.v[i] - m; a1[u % D] = fmaf(dy.v[i], d, a1[u % D]); a2[u * S + i % S] += dy.v[i]; a3[u * S + i % S] += d; }
     });
     double v[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-    for (int u = 0; u < B; ++u) { v[0] += (double)a1[u]; v[1] += (double)a2[u]; v[2] += (double)a3[u]; }
+    for (int u = 0; u < D; ++u) v[0] += (double)a1[u];
+#pragma unroll
+    for (int u = 0; u < kComposeHold; ++u) { v[1] += (double)a2[u]; v[2] += (double)a3[u]; }
     if (cs > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     cluster_sums(cluster, v, part, gather[0]);
     const float dvar = (float)((double)(-0.5f * r / va) * v[0]);                            // batch_norm.cu:492

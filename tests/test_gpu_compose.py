@@ -120,3 +120,23 @@ def test_large_layers_of_few_channels(shape):
 @pytest.mark.parametrize("shape", [(3, 1024, 55, 55), (8, 600, 55, 55), (2, 2048, 55, 55), (6, 295, 55, 55), (6, 297, 55, 55), (44, 300, 55, 55)])
 def test_scalar_rows_of_many_channels(shape):
     compare_with_float64(shape)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(2657, 3, 56, 56), (2755, 3, 55, 55), (500, 64, 56, 56), (1000, 40, 28, 28), (40, 5, 28, 28)])
+@pytest.mark.parametrize("value", [1.1, 0.7])
+def test_the_sums_of_the_adjoint_are_no_less_exact_than_the_ops(shape, value):
+    """Equal summands round the same way at every addition, so that a longer chain of additions shows."""
+    c, ax, axes = shape[1], (0, 2, 3), [0, 1]
+    x, dy = torch.full(shape, value, device="cuda"), torch.full(shape, 1.3 * value, device="cuda")
+    zero, one = torch.zeros(c, device="cuda"), torch.ones(c, device="cuda")
+    op_dvar, op_sum = torch.empty(c, device="cuda"), torch.empty(c, device="cuda")
+    ops.BatchNormalize2dBwdVarianceOp.apply(axes, dy, x, zero, one, op_dvar)
+    ops.BatchNormalize2dBwdMeanOp.apply(axes, dy, one, op_sum)
+    _, _, dvar = ops.batch_normalize_adjoint(axes, dy, x, zero, one)
+    _, dmean, _ = ops.batch_normalize_adjoint(axes, dy, torch.zeros_like(x), zero, one)      # dmean is -sum(dy) alone
+    want_dvar, want_sum = -0.5 * (dy.double() * x.double()).sum(ax), -dy.double().sum(ax)
+    # (a sum and its product with -0.5 are rounded once each: 2^-23 beside the chain's own error)
+    for got, op, want in ((dvar, op_dvar, want_dvar), (dmean, op_sum, want_sum)):
+        err, err_op = (((t.double() - want) / want).abs().max().item() for t in (got, op))
+        assert err <= err_op + 2.0 ** -22, (shape, value, err, err_op)
