@@ -125,7 +125,8 @@ __global__ void __launch_bounds__(kChanThreads, 2) bn_chan_kernel(const FusedArg
         for (int i = 0; i < VEC; ++i) { const float d = vx[k].v[i] - m; dev += d; q = fmaf(d, d, q); }
       }
     q = warp_sum_all(q); dev = warp_sum_all(dev);
-    r = make_float4(n, m, q, dev);
+    // (a sum that holds an infinity is one, whatever is left beside it)
+    r = make_float4(n, m, q, fabsf(m) <= 3.402823466e38f ? dev : 0.f);
   } else {
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll

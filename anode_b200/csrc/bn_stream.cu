@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamBlocks) bn_stream_kerne
           float t = 0.f;
 #pragma unroll
           for (int i = 0; i < kBatch; ++i) t += vx[i].v[e];
-          K[e] = t * inv;
+          K[e] = fabsf(t) < 1e36f ? t * inv : 0.f;      // (an infinity or a NaN is no shift, the sums show it)
         }
       }
       // batch by batch, so that a long column's sums are rounded once per batch

@@ -140,3 +140,33 @@ def test_the_sums_of_the_adjoint_are_no_less_exact_than_the_ops(shape, value):
     for got, op, want in ((dvar, op_dvar, want_dvar), (dmean, op_sum, want_sum)):
         err, err_op = (((t.double() - want) / want).abs().max().item() for t in (got, op))
         assert err <= err_op + 2.0 ** -22, (shape, value, err, err_op)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,kernel", [((2, 8, 7, 7), "register"), ((32, 64, 28, 28), "register"), ((9, 5, 55, 55), "register"),
+                                          ((1024, 64, 7, 7), "stream"), ((2000, 20, 12, 12), "stream"), ((64, 8, 56, 56), "tiled")])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+def test_the_mean_shows_an_infinity(shape, kernel, value):
+    """As the ops' own: the mean and the running mean of a channel that holds an infinity are that infinity, those of one that
+    holds both or a NaN are NaN; the variance and the output are NaN, and the other channels' results are what they are without."""
+    assert ops.serving_kernel(shape, 0) == kernel
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    x = torch.randn(shape, device="cuda", generator=g)
+    c = shape[1]
+
+    def run(x):
+        return ops.batch_normalize_2d(x, [0, 1], True, 0.1, 1e-5, torch.zeros(c, device="cuda"), torch.ones(c, device="cuda"))
+    clean = run(x)
+    for places in (((0, 0, 0, 0),), ((-1, 0, -1, -1),), ((0, 0, 0, 1), (-1, 0, 0, 2))):
+        p = x.clone()
+        for q in places:
+            p[q] = value
+        p[0, 1, 0, 0], p[-1, 1, -1, -1] = float("inf"), float("-inf")
+        y, mean, var, am, av = run(p)
+        want = torch.full((), value)
+        for t in (mean, am):
+            assert torch.equal(t[:1].cpu().nan_to_num(7.0, 8.0, 9.0), want[None].nan_to_num(7.0, 8.0, 9.0)) and bool(t[1].isnan()), (places, t[:2])
+        assert bool(var[:2].isnan().all() and av[:2].isnan().all() and y[:, :2].isnan().all())
+        for got, ref in zip((y[:, 2:], mean[2:], var[2:], am[2:], av[2:]), (clean[0][:, 2:],) + tuple(t[2:] for t in clean[1:])):
+            assert torch.equal(got, ref)
