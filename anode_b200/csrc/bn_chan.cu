@@ -291,6 +291,10 @@ bool chan_applies(const FusedArgs &a, int dir, bool aligned)
 // [16,512,56,56] 82 and 59, [35,512,28,28] 42 and 36, but [64,1024,18,18] 69 and 71, [1,2048,100,100] 51 and 54; residual
 // [16,512,56,56] 80 / 109 and 62 / 96, [8,1024,56,56] 68 / 100 and 61 / 98, but [2,512,128,128] 41 / 61 and 44 / 65,
 // [25,1024,28,28] 51 / 76 and 57 / 80.  (Forward passes: [64,512,28,28] 52 and 52, [25,1024,28,28] 36 and 47.)
+// Nor below rows of 480 floats: 1024 channels of 31 K floats, backward, residual forward and backward, here and there, rows of
+// 324 86 / 78 / 120 and 107 / 91 / 137, 400 84 / 77 / 117 and 95 / 84 / 122, but 484 85 / 78 / 118 and 88 / 81 / 118, 676
+// 85 / 77 / 117 and 77 / 77 / 117, and of 25 K floats 484 77 / 70 / 105 and 68 / 63 / 96.
+constexpr uint32_t kChanTiledRow = 480;
 constexpr uint64_t kChanTiled = 16u << 20, kChanTiledExtra = 18u << 20, kChanTiledChannel = 24u << 10;
 constexpr uint64_t kChanLarge = 8u << 20, kChanLargeScalar = 3u << 20, kChanLargeExtra = 5u << 20;
 constexpr uint64_t kChanWaves = 1500000, kChanShortest = 1200000;
@@ -305,8 +309,8 @@ bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
   const uint64_t channel = (uint64_t)a.plan.dim0 * a.plan.N, elements = channel * a.plan.C;
   const uint32_t most = dir == 0 && !extra ? 32u : 16u;
   if (g.vec == 4) {
-    if (tiled_ok && (dir == 1 || extra) && channel >= kChanTiledChannel && elements >= (extra ? kChanTiledExtra : kChanTiled) &&
-        tiled_takes(a.plan.dim0, elements, dir, extra)) return false;
+    if (tiled_ok && (dir == 1 || extra) && a.plan.dim0 >= kChanTiledRow && channel >= kChanTiledChannel &&
+        elements >= (extra ? kChanTiledExtra : kChanTiled) && tiled_takes(a.plan.dim0, elements, dir, extra)) return false;
     if (elements < kChanLarge || channel <= (uint64_t)kChanThreads * kChanCluster * most / 2) return true;
     return !stream_preferred(a, dir, aligned, tiled_ok) &&
            !(tiled_ok && ((dir == 0 && !extra) || tiled_takes(a.plan.dim0, elements, dir, extra)));

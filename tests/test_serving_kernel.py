@@ -175,3 +175,9 @@ def test_ragged_tiles_hold_equally_many_rows():
     ((25, 1024, 28, 28), ("register", "register"), ("register", "register"))])
 def test_routes_between_the_streaming_the_register_resident_and_the_tiled_kernel(shape, one, residual):
     assert routes(shape) == one + residual
+
+
+@pytest.mark.parametrize("shape,kernel", [((96, 1024, 18, 18), "register"), ((98, 1024, 16, 20), "register"), ((78, 1024, 20, 20), "register"),
+                                          ((65, 1024, 22, 22), "tiled"), ((47, 1024, 26, 26), "tiled")])
+def test_channels_that_a_team_holds_stay_there_below_rows_of_480_floats(shape, kernel):
+    assert routes(shape) == ("register", kernel, kernel, kernel)
