@@ -170,3 +170,46 @@ def test_the_mean_shows_an_infinity(shape, kernel, value):
         assert bool(var[:2].isnan().all() and av[:2].isnan().all() and y[:, :2].isnan().all())
         for got, ref in zip((y[:, 2:], mean[2:], var[2:], am[2:], av[2:]), (clean[0][:, 2:],) + tuple(t[2:] for t in clean[1:])):
             assert torch.equal(got, ref)
+
+
+# forward passes that the streaming kernel serves, and large layers whose fused calls are other kernels' but whose composition is not
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,kernel", [((1024, 64, 7, 7), "stream"), ((512, 128, 7, 7), "stream"), ((2000, 20, 12, 12), "stream"),
+                                          ((64, 8, 56, 56), "tiled"), ((64, 95, 55, 55), "tiled"), ((512, 64, 19, 19), "plain")])
+def test_every_route_of_the_composition(shape, kernel):
+    assert ops.serving_kernel(shape, 0) == kernel
+    compare_with_float64(shape, seed=1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(2, 512, 7, 7), (64, 8, 56, 56), (1024, 64, 7, 7), (1400, 2, 28, 28), (9, 60, 55, 55)])
+def test_a_chain_of_overlapping_compositions(shape):
+    """Each launch may begin before the one ahead of it on the stream has ended and reads what that one writes: the same results
+    as with a synchronisation after every call, in a loop and as one captured graph."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    x, dy = torch.randn(shape, device="cuda", generator=g), torch.randn(shape, device="cuda", generator=g)
+    am, av = torch.zeros(shape[1], device="cuda"), torch.ones(shape[1], device="cuda")
+
+    def chain(after):
+        am.zero_(), av.fill_(1.0)
+        out, t = [], x
+        for _ in range(3):
+            y, mean, var, _, _ = ops.batch_normalize_2d(t, [0, 1], True, 0.1, 1e-5, am, av); after()
+            y = ops.relu(y, inplace=True); after()
+            dz = ops.PositiveClipBwdOp.apply(dy, y, torch.empty_like(y)); after()
+            dx, dmean, dvar = ops.batch_normalize_adjoint([0, 1], dz, t, mean, var); after()
+            out += [y, mean, var, dz, dx, dmean, dvar]
+            t = dx
+        return out + [am, av]
+    want = [a.clone() for a in chain(torch.cuda.synchronize)]
+    for _ in range(10):
+        for i, (a, b) in enumerate(zip(chain(lambda: None), want)):
+            assert torch.equal(a, b), i
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = chain(lambda: None)
+    for _ in range(3):
+        graph.replay()
+        for i, (a, b) in enumerate(zip(got, want)):
+            assert torch.equal(a, b), i
