@@ -57,7 +57,6 @@ struct RingCtl {
   unsigned long long full[kMaxSlots], empty[kMaxSlots];
   unsigned long long res_full[kResQ], res_empty[kResQ];
   unsigned long long coef_full[kCoefQ], coef_empty[kCoefQ];
-  float mom[3 * (kConsumers / 32)];
   volatile uint32_t abort;
   uint32_t last_block;
   uint32_t parity;       // which of the two tagged-partial buffers this launch uses
@@ -622,19 +621,6 @@ __device__ __forceinline__ Moments64 merge64(Moments64 a, Moments64 b)
   const double f = b.n / n, d = b.mean - a.mean;
   return Moments64{n, a.mean + d * f, a.m2 + b.m2 + d * d * a.n * f};
 }
-__device__ __forceinline__ Moments64 warp_merge64(Moments64 a)
-{
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    Moments64 b;
-    b.n = __shfl_down_sync(0xffffffffu, a.n, o);
-    b.mean = __shfl_down_sync(0xffffffffu, a.mean, o);
-    b.m2 = __shfl_down_sync(0xffffffffu, a.m2, o);
-    a = merge64(a, b);
-  }
-  return a;
-}
-constexpr int kFinBatch = 8;     // partial loads a lane keeps in flight (regime S)
 constexpr int kFinRegs = 16;     // partials a lane holds in registers (regime R: 512 tiles per unit)
 
 // Regime R: one channel, up to thousands of partials.  The merge sits on the critical path of the
