@@ -292,11 +292,10 @@ uint64_t ring_ws_bytes(const FusedArgs &a, int dir, bool aligned)
 }
 
 // Whether the tiled kernel, which can serve the call, is the faster form.  Not for the residual epilogue on ragged rows below
-// these lengths (forward, backward), us here and on the plain kernel: forward [2123,21,139] 51 and 48, but [998,17,145] 25
-// and 36; backward [1841,15,165] 60 and 47, [177,77,183] 39 and 36, but [966,13,191] 31 and 35.
-// (On large layers of long aligned rows that leave much of a slot empty the plain kernel would be the faster form of the
-// residual forward pass, [118,100,3516] 190 and 141, but its partials lie over the tagged words that an ordinary call of the
-// tiled kernel keeps in the same workspace.  A ragged plan's words lie apart.)
+// these lengths (forward, backward).  The lines were drawn when the kernel read every tile twice, us here and on the plain
+// kernel: forward [2123,21,139] 51 and 48, but [998,17,145] 25 and 36; backward [1841,15,165] 60 and 47, [177,77,183] 39 and
+// 36, but [966,13,191] 31 and 35.  With tiles in tensor memory it is the faster one below them, too: 41 and 61, 23 and 40; 41
+// and 48, 29 and 36, 25 and 36.
 constexpr uint32_t kRaggedMinRowExtra[2] = {144, 184};
 static bool tiled_preferred(const FusedArgs &a, int dir)
 {
@@ -304,7 +303,9 @@ static bool tiled_preferred(const FusedArgs &a, int dir)
 }
 
 // Layers of 16-byte aligned rows from which on the tiled kernel is faster than the streaming kernel: it reads a layer once,
-// the other one twice, but a tile costs it some 2 us whatever its size.  Forward / backward in us, tiled and streaming:
+// the other one twice, but a tile costs it some 2 us whatever its size.  One line for all rows of 320 floats and more, drawn
+// where the shortest of them cross; longer rows cross earlier ([100,128,28,28], 10 M, backward and residual forward / backward:
+// streaming kernel 40 and 33 / 50, tiled 29 and 28 / 42).  Forward / backward in us, tiled and streaming:
 //   rows of 256   24 M elements 46 / 84 and 49 / 83, 67 M [4096,64,16,16] 107 / 229 and 131 / 228, [512,512,16,16] 105 / 231, 104 / 177
 //   rows of 324   10 M 25 / 36 and 21 / 35, 14 M 31 / 48 and 29 / 50, 24 M 45 / 75 and 56 / 78
 //   rows of 576   10 M 22 / 30 and 18 / 30, 14 M 26 / 38 and 26 / 43, 24 M 40 / 60 and 43 / 73

@@ -354,7 +354,8 @@ bool stream_applies(const FusedArgs &a, int dir, bool aligned)
 
 // Where this kernel is taken (after the register-resident kernel): all rows that the tiled kernel does not serve, and of
 // those it does serve (`tiled_ok`) the short ones and the medium ones of layers and channels that are not too large
-// (tiled_takes; beyond that line by the channel's size, as measured when the tiled kernel read every tile twice).
+// (tiled_takes; short of that line by the channel's size, as measured when the tiled kernel read every tile twice: of rows of
+// 784 and 1024 floats it would have more now, see there).
 constexpr uint32_t kStreamShortRow = 512, kStreamMediumRow = 600, kStreamLongRow = 1024;
 // Layers of few channels leave the device to a few clusters whose threads walk hundreds of samples.  With rows that the
 // tiled kernel serves it is the faster one there, forward / backward, here and there: [7663,4,412] 47 / 119 and 31 / 54,

@@ -40,8 +40,8 @@ WORKLOADS = {
 }
 DEFAULT = "cfg3_syncbn"
 # DRAM bytes per element of the default workload's kernels come from the ncu summary under profiles/
-# (row "traffic per element" of its counter table: dram__bytes_read.sum + dram__bytes_write.sum per launch
-# / elements, captured on a 16-channel case of the same per-channel geometry; the kernels work channel by
+# (row "traffic per element" of its first counter table: dram__bytes_read.sum and the output tensor per launch
+# / elements, captured on a 32-channel case of the same per-channel geometry; the kernels work channel by
 # channel, so traffic is proportional to the channel count and is scaled by elements here).
 TRAFFIC_SOURCE = "profiles/bn_ring_kernels_cfg3_syncbn.md"
 
@@ -629,7 +629,7 @@ def main():
     for key, rk in (("bwd", "roofline"), ("fwd", "roofline_fwd")):
         if key in tr:
             line[rk]["traffic"] = tr[key] * main_res["elements_local"]
-            line[rk]["traffic_source"] = TRAFFIC_SOURCE + " (16-channel capture, scaled by elements)"
+            line[rk]["traffic_source"] = TRAFFIC_SOURCE + " (32-channel capture, scaled by elements)"
 
     if world == 1 and not args.no_extras:
         others = {}
