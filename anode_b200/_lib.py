@@ -98,7 +98,7 @@ SIGNATURES = {
     "anode_gpu_batch_norm_stream_geometry": (c_int, _D + [c_int, ctypes.POINTER(u32)]),
     "anode_gpu_batch_norm_tiled_geometry": (c_int, _D + [c_int, ctypes.POINTER(u32)]),
     "anode_gpu_batch_norm_tiled_keep": (c_int, _D + [c_int, c_int, u32, u32, ctypes.POINTER(u32)]),
-    "anode_gpu_batch_norm_ragged_whole": (c_int, [c_int, u32]),
+    "anode_gpu_batch_norm_tiled_last_piece": (u32, _D + [c_int, c_int]),
     "anode_gpu_batch_norm_fused_serving_kernel": (c_int, _D + [c_int] * 4),
     "anode_gpu_batch_norm_fused_kernel_kind": (c_int, _D + [c_int]),
     "anode_gpu_batch_norm_add_act_fused_kernel_kind": (c_int, _D + [c_int]),

@@ -198,6 +198,12 @@ static bool ring_plan_with(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool 
   // short rows (regime S) belong to the cluster kernel or the plain kernel
   if (p.regime != 0) return false;
   if (ragged) {
+    // no last piece of a row of fewer than four floats (ragged_whole)
+    while (p.pieces > 1 && dim0 - (p.pieces - 1) * p.piece_len < 4) {
+      p.piece_len -= 4; p.pieces = ceil_div_u32(dim0, p.piece_len);
+      p.tiles_per_unit = p.sample_blocks * p.pieces; p.total_tiles = p.units * p.tiles_per_unit;
+      p.grid = p.total_tiles < sm_count() * bps ? p.total_tiles : sm_count() * bps;
+    }
     // Equal tiles: the last of a channel would hold what is left over and cost a step all the same.  Forward, before and
     // now: [846,106,131] 67.8 and 61.8 us, [371,210,135] 65.8 and 55.5, [64,95,55,55] 41.9 and 42.0.
     p.rows_per_tile = ceil_div_u32(N, p.sample_blocks);
@@ -876,8 +882,14 @@ extern "C" int anode_gpu_batch_norm_tiled_keep(uint32_t dim0, uint32_t dim1, uin
   return ANODE_OK;
 }
 
-// ---- diagnostics: the tiled kernel's test for the inner vectors of a ragged row piece (no GPU needed) ----
-extern "C" int anode_gpu_batch_norm_ragged_whole(int first, uint32_t len) { return anode_b200::ragged_whole(first, len) ? 1 : 0; }
+// ---- diagnostics: floats of a row's last piece in the tiled kernel, 0 where it does not apply (no GPU needed) ----
+extern "C" uint32_t anode_gpu_batch_norm_tiled_last_piece(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual)
+{
+  using namespace anode_b200;
+  Plan p; RingGeom g;
+  if ((dir != 0 && dir != 1) || check_dims(dim0, dim1, dim2) || !ring_plan_for(dim0, dim1, dim2, true, dir, residual != 0, p, g)) return 0;
+  return dim0 - (p.pieces - 1) * p.piece_len;
+}
 
 // ---- diagnostics: the tile plan, for tests of the index arithmetic (no GPU needed) ----------
 extern "C" int anode_gpu_batch_norm_fused_plan(uint32_t dim0, uint32_t dim1, uint32_t dim2, int aligned,

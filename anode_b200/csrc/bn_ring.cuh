@@ -384,7 +384,7 @@ __device__ __forceinline__ void visit_reduce(const FusedArgs &a, const RingGeom 
       auto take = [&](const Quad &v, bool live) {
         const int i0 = live ? w.first() : len;
         Quad e{add2(v.a, nK), add2(v.b, nK)};
-        if (ragged_whole(i0, d.z)) {
+        if (ragged_whole(i0, len)) {
           n += 4;
         } else {      // foreign floats at a row's ends count nothing
           const float4 t = floats(e);
@@ -450,7 +450,7 @@ __device__ __forceinline__ void visit_reduce(const FusedArgs &a, const RingGeom 
         if constexpr (EXTRA) { if (dres && live) stg_quad(dres + w.at, z); }
       } else {
         const int i0 = live ? w.first() : len;
-        if (ragged_whole(i0, d.z)) {
+        if (ragged_whole(i0, len)) {
           if constexpr (EXTRA) { if (dres) stg_quad(dres + w.vector(), z); }
         } else {      // (foreign floats may be anything, an infinity or a NaN too)
           const float4 t = floats(z), u = floats(e);
@@ -527,7 +527,7 @@ __device__ __forceinline__ void visit_apply(const FusedArgs &a, const RingGeom &
     }
     float *p = a.out + (RAGGED ? w.vector() : w.at);
     const int i0 = RAGGED ? w.first() : 0;
-    if (!RAGGED || ragged_whole(i0, d.z)) {
+    if (!RAGGED || ragged_whole(i0, len)) {
       if (acc) { const Quad old = ldg_quad(p); o.a = add2(old.a, o.a); o.b = add2(old.b, o.b); }
       stg_stream(p, o);
       if constexpr (EXTRA && DIR == 1) { if (dres) stg_stream(dres + (p - a.out), z); }
@@ -1018,8 +1018,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
         }
       } else {
         // from the boundary below each row's start to the one above its end, but never past the tensor's own end:
-        // the last floats of a tensor whose size is no multiple of four are stored by three lanes instead (they may
-        // belong to two pieces of the last row: the last one may hold a single float)
+        // the last floats of a tensor whose size is no multiple of four are stored by three lanes instead
         const uint32_t per_row = ragged_pitch(len), total = rs * P.N, whole = total & ~3u;
         auto span = [&](uint32_t r, uint32_t &start) {      // bytes of row r, and the float it is fetched from
           const uint32_t first = base + r * rs;

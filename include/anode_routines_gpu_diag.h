@@ -64,9 +64,9 @@ int anode_gpu_batch_norm_tiled_geometry(uint32_t dim0, uint32_t dim1, uint32_t d
 int anode_gpu_batch_norm_tiled_keep(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual,
                                     uint32_t tile, uint32_t warp, uint32_t *out);
 
-/* Whether the tiled kernel takes the 16-byte vector that begins with float number `first` (below 0: before it) of a ragged
- * row piece of `len` floats for one that lies wholly within the piece (1 or 0). */
-int anode_gpu_batch_norm_ragged_whole(int first, uint32_t len);
+/* Floats of the last of the pieces that the tiled kernel cuts a row into (the whole row where it cuts none), for direction
+ * `dir` of a call on 16-byte aligned tensors, with or without the residual epilogue; 0 where it does not apply. */
+uint32_t anode_gpu_batch_norm_tiled_last_piece(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual);
 
 /* Plan of the slice-resident kernel for `planes` tensors per shared-memory slot.  out (16 values): applies,
  * rows per piece, parts per row, floats per part, pieces per channel, blocks per team, teams, grid, pieces

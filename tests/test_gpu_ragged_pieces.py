@@ -1,6 +1,5 @@
-"""The tiled kernel on ragged rows whose last piece holds one to three floats (tests/test_ragged_pieces.py): results against
-float64, and not a float written outside y, dx and dresidual.  With two rows of 511 x 511 the tensor ends two floats behind a
-16-byte boundary, one of which belongs to the last piece but one."""
+"""The tiled kernel on ragged rows whose pieces are cut so that the last one holds four floats or more
+(tests/test_ragged_pieces.py): results against float64, and not a float written outside y, dx and dresidual."""
 import numpy as np
 import pytest
 import torch
@@ -22,7 +21,7 @@ def guarded(shape, fill):
     return a, t
 
 
-@pytest.mark.parametrize("shape", [s for s, _ in SHORT])
+@pytest.mark.parametrize("shape", SHORT)
 @pytest.mark.parametrize("residual", [False, True])
 def test_short_last_pieces(shape, residual):
     from anode_b200 import ops

@@ -1,30 +1,36 @@
-"""Ragged rows that the tiled kernel cuts into pieces of which the last holds one to three floats: which vectors count as lying
-wholly within a piece, and which shapes have such a piece (no GPU needed)."""
-import ctypes
+"""Ragged rows that the tiled kernel cuts into pieces: none may hold fewer than four floats, since a 16-byte vector of it is then
+taken for one that lies wholly within it (no GPU needed)."""
+import random
 
 import pytest
 import torch
 
 from anode_b200 import _lib, ops
 
-#: shape, and the directions in which its last piece is that short
-SHORT = [((1, 1, 511, 511), (0, 1)), ((2, 1, 511, 511), (0,)), ((1, 2, 511, 511), (0,)), ((1, 1, 513, 513), (0, 1)),
-         ((1, 1, 589, 589), (1,)), ((1, 1, 1023, 1023), (0,))]
+#: shapes whose pieces of an even size would leave one of one to three floats, in the forward or the backward pass
+SHORT = [(1, 1, 511, 511), (2, 1, 511, 511), (1, 2, 511, 511), (1, 1, 513, 513), (1, 1, 589, 589), (1, 1, 1023, 1023)]
 
 
-@pytest.mark.parametrize("length", list(range(1, 14)) + [1021, 65531])
-def test_a_whole_vector_lies_within_its_piece(length):
-    whole = _lib.load().anode_gpu_batch_norm_ragged_whole
-    for first in list(range(-3, min(length, 20) + 5)) + list(range(max(0, length - 9), length + 5)):
-        assert whole(first, length) == int(first >= 0 and first + 4 <= length), (first, length)
-    assert whole(length, length) == 0            # how a missing vector is described
+def last_pieces(d0, c, n):
+    return [_lib.load().anode_gpu_batch_norm_tiled_last_piece(d0, c, n, direction, residual) for direction in (0, 1) for residual in (0, 1)]
 
 
-@pytest.mark.parametrize("shape,directions", SHORT)
-def test_shapes_with_a_short_last_piece(shape, directions):
-    for direction in directions:
-        out = (ctypes.c_uint32 * 12)()
-        d0, c, n = ops.dims_of(torch.empty(shape, device="meta"))
-        assert _lib.load().anode_gpu_batch_norm_tiled_geometry(d0, c, n, direction, out) == 0
-        assert out[0] and 1 <= d0 % out[2] <= 3, list(out)
-        assert ops.serving_kernel(shape, direction) == "tiled"
+@pytest.mark.parametrize("shape", SHORT)
+def test_shapes_that_were_cut_short(shape):
+    pieces = last_pieces(*ops.dims_of(torch.empty(shape, device="meta")))
+    assert all(p >= 4 for p in pieces), pieces
+    assert [ops.serving_kernel(shape, direction) for direction in (0, 1)] == ["tiled", "tiled"]
+
+
+def test_no_piece_of_fewer_than_four_floats():
+    rng = random.Random(1)
+    rows = list(range(1001, 40000, 14)) + [rng.randrange(40000, 4000000) for _ in range(4000)] + [4091 * 4091, 16777217, 2 ** 27 + 1]
+    cut = 0
+    for d0 in rows:
+        for c, n in ((1, 1), (2, 1), (3, 5), (95, 2)):
+            if d0 * c * n >= 1 << 32:
+                continue
+            pieces = last_pieces(d0, c, n)
+            assert all(p >= 4 for p in pieces if p), (d0, c, n, pieces)
+            cut += sum(0 < p < d0 for p in pieces)
+    assert cut > 10000
