@@ -1,0 +1,620 @@
+// Fused batch-norm (+activation, +residual) for large layers of short rows, e.g. [1024, 2048, 7, 7]: what the streaming kernel
+// (bn_stream.cu) hands over, because it reads every tensor twice and leaves SMs idle between its clusters' steps.
+//
+// One persistent block per SM walks tiles of bands (bn_band.cuh) in unit-major order, as the tiled kernel (bn_ring.cuh) does with
+// tiles of rows: at step s it reduces its tile number s and applies number s - look.  Every tile stays on chip in between, in
+// tensor memory (256 KB per SM: look + 1 tiles of 62 KB), so each tensor crosses HBM once.
+//   producer warp     streams tiles into a ring of slots: one tensor copy (cp.async.bulk.tensor) per box, hundreds of runs of a
+//                     few hundred bytes in one instruction, where a bulk copy per run would be the producer's bound
+//   consumer warps    (8) a thread keeps its column's vectors of a tile, at most 16 per tensor, sums them up (two floats per
+//                     instruction) and leaves them in tensor memory (forward: x; backward: x - mean and dz); later reads them
+//                     back, applies the coefficients and stores
+//   delivery warp     folds the threads' sums of a tile to channels and stores one 8-byte word per channel and tile, forward (mean,
+//                     M2), backward (sum dz, sum dz*(x-mean)), never zero; no counter, fence or atomic
+//   coefficient warp  polls the words of the unit that is applied next until none is zero and merges them in a fixed order in
+//                     double precision (bit-identical in every block); the block of a unit's first tile writes its results
+// Two buffers of words alternate launch by launch: a delivery zeroes its word of the other one.  Every wait is bounded; one that
+// runs out sets a status bit and the block drains and leaves.  The launch is cooperative and takes the SM's whole shared memory,
+// so that no other block holds columns of tensor memory or waits for them.
+//
+// What bounds it: HBM, and some 10 us in which the schedule fills and drains.  Streaming kernel and this one, forward / backward:
+// [1024,2048,7,7] 179 / 298 and 143 / 203 us (0.88 / 0.93 of the copy bandwidth), residual epilogue 246 / 427 and 204 / 339 (0.92 /
+// 0.93); [256,1024,14,14] backward 148 -> 104, residual 137 / 211 -> 109 / 163.  On the way there: sixteen consumer warps (96
+// registers) 150 / 218; all vectors of the threads' sums added up one by one in double precision 156 / 238.
+#include <cuda.h>      // types only: the one function is looked up at run time
+
+#include "bn_band.cuh"
+#include "bn_host.h"
+#include "bn_pipe.cuh"
+
+namespace anode_b200 {
+
+struct BandCtl {
+  unsigned long long full[kBandMaxSlots], empty[kBandMaxSlots];
+  unsigned long long res_full[kBandQ], res_empty[kBandQ], coef_full[kBandQ], coef_empty[kBandQ];
+  volatile uint32_t abort;
+  uint32_t last_block, parity, tmem;
+};
+static_assert(sizeof(BandCtl) <= kBandCtlBytes, "BandCtl outgrew the room reserved for it");
+
+// x; dy; the residual (forward) or the saved output (backward): two-dimensional, [samples][C * dim0] floats
+struct BandMaps { CUtensorMap x, dy, e; };
+
+__device__ __forceinline__ void tensor_g2s(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t y, unsigned long long *bar, uint64_t policy)
+{
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;"
+               ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)), "l"(policy) : "memory");
+}
+
+// The tiles b, b + G, ... of a block, one after another: unit and number within the unit.
+struct BandWalk {
+  uint32_t unit, k, dq, dr, tiles;
+  __device__ __forceinline__ BandWalk(const BandGeom &g, uint32_t first, uint32_t G) : tiles(g.tiles)
+  {
+    unit = first / tiles; k = first - unit * tiles;
+    dq = G / tiles; dr = G - dq * tiles;
+  }
+  __device__ __forceinline__ void next()
+  {
+    unit += dq; k += dr;
+    if (k >= tiles) { k -= tiles; ++unit; }
+  }
+};
+
+__device__ __forceinline__ unsigned long long band_word(float lo, float hi)
+{
+  const unsigned long long w = ((unsigned long long)__float_as_uint(hi) << 32) | __float_as_uint(lo);
+  return w ? w : 1ull << 32;      // never zero ("not delivered")
+}
+
+template <int DIR, bool EXTRA>
+__global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArgs a, const BandGeom g, const __grid_constant__ BandMaps maps)
+{
+  extern __shared__ __align__(128) unsigned char sm[];
+  BandCtl *ctl = reinterpret_cast<BandCtl *>(sm);
+  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  uint32_t *status = a.status;
+  uint32_t *exit_ctr = reinterpret_cast<uint32_t *>(a.ws + g.hdr), *parity = exit_ctr + 1;
+  constexpr uint32_t kKept = DIR == 0 ? 1u : 2u;                    // tensors kept in tensor memory
+  constexpr uint32_t kPlanes = DIR == 0 ? 1u : EXTRA ? 3u : 2u;     // tensors of a reduce visit
+  constexpr bool kSlotToo = DIR == 0 && EXTRA;                      // apply visits fetch the residual
+
+  if (tid == 0) {
+    for (uint32_t i = 0; i < g.slots; ++i) { mbar_init(&ctl->full[i], 1); mbar_init(&ctl->empty[i], kBandWarps); }
+    for (uint32_t i = 0; i < kBandQ; ++i) {
+      mbar_init(&ctl->res_full[i], kBandWarps); mbar_init(&ctl->res_empty[i], 1);
+      mbar_init(&ctl->coef_full[i], 1); mbar_init(&ctl->coef_empty[i], kBandWarps);
+    }
+    ctl->abort = 0; ctl->last_block = 0; ctl->parity = *parity & 1u;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 0) { __syncwarp(); tmem_alloc(&ctl->tmem); tmem_fence_before(); }
+  __syncthreads();
+  tmem_fence_after();
+
+  const uint32_t dim0 = a.plan.dim0, C = a.plan.C, N = a.plan.N, rs = C * dim0;
+  const uint32_t b = blockIdx.x, G = gridDim.x;
+  const uint32_t mine = b < g.total ? (g.total - b + G - 1) / G : 0, steps = mine ? mine + g.look : 0;
+
+  if (warp < kBandWarps) {
+    // ------------------------------------------------------------------ consumers
+    const uint32_t grp0 = tid / g.L4;
+    const bool live = grp0 < g.groups;
+    const uint32_t grp = live ? grp0 : 0, v = live ? tid - grp0 * g.L4 : 0;
+    const uint32_t chA = 4 * v / dim0, eB = (chA + 1) * dim0 - 4 * v, chB = eB < 4 ? chA + 1 : chA;
+    const uint32_t pitch = g.box4 * 16, box = v / g.box4;
+    const uint32_t off_s = box * g.box_bytes + grp * pitch + (v - box * g.box4) * 16, step_s = g.groups * pitch;
+    const uint32_t off_g = grp * rs + 4 * v, step_g = g.groups * rs;
+    // places of a channel's elements that make the shift of its sums
+    auto place = [&](uint32_t f) { const uint32_t j = f / (g.box4 * 4); return j * g.box_bytes + (f - j * g.box4 * 4) * 4; };
+    uint32_t kA[3], kB[3];
+    if (DIR == 0) {
+      const uint32_t at[3] = {dim0 / 6, dim0 / 2, dim0 - 1 - dim0 / 6};
+#pragma unroll
+      for (int i = 0; i < 3; ++i) { kA[i] = place(chA * dim0 + at[i]); kB[i] = place(chB * dim0 + at[i]); }
+    }
+    const float slope = a.neg_slope;
+    const uint32_t tm0 = ctl->tmem + ((warp & 3u) << 21) + (warp >> 2) * (kTmemCols * 4 / kBandWarps), tm_step = g.vpt * 4 * kKept;
+    // a value per channel, for the thread's four floats
+    const bool b1 = eB > 1, b2 = eB > 2, b3 = eB > 3;
+    auto spread = [&](float A, float B) { return Quad{pair(A, b1 ? A : B), pair(b2 ? A : B, b3 ? A : B)}; };
+    // the thread's sums for its two channels
+    auto fold = [&](const f32x2 &sa, const f32x2 &sb, const f32x2 &qa, const f32x2 &qb) {
+      const float2 s0 = split(sa), s1 = split(sb), q0 = split(qa), q1 = split(qb);
+      float4 o;
+      o.x = (s0.x + (b1 ? s0.y : 0.f)) + ((b2 ? s1.x : 0.f) + (b3 ? s1.y : 0.f));
+      o.y = (q0.x + (b1 ? q0.y : 0.f)) + ((b2 ? q1.x : 0.f) + (b3 ? q1.y : 0.f));
+      o.z = (b1 ? 0.f : s0.y) + ((b2 ? 0.f : s1.x) + (b3 ? 0.f : s1.y));
+      o.w = (b1 ? 0.f : q0.y) + ((b2 ? 0.f : q1.x) + (b3 ? 0.f : q1.y));
+      return o;
+    };
+    // One tile.  FULL: it has all its rows, so no vector is missing (what threads without a column read and add up is not used).
+    auto reduce = [&](auto full, uint32_t rows, uint32_t slot, uint32_t tm, float4 *part) {
+      constexpr bool FULL = decltype(full)::value;
+      const uint32_t slot_off = g.off_slots + slot * g.slot_stride;
+      uint32_t ax = smem_u32(sm) + slot_off + off_s, r = grp;
+      if constexpr (DIR == 0) {
+        // shift of the sums: per channel the median of three elements
+        float Ka, Kb;
+        {
+          const uint32_t r1 = rows / 2 * pitch, r2 = (rows - 1) * pitch;
+          const unsigned char *xs = sm + slot_off;
+          auto at = [&](uint32_t o) { return *reinterpret_cast<const float *>(xs + o); };
+          Ka = median3(at(kA[0]), at(kA[1] + r1), at(kA[2] + r2));
+          Kb = median3(at(kB[0]), at(kB[1] + r1), at(kB[2] + r2));
+          Ka = fabsf(Ka) < 1e36f ? Ka : 0.f; Kb = fabsf(Kb) < 1e36f ? Kb : 0.f;      // (an infinity is no shift)
+        }
+        const Quad Kq = spread(Ka, Kb), nK = spread(-Ka, -Kb);
+        f32x2 sa = 0, sb = 0, qa = 0, qb = 0;
+        auto load = [&](Quad &x) {
+          if constexpr (FULL) x = lds_quad(ax);
+          else { x = Kq; if (r < rows) x = lds_quad(ax); r += g.groups; }
+          ax += step_s;
+        };
+        auto take = [&](const Quad &x) {
+          const f32x2 da = add2(x.a, nK.a), db = add2(x.b, nK.b);
+          sa = add2(sa, da); qa = fma2(da, da, qa); sb = add2(sb, db); qb = fma2(db, db, qb);
+        };
+        uint32_t i = 0;
+        for (; i + 4 <= g.vpt; i += 4, tm += 16) {
+          Quad x0, x1, x2, x3;
+          load(x0); load(x1); load(x2); load(x3);
+          if constexpr (!FULL) __syncwarp();
+          tmem_st(tm, x0, x1, x2, x3);
+          take(x0); take(x1); take(x2); take(x3);
+        }
+        for (; i < g.vpt; ++i, tm += 4) {
+          Quad x0;
+          load(x0);
+          if constexpr (!FULL) __syncwarp();
+          tmem_st(tm, x0);
+          take(x0);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ctl->empty[slot]);
+        if (live && grp == 0) {
+          float *kbox = reinterpret_cast<float *>(part + kBandConsumers);
+          if (4 * v == chA * dim0) kbox[chA] = Ka;
+          if (chB != chA) kbox[chB] = Kb;
+        }
+        part[tid] = fold(sa, sb, qa, qb);
+      } else {
+        const float4 *side = reinterpret_cast<const float4 *>(sm + g.off_side) + slot * kBandChannels;
+        const float4 pA = side[chA], pB = side[chB];
+        const Quad mean = spread(pA.x, pB.x), nmean = spread(-pA.x, -pB.x), scale = spread(pA.y, pB.y), beta = spread(pA.z, pB.z);
+        f32x2 s1a = 0, s1b = 0, s2a = 0, s2b = 0;
+        // a missing vector is (mean, 0), which adds nothing
+        auto load = [&](Quad &x, Quad &gy, Quad &y) {
+          y = quad(0.f);
+          if constexpr (!FULL) { x = mean; gy = quad(0.f); }
+          if (FULL || r < rows) {
+            x = lds_quad(ax); gy = lds_quad(ax + g.plane_bytes);
+            if constexpr (EXTRA) y = lds_quad(ax + 2 * g.plane_bytes);
+          }
+          ax += step_s;
+          if constexpr (!FULL) r += g.groups;
+        };
+        auto work = [&](const Quad &x, const Quad &gy, Quad y, Quad &e, Quad &z) {
+          e.a = add2(x.a, nmean.a); e.b = add2(x.b, nmean.b);
+          if constexpr (!EXTRA) { y.a = fma2(e.a, scale.a, beta.a); y.b = fma2(e.b, scale.b, beta.b); }
+          // dz = dy * act'(y)  (routines_gpu/flat_map.cu:191-192)
+          z.a = mul2(gy.a, slopes(y.a, slope)); z.b = mul2(gy.b, slopes(y.b, slope));
+          s1a = add2(s1a, z.a); s2a = fma2(z.a, e.a, s2a); s1b = add2(s1b, z.b); s2b = fma2(z.b, e.b, s2b);
+        };
+        uint32_t i = 0;
+        for (; i + 2 <= g.vpt; i += 2, tm += 16) {
+          Quad x0, g0, y0, x1, g1, y1, e0, z0, e1, z1;
+          load(x0, g0, y0); load(x1, g1, y1);
+          work(x0, g0, y0, e0, z0); work(x1, g1, y1, e1, z1);
+          if constexpr (!FULL) __syncwarp();
+          tmem_st(tm, e0, z0, e1, z1);
+        }
+        if (i < g.vpt) {
+          Quad x0, g0, y0, e0, z0;
+          load(x0, g0, y0);
+          work(x0, g0, y0, e0, z0);
+          if constexpr (!FULL) __syncwarp();
+          tmem_st(tm, e0, z0);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ctl->empty[slot]);
+        part[tid] = fold(s1a, s1b, s2a, s2b);
+      }
+    };
+    // alive: the thread has a column of this unit; base: the tile's first float, from which a thread's places are below 4 GB
+    auto apply = [&](auto full, uint32_t rows, bool alive, size_t base, uint32_t slot, uint32_t tm, const float4 *coef) {
+      constexpr bool FULL = decltype(full)::value;
+      const float4 pA = coef[2 * chA], pB = coef[2 * chB];
+      const Quad scale = spread(pA.y, pB.y);
+      unsigned char *out = reinterpret_cast<unsigned char *>(a.out + base);
+      uint32_t at = 4 * off_g, r = grp;
+      tmem_wait_st();      // what this warp stored in the reduce visits
+      auto next = [&] { at += 4 * step_g; if constexpr (!FULL) r += g.groups; };
+      auto there = [&] { return alive && (FULL || r < rows); };
+      if constexpr (DIR == 0) {
+        uint32_t ae = smem_u32(sm) + g.off_slots + slot * g.slot_stride + off_s;
+        const Quad nmean = spread(-pA.x, -pB.x), beta = spread(pA.z, pB.z);
+        auto one = [&](const Quad &x) {
+          Quad o;
+          o.a = fma2(add2(x.a, nmean.a), scale.a, beta.a); o.b = fma2(add2(x.b, nmean.b), scale.b, beta.b);
+          if constexpr (EXTRA) { const Quad e = lds_quad(ae); o.a = add2(o.a, e.a); o.b = add2(o.b, e.b); ae += step_s; }
+          o.a = mul2(o.a, slopes(o.a, slope)); o.b = mul2(o.b, slopes(o.b, slope));
+          if (there()) stg_stream(reinterpret_cast<float *>(out + at), o);
+          next();
+        };
+        uint32_t i = 0;
+        for (; i + 4 <= g.vpt; i += 4, tm += 16) {
+          Quad x0, x1, x2, x3;
+          tmem_ld(tm, x0, x1, x2, x3);
+          one(x0); one(x1); one(x2); one(x3);
+          __syncwarp();
+        }
+        for (; i < g.vpt; ++i, tm += 4) {
+          Quad x0;
+          tmem_ld(tm, x0);
+          one(x0);
+          __syncwarp();
+        }
+      } else {
+        const Quad cB = spread(pA.w, pB.w), cC = spread(coef[2 * chA + 1].x, coef[2 * chB + 1].x);
+        const bool acc = a.accumulate != 0;
+        unsigned char *dres = EXTRA && a.dres ? reinterpret_cast<unsigned char *>(a.dres + base) : nullptr;
+        auto one = [&](const Quad &e, const Quad &z) {
+          Quad o;
+          o.a = fma2(scale.a, z.a, fma2(cB.a, e.a, cC.a)); o.b = fma2(scale.b, z.b, fma2(cB.b, e.b, cC.b));
+          if (there()) {
+            float *p = reinterpret_cast<float *>(out + at);
+            if (acc) { const Quad old = ldg_quad(p); o.a = add2(old.a, o.a); o.b = add2(old.b, o.b); }
+            stg_stream(p, o);
+            if constexpr (EXTRA) { if (dres) stg_stream(reinterpret_cast<float *>(dres + at), z); }
+          }
+          next();
+        };
+        uint32_t i = 0;
+        for (; i + 2 <= g.vpt; i += 2, tm += 16) {
+          Quad e0, z0, e1, z1;
+          tmem_ld(tm, e0, z0, e1, z1);
+          one(e0, z0); one(e1, z1);
+          __syncwarp();
+        }
+        if (i < g.vpt) {
+          Quad e0, z0;
+          tmem_ld(tm, e0, z0);
+          one(e0, z0);
+        }
+      }
+      __syncwarp();
+    };
+    BandWalk red(g, b, G), app(g, b, G);
+    uint32_t slot = g.slots - 1, par = 1, qres = 0, rpar = 1, qcoef = 0, cpar = 0;
+    uint32_t red_place = 0, app_place = 0;
+    for (uint32_t s = 0; s < steps; ++s) {
+      if (s < mine) {
+        if (++slot == g.slots) { slot = 0; par ^= 1u; }
+        bool ok = warp_wait(&ctl->res_empty[qres], rpar, ctl, status, ANODE_ST_WAIT_STATS);
+        ok = ok && warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS);
+        if (!ok) break;
+        float4 *part = reinterpret_cast<float4 *>(sm + g.off_res + qres * (kBandConsumers * 16 + 256));
+        const uint32_t rows = N - red.k * g.rows, tm = tm0 + red_place * tm_step;
+        if (rows >= g.rows) reduce(std::true_type{}, g.rows, slot, tm, part);
+        else reduce(std::false_type{}, rows, slot, tm, part);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ctl->res_full[qres]);
+        if (++qres == kBandQ) { qres = 0; rpar ^= 1u; }
+        if (++red_place > g.look) red_place = 0;
+        red.next();
+      }
+      if (s >= g.look) {
+        if (!warp_wait(&ctl->coef_full[qcoef], cpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
+        if constexpr (kSlotToo) {
+          if (++slot == g.slots) { slot = 0; par ^= 1u; }
+          if (!warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS)) break;
+        }
+        const uint32_t n0 = app.k * g.rows, c0 = app.unit * g.cb, rows = N - n0, tm = tm0 + app_place * tm_step;
+        const bool alive = live && 4 * v < (C - c0) * dim0;
+        const size_t base = (size_t)n0 * rs + (size_t)c0 * dim0;
+        const float4 *coef = reinterpret_cast<const float4 *>(sm + g.off_coef) + qcoef * 2 * kBandChannels;
+        if (rows >= g.rows) apply(std::true_type{}, g.rows, alive, base, slot, tm, coef);
+        else apply(std::false_type{}, rows, alive, base, slot, tm, coef);
+        if (lane == 0) { if (kSlotToo) mbar_arrive(&ctl->empty[slot]); mbar_arrive(&ctl->coef_empty[qcoef]); }
+        if (++qcoef == kBandQ) { qcoef = 0; cpar ^= 1u; }
+        if (++app_place > g.look) app_place = 0;
+        app.next();
+      }
+    }
+  } else if (warp == kBandWarps) {
+    // ------------------------------------------------------------------ producer
+    const uint64_t pol = policy_drop();
+    BandWalk red(g, b, G), app(g, b, G);
+    uint32_t slot = g.slots - 1, par = 1, k = 0;
+    bool ok = true;
+    // backward: lane l has the parameters of the next tile's channel number l
+    float4 raw = make_float4(0.f, 1.f, 1.f, 0.f);
+    auto params = [&](uint32_t unit) {
+      const uint32_t c = unit * g.cb + lane;
+      if (DIR == 1 && lane < g.cb && c < C) {
+        raw.x = a.mean_in[c]; raw.y = a.var_in[c];
+        raw.z = a.gamma ? a.gamma[c] : 1.0f; raw.w = a.gamma && a.beta ? a.beta[c] : 0.f;
+      }
+    };
+    if (mine) params(red.unit);
+    for (uint32_t t = 0; ok && t < 2 * steps; ++t) {
+      const uint32_t s = t >> 1, kind = t & 1u;
+      if (kind == 0 ? s >= mine : !kSlotToo || s < g.look) continue;
+      BandWalk &w = kind == 0 ? red : app;
+      ++k;
+      if (++slot == g.slots) { slot = 0; par ^= 1u; }
+      uint32_t okw = 1;
+      if (lane == 0) okw = mbar_wait(&ctl->empty[slot], par ^ 1u, ctl, status, ANODE_ST_WAIT_STATS) ? 1u : 0u;
+      ok = __shfl_sync(0xffffffffu, okw, 0) != 0;
+      if (!ok) { --k; break; }
+      const uint32_t planes = kind == 0 ? kPlanes : 1u;
+      if (lane == 0) mbar_expect_tx(&ctl->full[slot], planes * g.boxes * g.rows * g.box4 * 16);
+      __syncwarp();
+      if (lane < planes * g.boxes) {
+        const uint32_t plane = lane / g.boxes, j = lane - plane * g.boxes;
+        const CUtensorMap *map = kind == 1 || plane == 2 ? &maps.e : plane == 1 ? &maps.dy : &maps.x;
+        tensor_g2s(smem_u32(sm + g.off_slots + (size_t)slot * g.slot_stride) + plane * g.plane_bytes + j * g.box_bytes, map,
+                   w.unit * g.cb * dim0 + j * g.box4 * 4, w.k * g.rows, &ctl->full[slot], pol);
+      }
+      if (kind == 0 && DIR == 1) {
+        float4 *side = reinterpret_cast<float4 *>(sm + g.off_side) + slot * kBandChannels;
+        if (lane < g.cb) side[lane] = make_float4(raw.x, raw.z * inv_std(raw.y), raw.w, 0.f);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl->full[slot]);
+      w.next();
+      if (kind == 0 && DIR == 1 && s + 1 < mine) params(w.unit);
+    }
+    // after an abort: wait (bounded) for copies that were issued but will not be consumed
+    if (!ok && lane == 0) {
+      const uint32_t first = k > g.slots ? k - g.slots : 0;
+      for (uint32_t kk = first; kk < k; ++kk) {
+        const long long t0 = clock64();
+        while (!mbar_test(&ctl->full[kk % g.slots], (kk / g.slots) & 1u) && clock64() - t0 < kWaitCycles / 8) {}
+      }
+    }
+  } else if (warp == kBandWarps + 1) {
+    // ------------------------------------------------------------------ delivery warp
+    const uint32_t lp = 1u << g.lane_shift, ci = lane >> g.lane_shift, sub = lane & (lp - 1u);
+    const uint32_t v0 = ci * dim0 / 4, v1 = (ci * dim0 + dim0 - 1) / 4;      // the channel's first and last vector
+    unsigned long long *buf = reinterpret_cast<unsigned long long *>(a.ws + g.tag);
+    const size_t other = (size_t)g.total * g.cb;
+    unsigned long long *now = buf + (ctl->parity ? other : 0), *then = buf + (ctl->parity ? 0 : other);
+    BandWalk w(g, b, G);
+    uint32_t q = 0, qpar = 0;
+    size_t at = (size_t)b * g.cb + ci;
+    for (uint32_t j = 0; j < mine; ++j) {
+      const bool has = ci < g.cb && w.unit * g.cb + ci < C;
+      if (!warp_wait(&ctl->res_full[q], qpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
+      const float4 *part = reinterpret_cast<const float4 *>(sm + g.off_res + q * (kBandConsumers * 16 + 256));
+      double t1 = 0.0, t2 = 0.0;
+      float K = 0.f;
+      if (DIR == 0 && has) K = reinterpret_cast<const float *>(part + kBandConsumers)[ci];
+      // four of the lane's vectors at a time, their sums added in pairs: the loads are under way together and a quarter of the
+      // additions are in double precision (one vector after another in double precision: 2.5 us a tile, the kernel's bound)
+      uint32_t vi = v0 + sub, gi = has && vi <= v1 ? 0 : g.groups;
+      while (gi < g.groups) {
+        float2 p[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          p[u] = make_float2(0.f, 0.f);
+          if (gi < g.groups) {
+            // (a vector that begins in the channel before holds this one's sums behind those)
+            p[u] = reinterpret_cast<const float2 *>(part + gi * g.L4 + vi)[4 * vi >= ci * dim0 ? 0 : 1];
+            vi += lp;
+            if (vi > v1) { vi = v0 + sub; ++gi; }
+          }
+        }
+        t1 += (double)((p[0].x + p[1].x) + (p[2].x + p[3].x)); t2 += (double)((p[0].y + p[1].y) + (p[2].y + p[3].y));
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl->res_empty[q]);
+      if (++q == kBandQ) { q = 0; qpar ^= 1u; }
+      for (uint32_t o = lp >> 1; o > 0; o >>= 1) { t1 += __shfl_xor_sync(0xffffffffu, t1, o); t2 += __shfl_xor_sync(0xffffffffu, t2, o); }
+      if (has && sub == 0) {
+        float lo = (float)t1, hi = (float)t2;
+        if (DIR == 0) {
+          const double m = t1 * (w.k + 1 == g.tiles ? g.inv_tail : g.inv_full);
+          lo = (float)((double)K + m); hi = (float)not_below_zero(t2 - t1 * m);
+        }
+        st_relaxed_gpu_u64(now + at, band_word(lo, hi));
+        then[at] = 0ull;
+      }
+      at += (size_t)G * g.cb;
+      w.next();
+    }
+  } else {
+    // ------------------------------------------------------------------ coefficient warp
+    const uint32_t lp = 1u << g.lane_shift, ci = lane >> g.lane_shift, sub = lane & (lp - 1u);
+    const unsigned long long *buf = reinterpret_cast<const unsigned long long *>(a.ws + g.tag) + (ctl->parity ? (size_t)g.total * g.cb : 0);
+    const double n_full = (double)g.rows * dim0, n_tail = (double)(N - (g.tiles - 1) * g.rows) * dim0;
+    BandWalk w(g, b, G);
+    uint32_t q = 0, qpar = 1;
+    float gm = 1.f, bt = 0.f, mean = 0.f, var = 1.f;
+    auto params = [&](uint32_t unit) {
+      const uint32_t c = unit * g.cb + ci;
+      if (ci < g.cb && c < C) {
+        gm = a.gamma ? a.gamma[c] : 1.0f; bt = a.gamma && a.beta ? a.beta[c] : 0.f;
+        if (DIR == 1) { mean = a.mean_in[c]; var = a.var_in[c]; }
+      }
+    };
+    if (mine) params(w.unit);
+    bool ok = true;
+    for (uint32_t n = 0; ok && n < mine; ++n) {
+      const uint32_t c = w.unit * g.cb + ci;
+      const bool has = ci < g.cb && c < C;
+      const unsigned long long *words = buf + (size_t)w.unit * g.tiles * g.cb + ci;
+      double s1 = 0.0, s2 = 0.0, K = 0.0;
+      const long long t0 = clock64();
+      constexpr int kPull = 8;
+      for (uint32_t k0 = 0; ok && k0 < g.tiles; k0 += kPull * lp) {
+        unsigned long long r[kPull];
+        for (;;) {
+          bool all = true;
+#pragma unroll
+          for (int i = 0; i < kPull; ++i) {
+            const uint32_t k = k0 + sub + i * lp;
+            r[i] = has && k < g.tiles ? ld_relaxed_gpu_u64(words + (size_t)k * g.cb) : 1ull;
+            all = all && r[i] != 0ull;
+          }
+          if (__all_sync(0xffffffffu, all)) break;
+          __nanosleep(100);
+          uint32_t stop = 0;
+          if (lane == 0) {
+            if (ctl->abort) stop = 1;
+            else if (clock64() - t0 > kWaitCycles) { atomicOr(status, ANODE_ST_WAIT_STATS); ctl->abort = 1; stop = 1; }
+          }
+          if (__shfl_sync(0xffffffffu, stop, 0)) { ok = false; break; }
+        }
+        if (!ok) break;
+        if (DIR == 0 && k0 == 0) {      // shift: the mean of the first tile (an infinity or a NaN is none, the sums show it)
+          const float first = __shfl_sync(0xffffffffu, __uint_as_float((uint32_t)r[0]), ci << g.lane_shift);
+          K = fabsf(first) < 1e36f ? (double)first : 0.0;
+        }
+#pragma unroll
+        for (int i = 0; i < kPull; ++i) {
+          const uint32_t k = k0 + sub + i * lp;
+          if (k < g.tiles) {
+            const double lo = (double)__uint_as_float((uint32_t)r[i]), hi = (double)__uint_as_float((uint32_t)(r[i] >> 32));
+            if (DIR == 0) {
+              const double cnt = k + 1 == g.tiles ? n_tail : n_full, d = lo - K;
+              s1 = fma(cnt, d, s1); s2 += fma(cnt * d, d, hi);
+            } else { s1 += lo; s2 += hi; }
+          }
+        }
+      }
+      if (!ok) break;
+      for (uint32_t o = lp >> 1; o > 0; o >>= 1) { s1 += __shfl_xor_sync(0xffffffffu, s1, o); s2 += __shfl_xor_sync(0xffffffffu, s2, o); }
+      if (!warp_wait(&ctl->coef_empty[q], qpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
+      float4 *coef = reinterpret_cast<float4 *>(sm + g.off_coef) + q * 2 * kBandChannels + 2 * ci;
+      const bool owner = w.k == 0;
+      if (has && sub == 0) {
+        if (DIR == 0) {
+          const double m = s1 * g.inv_count;
+          const float mf = (float)(K + m);
+          const float vf = (float)(not_below_zero(s2 - s1 * m) * g.inv_count + (double)a.epsilon);      // biased, epsilon folded in (batch_norm.cu:160)
+          coef[0] = make_float4(mf, gm * inv_std(vf), bt, 0.f);
+          if (owner) {
+            a.mean[c] = mf; a.var[c] = vf;
+            if (a.run_mean) { const float o = a.run_mean[c]; a.run_mean[c] = o + a.avg_rate * (mf - o); }
+            if (a.run_var) { const float o = a.run_var[c]; a.run_var[c] = o + a.avg_rate * (vf - o); }
+          }
+        } else {
+          const float rstd = inv_std(var);
+          const double rs2 = (double)rstd * s2;                  // sum(dz * xhat)
+          const double A = (double)gm * (double)rstd;
+          coef[0] = make_float4(mean, gm * rstd, bt, (float)(-A * (double)rstd * rs2 * g.inv_count));
+          coef[1] = make_float4((float)(-A * s1 * g.inv_count), 0.f, 0.f, 0.f);
+          if (owner) {
+            if (a.dbeta) a.dbeta[c] = (float)s1;
+            if (a.dgamma) a.dgamma[c] = (float)rs2;
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl->coef_full[q]);
+      if (++q == kBandQ) { q = 0; qpar ^= 1u; }
+      w.next();
+      if (n + 1 < mine) params(w.unit);
+    }
+  }
+
+  // ---- leave
+  if (warp < kBandWarps) { __syncwarp(); tmem_wait_st(); }
+  tmem_fence_before();
+  __syncthreads();
+  if (warp == 0) { tmem_fence_after(); tmem_free(ctl->tmem); }
+  if (ctl->abort) {
+    if (tid == 0) atomicOr(status, ANODE_ST_ABORTED);
+    return;
+  }
+  if (tid == 0) {
+    __threadfence();
+    if (atomicAdd(exit_ctr, 1u) + 1 == gridDim.x) { *parity = ctl->parity ^ 1u; *exit_ctr = 0; }
+  }
+}
+
+// ---- host side -------------------------------------------------------------------------------
+
+typedef CUresult (*EncodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static EncodeTiled encode_tiled()
+{
+  static const EncodeTiled f = [] {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult r;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &r) != cudaSuccess || r != cudaDriverEntryPointSuccess) {
+      (void)cudaGetLastError();
+      p = nullptr;
+    }
+    return (EncodeTiled)p;
+  }();
+  return f;
+}
+
+static bool tensor_map(CUtensorMap &m, const float *p, uint32_t width, uint32_t N, uint32_t box, uint32_t rows)
+{
+  const cuuint64_t dims[2] = {width, N}, strides[1] = {4ull * width};
+  const cuuint32_t boxes[2] = {box, rows}, one[2] = {1, 1};
+  return encode_tiled()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(p), dims, strides, boxes, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Where the streaming kernel hands a layer over: rows below those that the tiled kernel takes (tiled_takes), from so many elements
+// on.  Below, the fill and the drain of the schedule, some 10 us, outweigh the second walk it saves.  Streaming kernel and this
+// one, us:
+//   forward    6.4 M [64,2048,7,7] 17.7 and 21.4, 8.4 M [512,256,8,8] 17.8 and 21.4, 12.8 M [128,2048,7,7] 24.8 and 24.9,
+//              16.8 M [512,128,16,16] 34.3 and 31.6, 25.7 M [256,2048,7,7] 56.6 and 47.5
+//   backward   4.8 M [100,400,11,11] 16.7 and 19.8, 6.4 M [64,2048,7,7] 26.3 and 22.5, [128,256,14,14] 24.8 and 25.4, 8.4 M [512,256,8,8]
+//              31.5 and 24.5, 12.8 M 45.4 and 32.8
+//   residual   6.4 M 24.5 / 33.2 and 22.7 / 28.8 ([64,2048,7,7]), 22.1 / 32.0 and 24.4 / 32.7 ([128,256,14,14]), 8.4 M 23.6 / 39.2 and
+//              23.9 / 33.8, 12.8 M 36.6 / 58.6 and 30.1 / 45.7
+constexpr uint32_t kBandLongRow = 320;
+constexpr uint64_t kBandLeast[2][2] = {{15000000, 9000000}, {8000000, 8000000}};      // [direction][residual]
+
+bool band_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, BandGeom &g)
+{
+  if ((uint64_t)dim0 * C * N < kBandLeast[dir][extra] || dim0 >= kBandLongRow) return false;
+  return band_geom(dim0, C, N, dir, extra, sm_count(), g);
+}
+
+int launch_band(FusedArgs &a, const BandGeom &g, int dir, cudaStream_t stream)
+{
+  const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
+  if (!encode_tiled()) return ANODE_E_LAUNCH;
+  BandMaps m;
+  const uint32_t width = a.plan.C * a.plan.dim0;
+  if (!tensor_map(m.x, a.x, width, a.plan.N, g.box4 * 4, g.rows)) return ANODE_E_LAUNCH;
+  m.dy = m.x; m.e = m.x;
+  if (dir == 1 && !tensor_map(m.dy, a.dy, width, a.plan.N, g.box4 * 4, g.rows)) return ANODE_E_LAUNCH;
+  if (extra && !tensor_map(m.e, dir == 0 ? a.res : a.ymask, width, a.plan.N, g.box4 * 4, g.rows)) return ANODE_E_LAUNCH;
+  const void *k = dir == 0 ? (extra ? (const void *)bn_band_kernel<0, true> : (const void *)bn_band_kernel<0, false>)
+                           : (extra ? (const void *)bn_band_kernel<1, true> : (const void *)bn_band_kernel<1, false>);
+  static std::mutex mu;
+  static std::map<std::pair<const void *, int>, bool> ready;
+  {
+    int dev = 0;
+    (void)cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    const auto key = std::make_pair(k, dev);
+    auto it = ready.find(key);
+    if (it == ready.end()) {
+      const bool ok = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBandSmem) == cudaSuccess;
+      if (!ok) (void)cudaGetLastError();
+      it = ready.emplace(key, ok).first;
+    }
+    if (!it->second) return ANODE_E_LAUNCH;
+  }
+  BandGeom gg = g;
+  void *params[] = {(void *)&a, (void *)&gg, (void *)&m};
+  if (cudaLaunchCooperativeKernel(k, dim3(g.grid), dim3(kBandThreads), params, kBandSmem, stream) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return ANODE_E_LAUNCH;
+  }
+  return ANODE_OK;
+}
+
+}  // namespace anode_b200

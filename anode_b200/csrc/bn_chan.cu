@@ -296,6 +296,12 @@ bool chan_applies(const FusedArgs &a, int dir, bool aligned)
 // 85 / 77 / 117 and 77 / 77 / 117, and of 25 K floats 484 77 / 70 / 105 and 68 / 63 / 96.
 constexpr uint32_t kChanTiledRow = 480;
 constexpr uint64_t kChanTiled = 16u << 20, kChanTiledExtra = 18u << 20, kChanTiledChannel = 24u << 10;
+// Aligned rows below 320 floats go to the band kernel (the streaming kernel's form for large layers) from these sizes on.  Us here
+// and there, forward: [100,1024,16,16] 26 M 45 and 49, [180,1024,14,14] 36 M 66.4 and 65.7, [256,1024,14,14] 98 and 88, [2000,2048,4,4] 115
+// and 91; backward: [50,2048,12,12] 15 M 36.4 and 38.4, [100,1024,14,14] 20 M 55 and 47, [256,1024,14,14] 163 and 104; residual forward
+// 20 M 50 and 53, [200,2048,8,8] 26 M 63 and 58; residual backward 15 M 52 and 53, 20 M 77 and 68.
+constexpr uint32_t kChanBandRow = 320;
+constexpr uint64_t kChanBand[2][2] = {{40000000, 24000000}, {18000000, 18000000}};      // [direction][residual]
 constexpr uint64_t kChanLarge = 8u << 20, kChanLargeScalar = 3u << 20, kChanLargeExtra = 5u << 20;
 constexpr uint64_t kChanWaves = 1500000, kChanShortest = 1200000;
 constexpr uint32_t kChanFewSamples = 32;
@@ -308,9 +314,12 @@ bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
   if (!chan_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, extra, aligned, g)) return false;
   const uint64_t channel = (uint64_t)a.plan.dim0 * a.plan.N, elements = channel * a.plan.C;
   const uint32_t most = dir == 0 && !extra ? 32u : 16u;
+  BandGeom band;
   if (g.vec == 4) {
     if (tiled_ok && (dir == 1 || extra) && a.plan.dim0 >= kChanTiledRow && channel >= kChanTiledChannel &&
         elements >= (extra ? kChanTiledExtra : kChanTiled) && tiled_takes(a.plan.dim0, elements, dir, extra)) return false;
+    if (a.plan.dim0 < kChanBandRow && elements >= kChanBand[dir][extra] && band_geom_of(a, dir, band) &&
+        stream_preferred(a, dir, aligned, tiled_ok)) return false;
     if (elements < kChanLarge || channel <= (uint64_t)kChanThreads * kChanCluster * most / 2) return true;
     return !stream_preferred(a, dir, aligned, tiled_ok) &&
            !(tiled_ok && ((dir == 0 && !extra) || tiled_takes(a.plan.dim0, elements, dir, extra)));

@@ -22,7 +22,7 @@ namespace anode_b200 {
 // 63 x 63 43 / 62 (113 / 155).
 constexpr uint32_t kRaggedMinRow[2] = {112, 160};
 // Workspace header: (exit counter, parity) of the tiled kernel's plans (words 3 and 4 are the slice-resident kernel's)
-constexpr uint32_t kRingHdr = 4, kRingHdrRagged = 32, kRingHdrExtra = 40;
+constexpr uint32_t kRingHdr = 4, kRingHdrRagged = 32, kRingHdrExtra = 40, kBandHdr = 48, kBandHdrExtra = 56;
 
 // ---- planner constants, from sweeps on B200 -------------------------------------------------------
 #ifndef ANODE_SLACK_STEPS
@@ -89,6 +89,8 @@ struct ShapeInfo {
   Plan ring_plan[2][2];
   RingGeom ring_geom[2][2];
   uint64_t tiled_bytes, static_bytes, part_bytes;      // see fill_shape_info
+  bool band_ok[2][2];            // the streaming kernel's form for the largest layers, likewise
+  BandGeom band[2][2];
 };
 constexpr uint32_t kShapeCache = 64;      // entries per thread, direct mapped
 
@@ -437,6 +439,27 @@ static void fill_shape_info(ShapeInfo &s)
       s.ring_geom[dir][ex].hdr = ex ? kRingHdrExtra : kRingHdrRagged;
       if (end > s.part_bytes) s.part_bytes = end;
     }
+  // so does the band kernel
+  for (int dir = 0; dir < 2; ++dir)
+    for (int ex = 0; ex < 2; ++ex) {
+      BandGeom &g = s.band[dir][ex];
+      s.band_ok[dir][ex] = band_plan(s.dim0, s.C, s.N, dir, ex != 0, g);
+      if (!s.band_ok[dir][ex]) continue;
+      g.hdr = ex ? kBandHdrExtra : kBandHdr;
+      const uint64_t end = align_up_u64(s.part_bytes + band_words(g) * 16ull, 256);
+      if (end > 0xffffffffull) { s.band_ok[dir][ex] = false; continue; }
+      g.tag = (uint32_t)s.part_bytes;
+      s.part_bytes = end;
+    }
+}
+
+bool band_geom_of(const FusedArgs &a, int dir, BandGeom &g)
+{
+  const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
+  const ShapeInfo &s = shape_info(a.plan.dim0, a.plan.C, a.plan.N);
+  if (!s.band_ok[dir][extra]) return false;
+  g = s.band[dir][extra];
+  return a.bands && a.ws_capacity >= g.tag + 16ull * band_words(g);
 }
 
 // Bytes of a part taken by the tile-plan kernels (plain, warp-specialised, cluster); the records of the
@@ -509,6 +532,8 @@ int launch_best(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)
   int kind = pick_kernel_kind(a, dir, aligned);
   if (kind == ANODE_KERNEL_REGISTER) return launch_chan(a, dir, aligned, stream);
   if (kind == ANODE_KERNEL_STREAM) {
+    BandGeom bg;
+    if (band_geom_of(a, dir, bg) && launch_band(a, bg, dir, stream) == ANODE_OK) return ANODE_OK;
     if (launch_stream(a, dir, stream) == ANODE_OK) return ANODE_OK;
     kind = segres_applies(a, dir, aligned) ? ANODE_KERNEL_CLUSTER : ANODE_KERNEL_PLAIN;
   }
@@ -609,6 +634,7 @@ int prepare_fwd(FusedArgs &a, uint32_t dim0, uint32_t dim1, uint32_t dim2, float
   a.mode = MODE_FUSED;
   a.count_total = (double)dim0 * (double)dim2;
   a.wait_cycles = wait_limit_cycles();
+  a.bands = 1u;
   return ANODE_OK;
 }
 
@@ -634,6 +660,7 @@ int prepare_bwd(FusedArgs &a, uint32_t dim0, uint32_t dim1, uint32_t dim2, int r
   a.mode = MODE_FUSED;
   a.count_total = (double)dim0 * (double)dim2;
   a.wait_cycles = wait_limit_cycles();
+  a.bands = 1u;
   return ANODE_OK;
 }
 
@@ -800,6 +827,7 @@ static FusedArgs probe_call(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool
   a.mode = MODE_FUSED;
   a.world = world > 1 ? (uint32_t)world : 0u;
   a.ws_capacity = workspace_part_bytes(dim0, C, N);
+  a.bands = 1u;
   if (residual) (dir == 0 ? a.res : a.ymask) = &dummy;       // only their presence matters here
   return a;
 }
@@ -889,6 +917,20 @@ extern "C" uint32_t anode_gpu_batch_norm_tiled_last_piece(uint32_t dim0, uint32_
   Plan p; RingGeom g;
   if ((dir != 0 && dir != 1) || check_dims(dim0, dim1, dim2) || !ring_plan_for(dim0, dim1, dim2, true, dir, residual != 0, p, g)) return 0;
   return dim0 - (p.pieces - 1) * p.piece_len;
+}
+
+// ---- diagnostics: geometry of the band kernel (no GPU needed) --------------------------------------
+extern "C" int anode_gpu_batch_norm_band_geometry(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual, uint32_t *out)
+{
+  using namespace anode_b200;
+  if (!out || (dir != 0 && dir != 1) || check_dims(dim0, dim1, dim2)) return ANODE_E_DIMS;
+  BandGeom g{};
+  const bool taken = band_geom_of(probe_call(dim0, dim1, dim2, dir, residual != 0, true, 1), dir, g);
+  if (!taken && !band_geom(dim0, dim1, dim2, dir, residual != 0, sm_count(), g)) g = BandGeom{};
+  const uint32_t v[16] = {taken ? 1u : 0u, g.cb, g.units, g.groups, g.vpt, g.rows, g.tiles, g.grid, g.look, g.boxes, g.box4, g.box_bytes,
+                          g.slots, g.slot_stride, g.smem_bytes, g.lane_shift};
+  for (int i = 0; i < 16; ++i) out[i] = v[i];
+  return ANODE_OK;
 }
 
 // ---- diagnostics: the tile plan, for tests of the index arithmetic (no GPU needed) ----------

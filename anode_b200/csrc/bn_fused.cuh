@@ -46,6 +46,7 @@ struct FusedArgs {
   float epsilon, avg_rate;
   uint32_t relu, accumulate, mode;
   float neg_slope;         // activation t*(t > 0 ? 1 : neg_slope): 0 = ReLU, 1 = none, c = leaky ReLU (flat_map.cu:44-52)
+  uint32_t bands;          // the workspace holds the band kernel's words (a caller's own one, of the full size)
   uint32_t use_rec;        // publish tagged records (the warp-specialised kernel reads them)
   double count_total;      // elements per channel over all participating GPUs
   // cross-GPU exchange inside the kernel (world > 1): xchg[r] is rank r's exchange buffer as

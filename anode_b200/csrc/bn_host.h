@@ -11,6 +11,7 @@
 #include <utility>
 
 #include "../../include/anode_routines_gpu.h"
+#include "bn_band.cuh"
 #include "bn_fused.cuh"
 
 namespace anode_b200 {
@@ -60,6 +61,10 @@ bool stream_applies(const FusedArgs &a, int dir, bool aligned);
 uint32_t stream_cluster(const FusedArgs &a, int dir, bool aligned);
 bool stream_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok);
 int launch_stream(FusedArgs &a, int dir, cudaStream_t stream);
+// its form for the largest of them (bn_band.cu): the geometry of a shape where it is taken, and of a prepared call
+bool band_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, BandGeom &g);
+bool band_geom_of(const FusedArgs &a, int dir, BandGeom &g);
+int launch_band(FusedArgs &a, const BandGeom &g, int dir, cudaStream_t stream);
 uint64_t workspace_part_bytes(uint32_t dim0, uint32_t C, uint32_t N);
 uint64_t workspace_static_bytes(uint32_t dim0, uint32_t C, uint32_t N);
 uint64_t ring_ws_bytes(const FusedArgs &a, int dir, bool aligned);

@@ -38,12 +38,10 @@
 // ANODE_RING_NS naming the namespace of the instantiation and ANODE_RING_CONSUMERS the number of
 // consumer threads (the forward pass runs best with 8 consumer warps, the backward pass with 16).
 #include "bn_fused.cuh"
+#include "bn_pipe.cuh"
 
 #if !defined(ANODE_RING_NS) || !defined(ANODE_RING_CONSUMERS)
 #error "define ANODE_RING_NS and ANODE_RING_CONSUMERS before including bn_ring.cuh"
-#endif
-#ifndef ANODE_RING_BACKOFF_NS
-#define ANODE_RING_BACKOFF_NS 100
 #endif
 
 namespace anode_b200 {
@@ -51,7 +49,6 @@ namespace ANODE_RING_NS {
 
 constexpr uint32_t kConsumers = ANODE_RING_CONSUMERS;   // consumer threads (a power of two, 256..1024)
 constexpr uint32_t kRingThreads = kConsumers + 96;   // + producer, delivery and coefficient warps
-constexpr long long kWaitCycles = 3000000000ll;      // about 1.5 s at 2 GHz
 
 struct RingCtl {
   unsigned long long full[kMaxSlots], empty[kMaxSlots];
@@ -64,94 +61,11 @@ struct RingCtl {
 };
 static_assert(sizeof(RingCtl) <= kRingCtlBytes, "RingCtl outgrew the room reserved for it");
 
-// ---- mbarrier / bulk-copy primitives --------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(unsigned long long *bar, uint32_t count)
-{
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(unsigned long long *bar)
-{
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, uint32_t bytes)
-{
-  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_test(unsigned long long *bar, uint32_t parity)
-{
-  uint32_t ok;
-  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-               : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool mbar_try(unsigned long long *bar, uint32_t parity)
-{
-  uint32_t ok;
-  // the last operand lets the hardware keep the thread suspended (up to that many nanoseconds)
-  // until the phase completes, instead of returning early to a polling loop
-  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-               : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"(100000u) : "memory");
-  return ok != 0;
-}
-// Bounded wait.  Returns false (after raising the abort flag) when the barrier did not flip in time
-// or when another role already gave up.
-__device__ __forceinline__ bool mbar_wait(unsigned long long *bar, uint32_t parity, RingCtl *ctl, uint32_t *status, uint32_t bit)
-{
-  if (mbar_try(bar, parity)) return true;
-  const long long t0 = clock64();
-  uint32_t it = 0;
-  for (;;) {
-    if (mbar_try(bar, parity)) return true;
-    // back off: a spinning waiter takes issue slots from the warps that do the work
-    __nanosleep(ANODE_RING_BACKOFF_NS);
-    if ((++it & 15u) == 0u) {
-      if (ctl->abort) return false;
-      if (clock64() - t0 > kWaitCycles) {
-        atomicOr(status, bit);
-        ctl->abort = 1;
-        return false;
-      }
-    }
-  }
-}
-// Every lane gets the same answer.  The common case, a phase that is already complete (or completes while the
-// hardware holds the warp), is one instruction for the whole warp; only a wait that outlasts that is handed to
-// one lane, which polls with the time limit.
-__device__ __forceinline__ bool warp_wait(unsigned long long *bar, uint32_t parity, RingCtl *ctl, uint32_t *status, uint32_t bit)
-{
-  if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
-  uint32_t ok = 1;
-  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, ctl, status, bit) ? 1u : 0u;
-  return __shfl_sync(0xffffffffu, ok, 0) != 0;
-}
-// global -> shared bulk copy, completion counted on `bar`; bytes and both addresses are multiples of 16
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, unsigned long long *bar, uint64_t policy)
-{
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
-               ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy) : "memory");
-}
 // ---- tensor memory as a store for tiles ---------------------------------------------------------
 // The SM's 256 KB of tensor memory hold what the reduce visits of `keep_slots` out of every keep_period tiles have read
 // (forward: x; backward: x - mean and dz), so that their apply visits need neither L2 nor a slot of the ring.  A warp
 // reaches the 32 lanes of its place in its group of four warps; the groups divide the 512 columns among them.
 // Every instruction here is the whole warp's.
-constexpr uint32_t kTmemCols = 512;
-__device__ __forceinline__ void tmem_alloc(uint32_t *dst)
-{
-  // never waits: the launch takes the SM's whole shared memory, so that no other block holds columns (launch_ring)
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst)), "n"(kTmemCols) : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_free(uint32_t base)
-{
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "n"(kTmemCols) : "memory");
-}
-__device__ __forceinline__ void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
 // ---- the block's schedule --------------------------------------------------------------------
 // The visits of a block: steps s = 0, 1, ...; at step s first REDUCE its tile number s (if any is left), then APPLY number
 // s - look (if s >= look).  Tile number n of the block is tile b + n*G.  Every role walks this same sequence by itself.
@@ -195,78 +109,6 @@ __device__ __forceinline__ float4 *coef_box(unsigned char *sm, const RingGeom &g
 constexpr uint32_t kCWarps = kConsumers / 32;
 constexpr uint32_t kVecStride = kConsumers * 16;     // bytes between consecutive vectors of one thread
 
-// ---- pairs of floats: one instruction for two, each rounded as its scalar form
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pair(float lo, float hi) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi)); return r; }
-__device__ __forceinline__ f32x2 pair(float v) { return pair(v, v); }
-__device__ __forceinline__ float2 split(f32x2 v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
-__device__ __forceinline__ f32x2 slopes(f32x2 y, float slope)      // act'(y)
-{
-  const float2 t = split(y);
-  return pair(t.x > 0.0f ? 1.0f : slope, t.y > 0.0f ? 1.0f : slope);
-}
-struct Quad { f32x2 a, b; };     // a 16-byte vector
-__device__ __forceinline__ Quad quad(float v) { const f32x2 p = pair(v); return Quad{p, p}; }
-__device__ __forceinline__ float4 floats(const Quad &q) { const float2 a = split(q.a), b = split(q.b); return make_float4(a.x, a.y, b.x, b.y); }
-__device__ __forceinline__ Quad lds_quad(uint32_t saddr)
-{
-  Quad r;
-  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(r.a), "=l"(r.b) : "r"(saddr) : "memory");
-  return r;
-}
-__device__ __forceinline__ Quad ldg_quad(const float *p)
-{
-  Quad r;
-  asm volatile("ld.global.v2.b64 {%0, %1}, [%2];" : "=l"(r.a), "=l"(r.b) : "l"(p) : "memory");
-  return r;
-}
-__device__ __forceinline__ void stg_quad(float *p, const Quad &q) { asm volatile("st.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(q.a), "l"(q.b) : "memory"); }
-__device__ __forceinline__ void stg_stream(float *p, const Quad &q) { asm volatile("st.global.cs.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(q.a), "l"(q.b) : "memory"); }
-
-// ---- tensor memory, a vector per thread and four columns (the whole warp)
-#define ANODE_T16 "{t0, t1, t2, t3, t4, t5, t6, t7, t8, t9, t10, t11, t12, t13, t14, t15}"
-__device__ __forceinline__ void tmem_st(uint32_t at, const Quad &a)
-{
-  asm volatile("{\n\t.reg .b32 t<4>;\n\tmov.b64 {t0, t1}, %1;\n\tmov.b64 {t2, t3}, %2;\n\t"
-               "tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {t0, t1, t2, t3};\n\t}" ::"r"(at), "l"(a.a), "l"(a.b) : "memory");
-}
-__device__ __forceinline__ void tmem_st(uint32_t at, const Quad &a, const Quad &b)
-{
-  asm volatile("{\n\t.reg .b32 t<8>;\n\tmov.b64 {t0, t1}, %1;\n\tmov.b64 {t2, t3}, %2;\n\tmov.b64 {t4, t5}, %3;\n\tmov.b64 {t6, t7}, %4;\n\t"
-               "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {t0, t1, t2, t3, t4, t5, t6, t7};\n\t}"
-               ::"r"(at), "l"(a.a), "l"(a.b), "l"(b.a), "l"(b.b) : "memory");
-}
-__device__ __forceinline__ void tmem_st(uint32_t at, const Quad &a, const Quad &b, const Quad &c, const Quad &d)
-{
-  asm volatile("{\n\t.reg .b32 t<16>;\n\tmov.b64 {t0, t1}, %1;\n\tmov.b64 {t2, t3}, %2;\n\tmov.b64 {t4, t5}, %3;\n\tmov.b64 {t6, t7}, %4;\n\t"
-               "mov.b64 {t8, t9}, %5;\n\tmov.b64 {t10, t11}, %6;\n\tmov.b64 {t12, t13}, %7;\n\tmov.b64 {t14, t15}, %8;\n\t"
-               "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], " ANODE_T16 ";\n\t}"
-               ::"r"(at), "l"(a.a), "l"(a.b), "l"(b.a), "l"(b.b), "l"(c.a), "l"(c.b), "l"(d.a), "l"(d.b) : "memory");
-}
-// (the wait stands in the same statement as the load, so that nothing can use a register before it has arrived)
-__device__ __forceinline__ void tmem_ld(uint32_t at, Quad &a)
-{
-  asm volatile("{\n\t.reg .b32 t<4>;\n\ttcgen05.ld.sync.aligned.32x32b.x4.b32 {t0, t1, t2, t3}, [%2];\n\ttcgen05.wait::ld.sync.aligned;\n\t"
-               "mov.b64 %0, {t0, t1};\n\tmov.b64 %1, {t2, t3};\n\t}" : "=l"(a.a), "=l"(a.b) : "r"(at) : "memory");
-}
-__device__ __forceinline__ void tmem_ld(uint32_t at, Quad &a, Quad &b)
-{
-  asm volatile("{\n\t.reg .b32 t<8>;\n\ttcgen05.ld.sync.aligned.32x32b.x8.b32 {t0, t1, t2, t3, t4, t5, t6, t7}, [%4];\n\ttcgen05.wait::ld.sync.aligned;\n\t"
-               "mov.b64 %0, {t0, t1};\n\tmov.b64 %1, {t2, t3};\n\tmov.b64 %2, {t4, t5};\n\tmov.b64 %3, {t6, t7};\n\t}"
-               : "=l"(a.a), "=l"(a.b), "=l"(b.a), "=l"(b.b) : "r"(at) : "memory");
-}
-__device__ __forceinline__ void tmem_ld(uint32_t at, Quad &a, Quad &b, Quad &c, Quad &d)
-{
-  asm volatile("{\n\t.reg .b32 t<16>;\n\ttcgen05.ld.sync.aligned.32x32b.x16.b32 " ANODE_T16 ", [%8];\n\ttcgen05.wait::ld.sync.aligned;\n\t"
-               "mov.b64 %0, {t0, t1};\n\tmov.b64 %1, {t2, t3};\n\tmov.b64 %2, {t4, t5};\n\tmov.b64 %3, {t6, t7};\n\t"
-               "mov.b64 %4, {t8, t9};\n\tmov.b64 %5, {t10, t11};\n\tmov.b64 %6, {t12, t13};\n\tmov.b64 %7, {t14, t15};\n\t}"
-               : "=l"(a.a), "=l"(a.b), "=l"(b.a), "=l"(b.b), "=l"(c.a), "=l"(c.b), "=l"(d.a), "=l"(d.b) : "r"(at) : "memory");
-}
-#undef ANODE_T16
-
 // Shift of the sums: the median of three elements.  A single one is no shift to rely on: the first of an image is the corner
 // that a zero-padded convolution makes, and far from the mean it costs the variance its digits.  Relative error of the
 // variance with the first element of each row at 100 standard deviations, that element and the median as the shift:
@@ -274,7 +116,6 @@ __device__ __forceinline__ void tmem_ld(uint32_t at, Quad &a, Quad &b, Quad &c, 
 // vector, ragged ones from the tile's beginning, middle and end.  (Aligned rows with the latter, the residual epilogue's
 // forward pass on [256,256,56,56]: 522 -> 560 us, although each warp does less; with the former 526.  A mean of the warp's
 // first vectors: 542 - 570.)
-__device__ __forceinline__ float median3(float a, float b, float c) { return fmaxf(fminf(a, b), fminf(fmaxf(a, b), c)); }
 
 // Backward pass of the residual epilogue: dres = dz leaves during the reduce visit and the apply visit reads it back
 // (from L2) in the place of dy and the saved output, unless there is no dres or it is x itself (FusedArgs::dres_early).
@@ -681,16 +522,6 @@ __device__ __forceinline__ void warp_finish_unit_R(const FusedArgs &a, uint32_t 
 __device__ __forceinline__ unsigned long long *tag_buf(const FusedArgs &a, uint32_t parity)
 {
   return reinterpret_cast<unsigned long long *>(a.ws + a.plan.off_tag) + (size_t)parity * a.plan.total_tiles * a.plan.cb;
-}
-__device__ __forceinline__ unsigned long long ld_relaxed_gpu_u64(const unsigned long long *p)
-{
-  unsigned long long v;
-  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_relaxed_gpu_u64(unsigned long long *p, unsigned long long v)
-{
-  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 __device__ __forceinline__ unsigned long long ld_relaxed_sys_u64(const unsigned long long *p)
 {

@@ -88,6 +88,7 @@ extern "C" int anode_gpu_batch_norm_relu_fused_fwd_static_3d1_packed_f32(
                              run_mean, run_var, scratch, (size_t)workspace_part_bytes(dim0, dim1, dim2));
   if (rc) return rc;
   const bool aligned = aligned16(x) && aligned16(y);
+  a.bands = 0;      // the array has no words that stay zero between calls
   if (a.ws_capacity > ANODE_STATIC_SCRATCH_BYTES) a.ws_capacity = ANODE_STATIC_SCRATCH_BYTES;
   uint64_t need = 0, clear = 0;
   static_need(a, aligned, need, clear);

@@ -11,6 +11,8 @@
 //      that one is still in registers, the others come from L2.  The cluster size keeps what all resident blocks have
 //      between their two walks within reach of L2 (kStreamWindow).
 //
+// (The largest of these layers are walked once, by bn_band.cu, where the call has a workspace.)
+//
 // What bounds it: HBM and the loads in flight.  Nothing is staged in shared memory, so the blocks per SM are limited by
 // registers only and some stream while others fold and wait; the kernel that holds the slices in shared memory
 // (bn_segres.cu) runs its load, six dependent phases and store one after the other.

@@ -188,7 +188,8 @@ void anode_gpu_positive_clip_flat_map_bwd_f32(
  *   PLAIN     plain loads and stores (any shape, any alignment; one GPU);
  *   REGISTER  channels held in the registers of a warp, a block or a cluster (small layers, any alignment;
  *             one GPU);
- *   STREAM    clusters that walk a block of channels twice (large layers of short rows; one GPU).
+ *   STREAM    clusters that walk a block of channels twice (layers of short rows; one GPU); the largest of them in one
+ *             walk, with the tiles in tensor memory between reduction and normalization, where the call has a workspace.
  * anode_gpu_batch_norm_fused_set_kernel makes another choice process-wide: that kernel is used wherever it
  * applies, elsewhere one of the first four by the shape.  Meant for tests and measurements; which kernel a
  * call launches is answered by anode_gpu_batch_norm_fused_serving_kernel (anode_routines_gpu_diag.h). */

@@ -51,6 +51,12 @@ int anode_gpu_batch_norm_segres_geometry(uint32_t dim0, uint32_t dim1, uint32_t 
  * block, sample groups of a block, threads. */
 int anode_gpu_batch_norm_stream_geometry(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, uint32_t *out);
 
+/* Geometry of the band kernel, the streaming kernel's form for large layers.  out (16 values): taken by a call with a workspace
+ * of the full size (zeros behind a 0: the kernel cannot take the shape at all), channels per unit, units, sample groups of a tile,
+ * samples per thread, samples of a tile, tiles per unit, blocks, steps between a tile's two visits, boxes per band, vectors of
+ * a box's row, bytes of a box, slots, bytes of a slot, shared-memory bytes, log2 of the lanes per channel in the service warps. */
+int anode_gpu_batch_norm_band_geometry(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual, uint32_t *out);
+
 /* Geometry of the tiled kernel (bn_ring.cuh) for direction `dir` of a fused call on 16-byte aligned tensors.
  * out (12 values): applies, rows per tile, floats per row piece, tiles per unit, slots, bytes per slot, dynamic
  * shared memory bytes of the layout (the one-launch forms take the SM's whole), KiB between a tile's two visits, the

@@ -1,0 +1,142 @@
+"""The band kernel at the sizes where its splits have remainders: a last unit of fewer channels, a last tile of fewer samples,
+vectors shared by two channels, one sample group and many, one box and several, the most channels of a unit; the residual
+epilogue, outputs over inputs, a channel with a NaN or an infinity, and other kernels between its launches on one workspace."""
+import ctypes
+
+import pytest
+import torch
+
+from tests.test_band_plan import band
+from tests.test_gpu_tiled_forms import outputs_over_inputs
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(1283, 244, 7, 7), (300, 257, 14, 14), (500, 2003, 4, 4), (1999, 64, 11, 11), (81, 900, 15, 15), (1000, 2602, 2, 3), (60, 1004, 16, 17),
+          (1024, 250, 8, 8), (333, 1000, 7, 7)]
+
+
+@pytest.fixture
+def stream():
+    from anode_b200 import ops
+    ops.set_kernel("stream")
+    yield ops
+    ops.set_kernel("auto")
+
+
+def inputs(shape, seed):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    c = shape[1]
+    x = torch.randn(shape, device="cuda", generator=g) * 2 + 3 * torch.rand(1, c, 1, 1, device="cuda", generator=g)
+    return dict(x=x, dy=torch.randn(shape, device="cuda", generator=g), res=torch.randn(shape, device="cuda", generator=g),
+                gamma=torch.rand(c, device="cuda", generator=g) + 0.5, beta=torch.rand(c, device="cuda", generator=g) * 0.2 - 0.1)
+
+
+def run(ops, d, residual, slope, ws=None):
+    x, c = d["x"], d["x"].shape[1]
+    z = lambda: torch.zeros(c, device="cuda")
+    r = dict(mean=z(), var=z(), run_mean=z(), run_var=z() + 1, dgamma=z(), dbeta=z(), y=torch.full_like(x, float("nan")), dx=torch.full_like(x, float("nan")))
+    ws = ws or ops.Workspace(*ops.dims_of(x), x.device)
+    if residual:
+        r["dres"] = torch.full_like(x, float("nan"))
+        op = ops.BatchNormalize2dAddActFusedOp
+        op.apply([0, 1], 1e-5, 0.1, x, d["res"], r["y"], r["mean"], r["var"], r["run_mean"], r["run_var"], d["gamma"], d["beta"], slope, ws)
+        op.adjoint([0, 1], d["dy"], x, r["y"], r["mean"], r["var"], r["dx"], r["dres"], d["gamma"], d["beta"], r["dgamma"], r["dbeta"], slope, workspace=ws)
+    else:
+        ops.BatchNormalize2dFusedOp.apply([0, 1], 1e-5, 0.1, x, r["y"], r["mean"], r["var"], r["run_mean"], r["run_var"], d["gamma"], d["beta"],
+                                          workspace=ws, neg_slope=slope)
+        ops.BatchNormalize2dBwdFusedOp.apply([0, 1], d["dy"], x, r["mean"], r["var"], r["dx"], d["gamma"], d["beta"], r["dgamma"], r["dbeta"],
+                                             workspace=ws, neg_slope=slope)
+    assert ws.status() == 0
+    return r, ws
+
+
+def check(d, got, residual, slope, what):
+    """Against float64 with the layer's own activation decisions, exact ones away from zero; the tolerance of tests/util.py."""
+    x, dy = d["x"].double(), d["dy"].double()
+    ax, m = (0, 2, 3), x.numel() // x.shape[1]
+    v = lambda t: t.double().view(1, -1, 1, 1)
+    mean, var = x.mean(ax), x.var(ax, unbiased=False) + 1e-5
+    rstd = 1 / var.sqrt()
+    xhat = (x - v(mean)) * v(rstd)
+    pre = xhat * v(d["gamma"]) + v(d["beta"]) + (d["res"].double() if residual else 0)
+    mask = got["y"] > 0
+    assert not ((mask != (pre > 0)) & (pre.abs() >= 1e-5)).any(), what
+    act = torch.where(mask, 1.0, slope).double()
+    dz = dy * act
+    s1, s2 = dz.sum(ax), (dz * xhat).sum(ax)
+    want = dict(y=pre * act, mean=mean, var=var, run_mean=0.1 * mean, run_var=1 + 0.1 * (var - 1), dbeta=s1, dgamma=s2,
+                dx=v(d["gamma"]) * v(rstd) * (dz - v(s1) / m - xhat * v(s2) / m))
+    if residual:
+        want["dres"] = dz
+    for k, w in want.items():
+        atol = 1e-5 + (1e-4 * float(w.square().mean().sqrt()) if k in ("dgamma", "dbeta") else 0.0)
+        off = (got[k].double() - w).abs() > atol + 1e-4 * w.abs()
+        assert not off.any(), (what, k, int(off.sum()), off.nonzero()[0].tolist())
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("residual", [False, True])
+def test_against_float64(stream, shape, residual):
+    ops = stream
+    for direction in (0, 1):
+        assert band(shape, direction, residual)["taken"] == 1 and ops.serving_kernel(shape, direction, residual=residual) == "stream"
+    d, slope = inputs(shape, sum(shape)), 0.1 if shape[0] % 2 else 0.0
+    got, ws = run(ops, d, residual, slope)
+    check(d, got, residual, slope, shape)
+    for _ in range(2):                           # the other buffer of words, and the first one again
+        again, _ = run(ops, d, residual, slope, ws)
+        assert all(torch.equal(again[k], got[k]) for k in got), shape
+
+
+@pytest.mark.parametrize("form", ["dres is dy", "dres is y", "dres is x", "no dres", "dx is dy", "dx is x", "accumulate"])
+def test_outputs_over_inputs(form):
+    from anode_b200 import ops
+    assert band((1411, 132, 7, 7), 1, 1)["taken"] == 1
+    outputs_over_inputs(ops, (1411, 132, 7, 7), form, "stream")
+
+
+def test_other_kernels_between_its_launches_on_one_workspace(stream):
+    ops, shape = stream, (1283, 244, 7, 7)
+    d = inputs(shape, 7)
+    want, ws = run(ops, d, False, 0.0)
+    want_res, _ = run(ops, d, True, 0.0, ws)
+    for kernel in ("plain", "auto", "register", "cluster"):
+        ops.set_kernel(kernel)
+        check(d, run(ops, d, False, 0.0, ws)[0], False, 0.0, kernel)
+        ops.set_kernel("stream")
+        for residual, w in ((False, want), (True, want_res)):
+            got, _ = run(ops, d, residual, 0.0, ws)
+            assert all(torch.equal(got[k], w[k]) for k in w), (kernel, residual)
+
+
+def test_a_poisoned_channel_has_no_variance(stream):
+    ops, shape = stream, (1283, 244, 7, 7)
+    d = inputs(shape, 8)
+    clean, _ = run(ops, d, False, 0.0)
+    for place in (0, 777):
+        x = d["x"].clone()
+        x[place, 0, 3, 2], x[place, 2, 6, 6] = float("nan"), float("inf")
+        got, _ = run(ops, dict(d, x=x), False, 0.0)
+        for c in (0, 2):
+            assert torch.isnan(got["var"][c]) and torch.isnan(got["run_var"][c]) and not torch.isfinite(got["mean"][c])
+            assert torch.isnan(got["y"][:, c]).all()
+        assert got["mean"][2] == float("inf")
+        rest = [c for c in range(shape[1]) if c not in (0, 2)]
+        for k in ("mean", "var", "run_mean", "run_var", "dgamma", "dbeta"):
+            assert torch.equal(got[k][rest], clean[k][rest]), k
+        for k in ("y", "dx"):
+            assert torch.equal(got[k][:, rest], clean[k][:, rest]), k
+
+
+def test_means_far_from_zero_keep_the_variances_digits(stream):
+    """The shift of a channel's sums comes from three of its elements in each tile; with the mean at 300 standard deviations the
+    bound is that of the inputs' own rounding, 2^-24 * 300 relative to a deviation, for the mean of a few thousand of them."""
+    ops, shape = stream, (1024, 320, 7, 7)
+    d = inputs(shape, 9)
+    d["x"] = torch.randn(shape, device="cuda") + 300.0
+    got, _ = run(ops, d, False, 0.0)
+    x = d["x"].double()
+    var = x.var((0, 2, 3), unbiased=False) + 1e-5
+    assert float(((got["var"].double() - var) / var).abs().max()) < 300 * 2.0 ** -24
+    assert float((got["mean"].double() - x.mean((0, 2, 3))).abs().max()) < 300 * 2.0 ** -23
