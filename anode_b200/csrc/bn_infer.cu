@@ -8,15 +8,18 @@
 // (var is what anode stores: biased variance + epsilon.)  One read and one write of the tensor:
 // 8 bytes per element, HBM-bound.  A thread owns one 16-byte column of the sample (its channel
 // never changes), computes its coefficients once and walks down the samples.
-// On small layers the launch gap, a 64-bit division and the chain coefficients -> load -> store are the time: with the
-// launch overlapping the kernel before it, 32-bit indexes and the first load ahead of the coefficients [8,256,28,28]
-// went from 6.2 to 4.1 us per call, [32,64,56,56] from 10.3 to 8.2, [256,64,56,56] from 68.6 to 65.2.
+// On small layers the launch gap and the chain coefficients -> load -> store are the time, on ragged ones (float by float) what a
+// thread has in flight: a thread loads four samples at a time, the first four ahead of its coefficients, and the grid is no
+// larger than gives most threads four.  With one sample in flight and a thread for each of up to 32 blocks per SM, and so, us
+// from buffer to buffer: [8,256,28,28] 4.1 and 3.3, [32,256,14,14] 4.1 and 2.9, [64,512,7,7] 6.8 and 3.7, [32,64,56,56] 11.7 and 9.9,
+// [256,2048,7,7] 37.0 and 33.8, [64,95,55,55] 44.6 and 27.6, [256,256,56,56] 254 and 247 (1.01 of the copy bandwidth).
 #include "bn_device.cuh"
 #include "bn_host.h"
 
 namespace anode_b200 {
 
 constexpr uint32_t kInferThreads = 256;
+constexpr uint32_t kInferFlight = 4;      // samples in flight per thread
 
 // The inputs carry no __restrict__: it would let the compiler treat their loads as reads of memory that nothing writes while
 // the kernel runs and move them above pdl_wait(), where the kernel before this one may still be writing them (the running
@@ -31,11 +34,19 @@ __global__ void __launch_bounds__(kInferThreads) bn_infer_kernel(uint32_t dim0, 
   if (col >= per_sample) return;
   // channel of each of this thread's elements, and its coefficients (a sample has less than 2^32 floats, check_dims)
   uint32_t c = (uint32_t)col / dim0, off = (uint32_t)col - c * dim0;
+  // this thread's samples: blockIdx.y, + gridDim.y, ...; `left` of the batch from the next one on
+  uint32_t left = N - blockIdx.y;
+  const size_t step = (size_t)gridDim.y * per_sample;
+  size_t at = (size_t)blockIdx.y * per_sample + col;
+  Pack<VEC> p[kInferFlight];
+  auto load = [&] {
+#pragma unroll
+    for (int u = 0; u < kInferFlight; ++u)
+      if (u * gridDim.y < left) p[u] = Pack<VEC>::load(x + at + u * step);
+  };
   pdl_wait();
-  // the first sample's floats are on their way while the coefficients are made
-  uint32_t n = blockIdx.y;
-  size_t at = (size_t)n * per_sample + col;
-  Pack<VEC> p = Pack<VEC>::load(x + at);
+  // the first samples' floats are on their way while the coefficients are made
+  load();
   float sc[VEC], sh[VEC], mu[VEC];
   uint32_t prev = 0xffffffffu;
   float s0 = 0.f, b0 = 0.f, m0 = 0.f;
@@ -49,17 +60,20 @@ __global__ void __launch_bounds__(kInferThreads) bn_infer_kernel(uint32_t dim0, 
     mu[i] = m0; sc[i] = s0; sh[i] = b0;
     if (++off == dim0) { off = 0; ++c; }
   }
-  const size_t step = (size_t)gridDim.y * per_sample;
   for (;;) {
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-      const float t = fmaf(p.v[i] - mu[i], sc[i], sh[i]);
-      p.v[i] = t * (t > 0.0f ? 1.0f : neg_slope);
-    }
-    p.store_stream(y + at);
-    if (N - n <= gridDim.y) break;
-    n += gridDim.y; at += step;
-    p = Pack<VEC>::load(x + at);      // (with the next sample's load ahead of the store: [256,256,56,56] 258 -> 275 us)
+    for (int u = 0; u < kInferFlight; ++u)
+      if (u * gridDim.y < left) {
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) {
+          const float t = fmaf(p[u].v[i] - mu[i], sc[i], sh[i]);
+          p[u].v[i] = t * (t > 0.0f ? 1.0f : neg_slope);
+        }
+        p[u].store_stream(y + at + u * step);
+      }
+    if (left <= kInferFlight * gridDim.y) break;
+    left -= kInferFlight * gridDim.y; at += kInferFlight * step;
+    load();
   }
 }
 
@@ -82,12 +96,16 @@ extern "C" int anode_gpu_batch_norm_act_infer_3d1_packed_f32(
   const uint64_t cols = vec ? per_sample / 4 : per_sample;
   const uint64_t bx = (cols + kInferThreads - 1) / kInferThreads;
   if (bx > 0x7fffffffull) return ANODE_E_DIMS;
-  // enough blocks to fill the device a few times over; the rest of the samples are walked in the loop
-  const uint64_t want = (uint64_t)sm_count() * 32;
-  uint64_t by = (want + bx - 1) / bx;
-  if (by > dim2) by = dim2;
-  if (by > 65535) by = 65535;
-  if (by < 1) by = 1;
+  // Samples per thread: a multiple of four that makes no more than `most` blocks per SM (eight are resident: where the launch is the
+  // time one wave and a half, [8,95,55,55] 4.1 us with twelve and 5.0 with 16 to 64; on large layers more of them keep HBM busier,
+  // [256,256,56,56] 266 us with twelve, 253 with 32 and 248 with 64, but [256,2048,7,7] 34.6, 33.9 and 35.7), or fewer than four where
+  // that leaves SMs with one block ([8,256,28,28] 2.9 us with two of them, 3.5 with four and more).
+  const uint64_t elements = per_sample * dim2, most = (uint64_t)sm_count() * (!vec || elements < (16u << 20) ? 12 : elements < (64u << 20) ? 32 : 64);
+  const uint64_t rows = most / bx;                   // blocks one below the other, at most
+  uint64_t each = rows ? (dim2 + rows - 1) / rows : dim2;
+  each = (each + kInferFlight - 1) / kInferFlight * kInferFlight;
+  while (each > 1 && bx * ((dim2 + each - 1) / each) < 2ull * sm_count()) each /= 2;
+  const uint64_t by = (dim2 + each - 1) / each;      // (no more than `most`, so below 65536)
   const dim3 grid((unsigned)bx, (unsigned)by);
   // The launch may overlap the tail of the kernel before it (every block waits for that kernel's results before it
   // touches memory): in a network at a serving batch the layers last a few microseconds each.
