@@ -11,7 +11,7 @@
 // theirs; the expressions here are the reference's op by op (rsqrtf; mean need not be the batch's in the adjoint).
 //
 // What bounds the composition, [64,128,28,28] (26 MB tensors): seventeen launches and twenty passes over L2 took 114.5 us,
-// composition and adjoint in one launch each and the two ReLU maps 52.
+// composition and adjoint in one launch each and the two ReLU maps 47.
 #include <cooperative_groups.h>
 
 #include "bn_device.cuh"
@@ -24,6 +24,7 @@ namespace anode_b200 {
 constexpr uint32_t kComposeThreads = 512, kComposeCluster = 8;
 constexpr uint64_t kComposeSmall = 128u << 10;      // floats of a small channel (launch_compose)
 constexpr int kComposeHold = 4;       // vectors per tensor that a thread holds (64 registers: two blocks per SM)
+constexpr int kComposeScalars = 8;    // floats in flight per thread and tensor where rows are loaded float by float
 
 struct ComposeArgs {
   uint32_t dim0, C, N;
@@ -71,10 +72,11 @@ __global__ void __launch_bounds__(kComposeThreads, 2) bn_compose_kernel(const Co
 
   // the thread's vectors are j0, j0 + stride, ... of the channel, B of them in flight; places by walking (row, column) along
   // (float offsets are below 2^32, check_dims)
-  // (H batches a turn, so that the adjoint's plain sums have four chains of additions per thread, as the ops they stand for,
-  // and that of dy * (x - mean) two: with two chains each the sum of 8 M equal dy was off by 8.0e-6, the ops' by 4.2e-6)
-  constexpr int B = HOLD || DIR == 0 ? kComposeHold : kComposeHold / 2, H = VEC == 1 ? kComposeHold / B : 1;
-  constexpr int S = kComposeHold / (B * H), D = HOLD ? kComposeHold : kComposeHold / 2;
+  // Four chains of additions per thread (that of dy * (x - mean) two or four).  Where the cluster is chosen for the waves of blocks
+  // (launch_compose) they are emptied into double precision after every batch, so that a chain is two to four additions however much a
+  // thread walks: the adjoint's sums are no further from float64 than with the larger clusters (it costs nothing: the walk waits for loads).
+  constexpr int B = HOLD ? kComposeHold : VEC == 1 ? kComposeScalars : DIR == 0 ? kComposeHold : kComposeHold / 2;
+  constexpr int S = B < kComposeHold ? kComposeHold / B : 1, D = HOLD || VEC == 1 ? kComposeHold : kComposeHold / 2;
   const uint32_t per_row = g.dim0 / VEC, total = per_row * g.N, rs = g.C * g.dim0;
   const uint32_t stride = cs * blockDim.x, j0 = rank * blockDim.x + threadIdx.x;
   const uint32_t row0 = j0 / per_row, drow = stride / per_row;
@@ -86,54 +88,52 @@ __global__ void __launch_bounds__(kComposeThreads, 2) bn_compose_kernel(const Co
   pdl_trigger();
 
   Pack<VEC> vx[B], vd[DIR == 1 ? B : 1];
-  // visit(f): f(x, dy, offset, number of its chain) for every vector, B loads in flight; the first visit of a held channel loads it
+  // visit(f, turn): f(x, dy, offset, number of the vector in its batch) for every vector, B loads in flight, and turn() after every
+  // batch; the first visit of a held channel loads it
   bool loaded = false;
-  auto visit = [&](auto f) {
+  auto visit = [&](auto f, auto turn) {
     uint32_t off = off0, col = col0;
-    for (uint32_t k0 = 0; k0 < cnt; k0 += B * H) {
+    for (uint32_t k = 0; k < cnt; k += B) {
+      uint32_t at[B];
 #pragma unroll
-      for (int h = 0; h < H; ++h) {
-        const uint32_t k = k0 + h * B;
-        uint32_t at[B];
-#pragma unroll
-        for (int u = 0; u < B; ++u) {
-          at[u] = off;
-          if (k + u < cnt && !(HOLD && loaded)) {
-            vx[u] = Pack<VEC>::load(g.x + off);
-            if (DIR == 1) vd[u] = Pack<VEC>::load(g.dy + off);
-          }
-          off += step; col += dcol;
-          if (col >= per_row) { col -= per_row; off += wrap; }
+      for (int u = 0; u < B; ++u) {
+        at[u] = off;
+        if (k + u < cnt && !(HOLD && loaded)) {
+          vx[u] = Pack<VEC>::load(g.x + off);
+          if (DIR == 1) vd[u] = Pack<VEC>::load(g.dy + off);
         }
-#pragma unroll
-        for (int u = 0; u < B; ++u)
-          if (k + u < cnt) f(vx[u], vd[DIR == 1 ? u : 0], at[u], u + h * B);
+        off += step; col += dcol;
+        if (col >= per_row) { col -= per_row; off += wrap; }
       }
+#pragma unroll
+      for (int u = 0; u < B; ++u)
+        if (k + u < cnt) f(vx[u], vd[DIR == 1 ? u : 0], at[u], u);
       if (HOLD) break;
+      if (DIR == 1 || VEC == 1) turn();
     }
     loaded = true;
   };
   const float norm = (float)g.dim0 * (float)g.N;
 
+  auto nothing = [] {};
   if constexpr (DIR == 0) {
-    float acc[B] = {};
+    float acc[kComposeHold] = {};
+    double v[1] = {0.0};
+    auto empty = [&] { v[0] += ((double)acc[0] + (double)acc[1]) + ((double)acc[2] + (double)acc[3]); acc[0] = acc[1] = acc[2] = acc[3] = 0.f; };
     visit([&](const Pack<VEC> &x, const Pack<VEC> &, uint32_t, int u) {
 #pragma unroll
-      for (int i = 0; i < VEC; ++i) acc[u] += x.v[i];
-    });
-    double v[1] = {0.0};
-#pragma unroll
-    for (int u = 0; u < B; ++u) { v[0] += (double)acc[u]; acc[u] = 0.f; }
+      for (int i = 0; i < VEC; ++i) acc[u % kComposeHold] += x.v[i];
+    }, empty);
+    empty();
     if (cs > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     cluster_sums(cluster, v, part, gather[0]);
     const float m = (float)v[0] / norm;                               // batch_norm.cu:54
+    v[0] = 0.0;
     visit([&](const Pack<VEC> &x, const Pack<VEC> &, uint32_t, int u) {
 #pragma unroll
-      for (int i = 0; i < VEC; ++i) { const float d = x.v[i] - m; acc[u] += d * d; }
-    });
-    v[0] = 0.0;
-#pragma unroll
-    for (int u = 0; u < B; ++u) v[0] += (double)acc[u];
+      for (int i = 0; i < VEC; ++i) { const float d = x.v[i] - m; acc[u % kComposeHold] += d * d; }
+    }, empty);
+    empty();
     cluster_sums(cluster, v, part, gather[1]);
     const float var = (float)v[0] / norm + g.epsilon;                 // batch_norm.cu:160
     if (rank == 0 && threadIdx.x == 0) {
@@ -148,19 +148,26 @@ __global__ void __launch_bounds__(kComposeThreads, 2) bn_compose_kernel(const Co
 #pragma unroll
       for (int i = 0; i < VEC; ++i) o.v[i] = (x.v[i] - m) * r;
       o.put(g.out + at);
-    });
+    }, nothing);
   } else {
     const float m = g.mean_in[c], va = g.var_in[c], r = rsqrtf(va);
     float a1[D] = {}, a2[kComposeHold] = {}, a3[kComposeHold] = {};
+    double v[3] = {0.0, 0.0, 0.0};
+    auto empty = [&] {
+#pragma unroll
+      for (int u = 0; u < D; ++u) { v[0] += (double)a1[u]; a1[u] = 0.f; }
+      v[1] += (double)a2[0] + (double)a2[1] + ((double)a2[2] + (double)a2[3]); v[2] += (double)a3[0] + (double)a3[1] + ((double)a3[2] + (double)a3[3]);
+      a2[0] = a2[1] = a2[2] = a2[3] = a3[0] = a3[1] = a3[2] = a3[3] = 0.f;
+    };
     visit([&](const Pack<VEC> &x, const Pack<VEC> &dy, uint32_t, int u) {
 #pragma unroll
-      for (int i = 0; i < VEC; ++i) { const float d = x.v[i] - m; a1[u % D] = fmaf(dy.v[i], d, a1[u % D]); a2[u * S + i % S] += dy.v[i]; a3[u * S + i % S] += d; }
-    });
-    double v[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-    for (int u = 0; u < D; ++u) v[0] += (double)a1[u];
-#pragma unroll
-    for (int u = 0; u < kComposeHold; ++u) { v[1] += (double)a2[u]; v[2] += (double)a3[u]; }
+      for (int i = 0; i < VEC; ++i) {
+        const int chain = (u * S + i % S) % kComposeHold;
+        const float d = x.v[i] - m;
+        a1[u % D] = fmaf(dy.v[i], d, a1[u % D]); a2[chain] += dy.v[i]; a3[chain] += d;
+      }
+    }, empty);
+    empty();
     if (cs > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     cluster_sums(cluster, v, part, gather[0]);
     const float dvar = (float)((double)(-0.5f * r / va) * v[0]);                            // batch_norm.cu:492
@@ -172,7 +179,7 @@ __global__ void __launch_bounds__(kComposeThreads, 2) bn_compose_kernel(const Co
 #pragma unroll
       for (int i = 0; i < VEC; ++i) o.v[i] = fmaf(dy.v[i], r, fmaf(x.v[i] - m, k1, k0));
       o.put(g.out + at);
-    });
+    }, nothing);
   }
 }
 
@@ -194,17 +201,28 @@ static int launch_compose(const ComposeArgs &g, bool aligned, cudaStream_t strea
 {
   const bool vec = g.dim0 % 4 == 0 && aligned;
   const uint64_t total = (uint64_t)(vec ? g.dim0 / 4 : g.dim0) * g.N;
-  // The smallest cluster that holds the channel; else enough blocks for the device.  Forward passes that load the floats of
-  // small channels one by one: no larger than makes eight blocks per SM, more blocks only repeat the fixed steps of a cluster
-  // for a few floats a thread.  Us with the cluster that would hold the channel, with this one, and op by op: [3,1024,55,55]
-  // 91, 48, 60, [8,2048,55,55] 395, 152, 313, [16,1024,33,33] 181, 78, 113, [6,512,55,55] 83, 49, 60, but [65,1024,55,55] 684,
-  // 798, 1251.
-  const uint64_t most = DIR == 0 && !vec && total <= kComposeSmall ? 8ull * sm_count() : ~0ull;
+  // The smallest cluster that holds the channel, else one of eight; but the adjoint, and forward passes that load the floats of small
+  // channels one by one, no larger than makes two blocks per SM, what is resident: more blocks only repeat the fixed steps of a cluster.
+  // (Two where a thread of one block would have 64 floats and more; two that hold the channel.)  Adjoint with the cluster that
+  // holds the channel or eight, and so, us: [64,128,28,28] 25.2 and 20.0, [32,64,56,56] 25.9 and 19.6, [64,512,28,28] 88 and 76, [64,128,27,27]
+  // 32.4 and 21.2, [40,300,15,15] 39.5 and 15.4, [256,1024,7,7] 132 and 49, [16,95,55,55] 24.6 and 19.6.  Forward [32,512,27,27] 66 and 40,
+  // but [65,1024,55,55] 684 and 798.  (With two and four floats in flight per thread in the place of eight, the adjoint's scalar
+  // rows took 38.8 us, [64,128,27,27], and 29.3, [16,95,55,55].)
+  const bool waves = DIR == 1 || (!vec && total <= kComposeSmall);
+  const uint32_t lanes = vec ? 4u : 1u;
+  auto holds = [&](uint32_t n) { return total <= (uint64_t)n * kComposeThreads * kComposeHold; };
   uint32_t cs = 1;
-  while (cs < kComposeCluster && total > (uint64_t)cs * kComposeThreads * kComposeHold && (uint64_t)g.C * cs < most) cs *= 2;
-  const bool hold = total <= (uint64_t)cs * kComposeThreads * kComposeHold;
+  while (cs < kComposeCluster && !holds(cs) &&
+         (!waves || (uint64_t)g.C * cs * 2 <= 2ull * sm_count() || (cs == 1 && (total * lanes >= 64ull * kComposeThreads || (vec && holds(2)))))) cs *= 2;
+  const bool hold = holds(cs);
+  // threads of a block: a vector each where all of them are resident at once, else up to what one holds
   const uint64_t each = (total + cs - 1) / cs;
-  const uint32_t threads = each < kComposeThreads ? (uint32_t)(each + 31) / 32 * 32 : kComposeThreads;
+  uint32_t threads = kComposeThreads;
+  for (uint32_t k = 1; k <= kComposeHold; ++k) {
+    const uint64_t t = ((each + k - 1) / k + 31) / 32 * 32;
+    if (t < threads && (hold || k == 1)) threads = (uint32_t)t;
+    if (!hold || (uint64_t)g.C * cs * threads <= 1024ull * sm_count()) break;
+  }
   if ((uint64_t)g.C * cs > 0x7fffffffull) return ANODE_E_DIMS;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(g.C * cs);
