@@ -128,14 +128,28 @@ static uint32_t ring_tile_vecs(const Plan &p) { return p.rows_per_tile * ring_pi
 // consumer warps of direction `dir` (the two instantiations of bn_ring.cuh)
 static uint32_t ring_warps(int dir) { return dir == 0 ? 8u : 16u; }
 
-// Forward pass of the residual epilogue on ragged rows from this length on: no tile stays in tensor memory.  The two forms of
-// a ragged visit are long, and consumers that run one of them alone are faster than tensor memory makes them; on shorter rows
-// the producer's copies, one per row and tensor, bound the kernel, and a kept tile needs one less.  Us with tensor memory, and
-// without either: 40 M elements of 131 channels, rows of 301 119 and 144, 451 107 and 116, 601 103 and 103, 713 104 and 99,
-// 1201 109 and 99; [34,123,6374] 96 and 70, [50,119,12674] 268 and 202, [200,100,5041] 357 and 273 (where every second visit
-// was one from L2, in an older form of both: 76, 238, 279).
-constexpr uint32_t kRaggedKeepMost = 640;
-static bool ring_keeps(const Plan &p, int dir, bool extra) { return !(dir == 0 && extra && p.dim0 % 4 != 0 && p.dim0 >= kRaggedKeepMost); }
+// Bytes between the two visits of a tile: what L2 has to hold for the apply visit to find its tile there.
+static uint64_t ring_window_bytes(const Plan &p, int dir)
+{
+  return (uint64_t)p.lookahead_steps * p.grid * p.rows_per_tile * p.piece_len * 4 * (dir == 1 ? 2 : 1);
+}
+
+// Forward passes on ragged rows from this length on: no tile stays in tensor memory.  The two forms of a ragged visit are long, and
+// consumers that run one of them alone are faster than tensor memory makes them; on shorter rows the producer's copies, one per
+// row and tensor, bound the kernel, and a kept tile needs one less.  Us with tensor memory, and without: [64,95,55,55] 39.8 and 35.5,
+// [512,128,55,55] 328 and 295, [256,64,111,111] 328 and 305, [300,301,31,31] 149 and 146, but [1024,101,21,21] 84.7 and 85.3.  (A form
+// with nothing but kept tiles: 40.4, 308, 303, 138.)  Not where L2 does not keep what lies between two visits, nor in layers of few
+// channels, which come near that line from one size to the next: [1252,6,7485] 97 and 101, [952,3,14225] 75.5 and 76.6, but
+// [598,11,1991] 29 and 25.
+// Residual epilogue, with tensor memory, and without either: 40 M elements of 131 channels, rows of 301 119 and 144, 451 107 and 116,
+// 601 103 and 103, 713 104 and 99, 1201 109 and 99; [34,123,6374] 96 and 70, [50,119,12674] 268 and 202, [200,100,5041] 357 and 273
+// (where every second visit was one from L2, in an older form of both: 76, 238, 279).
+constexpr uint32_t kRaggedKeepMost = 640, kRaggedKeepChannels = 24;
+static bool ring_keeps(const Plan &p, int dir, bool extra)
+{
+  if (dir != 0 || p.dim0 % 4 == 0 || p.dim0 < kRaggedKeepMost) return true;
+  return !extra && (p.C < kRaggedKeepChannels || ring_window_bytes(p, dir) > kRingLargeWindowMax);
+}
 
 // Fused mode: the tiles that stay in tensor memory.
 static void ring_keep(const Plan &p, int dir, bool extra, RingGeom &g)
@@ -219,12 +233,6 @@ static bool ring_plan_with(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool 
   g = ring_geom(p, dir, extra, slots, slot_floats);
   while (g.smem_bytes > kRingSmemBudget && slots > 2) { --slots; g = ring_geom(p, dir, extra, slots, slot_floats); }
   return g.smem_bytes <= kRingSmemBudget;
-}
-
-// Bytes between the two visits of a tile: what L2 has to hold for the apply visit to find its tile there.
-static uint64_t ring_window_bytes(const Plan &p, int dir)
-{
-  return (uint64_t)p.lookahead_steps * p.grid * p.rows_per_tile * p.piece_len * 4 * (dir == 1 ? 2 : 1);
 }
 
 // Backward pass: three slots of larger tiles are faster than four of the standard ones as long as the larger
@@ -337,7 +345,7 @@ static RingKernel pick_ring_kernel(const Plan &p, int dir, bool extra, uint32_t 
   const bool ragged = p.dim0 % 4 != 0;
   threads = dir == 0 ? ring8::kRingThreads : ring16::kRingThreads;
   if (dir == 0) {
-    if (extra && !ring_keeps(p, dir, extra)) return ring8::bn_ring_kernel<0, true, true, false>;
+    if (!ring_keeps(p, dir, extra)) return extra ? ring8::bn_ring_kernel<0, true, true, false> : ring8::bn_ring_kernel<0, false, true, false>;
     if (extra) return ragged ? ring8::bn_ring_kernel<0, true, true> : ring8::bn_ring_kernel<0, true, false>;
     return ragged ? ring8::bn_ring_kernel<0, false, true> : ring8::bn_ring_kernel<0, false, false>;
   }

@@ -47,3 +47,21 @@ def test_residual_rows_on_both_sides_of_the_line_below_which_tiles_stay(row):
         check_layer_own_mask(d, run_add_act(ops, d, res, 0.1), "%r " % (shape,), residual=res, slope=0.1)
     finally:
         ops.set_kernel("auto")
+
+
+@pytest.mark.parametrize("shape", [(120, 24, 1, 639), (120, 24, 1, 641), (64, 25, 55, 55), (3, 31, 111, 111), (1, 24, 1, 65543)])
+def test_forward_rows_on_both_sides_of_the_line_below_which_tiles_stay(shape):
+    from anode_b200 import ops
+    d0 = shape[2] * shape[3]
+    assert bool(keep((d0, shape[1], shape[0]), 0, 0, 0, 0)["slots"]) == (d0 <= 640)
+    d = make_inputs(shape, seed=d0, loc=0.5, scale=2.0)
+    ops.set_kernel("tiled")
+    try:
+        assert ops.serving_kernel(shape, 0) == "tiled"
+        got, ws = run_fused(ops, d)
+        check_layer_own_mask(d, got, "%r " % (shape,))
+        again, _ = run_fused(ops, d, ws=ws)
+        for k in ("y", "dx", "mean", "var"):
+            assert np.array_equal(again[k], got[k]), (shape, k)
+    finally:
+        ops.set_kernel("auto")

@@ -65,3 +65,10 @@ def test_long_ragged_rows_of_the_residual_forward_pass_keep_no_tiles():
         shape = (d0, 20, 300)
         assert [bool(keep(shape, d, 1, 0, 0)["slots"]) for d in (0, 1)] == [forward, True], d0
         assert all(keep(shape, d, 0, 0, 0)["slots"] for d in (0, 1)), d0
+
+
+def test_long_ragged_rows_of_the_forward_pass_keep_no_tiles():
+    """Ordinary layers: from 24 channels on, where L2 keeps what lies between a tile's two visits; backward passes keep theirs."""
+    for d0, c, n, forward in ((639, 95, 300, True), (641, 95, 300, False), (644, 95, 300, True), (3025, 95, 64, False), (3025, 23, 64, True),
+                              (3025, 24, 64, False), (7485, 30, 1252, True)):
+        assert [bool(keep((d0, c, n), d, 0, 0, 0)["slots"]) for d in (0, 1)] == [forward, True], (d0, c, n)
