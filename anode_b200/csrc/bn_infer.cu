@@ -100,13 +100,17 @@ extern "C" int anode_gpu_batch_norm_act_infer_3d1_packed_f32(
   // time one wave and a half, [8,95,55,55] 4.1 us with twelve and 5.0 with 16 to 64; on large layers more of them keep HBM busier,
   // [256,256,56,56] 266 us with twelve, 253 with 32 and 248 with 64, but [256,2048,7,7] 34.6, 33.9 and 35.7), or fewer than four where
   // that leaves SMs with one block ([8,256,28,28] 2.9 us with two of them, 3.5 with four and more).
-  const uint64_t elements = per_sample * dim2, most = (uint64_t)sm_count() * (!vec || elements < (16u << 20) ? 12 : elements < (64u << 20) ? 32 : 64);
-  const uint64_t rows = most / bx;                   // blocks one below the other, at most
-  uint64_t each = rows ? (dim2 + rows - 1) / rows : dim2;
-  each = (each + kInferFlight - 1) / kInferFlight * kInferFlight;
-  while (each > 1 && bx * ((dim2 + each - 1) / each) < 2ull * sm_count()) each /= 2;
-  const uint64_t by = (dim2 + each - 1) / each;      // (no more than `most`, so below 65536)
-  const dim3 grid((unsigned)bx, (unsigned)by);
+  // (32-bit arithmetic: a 64-bit division costs what two per cent of the call do)
+  const uint64_t elements = per_sample * dim2;
+  const uint32_t sms = sm_count(), most = sms * (!vec || elements < (16u << 20) ? 12 : elements < (64u << 20) ? 32 : 64), wide = (uint32_t)bx;
+  const uint32_t rows = most / wide;                 // blocks one below the other, at most
+  uint32_t each = rows ? dim2 / rows + (dim2 % rows != 0) : dim2, by = 1;
+  if (each < dim2) each = (each + kInferFlight - 1) / kInferFlight * kInferFlight;
+  for (;; each /= 2) {
+    by = dim2 / each + (dim2 % each != 0);           // (no more than `most`, so below 65536)
+    if (each <= 1 || wide >= 2 * sms || wide * by >= 2 * sms) break;
+  }
+  const dim3 grid(wide, by);
   // The launch may overlap the tail of the kernel before it (every block waits for that kernel's results before it
   // touches memory): in a network at a serving batch the layers last a few microseconds each.
   cudaLaunchConfig_t cfg_ = {};
