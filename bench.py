@@ -439,7 +439,7 @@ KERNEL_NAMES = {"tiled": ("bn_ring_kernel", "fused reduce+apply, tiled"),
                 "resident": ("bn_resident_kernel", "fused reduce+apply, slices resident in shared memory"),
                 "plain": ("bn_pipeline_kernel", "fused reduce+apply, plain"),
                 "register": ("bn_chan_kernel", "fused reduce+apply, channels in registers"),
-                "stream": ("bn_stream_kernel", "fused reduce+apply, streaming clusters")}
+                "stream": ("bn_stream_kernel / bn_band_kernel", "fused reduce+apply, short rows: streaming clusters, large layers tiles of bands")}
 
 
 def bench_infer(layer, x, y, steps, warmup):
