@@ -13,6 +13,7 @@ constexpr uint32_t kBandWarps = 8, kBandConsumers = 32 * kBandWarps;      // con
 constexpr uint32_t kBandThreads = kBandConsumers + 96;                     // + producer, delivery and coefficient warps
 constexpr uint32_t kBandChannels = 32;      // most channels of a unit
 constexpr uint32_t kBandVecs = 64;          // vectors of tensor memory per consumer thread (512 columns for four warps)
+constexpr double kBandWordCost = 3.5, kBandRunCost = 140.0;      // band_geom: vectors that a word costs, bytes that a run's ends cost
 constexpr uint32_t kBandWords = 512;        // most words of a unit
 constexpr uint32_t kBandBox = 64;           // most vectors of a box (256 floats, the most a tensor map takes)
 constexpr uint32_t kBandMaxSlots = 8, kBandQ = 3;
@@ -42,10 +43,13 @@ inline bool band_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra
   if (dim0 < 4 || (uint64_t)C * dim0 % 4 != 0) return false;
   uint32_t q = 4; if (dim0 % 2 == 0) q = 2; if (dim0 % 4 == 0) q = 1;      // cb*dim0 must be a multiple of 4
   const uint32_t kept = dir == 0 ? 1u : 2u, most = kBandVecs / 4 / kept;      // tensors kept; most samples per thread, for four tiles
-  // Channels of a unit and samples per thread: the least (steps + 3) * (fixed cost of a step + vectors of a tile), the fixed cost
-  // (merge, barriers, parameters) as vectors.  [1024,2048,7,7] forward / backward with tiles of 16 / 8, 12 / 6, 8 / 4 samples per
-  // thread: 143 / 202, 145 / 231, 169 / 300 us.  Runs of 512 bytes at least where the channels make them.
-  // (The words of a unit weigh in: [200,2048,8,8] backward with units of 16 channels and 400 words 64 us, of 2 and 22 words 60.)
+  // Channels of a unit and samples per thread: the least (steps + 3) * (cost of a step) * (cost of the runs), fitted to measurements.
+  //   A step: a fixed part (merge, barriers, parameters), the tile's vectors, the unit's words.  [1024,2048,7,7] forward / backward with
+  //   tiles of 16 / 8, 12 / 6, 8 / 4 samples per thread 143 / 202, 145 / 231, 169 / 300 us; [200,2048,8,8] backward with units of 16
+  //   channels and 400 words 64 us, of 2 and 22 words 60; [400,2048,8,8] forward with 400 words 82 us, with 15 76.
+  //   The runs: short ones cost HBM and the copies more (a run that ends within a 32-byte sector shares it with another block's).
+  //   [256,1024,14,14] forward with runs of 784, 1568, 3136, 3920 bytes 92, 84, 80, 80 us; [100,2048,12,12] of 576 and 4032 bytes 59 and 49.
+  // Runs of 512 bytes at least where the channels make them.
   const double fixed = dir == 0 ? 1000.0 : 1900.0;
   double best = 0.0;
   for (uint32_t cb = q; cb <= C && cb <= kBandChannels && (uint64_t)cb * dim0 <= 4 * kBandConsumers; cb += q) {
@@ -61,7 +65,7 @@ inline bool band_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra
       if (tiles > sms || tiles * cb > kBandWords || 4ull * rows * C * dim0 >> 32) continue;      // (a thread's places within a tile: 32 bits)
       const uint32_t total = units * tiles;
       if (total < sms) continue;
-      const double cost = (double)(ceil_div_u32(total, sms) + 3) * (fixed + (double)(rows * L4) + 0.8 * (double)(tiles * cb));
+      const double cost = (double)(ceil_div_u32(total, sms) + 3) * (fixed + (double)(rows * L4) + kBandWordCost * (double)(tiles * cb)) * (1.0 + kBandRunCost / (16.0 * L4));
       if (best != 0.0 && cost > 0.98 * best) continue;
       best = cost;
       g.cb = cb; g.L4 = L4; g.units = units; g.groups = groups; g.vpt = per; g.rows = rows; g.tiles = tiles; g.total = total;

@@ -297,11 +297,11 @@ bool chan_applies(const FusedArgs &a, int dir, bool aligned)
 constexpr uint32_t kChanTiledRow = 480;
 constexpr uint64_t kChanTiled = 16u << 20, kChanTiledExtra = 18u << 20, kChanTiledChannel = 24u << 10;
 // Aligned rows below 320 floats go to the band kernel (the streaming kernel's form for large layers) from these sizes on.  Us here
-// and there, forward: [100,1024,16,16] 26 M 45 and 49, [180,1024,14,14] 36 M 66.4 and 65.7, [256,1024,14,14] 98 and 88, [2000,2048,4,4] 115
-// and 91; backward: [50,2048,12,12] 15 M 36.4 and 38.4, [100,1024,14,14] 20 M 55 and 47, [256,1024,14,14] 163 and 104; residual forward
-// 20 M 50 and 53, [200,2048,8,8] 26 M 63 and 58; residual backward 15 M 52 and 53, 20 M 77 and 68.
+// and there, forward: [80,1024,14,14] 16 M 27.9 and 33.2, [100,1024,16,16] 26 M 45 and 50, [100,1000,10,30] 30 M 52.2 and 52.1,
+// [180,1024,14,14] 36 M 66 and 58, [256,1024,14,14] 98 and 75; backward: [50,2048,12,12] 15 M 36.4 and 38.4, [100,1024,14,14] 20 M 55 and 47,
+// [256,1024,14,14] 163 and 104; residual forward 16 M 38.7 and 38.5, 20 M 50 and 42; residual backward 15 M 52 and 53, 20 M 77 and 68.
 constexpr uint32_t kChanBandRow = 320;
-constexpr uint64_t kChanBand[2][2] = {{40000000, 24000000}, {18000000, 18000000}};      // [direction][residual]
+constexpr uint64_t kChanBand[2][2] = {{28000000, 18000000}, {18000000, 18000000}};      // [direction][residual]
 constexpr uint64_t kChanLarge = 8u << 20, kChanLargeScalar = 3u << 20, kChanLargeExtra = 5u << 20;
 constexpr uint64_t kChanWaves = 1500000, kChanShortest = 1200000;
 constexpr uint32_t kChanFewSamples = 32;
