@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
     }
   } else if (warp == kBandWarps) {
     // ------------------------------------------------------------------ producer
-    const uint64_t pol = policy_drop();
+    const uint64_t pol = g.whole ? policy_drop() : policy_normal();
     BandWalk red(g, b, G), app(g, b, G);
     uint32_t slot = g.slots - 1, par = 1, k = 0;
     bool ok = true;
@@ -581,6 +581,11 @@ bool band_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, BandG
   return band_geom(dim0, C, N, dir, extra, sm_count(), g);
 }
 
+// Lines that two units share are read by two blocks, one after the other.  Loaded to be evicted first, as all others, they may be gone by
+// then: ordinary backward passes over tensors beyond L2 load them with the normal priority.  Us with the one and the other, backward:
+// [1024,2048,7,7] 214 and 202 (206 and 204 on another device; step 369 and 362), [2048,1024,7,7] 212 and 205, [512,2048,7,7] 108 and 106; but
+// [128,2048,7,7] 33 and 36, runs of whole lines [2000,2048,4,4] 134 and 136, residual step of [256,1024,14,14] 279 and 280.
+constexpr uint64_t kBandShared = 192ull << 20;      // bytes of x and dy
 int launch_band(FusedArgs &a, const BandGeom &g, int dir, cudaStream_t stream)
 {
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
@@ -609,6 +614,7 @@ int launch_band(FusedArgs &a, const BandGeom &g, int dir, cudaStream_t stream)
     if (!it->second) return ANODE_E_LAUNCH;
   }
   BandGeom gg = g;
+  gg.whole = dir == 0 || extra || (uint64_t)width * a.plan.N * 8 < kBandShared || g.L4 % 8 == 0;
   void *params[] = {(void *)&a, (void *)&gg, (void *)&m};
   if (cudaLaunchCooperativeKernel(k, dim3(g.grid), dim3(kBandThreads), params, kBandSmem, stream) != cudaSuccess) {
     (void)cudaGetLastError();

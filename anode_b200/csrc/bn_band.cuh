@@ -27,6 +27,7 @@ struct BandGeom {
   uint32_t boxes, box4, box_bytes;     // boxes of a band, vectors of a box's row, bytes of a box in a slot
   uint32_t slots, plane_bytes, slot_stride, off_side, off_res, off_coef, off_slots, smem_bytes;
   uint32_t lane_shift;                 // log2 of the lanes that work on one channel in the service warps
+  uint32_t whole;                      // loads: 1 the lines are dead once read, 0 neighbouring units' blocks read parts of them, too
   uint32_t tag, hdr;                   // workspace: tagged words, exit counter and parity word (byte offsets)
   double inv_full, inv_tail, inv_count;      // reciprocals of a channel's elements in a tile, in a unit's last tile, in the layer
 };

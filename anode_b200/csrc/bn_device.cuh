@@ -57,6 +57,13 @@ __device__ __forceinline__ uint64_t policy_keep_fraction(float f)
   asm volatile("createpolicy.fractional.L2::evict_last.L2::evict_first.b64 %0, %1;" : "=l"(p) : "f"(f));
   return p;
 }
+// neither
+__device__ __forceinline__ uint64_t policy_normal()
+{
+  uint64_t p;
+  asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
 __device__ __forceinline__ uint64_t policy_drop()
 {
   uint64_t p;
