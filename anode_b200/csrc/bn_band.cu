@@ -18,8 +18,8 @@
 // so that no other block holds columns of tensor memory or waits for them.
 //
 // What bounds it: HBM, and some 10 us in which the schedule fills and drains.  Streaming kernel and this one, forward / backward:
-// [1024,2048,7,7] 179 / 298 and 143 / 203 us (0.88 / 0.93 of the copy bandwidth), residual epilogue 246 / 427 and 204 / 339 (0.92 /
-// 0.93); [256,1024,14,14] backward 148 -> 104, residual 137 / 211 -> 109 / 163.  On the way there: sixteen consumer warps (96
+// [1024,2048,7,7] 179 / 298 and 143 / 202 us (0.88 / 0.93 of the copy bandwidth), residual epilogue 246 / 427 and 204 / 339 (0.92 /
+// 0.93); [256,1024,14,14] 102 / 148 and 75 / 104, residual 137 / 211 and 101 / 163.  On the way there: sixteen consumer warps (96
 // registers) 150 / 218; all vectors of the threads' sums added up one by one in double precision 156 / 238.
 #include <cuda.h>      // types only: the one function is looked up at run time
 
