@@ -333,10 +333,27 @@ static bool stream_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, StreamGe
   uint32_t cl = 1;
   while (cl < 16 && cl * 2 * g.cb <= kStreamRecords &&
          (wave * unit_bytes / cl > kStreamWindow || (g.units * cl * 2 <= most && N / (cl * 2) >= g.groups * least))) cl *= 2;
+  // A wave and less than a third of another: the rest of the blocks costs most of a second wave.  Another unit and cluster may make
+  // nearly a whole one, with nearly all threads.  Forward / backward, us, before and after: [128,2048,7,7] 512 and 412 blocks 26.4 / 33.0 and
+  // 21.2 / 33.0 (backward in three waves either way), [64,2048,7,7] 17.9 / 25.8 and 15.4 / 20.5, [32,2048,7,7] 11.4 / 15.4 and 10.0 / 13.8,
+  // [150,1000,6,6] 500 and 400 blocks 16.8 / 22.2 and 12.7 / 17.9.
+  uint32_t run = L4;      // vectors
+  if (!split && g.units * cl > wave && g.units * cl * 3 <= wave * 4 && g.groups * L4 > 192) {      // (of fewer threads four blocks are resident)
+    uint32_t most_threads = wave * kStreamThreads * 25 / 32;
+    for (uint32_t cb = q; cb <= C && cb <= kStreamChannels && (uint64_t)cb * dim0 <= 4 * kStreamThreads; cb += q) {
+      const uint32_t V = cb * dim0 / 4, units = ceil_div_u32(C, cb), groups = kStreamThreads / V < N ? kStreamThreads / V : N;
+      if (cb * dim0 < 128) continue;
+      for (uint32_t n = 1; n <= 8 && n * cb <= kStreamRecords && N / n >= groups * least; n *= 2)
+        if (units * n <= wave && units * n * groups * V > most_threads && wave * (16ull * V * N * (dir == 1 ? 2 : 1)) / n <= kStreamWindow) {
+          most_threads = units * n * groups * V;
+          cl = n; run = V; g.cb = cb; g.units = units; g.groups = groups;
+        }
+    }
+  }
   g.cluster = cl;
   g.rows = ceil_div_u32(N, cl);
   if (g.groups > g.rows) g.groups = g.rows;
-  g.threads = (g.groups * L4 + 31) / 32 * 32;
+  g.threads = (g.groups * run + 31) / 32 * 32;
   g.inv_count = 1.0 / ((double)dim0 * (double)N);
   return true;
 }
