@@ -1,0 +1,40 @@
+"""Layers whose first choice of unit and cluster makes one wave of blocks and less than a third of another: the streaming kernel
+takes another unit and cluster there.  Its geometry, and its results where the last unit is narrower, the samples do not divide
+by the blocks of a cluster, or one row of a unit takes a whole block."""
+import numpy as np
+import pytest
+
+from tests.test_gpu_fused import run_fused
+from tests.test_gpu_random_shapes import run_add_act
+from tests.test_serving_kernel import stream_geometry
+from tests.util import check_layer_own_mask, make_inputs
+
+SHAPES = [(33, 2048, 7, 7), (64, 2000, 5, 5), (35, 2044, 7, 7), (302, 233, 10, 10), (36, 482, 14, 14), (313, 911, 4, 4)]
+WAVE = 3 * 148                          # blocks of 256 threads that the device holds
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_one_wave_of_blocks(shape):
+    n, c, d0 = shape[0], shape[1], shape[2] * shape[3]
+    g = stream_geometry(shape, 0)
+    assert g["applies"] == 1 and g["units"] * g["cluster"] <= WAVE, g
+    assert g["cb"] * d0 % 4 == 0 and g["cb"] <= 128 and g["cb"] * g["cluster"] <= 1024 and g["units"] == -(-c // g["cb"])
+    assert g["cluster"] in (1, 2, 4, 8) and g["cluster"] * g["rows"] >= n >= g["rows"] >= g["groups"] >= 1
+    assert 192 < g["groups"] * g["cb"] * d0 // 4 <= g["threads"] <= 256
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", SHAPES)
+def test_results(shape):
+    from anode_b200 import ops
+    ops.set_kernel("stream")
+    try:
+        assert [ops.serving_kernel(shape, d, residual=r) for r in (False, True) for d in (0, 1)] == ["stream"] * 4
+        d = make_inputs(shape, seed=sum(shape), loc=3.0, scale=2.0)
+        got, _ = run_fused(ops, d)
+        check_layer_own_mask(d, got, "%r " % (shape,))
+        res = np.random.default_rng(5).standard_normal(shape).astype(np.float32)
+        got = run_add_act(ops, d, res, 0.1)
+        check_layer_own_mask(d, got, "%r residual " % (shape,), residual=res, slope=0.1)
+    finally:
+        ops.set_kernel("auto")
