@@ -283,7 +283,13 @@ bool chan_applies(const FusedArgs &a, int dir, bool aligned)
 // the teams take more than one wave of blocks, so that their load, exchange and store come twice: backward passes and the
 // residual epilogue, us here and on the streaming kernel: residual backward [103,304,53] 15.2 and 8.8, residual forward
 // [115,704,29] 11.8 and 7.4, backward [230,384,31] 13.7 and 8.8; but one wave, backward [19,728,145] 8.0 and 9.4, few
-// samples, [15,1516,130] 10.8 and 12.5, clusters of sixteen, [336,212,29] 8.7 and 12.9.  Rows of 1 - 3 floats, which the
+// samples, [15,1516,130] 10.8 and 12.5, clusters of sixteen, [336,212,29] 8.7 and 12.9.  With 20 to 31 samples a block of the
+// streaming kernel has few rows to stream, and only grids of one wave without clusters of four gain: backward / residual forward
+// [31,320,222] 14.2 / 14.7 and 10.8 / 9.4, [28,15964,5] 17.7 / 19.3 and 12.2 / 10.8, [27,1376,67] 13.6 / 14.0 and 11.6 / 10.4, but
+// [31,6844,14], 685 blocks, 13.9 / 15.4 and 15.8 / 15.8, [27,5376,17], clusters of four, 12.9 / 14.1 and 15.8 / 14.7.  The residual
+// backward, three tensors a thread, stalls in these teams at any number of waves: from 20 samples and a million elements it goes,
+// [30,948,39], 1.1 M, 13.4 and 8.7, [81,680,35] 15.9 and 11.7, [28,340,218] 26.1 and 12.5, [31,6844,14] 27.1 and 19.2, but
+// [20,848,43], 0.7 M, 6.5 and 6.4, [181,168,21], 0.6 M, 7.1 and 7.9.  Rows of 1 - 3 floats, which the
 // threads fetch from far apart, on the shared-memory kernel: [1024,512,3] residual backward 25.8 and 18.5, [1540,632,2]
 // backward 24.4 and 18.7, [1457,828,1] residual forward 23.6 and 20.6.
 // Backward passes and the residual epilogue of large layers of medium and long aligned rows go to the tiled kernel although a
@@ -303,8 +309,8 @@ constexpr uint64_t kChanTiled = 16u << 20, kChanTiledExtra = 18u << 20, kChanTil
 constexpr uint32_t kChanBandRow = 320;
 constexpr uint64_t kChanBand[2][2] = {{28000000, 18000000}, {18000000, 18000000}};      // [direction][residual]
 constexpr uint64_t kChanLarge = 8u << 20, kChanLargeScalar = 3u << 20, kChanLargeExtra = 5u << 20;
-constexpr uint64_t kChanWaves = 1500000, kChanShortest = 1200000;
-constexpr uint32_t kChanFewSamples = 32;
+constexpr uint64_t kChanWaves = 1500000, kChanShortest = 1200000, kChanShortestExtra = 1000000;
+constexpr uint32_t kChanFewSamples = 32, kChanFewestSamples = 20;
 constexpr uint32_t kChanLongRow = 300;
 bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
 {
@@ -325,14 +331,20 @@ bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
            !(tiled_ok && ((dir == 0 && !extra) || tiled_takes(a.plan.dim0, elements, dir, extra)));
   }
   if (elements < kChanLargeScalar) {
-    if ((dir == 0 && !extra) || elements < kChanShortest) return true;
+    const bool extra_bwd = extra && dir == 1 && a.plan.dim0 >= 4;
+    if ((dir == 0 && !extra) || elements < (extra_bwd ? kChanShortestExtra : kChanShortest)) return true;
     if (a.plan.dim0 < 4) {
       const uint32_t blocks = segres_blocks(a, dir, aligned);
       return blocks == 0 || blocks > 2 * sm_count();
     }
     const uint64_t places = (uint64_t)sm_count() * (2 * kChanThreads / g.threads);
-    if (elements < kChanWaves || a.plan.N < kChanFewSamples || (uint64_t)a.plan.C * g.cluster <= places) return true;
-    const uint32_t cluster = stream_cluster(a, dir, aligned);
+    const bool waves = elements >= kChanWaves && a.plan.N >= kChanFewSamples && (uint64_t)a.plan.C * g.cluster > places;
+    uint32_t blocks = 0;
+    const uint32_t cluster = stream_cluster(a, dir, aligned, blocks);
+    if (!waves) {
+      if (a.plan.N < kChanFewestSamples || !stream_preferred(a, dir, aligned, tiled_ok)) return true;
+      if (!extra_bwd && (elements < kChanWaves || (uint64_t)a.plan.C * g.cluster <= places || cluster > 2 || blocks > 3 * sm_count())) return true;
+    }
     return cluster == 0 || cluster > 8;
   }
   if (stream_preferred(a, dir, aligned, tiled_ok)) return false;

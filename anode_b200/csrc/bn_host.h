@@ -58,7 +58,7 @@ bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok);
 int launch_chan(FusedArgs &a, int dir, bool aligned, cudaStream_t stream);
 // the streaming cluster kernel for large layers of short rows (bn_stream.cu); one GPU
 bool stream_applies(const FusedArgs &a, int dir, bool aligned);
-uint32_t stream_cluster(const FusedArgs &a, int dir, bool aligned);
+uint32_t stream_cluster(const FusedArgs &a, int dir, bool aligned, uint32_t &blocks);
 bool stream_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok);
 int launch_stream(FusedArgs &a, int dir, cudaStream_t stream);
 // its form for the largest of them (bn_band.cu): the geometry of a shape where it is taken, and of a prepared call

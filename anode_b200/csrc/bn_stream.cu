@@ -358,11 +358,13 @@ static bool stream_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, StreamGe
   return true;
 }
 
-// Blocks of a cluster for this call; 0 where the kernel does not apply.
-uint32_t stream_cluster(const FusedArgs &a, int dir, bool aligned)
+// Blocks of a cluster, and of the grid, for this call; 0 where the kernel does not apply.
+uint32_t stream_cluster(const FusedArgs &a, int dir, bool aligned, uint32_t &blocks)
 {
   StreamGeom g;
-  return stream_applies(a, dir, aligned) && stream_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, g) ? g.cluster : 0u;
+  if (!stream_applies(a, dir, aligned) || !stream_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, g)) return 0u;
+  blocks = g.units * g.cluster;
+  return g.cluster;
 }
 
 bool stream_applies(const FusedArgs &a, int dir, bool aligned)

@@ -1,12 +1,13 @@
 """Layers whose first choice of unit and cluster makes one wave of blocks and less than a third of another: the streaming kernel
 takes another unit and cluster there.  Its geometry, and its results where the last unit is narrower, the samples do not divide
-by the blocks of a cluster, or one row of a unit takes a whole block."""
+by the blocks of a cluster, or one row of a unit takes a whole block; and the small layers of
+scalar rows that come to it from the register-resident kernel."""
 import numpy as np
 import pytest
 
 from tests.test_gpu_fused import run_fused
 from tests.test_gpu_random_shapes import run_add_act
-from tests.test_serving_kernel import stream_geometry
+from tests.test_serving_kernel import routes, stream_geometry
 from tests.util import check_layer_own_mask, make_inputs
 
 SHAPES = [(33, 2048, 7, 7), (64, 2000, 5, 5), (35, 2044, 7, 7), (302, 233, 10, 10), (36, 482, 14, 14), (313, 911, 4, 4)]
@@ -38,3 +39,30 @@ def test_results(shape):
         check_layer_own_mask(d, got, "%r residual " % (shape,), residual=res, slope=0.1)
     finally:
         ops.set_kernel("auto")
+
+
+# Rows of one float at a time in the register-resident kernel, 1 - 3 M elements: (shape, routes of routes())
+LINES = [((25, 932, 1, 45), ("register",) * 3 + ("stream",)),         # one wave of teams: the residual backward alone
+         ((20, 848, 1, 43), ("register",) * 4),                       # below a million elements
+         ((19, 1496, 1, 57), ("register",) * 4),                      # fewer than twenty samples
+         ((29, 1248, 1, 57), ("register", "stream", "stream", "stream")),
+         ((25, 932, 1, 130), ("register", "register", "register", "stream")),     # two waves of the streaming kernel's blocks
+         ((30, 520, 1, 145), ("register", "stream", "stream", "stream")),
+         ((300, 188, 1, 23), ("register",) * 3 + ("stream",))]
+
+
+@pytest.mark.parametrize("shape,want", LINES)
+def test_small_layers_of_scalar_rows(shape, want):
+    assert routes(shape) == want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [s for s, w in LINES if "stream" in w])
+def test_results_of_small_layers_of_scalar_rows(shape):
+    from anode_b200 import ops
+    d = make_inputs(shape, seed=sum(shape), loc=1.0, scale=2.0)
+    got, _ = run_fused(ops, d)
+    check_layer_own_mask(d, got, "%r " % (shape,))
+    res = np.random.default_rng(7).standard_normal(shape).astype(np.float32)
+    got = run_add_act(ops, d, res, 0.0)
+    check_layer_own_mask(d, got, "%r residual " % (shape,), residual=res, slope=0.0)
