@@ -367,12 +367,12 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
       w.next();
       if (kind == 0 && DIR == 1 && s + 1 < mine) params(w.unit);
     }
-    // after an abort: wait (bounded) for copies that were issued but will not be consumed
-    if (!ok && lane == 0) {
+    // wait (bounded) for every copy that was issued: after an abort, of this warp or, now or later, of another, nobody else may
+    if (lane == 0) {
       const uint32_t first = k > g.slots ? k - g.slots : 0;
       for (uint32_t kk = first; kk < k; ++kk) {
         const long long t0 = clock64();
-        while (!mbar_test(&ctl->full[kk % g.slots], (kk / g.slots) & 1u) && clock64() - t0 < kWaitCycles / 8) {}
+        while (!mbar_try(&ctl->full[kk % g.slots], (kk / g.slots) & 1u) && clock64() - t0 < kDrainCycles) {}
       }
     }
   } else if (warp == kBandWarps + 1) {

@@ -71,6 +71,9 @@ __device__ __forceinline__ uint64_t policy_drop()
   return p;
 }
 
+// How long a block that leaves waits for its own copies into shared memory, in SM clock cycles (about 0.2 s); they take microseconds.
+constexpr long long kDrainCycles = 375000000ll;
+
 // ---- packs of VEC floats ----------------------------------------------------------------
 template <int VEC> struct Pack;
 template <> struct Pack<4> {

@@ -24,13 +24,6 @@ __device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, uint32_t
 {
   asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ bool mbar_test(unsigned long long *bar, uint32_t parity)
-{
-  uint32_t ok;
-  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-               : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-  return ok != 0;
-}
 __device__ __forceinline__ bool mbar_try(unsigned long long *bar, uint32_t parity)
 {
   uint32_t ok;

@@ -602,12 +602,12 @@ __global__ void __launch_bounds__(kResThreads, 1) bn_resident_kernel(const Fused
       if (lane == 0) { __threadfence_block(); ctl->issued = nload; }
       return true;
     });
-    // after an abort: wait (bounded) for copies that were issued but will not be consumed
-    if (ctl->abort && lane == 0) {
+    // wait (bounded) for every copy that was issued: after an abort, of this warp or, now or later, of another, nobody else may
+    if (lane == 0) {
       for (uint32_t s = 0; s < g.Q; ++s) {
         if (!((used >> s) & 1ull)) continue;
         const long long t0 = clock64();
-        while (!mbar_test(&ctl->full[s], (uint32_t)((lpar >> s) & 1ull)) && clock64() - t0 < limit / 8) {}
+        while (!mbar_try(&ctl->full[s], (uint32_t)((lpar >> s) & 1ull)) && clock64() - t0 < kDrainCycles) {}
       }
     }
   } else if (warp == W + 1) {
