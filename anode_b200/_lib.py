@@ -104,6 +104,7 @@ SIGNATURES = {
     "anode_gpu_batch_norm_fused_kernel_kind": (c_int, _D + [c_int]),
     "anode_gpu_batch_norm_add_act_fused_kernel_kind": (c_int, _D + [c_int]),
     "anode_gpu_batch_norm_fused_set_wait_limit_ms": (c_int, [u32]),
+    "anode_gpu_batch_norm_fused_set_wait_limit_cycles": (c_int, [u32]),
     "anode_gpu_batch_norm_fused_set_kernel": (c_int, [c_int]),
     "anode_gpu_batch_norm_resident_plan": (c_int, _D + [u32, ctypes.POINTER(u32)]),
     "anode_gpu_batch_norm_resident_schedule":

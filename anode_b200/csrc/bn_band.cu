@@ -34,6 +34,7 @@ struct BandCtl {
   unsigned long long res_full[kBandQ], res_empty[kBandQ], coef_full[kBandQ], coef_empty[kBandQ];
   volatile uint32_t abort;
   uint32_t last_block, parity, tmem;
+  long long limit;       // of the waits (FusedArgs::wait_cycles)
 };
 static_assert(sizeof(BandCtl) <= kBandCtlBytes, "BandCtl outgrew the room reserved for it");
 
@@ -85,7 +86,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
       mbar_init(&ctl->res_full[i], kBandWarps); mbar_init(&ctl->res_empty[i], 1);
       mbar_init(&ctl->coef_full[i], 1); mbar_init(&ctl->coef_empty[i], kBandWarps);
     }
-    ctl->abort = 0; ctl->last_block = 0; ctl->parity = *parity & 1u;
+    ctl->abort = 0; ctl->last_block = 0; ctl->parity = *parity & 1u; ctl->limit = a.wait_cycles;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -464,7 +465,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
           uint32_t stop = 0;
           if (lane == 0) {
             if (ctl->abort) stop = 1;
-            else if (clock64() - t0 > kWaitCycles) { atomicOr(status, ANODE_ST_WAIT_STATS); ctl->abort = 1; stop = 1; }
+            else if (clock64() - t0 > 2 * a.wait_cycles) { atomicOr(status, ANODE_ST_WAIT_STATS); ctl->abort = 1; stop = 1; }
           }
           if (__shfl_sync(0xffffffffu, stop, 0)) { ok = false; break; }
         }

@@ -22,7 +22,6 @@ namespace anode_b200 {
 
 enum : uint32_t { MODE_FUSED = 0, MODE_STATS = 1, MODE_APPLY = 2 };
 
-constexpr uint32_t kSpinLimit = 1u << 20;   // about a second of polling, then give up
 constexpr uint32_t kSegMaxFloats = 4 * kThreads * kSegSlots;
 constexpr uint32_t kSegMaxChannels = 256;
 
@@ -686,10 +685,11 @@ __global__ void __launch_bounds__(kThreads) bn_pipeline_kernel(const FusedArgs a
       if (a.mode == MODE_FUSED) {
         if (tid == 0) {
           uint32_t ok = 1, it = 0;
+          const long long t0 = clock64();
           while (ld_acquire_gpu(ready + tr.unit) == 0u) {
             __nanosleep(100);
             ++it;
-            if (it > kSpinLimit) { atomicOr(status, ANODE_ST_WAIT_STATS); ok = 0; break; }
+            if (clock64() - t0 > 2 * a.wait_cycles) { atomicOr(status, ANODE_ST_WAIT_STATS); ok = 0; break; }
             if ((it & 255u) == 0u && ld_relaxed_gpu(status) != 0u) { ok = 0; break; }
           }
           sc.go = ok;

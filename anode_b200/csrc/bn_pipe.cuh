@@ -6,7 +6,6 @@
 
 namespace anode_b200 {
 
-constexpr long long kWaitCycles = 3000000000ll;      // about 1.5 s at 2 GHz
 constexpr uint32_t kBackoffNs = 100;
 
 // ---- mbarrier / bulk-copy primitives --------------------------------------------------------
@@ -34,7 +33,8 @@ __device__ __forceinline__ bool mbar_try(unsigned long long *bar, uint32_t parit
   return ok != 0;
 }
 // Bounded wait.  Returns false (after raising the abort flag) when the barrier did not flip in time
-// or when another role already gave up.
+// or when another role already gave up.  The bound is three times ctl->limit, the caller's one: a barrier hangs on the waits
+// for words and records (twice the limit, and once), which should run out first and say in the status word what was missing.
 template <typename Ctl>
 __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, uint32_t parity, Ctl *ctl, uint32_t *status, uint32_t bit)
 {
@@ -47,7 +47,7 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, uint32_t pari
     __nanosleep(kBackoffNs);
     if ((++it & 15u) == 0u) {
       if (ctl->abort) return false;
-      if (clock64() - t0 > kWaitCycles) {
+      if (clock64() - t0 > 3 * ctl->limit) {
         atomicOr(status, bit);
         ctl->abort = 1;
         return false;

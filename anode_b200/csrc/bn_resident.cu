@@ -722,12 +722,13 @@ __global__ void __launch_bounds__(kResThreads, 1) bn_resident_kernel(const Fused
 }  // namespace res
 
 // ---- host side ----------------------------------------------------------------------------------------
-static std::atomic<uint32_t> g_wait_ms{1500};
+// device clock64 ticks at the SM clock (about 2 GHz at most): bounds in milliseconds are approximate by design
+constexpr long long kCyclesPerMs = 2000000ll;
+static std::atomic<long long> g_wait_cycles{1500 * kCyclesPerMs};
 
 long long wait_limit_cycles()
 {
-  // device clock64 ticks at the SM clock (about 2 GHz at most): the bound is approximate by design
-  return (long long)g_wait_ms.load(std::memory_order_relaxed) * 2000000ll;
+  return g_wait_cycles.load(std::memory_order_relaxed);
 }
 
 // Planner inputs, from measurements on B200: bytes of reduce work that should separate the end of a
@@ -805,7 +806,15 @@ using namespace anode_b200;
 extern "C" int anode_gpu_batch_norm_fused_set_wait_limit_ms(uint32_t ms)
 {
   if (ms == 0) return ANODE_E_DIMS;
-  g_wait_ms.store(ms, std::memory_order_relaxed);
+  g_wait_cycles.store((long long)ms * kCyclesPerMs, std::memory_order_relaxed);
+  return ANODE_OK;
+}
+
+// ---- diagnostics: a bound so short that waits run out (every kernel drains and leaves then) --------------
+extern "C" int anode_gpu_batch_norm_fused_set_wait_limit_cycles(uint32_t cycles)
+{
+  if (cycles == 0) return ANODE_E_DIMS;
+  g_wait_cycles.store((long long)cycles, std::memory_order_relaxed);
   return ANODE_OK;
 }
 

@@ -58,6 +58,7 @@ struct RingCtl {
   uint32_t last_block;
   uint32_t parity;       // which of the two tagged-partial buffers this launch uses
   uint32_t tmem;         // base address of the block's tensor memory (g.keep_slots > 0)
+  long long limit;       // of the waits (FusedArgs::wait_cycles)
 };
 static_assert(sizeof(RingCtl) <= kRingCtlBytes, "RingCtl outgrew the room reserved for it");
 
@@ -589,7 +590,7 @@ __device__ __forceinline__ bool pull_merge_unit(const FusedArgs &a, RingCtl *ctl
       uint32_t stop = 0;
       if (lane == 0) {
         if (ctl->abort) stop = 1;
-        else if (clock64() - t0 > kWaitCycles) { atomicOr(status, ANODE_ST_WAIT_STATS); ctl->abort = 1; stop = 1; }
+        else if (clock64() - t0 > 2 * a.wait_cycles) { atomicOr(status, ANODE_ST_WAIT_STATS); ctl->abort = 1; stop = 1; }
       }
       if (__shfl_sync(0xffffffffu, stop, 0)) return false;
     }
@@ -718,7 +719,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
     for (uint32_t i = 0; i < g.slots; ++i) { mbar_init(&ctl->full[i], 1); mbar_init(&ctl->empty[i], kCWarps); }
     for (uint32_t i = 0; i < kResQ; ++i) { mbar_init(&ctl->res_full[i], kCWarps); mbar_init(&ctl->res_empty[i], 1); }
     for (uint32_t i = 0; i < kCoefQ; ++i) { mbar_init(&ctl->coef_full[i], 1); mbar_init(&ctl->coef_empty[i], kCWarps); }
-    ctl->abort = 0; ctl->last_block = 0;
+    ctl->abort = 0; ctl->last_block = 0; ctl->limit = a.wait_cycles;
     ctl->parity = *ws_u32(a, g.hdr + 4) & 1u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

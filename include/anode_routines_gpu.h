@@ -203,7 +203,8 @@ void anode_gpu_positive_clip_flat_map_bwd_f32(
 int anode_gpu_batch_norm_fused_set_kernel(int kernel);
 
 /* Bound of every wait inside the kernels (for a channel's statistics, for another GPU's records), in
- * milliseconds of SM clock at 2 GHz; default 1500.  A wait that runs out sets ANODE_ST_WAIT_* and
+ * milliseconds of SM clock at 2 GHz; default 1500.  (Waits that hang on other waits: two and three times
+ * that, so that the status word names what was missing first.)  A wait that runs out sets ANODE_ST_WAIT_* and
  * ANODE_ST_ABORTED in the status word, the kernel drains and returns, and the workspace has to be
  * re-initialised before its next use.  Process-wide; applies to calls made afterwards. */
 int anode_gpu_batch_norm_fused_set_wait_limit_ms(uint32_t ms);

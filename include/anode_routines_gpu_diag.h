@@ -74,6 +74,9 @@ int anode_gpu_batch_norm_tiled_keep(uint32_t dim0, uint32_t dim1, uint32_t dim2,
  * `dir` of a call on 16-byte aligned tensors, with or without the residual epilogue; 0 where it does not apply. */
 uint32_t anode_gpu_batch_norm_tiled_last_piece(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual);
 
+/* anode_gpu_batch_norm_fused_set_wait_limit_ms in SM clock cycles, for tests of what follows when a wait inside a kernel runs out. */
+int anode_gpu_batch_norm_fused_set_wait_limit_cycles(uint32_t cycles);
+
 /* Plan of the slice-resident kernel for `planes` tensors per shared-memory slot.  out (16 values): applies,
  * rows per piece, parts per row, floats per part, pieces per channel, blocks per team, teams, grid, pieces
  * per block and channel, slot bytes, slots, resident-ring slots, streaming-ring slots, resident pieces per

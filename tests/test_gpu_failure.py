@@ -76,6 +76,55 @@ def test_wait_for_an_absent_peer_runs_out_and_the_workspace_recovers(short_waits
     check_layer(got, truth, d["x"], d["gamma"], d["beta"], "after recovery ")
 
 
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("kernel,shape", [("stream", (1283, 244, 7, 7)), ("stream", (256, 512, 14, 14)), ("tiled", (64, 95, 55, 55)),
+                                          ("tiled", (64, 64, 56, 56))])
+def test_a_wait_that_runs_out_leaves_no_copy_and_no_state_behind(kernel, shape, residual):
+    """A bound of one cycle: the first poll for a channel's words finds none, in every block, with copies on their way into the
+    slots.  The call says so, returns at once (the default bound is 1.5 s), and after a re-initialisation the workspace serves."""
+    from anode_b200 import _lib, ops
+    from tests.test_gpu_band import inputs, run
+    d = inputs(shape, 3)
+    c, x = shape[1], d["x"]
+    ops.set_kernel(kernel)
+    try:
+        want, ws = run(ops, d, residual, 0.1)
+        z = [torch.zeros(c, device="cuda") for _ in range(4)]
+        y, dx, dres = (torch.empty_like(x) for _ in range(3))
+        if residual:
+            op = ops.BatchNormalize2dAddActFusedOp
+            calls = [lambda: op.apply([0, 1], 1e-5, 0.1, x, d["res"], y, z[0], z[1], z[2], z[3], d["gamma"], d["beta"], 0.1, ws),
+                     lambda: op.adjoint([0, 1], d["dy"], x, want["y"], want["mean"], want["var"], dx, dres, d["gamma"], d["beta"], z[0], z[1], 0.1,
+                                        workspace=ws)]
+        else:
+            calls = [lambda: ops.BatchNormalize2dFusedOp.apply([0, 1], 1e-5, 0.1, x, y, z[0], z[1], z[2], z[3], d["gamma"], d["beta"], workspace=ws, neg_slope=0.1),
+                     lambda: ops.BatchNormalize2dBwdFusedOp.apply([0, 1], d["dy"], x, want["mean"], want["var"], dx, d["gamma"], d["beta"], z[0], z[1],
+                                                                  workspace=ws, neg_slope=0.1)]
+        for call in calls:
+            t0, t1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            assert _lib.load().anode_gpu_batch_norm_fused_set_wait_limit_cycles(1) == 0
+            t0.record()
+            call()
+            t1.record()
+            torch.cuda.synchronize()
+            ops.set_wait_limit_ms(1500)
+            assert ws.status() == WAIT_STATS | ABORTED
+            assert t0.elapsed_time(t1) < 500.0
+            ws.reset()
+        for _ in range(2):
+            again, _ = run(ops, d, residual, 0.1, ws)
+            assert all(torch.equal(again[k], want[k]) for k in want)
+    finally:
+        ops.set_wait_limit_ms(1500)
+        ops.set_kernel("auto")
+
+
+def test_the_wait_limit_is_never_nothing():
+    from anode_b200 import _lib
+    lib = _lib.load()
+    assert lib.anode_gpu_batch_norm_fused_set_wait_limit_ms(0) == -2 and lib.anode_gpu_batch_norm_fused_set_wait_limit_cycles(0) == -2      # ANODE_E_DIMS
+
+
 def test_exchange_only_communicator_refuses_what_it_cannot_do():
     from anode_b200 import _lib, sync
     lib = _lib.load()
