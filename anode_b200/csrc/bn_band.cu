@@ -9,10 +9,14 @@
 //   consumer warps    (8) a thread keeps its column's vectors of a tile, at most 16 per tensor, sums them up (two floats per
 //                     instruction) and leaves them in tensor memory (forward: x; backward: x - mean and dz); later reads them
 //                     back, applies the coefficients and stores
-//   delivery warp     folds the threads' sums of a tile to channels and stores one 8-byte word per channel and tile, forward (mean,
-//                     M2), backward (sum dz, sum dz*(x-mean)), never zero; no counter, fence or atomic
-//   coefficient warp  polls the words of the unit that is applied next until none is zero and merges them in a fixed order in
-//                     double precision (bit-identical in every block); the block of a unit's first tile writes its results
+//   delivery warp     folds the threads' sums of a tile to channels and stores one pair of doubles per channel and tile, forward
+//                     (sum x, sum x^2), backward (sum dz, sum dz*(x-mean)), as two words that are never zero; no counter, fence or atomic
+//   coefficient warp  polls the words of the unit that is applied next until none is zero and merges them in a fixed order
+//                     (bit-identical in every block); the block of a unit's first tile writes its results
+// Precision: at most 16 samples of a column are added up in f32, about a shift; everything beyond that is in double precision, as in the
+// streaming kernel, whose f32 sums are longer.  Relative error against float64 (2-norm over the channels, geometric mean over nine shapes and three
+// distributions), streaming kernel and this one: mean 4.6e-8 and 3.9e-8, variance 2.89e-8 and 2.86e-8, dgamma 2.2e-7 and 2.0e-7, dbeta
+// 1.6e-7 and 1.2e-7.  (With f32 words and f32 sums of four columns: 5.8e-8, 3.13e-8, 2.2e-7, 1.7e-7.)
 // Two buffers of words alternate launch by launch: a delivery zeroes its word of the other one.  Every wait is bounded; one that
 // runs out sets a status bit and the block drains and leaves.  The launch is cooperative and takes the SM's whole shared memory,
 // so that no other block holds columns of tensor memory or waits for them.
@@ -62,10 +66,34 @@ struct BandWalk {
   }
 };
 
-__device__ __forceinline__ unsigned long long band_word(float lo, float hi)
+// What the consumer threads leave of a tile: [thread] its sums for its first channel, [group][channel] those of the vector that begins in
+// the channel before.
+struct BandSums {
+  double2 *first, *second;
+  __device__ __forceinline__ BandSums(unsigned char *sm, const BandGeom &g, uint32_t q)
+  {
+    unsigned char *at = sm + g.off_res + q * g.res_bytes;
+    first = reinterpret_cast<double2 *>(at); second = reinterpret_cast<double2 *>(at + g.off_second);
+  }
+};
+
+// A channel's pair of doubles for a tile: two 8-byte words that are never all zero bits ("not delivered"): a zero has its sign set.
+struct BandWord { unsigned long long lo, hi; };
+static_assert(sizeof(BandWord) == kBandWordBytes, "the geometry's room for a word");
+__device__ __forceinline__ unsigned long long band_bits(double v)
 {
-  const unsigned long long w = ((unsigned long long)__float_as_uint(hi) << 32) | __float_as_uint(lo);
-  return w ? w : 1ull << 32;      // never zero ("not delivered")
+  const long long b = __double_as_longlong(v);
+  return b ? (unsigned long long)b : 1ull << 63;
+}
+__device__ __forceinline__ void st_word(BandWord *p, double lo, double hi)
+{
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(band_bits(lo)), "l"(band_bits(hi)) : "memory");
+}
+__device__ __forceinline__ BandWord ld_word(const BandWord *p)
+{
+  BandWord w;
+  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w.lo), "=l"(w.hi) : "l"(p) : "memory");
+  return w;
 }
 
 template <int DIR, bool EXTRA>
@@ -107,84 +135,82 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
     const uint32_t pitch = g.box4 * 16, box = v / g.box4;
     const uint32_t off_s = box * g.box_bytes + grp * pitch + (v - box * g.box4) * 16, step_s = g.groups * pitch;
     const uint32_t off_g = grp * rs + 4 * v, step_g = g.groups * rs;
-    // places of a channel's elements that make the shift of its sums
-    auto place = [&](uint32_t f) { const uint32_t j = f / (g.box4 * 4); return j * g.box_bytes + (f - j * g.box4 * 4) * 4; };
-    uint32_t kA[3], kB[3];
-    if (DIR == 0) {
-      const uint32_t at[3] = {dim0 / 6, dim0 / 2, dim0 - 1 - dim0 / 6};
-#pragma unroll
-      for (int i = 0; i < 3; ++i) { kA[i] = place(chA * dim0 + at[i]); kB[i] = place(chB * dim0 + at[i]); }
-    }
     const float slope = a.neg_slope;
     const uint32_t tm0 = ctl->tmem + ((warp & 3u) << 21) + (warp >> 2) * (kTmemCols * 4 / kBandWarps), tm_step = g.vpt * 4 * kKept;
     // a value per channel, for the thread's four floats
     const bool b1 = eB > 1, b2 = eB > 2, b3 = eB > 3;
     auto spread = [&](float A, float B) { return Quad{pair(A, b1 ? A : B), pair(b2 ? A : B, b3 ? A : B)}; };
-    // the thread's sums for its two channels
-    auto fold = [&](const f32x2 &sa, const f32x2 &sb, const f32x2 &qa, const f32x2 &qb) {
-      const float2 s0 = split(sa), s1 = split(sb), q0 = split(qa), q1 = split(qb);
-      float4 o;
-      o.x = (s0.x + (b1 ? s0.y : 0.f)) + ((b2 ? s1.x : 0.f) + (b3 ? s1.y : 0.f));
-      o.y = (q0.x + (b1 ? q0.y : 0.f)) + ((b2 ? q1.x : 0.f) + (b3 ? q1.y : 0.f));
-      o.z = (b1 ? 0.f : s0.y) + ((b2 ? 0.f : s1.x) + (b3 ? 0.f : s1.y));
-      o.w = (b1 ? 0.f : q0.y) + ((b2 ? 0.f : q1.x) + (b3 ? 0.f : q1.y));
-      return o;
+    // the thread's sums for its two channels: its columns' own sums are in f32, 16 samples at most, everything beyond them is in double
+    // precision, as in the streaming kernel.  Forward: of x and x^2 about zero, from n samples' sums about K
+    auto fold = [&](const BandSums &part, uint32_t n, const Quad &K, const f32x2 &sa, const f32x2 &sb, const f32x2 &qa, const f32x2 &qb) {
+      const float2 s0 = split(sa), s1 = split(sb), q0 = split(qa), q1 = split(qb), k0 = split(K.a), k1 = split(K.b);
+      double S[4] = {s0.x, s0.y, s1.x, s1.y}, Q[4] = {q0.x, q0.y, q1.x, q1.y};
+      if (DIR == 0) {
+        const double k[4] = {k0.x, k0.y, k1.x, k1.y}, cnt = n;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { Q[e] = fma(k[e], fma(cnt, k[e], 2.0 * S[e]), Q[e]); S[e] = fma(cnt, k[e], S[e]); }
+      }
+      part.first[tid] = make_double2((S[0] + (b1 ? S[1] : 0.0)) + ((b2 ? S[2] : 0.0) + (b3 ? S[3] : 0.0)),
+                                     (Q[0] + (b1 ? Q[1] : 0.0)) + ((b2 ? Q[2] : 0.0) + (b3 ? Q[3] : 0.0)));
+      if (!b3 && live)
+        part.second[grp * g.cb + chB] = make_double2((b1 ? 0.0 : S[1]) + ((b2 ? 0.0 : S[2]) + S[3]), (b1 ? 0.0 : Q[1]) + ((b2 ? 0.0 : Q[2]) + Q[3]));
     };
     // One tile.  FULL: it has all its rows, so no vector is missing (what threads without a column read and add up is not used).
-    auto reduce = [&](auto full, uint32_t rows, uint32_t slot, uint32_t tm, float4 *part) {
+    auto reduce = [&](auto full, uint32_t rows, uint32_t slot, uint32_t tm, const BandSums &part) {
       constexpr bool FULL = decltype(full)::value;
       const uint32_t slot_off = g.off_slots + slot * g.slot_stride;
-      uint32_t ax = smem_u32(sm) + slot_off + off_s, r = grp;
+      uint32_t ax = smem_u32(sm) + slot_off + off_s;
       if constexpr (DIR == 0) {
-        // shift of the sums: per channel the median of three elements
-        float Ka, Kb;
-        {
-          const uint32_t r1 = rows / 2 * pitch, r2 = (rows - 1) * pitch;
-          const unsigned char *xs = sm + slot_off;
-          auto at = [&](uint32_t o) { return *reinterpret_cast<const float *>(xs + o); };
-          Ka = median3(at(kA[0]), at(kA[1] + r1), at(kA[2] + r2));
-          Kb = median3(at(kB[0]), at(kB[1] + r1), at(kB[2] + r2));
-          Ka = fabsf(Ka) < 1e36f ? Ka : 0.f; Kb = fabsf(Kb) < 1e36f ? Kb : 0.f;      // (an infinity is no shift)
-        }
-        const Quad Kq = spread(Ka, Kb), nK = spread(-Ka, -Kb);
+        Quad K = quad(0.f), nK = K;      // shift of the sums: per column the mean of its first four samples (or its first one)
         f32x2 sa = 0, sb = 0, qa = 0, qb = 0;
-        auto load = [&](Quad &x) {
-          if constexpr (FULL) x = lds_quad(ax);
-          else { x = Kq; if (r < rows) x = lds_quad(ax); r += g.groups; }
-          ax += step_s;
+        const uint32_t n = FULL ? g.vpt : grp < rows ? min(g.vpt, (rows - grp - 1) / g.groups + 1) : 0u;
+        auto there = [&](uint32_t i) { return FULL || i < n; };
+        auto load = [&](Quad &x, uint32_t i) { if (there(i)) x = lds_quad(ax); ax += step_s; };      // (a missing vector is the shift)
+        auto shift = [&](const Quad &sum, float inv) {
+          auto of = [&](const f32x2 &s) { const float2 t = split(s); return pair(fabsf(t.x) < 1e36f ? t.x * inv : 0.f, fabsf(t.y) < 1e36f ? t.y * inv : 0.f); };
+          K.a = of(sum.a); K.b = of(sum.b);      // (an infinity or a NaN is no shift, the sums show it)
+          nK.a = mul2(K.a, pair(-1.f, -1.f)); nK.b = mul2(K.b, pair(-1.f, -1.f));
         };
-        auto take = [&](const Quad &x) {
+        // (four samples' sums by themselves first, so that the thread's are rounded once per four of them)
+        auto take = [&](const Quad &x0, const Quad &x1, const Quad &x2, const Quad &x3) {
+          const f32x2 a0 = add2(x0.a, nK.a), a1 = add2(x1.a, nK.a), a2 = add2(x2.a, nK.a), a3 = add2(x3.a, nK.a);
+          const f32x2 c0 = add2(x0.b, nK.b), c1 = add2(x1.b, nK.b), c2 = add2(x2.b, nK.b), c3 = add2(x3.b, nK.b);
+          sa = add2(sa, add2(add2(a0, a1), add2(a2, a3))); sb = add2(sb, add2(add2(c0, c1), add2(c2, c3)));
+          qa = add2(qa, fma2(a3, a3, fma2(a2, a2, fma2(a1, a1, mul2(a0, a0))))); qb = add2(qb, fma2(c3, c3, fma2(c2, c2, fma2(c1, c1, mul2(c0, c0)))));
+        };
+        auto take1 = [&](const Quad &x) {
           const f32x2 da = add2(x.a, nK.a), db = add2(x.b, nK.b);
           sa = add2(sa, da); qa = fma2(da, da, qa); sb = add2(sb, db); qb = fma2(db, db, qb);
         };
         uint32_t i = 0;
         for (; i + 4 <= g.vpt; i += 4, tm += 16) {
-          Quad x0, x1, x2, x3;
-          load(x0); load(x1); load(x2); load(x3);
+          Quad x0 = K, x1 = K, x2 = K, x3 = K;
+          load(x0, i); load(x1, i + 1); load(x2, i + 2); load(x3, i + 3);
+          if (i == 0) {
+            shift(Quad{add2(add2(x0.a, x1.a), add2(x2.a, x3.a)), add2(add2(x0.b, x1.b), add2(x2.b, x3.b))}, FULL ? 0.25f : __fdividef(1.f, (float)min(n, 4u)));
+            if constexpr (!FULL) { if (!there(0)) x0 = K; if (!there(1)) x1 = K; if (!there(2)) x2 = K; if (!there(3)) x3 = K; }
+          }
           if constexpr (!FULL) __syncwarp();
           tmem_st(tm, x0, x1, x2, x3);
-          take(x0); take(x1); take(x2); take(x3);
+          take(x0, x1, x2, x3);
         }
         for (; i < g.vpt; ++i, tm += 4) {
-          Quad x0;
-          load(x0);
+          Quad x0 = K;
+          load(x0, i);
+          if (i == 0) shift(x0, 1.f);
           if constexpr (!FULL) __syncwarp();
           tmem_st(tm, x0);
-          take(x0);
+          take1(x0);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&ctl->empty[slot]);
-        if (live && grp == 0) {
-          float *kbox = reinterpret_cast<float *>(part + kBandConsumers);
-          if (4 * v == chA * dim0) kbox[chA] = Ka;
-          if (chB != chA) kbox[chB] = Kb;
-        }
-        part[tid] = fold(sa, sb, qa, qb);
+        fold(part, n, K, sa, sb, qa, qb);
       } else {
         const float4 *side = reinterpret_cast<const float4 *>(sm + g.off_side) + slot * kBandChannels;
         const float4 pA = side[chA], pB = side[chB];
         const Quad mean = spread(pA.x, pB.x), nmean = spread(-pA.x, -pB.x), scale = spread(pA.y, pB.y), beta = spread(pA.z, pB.z);
         f32x2 s1a = 0, s1b = 0, s2a = 0, s2b = 0;
+        [[maybe_unused]] uint32_t r = grp;
         // a missing vector is (mean, 0), which adds nothing
         auto load = [&](Quad &x, Quad &gy, Quad &y) {
           y = quad(0.f);
@@ -220,7 +246,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&ctl->empty[slot]);
-        part[tid] = fold(s1a, s1b, s2a, s2b);
+        fold(part, 0, mean, s1a, s1b, s2a, s2b);
       }
     };
     // alive: the thread has a column of this unit; base: the tile's first float, from which a thread's places are below 4 GB
@@ -260,7 +286,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
       } else {
         const Quad cB = spread(pA.w, pB.w), cC = spread(coef[2 * chA + 1].x, coef[2 * chB + 1].x);
         const bool acc = a.accumulate != 0;
-        unsigned char *dres = EXTRA && a.dres ? reinterpret_cast<unsigned char *>(a.dres + base) : nullptr;
+        [[maybe_unused]] unsigned char *dres = EXTRA && a.dres ? reinterpret_cast<unsigned char *>(a.dres + base) : nullptr;
         auto one = [&](const Quad &e, const Quad &z) {
           Quad o;
           o.a = fma2(scale.a, z.a, fma2(cB.a, e.a, cC.a)); o.b = fma2(scale.b, z.b, fma2(cB.b, e.b, cC.b));
@@ -296,7 +322,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
         bool ok = warp_wait(&ctl->res_empty[qres], rpar, ctl, status, ANODE_ST_WAIT_STATS);
         ok = ok && warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS);
         if (!ok) break;
-        float4 *part = reinterpret_cast<float4 *>(sm + g.off_res + qres * (kBandConsumers * 16 + 256));
+        const BandSums part(sm, g, qres);
         const uint32_t rows = N - red.k * g.rows, tm = tm0 + red_place * tm_step;
         if (rows >= g.rows) reduce(std::true_type{}, g.rows, slot, tm, part);
         else reduce(std::false_type{}, rows, slot, tm, part);
@@ -380,48 +406,41 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
     // ------------------------------------------------------------------ delivery warp
     const uint32_t lp = 1u << g.lane_shift, ci = lane >> g.lane_shift, sub = lane & (lp - 1u);
     const uint32_t v0 = ci * dim0 / 4, v1 = (ci * dim0 + dim0 - 1) / 4;      // the channel's first and last vector
-    unsigned long long *buf = reinterpret_cast<unsigned long long *>(a.ws + g.tag);
+    BandWord *buf = reinterpret_cast<BandWord *>(a.ws + g.tag);
     const size_t other = (size_t)g.total * g.cb;
-    unsigned long long *now = buf + (ctl->parity ? other : 0), *then = buf + (ctl->parity ? 0 : other);
+    BandWord *now = buf + (ctl->parity ? other : 0), *then = buf + (ctl->parity ? 0 : other);
     BandWalk w(g, b, G);
     uint32_t q = 0, qpar = 0;
     size_t at = (size_t)b * g.cb + ci;
     for (uint32_t j = 0; j < mine; ++j) {
       const bool has = ci < g.cb && w.unit * g.cb + ci < C;
       if (!warp_wait(&ctl->res_full[q], qpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
-      const float4 *part = reinterpret_cast<const float4 *>(sm + g.off_res + q * (kBandConsumers * 16 + 256));
+      const BandSums part(sm, g, q);
       double t1 = 0.0, t2 = 0.0;
-      float K = 0.f;
-      if (DIR == 0 && has) K = reinterpret_cast<const float *>(part + kBandConsumers)[ci];
-      // four of the lane's vectors at a time, their sums added in pairs: the loads are under way together and a quarter of the
-      // additions are in double precision (one vector after another in double precision: 2.5 us a tile, the kernel's bound)
+      // four of the lane's vectors at a time, their sums added in pairs: the loads are under way together (one vector after another:
+      // 2.5 us a tile, the kernel's bound)
       uint32_t vi = v0 + sub, gi = has && vi <= v1 ? 0 : g.groups;
       while (gi < g.groups) {
-        float2 p[4];
+        double2 p[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-          p[u] = make_float2(0.f, 0.f);
+          p[u] = make_double2(0.0, 0.0);
           if (gi < g.groups) {
             // (a vector that begins in the channel before holds this one's sums behind those)
-            p[u] = reinterpret_cast<const float2 *>(part + gi * g.L4 + vi)[4 * vi >= ci * dim0 ? 0 : 1];
+            p[u] = 4 * vi >= ci * dim0 ? part.first[gi * g.L4 + vi] : part.second[gi * g.cb + ci];
             vi += lp;
             if (vi > v1) { vi = v0 + sub; ++gi; }
           }
         }
-        t1 += (double)((p[0].x + p[1].x) + (p[2].x + p[3].x)); t2 += (double)((p[0].y + p[1].y) + (p[2].y + p[3].y));
+        t1 += (p[0].x + p[1].x) + (p[2].x + p[3].x); t2 += (p[0].y + p[1].y) + (p[2].y + p[3].y);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl->res_empty[q]);
       if (++q == kBandQ) { q = 0; qpar ^= 1u; }
       for (uint32_t o = lp >> 1; o > 0; o >>= 1) { t1 += __shfl_xor_sync(0xffffffffu, t1, o); t2 += __shfl_xor_sync(0xffffffffu, t2, o); }
       if (has && sub == 0) {
-        float lo = (float)t1, hi = (float)t2;
-        if (DIR == 0) {
-          const double m = t1 * (w.k + 1 == g.tiles ? g.inv_tail : g.inv_full);
-          lo = (float)((double)K + m); hi = (float)not_below_zero(t2 - t1 * m);
-        }
-        st_relaxed_gpu_u64(now + at, band_word(lo, hi));
-        then[at] = 0ull;
+        st_word(now + at, t1, t2);
+        then[at] = BandWord{0ull, 0ull};
       }
       at += (size_t)G * g.cb;
       w.next();
@@ -429,8 +448,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
   } else {
     // ------------------------------------------------------------------ coefficient warp
     const uint32_t lp = 1u << g.lane_shift, ci = lane >> g.lane_shift, sub = lane & (lp - 1u);
-    const unsigned long long *buf = reinterpret_cast<const unsigned long long *>(a.ws + g.tag) + (ctl->parity ? (size_t)g.total * g.cb : 0);
-    const double n_full = (double)g.rows * dim0, n_tail = (double)(N - (g.tiles - 1) * g.rows) * dim0;
+    const BandWord *buf = reinterpret_cast<const BandWord *>(a.ws + g.tag) + (ctl->parity ? (size_t)g.total * g.cb : 0);
     BandWalk w(g, b, G);
     uint32_t q = 0, qpar = 1;
     float gm = 1.f, bt = 0.f, mean = 0.f, var = 1.f;
@@ -446,46 +464,46 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
     for (uint32_t n = 0; ok && n < mine; ++n) {
       const uint32_t c = w.unit * g.cb + ci;
       const bool has = ci < g.cb && c < C;
-      const unsigned long long *words = buf + (size_t)w.unit * g.tiles * g.cb + ci;
-      double s1 = 0.0, s2 = 0.0, K = 0.0;
+      const BandWord *words = buf + (size_t)w.unit * g.tiles * g.cb + ci;
+      double s1 = 0.0, s2 = 0.0;
       const long long t0 = clock64();
-      constexpr int kPull = 8;
-      for (uint32_t k0 = 0; ok && k0 < g.tiles; k0 += kPull * lp) {
-        unsigned long long r[kPull];
-        for (;;) {
-          bool all = true;
+      // The unit's words, P per lane at a time: all of them under way together, and added up in pairs.  The merge is the longest chain of a
+      // step of many words, and every P beyond what a lane has costs instructions: always eight, and by their number, us backward,
+      // [4096,1024,7,7], 412 words, 449 and 421, [128,2048,7,7], 64 words, 32.6 and 31.3.
+      auto pull = [&](auto count) {
+        constexpr uint32_t P = decltype(count)::value;
+        for (uint32_t k0 = 0; k0 < g.tiles; k0 += P * lp) {
+          BandWord r[P];
 #pragma unroll
-          for (int i = 0; i < kPull; ++i) {
-            const uint32_t k = k0 + sub + i * lp;
-            r[i] = has && k < g.tiles ? ld_relaxed_gpu_u64(words + (size_t)k * g.cb) : 1ull;
-            all = all && r[i] != 0ull;
-          }
-          if (__all_sync(0xffffffffu, all)) break;
-          __nanosleep(100);
-          uint32_t stop = 0;
-          if (lane == 0) {
-            if (ctl->abort) stop = 1;
-            else if (clock64() - t0 > 2 * a.wait_cycles) { atomicOr(status, ANODE_ST_WAIT_STATS); ctl->abort = 1; stop = 1; }
-          }
-          if (__shfl_sync(0xffffffffu, stop, 0)) { ok = false; break; }
-        }
-        if (!ok) break;
-        if (DIR == 0 && k0 == 0) {      // shift: the mean of the first tile (an infinity or a NaN is none, the sums show it)
-          const float first = __shfl_sync(0xffffffffu, __uint_as_float((uint32_t)r[0]), ci << g.lane_shift);
-          K = fabsf(first) < 1e36f ? (double)first : 0.0;
-        }
+          for (uint32_t i = 0; i < P; ++i) r[i].lo = r[i].hi = has && k0 + sub + i * lp < g.tiles ? 0ull : 1ull << 63;
+          for (;;) {
+            bool all = true;
 #pragma unroll
-        for (int i = 0; i < kPull; ++i) {
-          const uint32_t k = k0 + sub + i * lp;
-          if (k < g.tiles) {
-            const double lo = (double)__uint_as_float((uint32_t)r[i]), hi = (double)__uint_as_float((uint32_t)(r[i] >> 32));
-            if (DIR == 0) {
-              const double cnt = k + 1 == g.tiles ? n_tail : n_full, d = lo - K;
-              s1 = fma(cnt, d, s1); s2 += fma(cnt * d, d, hi);
-            } else { s1 += lo; s2 += hi; }
+            for (uint32_t i = 0; i < P; ++i) {
+              if (r[i].lo == 0ull || r[i].hi == 0ull) r[i] = ld_word(words + (size_t)(k0 + sub + i * lp) * g.cb);      // (one that has come is not asked for again)
+              all = all && r[i].lo != 0ull && r[i].hi != 0ull;
+            }
+            if (__all_sync(0xffffffffu, all)) break;
+            __nanosleep(100);
+            uint32_t stop = 0;
+            if (lane == 0) {
+              if (ctl->abort) stop = 1;
+              else if (clock64() - t0 > 2 * a.wait_cycles) { atomicOr(status, ANODE_ST_WAIT_STATS); ctl->abort = 1; stop = 1; }
+            }
+            if (__shfl_sync(0xffffffffu, stop, 0)) return false;
           }
+          double lo[P], hi[P];
+#pragma unroll
+          for (uint32_t i = 0; i < P; ++i) { lo[i] = __longlong_as_double((long long)r[i].lo); hi[i] = __longlong_as_double((long long)r[i].hi); }
+#pragma unroll
+          for (uint32_t h = P / 2; h > 0; h /= 2)
+#pragma unroll
+            for (uint32_t i = 0; i < h; ++i) { lo[i] += lo[i + h]; hi[i] += hi[i + h]; }
+          s1 += lo[0]; s2 += hi[0];
         }
-      }
+        return true;
+      };
+      ok = g.tiles > 8 * lp ? pull(std::integral_constant<uint32_t, 16>{}) : g.tiles > 4 * lp ? pull(std::integral_constant<uint32_t, 8>{}) : pull(std::integral_constant<uint32_t, 4>{});
       if (!ok) break;
       for (uint32_t o = lp >> 1; o > 0; o >>= 1) { s1 += __shfl_xor_sync(0xffffffffu, s1, o); s2 += __shfl_xor_sync(0xffffffffu, s2, o); }
       if (!warp_wait(&ctl->coef_empty[q], qpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
@@ -494,7 +512,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
       if (has && sub == 0) {
         if (DIR == 0) {
           const double m = s1 * g.inv_count;
-          const float mf = (float)(K + m);
+          const float mf = (float)m;
           const float vf = (float)(not_below_zero(s2 - s1 * m) * g.inv_count + (double)a.epsilon);      // biased, epsilon folded in (batch_norm.cu:160)
           coef[0] = make_float4(mf, gm * inv_std(vf), bt, 0.f);
           if (owner) {

@@ -18,6 +18,7 @@ constexpr uint32_t kBandWords = 512;        // most words of a unit
 constexpr uint32_t kBandBox = 64;           // most vectors of a box (256 floats, the most a tensor map takes)
 constexpr uint32_t kBandMaxSlots = 8, kBandQ = 3;
 constexpr uint32_t kBandCtlBytes = 1024;
+constexpr uint32_t kBandWordBytes = 16;     // a tile's pair of doubles for a channel
 constexpr uint32_t kBandSmem = 227u * 1024u;
 
 struct BandGeom {
@@ -26,10 +27,11 @@ struct BandGeom {
   uint32_t tiles, total, grid, look;   // tiles of a unit, of the layer; blocks; steps between a tile's two visits
   uint32_t boxes, box4, box_bytes;     // boxes of a band, vectors of a box's row, bytes of a box in a slot
   uint32_t slots, plane_bytes, slot_stride, off_side, off_res, off_coef, off_slots, smem_bytes;
+  uint32_t off_second, res_bytes;      // of an entry of the threads' sums (BandSums)
   uint32_t lane_shift;                 // log2 of the lanes that work on one channel in the service warps
   uint32_t whole;                      // loads: 1 the lines are dead once read, 0 neighbouring units' blocks read parts of them, too
   uint32_t tag, hdr;                   // workspace: tagged words, exit counter and parity word (byte offsets)
-  double inv_full, inv_tail, inv_count;      // reciprocals of a channel's elements in a tile, in a unit's last tile, in the layer
+  double inv_count;                    // reciprocal of a channel's elements in the layer
 };
 
 // Tagged words of one of the two buffers.
@@ -61,8 +63,8 @@ inline bool band_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra
       if (vpt * groups > 256) continue;                                         // (rows of a box)
       const uint32_t per = ceil_div_u32(ceil_div_u32(N, ceil_div_u32(N, groups * vpt)), groups), rows = groups * per;      // equal tiles
       const uint32_t tiles = ceil_div_u32(N, rows);
-      // A unit's tiles make one step of the grid at most, and every block merges a unit's words: sixteen per lane at most.  (Forward,
-      // streaming kernel and this one with more of them: [8000,20,11,11] 66 and 103 us, [20000,12,7,9] 72 and 109.)
+      // A unit's tiles make one step of the grid at most, and every block merges a unit's words: sixteen per lane at most where the channels
+      // are a power of two, thirty where a lane has a channel of 17 to itself.  (Forward, streaming kernel and this one with more of them: [8000,20,11,11] 66 and 103 us, [20000,12,7,9] 72 and 109.)
       if (tiles > sms || tiles * cb > kBandWords || 4ull * rows * C * dim0 >> 32) continue;      // (a thread's places within a tile: 32 bits)
       const uint32_t total = units * tiles;
       if (total < sms) continue;
@@ -81,7 +83,9 @@ inline bool band_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra
   while (g.lane_shift && (32u >> g.lane_shift) < g.cb) --g.lane_shift;
   uint32_t off = kBandCtlBytes;
   g.off_side = off; off += kBandMaxSlots * kBandChannels * 16;                          // per slot (mean, scale, beta) of the channels
-  g.off_res = off; off += kBandQ * (kBandConsumers * 16 + 256);                         // per entry: the threads' sums, the channels' shifts
+  // per entry: the threads' sums for their first channels, and for their second ones (a channel has one such vector per group)
+  g.off_second = kBandConsumers * 16; g.res_bytes = g.off_second + (dim0 % 4 ? g.groups * g.cb * 16 : 0);
+  g.off_res = off; off += kBandQ * g.res_bytes;
   g.off_coef = off; off += kBandQ * 2 * kBandChannels * 16;                             // per entry: the channels' coefficients
   g.off_slots = off = (off + 127) / 128 * 128;
   g.slot_stride = g.plane_bytes * band_planes(dir, extra);
@@ -89,8 +93,6 @@ inline bool band_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra
   if (g.slots < 2) return false;
   if (g.slots > kBandMaxSlots) g.slots = kBandMaxSlots;
   g.smem_bytes = off + g.slots * g.slot_stride;
-  g.inv_full = 1.0 / ((double)g.rows * dim0);
-  g.inv_tail = 1.0 / ((double)(N - (g.tiles - 1) * g.rows) * dim0);
   g.inv_count = 1.0 / ((double)dim0 * (double)N);
   return true;
 }

@@ -454,7 +454,7 @@ static void fill_shape_info(ShapeInfo &s)
       s.band_ok[dir][ex] = band_plan(s.dim0, s.C, s.N, dir, ex != 0, g);
       if (!s.band_ok[dir][ex]) continue;
       g.hdr = ex ? kBandHdrExtra : kBandHdr;
-      const uint64_t end = align_up_u64(s.part_bytes + band_words(g) * 16ull, 256);
+      const uint64_t end = align_up_u64(s.part_bytes + band_words(g) * 2 * kBandWordBytes, 256);
       if (end > 0xffffffffull) { s.band_ok[dir][ex] = false; continue; }
       g.tag = (uint32_t)s.part_bytes;
       s.part_bytes = end;
@@ -467,7 +467,7 @@ bool band_geom_of(const FusedArgs &a, int dir, BandGeom &g)
   const ShapeInfo &s = shape_info(a.plan.dim0, a.plan.C, a.plan.N);
   if (!s.band_ok[dir][extra]) return false;
   g = s.band[dir][extra];
-  return a.bands && a.ws_capacity >= g.tag + 16ull * band_words(g);
+  return a.bands && a.ws_capacity >= g.tag + band_words(g) * 2 * kBandWordBytes;
 }
 
 // Bytes of a part taken by the tile-plan kernels (plain, warp-specialised, cluster); the records of the

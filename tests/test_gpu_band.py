@@ -130,7 +130,7 @@ def test_a_poisoned_channel_has_no_variance(stream):
 
 
 def test_means_far_from_zero_keep_the_variances_digits(stream):
-    """The shift of a channel's sums comes from three of its elements in each tile; with the mean at 300 standard deviations the
+    """The shift of a thread's sums comes from four of its samples in each tile; with the mean at 300 standard deviations the
     bound is that of the inputs' own rounding, 2^-24 * 300 relative to a deviation, for the mean of a few thousand of them."""
     ops, shape = stream, (1024, 320, 7, 7)
     d = inputs(shape, 9)
@@ -140,3 +140,42 @@ def test_means_far_from_zero_keep_the_variances_digits(stream):
     var = x.var((0, 2, 3), unbiased=False) + 1e-5
     assert float(((got["var"].double() - var) / var).abs().max()) < 300 * 2.0 ** -24
     assert float((got["mean"].double() - x.mean((0, 2, 3))).abs().max()) < 300 * 2.0 ** -23
+
+
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("shape", [(1024, 320, 7, 7), (1283, 244, 7, 7), (300, 257, 14, 14), (1999, 64, 11, 11), (700, 4500, 1, 5), (500, 2003, 4, 4)])
+def test_sums_are_rounded_once(stream, shape, residual):
+    """Whole numbers, such that what a thread adds up in f32 is exact (forward: squares of quarters below 256, 16 of them, are sixteenths below
+    2^20; backward: 8 numbers below 2^20): the results are the exact sums, rounded once to f32, 2^-24 relative.  (No last tile here leaves a
+    thread with three samples, whose mean is no shift in quarters.)"""
+    ops = stream
+    for direction in (0, 1):
+        assert band(shape, direction, residual)["taken"] == 1
+    g = torch.Generator(device="cuda")
+    g.manual_seed(sum(shape))
+    c, n = shape[1], shape[0] * shape[2] * shape[3]
+    ints = lambda low, high: torch.randint(low, high, shape, device="cuda", generator=g).float()
+    z = lambda: torch.zeros(c, device="cuda")
+    x = ints(-100, 101) + torch.randint(-50, 51, (1, c, 1, 1), device="cuda", generator=g).float()
+    y, mean, var = torch.empty_like(x), z(), z()
+    ws = ops.Workspace(*ops.dims_of(x), x.device)
+    if residual:
+        ops.BatchNormalize2dAddActFusedOp.apply([0, 1], 1e-5, 0.1, x, x, y, mean, var, z(), z(), None, None, 1.0, ws)
+    else:
+        ops.BatchNormalize2dFusedOp.apply([0, 1], 1e-5, 0.1, x, y, mean, var, z(), z(), None, None, workspace=ws, neg_slope=1.0)
+    ax = (0, 2, 3)
+    s1, s2 = x.double().sum(ax), x.double().square().sum(ax)
+    epsilon = float(torch.tensor(1e-5))
+    once = lambda got, want, what: float(((got.double() - want).abs() - 2.0 ** -24 * (1 + 1e-6) * want.abs()).max()) <= 0 or pytest.fail(what)
+    once(mean, s1 / n, "mean")
+    once(var, (s2 - s1 * s1 / n) / n + epsilon, "var")
+    # about a mean of zero and with a variance of one, whose 1 / std has its lowest bit set (inv_std): dgamma is sum(dz * x), with x of -1, 0, 1
+    x, dy = ints(-1, 2), ints(-(2 ** 20) + 1, 2 ** 20)
+    dx, dgamma, dbeta = torch.empty_like(x), z(), z()
+    if residual:
+        ops.BatchNormalize2dAddActFusedOp.adjoint([0, 1], dy, x, y, z(), z() + 1, dx, torch.empty_like(x), None, None, dgamma, dbeta, 1.0, workspace=ws)
+    else:
+        ops.BatchNormalize2dBwdFusedOp.apply([0, 1], dy, x, z(), z() + 1, dx, None, None, dgamma, dbeta, workspace=ws, neg_slope=1.0)
+    assert ws.status() == 0
+    once(dbeta, dy.double().sum(ax), "dbeta")
+    once(dgamma, (dy.double() * x.double()).sum(ax) * (1 + 2.0 ** -23), "dgamma")

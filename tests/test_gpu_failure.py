@@ -88,6 +88,7 @@ def test_a_wait_that_runs_out_leaves_no_copy_and_no_state_behind(kernel, shape, 
     c, x = shape[1], d["x"]
     ops.set_kernel(kernel)
     try:
+        assert [ops.serving_kernel(shape, direction, residual=residual) for direction in (0, 1)] == [kernel] * 2
         want, ws = run(ops, d, residual, 0.1)
         z = [torch.zeros(c, device="cuda") for _ in range(4)]
         y, dx, dres = (torch.empty_like(x) for _ in range(3))
