@@ -509,6 +509,7 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
     case ANODE_KERNEL_PLAIN: if (plain_ok) return ANODE_KERNEL_PLAIN; break;
     case ANODE_KERNEL_REGISTER: if (chan_applies(a, dir, aligned)) return ANODE_KERNEL_REGISTER; break;
     case ANODE_KERNEL_STREAM: if (stream_applies(a, dir, aligned)) return ANODE_KERNEL_STREAM; break;
+    case ANODE_KERNEL_BAND: { BandGeom bg; if (stream_applies(a, dir, aligned) && band_geom_of(a, dir, bg)) return ANODE_KERNEL_STREAM; break; }
     default:
       if (chan_preferred(a, dir, aligned, tiled_ok)) return ANODE_KERNEL_REGISTER;
       if (stream_preferred(a, dir, aligned, tiled_ok)) return ANODE_KERNEL_STREAM;
@@ -533,20 +534,24 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
   return resident_applies(a, dir, aligned) ? ANODE_KERNEL_RESIDENT : -1;
 }
 
+static thread_local int t_last_kernel = -1;
+
 // Launches direction `dir` of a prepared call with the kernel pick_kernel_kind names.  A cluster launch
 // the device refuses falls back to the next kernel that applies.
 int launch_best(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)
 {
   int kind = pick_kernel_kind(a, dir, aligned);
-  if (kind == ANODE_KERNEL_REGISTER) return launch_chan(a, dir, aligned, stream);
+  auto launched = [&](int k, int rc) { if (rc == ANODE_OK) t_last_kernel = k; return rc; };
+  if (kind == ANODE_KERNEL_REGISTER) return launched(kind, launch_chan(a, dir, aligned, stream));
   if (kind == ANODE_KERNEL_STREAM) {
     BandGeom bg;
-    if (band_geom_of(a, dir, bg) && launch_band(a, bg, dir, stream) == ANODE_OK) return ANODE_OK;
-    if (launch_stream(a, dir, stream) == ANODE_OK) return ANODE_OK;
+    if (kernel_choice() != ANODE_KERNEL_STREAM && band_geom_of(a, dir, bg) &&
+        launched(ANODE_KERNEL_BAND, launch_band(a, bg, dir, stream)) == ANODE_OK) return ANODE_OK;
+    if (launched(kind, launch_stream(a, dir, stream)) == ANODE_OK) return ANODE_OK;
     kind = segres_applies(a, dir, aligned) ? ANODE_KERNEL_CLUSTER : ANODE_KERNEL_PLAIN;
   }
   if (kind == ANODE_KERNEL_CLUSTER) {
-    if (launch_segres(a, dir, stream) == ANODE_OK) return ANODE_OK;
+    if (launched(kind, launch_segres(a, dir, stream)) == ANODE_OK) return ANODE_OK;
     Plan rp; RingGeom g;
     if (ring_plan_of(a, dir, aligned, rp, g)) kind = ANODE_KERNEL_TILED;
     else if (resident_applies(a, dir, aligned)) kind = ANODE_KERNEL_RESIDENT;
@@ -556,10 +561,10 @@ int launch_best(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)
     Plan rp; RingGeom g;
     if (!ring_plan_of(a, dir, aligned, rp, g)) return ANODE_E_LAUNCH;
     a.plan = rp;
-    return launch_ring(a, g, dir, stream);
+    return launched(kind, launch_ring(a, g, dir, stream));
   }
-  if (kind == ANODE_KERNEL_RESIDENT) return launch_resident(a, dir, tiled_part_bytes(a.plan.dim0, a.plan.C, a.plan.N), stream);
-  if (kind == ANODE_KERNEL_PLAIN) return launch_pipeline(a, dir, stream);
+  if (kind == ANODE_KERNEL_RESIDENT) return launched(kind, launch_resident(a, dir, tiled_part_bytes(a.plan.dim0, a.plan.C, a.plan.N), stream));
+  if (kind == ANODE_KERNEL_PLAIN) return launched(kind, launch_pipeline(a, dir, stream));
   return ANODE_E_LAUNCH;
 }
 
@@ -848,6 +853,8 @@ extern "C" int anode_gpu_batch_norm_fused_serving_kernel(uint32_t dim0, uint32_t
   return k < 0 ? ANODE_KERNEL_AUTO : k;
 }
 
+extern "C" int anode_gpu_batch_norm_fused_last_kernel(void) { return t_last_kernel; }
+
 // The family, among the first four kernels, of the shape of a one-GPU call on aligned tensors.
 static int family(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool residual)
 {
@@ -875,7 +882,7 @@ extern "C" int anode_gpu_batch_norm_add_act_fused_kernel_kind(uint32_t dim0, uin
 
 extern "C" int anode_gpu_batch_norm_fused_set_kernel(int kernel)
 {
-  if (kernel < ANODE_KERNEL_AUTO || kernel > ANODE_KERNEL_STREAM) return ANODE_E_DIMS;
+  if (kernel < ANODE_KERNEL_AUTO || kernel > ANODE_KERNEL_BAND) return ANODE_E_DIMS;
   g_kernel_choice.store(kernel, std::memory_order_relaxed);
   return ANODE_OK;
 }

@@ -322,12 +322,14 @@ def relu(x, inplace=False, cfg=None, stream=None):
 # --------------------------------------------------------------------------------------------
 
 KERNELS = {"auto": 0, "tiled": 1, "cluster": 2, "resident": 3, "plain": 4, "register": 5, "stream": 6}
+#: the streaming kernel's form for large layers; serving_kernel counts it as "stream"
+BAND = 7
 
 
 def set_kernel(name):
     """Process-wide kernel preference of the fused calls (anode_gpu_batch_norm_fused_set_kernel):
-    a name of KERNELS.  For tests and measurements."""
-    check(_lib.load().anode_gpu_batch_norm_fused_set_kernel(KERNELS[name]), "anode_gpu_batch_norm_fused_set_kernel")
+    a name of KERNELS, or "band".  For tests and measurements."""
+    check(_lib.load().anode_gpu_batch_norm_fused_set_kernel(BAND if name == "band" else KERNELS[name]), "anode_gpu_batch_norm_fused_set_kernel")
 
 
 def serving_kernel(shape, dir, residual=False, aligned=True, world=1):
@@ -340,6 +342,12 @@ def serving_kernel(shape, dir, residual=False, aligned=True, world=1):
     if k < 0:
         raise AnodeError(k, "anode_gpu_batch_norm_fused_serving_kernel")
     return {v: n for n, v in KERNELS.items()}[k] if k else None
+
+
+def last_kernel():
+    """Name of the kernel that this thread's last fused call launched, "band" and "stream" told apart; None before the first."""
+    k = _lib.load().anode_gpu_batch_norm_fused_last_kernel()
+    return "band" if k == BAND else {v: n for n, v in KERNELS.items()}.get(k)
 
 
 def set_wait_limit_ms(ms):

@@ -242,12 +242,17 @@ def run_reference(args, rank):
 
 def time_layer(layer, x, dy, y, dx, steps, warmup, dist, sampler=None):
     """W warm-up steps, then K timed steps bracketed by barrier + synchronize; device time by CUDA
-    events on the launching stream; per-kernel events inside.  Returns (total_ms, fwd_ms, bwd_ms)."""
+    events on the launching stream; per-kernel events inside.  Returns (total_ms, fwd_ms, bwd_ms, clocks,
+    names of the kernels that the last warm-up step launched)."""
     import torch
+    from anode_b200 import ops
     if sampler:
         sampler.start()
     for _ in range(warmup):
-        layer.forward(x, out=y); layer.backward(dy, out=dx)
+        layer.forward(x, out=y)
+        launched = [ops.last_kernel()]
+        layer.backward(dy, out=dx)
+        launched.append(ops.last_kernel())
     torch.cuda.synchronize()
     if dist is not None:
         dist.barrier()
@@ -271,7 +276,7 @@ def time_layer(layer, x, dy, y, dx, steps, warmup, dist, sampler=None):
     total = ev[0][0].elapsed_time(ev[-1][2])
     fwd = sum(e[0].elapsed_time(e[1]) for e in ev) / steps
     bwd = sum(e[1].elapsed_time(e[2]) for e in ev) / steps
-    return total, fwd, bwd, clocks
+    return total, fwd, bwd, clocks, launched
 
 
 def parity_check(layer, x, dy, y, dx, dist, device, eps=1e-5):
@@ -376,7 +381,7 @@ def bench_workload(ops, name, rank, world, steps, warmup, dist, device, sample_c
     y = torch.empty_like(x); dx = torch.empty_like(x)
     layer = make_layer(ops, x.shape[1], world, gamma, beta)
     sampler = ClockSampler(device.index) if (sample_clocks and rank == 0) else None
-    total, fwd, bwd, clocks = time_layer(layer, x, dy, y, dx, steps, warmup, dist, sampler)
+    total, fwd, bwd, clocks, launched = time_layer(layer, x, dy, y, dx, steps, warmup, dist, sampler)
     status = layer.status()
     t = torch.tensor([total, fwd, bwd, float(status)], dtype=torch.float64, device=device)
     if dist is not None:
@@ -390,7 +395,7 @@ def bench_workload(ops, name, rank, world, steps, warmup, dist, device, sample_c
     ms = total / steps
     res = {"ms_per_step": ms, "fwd_ms": fwd, "bwd_ms": bwd, "elements_local": n_local, "elements_global": n_global,
            "value": n_global / (ms * 1e-3), "clocks": clocks, "launches_per_step": layer.launches_per_step, "parity": parity,
-           "exchange": world == 1 or getattr(layer.comm, "_exchange", None) is not None}
+           "launched": launched, "exchange": world == 1 or getattr(layer.comm, "_exchange", None) is not None}
     if with_e2e:
         res["e2e"] = bench_e2e(ops, layer, x, dy, y, dx, dist, device, min(steps, 3))     # first: it compares with y, dx of the timed steps
         res["infer"] = bench_infer(layer, x, y, steps, warmup)
@@ -408,19 +413,25 @@ def bench_residual(ops, layer, x, dy, y, dx, steps, warmup):
     axes = list(range(x.dim() - 2))
     ws = ops.Workspace(*ops.dims_of(x), x.device)
 
-    def step():
+    def forward():
         ops.BatchNormalize2dAddActFusedOp.apply(axes, layer.epsilon, layer.avg_rate, x, res, y, layer.mean, layer.var,
                                                 layer.avg_mean, layer.avg_var, layer.gamma, layer.beta, 0.0, ws)
+
+    def backward():
         ops.BatchNormalize2dAddActFusedOp.adjoint(axes, dy, x, y, layer.mean, layer.var, dx, dres, layer.gamma, layer.beta,
                                                   layer.dgamma, layer.dbeta, 0.0, workspace=ws)
     for _ in range(max(warmup, 3)):
-        step()
+        forward()
+        launched = [ops.last_kernel()]
+        backward()
+        launched.append(ops.last_kernel())
     torch.cuda.synchronize()
     k = max(5, steps // 3)
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     e0.record()
     for _ in range(k):
-        step()
+        forward()
+        backward()
     e1.record()
     torch.cuda.synchronize()
     assert ws.status() == 0
@@ -428,7 +439,7 @@ def bench_residual(ops, layer, x, dy, y, dx, steps, warmup):
     peak, kind = hbm_peak()
     gbs = 32.0 * x.numel() / (ms * 1e-3) / 1e9
     del res, dres
-    kk = [KERNEL_NAMES[ops.serving_kernel(x.shape, d, residual=True)][0] for d in (0, 1)]
+    kk = [KERNEL_NAMES[k][0] for k in launched]
     return {"kernel": "%s (forward), %s (backward), residual epilogue" % tuple(kk), "ms_per_step": ms,
             "elements_per_s": x.numel() / (ms * 1e-3), "achieved_gbs": gbs, "frac_of_hbm_peak": gbs / peak, "peak_kind": kind}
 
@@ -439,7 +450,8 @@ KERNEL_NAMES = {"tiled": ("bn_ring_kernel", "fused reduce+apply, tiled"),
                 "resident": ("bn_resident_kernel", "fused reduce+apply, slices resident in shared memory"),
                 "plain": ("bn_pipeline_kernel", "fused reduce+apply, plain"),
                 "register": ("bn_chan_kernel", "fused reduce+apply, channels in registers"),
-                "stream": ("bn_stream_kernel / bn_band_kernel", "fused reduce+apply, short rows: streaming clusters, large layers tiles of bands")}
+                "stream": ("bn_stream_kernel", "fused reduce+apply, streaming clusters"),
+                "band": ("bn_band_kernel", "fused reduce+apply, tiles of bands of short rows")}
 
 
 def bench_infer(layer, x, y, steps, warmup):
@@ -595,10 +607,10 @@ def main():
     def kernel_name(direction):
         if not main_res["exchange"]:
             return "reduce kernel + all-gather + merge kernel + apply kernel (%s)" % direction
-        kind = ops.serving_kernel(local_shape(w, rank, world), 0 if direction == "fwd" else 1, world=world)
-        if kind is None:
+        launched = main_res["launched"][0 if direction == "fwd" else 1]
+        if ops.serving_kernel(local_shape(w, rank, world), 0 if direction == "fwd" else 1, world=world) is None:
             return "reduce kernel + exchange kernel + apply kernel (%s)" % direction
-        return "%s<%s> (%s)" % (KERNEL_NAMES[kind][0], direction, KERNEL_NAMES[kind][1])
+        return "%s<%s> (%s)" % (KERNEL_NAMES[launched][0], direction, KERNEL_NAMES[launched][1])
     line = {
         "metric": "bn_relu_fwd_bwd_elements_per_s", "value": main_res["value"], "unit": "elements/s",
         "n_gpus": world, "steps": args.steps, "warmup": args.warmup, "ms_per_step": main_res["ms_per_step"],

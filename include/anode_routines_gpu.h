@@ -188,11 +188,14 @@ void anode_gpu_positive_clip_flat_map_bwd_f32(
  *   PLAIN     plain loads and stores (any shape, any alignment; one GPU);
  *   REGISTER  channels held in the registers of a warp, a block or a cluster (small layers, any alignment;
  *             one GPU);
- *   STREAM    clusters that walk a block of channels twice (layers of short rows; one GPU); the largest of them in one
- *             walk, with the tiles in tensor memory between reduction and normalization, where the call has a workspace.
+ *   STREAM    clusters that walk a block of channels twice (layers of short rows; one GPU);
+ *   BAND      its form for the largest of them, where the call has a workspace: one walk, with the tiles in tensor memory
+ *             between reduction and normalization.  Queries by shape count it as STREAM.  It is launched cooperatively and takes
+ *             the whole device, so other streams' kernels run before or after it, not beside it.
  * anode_gpu_batch_norm_fused_set_kernel makes another choice process-wide: that kernel is used wherever it
  * applies, elsewhere one of the first four by the shape.  Meant for tests and measurements; which kernel a
- * call launches is answered by anode_gpu_batch_norm_fused_serving_kernel (anode_routines_gpu_diag.h). */
+ * call launches is answered by anode_gpu_batch_norm_fused_serving_kernel, which one the last call launched by
+ * anode_gpu_batch_norm_fused_last_kernel (anode_routines_gpu_diag.h). */
 #define ANODE_KERNEL_AUTO      0
 #define ANODE_KERNEL_TILED     1
 #define ANODE_KERNEL_CLUSTER   2
@@ -200,6 +203,7 @@ void anode_gpu_positive_clip_flat_map_bwd_f32(
 #define ANODE_KERNEL_PLAIN     4
 #define ANODE_KERNEL_REGISTER  5
 #define ANODE_KERNEL_STREAM    6
+#define ANODE_KERNEL_BAND      7
 int anode_gpu_batch_norm_fused_set_kernel(int kernel);
 
 /* Bound of every wait inside the kernels (for a channel's statistics, for another GPU's records), in

@@ -20,6 +20,10 @@ extern "C" {
 int anode_gpu_batch_norm_fused_serving_kernel(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual,
                                               int aligned, int world);
 
+/* ANODE_KERNEL_* value of the kernel that this thread's last fused call launched, in one launch or with the exchange apart, BAND and
+ * STREAM told apart; -1 before the first one. */
+int anode_gpu_batch_norm_fused_last_kernel(void);
+
 /* Family, among the first four ANODE_KERNEL_* values, that the shape of a plain fused call on 16-byte aligned tensors
  * belongs to.  (The REGISTER and STREAM kernels and the TILED kernel's ragged rows count as the family whose shapes they
  * take over on one GPU; for the kernel that is launched ask anode_gpu_batch_norm_fused_serving_kernel.) */

@@ -37,6 +37,7 @@ pub const ANODE_KERNEL_RESIDENT: c_int = 3;
 pub const ANODE_KERNEL_PLAIN: c_int = 4;
 pub const ANODE_KERNEL_REGISTER: c_int = 5;
 pub const ANODE_KERNEL_STREAM: c_int = 6;
+pub const ANODE_KERNEL_BAND: c_int = 7;
 pub const ANODE_STATIC_SCRATCH_BYTES: usize = 4 << 20;
 
 #[link(name = "anode_routines_gpu")]

@@ -1,6 +1,7 @@
 """The band kernel at the sizes where its splits have remainders: a last unit of fewer channels, a last tile of fewer samples,
 vectors shared by two channels, one sample group and many, one box and several, the most channels of a unit; the residual
-epilogue, outputs over inputs, a channel with a NaN or an infinity, and other kernels between its launches on one workspace."""
+epilogue, outputs over inputs, a channel with a NaN or an infinity, and other kernels between its launches on one workspace.  Every call is
+asserted to have launched it: where the device refuses it, the streaming kernel serves."""
 import ctypes
 
 import pytest
@@ -16,9 +17,9 @@ SHAPES = [(1283, 244, 7, 7), (300, 257, 14, 14), (500, 2003, 4, 4), (1999, 64, 1
 
 
 @pytest.fixture
-def stream():
+def forced():
     from anode_b200 import ops
-    ops.set_kernel("stream")
+    ops.set_kernel("band")
     yield ops
     ops.set_kernel("auto")
 
@@ -32,7 +33,10 @@ def inputs(shape, seed):
                 gamma=torch.rand(c, device="cuda", generator=g) + 0.5, beta=torch.rand(c, device="cuda", generator=g) * 0.2 - 0.1)
 
 
-def run(ops, d, residual, slope, ws=None):
+def run(ops, d, residual, slope, ws=None, launched="band"):
+    """Forward and backward call, each launched by the kernel of that name (None: by any)."""
+    def check_kernel():
+        assert launched is None or ops.last_kernel() == launched, (tuple(d["x"].shape), ops.last_kernel())
     x, c = d["x"], d["x"].shape[1]
     z = lambda: torch.zeros(c, device="cuda")
     r = dict(mean=z(), var=z(), run_mean=z(), run_var=z() + 1, dgamma=z(), dbeta=z(), y=torch.full_like(x, float("nan")), dx=torch.full_like(x, float("nan")))
@@ -41,12 +45,15 @@ def run(ops, d, residual, slope, ws=None):
         r["dres"] = torch.full_like(x, float("nan"))
         op = ops.BatchNormalize2dAddActFusedOp
         op.apply([0, 1], 1e-5, 0.1, x, d["res"], r["y"], r["mean"], r["var"], r["run_mean"], r["run_var"], d["gamma"], d["beta"], slope, ws)
+        check_kernel()
         op.adjoint([0, 1], d["dy"], x, r["y"], r["mean"], r["var"], r["dx"], r["dres"], d["gamma"], d["beta"], r["dgamma"], r["dbeta"], slope, workspace=ws)
     else:
         ops.BatchNormalize2dFusedOp.apply([0, 1], 1e-5, 0.1, x, r["y"], r["mean"], r["var"], r["run_mean"], r["run_var"], d["gamma"], d["beta"],
                                           workspace=ws, neg_slope=slope)
+        check_kernel()
         ops.BatchNormalize2dBwdFusedOp.apply([0, 1], d["dy"], x, r["mean"], r["var"], r["dx"], d["gamma"], d["beta"], r["dgamma"], r["dbeta"],
                                              workspace=ws, neg_slope=slope)
+    check_kernel()
     assert ws.status() == 0
     return r, ws
 
@@ -77,8 +84,8 @@ def check(d, got, residual, slope, what):
 
 @pytest.mark.parametrize("shape", SHAPES)
 @pytest.mark.parametrize("residual", [False, True])
-def test_against_float64(stream, shape, residual):
-    ops = stream
+def test_against_float64(forced, shape, residual):
+    ops = forced
     for direction in (0, 1):
         assert band(shape, direction, residual)["taken"] == 1 and ops.serving_kernel(shape, direction, residual=residual) == "stream"
     d, slope = inputs(shape, sum(shape)), 0.1 if shape[0] % 2 else 0.0
@@ -93,25 +100,26 @@ def test_against_float64(stream, shape, residual):
 def test_outputs_over_inputs(form):
     from anode_b200 import ops
     assert band((1411, 132, 7, 7), 1, 1)["taken"] == 1
-    outputs_over_inputs(ops, (1411, 132, 7, 7), form, "stream")
+    outputs_over_inputs(ops, (1411, 132, 7, 7), form, "band")
+    assert ops.last_kernel() == "band"
 
 
-def test_other_kernels_between_its_launches_on_one_workspace(stream):
-    ops, shape = stream, (1283, 244, 7, 7)
+def test_other_kernels_between_its_launches_on_one_workspace(forced):
+    ops, shape = forced, (1283, 244, 7, 7)
     d = inputs(shape, 7)
     want, ws = run(ops, d, False, 0.0)
     want_res, _ = run(ops, d, True, 0.0, ws)
-    for kernel in ("plain", "auto", "register", "cluster"):
+    for kernel in ("plain", "auto", "register", "stream"):
         ops.set_kernel(kernel)
-        check(d, run(ops, d, False, 0.0, ws)[0], False, 0.0, kernel)
-        ops.set_kernel("stream")
+        check(d, run(ops, d, False, 0.0, ws, launched="band" if kernel == "auto" else kernel)[0], False, 0.0, kernel)
+        ops.set_kernel("band")
         for residual, w in ((False, want), (True, want_res)):
             got, _ = run(ops, d, residual, 0.0, ws)
             assert all(torch.equal(got[k], w[k]) for k in w), (kernel, residual)
 
 
-def test_a_poisoned_channel_has_no_variance(stream):
-    ops, shape = stream, (1283, 244, 7, 7)
+def test_a_poisoned_channel_has_no_variance(forced):
+    ops, shape = forced, (1283, 244, 7, 7)
     d = inputs(shape, 8)
     clean, _ = run(ops, d, False, 0.0)
     for place in (0, 777):
@@ -129,10 +137,10 @@ def test_a_poisoned_channel_has_no_variance(stream):
             assert torch.equal(got[k][:, rest], clean[k][:, rest]), k
 
 
-def test_means_far_from_zero_keep_the_variances_digits(stream):
+def test_means_far_from_zero_keep_the_variances_digits(forced):
     """The shift of a thread's sums comes from four of its samples in each tile; with the mean at 300 standard deviations the
     bound is that of the inputs' own rounding, 2^-24 * 300 relative to a deviation, for the mean of a few thousand of them."""
-    ops, shape = stream, (1024, 320, 7, 7)
+    ops, shape = forced, (1024, 320, 7, 7)
     d = inputs(shape, 9)
     d["x"] = torch.randn(shape, device="cuda") + 300.0
     got, _ = run(ops, d, False, 0.0)
@@ -144,11 +152,11 @@ def test_means_far_from_zero_keep_the_variances_digits(stream):
 
 @pytest.mark.parametrize("residual", [False, True])
 @pytest.mark.parametrize("shape", [(1024, 320, 7, 7), (1283, 244, 7, 7), (300, 257, 14, 14), (1999, 64, 11, 11), (700, 4500, 1, 5), (500, 2003, 4, 4)])
-def test_sums_are_rounded_once(stream, shape, residual):
+def test_sums_are_rounded_once(forced, shape, residual):
     """Whole numbers, such that what a thread adds up in f32 is exact (forward: squares of quarters below 256, 16 of them, are sixteenths below
     2^20; backward: 8 numbers below 2^20): the results are the exact sums, rounded once to f32, 2^-24 relative.  (No last tile here leaves a
     thread with three samples, whose mean is no shift in quarters.)"""
-    ops = stream
+    ops = forced
     for direction in (0, 1):
         assert band(shape, direction, residual)["taken"] == 1
     g = torch.Generator(device="cuda")

@@ -77,7 +77,7 @@ def test_wait_for_an_absent_peer_runs_out_and_the_workspace_recovers(short_waits
 
 
 @pytest.mark.parametrize("residual", [False, True])
-@pytest.mark.parametrize("kernel,shape", [("stream", (1283, 244, 7, 7)), ("stream", (256, 512, 14, 14)), ("tiled", (64, 95, 55, 55)),
+@pytest.mark.parametrize("kernel,shape", [("band", (1283, 244, 7, 7)), ("band", (256, 512, 14, 14)), ("tiled", (64, 95, 55, 55)),
                                           ("tiled", (64, 64, 56, 56))])
 def test_a_wait_that_runs_out_leaves_no_copy_and_no_state_behind(kernel, shape, residual):
     """A bound of one cycle: the first poll for a channel's words finds none, in every block, with copies on their way into the
@@ -88,8 +88,7 @@ def test_a_wait_that_runs_out_leaves_no_copy_and_no_state_behind(kernel, shape, 
     c, x = shape[1], d["x"]
     ops.set_kernel(kernel)
     try:
-        assert [ops.serving_kernel(shape, direction, residual=residual) for direction in (0, 1)] == [kernel] * 2
-        want, ws = run(ops, d, residual, 0.1)
+        want, ws = run(ops, d, residual, 0.1, launched=kernel)
         z = [torch.zeros(c, device="cuda") for _ in range(4)]
         y, dx, dres = (torch.empty_like(x) for _ in range(3))
         if residual:
@@ -113,7 +112,7 @@ def test_a_wait_that_runs_out_leaves_no_copy_and_no_state_behind(kernel, shape, 
             assert t0.elapsed_time(t1) < 500.0
             ws.reset()
         for _ in range(2):
-            again, _ = run(ops, d, residual, 0.1, ws)
+            again, _ = run(ops, d, residual, 0.1, ws, launched=kernel)
             assert all(torch.equal(again[k], want[k]) for k in want)
     finally:
         ops.set_wait_limit_ms(1500)

@@ -49,6 +49,37 @@ def test_a_forced_kernel_is_the_one_that_serves(name):
         ops.set_kernel("auto")
 
 
+def test_forcing_the_streaming_kernel_or_its_form_for_large_layers():
+    ops.set_kernel("band")
+    try:
+        assert [ops.serving_kernel((1024, 2048, 7, 7), d) for d in (0, 1)] == ["stream"] * 2      # (its family by shape)
+        assert ops.serving_kernel((100, 1024, 14, 14), 0) == "stream"                              # where "auto" takes another one
+        assert ops.serving_kernel((64, 16, 7, 7), 0) != "stream"                                   # a layer that has no band form
+    finally:
+        ops.set_kernel("auto")
+    assert "band" not in ops.KERNELS and ops.serving_kernel((100, 1024, 14, 14), 0) == "register"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["tiled", "cluster", "resident", "plain", "register", "stream", "band"])
+def test_a_forced_kernel_is_the_one_that_was_launched(name):
+    """A large layer of short rows, which the band kernel serves unless another one is forced; and the forms of other shapes."""
+    shape = {"tiled": (9, 5, 55, 55), "resident": (16, 8, 56, 56), "cluster": (64, 96, 7, 7)}.get(name, (1283, 244, 7, 7))
+    x = torch.randn(shape, device="cuda")
+    layer = ops.FusedBatchNormRelu(shape[1])
+    ops.set_kernel(name)
+    try:
+        layer.forward(x)
+        first = ops.last_kernel()
+        layer.backward(x)
+        assert [first, ops.last_kernel()] == [name] * 2
+    finally:
+        ops.set_kernel("auto")
+    if name == "stream":
+        layer.forward(x)
+        assert ops.last_kernel() == "band"
+
+
 class Comm:
     """Ranks of a synchronized layer, as far as it is asked for the launches of a step."""
     def __init__(self, world, exchange):
