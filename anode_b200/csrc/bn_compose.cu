@@ -24,6 +24,7 @@ namespace anode_b200 {
 constexpr uint32_t kComposeThreads = 512, kComposeCluster = 8;
 constexpr uint64_t kComposeSmall = 128u << 10;      // floats of a small channel (launch_compose)
 constexpr int kComposeHold = 4;       // vectors per tensor that a thread holds (64 registers: two blocks per SM)
+constexpr uint64_t kComposeWindow = 100u << 20;      // bytes between the two walks of an adjoint, where all blocks are resident (launch_compose)
 constexpr int kComposeScalars = 8;    // floats in flight per thread and tensor where rows are loaded float by float
 
 struct ComposeArgs {
@@ -72,11 +73,13 @@ __global__ void __launch_bounds__(kComposeThreads, 2) bn_compose_kernel(const Co
 
   // the thread's vectors are j0, j0 + stride, ... of the channel, B of them in flight; places by walking (row, column) along
   // (float offsets are below 2^32, check_dims)
-  // Four chains of additions per thread (that of dy * (x - mean) two or four).  Where the cluster is chosen for the waves of blocks
+  // Four chains of additions per thread (that of dy * (x - mean) three or four).  Where the cluster is chosen for the waves of blocks
   // (launch_compose) they are emptied into double precision after every batch, so that a chain is two to four additions however much a
-  // thread walks: the adjoint's sums are no further from float64 than with the larger clusters (it costs nothing: the walk waits for loads).
-  constexpr int B = HOLD ? kComposeHold : VEC == 1 ? kComposeScalars : DIR == 0 ? kComposeHold : kComposeHold / 2;
-  constexpr int S = B < kComposeHold ? kComposeHold / B : 1, D = HOLD || VEC == 1 ? kComposeHold : kComposeHold / 2;
+  // thread walks: the adjoint's sums are no further from float64 than with the larger clusters, relative error of dmean of [300,16,56,56] 7.1e-8
+  // and, without, 1.1e-7.  It costs three to six per cent where the cluster is the same anyway, which a third vector in flight makes good, us
+  // without and with both: [3483,7,16,16] 35.9 and 32.8, [2426,4,16,16] 24.5 and 22.7, but [192,6,28,28] 7.3 and 7.7, [52,32,35,60] 12.5 and 14.2.
+  constexpr int B = HOLD ? kComposeHold : VEC == 1 ? kComposeScalars : DIR == 0 ? kComposeHold : kComposeHold - 1;      // (four of the adjoint's spill)
+  constexpr int D = HOLD || VEC == 1 ? kComposeHold : kComposeHold - 1;
   const uint32_t per_row = g.dim0 / VEC, total = per_row * g.N, rs = g.C * g.dim0;
   const uint32_t stride = cs * blockDim.x, j0 = rank * blockDim.x + threadIdx.x;
   const uint32_t row0 = j0 / per_row, drow = stride / per_row;
@@ -162,9 +165,9 @@ __global__ void __launch_bounds__(kComposeThreads, 2) bn_compose_kernel(const Co
     visit([&](const Pack<VEC> &x, const Pack<VEC> &dy, uint32_t, int u) {
 #pragma unroll
       for (int i = 0; i < VEC; ++i) {
-        const int chain = (u * S + i % S) % kComposeHold;
+        const int chain = (u + i) % kComposeHold;
         const float d = x.v[i] - m;
-        a1[u % D] = fmaf(dy.v[i], d, a1[u % D]); a2[chain] += dy.v[i]; a3[chain] += d;
+        a1[(u + i) % D] = fmaf(dy.v[i], d, a1[(u + i) % D]); a2[chain] += dy.v[i]; a3[chain] += d;
       }
     }, empty);
     empty();
@@ -206,14 +209,32 @@ static int launch_compose(const ComposeArgs &g, bool aligned, cudaStream_t strea
   // (Two where a thread of one block would have 64 floats and more; two that hold the channel.)  Adjoint with the cluster that
   // holds the channel or eight, and so, us: [64,128,28,28] 25.2 and 20.0, [32,64,56,56] 25.9 and 19.6, [64,512,28,28] 88 and 76, [64,128,27,27]
   // 32.4 and 21.2, [40,300,15,15] 39.5 and 15.4, [256,1024,7,7] 132 and 49, [16,95,55,55] 24.6 and 19.6.  Forward [32,512,27,27] 66 and 40,
-  // but [65,1024,55,55] 684 and 798.  (With two and four floats in flight per thread in the place of eight, the adjoint's scalar
-  // rows took 38.8 us, [64,128,27,27], and 29.3, [16,95,55,55].)
+  // but [65,1024,55,55] 684 and 798.
+  // The adjoint's second walk wants to find the channels in flight in L2 (kComposeWindow): with the cluster by waves alone, and larger ones up to
+  // eight while they exceed it, [256,150,28,28] 121 and 90, [256,512,28,28] 330 and 283, [91,512,32,32] 149 and 129.
+  // (Less where blocks leave and others come: [207,646,28,28] with 96 MB 317 and, with 48, 285; [408,143,14,14], resident, with 91 MB 36.6 and 41.4.
+  // Not where eight would exceed it by far, [1285,108,28,28] 336 and 353, nor scalar rows, which wait for less, [958,128,353] 149 and 159.)
+  // And clusters of four and eight do not fill the device, their SMs lie together: [64,n,28,28] with 70 of four 12.4, with 72 17.7 ([1184,71,33], 71 of them, 12.4 and, of two, 13.5).
   const bool waves = DIR == 1 || (!vec && total <= kComposeSmall);
-  const uint32_t lanes = vec ? 4u : 1u;
+  const uint32_t lanes = vec ? 4u : 1u, wave = 2 * sm_count();
   auto holds = [&](uint32_t n) { return total <= (uint64_t)n * kComposeThreads * kComposeHold; };
+  auto window = [&](uint32_t n) { return (g.C < wave / n ? g.C : wave / n) * total * lanes * 8; };
+  const bool near = DIR == 1 && vec && window(kComposeCluster) <= kComposeWindow * 3 / 2;
   uint32_t cs = 1;
   while (cs < kComposeCluster && !holds(cs) &&
-         (!waves || (uint64_t)g.C * cs * 2 <= 2ull * sm_count() || (cs == 1 && (total * lanes >= 64ull * kComposeThreads || (vec && holds(2)))))) cs *= 2;
+         (!waves || (uint64_t)g.C * cs * 2 <= (cs == 1 || DIR == 0 ? wave : wave * 24 / 25) ||
+          (cs == 1 && (total * lanes >= 64ull * kComposeThreads || (vec && holds(2)))) || (near && window(cs) > ((uint64_t)g.C * cs <= wave ? kComposeWindow : kComposeWindow * 4 / 5)))) cs *= 2;
+  if (DIR == 1 && vec && !holds(cs) && holds(kComposeCluster)) {
+    // A cluster that holds the channel needs no second walk.  It is the faster one where the others leave a few SMs with one block more than the
+    // rest or with a wave of their own, and beyond a wave where its threads are nearly full of what they hold.  Us without and with:
+    // [64,75,28,28] 16.6 and 15.9, [48,75,28,28] 13.2 and 11.9, [64,150,28,28] 29.5 and 27.0, [24,310,28,28] 23.2 and 18.8; [14,969,40,55] 94 and 77,
+    // [5,512,112,112] 90 and 87, but two thirds full, [45,512,32,32], 67 and 74.
+    const uint64_t blocks = (uint64_t)g.C * cs;
+    uint32_t n = 2 * cs;
+    while (!holds(n)) n *= 2;
+    if ((blocks * 2 > wave && blocks * 10 <= wave * 7ull) || (blocks > wave && blocks < 3ull * wave && blocks % wave && blocks % wave * 4 <= wave) ||
+        (blocks > wave && total * 8 >= 7ull * n * kComposeThreads * kComposeHold)) cs = n;
+  }
   const bool hold = holds(cs);
   // threads of a block: a vector each where all of them are resident at once, else up to what one holds
   const uint64_t each = (total + cs - 1) / cs;

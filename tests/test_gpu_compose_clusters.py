@@ -10,9 +10,13 @@ CLUSTERS = [(n, c) + hw for c in (37, 38, 74, 75, 148, 149, 300) for n, hw in ((
 # one block: threads of 64 floats and more have two; channels that two blocks hold; up to four vectors held per thread, blocks of all sizes
 EDGES = [(2048, 150, 4, 4), (2047, 150, 4, 4), (669, 150, 7, 7), (668, 150, 7, 7), (1024, 150, 4, 4), (1025, 150, 4, 4), (513, 150, 4, 4),
          (9, 2048, 5, 5), (16, 2048, 7, 7), (20, 2048, 8, 8), (128, 700, 8, 8), (129, 700, 8, 8), (1, 2500, 1, 3)]
+# channels that a cluster of eight or four holds: on both sides of the lines between it and smaller ones by the number of blocks; and channels
+# whose second walk is kept within reach of L2
+HELD = [(64, c, 28, 28) for c in (35, 36, 70, 71, 75, 88, 89, 150, 185, 186)] + [(37, 149, 28, 28), (24, 310, 28, 28), (14, 300, 40, 55)]
+WINDOWS = [(127, 128, 32, 32), (256, 150, 28, 28), (33, 186, 55, 55)]
 
 
-@pytest.mark.parametrize("shape", CLUSTERS + EDGES)
+@pytest.mark.parametrize("shape", CLUSTERS + EDGES + HELD + WINDOWS)
 def test_adjoint_and_composition(shape):
     from anode_b200 import ops
     g = torch.Generator(device="cuda")
