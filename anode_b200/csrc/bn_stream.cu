@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamBlocks) bn_stream_kerne
 constexpr uint64_t kStreamWindow = 96ull << 20;
 constexpr uint64_t kStreamSplit = 72ull << 20;
 
-static bool stream_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, StreamGeom &g)
+static bool stream_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, StreamGeom &g)
 {
   if (dim0 < 4 || (uint64_t)C * dim0 % 4 != 0) return false;
   uint32_t q = 4; if (dim0 % 2 == 0) q = 2; if (dim0 % 4 == 0) q = 1;      // cb*dim0 must be a multiple of 4
@@ -337,17 +337,23 @@ static bool stream_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, StreamGe
   // nearly a whole one, with nearly all threads.  Forward / backward, us, before and after: [128,2048,7,7] 512 and 412 blocks 26.4 / 33.0 and
   // 21.2 / 33.0 (backward in three waves either way), [64,2048,7,7] 17.9 / 25.8 and 15.4 / 20.5, [32,2048,7,7] 11.4 / 15.4 and 10.0 / 13.8,
   // [150,1000,6,6] 500 and 400 blocks 16.8 / 22.2 and 12.7 / 17.9.
+  // The SMs of a cluster lie together, so larger ones leave places empty, and one that does not fit makes a second wave: in clusters of eight 376
+  // blocks are resident and 400 are not, in clusters of four 412 are and 432 not.  [112,1000,7,7], 500 blocks and 400 in clusters of eight,
+  // 17.2 / 22.4 and 19.5 / 27.9, [723,2048,4,4], 512 and 432 in clusters of four, 50 and 58, but [140,940,7,7], 470 and 376, 17.5 and 16.6.
+  // The residual backward pass wants six samples per thread, too: [20,2000,7,7] 11.9 and, with five, 12.9.
   uint32_t run = L4;      // vectors
   if (!split && g.units * cl > wave && g.units * cl * 3 <= wave * 4 && g.groups * L4 > 192) {      // (of fewer threads four blocks are resident)
     uint32_t most_threads = wave * kStreamThreads * 25 / 32;
     for (uint32_t cb = q; cb <= C && cb <= kStreamChannels && (uint64_t)cb * dim0 <= 4 * kStreamThreads; cb += q) {
       const uint32_t V = cb * dim0 / 4, units = ceil_div_u32(C, cb), groups = kStreamThreads / V < N ? kStreamThreads / V : N;
       if (cb * dim0 < 128) continue;
-      for (uint32_t n = 1; n <= 8 && n * cb <= kStreamRecords && N / n >= groups * least; n *= 2)
-        if (units * n <= wave && units * n * groups * V > most_threads && wave * (16ull * V * N * (dir == 1 ? 2 : 1)) / n <= kStreamWindow) {
-          most_threads = units * n * groups * V;
+      for (uint32_t n = 1; n <= 8 && n * cb <= kStreamRecords && N / n >= groups * (dir == 1 && extra ? 6 : least); n *= 2) {
+        const uint32_t blocks = units * n, resident = n == 8 ? wave * 17 / 20 : n == 4 ? wave * 15 / 16 : wave;
+        if (blocks <= resident && blocks * groups * V > most_threads && wave * (16ull * V * N * (dir == 1 ? 2 : 1)) / n <= kStreamWindow) {
+          most_threads = blocks * groups * V;
           cl = n; run = V; g.cb = cb; g.units = units; g.groups = groups;
         }
+      }
     }
   }
   g.cluster = cl;
@@ -358,11 +364,13 @@ static bool stream_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, StreamGe
   return true;
 }
 
+static bool stream_extra(const FusedArgs &a, int dir) { return (dir == 0 ? a.res : a.ymask) != nullptr; }
+
 // Blocks of a cluster, and of the grid, for this call; 0 where the kernel does not apply.
 uint32_t stream_cluster(const FusedArgs &a, int dir, bool aligned, uint32_t &blocks)
 {
   StreamGeom g;
-  if (!stream_applies(a, dir, aligned) || !stream_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, g)) return 0u;
+  if (!stream_applies(a, dir, aligned) || !stream_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, stream_extra(a, dir), g)) return 0u;
   blocks = g.units * g.cluster;
   return g.cluster;
 }
@@ -370,7 +378,7 @@ uint32_t stream_cluster(const FusedArgs &a, int dir, bool aligned, uint32_t &blo
 bool stream_applies(const FusedArgs &a, int dir, bool aligned)
 {
   StreamGeom g;
-  return aligned && a.mode == MODE_FUSED && a.world <= 1 && stream_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, g);
+  return aligned && a.mode == MODE_FUSED && a.world <= 1 && stream_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, stream_extra(a, dir), g);
 }
 
 // Where this kernel is taken (after the register-resident kernel): all rows that the tiled kernel does not serve, and of
@@ -389,7 +397,7 @@ bool stream_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
 {
   const uint32_t dim0 = a.plan.dim0;
   StreamGeom g;
-  if (!stream_applies(a, dir, aligned) || !stream_geom(dim0, a.plan.C, a.plan.N, dir, g)) return false;
+  if (!stream_applies(a, dir, aligned) || !stream_geom(dim0, a.plan.C, a.plan.N, dir, stream_extra(a, dir), g)) return false;
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
   const uint32_t walk = ceil_div_u32(g.rows, g.groups), blocks = g.units * g.cluster;
   if (tiled_ok && walk >= kStreamLongWalk) return false;
@@ -404,7 +412,7 @@ bool stream_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
 int launch_stream(FusedArgs &a, int dir, cudaStream_t stream)
 {
   StreamGeom g;
-  if (!stream_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, g)) return ANODE_E_LAUNCH;
+  if (!stream_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, stream_extra(a, dir), g)) return ANODE_E_LAUNCH;
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
   // dres may be stored before x is read again only where it is not x itself
   a.dres_early = a.dres && a.dres != a.x ? 1u : 0u;
@@ -448,7 +456,7 @@ extern "C" int anode_gpu_batch_norm_stream_geometry(uint32_t dim0, uint32_t dim1
   using namespace anode_b200;
   if (!out || (dir != 0 && dir != 1) || check_dims(dim0, dim1, dim2)) return ANODE_E_DIMS;
   StreamGeom g{};
-  const bool ok = stream_geom(dim0, dim1, dim2, dir, g);
+  const bool ok = stream_geom(dim0, dim1, dim2, dir, false, g);
   const uint32_t v[7] = {ok ? 1u : 0u, g.cb, g.units, g.cluster, g.rows, g.groups, g.threads};
   for (int i = 0; i < 7; ++i) out[i] = v[i];
   return ANODE_OK;

@@ -52,7 +52,7 @@ int anode_gpu_batch_norm_fused_plan_walk(uint32_t dim0, uint32_t dim1, uint32_t 
 int anode_gpu_batch_norm_segres_geometry(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, uint32_t *out);
 
 /* Geometry of the streaming kernel.  out (7 values): applies, channels per unit, units, blocks per cluster, samples per
- * block, sample groups of a block, threads. */
+ * block, sample groups of a block, threads (of an ordinary call, without the residual epilogue). */
 int anode_gpu_batch_norm_stream_geometry(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, uint32_t *out);
 
 /* Geometry of the band kernel, the streaming kernel's form for large layers.  out (16 values): taken by a call with a workspace

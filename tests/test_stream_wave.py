@@ -24,8 +24,18 @@ def test_one_wave_of_blocks(shape):
     assert 192 < g["groups"] * g["cb"] * d0 // 4 <= g["threads"] <= 256
 
 
+@pytest.mark.parametrize("shape", [(103, 1000, 7, 7), (117, 1000, 7, 7), (365, 1000, 5, 5), (1015, 512, 4, 4), (723, 2048, 4, 4), (302, 233, 10, 10),
+                                   (140, 940, 7, 7), (64, 2048, 7, 7)])
+def test_no_wave_of_clusters_that_are_not_all_resident(shape):
+    """Clusters of eight fill 85 per cent of the device's places, of four 94: a grid that is chosen to be one wave fits those."""
+    for direction in (0, 1):
+        g = stream_geometry(shape, direction)
+        blocks = g["units"] * g["cluster"]
+        assert blocks > WAVE or blocks <= {8: 377, 4: 416}.get(g["cluster"], WAVE), (direction, g)
+
+
 @pytest.mark.gpu
-@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("shape", SHAPES + [(103, 1000, 7, 7), (153, 940, 7, 7)])
 def test_results(shape):
     from anode_b200 import ops
     ops.set_kernel("stream")
