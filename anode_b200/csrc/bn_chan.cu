@@ -289,7 +289,9 @@ bool chan_applies(const FusedArgs &a, int dir, bool aligned)
 // [31,6844,14], 685 blocks, 13.9 / 15.4 and 15.8 / 15.8, [27,5376,17], clusters of four, 12.9 / 14.1 and 15.8 / 14.7.  The residual
 // backward, three tensors a thread, stalls in these teams at any number of waves: from 20 samples and a million elements it goes,
 // [30,948,39], 1.1 M, 13.4 and 8.7, [81,680,35] 15.9 and 11.7, [28,340,218] 26.1 and 12.5, [31,6844,14] 27.1 and 19.2, but
-// [20,848,43], 0.7 M, 6.5 and 6.4, [181,168,21], 0.6 M, 7.1 and 7.9.  Rows of 1 - 3 floats, which the
+// [20,848,43], 0.7 M, 6.5 and 6.4, [181,168,21], 0.6 M, 7.1 and 7.9; and units of 52 or 92 channels, which a block of few samples folds one by
+// one, stay here, [25,3720,11] 11.1 and 14.3, [24,10100,11] 25.8 and 29.5.  (Of 280 residual backward passes of 1 - 3 M elements and 18 to 400
+// samples, 190 went over, 0.95 of the time over all, six of them slower, all of such units.)  Rows of 1 - 3 floats, which the
 // threads fetch from far apart, on the shared-memory kernel: [1024,512,3] residual backward 25.8 and 18.5, [1540,632,2]
 // backward 24.4 and 18.7, [1457,828,1] residual forward 23.6 and 20.6.
 // Backward passes and the residual epilogue of large layers of medium and long aligned rows go to the tiled kernel although a
@@ -311,7 +313,7 @@ constexpr uint64_t kChanBand[2][2] = {{28000000, 18000000}, {18000000, 18000000}
 constexpr uint64_t kChanLarge = 8u << 20, kChanLargeScalar = 3u << 20, kChanLargeExtra = 5u << 20;
 constexpr uint64_t kChanWaves = 1500000, kChanShortest = 1200000, kChanShortestExtra = 1000000;
 constexpr uint32_t kChanFewSamples = 32, kChanFewestSamples = 20;
-constexpr uint32_t kChanLongRow = 300;
+constexpr uint32_t kChanLongRow = 300, kChanUnit = 32;
 bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
 {
   ChanGeom g;
@@ -343,6 +345,7 @@ bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
     const uint32_t cluster = stream_cluster(a, dir, aligned, blocks);
     if (!waves) {
       if (a.plan.N < kChanFewestSamples || !stream_preferred(a, dir, aligned, tiled_ok)) return true;
+      if ((uint64_t)blocks * kChanUnit < (uint64_t)a.plan.C * cluster) return true;      // (more channels to a unit)
       if (!extra_bwd && (elements < kChanWaves || (uint64_t)a.plan.C * g.cluster <= places || cluster > 2 || blocks > 3 * sm_count())) return true;
     }
     return cluster == 0 || cluster > 8;
