@@ -585,18 +585,26 @@ static bool tensor_map(CUtensorMap &m, const float *p, uint32_t width, uint32_t 
 // Where the streaming kernel hands a layer over: rows below those that the tiled kernel takes (tiled_takes), from so many elements
 // on.  Below, the fill and the drain of the schedule, some 10 us, outweigh the second walk it saves.  Streaming kernel and this
 // one, us:
-//   forward    6.4 M [64,2048,7,7] 17.7 and 21.4, 8.4 M [512,256,8,8] 17.8 and 21.4, 12.8 M [128,2048,7,7] 24.8 and 24.9,
-//              16.8 M [512,128,16,16] 34.3 and 31.6, 25.7 M [256,2048,7,7] 56.6 and 47.5
-//   backward   4.8 M [100,400,11,11] 16.7 and 19.8, 6.4 M [64,2048,7,7] 26.3 and 22.5, [128,256,14,14] 24.8 and 25.4, 8.4 M [512,256,8,8]
-//              31.5 and 24.5, 12.8 M 45.4 and 32.8
-//   residual   6.4 M 24.5 / 33.2 and 22.7 / 28.8 ([64,2048,7,7]), 22.1 / 32.0 and 24.4 / 32.7 ([128,256,14,14]), 8.4 M 23.6 / 39.2 and
-//              23.9 / 33.8, 12.8 M 36.6 / 58.6 and 30.1 / 45.7
-constexpr uint32_t kBandLongRow = 320;
+//   forward    15.0 M [3699,203,20] 37.4 and 29.9, [548,596,46] 40.6 and 30.3, 16.1 M [320,1024,7,7] 32.1 and 30.6, 16.8 M [512,128,16,16] 34.2
+//              and 30.8, 25.7 M [256,2048,7,7] 57.5 and 41.1
+//   backward   8.0 M [80,2048,7,7] 24.1 and 24.0, [160,1024,7,7] 30.5 and 24.7, 9.7 M [200,400,11,11] 39.2 and 27.2, 12.8 M [128,2048,7,7]
+//              45.4 and 32.6
+//   residual   9.9 M [1508,71,92] 29.6 and 27.6, 10.0 M [200,1024,7,7] 29.4 and 28.8, 12.8 M [256,256,14,14] 34.8 and 27.5; backward 8.0 M
+//              [80,2048,7,7] 34.1 and 32.9, [160,1024,7,7] 40.8 and 33.2
+constexpr uint32_t kBandLongRow = 320, kBandWaveRow = 40;
+// Forward passes of rows of 40 floats and more that the streaming kernel has in one wave of resident blocks (stream_one_wave) stay with it longer:
+//   forward    [320,400,11,11] 15.5 M 23.4 and 27.9, [400,400,11,11] 19.4 M 33.1 and 32.9, [200,2048,7,7] 20.1 M 36.8 and 40.2,
+//              [224,2048,7,7] 22.5 M 45.1 and 38.8, but [512,2048,4,4] 16.8 M 29.6 and 26.9, [512,1000,6,6] 18.4 M 31.7 and 31.0
+//   residual   [96,2048,7,7] 9.6 M 24.1 and 27.1, [112,2048,7,7] 11.2 M 27.3 and 29.9, [256,400,11,11] 12.4 M 29.3 and 30.0,
+//              [128,2048,7,7] 12.8 M 27.7 and 26.8
 constexpr uint64_t kBandLeast[2][2] = {{15000000, 9000000}, {8000000, 8000000}};      // [direction][residual]
+constexpr uint64_t kBandLeastWave[2] = {21000000, 12500000};      // forward, [residual]
 
 bool band_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, BandGeom &g)
 {
-  if ((uint64_t)dim0 * C * N < kBandLeast[dir][extra] || dim0 >= kBandLongRow) return false;
+  const uint64_t elements = (uint64_t)dim0 * C * N;
+  if (elements < kBandLeast[dir][extra] || dim0 >= kBandLongRow) return false;
+  if (dir == 0 && elements < kBandLeastWave[extra] && dim0 >= kBandWaveRow && stream_one_wave(dim0, C, N, dir, extra)) return false;
   return band_geom(dim0, C, N, dir, extra, sm_count(), g);
 }
 

@@ -61,6 +61,7 @@ bool stream_applies(const FusedArgs &a, int dir, bool aligned);
 uint32_t stream_cluster(const FusedArgs &a, int dir, bool aligned, uint32_t &blocks);
 bool stream_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok);
 int launch_stream(FusedArgs &a, int dir, cudaStream_t stream);
+bool stream_one_wave(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra);      // its grid, where it fills the device once
 // its form for the largest of them (bn_band.cu): the geometry of a shape where it is taken, and of a prepared call
 bool band_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, BandGeom &g);
 bool band_geom_of(const FusedArgs &a, int dir, BandGeom &g);

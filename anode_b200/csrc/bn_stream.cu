@@ -364,6 +364,15 @@ static bool stream_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool ext
   return true;
 }
 
+// Whether the grid is one wave of blocks, all resident, that fills the device: nothing of a second wave to pay for.
+bool stream_one_wave(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra)
+{
+  StreamGeom g;
+  if (!stream_geom(dim0, C, N, dir, extra, g)) return false;
+  const uint32_t wave = kStreamBlocks * sm_count(), blocks = g.units * g.cluster;
+  return g.cluster <= 4 && blocks * 20 >= wave * 17 && blocks <= (g.cluster == 4 ? wave * 15 / 16 : wave);
+}
+
 static bool stream_extra(const FusedArgs &a, int dir) { return (dir == 0 ? a.res : a.ymask) != nullptr; }
 
 // Blocks of a cluster, and of the grid, for this call; 0 where the kernel does not apply.

@@ -50,6 +50,9 @@ def test_layers_that_are_handed_over():
     assert taken((32, 2048, 7, 7)) == (0, 0, 0, 0)
     assert taken((8000, 20, 11, 11)) == (0, 0, 0, 0)             # more words to a unit than a warp merges in time
     assert taken((256, 512, 20, 20)) == (0, 0, 0, 0)             # rows that the tiled kernel takes
+    # forward passes that the streaming kernel has in one wave of resident blocks stay with it longer
+    assert taken((320, 400, 11, 11)) == (0, 1, 1, 1) and taken((200, 2048, 7, 7)) == (0, 1, 1, 1) and taken((224, 2048, 7, 7)) == (1, 1, 1, 1)
+    assert taken((112, 2048, 7, 7)) == (0, 1, 0, 1) and taken((512, 2048, 4, 4)) == (1, 1, 1, 1) and taken((548, 596, 1, 46)) == (1, 1, 1, 1)
     # channels that a team's registers hold, where the band kernel is the faster one
     assert tuple(ops.serving_kernel((256, 1024, 14, 14), d, residual=r) for r in (False, True) for d in (0, 1)) == ("stream",) * 4
     assert tuple(ops.serving_kernel((100, 1024, 14, 14), d, residual=r) for r in (False, True) for d in (0, 1)) == ("register", "stream", "stream", "stream")
