@@ -608,10 +608,11 @@ bool band_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, BandG
   return band_geom(dim0, C, N, dir, extra, sm_count(), g);
 }
 
-// Lines that two units share are read by two blocks, one after the other.  Loaded to be evicted first, as all others, they may be gone by
-// then: ordinary backward passes over tensors beyond L2 load them with the normal priority.  Us with the one and the other, backward:
-// [1024,2048,7,7] 214 and 202 (206 and 204 on another device; step 369 and 362), [2048,1024,7,7] 212 and 205, [512,2048,7,7] 108 and 106; but
-// [128,2048,7,7] 33 and 36, runs of whole lines [2000,2048,4,4] 134 and 136, residual step of [256,1024,14,14] 279 and 280.
+// Lines that two units share are read by two blocks, one after the other.  Ordinary backward passes over tensors beyond L2 load them with the
+// normal priority in the place of the one to be evicted first.  Us so and with the latter, backward, on two devices: [1024,2048,7,7] 202 and 206,
+// [2048,1024,7,7] 205 and 210, [4096,1024,7,7] 418 and 436, [3000,512,7,7] 159 and 165, [2000,500,9,9] 172 and 177, [400,1024,14,14] 161 - 165 and
+// 161; but [128,2048,7,7] 33 and 36 the other way round, runs of whole lines [2000,2048,4,4] 134 and 136.  It is not the traffic, every byte comes from
+// HBM once either way ([1024,2048,7,7]: 822.4 and 822.9 MB for 822.1 of x and dy); why it gains is not known.
 constexpr uint64_t kBandShared = 192ull << 20;      // bytes of x and dy
 int launch_band(FusedArgs &a, const BandGeom &g, int dir, cudaStream_t stream)
 {
