@@ -447,18 +447,22 @@ static void fill_shape_info(ShapeInfo &s)
       s.ring_geom[dir][ex].hdr = ex ? kRingHdrExtra : kRingHdrRagged;
       if (end > s.part_bytes) s.part_bytes = end;
     }
-  // so does the band kernel
-  for (int dir = 0; dir < 2; ++dir)
+  // so does the band kernel; a part serves one direction, so both directions' words may begin at the same place
+  const uint64_t bands = s.part_bytes;
+  for (int dir = 0; dir < 2; ++dir) {
+    uint64_t at = bands;
     for (int ex = 0; ex < 2; ++ex) {
       BandGeom &g = s.band[dir][ex];
       s.band_ok[dir][ex] = band_plan(s.dim0, s.C, s.N, dir, ex != 0, g);
       if (!s.band_ok[dir][ex]) continue;
       g.hdr = ex ? kBandHdrExtra : kBandHdr;
-      const uint64_t end = align_up_u64(s.part_bytes + band_words(g) * 2 * kBandWordBytes, 256);
+      const uint64_t end = align_up_u64(at + band_words(g) * 2 * kBandWordBytes, 256);
       if (end > 0xffffffffull) { s.band_ok[dir][ex] = false; continue; }
-      g.tag = (uint32_t)s.part_bytes;
-      s.part_bytes = end;
+      g.tag = (uint32_t)at;
+      at = end;
     }
+    if (at > s.part_bytes) s.part_bytes = at;
+  }
 }
 
 bool band_geom_of(const FusedArgs &a, int dir, BandGeom &g)

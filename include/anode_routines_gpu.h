@@ -215,7 +215,8 @@ int anode_gpu_batch_norm_fused_set_wait_limit_ms(uint32_t ms);
 
 /* Scratch the fused kernels need for a [dim0, dim1, dim2] problem: per-tile partial
  * statistics, per-channel coefficients, progress counters; one part per direction (each
- * direction keeps state in its part from launch to launch).  A few hundred KB to a few MB. */
+ * direction keeps state in its part from launch to launch).  A few hundred KB to some tens
+ * of MB: 15.6 for [1024,2048,7,7], 27.6 for [2048,256,56,56], 30.7 for [4096,1024,7,7]. */
 size_t anode_gpu_batch_norm_fused_workspace_bytes(uint32_t dim0, uint32_t dim1, uint32_t dim2);
 
 /* Zeroes a workspace (cudaMemsetAsync on `stream`).  Needed once after allocation, after any call

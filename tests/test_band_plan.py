@@ -68,3 +68,17 @@ def test_its_words_have_their_own_place_in_the_workspace():
         d = ops.dims_of(torch.empty(shape, device="meta"))
         assert lib.anode_gpu_batch_norm_fused_plan(*d, 1, 0, 0, 0, plan, 15) == 0
         assert lib.anode_gpu_batch_norm_fused_workspace_bytes(*d) >= 2 * (plan[13] + words)
+
+
+def test_the_words_of_both_directions_share_their_place():
+    """A part of the workspace serves one direction: behind what the other kernels use there is room for the larger direction's words, twice
+    a pair of doubles per tile and channel in each of its two forms, and no more."""
+    lib = _lib.load()
+    for shape in ((1024, 2048, 7, 7), (256, 2048, 7, 7), (1283, 244, 7, 7), (128, 2048, 7, 7)):      # (no other kernel keeps words of its own here)
+        forms = [[band(shape, d, r) for r in (0, 1)] for d in (0, 1)]
+        room = max(sum(-(-32 * g["units"] * g["tiles"] * g["cb"] // 256) * 256 for g in f if g["taken"]) for f in forms)
+        d = ops.dims_of(torch.empty(shape, device="meta"))
+        part = lib.anode_gpu_batch_norm_fused_workspace_bytes(*d) // 2
+        plan = (ctypes.c_uint32 * 15)()
+        assert lib.anode_gpu_batch_norm_fused_plan(*d, 1, 0, 0, 0, plan, 15) == 0
+        assert part == plan[13] + room, (shape, plan[13], room, part)
