@@ -9,7 +9,9 @@ from anode_b200 import _lib, ops
 
 FIELDS = ["taken", "cb", "units", "groups", "vpt", "rows", "tiles", "grid", "look", "boxes", "box4", "box_bytes", "slots", "stride", "smem", "shift"]
 SHAPES = [(1024, 2048, 7, 7), (256, 1024, 14, 14), (128, 2048, 7, 7), (1283, 244, 7, 7), (300, 257, 14, 14), (500, 2003, 4, 4), (2000, 64, 11, 11),
-          (80, 900, 15, 15), (1000, 2602, 2, 3), (60, 1004, 16, 17), (4096, 64, 16, 16), (2500, 1000, 2, 2), (4099, 2048, 1, 5), (1, 1004, 17, 18)]
+          (80, 900, 15, 15), (1000, 2602, 2, 3), (60, 1004, 16, 17), (4096, 64, 16, 16), (801, 5002, 2, 2), (700, 4500, 1, 5), (1, 1004, 17, 18)]
+# more words to a unit than a warp merges, or units that fit no thread; rows of three floats; channels whose bands are no whole vectors
+REFUSED = [(2500, 1000, 2, 2), (4099, 2048, 1, 5), (8000, 20, 11, 11), (9000, 2000, 1, 3), (2000, 1001, 1, 7)]
 
 
 def band(shape, direction, residual):
@@ -24,8 +26,7 @@ def band(shape, direction, residual):
 def test_geometry(shape, direction, residual):
     d0, c, n = ops.dims_of(torch.empty(shape, device="meta"))
     g = band(shape, direction, residual)
-    if not g["cb"]:
-        return
+    assert g["cb"] > 0
     vectors, kept, planes = g["cb"] * d0 // 4, 1 + direction, 1 + direction + (direction and residual)
     assert g["cb"] * d0 % 4 == 0 and g["cb"] <= min(c, 32) and g["units"] == -(-c // g["cb"])
     # a thread per column and group; the tile's rows cover the samples, the last tile is not empty
@@ -40,6 +41,13 @@ def test_geometry(shape, direction, residual):
     # a unit is reduced before it is applied, and its words fit what a warp merges
     assert g["look"] * g["grid"] >= g["tiles"] + g["grid"] and g["tiles"] * g["cb"] <= 512
     assert (32 >> g["shift"]) >= g["cb"] and 4 * g["rows"] * c * d0 < 1 << 32
+
+
+@pytest.mark.parametrize("shape", REFUSED)
+def test_shapes_that_the_kernel_cannot_take(shape):
+    for direction in (0, 1):
+        for residual in (0, 1):
+            assert not any(band(shape, direction, residual).values())
 
 
 def test_layers_that_are_handed_over():

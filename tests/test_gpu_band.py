@@ -13,7 +13,7 @@ from tests.test_gpu_tiled_forms import outputs_over_inputs
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(1283, 244, 7, 7), (300, 257, 14, 14), (500, 2003, 4, 4), (1999, 64, 11, 11), (81, 900, 15, 15), (1000, 2602, 2, 3), (60, 1004, 16, 17),
-          (1024, 250, 8, 8), (333, 1000, 7, 7)]
+          (1024, 250, 8, 8), (333, 1000, 7, 7), (801, 5002, 2, 2), (700, 4500, 1, 5)]
 
 
 @pytest.fixture
@@ -102,6 +102,37 @@ def test_outputs_over_inputs(form):
     assert band((1411, 132, 7, 7), 1, 1)["taken"] == 1
     outputs_over_inputs(ops, (1411, 132, 7, 7), form, "band")
     assert ops.last_kernel() == "band"
+
+
+def test_calls_without_what_is_optional(forced):
+    """No gamma and beta, no averages, no gradients of gamma and beta, dx accumulated: the ordinary form and the residual epilogue."""
+    ops, shape = forced, (1283, 244, 7, 7)
+    d = inputs(shape, 6)
+    c, x, dy = shape[1], d["x"], d["dy"]
+    m = x.numel() // c
+    v = lambda t: t.double().view(1, -1, 1, 1)
+    ws = ops.Workspace(*ops.dims_of(x), x.device)
+    launched = lambda: ops.last_kernel() == "band" or pytest.fail(str(ops.last_kernel()))
+    for residual in (False, True):
+        mean, var, y, dx = torch.zeros(c, device="cuda"), torch.zeros(c, device="cuda"), torch.empty_like(x), torch.ones_like(x)
+        if residual:
+            ops.BatchNormalize2dAddActFusedOp.apply([0, 1], 1e-5, 0.1, x, d["res"], y, mean, var, workspace=ws)
+            launched()
+            ops.BatchNormalize2dAddActFusedOp.adjoint([0, 1], dy, x, y, mean, var, dx, cap=ops.WriteCap.Accumulate, workspace=ws)
+        else:
+            ops.BatchNormalize2dFusedOp.apply([0, 1], 1e-5, 0.1, x, y, mean, var, workspace=ws)
+            launched()
+            ops.BatchNormalize2dBwdFusedOp.apply([0, 1], dy, x, mean, var, dx, cap=ops.WriteCap.Accumulate, workspace=ws)
+        launched()
+        assert ws.status() == 0
+        xhat = (x.double() - v(x.double().mean((0, 2, 3)))) / v((x.double().var((0, 2, 3), unbiased=False) + 1e-5).sqrt())
+        pre = xhat + (d["res"].double() if residual else 0)
+        mask = y > 0
+        assert not ((mask != (pre > 0)) & (pre.abs() >= 1e-5)).any()
+        dz = dy.double() * mask
+        want = 1 + (dz - v(dz.sum((0, 2, 3))) / m - xhat * v((dz * xhat).sum((0, 2, 3))) / m) / v(var.double().sqrt())
+        for got, w in ((y, pre * mask), (dx, want)):      # the tolerance of tests/util.py
+            assert not ((got.double() - w).abs() > 1e-5 + 1e-4 * w.abs()).any(), residual
 
 
 def test_other_kernels_between_its_launches_on_one_workspace(forced):

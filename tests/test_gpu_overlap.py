@@ -6,7 +6,8 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [(2, 512, 7, 7), (1, 53, 39, 25), (32, 64, 28, 28), (4, 16, 112, 112), (1411, 128, 7, 7), (64, 8, 56, 56)]
+SHAPES = [(2, 512, 7, 7), (1, 53, 39, 25), (32, 64, 28, 28), (4, 16, 112, 112), (1411, 128, 7, 7), (64, 8, 56, 56),
+          (1283, 244, 7, 7)]      # (the last one's forward and backward passes are cooperative launches of the band kernel)
 
 
 def make(ops, shape):
