@@ -38,7 +38,6 @@ struct BandCtl {
   unsigned long long res_full[kBandQ], res_empty[kBandQ], coef_full[kBandQ], coef_empty[kBandQ];
   volatile uint32_t abort;
   uint32_t last_block, parity, tmem;
-  long long limit;       // of the waits (FusedArgs::wait_cycles)
 };
 static_assert(sizeof(BandCtl) <= kBandCtlBytes, "BandCtl outgrew the room reserved for it");
 
@@ -114,7 +113,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
       mbar_init(&ctl->res_full[i], kBandWarps); mbar_init(&ctl->res_empty[i], 1);
       mbar_init(&ctl->coef_full[i], 1); mbar_init(&ctl->coef_empty[i], kBandWarps);
     }
-    ctl->abort = 0; ctl->last_block = 0; ctl->parity = *parity & 1u; ctl->limit = a.wait_cycles;
+    ctl->abort = 0; ctl->last_block = 0; ctl->parity = *parity & 1u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -319,8 +318,8 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
     for (uint32_t s = 0; s < steps; ++s) {
       if (s < mine) {
         if (++slot == g.slots) { slot = 0; par ^= 1u; }
-        bool ok = warp_wait(&ctl->res_empty[qres], rpar, ctl, status, ANODE_ST_WAIT_STATS);
-        ok = ok && warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS);
+        bool ok = warp_wait(&ctl->res_empty[qres], rpar, ctl, status, ANODE_ST_WAIT_STATS, a.wait_cycles);
+        ok = ok && warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS, a.wait_cycles);
         if (!ok) break;
         const BandSums part(sm, g, qres);
         const uint32_t rows = N - red.k * g.rows, tm = tm0 + red_place * tm_step;
@@ -333,10 +332,10 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
         red.next();
       }
       if (s >= g.look) {
-        if (!warp_wait(&ctl->coef_full[qcoef], cpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
+        if (!warp_wait(&ctl->coef_full[qcoef], cpar, ctl, status, ANODE_ST_WAIT_STATS, a.wait_cycles)) break;
         if constexpr (kSlotToo) {
           if (++slot == g.slots) { slot = 0; par ^= 1u; }
-          if (!warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS)) break;
+          if (!warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS, a.wait_cycles)) break;
         }
         const uint32_t n0 = app.k * g.rows, c0 = app.unit * g.cb, rows = N - n0, tm = tm0 + app_place * tm_step;
         const bool alive = live && 4 * v < (C - c0) * dim0;
@@ -373,7 +372,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
       ++k;
       if (++slot == g.slots) { slot = 0; par ^= 1u; }
       uint32_t okw = 1;
-      if (lane == 0) okw = mbar_wait(&ctl->empty[slot], par ^ 1u, ctl, status, ANODE_ST_WAIT_STATS) ? 1u : 0u;
+      if (lane == 0) okw = mbar_wait(&ctl->empty[slot], par ^ 1u, ctl, status, ANODE_ST_WAIT_STATS, a.wait_cycles) ? 1u : 0u;
       ok = __shfl_sync(0xffffffffu, okw, 0) != 0;
       if (!ok) { --k; break; }
       const uint32_t planes = kind == 0 ? kPlanes : 1u;
@@ -414,7 +413,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
     size_t at = (size_t)b * g.cb + ci;
     for (uint32_t j = 0; j < mine; ++j) {
       const bool has = ci < g.cb && w.unit * g.cb + ci < C;
-      if (!warp_wait(&ctl->res_full[q], qpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
+      if (!warp_wait(&ctl->res_full[q], qpar, ctl, status, ANODE_ST_WAIT_STATS, a.wait_cycles)) break;
       const BandSums part(sm, g, q);
       double t1 = 0.0, t2 = 0.0;
       // four of the lane's vectors at a time, their sums added in pairs: the loads are under way together (one vector after another:
@@ -506,7 +505,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
       ok = g.tiles > 8 * lp ? pull(std::integral_constant<uint32_t, 16>{}) : g.tiles > 4 * lp ? pull(std::integral_constant<uint32_t, 8>{}) : pull(std::integral_constant<uint32_t, 4>{});
       if (!ok) break;
       for (uint32_t o = lp >> 1; o > 0; o >>= 1) { s1 += __shfl_xor_sync(0xffffffffu, s1, o); s2 += __shfl_xor_sync(0xffffffffu, s2, o); }
-      if (!warp_wait(&ctl->coef_empty[q], qpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
+      if (!warp_wait(&ctl->coef_empty[q], qpar, ctl, status, ANODE_ST_WAIT_STATS, a.wait_cycles)) break;
       float4 *coef = reinterpret_cast<float4 *>(sm + g.off_coef) + q * 2 * kBandChannels + 2 * ci;
       const bool owner = w.k == 0;
       if (has && sub == 0) {

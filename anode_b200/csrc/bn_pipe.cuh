@@ -33,10 +33,11 @@ __device__ __forceinline__ bool mbar_try(unsigned long long *bar, uint32_t parit
   return ok != 0;
 }
 // Bounded wait.  Returns false (after raising the abort flag) when the barrier did not flip in time
-// or when another role already gave up.  The bound is three times ctl->limit, the caller's one: a barrier hangs on the waits
+// or when another role already gave up.  The bound is three times `limit`, the caller's one (FusedArgs::wait_cycles, by reference: read
+// from the parameters where it is compared; as a word of Ctl it cost [256,64,112,112] 0.6 %): a barrier hangs on the waits
 // for words and records (twice the limit, and once), which should run out first and say in the status word what was missing.
 template <typename Ctl>
-__device__ __forceinline__ bool mbar_wait(unsigned long long *bar, uint32_t parity, Ctl *ctl, uint32_t *status, uint32_t bit)
+__device__ __forceinline__ bool mbar_wait(unsigned long long *bar, uint32_t parity, Ctl *ctl, uint32_t *status, uint32_t bit, const long long &limit)
 {
   if (mbar_try(bar, parity)) return true;
   const long long t0 = clock64();
@@ -47,7 +48,7 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, uint32_t pari
     __nanosleep(kBackoffNs);
     if ((++it & 15u) == 0u) {
       if (ctl->abort) return false;
-      if (clock64() - t0 > 3 * ctl->limit) {
+      if (clock64() - t0 > 3 * limit) {
         atomicOr(status, bit);
         ctl->abort = 1;
         return false;
@@ -59,11 +60,11 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, uint32_t pari
 // hardware holds the warp), is one instruction for the whole warp; only a wait that outlasts that is handed to
 // one lane, which polls with the time limit.
 template <typename Ctl>
-__device__ __forceinline__ bool warp_wait(unsigned long long *bar, uint32_t parity, Ctl *ctl, uint32_t *status, uint32_t bit)
+__device__ __forceinline__ bool warp_wait(unsigned long long *bar, uint32_t parity, Ctl *ctl, uint32_t *status, uint32_t bit, const long long &limit)
 {
   if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
   uint32_t ok = 1;
-  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, ctl, status, bit) ? 1u : 0u;
+  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, ctl, status, bit, limit) ? 1u : 0u;
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 // global -> shared bulk copy, completion counted on `bar`; bytes and both addresses are multiples of 16

@@ -58,7 +58,6 @@ struct RingCtl {
   uint32_t last_block;
   uint32_t parity;       // which of the two tagged-partial buffers this launch uses
   uint32_t tmem;         // base address of the block's tensor memory (g.keep_slots > 0)
-  long long limit;       // of the waits (FusedArgs::wait_cycles)
 };
 static_assert(sizeof(RingCtl) <= kRingCtlBytes, "RingCtl outgrew the room reserved for it");
 
@@ -719,7 +718,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
     for (uint32_t i = 0; i < g.slots; ++i) { mbar_init(&ctl->full[i], 1); mbar_init(&ctl->empty[i], kCWarps); }
     for (uint32_t i = 0; i < kResQ; ++i) { mbar_init(&ctl->res_full[i], kCWarps); mbar_init(&ctl->res_empty[i], 1); }
     for (uint32_t i = 0; i < kCoefQ; ++i) { mbar_init(&ctl->coef_full[i], 1); mbar_init(&ctl->coef_empty[i], kCWarps); }
-    ctl->abort = 0; ctl->last_block = 0; ctl->limit = a.wait_cycles;
+    ctl->abort = 0; ctl->last_block = 0;
     ctl->parity = *ws_u32(a, g.hdr + 4) & 1u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -738,8 +737,8 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
       if (sc.reduce_at(s)) {
         if (++slot == g.slots) { slot = 0; par ^= 1u; }
         // the partial mailbox entry must have been emptied by the delivery warp (first pass: free)
-        bool ok = warp_wait(&ctl->res_empty[qres], rpar, ctl, status, ANODE_ST_WAIT_STATS);
-        ok = ok && warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS);
+        bool ok = warp_wait(&ctl->res_empty[qres], rpar, ctl, status, ANODE_ST_WAIT_STATS, a.wait_cycles);
+        ok = ok && warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS, a.wait_cycles);
         if (!ok) break;                                 // warps are independent: no barrier to honour
         const uint4 d = *reinterpret_cast<const uint4 *>(slot_side<DIR, EXTRA>(sm, g, slot));
         float4 *res = res_box(sm, g, qres);
@@ -749,13 +748,13 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
         if (++qres == kResQ) { qres = 0; rpar ^= 1u; }
       }
       if (sc.apply_at(s)) {
-        if (!warp_wait(&ctl->coef_full[qcoef], cpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
+        if (!warp_wait(&ctl->coef_full[qcoef], cpar, ctl, status, ANODE_ST_WAIT_STATS, a.wait_cycles)) break;
         const float4 *coef = coef_box(sm, g, qcoef);
         const uint4 d = *reinterpret_cast<const uint4 *>(coef + 2);
         const bool kept = TMEM && (d.x >> 16) != 0;
         if (!kept || kSlotAlways<DIR, EXTRA>) {
           if (++slot == g.slots) { slot = 0; par ^= 1u; }
-          if (!warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS)) break;
+          if (!warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS, a.wait_cycles)) break;
         }
         if (TMEM && kept) visit_apply<DIR, EXTRA, RAGGED, true>(a, g, sm, ctl, d, slot, coef, qcoef);
         else visit_apply<DIR, EXTRA, RAGGED, false>(a, g, sm, ctl, d, slot, coef, qcoef);
@@ -802,7 +801,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
       // (one lane polls here: a producer that reacts sooner was measured slower where the window between the two
       // visits exceeds what L2 keeps, and hardly faster elsewhere)
       uint32_t okw = 1;
-      if (lane == 0) okw = mbar_wait(&ctl->empty[slot], par ^ 1u, ctl, status, ANODE_ST_WAIT_STATS) ? 1u : 0u;
+      if (lane == 0) okw = mbar_wait(&ctl->empty[slot], par ^ 1u, ctl, status, ANODE_ST_WAIT_STATS, a.wait_cycles) ? 1u : 0u;
       if constexpr (DIR == 1 && EXTRA) {
         // the dz this visit reads back was stored by visit kr (counting those that use a slot), which must have been
         // given back: implied by the wait above unless fewer than `slots` visits lie in between
@@ -810,7 +809,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
           const uint32_t before = n > sc.look ? n - sc.look : 0u;
           const uint32_t kr = n + before - kept_before(g, before);
           if (k - 1 - kr < g.slots)
-            okw = mbar_wait(&ctl->empty[kr % g.slots], (kr / g.slots) & 1u, ctl, status, ANODE_ST_WAIT_STATS) ? 1u : 0u;
+            okw = mbar_wait(&ctl->empty[kr % g.slots], (kr / g.slots) & 1u, ctl, status, ANODE_ST_WAIT_STATS, a.wait_cycles) ? 1u : 0u;
         }
       }
       ok = __shfl_sync(0xffffffffu, okw, 0) != 0;     // one lane decides for the warp
@@ -902,7 +901,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
     // Reduce visit j of this block is tile b + j*G.  The consumer warps' partials of a tile are merged in a fixed order.
     uint32_t q = 0, qpar = 0, tile = sc.b;
     for (uint32_t j = 0; j < sc.reduces; ++j) {
-      if (!warp_wait(&ctl->res_full[q], qpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
+      if (!warp_wait(&ctl->res_full[q], qpar, ctl, status, ANODE_ST_WAIT_STATS, a.wait_cycles)) break;
       float4 v = lane < kCWarps ? res_box(sm, g, q)[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
       if constexpr (DIR == 0) {
         Moments m{v.x, v.y, v.z};
@@ -975,7 +974,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
           if constexpr (DIR == 1) { in.z = a.mean_in[unit]; in.w = inv_std(a.var_in[unit]); }
         }
       }
-      if (!warp_wait(&ctl->coef_empty[q], qpar, ctl, status, ANODE_ST_WAIT_STATS)) break;
+      if (!warp_wait(&ctl->coef_empty[q], qpar, ctl, status, ANODE_ST_WAIT_STATS, a.wait_cycles)) break;
       const uint32_t u = __shfl_sync(0xffffffffu, unit, at);
       if (u != have) {
         if (a.mode == MODE_FUSED) {
