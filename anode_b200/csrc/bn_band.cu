@@ -21,10 +21,10 @@
 // runs out sets a status bit and the block drains and leaves.  The launch is cooperative and takes the SM's whole shared memory,
 // so that no other block holds columns of tensor memory or waits for them.
 //
-// What bounds it: HBM, and some 10 us in which the schedule fills and drains.  Streaming kernel and this one, forward / backward:
-// [1024,2048,7,7] 179 / 298 and 143 / 202 us (0.88 / 0.93 of the copy bandwidth), residual epilogue 246 / 427 and 204 / 339 (0.92 /
-// 0.93); [256,1024,14,14] 102 / 148 and 75 / 104, residual 137 / 211 and 101 / 163.  On the way there: sixteen consumer warps (96
-// registers) 150 / 218; all vectors of the threads' sums added up one by one in double precision 156 / 238.
+// What bounds it: HBM, and some 10 us in which the schedule fills and drains.  Streaming kernel and this one, us from launch to launch of the
+// same call over buffers beyond L2, forward / backward: [1024,2048,7,7] 179 / 298 and 151 / 204 (0.83 / 0.92 of the copy bandwidth), residual
+// epilogue 246 / 427 and 216 / 347 (0.87 / 0.90); [256,1024,14,14] 102 / 148 and 82 / 106, residual 137 / 211 and 110 / 167.  On the way there, in an
+// older form: sixteen consumer warps (96 registers) 150 / 218 in the place of 143 / 203; all vectors of the threads' sums added up one by one 156 / 238.
 #include <cuda.h>      // types only: the one function is looked up at run time
 
 #include "bn_band.cuh"

@@ -305,9 +305,10 @@ bool chan_applies(const FusedArgs &a, int dir, bool aligned)
 constexpr uint32_t kChanTiledRow = 480;
 constexpr uint64_t kChanTiled = 16u << 20, kChanTiledExtra = 18u << 20, kChanTiledChannel = 24u << 10;
 // Aligned rows below 320 floats go to the band kernel (the streaming kernel's form for large layers) from these sizes on.  Us here
-// and there, forward: [80,1024,14,14] 16 M 27.9 and 33.2, [100,1024,16,16] 26 M 45 and 50, [100,1000,10,30] 30 M 52.2 and 52.1,
-// [180,1024,14,14] 36 M 66 and 58, [256,1024,14,14] 98 and 75; backward: [50,2048,12,12] 15 M 36.4 and 38.4, [100,1024,14,14] 20 M 55 and 47,
-// [256,1024,14,14] 163 and 104; residual forward 16 M 38.7 and 38.5, 20 M 50 and 42; residual backward 15 M 52 and 53, 20 M 77 and 68.
+// and there, forward: [80,1024,14,14] 16 M 29.3 and 31.3, [100,1024,16,16] 26 M 46.7 and 47.8, [100,1000,10,30] 30 M 54.6 and 52.1,
+// [180,1024,14,14] 36 M 68 and 58, [256,1024,14,14] 99 and 81; backward: [50,2048,12,12] 15 M 37.2 and 35.0, [100,1024,14,14] 20 M 55 and 49,
+// [256,1024,14,14] 164 and 106; residual forward, 15 M 32.1 and 34.7, 16 M 40 and 36, 20 M 52 and 46; residual backward 15 M 53.7 and 55.7, 20 M 79
+// and 74.  (The last three lines lie higher than today's times ask for.)
 constexpr uint32_t kChanBandRow = 320;
 constexpr uint64_t kChanBand[2][2] = {{28000000, 18000000}, {18000000, 18000000}};      // [direction][residual]
 constexpr uint64_t kChanLarge = 8u << 20, kChanLargeScalar = 3u << 20, kChanLargeExtra = 5u << 20;
