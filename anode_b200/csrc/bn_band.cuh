@@ -47,7 +47,8 @@ inline bool band_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra
   uint32_t q = 4; if (dim0 % 2 == 0) q = 2; if (dim0 % 4 == 0) q = 1;      // cb*dim0 must be a multiple of 4
   const uint32_t kept = dir == 0 ? 1u : 2u, most = kBandVecs / 4 / kept;      // tensors kept; most samples per thread, for four tiles
   // Channels of a unit and samples per thread: the least (steps + 3) * (cost of a step) * (cost of the runs), fitted to measurements
-  // of the form with f32 words (a cost of 7 or 14 per word made no shape faster with today's, and [256,2048,7,7] forward 45.8 -> 51.3).
+  // of the form with f32 words.  (Twice the cost per word with today's, us: [256,2048,7,7] forward 45.8 -> 51.3, [256,1024,14,14] backward 106 -> 113,
+  // [4000,100,12,12] backward 139 -> 131.)
   //   A step: a fixed part (merge, barriers, parameters), the tile's vectors, the unit's words.  [1024,2048,7,7] forward / backward with
   //   tiles of 16 / 8, 12 / 6, 8 / 4 samples per thread 143 / 202, 145 / 231, 169 / 300 us; [200,2048,8,8] backward with units of 16
   //   channels and 400 words 64 us, of 2 and 22 words 60; [400,2048,8,8] forward with 400 words 82 us, with 15 76.

@@ -290,8 +290,9 @@ bool chan_applies(const FusedArgs &a, int dir, bool aligned)
 // backward, three tensors a thread, stalls in these teams at any number of waves: from 20 samples and a million elements it goes,
 // [30,948,39], 1.1 M, 13.4 and 8.7, [81,680,35] 15.9 and 11.7, [28,340,218] 26.1 and 12.5, [31,6844,14] 27.1 and 19.2, but
 // [20,848,43], 0.7 M, 6.5 and 6.4, [181,168,21], 0.6 M, 7.1 and 7.9; and units of 52 or 92 channels, which a block of few samples folds one by
-// one, stay here, [25,3720,11] 11.1 and 14.3, [24,10100,11] 25.8 and 29.5.  (Of 280 residual backward passes of 1 - 3 M elements and 18 to 400
-// samples, 190 went over, 0.95 of the time over all, six of them slower, all of such units.)  Rows of 1 - 3 floats, which the
+// one, stay here in small layers and with fewer than 26 samples: [25,3720,11] 11.1 and 14.3, [31,3708,11] 13.2 and 15.1, [24,10100,11] 25.8 and 29.5,
+// [21,5652,19] 22.4 and 23.1, but [28,6520,11] 20.8 and 19.4, [29,5156,19] 28.3 and 18.4.  (Those were all that lost by it of 280 residual
+// backward passes of 1 - 3 M elements and 18 to 400 samples.)  Rows of 1 - 3 floats, which the
 // threads fetch from far apart, on the shared-memory kernel: [1024,512,3] residual backward 25.8 and 18.5, [1540,632,2]
 // backward 24.4 and 18.7, [1457,828,1] residual forward 23.6 and 20.6.
 // Backward passes and the residual epilogue of large layers of medium and long aligned rows go to the tiled kernel although a
@@ -314,7 +315,7 @@ constexpr uint64_t kChanBand[2][2] = {{28000000, 18000000}, {18000000, 18000000}
 constexpr uint64_t kChanLarge = 8u << 20, kChanLargeScalar = 3u << 20, kChanLargeExtra = 5u << 20;
 constexpr uint64_t kChanWaves = 1500000, kChanShortest = 1200000, kChanShortestExtra = 1000000;
 constexpr uint32_t kChanFewSamples = 32, kChanFewestSamples = 20;
-constexpr uint32_t kChanLongRow = 300, kChanUnit = 32;
+constexpr uint32_t kChanLongRow = 300, kChanUnit = 32, kChanWideSamples = 26;
 bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
 {
   ChanGeom g;
@@ -346,7 +347,8 @@ bool chan_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
     const uint32_t cluster = stream_cluster(a, dir, aligned, blocks);
     if (!waves) {
       if (a.plan.N < kChanFewestSamples || !stream_preferred(a, dir, aligned, tiled_ok)) return true;
-      if ((uint64_t)blocks * kChanUnit < (uint64_t)a.plan.C * cluster) return true;      // (more channels to a unit)
+      const bool wide = cluster >= 4 && (uint64_t)blocks * kChanUnit < (uint64_t)a.plan.C * cluster;      // (more channels to a unit)
+      if (extra_bwd && wide && (elements < kChanWaves || a.plan.N < kChanWideSamples)) return true;
       if (!extra_bwd && (elements < kChanWaves || (uint64_t)a.plan.C * g.cluster <= places || cluster > 2 || blocks > 3 * sm_count())) return true;
     }
     return cluster == 0 || cluster > 8;

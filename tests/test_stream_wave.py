@@ -59,6 +59,7 @@ LINES = [((25, 932, 1, 45), ("register",) * 3 + ("stream",)),         # one wave
          ((25, 932, 1, 130), ("register", "register", "register", "stream")),     # two waves of the streaming kernel's blocks
          ((30, 520, 1, 145), ("register", "stream", "stream", "stream")),
          ((25, 3720, 1, 11), ("register",) * 4), ((24, 10100, 1, 11), ("register",) * 4),      # units of 92 channels
+         ((29, 5156, 1, 19), ("register",) * 3 + ("stream",)), ((24, 10828, 1, 6), ("register",) + ("stream",) * 3),
          ((300, 188, 1, 23), ("register",) * 3 + ("stream",))]
 
 
