@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
           Quad x0 = K, x1 = K, x2 = K, x3 = K;
           load(x0, i); load(x1, i + 1); load(x2, i + 2); load(x3, i + 3);
           if (i == 0) {
-            shift(Quad{add2(add2(x0.a, x1.a), add2(x2.a, x3.a)), add2(add2(x0.b, x1.b), add2(x2.b, x3.b))}, FULL ? 0.25f : __fdividef(1.f, (float)min(n, 4u)));
+            shift(Quad{add2(add2(x0.a, x1.a), add2(x2.a, x3.a)), add2(add2(x0.b, x1.b), add2(x2.b, x3.b))}, FULL ? 0.25f : __fdividef(1.f, (float)max(min(n, 4u), 1u)));      // (a thread may have none)
             if constexpr (!FULL) { if (!there(0)) x0 = K; if (!there(1)) x1 = K; if (!there(2)) x2 = K; if (!there(3)) x3 = K; }
           }
           if constexpr (!FULL) __syncwarp();

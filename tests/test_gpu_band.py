@@ -13,7 +13,8 @@ from tests.test_gpu_tiled_forms import outputs_over_inputs
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(1283, 244, 7, 7), (300, 257, 14, 14), (500, 2003, 4, 4), (1999, 64, 11, 11), (81, 900, 15, 15), (1000, 2602, 2, 3), (60, 1004, 16, 17),
-          (1024, 250, 8, 8), (333, 1000, 7, 7), (801, 5002, 2, 2), (700, 4500, 1, 5)]
+          (1024, 250, 8, 8), (333, 1000, 7, 7), (801, 5002, 2, 2), (700, 4500, 1, 5),
+          (1351, 244, 7, 7), (2481, 128, 7, 7)]         # a last tile of one sample: groups without any
 
 
 @pytest.fixture
