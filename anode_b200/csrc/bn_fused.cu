@@ -91,6 +91,8 @@ struct ShapeInfo {
   uint64_t tiled_bytes, static_bytes, part_bytes;      // see fill_shape_info
   bool band_ok[2][2];            // the streaming kernel's form for the largest layers, likewise
   BandGeom band[2][2];
+  bool masked_ok[2][2];          // the streaming kernel's masked form, likewise
+  StreamGeom masked[2][2];
 };
 constexpr uint32_t kShapeCache = 64;      // entries per thread, direct mapped
 
@@ -463,6 +465,17 @@ static void fill_shape_info(ShapeInfo &s)
     }
     if (at > s.part_bytes) s.part_bytes = at;
   }
+  for (int dir = 0; dir < 2; ++dir)
+    for (int ex = 0; ex < 2; ++ex) s.masked_ok[dir][ex] = masked_plan(s.dim0, s.C, s.N, dir, ex != 0, s.masked[dir][ex]);
+}
+
+bool masked_geom_of(const FusedArgs &a, int dir, StreamGeom &g)
+{
+  const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
+  if (a.mode != MODE_FUSED || a.world > 1) return false;
+  const ShapeInfo &s = shape_info(a.plan.dim0, a.plan.C, a.plan.N);
+  if (s.masked_ok[dir][extra]) g = s.masked[dir][extra];
+  return s.masked_ok[dir][extra];
 }
 
 bool band_geom_of(const FusedArgs &a, int dir, BandGeom &g)
@@ -504,7 +517,7 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
 {
   const bool extra = a.res || a.ymask || a.dres;        // residual epilogue
   const bool plain_ok = !(a.mode == MODE_FUSED && a.world > 1);
-  Plan rp; RingGeom g;
+  Plan rp; RingGeom g; StreamGeom mg;
   const bool tiled_ok = ring_plan_of(a, dir, aligned, rp, g) && (kernel_choice() != ANODE_KERNEL_AUTO || tiled_preferred(a, dir));
   switch (kernel_choice()) {
     case ANODE_KERNEL_TILED: if (tiled_ok) return ANODE_KERNEL_TILED; break;
@@ -512,7 +525,7 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
     case ANODE_KERNEL_RESIDENT: if (resident_applies(a, dir, aligned)) return ANODE_KERNEL_RESIDENT; break;
     case ANODE_KERNEL_PLAIN: if (plain_ok) return ANODE_KERNEL_PLAIN; break;
     case ANODE_KERNEL_REGISTER: if (chan_applies(a, dir, aligned)) return ANODE_KERNEL_REGISTER; break;
-    case ANODE_KERNEL_STREAM: if (stream_applies(a, dir, aligned)) return ANODE_KERNEL_STREAM; break;
+    case ANODE_KERNEL_STREAM: if (stream_applies(a, dir, aligned) || (aligned && masked_geom_of(a, dir, mg))) return ANODE_KERNEL_STREAM; break;
     case ANODE_KERNEL_BAND: { BandGeom bg; if (stream_applies(a, dir, aligned) && band_geom_of(a, dir, bg)) return ANODE_KERNEL_STREAM; break; }
     default:
       if (chan_preferred(a, dir, aligned, tiled_ok)) return ANODE_KERNEL_REGISTER;
@@ -568,7 +581,13 @@ int launch_best(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)
     return launched(kind, launch_ring(a, g, dir, stream));
   }
   if (kind == ANODE_KERNEL_RESIDENT) return launched(kind, launch_resident(a, dir, tiled_part_bytes(a.plan.dim0, a.plan.C, a.plan.N), stream));
-  if (kind == ANODE_KERNEL_PLAIN) return launched(kind, launch_pipeline(a, dir, stream));
+  if (kind == ANODE_KERNEL_PLAIN) {
+    // short rows without an aligned run of channels: the streaming kernel's masked form serves what the plain kernel is named for
+    StreamGeom sg;
+    if (kernel_choice() == ANODE_KERNEL_AUTO && aligned && masked_geom_of(a, dir, sg) &&
+        launched(ANODE_KERNEL_STREAM, launch_stream(a, dir, stream)) == ANODE_OK) return ANODE_OK;
+    return launched(kind, launch_pipeline(a, dir, stream));
+  }
   return ANODE_E_LAUNCH;
 }
 

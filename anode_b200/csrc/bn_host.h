@@ -16,6 +16,14 @@
 
 namespace anode_b200 {
 
+// Geometry of the streaming kernel (bn_stream.cu)
+struct StreamGeom {
+  uint32_t cb, units;        // channels per unit
+  uint32_t cluster, rows;    // blocks per unit, samples per block
+  uint32_t groups, threads;  // sample groups of a block: thread = group * vectors per run + vector
+  double inv_count;
+};
+
 struct Tunables {
   uint32_t tile_floats;     // target floats per tile
   uint32_t slack_steps;     // extra lookahead steps beyond the minimum
@@ -61,6 +69,9 @@ bool stream_applies(const FusedArgs &a, int dir, bool aligned);
 uint32_t stream_cluster(const FusedArgs &a, int dir, bool aligned, uint32_t &blocks);
 bool stream_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok);
 int launch_stream(FusedArgs &a, int dir, cudaStream_t stream);
+// its masked form for rows without an aligned run: the geometry of a shape, and of a prepared call on aligned tensors
+bool masked_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, StreamGeom &g);
+bool masked_geom_of(const FusedArgs &a, int dir, StreamGeom &g);
 bool stream_one_wave(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra);      // its grid, where it fills the device once
 // its form for the largest of them (bn_band.cu): the geometry of a shape where it is taken, and of a prepared call
 bool band_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, BandGeom &g);

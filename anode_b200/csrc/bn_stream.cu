@@ -13,6 +13,12 @@
 //
 // (The largest of these layers are walked once, by bn_band.cu, where the call has a workspace.)
 //
+// Rows without an aligned run (C*dim0 or every run of a few channels no multiple of four floats) take the masked form.  They went
+// float by float through the plain kernel, some 20 instructions per element and a grid-wide agreement; forward / backward, us, there
+// and here: [4096,23,7,7] 44 / 45 and 20 / 30, [647,340,351] 317 / 618 and 158 / 268, [2571,573,75] 450 / 610 and 240 / 369, [4160,7,33]
+// 21 / 20 and 8 / 10, residual [2374,147,83] 226 / 271 and 94 / 157.  Error against float64 over 60 shapes, there and here, geometric mean:
+// mean 4.9e-8 and 2.5e-8, variance 4.8e-8 and 3.0e-8, dgamma 1.5e-7 and 1.2e-7, dbeta 1.3e-7 and 7.9e-8.
+//
 // What bounds it: HBM and the loads in flight.  Nothing is staged in shared memory, so the blocks per SM are limited by
 // registers only and some stream while others fold and wait; the kernel that holds the slices in shared memory
 // (bn_segres.cu) runs its load, six dependent phases and store one after the other.
@@ -23,6 +29,8 @@
 //
 // Reference kernels this replaces: routines_gpu/batch_norm.cu:24-57, 125-163, 314-336 (forward), :181-206, 240-280,
 // 354-376, 408-444, 476-515 (backward), flat_map.cu:172-194 (ReLU).
+#include <math.h>
+
 #include "bn_device.cuh"
 #include "bn_host.h"
 
@@ -34,13 +42,6 @@ constexpr uint32_t kStreamThreads = 256, kStreamBlocks = 3;
 constexpr uint32_t kStreamRecords = 1024;    // most channels * blocks of a unit
 constexpr uint32_t kStreamChannels = 128;    // most channels of a unit
 
-struct StreamGeom {
-  uint32_t cb, units;        // channels per unit
-  uint32_t cluster, rows;    // blocks per unit, samples per block
-  uint32_t groups, threads;  // sample groups of a block: thread = group * vectors per run + vector
-  double inv_count;
-};
-
 // two doubles into the shared memory of block `rank` of the cluster, at the address `p` has in this block
 __device__ __forceinline__ void st_cluster_d2(void *p, uint32_t rank, double x, double y)
 {
@@ -50,10 +51,14 @@ __device__ __forceinline__ void st_cluster_d2(void *p, uint32_t rank, double x, 
   asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(remote), "d"(x), "d"(y) : "memory");
 }
 
-template <int DIR, bool EXTRA>
+// RAG: runs that begin anywhere (the masked form).  A thread's samples lie a multiple of four floats apart, so its 16-byte vectors,
+// from the boundary below the run's start to the one above its end, always lie over the run in the same way: floats lo to hi of a
+// vector are the run's, the others belong to a neighbour, have sums of their own in the thread and are left out when it is folded.
+template <int DIR, bool EXTRA, bool RAG>
 __global__ void __launch_bounds__(kStreamThreads, kStreamBlocks) bn_stream_kernel(const FusedArgs a, const StreamGeom g)
 {
-  constexpr int kBatch = DIR == 0 && !EXTRA ? 8 : 4;     // samples in flight per thread (more of them spill)
+  // samples in flight per thread (more of them spill; four of the masked residual backward, too)
+  constexpr int kBatch = DIR == 0 && !EXTRA ? 8 : RAG && DIR == 1 && EXTRA ? 3 : 4;
   __shared__ double2 part[2][kStreamThreads];            // per thread: its sums for the one or two channels of its column
   __shared__ double2 rec[kStreamRecords];                // [channel][block of the cluster]
   __shared__ float4 coef0[kStreamChannels];              // mean, gamma/std, beta, -
@@ -65,16 +70,33 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamBlocks) bn_stream_kerne
   // remote shared memory may only be written once its block runs (collected right before the first remote store)
   if (g.cluster > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   const uint32_t c0 = u * g.cb, cw = C - c0 < g.cb ? C - c0 : g.cb;
-  const uint32_t L4 = cw * dim0 / 4, rs = C * dim0;
+  const uint32_t run = cw * dim0, L4 = RAG ? (run + 6) / 4 : run / 4, rs = C * dim0;
   const uint32_t grp = tid / L4, v = tid - grp * L4;
   const uint32_t n0 = rank * g.rows, rows = n0 < N ? (N - n0 < g.rows ? N - n0 : g.rows) : 0;
-  const uint32_t nk = grp < g.groups && grp < rows ? (rows - grp - 1) / g.groups + 1 : 0;      // this thread's samples
   const uint32_t step = g.groups * rs;                   // float offsets are below 2^32 (check_dims) wherever k < nk
-  const uint32_t off0 = (n0 + grp) * rs + c0 * dim0 + 4 * v;
+  const uint32_t start = (n0 + grp) * rs + c0 * dim0, mis = RAG ? start & 3u : 0u;
+  const uint32_t off0 = start - mis + 4 * v;
+  const uint32_t lo = RAG && v == 0 ? mis : 0u, hi = !RAG || 4 * v + 4 <= run + mis ? 4u : 4 * v < run + mis ? run + mis - 4 * v : 0u;
+  const bool whole = !RAG || (lo == 0 && hi == 4);
+  const uint32_t nk = grp < g.groups && grp < rows && lo < hi ? (rows - grp - 1) / g.groups + 1 : 0;      // this thread's samples
   // the column's four floats lie in channel chA up to float eB, in the next one from there on
-  const uint32_t chA = grp < g.groups ? 4 * v / dim0 : 0;
-  const uint32_t eB = (chA + 1) * dim0 - 4 * v;
-  const uint32_t chB = eB < 4 && chA + 1 < cw ? chA + 1 : chA;
+  const uint32_t chA = grp < g.groups && lo < hi ? (4 * v + lo - mis) / dim0 : 0;
+  const uint32_t eB = (chA + 1) * dim0 + mis - 4 * v;
+  const uint32_t chB = eB < hi && chA + 1 < cw ? chA + 1 : chA;
+  // Of a tensor that ends inside a vector the floats up to its end are read one by one.
+  const uint32_t end = RAG ? N * rs - 4 : 0u;
+  auto load = [&](const float *p, uint32_t off, uint64_t pol) {
+    if (!RAG || off <= end) return Pack<4>::load(p + off, pol);
+    Pack<4> r = pack_fill<4>(0.f);
+#pragma unroll
+    for (int e = 0; e < 3; ++e) if (off + e < end + 4) r.v[e] = p[off + e];
+    return r;
+  };
+  auto store = [&](const Pack<4> &o, float *p, bool later) {      // later: the block reads it again
+    if (whole) { if (later) o.put(p); else o.store_stream(p); return; }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) if ((uint32_t)e >= lo && (uint32_t)e < hi) p[e] = o.v[e];
+  };
   const float slope = a.neg_slope;                       // activation: t * (t > 0 ? 1 : slope)
   const bool early = DIR == 1 && EXTRA && a.dres_early;  // dz is stored in the first walk and read back in the second
   const uint64_t keep = policy_keep(), drop = policy_drop();
@@ -103,9 +125,9 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamBlocks) bn_stream_kerne
       const uint32_t off = off0 + (k + i) * step;
       vx[i] = pack_fill<4>(0.f);
       if (k + i < nk) {
-        vx[i] = Pack<4>::load(a.x + off, keep);
-        if (DIR == 1) vd[i] = Pack<4>::load(a.dy + off, early ? drop : keep);
-        if (DIR == 1 && EXTRA) vm[i] = Pack<4>::load(a.ymask + off, early ? drop : keep);
+        vx[i] = load(a.x, off, keep);
+        if (DIR == 1) vd[i] = load(a.dy, off, early ? drop : keep);
+        if (DIR == 1 && EXTRA) vm[i] = load(a.ymask, off, early ? drop : keep);
       }
     }
     if (DIR == 0) {
@@ -142,7 +164,7 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamBlocks) bn_stream_kerne
             vd[i].v[e] *= yb > 0.0f ? 1.0f : slope;      // dz = dy * act'(y)  (routines_gpu/flat_map.cu:191-192)
             s[e] += vd[i].v[e]; q[e] = fmaf(vd[i].v[e], d, q[e]);
           }
-          if (EXTRA && early) vd[i].put(a.dres + (off0 + (k + i) * step));
+          if (EXTRA && early) store(vd[i], a.dres + (off0 + (k + i) * step), true);
         }
     }
   }
@@ -159,6 +181,7 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamBlocks) bn_stream_kerne
         t2 = fma(k, fma(n, k, 2.0 * t1), t2); t1 = fma(n, k, t1);
       }
       const bool b = (uint32_t)e >= eB;
+      if (RAG && ((uint32_t)e < lo || (uint32_t)e >= hi)) t1 = t2 = 0.0;
       p[0].x += b ? 0.0 : t1; p[0].y += b ? 0.0 : t2;
       p[1].x += b ? t1 : 0.0; p[1].y += b ? t2 : 0.0;
     }
@@ -169,11 +192,12 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamBlocks) bn_stream_kerne
   // ---- the block's sums: one warp per channel over the threads whose column touches it, in a fixed order
   if (g.cluster > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   for (uint32_t ci = warp; ci < cw; ci += warps) {
-    const uint32_t v0 = ci * dim0 / 4, nv = (ci * dim0 + dim0 - 1) / 4 - v0 + 1;
+    const uint32_t f0 = ci * dim0, nv = RAG ? (dim0 + 6) / 4 : (f0 + dim0 - 1) / 4 - f0 / 4 + 1;
     double t1 = 0.0, t2 = 0.0;
     for (uint32_t i = lane; i < nv * g.groups; i += 32) {
-      const uint32_t gi = i / nv, vi = v0 + i - gi * nv;
-      const double2 p = part[4 * vi < ci * dim0 ? 1 : 0][gi * L4 + vi];     // (a column that starts in the channel before)
+      const uint32_t gi = i / nv, m = RAG ? ((n0 + gi) * rs + c0 * dim0) & 3u : 0u, vi = (f0 + m) / 4 + i - gi * nv;
+      if (RAG && 4 * vi >= f0 + dim0 + m) continue;
+      const double2 p = part[ci > 0 && 4 * vi < f0 + m ? 1 : 0][gi * L4 + vi];     // (a column that starts in the channel before)
       t1 += p.x; t2 += p.y;
     }
     t1 = warp_sum_all(t1); t2 = warp_sum_all(t2);
@@ -233,14 +257,14 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamBlocks) bn_stream_kerne
     if (DIR == 0) {
       if (k != kb) {
 #pragma unroll
-        for (int i = 0; i < kBatch; ++i) vx[i] = Pack<4>::load(a.x + (off0 + (k + i) * step), drop);      // (only the last batch is short)
+        for (int i = 0; i < kBatch; ++i) vx[i] = load(a.x, off0 + (k + i) * step, drop);      // (only the last batch is short)
       }
 #pragma unroll
       for (int h = 0; h < kBatch; h += 4) {
         Pack<4> ve[EXTRA ? 4 : 1];
         if (EXTRA) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) if (k + h + i < nk) ve[i] = Pack<4>::load(a.res + (off0 + (k + h + i) * step), drop);
+          for (int i = 0; i < 4; ++i) if (k + h + i < nk) ve[i] = load(a.res, off0 + (k + h + i) * step, drop);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
@@ -252,7 +276,7 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamBlocks) bn_stream_kerne
               if (EXTRA) yb += ve[i].v[e];
               o.v[e] = yb * (yb > 0.0f ? 1.0f : slope);
             }
-            o.store_stream(a.out + (off0 + (k + h + i) * step));
+            store(o, a.out + (off0 + (k + h + i) * step), false);
           }
       }
     } else {
@@ -262,9 +286,9 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamBlocks) bn_stream_kerne
 #pragma unroll
         for (int i = 0; i < kBatch; ++i) {
           const uint32_t off = off0 + (k + i) * step;
-          vx[i] = Pack<4>::load(a.x + off, drop);
-          vd[i] = Pack<4>::load(second + off, drop);
-          if (EXTRA && !early) vm[i] = Pack<4>::load(a.ymask + off, drop);
+          vx[i] = load(a.x, off, drop);
+          vd[i] = load(second, off, drop);
+          if (EXTRA && !early) vm[i] = load(a.ymask, off, drop);
         }
         if (!early) {
 #pragma unroll
@@ -281,14 +305,14 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamBlocks) bn_stream_kerne
         if (k + i < nk) {
           const uint32_t off = off0 + (k + i) * step;
           Pack<4> o;
-          if (a.accumulate) o = Pack<4>::load(a.out + off);
+          if (a.accumulate) o = RAG ? load(a.out, off, drop) : Pack<4>::load(a.out + off);
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const float dx = fmaf(scale[e], vd[i].v[e], fmaf(cB[e], vx[i].v[e] - mean[e], cC[e]));
             o.v[e] = a.accumulate ? o.v[e] + dx : dx;
           }
-          o.store_stream(a.out + off);
-          if (EXTRA && !early && a.dres) vd[i].store_stream(a.dres + off);
+          store(o, a.out + off, false);
+          if (EXTRA && !early && a.dres) store(vd[i], a.dres + off, false);
         }
     }
     if (k == 0) break;
@@ -364,6 +388,50 @@ static bool stream_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool ext
   return true;
 }
 
+// The masked form (RAG): runs of any channels.  The samples of a thread lie a multiple of four floats apart, so the groups of a
+// block are an even number or a multiple of four where C*dim0 asks for it (unless a thread has one sample anyway), and rows are
+// no longer than leaves place for those.
+// Unit and cluster are those of the least estimated time: a fixed part per wave of blocks (clusters of 8 and 16 fill 85 and 78 per
+// cent of the device's places), and the larger of a thread's chain of batches and the bytes moved, where the cache lines that two
+// runs share come twice, what exceeds L2 between the two walks comes again, and idle threads leave bandwidth unused.  The
+// figures are fitted to 570 launches of 60 shapes (16 to 480 floats a row, 3 to 1500 channels, 0.6 to 120 M elements, four
+// directions) with up to 30 units and clusters each: what is chosen is 3 per cent above the best of them on average; the least
+// idle threads and the aligned form's clusters, as chosen there, were 11 per cent slower over 70 other shapes, a third at 3 to 10 channels.
+bool masked_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, StreamGeom &g)
+{
+  const uint32_t rs = C * dim0, m = rs % 4 == 0 ? 1u : rs % 2 == 0 ? 2u : 4u, wave = kStreamBlocks * sm_count();
+  StreamGeom aligned;
+  if (dim0 < 4 || stream_geom(dim0, C, N, dir, extra, aligned)) return false;
+  const double bytes = 4.0 * dim0 * C * N * (dir == 0 ? (extra ? 3 : 2) : extra ? 5 : 3);
+  const double batch_us = (dir == 0 && !extra ? 1.5 : 2.0) / (dir == 0 ? (extra ? 4 : 8) : extra ? 3 : 4);      // per sample of a thread
+  const double window = 77e6, rate = 5.15e6;      // bytes that L2 keeps; bytes per us
+  double best = 0;
+  for (uint32_t cb = 1; cb <= C && cb <= kStreamChannels && (cb * dim0 + 6) / 4 <= kStreamThreads; ++cb) {
+    const uint32_t run = cb * dim0, L4 = (run + 6) / 4, units = ceil_div_u32(C, cb);
+    if (run < 16 && cb < C) continue;
+    uint32_t groups = kStreamThreads / L4;
+    groups = groups >= N ? N : groups / m * m;
+    if (groups == 0) break;
+    for (uint32_t cl = 1; cl <= 16 && cl * cb <= kStreamRecords && (cl == 1 || N / cl >= groups * 2); cl *= 2) {
+      const uint64_t blocks = (uint64_t)units * cl, places = cl == 16 ? wave * 25 / 32 : cl == 8 ? wave * 17 / 20 : cl == 4 ? wave * 15 / 16 : wave;
+      const double waves = (double)((blocks + places - 1) / places), resident = (double)(blocks < places ? blocks : places);
+      const uint32_t rows = ceil_div_u32(N, cl), used = groups < rows ? groups : rows;
+      const double over = 4.0 * run * N * (dir == 1 ? 2 : 1) / cl * resident / window - 1;
+      const double again = (dir == 1 ? 0.5 : 0.17) * (over < 0 ? 0 : over > 1 ? 1 : over), lanes = resident * used * L4 / ((double)wave * kStreamThreads);
+      const double moved = bytes * (1 + 9.0 / run) * (1 + again) / rate * (0.9 + 0.1 / lanes);
+      const double chain = waves * ceil_div_u32(rows, used) * batch_us;
+      const double cost = 0.6 + waves * (3.0 + 0.024 * cl) + pow(pow(moved, 2.5) + pow(chain, 2.5), 0.4);
+      if (best == 0 || cost < best) {
+        best = cost;
+        g.cb = cb; g.units = units; g.cluster = cl; g.rows = rows; g.groups = used;
+        g.threads = (used * L4 + 31) / 32 * 32;
+      }
+    }
+  }
+  g.inv_count = 1.0 / ((double)dim0 * (double)N);
+  return best != 0;
+}
+
 // Whether the grid is one wave of blocks, all resident, that fills the device: nothing of a second wave to pay for.
 bool stream_one_wave(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra)
 {
@@ -421,12 +489,15 @@ bool stream_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
 int launch_stream(FusedArgs &a, int dir, cudaStream_t stream)
 {
   StreamGeom g;
-  if (!stream_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, stream_extra(a, dir), g)) return ANODE_E_LAUNCH;
+  const bool masked = !stream_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, stream_extra(a, dir), g);
+  if (masked && !masked_geom_of(a, dir, g)) return ANODE_E_LAUNCH;
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
   // dres may be stored before x is read again only where it is not x itself
   a.dres_early = a.dres && a.dres != a.x ? 1u : 0u;
-  auto kernel = dir == 0 ? (extra ? bn_stream_kernel<0, true> : bn_stream_kernel<0, false>)
-                         : (extra ? bn_stream_kernel<1, true> : bn_stream_kernel<1, false>);
+  auto kernel = dir == 0 ? (extra ? bn_stream_kernel<0, true, false> : bn_stream_kernel<0, false, false>)
+                         : (extra ? bn_stream_kernel<1, true, false> : bn_stream_kernel<1, false, false>);
+  if (masked) kernel = dir == 0 ? (extra ? bn_stream_kernel<0, true, true> : bn_stream_kernel<0, false, true>)
+                                : (extra ? bn_stream_kernel<1, true, true> : bn_stream_kernel<1, false, true>);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(g.units * g.cluster);
   cfg.blockDim = dim3(g.threads);
@@ -468,5 +539,16 @@ extern "C" int anode_gpu_batch_norm_stream_geometry(uint32_t dim0, uint32_t dim1
   const bool ok = stream_geom(dim0, dim1, dim2, dir, false, g);
   const uint32_t v[7] = {ok ? 1u : 0u, g.cb, g.units, g.cluster, g.rows, g.groups, g.threads};
   for (int i = 0; i < 7; ++i) out[i] = v[i];
+  return ANODE_OK;
+}
+
+extern "C" int anode_gpu_batch_norm_stream_masked_geometry(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual, uint32_t *out)
+{
+  using namespace anode_b200;
+  if (!out || (dir != 0 && dir != 1) || check_dims(dim0, dim1, dim2)) return ANODE_E_DIMS;
+  StreamGeom g{};
+  const bool ok = masked_plan(dim0, dim1, dim2, dir, residual != 0, g);
+  const uint32_t v[7] = {ok ? 1u : 0u, g.cb, g.units, g.cluster, g.rows, g.groups, g.threads};
+  for (int i = 0; i < 7; ++i) out[i] = ok || i == 0 ? v[i] : 0u;
   return ANODE_OK;
 }
