@@ -551,6 +551,32 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
   return resident_applies(a, dir, aligned) ? ANODE_KERNEL_RESIDENT : -1;
 }
 
+// Rows without an aligned run of channels, on one GPU: where the streaming kernel's masked form is launched in the place of the kernel
+// that pick_kernel_kind names.  Us there and here, forward, backward, residual forward and backward:
+//  - the plain kernel everywhere (figures at the head of bn_stream.cu);
+//  - the register-resident kernel, which loads such rows float by float, from these sizes and twenty samples on: [1084,111,18], 2.2 M,
+//    9.7, 16.6, 16.3, 29.7 and 8.6, 11.3, 10.4, 13.4; [270,490,49] 22.9, 34.9, 34.8, 61.1 and 15.8, 22.6, 19.6, 30.1; [356,2022,25] 59, 84, 85, 157
+//    and 35, 56, 46, 80; but [67,706,37], 1.75 M, 5.2, 8.1, 7.6, 15.7 and 6.6, 8.9, 8.4, 10.2, [802,67,19], 1.0 M, 4.5, 5.5, 5.0, 7.2 and 6.6,
+//    8.1, 7.8, 9.3, and few samples, [16,2017,151] 17.5, 22.2, 22.6, 39.7 and 22.4, 23.8, 25.1, 32.9;
+//  - the tiled kernel, which copies a row at a time, on rows below 200 floats: [604,18,221] 16.4, 20.5, 18.5, 25.6 and 9.3, 11.7, 10.6, 14.8,
+//    [1826,159,179] 128, 246, 213, - and 118, 186, 153, -, [1403,355,131] forward 191 and 143; but [1594,54,227] 54, 81, 77, 101 and 58, 80, 69, 107;
+//    on longer ones in small layers, where the tiled kernel's launch costs ten us: [947,13,350] 19.5, 25.0, 22.6, 27.5 and 13.3, 22.7, 20.1,
+//    30.6, but [2147,15,254], 8.2 M, 27.5, 42.0, 39.0, 49.4 and 29.2, 46.1, 42.6, 63.5.
+constexpr uint32_t kMaskedSamples = 20, kMaskedShortRow = 200;
+constexpr uint64_t kMaskedChan[2][2] = {{2100000, 1900000}, {1900000, 1100000}};        // [direction][residual]
+constexpr uint64_t kMaskedTiled[2][2] = {{8000000, 5000000}, {4500000, 2500000}};
+static bool masked_takes(const FusedArgs &a, int dir, int kind)
+{
+  StreamGeom g;
+  if (kernel_choice() != ANODE_KERNEL_AUTO || a.plan.dim0 % 4 == 0) return false;
+  if (kind != ANODE_KERNEL_REGISTER && kind != ANODE_KERNEL_TILED && kind != ANODE_KERNEL_PLAIN) return false;
+  const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
+  const uint64_t elements = (uint64_t)a.plan.dim0 * a.plan.C * a.plan.N;
+  if (kind == ANODE_KERNEL_REGISTER && (a.plan.N < kMaskedSamples || elements < kMaskedChan[dir][extra])) return false;
+  if (kind == ANODE_KERNEL_TILED && a.plan.dim0 >= kMaskedShortRow && (a.plan.N < kMaskedSamples || elements > kMaskedTiled[dir][extra])) return false;
+  return masked_geom_of(a, dir, g);
+}
+
 static thread_local int t_last_kernel = -1;
 
 // Launches direction `dir` of a prepared call with the kernel pick_kernel_kind names.  A cluster launch
@@ -559,6 +585,7 @@ int launch_best(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)
 {
   int kind = pick_kernel_kind(a, dir, aligned);
   auto launched = [&](int k, int rc) { if (rc == ANODE_OK) t_last_kernel = k; return rc; };
+  if (aligned && masked_takes(a, dir, kind) && launched(ANODE_KERNEL_STREAM, launch_stream(a, dir, stream)) == ANODE_OK) return ANODE_OK;
   if (kind == ANODE_KERNEL_REGISTER) return launched(kind, launch_chan(a, dir, aligned, stream));
   if (kind == ANODE_KERNEL_STREAM) {
     BandGeom bg;
@@ -581,13 +608,7 @@ int launch_best(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)
     return launched(kind, launch_ring(a, g, dir, stream));
   }
   if (kind == ANODE_KERNEL_RESIDENT) return launched(kind, launch_resident(a, dir, tiled_part_bytes(a.plan.dim0, a.plan.C, a.plan.N), stream));
-  if (kind == ANODE_KERNEL_PLAIN) {
-    // short rows without an aligned run of channels: the streaming kernel's masked form serves what the plain kernel is named for
-    StreamGeom sg;
-    if (kernel_choice() == ANODE_KERNEL_AUTO && aligned && masked_geom_of(a, dir, sg) &&
-        launched(ANODE_KERNEL_STREAM, launch_stream(a, dir, stream)) == ANODE_OK) return ANODE_OK;
-    return launched(kind, launch_pipeline(a, dir, stream));
-  }
+  if (kind == ANODE_KERNEL_PLAIN) return launched(kind, launch_pipeline(a, dir, stream));
   return ANODE_E_LAUNCH;
 }
 

@@ -185,12 +185,12 @@ void anode_gpu_positive_clip_flat_map_bwd_f32(
  *   CLUSTER   thread-block clusters keeping a unit's slice in shared memory (short rows, small channels);
  *   RESIDENT  slices resident in shared memory, all global traffic by bulk copies; takes the residual
  *             epilogue on long rows, also in synchronized calls;
- *   PLAIN     plain loads and stores (any shape, any alignment; one GPU).  Calls on 16-byte aligned tensors that fall to it by
- *             shape, short rows without an aligned run of channels, are launched as STREAM's masked form where that applies;
+ *   PLAIN     plain loads and stores (any shape, any alignment; one GPU);
  *   REGISTER  channels held in the registers of a warp, a block or a cluster (small layers, any alignment;
  *             one GPU);
  *   STREAM    clusters that walk a block of channels twice (layers of short rows; one GPU); its masked form takes runs of
- *             channels that begin anywhere;
+ *             channels that begin anywhere, in the place of PLAIN and, where it is the faster one, of REGISTER and TILED: queries by
+ *             shape name those;
  *   BAND      its form for the largest of them, where the call has a workspace: one walk, with the tiles in tensor memory
  *             between reduction and normalization.  Queries by shape count it as STREAM.  It is launched cooperatively and takes
  *             the whole device, so other streams' kernels run before or after it, not beside it.

@@ -6,6 +6,7 @@ import ctypes
 
 import numpy as np
 import pytest
+import torch
 
 from tests.test_gpu_fused import run_fused
 from tests.test_gpu_random_shapes import run_add_act
@@ -142,3 +143,28 @@ def test_it_serves_what_the_plain_kernel_is_named_for(shape):
     got, _ = run_fused(ops, d)
     assert ops.last_kernel() == "stream"
     check_layer_own_mask(d, got, "%r " % (shape,))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape,named,launched", [
+    ((1084, 111, 1, 18), ["register"] * 4, ["stream"] * 4), ((67, 706, 1, 37), ["register"] * 4, ["register"] * 3 + ["stream"]),
+    ((16, 2017, 1, 151), ["register"] * 4, ["register"] * 4), ((604, 18, 13, 17), ["tiled"] * 4, ["stream"] * 4),
+    ((2147, 15, 1, 254), ["tiled"] * 4, ["tiled"] * 4), ((1841, 15, 1, 165), ["tiled"] * 3 + ["plain"], ["stream"] * 4)])
+def test_where_it_is_launched(shape, named, launched):
+    from anode_b200 import ops
+    assert [ops.serving_kernel(shape, d, residual=r) for r in (False, True) for d in (0, 1)] == named
+    d = make_inputs(shape, seed=sum(shape), loc=1.0, scale=2.0)
+    x, dy = torch.from_numpy(d["x"]).cuda(), torch.from_numpy(d["dy"]).cuda()
+    c, got, op = shape[1], [], ops.BatchNormalize2dAddActFusedOp
+    z = lambda: torch.zeros(c, device="cuda")
+    mean, var, rm, rv, dg, db, y, dx, dr = z(), z(), z(), z(), z(), z(), torch.empty_like(x), torch.empty_like(x), torch.empty_like(x)
+    ws = ops.Workspace(*ops.dims_of(x), x.device)
+    for call in (lambda: ops.BatchNormalize2dFusedOp.apply([0, 1], 1e-5, 0.1, x, y, mean, var, rm, rv, None, None, workspace=ws, neg_slope=0.0),
+                 lambda: ops.BatchNormalize2dBwdFusedOp.apply([0, 1], dy, x, mean, var, dx, None, None, dg, db, workspace=ws, neg_slope=0.0),
+                 lambda: op.apply([0, 1], 1e-5, 0.1, x, dy, y, mean, var, rm, rv, None, None, 0.0, ws),
+                 lambda: op.adjoint([0, 1], dy, x, y, mean, var, dx, dr, None, None, dg, db, 0.0, workspace=ws)):
+        call()
+        got.append(ops.last_kernel())
+    assert got == launched and ws.status() == 0
+    run, _ = run_fused(ops, d)
+    check_layer_own_mask(d, run, "%r " % (shape,))
