@@ -57,11 +57,14 @@ struct FusedArgs {
 
 // 1/sqrt(v) as every kernel here computes it (IEEE divide and square root), so that the
 // forward pass and the backward pass derive bit-identical scales, hence identical ReLU masks.
-// The lowest mantissa bit is forced to one: the value can then never have an all-zero bit
-// pattern, which lets a 64-bit (mean, rstd) record double as its own "ready" flag.
+// Its lowest bit is one: of the two such values beside the rounded quotient the nearer one (with the bit set by an OR, upwards, y's
+// relative error against float64 over 100 layers was 8.3e-8 to 9.0e-8 by the kernel, so 7.1e-8 to 7.6e-8).
 __device__ __forceinline__ float inv_std(float v)
 {
-  return __uint_as_float(__float_as_uint(__fdiv_rn(1.0f, __fsqrt_rn(v))) | 1u);
+  const float r = __fdiv_rn(1.0f, __fsqrt_rn(v)), t = __fmul_rn(v, r);
+  const float past = fmaf(-t, r, 1.0f) - fmaf(v, r, -t) * r;      // 1 - v r^2: below zero where r lies above 1/sqrt(v)
+  const uint32_t u = __float_as_uint(r);
+  return __uint_as_float(u & 1u ? u : past < 0.0f ? u - 1u : u + 1u);      // (no number: as the OR)
 }
 
 // Tagged per-channel records in the workspace: zero = not ready; written once per launch with a
