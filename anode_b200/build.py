@@ -14,7 +14,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libanode_routines_gpu.so")
 NATIVE = os.path.join(HERE, "_native.so")
 NATIVE_SOURCE = os.path.join(CSRC, "bn_py.cpp")
-SOURCES = ["bn_fused.cu", "bn_legacy.cu", "bn_compose.cu", "bn_sync.cu", "bn_static.cu", "bn_hoststep.cu", "bn_segres.cu", "bn_chan.cu", "bn_stream.cu", "bn_band.cu", "bn_infer.cu", "bn_resident.cu", "bn_resident_diag.cpp"]
+SOURCES = ["bn_fused.cu", "bn_legacy.cu", "bn_compose.cu", "bn_sync.cu", "bn_static.cu", "bn_hoststep.cu", "bn_segres.cu", "bn_chan.cu", "bn_stream.cu", "bn_long.cu", "bn_band.cu", "bn_infer.cu", "bn_resident.cu", "bn_resident_diag.cpp"]
 HEADERS = ["bn_plan.h", "bn_device.cuh", "bn_fused.cuh", "bn_ring.cuh", "bn_pipe.cuh", "bn_band.cuh", "bn_resident_plan.h", "bn_host.h", "bn_sync.h",
            os.path.join("..", "..", "include", "anode_routines_gpu.h")]
 

@@ -134,6 +134,15 @@ __device__ __forceinline__ float positive_clip(float x) { return x * (x > 0.0f ?
 // a channel that holds a NaN or an infinity has no variance, and its running average must show it.
 __device__ __forceinline__ double not_below_zero(double v) { return v < 0.0 ? 0.0 : v; }
 
+// two doubles into the shared memory of block `rank` of the cluster, at the address `p` has in this block
+__device__ __forceinline__ void st_cluster_d2(void *p, uint32_t rank, double x, double y)
+{
+  const uint32_t local = (uint32_t)__cvta_generic_to_shared(p);
+  uint32_t remote;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
+  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(remote), "d"(x), "d"(y) : "memory");
+}
+
 // ---- reductions ------------------------------------------------------------------------
 struct Moments { float n, mean, m2; };
 

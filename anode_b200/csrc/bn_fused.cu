@@ -93,6 +93,8 @@ struct ShapeInfo {
   BandGeom band[2][2];
   bool masked_ok[2][2];          // the streaming kernel's masked form, likewise
   StreamGeom masked[2][2];
+  bool long_ok[2][2];            // its counterpart for long rows, likewise
+  LongGeom long_rows[2][2];
 };
 constexpr uint32_t kShapeCache = 64;      // entries per thread, direct mapped
 
@@ -466,7 +468,10 @@ static void fill_shape_info(ShapeInfo &s)
     if (at > s.part_bytes) s.part_bytes = at;
   }
   for (int dir = 0; dir < 2; ++dir)
-    for (int ex = 0; ex < 2; ++ex) s.masked_ok[dir][ex] = masked_plan(s.dim0, s.C, s.N, dir, ex != 0, s.masked[dir][ex]);
+    for (int ex = 0; ex < 2; ++ex) {
+      s.masked_ok[dir][ex] = masked_plan(s.dim0, s.C, s.N, dir, ex != 0, s.masked[dir][ex]);
+      s.long_ok[dir][ex] = long_plan(s.dim0, s.C, s.N, dir, ex != 0, s.long_rows[dir][ex]);
+    }
 }
 
 bool masked_geom_of(const FusedArgs &a, int dir, StreamGeom &g)
@@ -485,6 +490,15 @@ bool band_geom_of(const FusedArgs &a, int dir, BandGeom &g)
   if (!s.band_ok[dir][extra]) return false;
   g = s.band[dir][extra];
   return a.bands && a.ws_capacity >= g.tag + band_words(g) * 2 * kBandWordBytes;
+}
+
+bool long_geom_of(const FusedArgs &a, int dir, LongGeom &g)
+{
+  const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
+  if (a.mode != MODE_FUSED || a.world > 1) return false;
+  const ShapeInfo &s = shape_info(a.plan.dim0, a.plan.C, a.plan.N);
+  if (s.long_ok[dir][extra]) g = s.long_rows[dir][extra];
+  return s.long_ok[dir][extra];
 }
 
 // Bytes of a part taken by the tile-plan kernels (plain, warp-specialised, cluster); the records of the
@@ -565,16 +579,56 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
 constexpr uint32_t kMaskedSamples = 20, kMaskedShortRow = 200;
 constexpr uint64_t kMaskedChan[2][2] = {{2100000, 1900000}, {1900000, 1100000}};        // [direction][residual]
 constexpr uint64_t kMaskedTiled[2][2] = {{8000000, 5000000}, {4500000, 2500000}};
-static bool masked_takes(const FusedArgs &a, int dir, int kind)
+static bool masked_takes(const FusedArgs &a, int dir, int kind, StreamGeom &g)
 {
-  StreamGeom g;
-  if (kernel_choice() != ANODE_KERNEL_AUTO || a.plan.dim0 % 4 == 0) return false;
-  if (kind != ANODE_KERNEL_REGISTER && kind != ANODE_KERNEL_TILED && kind != ANODE_KERNEL_PLAIN) return false;
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
   const uint64_t elements = (uint64_t)a.plan.dim0 * a.plan.C * a.plan.N;
+  if (a.plan.dim0 % 4 == 0) return false;
   if (kind == ANODE_KERNEL_REGISTER && (a.plan.N < kMaskedSamples || elements < kMaskedChan[dir][extra])) return false;
   if (kind == ANODE_KERNEL_TILED && a.plan.dim0 >= kMaskedShortRow && (a.plan.N < kMaskedSamples || elements > kMaskedTiled[dir][extra])) return false;
   return masked_geom_of(a, dir, g);
+}
+
+// Rows of 250 floats and more, on one GPU: where the kernel for long rows (bn_long.cu) is launched in the place of the one that
+// pick_kernel_kind names.  Us there and here, forward, backward, residual forward and backward:
+//  - the tiled kernel where its launch (twelve us and the layer's bytes) is more than the estimate of the other: [1,3,64,64,64] 12.5,
+//    12.4, -, - and 6.0, 7.9, -, -, [1,11,99716] -, 13.8, 13.2, 13.0 and -, 7.2, 6.7, 9.2, [3,19,75580], 4.3 M, 16.6, 18.0, 17.7, 26.4 and 10.3, 15.2,
+//    15.1, 19.4; but [1,4,1630016], 6.5 M, 19.4, 25.2, 22.3, 31.8 and 28.6, 47.6, 47.3, 58.0.  By that rule 0.8 per cent are lost against the
+//    better of the two over 439 passes of 0.3 to 20 M elements;
+//  - the register-resident kernel on ragged rows, which it loads float by float, from these sizes or channels on: [8,217,2678] 18.5, 29.8,
+//    30.9, 52.6 and 12.7, 16.1, 14.5, 20.6, [2,5,19011] 3.8, 5.2, 5.2, 6.9 and 5.1, 4.1, 4.5, 4.6, [9,4,12887] forward 8.1 and 5.5, but
+//    [10,119,1502], 1.8 M, 5.4, 8.5, 8.0 and 7.9, 10.0, 9.8; and on aligned ones in the residual epilogue: [6,276,2060], 3.4 M, 11.7, 16.9 and 10.8,
+//    15.7, [7,331,1108], 2.6 M, backward 12.9 and 10.5.
+constexpr uint32_t kLongRow = 250;
+constexpr uint64_t kLongTiledMost = 12000000;
+constexpr uint64_t kLongChan[2][2] = {{3300000, 1800000}, {1800000, 700000}};           // [direction][residual]
+constexpr uint64_t kLongChannel[2][2] = {{64 << 10, 32 << 10}, {32 << 10, 24 << 10}};
+constexpr uint64_t kLongChanAligned[2][2] = {{~0ull, 3000000}, {~0ull, 2400000}};
+static bool long_takes(const FusedArgs &a, int dir, int kind, LongGeom &g)
+{
+  const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
+  const uint64_t channel = (uint64_t)a.plan.dim0 * a.plan.N, elements = channel * a.plan.C;
+  if (a.plan.dim0 < kLongRow) return false;
+  if (kind == ANODE_KERNEL_TILED)
+    return elements <= kLongTiledMost && long_geom_of(a, dir, g) && g.cost * 1.05f < 12.0f + (float)elements * (dir == 0 ? (extra ? 12 : 8) : extra ? 20 : 12) * 1.6e-7f;
+  if (kind != ANODE_KERNEL_REGISTER) return false;
+  return (a.plan.dim0 % 4 == 0 ? elements >= kLongChanAligned[dir][extra] : elements >= kLongChan[dir][extra] || channel >= kLongChannel[dir][extra]) &&
+         long_geom_of(a, dir, g);
+}
+
+// Launches the one of those two that takes the call, if any.
+static int launch_instead(FusedArgs &a, int dir, int kind, bool aligned, cudaStream_t stream)
+{
+  if (!aligned || a.mode != MODE_FUSED || a.world > 1 ||
+      (kind != ANODE_KERNEL_REGISTER && kind != ANODE_KERNEL_TILED && kind != ANODE_KERNEL_PLAIN)) return -1;
+  StreamGeom sg; LongGeom lg;
+  const int choice = kernel_choice();
+  bool masked = choice == ANODE_KERNEL_AUTO && masked_takes(a, dir, kind, sg);
+  bool rows = choice == ANODE_KERNEL_AUTO ? long_takes(a, dir, kind, lg) : choice == ANODE_KERNEL_LONG && long_geom_of(a, dir, lg);
+  if (masked && rows) (lg.cost < sg.cost ? masked : rows) = false;
+  if (masked && launch_stream(a, dir, stream) == ANODE_OK) return ANODE_KERNEL_STREAM;
+  if (rows && launch_long(a, lg, dir, stream) == ANODE_OK) return ANODE_KERNEL_LONG;
+  return -1;
 }
 
 static thread_local int t_last_kernel = -1;
@@ -585,7 +639,8 @@ int launch_best(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)
 {
   int kind = pick_kernel_kind(a, dir, aligned);
   auto launched = [&](int k, int rc) { if (rc == ANODE_OK) t_last_kernel = k; return rc; };
-  if (aligned && masked_takes(a, dir, kind) && launched(ANODE_KERNEL_STREAM, launch_stream(a, dir, stream)) == ANODE_OK) return ANODE_OK;
+  const int instead = launch_instead(a, dir, kind, aligned, stream);
+  if (instead >= 0) return launched(instead, ANODE_OK);
   if (kind == ANODE_KERNEL_REGISTER) return launched(kind, launch_chan(a, dir, aligned, stream));
   if (kind == ANODE_KERNEL_STREAM) {
     BandGeom bg;
@@ -926,7 +981,7 @@ extern "C" int anode_gpu_batch_norm_add_act_fused_kernel_kind(uint32_t dim0, uin
 
 extern "C" int anode_gpu_batch_norm_fused_set_kernel(int kernel)
 {
-  if (kernel < ANODE_KERNEL_AUTO || kernel > ANODE_KERNEL_BAND) return ANODE_E_DIMS;
+  if (kernel < ANODE_KERNEL_AUTO || kernel > ANODE_KERNEL_LONG) return ANODE_E_DIMS;
   g_kernel_choice.store(kernel, std::memory_order_relaxed);
   return ANODE_OK;
 }

@@ -21,8 +21,54 @@ struct StreamGeom {
   uint32_t cb, units;        // channels per unit
   uint32_t cluster, rows;    // blocks per unit, samples per block
   uint32_t groups, threads;  // sample groups of a block: thread = group * vectors per run + vector
+  float cost;                // masked form: estimated us
   double inv_count;
 };
+
+// Geometry of its counterpart for long rows (bn_long.cu)
+struct LongGeom {
+  uint32_t cluster, stride;         // blocks per channel, distance between a thread's vectors
+  uint32_t per_row, total;          // vectors per row and per channel
+  uint32_t step_rows, step_col;     // a step of `stride` vectors
+  float cost;                       // estimated us
+  double inv_count;
+};
+
+// Launch of a grid of clusters that may overlap the tail of the kernel before it on the stream (every block waits for that kernel's
+// results before it touches memory).  ANODE_E_LAUNCH where the device refuses it.
+template <typename Geom>
+inline int launch_clusters(void (*kernel)(const FusedArgs, const Geom), const FusedArgs &a, const Geom &g, uint32_t blocks, uint32_t threads,
+                           uint32_t cluster, cudaStream_t stream)
+{
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // (as launch_chan)
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 2;
+  if (cluster > 8) {
+    // larger than the portable size: asked for once per kernel and device
+    static std::mutex mu;
+    static std::map<std::pair<const void *, int>, bool> allowed;
+    int dev = 0;
+    (void)cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    const auto key = std::make_pair((const void *)kernel, dev);
+    auto it = allowed.find(key);
+    if (it == allowed.end()) {
+      const bool ok = cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+      if (!ok) (void)cudaGetLastError();
+      it = allowed.emplace(key, ok).first;
+    }
+    if (!it->second) return ANODE_E_LAUNCH;
+  }
+  if (cudaLaunchKernelEx(&cfg, kernel, a, g) != cudaSuccess) { (void)cudaGetLastError(); return ANODE_E_LAUNCH; }
+  return ANODE_OK;
+}
 
 struct Tunables {
   uint32_t tile_floats;     // target floats per tile
@@ -72,6 +118,10 @@ int launch_stream(FusedArgs &a, int dir, cudaStream_t stream);
 // its masked form for rows without an aligned run: the geometry of a shape, and of a prepared call on aligned tensors
 bool masked_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, StreamGeom &g);
 bool masked_geom_of(const FusedArgs &a, int dir, StreamGeom &g);
+// its counterpart for small layers of long rows (bn_long.cu), likewise
+bool long_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, LongGeom &g);
+bool long_geom_of(const FusedArgs &a, int dir, LongGeom &g);
+int launch_long(FusedArgs &a, const LongGeom &g, int dir, cudaStream_t stream);
 bool stream_one_wave(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra);      // its grid, where it fills the device once
 // its form for the largest of them (bn_band.cu): the geometry of a shape where it is taken, and of a prepared call
 bool band_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, BandGeom &g);

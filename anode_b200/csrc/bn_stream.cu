@@ -42,15 +42,6 @@ constexpr uint32_t kStreamThreads = 256, kStreamBlocks = 3;
 constexpr uint32_t kStreamRecords = 1024;    // most channels * blocks of a unit
 constexpr uint32_t kStreamChannels = 128;    // most channels of a unit
 
-// two doubles into the shared memory of block `rank` of the cluster, at the address `p` has in this block
-__device__ __forceinline__ void st_cluster_d2(void *p, uint32_t rank, double x, double y)
-{
-  const uint32_t local = (uint32_t)__cvta_generic_to_shared(p);
-  uint32_t remote;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
-  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(remote), "d"(x), "d"(y) : "memory");
-}
-
 // RAG: runs that begin anywhere (the masked form).  A thread's samples lie a multiple of four floats apart, so its 16-byte vectors,
 // from the boundary below the run's start to the one above its end, always lie over the run in the same way: floats lo to hi of a
 // vector are the run's, the others belong to a neighbour, have sums of their own in the thread and are left out when it is folded.
@@ -422,7 +413,7 @@ bool masked_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, Str
       const double chain = waves * ceil_div_u32(rows, used) * batch_us;
       const double cost = 0.6 + waves * (3.0 + 0.024 * cl) + pow(pow(moved, 2.5) + pow(chain, 2.5), 0.4);
       if (best == 0 || cost < best) {
-        best = cost;
+        best = cost; g.cost = (float)cost;
         g.cb = cb; g.units = units; g.cluster = cl; g.rows = rows; g.groups = used;
         g.threads = (used * L4 + 31) / 32 * 32;
       }
@@ -498,34 +489,7 @@ int launch_stream(FusedArgs &a, int dir, cudaStream_t stream)
                          : (extra ? bn_stream_kernel<1, true, false> : bn_stream_kernel<1, false, false>);
   if (masked) kernel = dir == 0 ? (extra ? bn_stream_kernel<0, true, true> : bn_stream_kernel<0, false, true>)
                                 : (extra ? bn_stream_kernel<1, true, true> : bn_stream_kernel<1, false, true>);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(g.units * g.cluster);
-  cfg.blockDim = dim3(g.threads);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // (as launch_chan)
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = g.cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = g.cluster > 1 ? 2 : 1;
-  if (g.cluster > 8) {
-    // larger than the portable size: asked for once per kernel and device
-    static std::mutex mu;
-    static std::map<std::pair<const void *, int>, bool> allowed;
-    int dev = 0;
-    (void)cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> lock(mu);
-    const auto key = std::make_pair((const void *)kernel, dev);
-    auto it = allowed.find(key);
-    if (it == allowed.end()) {
-      const bool ok = cudaFuncSetAttribute((const void *)kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-      if (!ok) (void)cudaGetLastError();
-      it = allowed.emplace(key, ok).first;
-    }
-    if (!it->second) return ANODE_E_LAUNCH;
-  }
-  if (cudaLaunchKernelEx(&cfg, kernel, a, g) != cudaSuccess) { (void)cudaGetLastError(); return ANODE_E_LAUNCH; }
-  return ANODE_OK;
+  return launch_clusters(kernel, a, g, g.units * g.cluster, g.threads, g.cluster, stream);
 }
 
 }  // namespace anode_b200

@@ -322,19 +322,21 @@ def relu(x, inplace=False, cfg=None, stream=None):
 # --------------------------------------------------------------------------------------------
 
 KERNELS = {"auto": 0, "tiled": 1, "cluster": 2, "resident": 3, "plain": 4, "register": 5, "stream": 6}
-#: the streaming kernel's form for large layers; serving_kernel counts it as "stream"
-BAND = 7
+#: forms that queries by shape count as another kernel: the streaming kernel's for large layers ("stream"), and its counterpart for
+#: small layers of long rows ("tiled" or "register")
+BAND, LONG = 7, 8
+FORMS = {"band": BAND, "long": LONG}
 
 
 def set_kernel(name):
     """Process-wide kernel preference of the fused calls (anode_gpu_batch_norm_fused_set_kernel):
-    a name of KERNELS, or "band".  For tests and measurements."""
-    check(_lib.load().anode_gpu_batch_norm_fused_set_kernel(BAND if name == "band" else KERNELS[name]), "anode_gpu_batch_norm_fused_set_kernel")
+    a name of KERNELS or FORMS.  For tests and measurements."""
+    check(_lib.load().anode_gpu_batch_norm_fused_set_kernel(FORMS.get(name) or KERNELS[name]), "anode_gpu_batch_norm_fused_set_kernel")
 
 
 def serving_kernel(shape, dir, residual=False, aligned=True, world=1):
-    """Name, in KERNELS, of the kernel that a fused call on a [N, C, *spatial] shape launches
-    (anode_gpu_batch_norm_fused_serving_kernel); None where a synchronized call takes three."""
+    """Name, in KERNELS, of the kernel that a fused call on a [N, C, *spatial] shape launches, or whose place one of its
+    counterparts takes (anode_gpu_batch_norm_fused_serving_kernel); None where a synchronized call takes three."""
     d0 = 1
     for s in shape[2:]:
         d0 *= int(s)
@@ -345,9 +347,9 @@ def serving_kernel(shape, dir, residual=False, aligned=True, world=1):
 
 
 def last_kernel():
-    """Name of the kernel that this thread's last fused call launched, "band" and "stream" told apart; None before the first."""
+    """Name, in KERNELS or FORMS, of the kernel that this thread's last fused call launched; None before the first."""
     k = _lib.load().anode_gpu_batch_norm_fused_last_kernel()
-    return "band" if k == BAND else {v: n for n, v in KERNELS.items()}.get(k)
+    return {v: n for n, v in {**KERNELS, **FORMS}.items()}.get(k)
 
 
 def set_wait_limit_ms(ms):

@@ -194,6 +194,8 @@ void anode_gpu_positive_clip_flat_map_bwd_f32(
  *   BAND      its form for the largest of them, where the call has a workspace: one walk, with the tiles in tensor memory
  *             between reduction and normalization.  Queries by shape count it as STREAM.  It is launched cooperatively and takes
  *             the whole device, so other streams' kernels run before or after it, not beside it.
+ *   LONG      clusters that walk a channel of long rows twice (small layers of few channels; one GPU), in the place of TILED and
+ *             REGISTER where it is the faster one.  Queries by shape name those.
  * anode_gpu_batch_norm_fused_set_kernel makes another choice process-wide: that kernel is used wherever it
  * applies, elsewhere one of the first four by the shape.  Meant for tests and measurements; which kernel a
  * call launches is answered by anode_gpu_batch_norm_fused_serving_kernel, which one the last call launched by
@@ -206,6 +208,7 @@ void anode_gpu_positive_clip_flat_map_bwd_f32(
 #define ANODE_KERNEL_REGISTER  5
 #define ANODE_KERNEL_STREAM    6
 #define ANODE_KERNEL_BAND      7
+#define ANODE_KERNEL_LONG      8
 int anode_gpu_batch_norm_fused_set_kernel(int kernel);
 
 /* Bound of every wait inside the kernels (for a channel's statistics, for another GPU's records), in

@@ -58,6 +58,10 @@ int anode_gpu_batch_norm_stream_geometry(uint32_t dim0, uint32_t dim1, uint32_t 
 /* The same of its masked form, which serves rows without an aligned run of channels (and of the residual epilogue's calls). */
 int anode_gpu_batch_norm_stream_masked_geometry(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual, uint32_t *out);
 
+/* Geometry of the kernel for small layers of long rows.  out (7 values): applies, blocks per channel, distance between a thread's
+ * vectors, vectors per row and per channel, rows and columns of such a distance. */
+int anode_gpu_batch_norm_long_geometry(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual, uint32_t *out);
+
 /* Geometry of the band kernel, the streaming kernel's form for large layers.  out (16 values): taken by a call with a workspace
  * of the full size (zeros behind a 0: the kernel cannot take the shape at all), channels per unit, units, sample groups of a tile,
  * samples per thread, samples of a tile, tiles per unit, blocks, steps between a tile's two visits, boxes per band, vectors of
