@@ -95,7 +95,8 @@ __device__ __forceinline__ BandWord ld_word(const BandWord *p)
   return w;
 }
 
-template <int DIR, bool EXTRA>
+// ADDS: the output is added to
+template <int DIR, bool EXTRA, bool ADDS>
 __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArgs a, const BandGeom g, const __grid_constant__ BandMaps maps)
 {
   extern __shared__ __align__(128) unsigned char sm[];
@@ -284,30 +285,43 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
         }
       } else {
         const Quad cB = spread(pA.w, pB.w), cC = spread(coef[2 * chA + 1].x, coef[2 * chB + 1].x);
-        const bool acc = a.accumulate != 0;
         [[maybe_unused]] unsigned char *dres = EXTRA && a.dres ? reinterpret_cast<unsigned char *>(a.dres + base) : nullptr;
-        auto one = [&](const Quad &e, const Quad &z) {
+        // Accumulating writes: the next four vectors' old values are on their way while two are worked on, and the producer has brought the
+        // tile to L2 ([256,1024,14,14]: one after the other from HBM 283 us, with both two ahead 202, four ahead 185).
+        uint32_t far = at, rf = r;
+        auto olds = [&](uint32_t i) {
+          Quad q = quad(0.f);
+          if constexpr (ADDS) {
+            if (i < g.vpt && alive && (FULL || rf < rows)) q = ldg_quad(reinterpret_cast<const float *>(out + far));
+            far += 4 * step_g; rf += g.groups;
+          }
+          return q;
+        };
+        auto one = [&](const Quad &e, const Quad &z, const Quad &old) {
           Quad o;
           o.a = fma2(scale.a, z.a, fma2(cB.a, e.a, cC.a)); o.b = fma2(scale.b, z.b, fma2(cB.b, e.b, cC.b));
           if (there()) {
             float *p = reinterpret_cast<float *>(out + at);
-            if (acc) { const Quad old = ldg_quad(p); o.a = add2(old.a, o.a); o.b = add2(old.b, o.b); }
+            if constexpr (ADDS) { o.a = add2(old.a, o.a); o.b = add2(old.b, o.b); }
             stg_stream(p, o);
             if constexpr (EXTRA) { if (dres) stg_stream(reinterpret_cast<float *>(dres + at), z); }
           }
           next();
         };
         uint32_t i = 0;
+        Quad o0 = olds(0), o1 = olds(1), o2 = olds(2), o3 = olds(3);
         for (; i + 2 <= g.vpt; i += 2, tm += 16) {
           Quad e0, z0, e1, z1;
           tmem_ld(tm, e0, z0, e1, z1);
-          one(e0, z0); one(e1, z1);
+          const Quad n0 = olds(i + 4), n1 = olds(i + 5);
+          one(e0, z0, o0); one(e1, z1, o1);
+          o0 = o2; o1 = o3; o2 = n0; o3 = n1;
           __syncwarp();
         }
         if (i < g.vpt) {
           Quad e0, z0;
           tmem_ld(tm, e0, z0);
-          one(e0, z0);
+          one(e0, z0, o0);
         }
       }
       __syncwarp();
@@ -383,6 +397,11 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
         const CUtensorMap *map = kind == 1 || plane == 2 ? &maps.e : plane == 1 ? &maps.dy : &maps.x;
         tensor_g2s(smem_u32(sm + g.off_slots + (size_t)slot * g.slot_stride) + plane * g.plane_bytes + j * g.box_bytes, map,
                    w.unit * g.cb * dim0 + j * g.box4 * 4, w.k * g.rows, &ctl->full[slot], pol);
+      }
+      if (ADDS && kind == 0) {
+        // what the apply visit adds to, on its way to L2
+        const uint32_t n0 = w.k * g.rows, c0 = w.unit * g.cb, run = (C - c0 < g.cb ? C - c0 : g.cb) * dim0 * 4;
+        for (uint32_t r = lane; r < g.rows && n0 + r < N; r += 32) bulk_prefetch(a.out + (size_t)(n0 + r) * rs + (size_t)c0 * dim0, run);
       }
       if (kind == 0 && DIR == 1) {
         float4 *side = reinterpret_cast<float4 *>(sm + g.off_side) + slot * kBandChannels;
@@ -623,8 +642,9 @@ int launch_band(FusedArgs &a, const BandGeom &g, int dir, cudaStream_t stream)
   m.dy = m.x; m.e = m.x;
   if (dir == 1 && !tensor_map(m.dy, a.dy, width, a.plan.N, g.box4 * 4, g.rows)) return ANODE_E_LAUNCH;
   if (extra && !tensor_map(m.e, dir == 0 ? a.res : a.ymask, width, a.plan.N, g.box4 * 4, g.rows)) return ANODE_E_LAUNCH;
-  const void *k = dir == 0 ? (extra ? (const void *)bn_band_kernel<0, true> : (const void *)bn_band_kernel<0, false>)
-                           : (extra ? (const void *)bn_band_kernel<1, true> : (const void *)bn_band_kernel<1, false>);
+  const void *k = dir == 0 ? (extra ? (const void *)bn_band_kernel<0, true, false> : (const void *)bn_band_kernel<0, false, false>)
+                  : a.accumulate ? (extra ? (const void *)bn_band_kernel<1, true, true> : (const void *)bn_band_kernel<1, false, true>)
+                                 : (extra ? (const void *)bn_band_kernel<1, true, false> : (const void *)bn_band_kernel<1, false, false>);
   static std::mutex mu;
   static std::map<std::pair<const void *, int>, bool> ready;
   {

@@ -86,6 +86,7 @@ __global__ void __launch_bounds__(kChanThreads, 2) bn_chan_kernel(const FusedArg
       if (k < cnt) {
         vx[k] = Pack<VEC>::load(a.x + off);
         if (DIR == 1) ve[k] = Pack<VEC>::load(a.dy + off);
+        if (DIR == 1 && a.accumulate) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.out + off));      // (added to below)
         if (DIR == 0 && EXTRA) ve[k] = Pack<VEC>::load(a.res + off);
         if (DIR == 1 && EXTRA) vm[k] = Pack<VEC>::load(a.ymask + off);
       }
@@ -187,11 +188,22 @@ __global__ void __launch_bounds__(kChanThreads, 2) bn_chan_kernel(const FusedArg
 
   // ---- apply
   uint32_t off = off0, col = col0;
+  // accumulating writes: what they add to was brought to L2 with the inputs and is loaded ahead of the first of them ([100,300,7,7]
+  // 14.6 us where each load waited for the store before it, and 8.9 so; [2,2048,14,108] 22.7 and 19.1)
+  Pack<VEC> old[DIR == 1 ? E : 1];
+  if (DIR == 1 && a.accumulate) {
+    uint32_t at = off0, to = col0;
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+      if (k < cnt) old[k] = Pack<VEC>::load(a.out + at);
+      at += g.step_off; to += g.step_col;
+      if (to >= g.d0v) { to -= g.d0v; at += g.wrap; }
+    }
+  }
 #pragma unroll
   for (int k = 0; k < E; ++k) {
     if (k < cnt) {
       Pack<VEC> o;
-      if (DIR == 1 && a.accumulate) o = Pack<VEC>::load(a.out + off);
 #pragma unroll
       for (int i = 0; i < VEC; ++i) {
         if (DIR == 0) {
@@ -200,7 +212,7 @@ __global__ void __launch_bounds__(kChanThreads, 2) bn_chan_kernel(const FusedArg
           o.v[i] = yb * (yb > 0.0f ? 1.0f : slope);
         } else {
           const float dx = fmaf(scale, ve[k].v[i], fmaf(cB, vx[k].v[i], cC));
-          o.v[i] = a.accumulate ? o.v[i] + dx : dx;
+          o.v[i] = a.accumulate ? old[k].v[i] + dx : dx;
         }
       }
       o.put(a.out + off);

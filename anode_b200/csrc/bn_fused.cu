@@ -344,7 +344,7 @@ bool tiled_takes(uint32_t dim0, uint64_t elements, int dir, bool extra)
 
 typedef void (*RingKernel)(const FusedArgs, const RingGeom);
 
-static RingKernel pick_ring_kernel(const Plan &p, int dir, bool extra, uint32_t &threads)
+static RingKernel pick_ring_kernel(const Plan &p, int dir, bool extra, bool adds, uint32_t &threads)
 {
   const bool ragged = p.dim0 % 4 != 0;
   threads = dir == 0 ? ring8::kRingThreads : ring16::kRingThreads;
@@ -352,6 +352,10 @@ static RingKernel pick_ring_kernel(const Plan &p, int dir, bool extra, uint32_t 
     if (!ring_keeps(p, dir, extra)) return extra ? ring8::bn_ring_kernel<0, true, true, false> : ring8::bn_ring_kernel<0, false, true, false>;
     if (extra) return ragged ? ring8::bn_ring_kernel<0, true, true> : ring8::bn_ring_kernel<0, true, false>;
     return ragged ? ring8::bn_ring_kernel<0, false, true> : ring8::bn_ring_kernel<0, false, false>;
+  }
+  if (adds) {
+    if (extra) return ragged ? ring16::bn_ring_kernel<1, true, true, true, true> : ring16::bn_ring_kernel<1, true, false, true, true>;
+    return ragged ? ring16::bn_ring_kernel<1, false, true, true, true> : ring16::bn_ring_kernel<1, false, false, true, true>;
   }
   if (extra) return ragged ? ring16::bn_ring_kernel<1, true, true> : ring16::bn_ring_kernel<1, true, false>;
   return ragged ? ring16::bn_ring_kernel<1, false, true> : ring16::bn_ring_kernel<1, false, false>;
@@ -362,7 +366,7 @@ int launch_ring(FusedArgs &a, const RingGeom &g_in, int dir, cudaStream_t stream
   RingGeom g = g_in;
   uint32_t threads = 0;
   const bool extra = a.res || a.ymask || a.dres;
-  RingKernel k = pick_ring_kernel(a.plan, dir, extra, threads);
+  RingKernel k = pick_ring_kernel(a.plan, dir, extra, dir == 1 && a.accumulate, threads);
   // the reduce visits may store dres before the apply visits read x only where it is not x itself
   a.dres_early = a.dres && a.dres != a.x ? 1u : 0u;
   static std::mutex mu;

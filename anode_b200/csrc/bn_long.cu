@@ -238,11 +238,15 @@ __global__ void __launch_bounds__(kLongThreads, kLongBlocks) bn_long_kernel(cons
 #pragma unroll
       for (int i = 0; i < kBatch; ++i) if (lanes[i]) ve[i] = load(a.res, off[i], lanes[i], drop);
     }
+    Pack<4> old[DIR == 1 ? kBatch : 1];
+    if (DIR == 1 && a.accumulate) {
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) if (lanes[i]) old[i] = load(a.out, off[i], lanes[i], drop);
+    }
 #pragma unroll
     for (int i = 0; i < kBatch; ++i)
       if (lanes[i]) {
         Pack<4> o;
-        if (DIR == 1 && a.accumulate) o = load(a.out, off[i], lanes[i], drop);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           if (DIR == 0) {
@@ -251,7 +255,7 @@ __global__ void __launch_bounds__(kLongThreads, kLongBlocks) bn_long_kernel(cons
             o.v[e] = yb * (yb > 0.0f ? 1.0f : slope);
           } else {
             const float dx = fmaf(scale, vd[i].v[e], fmaf(cB, vx[i].v[e] - mean, cC));
-            o.v[e] = a.accumulate ? o.v[e] + dx : dx;
+            o.v[e] = a.accumulate ? old[i].v[e] + dx : dx;
           }
         }
         store(o, a.out + off[i], lanes[i], false);

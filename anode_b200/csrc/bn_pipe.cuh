@@ -73,6 +73,11 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
                ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy) : "memory");
 }
+// global -> L2; bytes and address are multiples of 16
+__device__ __forceinline__ void bulk_prefetch(const void *src, uint32_t bytes)
+{
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
 // ---- tensor memory: 512 columns of 128 lanes; a warp reaches the 32 lanes of its place in its group of four ----------
 constexpr uint32_t kTmemCols = 512;
 __device__ __forceinline__ void tmem_alloc(uint32_t *dst)

@@ -332,7 +332,7 @@ __device__ __forceinline__ void visit_reduce(const FusedArgs &a, const RingGeom 
   if (lane == 0) res[threadIdx.x >> 5] = out;
 }
 
-template <int DIR, bool EXTRA, bool RAGGED, bool KEEP>
+template <int DIR, bool EXTRA, bool RAGGED, bool KEEP, bool ADDS>
 __device__ __forceinline__ void visit_apply(const FusedArgs &a, const RingGeom &g, unsigned char *sm, RingCtl *ctl,
                                             const uint4 &d, uint32_t slot, const float4 *coef, uint32_t coef_q)
 {
@@ -340,7 +340,6 @@ __device__ __forceinline__ void visit_apply(const FusedArgs &a, const RingGeom &
   const Mine<KEEP> mine(g, ctl, d);
   const uint32_t cnt = mine.cnt, steps = mine.steps;
   const float slope = a.neg_slope;      // activation: t * (t > 0 ? 1 : slope)
-  const bool acc = DIR == 1 && a.accumulate != 0;
   const bool early = EXTRA && DIR == 1 && a.dres_early;      // plane 1 holds dz (see fence_global_to_bulk)
   float *dres = EXTRA && DIR == 1 && !early ? a.dres : nullptr;
   const float4 c0 = coef[0];
@@ -350,8 +349,8 @@ __device__ __forceinline__ void visit_apply(const FusedArgs &a, const RingGeom &
   uint32_t ad = ax + g.slot_floats * 4;
   Walk w(a, g, d.y, mine.tid);
   // one vector: activation(bn(x)) or the input gradient.  x: the input (KEEP and backward: x - mean); gy: dy or dz;
-  // e: residual or saved output
-  auto one = [&](const Quad &x, const Quad &gy, const Quad &e) {
+  // e: residual or saved output; old: what an accumulating write adds to (aligned rows)
+  auto one = [&](const Quad &x, const Quad &gy, const Quad &e, const Quad &old) {
     Quad o, z;
     const Quad u = KEEP && DIR == 1 ? x : Quad{add2(x.a, nmean), add2(x.b, nmean)};
     if constexpr (DIR == 0) {
@@ -369,20 +368,34 @@ __device__ __forceinline__ void visit_apply(const FusedArgs &a, const RingGeom &
     float *p = a.out + (RAGGED ? w.vector() : w.at);
     const int i0 = RAGGED ? w.first() : 0;
     if (!RAGGED || ragged_whole(i0, len)) {
-      if (acc) { const Quad old = ldg_quad(p); o.a = add2(old.a, o.a); o.b = add2(old.b, o.b); }
+      if constexpr (ADDS) {
+        const Quad was = RAGGED ? ldg_quad(p) : old;
+        o.a = add2(was.a, o.a); o.b = add2(was.b, o.b);
+      }
       stg_stream(p, o);
       if constexpr (EXTRA && DIR == 1) { if (dres) stg_stream(dres + (p - a.out), z); }
     } else {
       const float4 t = floats(o), s = floats(z);
       auto put = [&](int k, float f, float r) {
         if ((uint32_t)(i0 + k) < (uint32_t)len) {
-          p[k] = acc ? p[k] + f : f;
+          p[k] = ADDS ? p[k] + f : f;
           if constexpr (EXTRA && DIR == 1) { if (dres) dres[(p - a.out) + k] = r; }
         }
       };
       put(0, t.x, s.x); put(1, t.y, s.y); put(2, t.z, s.z); put(3, t.w, s.w);
     }
     w.advance(g);
+  };
+  // Accumulating writes: the next vectors' old values are on their way while one is worked on, and the producer has brought the tile to
+  // L2.  (Loaded from HBM one after the other: [256,64,112,112] 768 us and, so, 545, [300,64,56,56] 222 and 164, [64,95,55,55] 88 and 72.)
+  Walk far = w;
+  auto olds = [&](bool live) {
+    Quad q = quad(0.f);
+    if constexpr (!RAGGED && ADDS) {
+      if (live) q = ldg_quad(a.out + far.at);
+      far.advance(g);
+    }
+    return q;
   };
   if constexpr (KEEP) {
     tmem_wait_st();      // what this warp stored in the reduce visits
@@ -392,7 +405,7 @@ __device__ __forceinline__ void visit_apply(const FusedArgs &a, const RingGeom &
         if (j >= cnt) return;
         Quad e = x;
         if constexpr (EXTRA) { e = lds_quad(ad); ad += kVecStride; }
-        one(x, x, e);
+        one(x, x, e, x);
       };
       if constexpr (!RAGGED) {
         // (ragged rows: [64,95,55,55] residual 60 -> 76 us with four at a time)
@@ -419,29 +432,35 @@ __device__ __forceinline__ void visit_apply(const FusedArgs &a, const RingGeom &
         __syncwarp();
       }
     } else {
+      Quad o0 = olds(0 < cnt), o1 = olds(1 < cnt);
       if constexpr (!RAGGED) {
         for (; i + 2 <= steps; i += 2, tm += 16) {
           Quad d0, z0, d1, z1;
           tmem_ld(tm, d0, z0, d1, z1);
-          one(d0, z0, d0);
-          if (i + 1 < cnt) one(d1, z1, d1);
+          const Quad n0 = olds(i + 2 < cnt), n1 = olds(i + 3 < cnt);
+          one(d0, z0, d0, o0);
+          if (i + 1 < cnt) one(d1, z1, d1, o1);
+          o0 = n0; o1 = n1;
           __syncwarp();
         }
       }
-      for (; i < steps; ++i, tm += 8) {
+      for (; i < steps; ++i, tm += 8) {      // (one at most, or all of a ragged visit)
         Quad d0, z0;
         tmem_ld(tm, d0, z0);
-        if (i < cnt) one(d0, z0, d0);
+        if (i < cnt) one(d0, z0, d0, o0);
         __syncwarp();
       }
     }
   } else {
+    Quad o0 = olds(0 < cnt), o1 = olds(1 < cnt);
     for (uint32_t i = 0; i < cnt; ++i, ax += kVecStride, ad += kVecStride) {
       const Quad x = lds_quad(ax);
       Quad gy = x, e = x;
       if constexpr (DIR == 1) gy = lds_quad(ad);
       if constexpr (EXTRA) { if (!early) e = lds_quad(DIR == 1 ? ad + g.slot_floats * 4 : ad); }
-      one(x, gy, e);
+      const Quad n1 = olds(i + 2 < cnt);
+      one(x, gy, e, o0);
+      o0 = o1; o1 = n1;
     }
   }
   __syncwarp();
@@ -702,8 +721,8 @@ __device__ __forceinline__ bool pull_merge_unit(const FusedArgs &a, RingCtl *ctl
 // Whole-row tiles only (one channel per unit): short-row shapes are served by the cluster kernel
 // (bn_segres.cu) and the plain kernel.
 // EXTRA: residual epilogue; RAGGED: rows that are not a multiple of four floats; TMEM: some tiles may stay in tensor memory
-// (ring_keeps).
-template <int DIR, bool EXTRA, bool RAGGED, bool TMEM = true>
+// (ring_keeps); ADDS: the output is added to.
+template <int DIR, bool EXTRA, bool RAGGED, bool TMEM = true, bool ADDS = false>
 __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArgs a, const RingGeom g)
 {
   extern __shared__ __align__(128) unsigned char sm[];
@@ -756,8 +775,8 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
           if (++slot == g.slots) { slot = 0; par ^= 1u; }
           if (!warp_wait(&ctl->full[slot], par, ctl, status, ANODE_ST_WAIT_STATS, a.wait_cycles)) break;
         }
-        if (TMEM && kept) visit_apply<DIR, EXTRA, RAGGED, true>(a, g, sm, ctl, d, slot, coef, qcoef);
-        else visit_apply<DIR, EXTRA, RAGGED, false>(a, g, sm, ctl, d, slot, coef, qcoef);
+        if (TMEM && kept) visit_apply<DIR, EXTRA, RAGGED, true, ADDS>(a, g, sm, ctl, d, slot, coef, qcoef);
+        else visit_apply<DIR, EXTRA, RAGGED, false, ADDS>(a, g, sm, ctl, d, slot, coef, qcoef);
         if (++qcoef == kCoefQ) { qcoef = 0; cpar ^= 1u; }
       }
     }
@@ -776,7 +795,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
     for (uint32_t v = 0; ok && v < 2 * sc.steps; ++v) {
       const uint32_t s = v >> 1, kind = v & 1u;
       if (kind == 0 ? !sc.reduce_at(s) : !sc.apply_at(s)) continue;
-      if (kind == 1 && !kSlotAlways<DIR, EXTRA> && g.keep_slots == g.keep_period) continue;      // all from tensor memory
+      if (kind == 1 && !kSlotAlways<DIR, EXTRA> && g.keep_slots == g.keep_period && !ADDS) continue;      // all from tensor memory
       const uint32_t n = kind == 0 ? s : s - sc.look;
       float4 raw = make_float4(0.f, 1.f, 1.f, 0.f);
       const bool fresh = (n & 31u) == 0u;
@@ -795,6 +814,15 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
       }
       const uint4 d = shfl4(kind == 0 ? red : app, n & 31u);
       const bool kept = (d.x >> 16) != 0;
+      if (ADDS && kind == 1) {
+        // what the apply visit adds to is brought to L2 some steps ahead of the consumers (of a ragged row what lies between two 16-byte boundaries)
+        const uint32_t whole = rs * P.N & ~3u;
+        for (uint32_t r = row0; r < d.w; r += 32) {
+          const uint32_t first = d.y + r * rs, from = RAGGED ? (first + 3) & ~3u : first, to = RAGGED ? (first + d.z) & ~3u : first + d.z;
+          const uint32_t at = from + off0 / 4;
+          if (at < to && to <= whole) bulk_prefetch(a.out + at, (to - at < kRingCopyBytes / 4 ? to - at : kRingCopyBytes / 4) * 4);
+        }
+      }
       if (kind == 1 && kept && !kSlotAlways<DIR, EXTRA>) continue;
       ++k;
       if (++slot == g.slots) { slot = 0; par ^= 1u; }

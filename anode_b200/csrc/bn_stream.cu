@@ -271,6 +271,10 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamBlocks) bn_stream_kerne
           }
       }
     } else {
+      if (a.accumulate) {      // what is added to, on its way to L2 (registers for all of a batch would spill)
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) if (k + i < nk) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.out + (off0 + (k + i) * step)));
+      }
       if (k != kb) {
         const float *second = early ? a.dres : a.dy;
         Pack<4> vm[EXTRA ? kBatch : 1];
@@ -296,7 +300,7 @@ __global__ void __launch_bounds__(kStreamThreads, kStreamBlocks) bn_stream_kerne
         if (k + i < nk) {
           const uint32_t off = off0 + (k + i) * step;
           Pack<4> o;
-          if (a.accumulate) o = RAG ? load(a.out, off, drop) : Pack<4>::load(a.out + off);
+          if (a.accumulate) o = load(a.out, off, drop);
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const float dx = fmaf(scale[e], vd[i].v[e], fmaf(cB[e], vx[i].v[e] - mean[e], cC[e]));
