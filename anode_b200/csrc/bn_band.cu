@@ -37,7 +37,7 @@ struct BandCtl {
   unsigned long long full[kBandMaxSlots], empty[kBandMaxSlots];
   unsigned long long res_full[kBandQ], res_empty[kBandQ], coef_full[kBandQ], coef_empty[kBandQ];
   volatile uint32_t abort;
-  uint32_t last_block, parity, tmem;
+  uint32_t parity, tmem;
 };
 static_assert(sizeof(BandCtl) <= kBandCtlBytes, "BandCtl outgrew the room reserved for it");
 
@@ -103,18 +103,17 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
   BandCtl *ctl = reinterpret_cast<BandCtl *>(sm);
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint32_t *status = a.status;
-  uint32_t *exit_ctr = reinterpret_cast<uint32_t *>(a.ws + g.hdr), *parity = exit_ctr + 1;
   constexpr uint32_t kKept = DIR == 0 ? 1u : 2u;                    // tensors kept in tensor memory
   constexpr uint32_t kPlanes = DIR == 0 ? 1u : EXTRA ? 3u : 2u;     // tensors of a reduce visit
   constexpr bool kSlotToo = DIR == 0 && EXTRA;                      // apply visits fetch the residual
 
-  if (tid == 0) {
+  if (tid == kBandWarps * 32) {      // (warp 0 allocates meanwhile)
     for (uint32_t i = 0; i < g.slots; ++i) { mbar_init(&ctl->full[i], 1); mbar_init(&ctl->empty[i], kBandWarps); }
     for (uint32_t i = 0; i < kBandQ; ++i) {
       mbar_init(&ctl->res_full[i], kBandWarps); mbar_init(&ctl->res_empty[i], 1);
       mbar_init(&ctl->coef_full[i], 1); mbar_init(&ctl->coef_empty[i], kBandWarps);
     }
-    ctl->abort = 0; ctl->last_block = 0; ctl->parity = *parity & 1u;
+    ctl->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -125,6 +124,14 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
   const uint32_t dim0 = a.plan.dim0, C = a.plan.C, N = a.plan.N, rs = C * dim0;
   const uint32_t b = blockIdx.x, G = gridDim.x;
   const uint32_t mine = b < g.total ? (g.total - b + G - 1) / G : 0, steps = mine ? mine + g.look : 0;
+
+  // for the two warps that use the tagged words
+  auto buffer = [&] {
+    uint32_t *counter = reinterpret_cast<uint32_t *>(a.ws + g.hdr);
+    const uint32_t p = buffer_of_launch(counter, counter + 1, 2);
+    if (lane == 0) ctl->parity = p;
+    __syncwarp();
+  };
 
   if (warp < kBandWarps) {
     // ------------------------------------------------------------------ consumers
@@ -426,6 +433,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
     const uint32_t v0 = ci * dim0 / 4, v1 = (ci * dim0 + dim0 - 1) / 4;      // the channel's first and last vector
     BandWord *buf = reinterpret_cast<BandWord *>(a.ws + g.tag);
     const size_t other = (size_t)g.total * g.cb;
+    buffer();
     BandWord *now = buf + (ctl->parity ? other : 0), *then = buf + (ctl->parity ? 0 : other);
     BandWalk w(g, b, G);
     uint32_t q = 0, qpar = 0;
@@ -466,6 +474,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
   } else {
     // ------------------------------------------------------------------ coefficient warp
     const uint32_t lp = 1u << g.lane_shift, ci = lane >> g.lane_shift, sub = lane & (lp - 1u);
+    buffer();
     const BandWord *buf = reinterpret_cast<const BandWord *>(a.ws + g.tag) + (ctl->parity ? (size_t)g.total * g.cb : 0);
     BandWalk w(g, b, G);
     uint32_t q = 0, qpar = 1;
@@ -563,14 +572,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
   tmem_fence_before();
   __syncthreads();
   if (warp == 0) { tmem_fence_after(); tmem_free(ctl->tmem); }
-  if (ctl->abort) {
-    if (tid == 0) atomicOr(status, ANODE_ST_ABORTED);
-    return;
-  }
-  if (tid == 0) {
-    __threadfence();
-    if (atomicAdd(exit_ctr, 1u) + 1 == gridDim.x) { *parity = ctl->parity ^ 1u; *exit_ctr = 0; }
-  }
+  if (ctl->abort && tid == 0) atomicOr(status, ANODE_ST_ABORTED);
 }
 
 // ---- host side -------------------------------------------------------------------------------

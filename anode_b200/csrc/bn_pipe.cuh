@@ -67,6 +67,20 @@ __device__ __forceinline__ bool warp_wait(unsigned long long *bar, uint32_t pari
   if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, ctl, status, bit, limit) ? 1u : 0u;
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
+// Which of its two buffers of tagged words a launch uses, for the whole warp; `warps` of them ask in every block.  The last of the grid
+// to have asked turns the word for the next launch: all of this one have their answer then.  (Asked ahead of the first barrier and
+// counted when a block left, that was a load, a fence and an atomic's way to L2 and back on every launch's critical path.)
+__device__ __forceinline__ uint32_t buffer_of_launch(uint32_t *counter, uint32_t *word, uint32_t warps)
+{
+  uint32_t p = 0;
+  if ((threadIdx.x & 31) == 0) {
+    p = ld_acquire_gpu(word) & 1u;
+    uint32_t before;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(before) : "l"(counter) : "memory");
+    if (before + 1 == warps * gridDim.x) { *counter = 0; *word = p ^ 1u; }
+  }
+  return __shfl_sync(0xffffffffu, p, 0);
+}
 // global -> shared bulk copy, completion counted on `bar`; bytes and both addresses are multiples of 16
 __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, unsigned long long *bar, uint64_t policy)
 {

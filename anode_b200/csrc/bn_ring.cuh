@@ -55,7 +55,6 @@ struct RingCtl {
   unsigned long long res_full[kResQ], res_empty[kResQ];
   unsigned long long coef_full[kCoefQ], coef_empty[kCoefQ];
   volatile uint32_t abort;
-  uint32_t last_block;
   uint32_t parity;       // which of the two tagged-partial buffers this launch uses
   uint32_t tmem;         // base address of the block's tensor memory (g.keep_slots > 0)
 };
@@ -730,15 +729,13 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
   const Plan &P = a.plan;
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint32_t *status = a.status;
-  uint32_t *exit_ctr = ws_u32(a, g.hdr);
   uint32_t *done = ws_u32(a, P.off_done);
 
-  if (tid == 0) {
+  if (tid == kConsumers) {      // (warp 0 allocates meanwhile)
     for (uint32_t i = 0; i < g.slots; ++i) { mbar_init(&ctl->full[i], 1); mbar_init(&ctl->empty[i], kCWarps); }
     for (uint32_t i = 0; i < kResQ; ++i) { mbar_init(&ctl->res_full[i], kCWarps); mbar_init(&ctl->res_empty[i], 1); }
     for (uint32_t i = 0; i < kCoefQ; ++i) { mbar_init(&ctl->coef_full[i], 1); mbar_init(&ctl->coef_empty[i], kCWarps); }
-    ctl->abort = 0; ctl->last_block = 0;
-    ctl->parity = *ws_u32(a, g.hdr + 4) & 1u;
+    ctl->abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -747,6 +744,14 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
   if (TMEM && g.keep_slots) tmem_fence_after();
 
   Sched sc; sc.init(a);
+  // the two warps that use the tagged words each see to it that ctl->parity is there for them (in shared memory: a register more and
+  // the backward pass was slower, 390 -> 426 us on [256,64,112,112])
+  auto buffer = [&] {
+    if (a.mode != MODE_FUSED) return;
+    const uint32_t p = buffer_of_launch(ws_u32(a, g.hdr), ws_u32(a, g.hdr + 4), 2);
+    if (lane == 0) ctl->parity = p;
+    __syncwarp();
+  };
 
   if (warp < kConsumers / 32) {
     // ------------------------------------------------------------------ consumers
@@ -928,6 +933,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
     // ------------------------------------------------------------------ delivery warp
     // Reduce visit j of this block is tile b + j*G.  The consumer warps' partials of a tile are merged in a fixed order.
     uint32_t q = 0, qpar = 0, tile = sc.b;
+    buffer();
     for (uint32_t j = 0; j < sc.reduces; ++j) {
       if (!warp_wait(&ctl->res_full[q], qpar, ctl, status, ANODE_ST_WAIT_STATS, a.wait_cycles)) break;
       float4 v = lane < kCWarps ? res_box(sm, g, q)[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -991,6 +997,7 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
     uint4 visit = make_uint4(0, 0, 0, 0);
     uint32_t unit = 0;
     float4 in = c0;
+    buffer();
     for (uint32_t n = 0; n < sc.applies; ++n) {
       const uint32_t at = n & 31u;
       if (at == 0 && n + lane < sc.my_tiles) {
@@ -1025,28 +1032,14 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
     }
   }
 
-  // ---- leave: the last block out lowers the ready flags so that the workspace is clean again
+  // ---- leave
   if (TMEM && g.keep_slots) {
     if (warp < kCWarps) { __syncwarp(); tmem_wait_st(); }
     tmem_fence_before();
   }
   __syncthreads();
   if (TMEM && g.keep_slots && warp == 0) { tmem_fence_after(); tmem_free(ctl->tmem); }
-  if (ctl->abort) {
-    if (tid == 0) atomicOr(status, ANODE_ST_ABORTED);
-    return;
-  }
-  if (a.mode == MODE_FUSED) {
-    if (tid == 0) {
-      __threadfence();
-      ctl->last_block = (atomicAdd(exit_ctr, 1u) + 1 == gridDim.x) ? 1u : 0u;
-    }
-    __syncthreads();
-    if (ctl->last_block && tid == 0) {
-      *ws_u32(a, g.hdr + 4) = ctl->parity ^ 1u;       // the next launch uses the other partial buffer
-      *exit_ctr = 0;
-    }
-  }
+  if (ctl->abort && tid == 0) atomicOr(status, ANODE_ST_ABORTED);
 }
 
 }  // namespace ANODE_RING_NS
