@@ -107,13 +107,19 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
   constexpr uint32_t kPlanes = DIR == 0 ? 1u : EXTRA ? 3u : 2u;     // tensors of a reduce visit
   constexpr bool kSlotToo = DIR == 0 && EXTRA;                      // apply visits fetch the residual
 
-  if (tid == kBandWarps * 32) {      // (warp 0 allocates meanwhile)
+  // Backward passes ask for the launch's buffer here and turn the word when they leave, as the tiled kernel did: asked for by the warps that
+  // use it (buffer_of_launch) forward passes are 1.5 us faster, [1024,2048,7,7] 150.9 and 149.4, backward ones no faster by themselves and
+  // slower behind a forward pass, [4096,512,7,7] both 391 and 396 - 399 (and with the atomic elsewhere in the launch 400 - 408).
+  constexpr bool kAsk = DIR == 0;
+  uint32_t *counter = reinterpret_cast<uint32_t *>(a.ws + g.hdr);
+  if (tid == (kAsk ? kBandWarps * 32 : 0)) {      // (warp 0 allocates meanwhile)
     for (uint32_t i = 0; i < g.slots; ++i) { mbar_init(&ctl->full[i], 1); mbar_init(&ctl->empty[i], kBandWarps); }
     for (uint32_t i = 0; i < kBandQ; ++i) {
       mbar_init(&ctl->res_full[i], kBandWarps); mbar_init(&ctl->res_empty[i], 1);
       mbar_init(&ctl->coef_full[i], 1); mbar_init(&ctl->coef_empty[i], kBandWarps);
     }
     ctl->abort = 0;
+    if (!kAsk) ctl->parity = counter[1] & 1u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -127,10 +133,11 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
 
   // for the two warps that use the tagged words
   auto buffer = [&] {
-    uint32_t *counter = reinterpret_cast<uint32_t *>(a.ws + g.hdr);
-    const uint32_t p = buffer_of_launch(counter, counter + 1, 2);
-    if (lane == 0) ctl->parity = p;
-    __syncwarp();
+    if constexpr (kAsk) {
+      const uint32_t p = buffer_of_launch(counter, counter + 1, 2);
+      if (lane == 0) ctl->parity = p;
+      __syncwarp();
+    }
   };
 
   if (warp < kBandWarps) {
@@ -572,7 +579,14 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
   tmem_fence_before();
   __syncthreads();
   if (warp == 0) { tmem_fence_after(); tmem_free(ctl->tmem); }
-  if (ctl->abort && tid == 0) atomicOr(status, ANODE_ST_ABORTED);
+  if (ctl->abort) {
+    if (tid == 0) atomicOr(status, ANODE_ST_ABORTED);
+    return;
+  }
+  if (!kAsk && tid == 0) {
+    __threadfence();
+    if (atomicAdd(counter, 1u) + 1 == gridDim.x) { counter[1] = ctl->parity ^ 1u; counter[0] = 0; }
+  }
 }
 
 // ---- host side -------------------------------------------------------------------------------

@@ -55,16 +55,20 @@ struct FusedArgs {
   long long wait_cycles;   // bound of every in-kernel wait, in SM clock cycles
 };
 
-// 1/sqrt(v) as every kernel here computes it (IEEE divide and square root), so that the
-// forward pass and the backward pass derive bit-identical scales, hence identical ReLU masks.
-// Its lowest bit is one: of the two such values beside the rounded quotient the nearer one (with the bit set by an OR, upwards, y's
-// relative error against float64 over 100 layers was 8.3e-8 to 9.0e-8 by the kernel, so 7.1e-8 to 7.6e-8).
+// 1/sqrt(v) as every kernel here computes it, so that the forward pass and the backward pass derive bit-identical scales, hence
+// identical ReLU masks (every step is one rounded operation, which no compiler fuses with its neighbours).  Newton's step from rsqrtf,
+// whose error 1 - v r^2 comes exact enough from two fused products; the quotient of a rounded square root took three times as long, in
+// the chain from a channel's last partial sum to its coefficients.
+// The lowest bit is one: of the two such values beside the rounded result the nearer one, known from what the rounding left (with the
+// bit set by an OR, upwards, y's relative error against float64 over 100 layers was 8.3e-8 to 9.0e-8 by the kernel, so 7.1e-8 to 7.6e-8).
 __device__ __forceinline__ float inv_std(float v)
 {
-  const float r = __fdiv_rn(1.0f, __fsqrt_rn(v)), t = __fmul_rn(v, r);
-  const float past = fmaf(-t, r, 1.0f) - fmaf(v, r, -t) * r;      // 1 - v r^2: below zero where r lies above 1/sqrt(v)
+  const float r0 = rsqrtf(v), t = __fmul_rn(v, r0);
+  const float h = __fmaf_rn(-__fmaf_rn(v, r0, -t), r0, __fmaf_rn(-t, r0, 1.0f));
+  const float d = __fmul_rn(__fmul_rn(0.5f, r0), h), r = __fadd_rn(r0, d), rest = __fadd_rn(__fsub_rn(r0, r), d);
+  if (!(fabsf(h) < 1.0f)) return __uint_as_float(__float_as_uint(r0) | 1u);      // of zero, an infinity, a NaN or below zero
   const uint32_t u = __float_as_uint(r);
-  return __uint_as_float(u & 1u ? u : past < 0.0f ? u - 1u : u + 1u);      // (no number: as the OR)
+  return __uint_as_float(u & 1u ? u : rest < 0.0f ? u - 1u : u + 1u);
 }
 
 // Tagged per-channel records in the workspace: zero = not ready; written once per launch with a
