@@ -13,6 +13,8 @@
 // larger than gives most threads four.  With one sample in flight and a thread for each of up to 32 blocks per SM, and so, us
 // from buffer to buffer: [8,256,28,28] 4.1 and 3.3, [32,256,14,14] 4.1 and 2.9, [64,512,7,7] 6.8 and 3.7, [32,64,56,56] 11.7 and 9.9,
 // [256,2048,7,7] 37.0 and 33.8, [64,95,55,55] 44.6 and 27.6, [256,256,56,56] 254 and 247 (1.01 of the copy bandwidth).
+#include <initializer_list>
+
 #include "bn_device.cuh"
 #include "bn_host.h"
 
@@ -20,29 +22,32 @@ namespace anode_b200 {
 
 constexpr uint32_t kInferThreads = 256;
 constexpr uint32_t kInferFlight = 4;      // samples in flight per thread
+constexpr uint64_t kInferCut = 1500000;   // floats of a single sample from which on its rows are cut
 
 // The inputs carry no __restrict__: it would let the compiler treat their loads as reads of memory that nothing writes while
 // the kernel runs and move them above pdl_wait(), where the kernel before this one may still be writing them (the running
 // averages of a training step, the activations of the layer below).
+// N samples, `step` floats apart, of C channels of `len` floats, `row` floats apart (a single sample's rows may be cut into pieces that
+// take the place of samples, see the launch).
 template <int VEC>
-__global__ void __launch_bounds__(kInferThreads) bn_infer_kernel(uint32_t dim0, uint32_t C, uint32_t N, float neg_slope,
+__global__ void __launch_bounds__(kInferThreads) bn_infer_kernel(uint32_t len, uint32_t C, uint32_t N, uint32_t row, uint32_t step, float neg_slope,
                                                                  const float *x, const float *mean, const float *var,
                                                                  const float *gamma, const float *beta, float *y)
 {
-  const uint64_t per_sample = (uint64_t)C * dim0;                 // floats
+  const uint64_t per_sample = (uint64_t)C * len;                  // floats
   const uint64_t col = ((uint64_t)blockIdx.x * kInferThreads + threadIdx.x) * VEC;
   if (col >= per_sample) return;
   // channel of each of this thread's elements, and its coefficients (a sample has less than 2^32 floats, check_dims)
-  uint32_t c = (uint32_t)col / dim0, off = (uint32_t)col - c * dim0;
+  uint32_t c = (uint32_t)col / len, off = (uint32_t)col - c * len;
   // this thread's samples: blockIdx.y, + gridDim.y, ...; `left` of the batch from the next one on
   uint32_t left = N - blockIdx.y;
-  const size_t step = (size_t)gridDim.y * per_sample;
-  size_t at = (size_t)blockIdx.y * per_sample + col;
+  const size_t down = (size_t)gridDim.y * step;
+  size_t at = (size_t)blockIdx.y * step + (size_t)c * row + off;
   Pack<VEC> p[kInferFlight];
   auto load = [&] {
 #pragma unroll
     for (int u = 0; u < kInferFlight; ++u)
-      if (u * gridDim.y < left) p[u] = Pack<VEC>::load(x + at + u * step);
+      if (u * gridDim.y < left) p[u] = Pack<VEC>::load(x + at + u * down);
   };
   pdl_wait();
   // the first samples' floats are on their way while the coefficients are made
@@ -58,7 +63,7 @@ __global__ void __launch_bounds__(kInferThreads) bn_infer_kernel(uint32_t dim0, 
       prev = c;
     }
     mu[i] = m0; sc[i] = s0; sh[i] = b0;
-    if (++off == dim0) { off = 0; ++c; }
+    if (++off == len) { off = 0; ++c; }
   }
   for (;;) {
 #pragma unroll
@@ -69,10 +74,10 @@ __global__ void __launch_bounds__(kInferThreads) bn_infer_kernel(uint32_t dim0, 
           const float t = fmaf(p[u].v[i] - mu[i], sc[i], sh[i]);
           p[u].v[i] = t * (t > 0.0f ? 1.0f : neg_slope);
         }
-        p[u].store_stream(y + at + u * step);
+        p[u].store_stream(y + at + u * down);
       }
     if (left <= kInferFlight * gridDim.y) break;
-    left -= kInferFlight * gridDim.y; at += kInferFlight * step;
+    left -= kInferFlight * gridDim.y; at += kInferFlight * down;
     load();
   }
 }
@@ -91,8 +96,17 @@ extern "C" int anode_gpu_batch_norm_act_infer_3d1_packed_f32(
   if (rc) return rc;
   if (!x || !y || !mean || !var) return ANODE_E_NULL;
   if (!aligned4(x) || !aligned4(y)) return ANODE_E_ALIGN;
-  const uint64_t per_sample = (uint64_t)dim1 * dim0;
-  const bool vec = aligned16(x) && aligned16(y) && per_sample % 4 == 0;
+  const bool vec = aligned16(x) && aligned16(y) && (uint64_t)dim1 * dim0 % 4 == 0;
+  // A single sample leaves a thread one load: its rows are cut into pieces, which take the place of samples ([1,515,64,64,64] 227 us, in
+  // four @A@, [1,16,96,96,96] 25.4 and @B@, [1,132,128,128] 4.6 and @C@).  Not small ones, where the launch is the time.
+  uint32_t len = dim0, samples = dim2, step = dim1 * dim0;
+  if (dim2 == 1 && (uint64_t)dim1 * dim0 >= kInferCut && (!vec || dim0 % 4 == 0)) {
+    const uint32_t lanes = vec ? 4u : 1u;
+    for (uint32_t n : {4u, 8u, 5u, 3u, 7u, 2u})
+      if (dim0 % (n * lanes) == 0) { len = dim0 / n; samples = n; step = len; break; }
+  }
+  dim2 = samples;
+  const uint64_t per_sample = (uint64_t)dim1 * len;
   const uint64_t cols = vec ? per_sample / 4 : per_sample;
   const uint64_t bx = (cols + kInferThreads - 1) / kInferThreads;
   if (bx > 0x7fffffffull) return ANODE_E_DIMS;
@@ -119,8 +133,8 @@ extern "C" int anode_gpu_batch_norm_act_infer_3d1_packed_f32(
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg_.attrs = attr; cfg_.numAttrs = 1;
-  const cudaError_t e = vec ? cudaLaunchKernelEx(&cfg_, bn_infer_kernel<4>, dim0, dim1, dim2, neg_slope, x, mean, var, gamma, beta, y)
-                            : cudaLaunchKernelEx(&cfg_, bn_infer_kernel<1>, dim0, dim1, dim2, neg_slope, x, mean, var, gamma, beta, y);
+  const cudaError_t e = vec ? cudaLaunchKernelEx(&cfg_, bn_infer_kernel<4>, len, dim1, dim2, dim0, step, neg_slope, x, mean, var, gamma, beta, y)
+                            : cudaLaunchKernelEx(&cfg_, bn_infer_kernel<1>, len, dim1, dim2, dim0, step, neg_slope, x, mean, var, gamma, beta, y);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return ANODE_E_LAUNCH; }
   return ANODE_OK;
 }
