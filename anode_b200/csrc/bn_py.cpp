@@ -8,6 +8,8 @@
 // torch reports some conditions by C++ exceptions (no driver, a tensor without storage inside a function transform, a
 // sparse one): every function turns them into Python errors (GUARDED), and nothing is asked of torch or CUDA once
 // an argument was refused.
+#include <ATen/ops/empty.h>
+#include <ATen/ops/empty_like.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <c10/cuda/CUDAStream.h>
@@ -257,46 +259,67 @@ PyObject *py_infer(PyObject *, PyObject *const *v, Py_ssize_t n)
   END_GUARDED
 }
 
-// normalize(axes, epsilon, avg_rate, x, y, mean, var, avg_mean, avg_var, stream)
+// The outputs of the front end's composition are made here: three tensors through the interpreter took longer than the call.
+at::Tensor like(const at::Tensor &x) { return at::empty_like(x); }
+at::Tensor per_channel(const at::Tensor &x) { return at::empty({x.size(1)}, x.options()); }
+Out data(const at::Tensor &t) { return static_cast<float *>(t.data_ptr()); }
+// (status, a, b, c)
+PyObject *answer(int rc, const at::Tensor &a, const at::Tensor &b, const at::Tensor &c)
+{
+  PyObject *t = PyTuple_New(4), *items[4] = {PyLong_FromLong(rc), THPVariable_Wrap(a), THPVariable_Wrap(b), THPVariable_Wrap(c)};
+  bool ok = t != nullptr;
+  for (int i = 0; i < 4; ++i) {
+    ok = ok && items[i];
+    if (t) PyTuple_SET_ITEM(t, i, items[i]); else Py_XDECREF(items[i]);
+  }
+  if (ok) return t;
+  Py_XDECREF(t);
+  return nullptr;
+}
+
+// normalize(axes, epsilon, avg_rate, x, avg_mean, avg_var, stream) -> status, y, mean, var
 PyObject *py_normalize(PyObject *, PyObject *const *v, Py_ssize_t n)
 {
   GUARDED
-  if (!want_args(n, 10)) return nullptr;
+  if (!want_args(n, 7)) return nullptr;
   Args a{v};
   uint32_t d[3] = {0, 0, 0};
   a.dims(0, 3, d);
   const float eps = a.f(1), rate = a.f(2);
   In x = a.ptr(3, false);
-  Out y = a.ptr(4, false), mean = a.ptr(5, false), var = a.ptr(6, false), rm = a.ptr(7, false), rv = a.ptr(8, false);
-  void *s = a.stream(9);
+  Out rm = a.ptr(4, false), rv = a.ptr(5, false);
+  void *s = a.stream(6);
   if (!a.ok || !bound(F_NORMALIZE)) return nullptr;
+  const at::Tensor &t = THPVariable_Unpack(v[3]);
+  const at::Tensor mean = per_channel(t), var = per_channel(t), y = like(t);
   int rc;
   {
     Unlocked unlocked;
-    rc = ((NormalizeFn)g_fn[F_NORMALIZE])(d[0], d[1], d[2], eps, rate, x, y, mean, var, rm, rv, &kDefaultCfg, s);
+    rc = ((NormalizeFn)g_fn[F_NORMALIZE])(d[0], d[1], d[2], eps, rate, x, data(y), data(mean), data(var), rm, rv, &kDefaultCfg, s);
   }
-  return PyLong_FromLong(rc);
+  return answer(rc, y, mean, var);
   END_GUARDED
 }
 
-// adjoint(axes, dy, x, mean, var, dx, dmean, dvar, stream)
+// adjoint(axes, dy, x, mean, var, stream) -> status, dx, dmean, dvar
 PyObject *py_adjoint(PyObject *, PyObject *const *v, Py_ssize_t n)
 {
   GUARDED
-  if (!want_args(n, 9)) return nullptr;
+  if (!want_args(n, 6)) return nullptr;
   Args a{v};
   uint32_t d[3] = {0, 0, 0};
   a.dims(0, 2, d);
   In dy = a.ptr(1, false), x = a.ptr(2, false), mean = a.ptr(3, false), var = a.ptr(4, false);
-  Out dx = a.ptr(5, false), dmean = a.ptr(6, false), dvar = a.ptr(7, false);
-  void *s = a.stream(8);
+  void *s = a.stream(5);
   if (!a.ok || !bound(F_ADJOINT)) return nullptr;
+  const at::Tensor &t = THPVariable_Unpack(v[2]);
+  const at::Tensor dvar = per_channel(t), dmean = per_channel(t), dx = like(t);
   int rc;
   {
     Unlocked unlocked;
-    rc = ((AdjointFn)g_fn[F_ADJOINT])(d[0], d[1], d[2], dy, x, mean, var, dx, dmean, dvar, &kDefaultCfg, s);
+    rc = ((AdjointFn)g_fn[F_ADJOINT])(d[0], d[1], d[2], dy, x, mean, var, data(dx), data(dmean), data(dvar), &kDefaultCfg, s);
   }
-  return PyLong_FromLong(rc);
+  return answer(rc, dx, dmean, dvar);
   END_GUARDED
 }
 

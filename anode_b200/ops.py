@@ -253,20 +253,18 @@ def batch_normalize_2d(x, axes, online, avg_rate, epsilon, avg_mean=None, avg_va
     (`switch(online, avg, batch)`, src/ops.rs:1671-1674).
     """
     c = x.shape[1]
-    fused = online and 0 < x.numel() < _FUSED_LIMIT
-    new = torch.empty if fused else torch.zeros
-    mean = new(c, device=x.device, dtype=torch.float32)
-    var = new(c, device=x.device, dtype=torch.float32)
     if avg_mean is None:
-        avg_mean = torch.zeros_like(mean)
+        avg_mean = torch.zeros(c, device=x.device, dtype=torch.float32)
     if avg_var is None:
-        avg_var = torch.zeros_like(var)
-    if fused:
+        avg_var = torch.zeros(c, device=x.device, dtype=torch.float32)
+    if online and 0 < x.numel() < _FUSED_LIMIT:
         _hint(cfg)
-        y = torch.empty_like(x)
-        check(native().normalize(axes, epsilon, avg_rate, x, y, mean, var, avg_mean, avg_var, stream),
-              "anode_gpu_batch_normalize_3d1_packed_f32")
+        rc, y, mean, var = native().normalize(axes, epsilon, avg_rate, x, avg_mean, avg_var, stream)
+        if rc:
+            check(rc, "anode_gpu_batch_normalize_3d1_packed_f32")
         return y, mean, var, avg_mean, avg_var
+    mean = torch.zeros(c, device=x.device, dtype=torch.float32)
+    var = torch.zeros(c, device=x.device, dtype=torch.float32)
     BatchMean2dOp.apply(axes, x, mean, cfg=cfg, stream=stream)
     BatchVariance2dOp.apply(axes, epsilon, x, mean, var, cfg=cfg, stream=stream)
     OnlineAverageOp.apply(avg_rate, mean, avg_mean, cfg=cfg, stream=stream)
@@ -293,9 +291,9 @@ def batch_normalize_adjoint(axes, dy_bn, x, mean, var, cfg=None, stream=None):
     c = x.shape[1]
     if 0 < x.numel() < _FUSED_LIMIT:
         _hint(cfg)
-        dvar, dmean = torch.empty(c, device=x.device, dtype=torch.float32), torch.empty(c, device=x.device, dtype=torch.float32)
-        dx = torch.empty_like(x)
-        check(native().adjoint(axes, dy_bn, x, mean, var, dx, dmean, dvar, stream), "anode_gpu_batch_normalize_adjoint_3d1_packed_f32")
+        rc, dx, dmean, dvar = native().adjoint(axes, dy_bn, x, mean, var, stream)
+        if rc:
+            check(rc, "anode_gpu_batch_normalize_adjoint_3d1_packed_f32")
         return dx, dmean, dvar
     dvar = torch.zeros(c, device=x.device, dtype=torch.float32)
     dmean = torch.zeros(c, device=x.device, dtype=torch.float32)
