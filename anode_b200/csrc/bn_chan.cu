@@ -24,6 +24,12 @@ constexpr uint32_t kChanThreads = 512;       // most threads of a block
 constexpr uint32_t kChanCluster = 8;         // most blocks of a team (the portable cluster size)
 constexpr uint32_t kChanWarpTeams = 4;       // one-warp teams per block
 
+// Threads that two blocks of an SM are compiled for: 64 registers each, or for teams of a few floats a thread 48 or 56, where blocks that
+// do not divide an SM's 1024 threads would leave a second wave (chan_dense).  Us with 64 and so, forward, [225,56,80] 6.4 and 4.3, [3,239,1451]
+// 6.0 and 4.3, [6,278,354] 5.5 and 3.8, residual backward [19,1970,65] 23.4 and 15.6; but with one wave either way backward [451,21,48] 3.6 and
+// 4.3, [108,84,29] 3.6 and 4.3.
+constexpr uint32_t chan_bound(int floats, bool dense) { return !dense ? kChanThreads : floats == 4 ? 640u : 576u; }
+
 struct ChanGeom {
   uint32_t vec, floats;      // floats per load (4 or 1) and per thread (the template's F)
   uint32_t threads, cluster; // team = cluster * threads; threads == 32: one-warp teams, kChanWarpTeams to a block
@@ -43,8 +49,8 @@ __device__ __forceinline__ void st_cluster_f4(void *p, uint32_t rank, float4 v)
 }
 
 // F: floats a thread holds per tensor
-template <int DIR, int VEC, int F, bool EXTRA>
-__global__ void __launch_bounds__(kChanThreads, 2) bn_chan_kernel(const FusedArgs a, const ChanGeom g)
+template <int DIR, int VEC, int F, bool EXTRA, bool DENSE>
+__global__ void __launch_bounds__(chan_bound(F, DENSE), 2) bn_chan_kernel(const FusedArgs a, const ChanGeom g)
 {
   constexpr int E = F / VEC;
   __shared__ float4 rec[kChanCluster * kChanThreads / 32];
@@ -86,7 +92,7 @@ __global__ void __launch_bounds__(kChanThreads, 2) bn_chan_kernel(const FusedArg
       if (k < cnt) {
         vx[k] = Pack<VEC>::load(a.x + off);
         if (DIR == 1) ve[k] = Pack<VEC>::load(a.dy + off);
-        if (DIR == 1 && a.accumulate) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.out + off));      // (added to below)
+        if (DIR == 1 && !EXTRA && a.accumulate) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.out + off));      // (added to below)
         if (DIR == 0 && EXTRA) ve[k] = Pack<VEC>::load(a.res + off);
         if (DIR == 1 && EXTRA) vm[k] = Pack<VEC>::load(a.ymask + off);
       }
@@ -190,8 +196,11 @@ __global__ void __launch_bounds__(kChanThreads, 2) bn_chan_kernel(const FusedArg
   uint32_t off = off0, col = col0;
   // accumulating writes: what they add to was brought to L2 with the inputs and is loaded ahead of the first of them ([100,300,7,7]
   // 14.6 us where each load waited for the store before it, and 8.9 so; [2,2048,14,108] 22.7 and 19.1)
-  Pack<VEC> old[DIR == 1 ? E : 1];
-  if (DIR == 1 && a.accumulate) {
+  // (sixteen single floats more would spill, and in the residual epilogue, three tensors already, the place for them costs the assigning
+  // form loads in flight: [41,643,136] 17.7 us and 22.5, [82,246,124] 13.8 and 17.1)
+  constexpr bool kAhead = DIR == 1 && !EXTRA && (VEC == 4 || F < 16);
+  Pack<VEC> old[kAhead ? E : 1];
+  if (kAhead && a.accumulate) {
     uint32_t at = off0, to = col0;
 #pragma unroll
     for (int k = 0; k < E; ++k) {
@@ -204,6 +213,7 @@ __global__ void __launch_bounds__(kChanThreads, 2) bn_chan_kernel(const FusedArg
   for (int k = 0; k < E; ++k) {
     if (k < cnt) {
       Pack<VEC> o;
+      if (DIR == 1 && !kAhead && a.accumulate) old[0] = Pack<VEC>::load(a.out + off);
 #pragma unroll
       for (int i = 0; i < VEC; ++i) {
         if (DIR == 0) {
@@ -212,7 +222,7 @@ __global__ void __launch_bounds__(kChanThreads, 2) bn_chan_kernel(const FusedArg
           o.v[i] = yb * (yb > 0.0f ? 1.0f : slope);
         } else {
           const float dx = fmaf(scale, ve[k].v[i], fmaf(cB, vx[k].v[i], cC));
-          o.v[i] = a.accumulate ? old[k].v[i] + dx : dx;
+          o.v[i] = a.accumulate ? old[kAhead ? k : 0].v[i] + dx : dx;
         }
       }
       o.put(a.out + off);
@@ -227,21 +237,27 @@ __global__ void __launch_bounds__(kChanThreads, 2) bn_chan_kernel(const FusedArg
 
 typedef void (*ChanKernel)(const FusedArgs, const ChanGeom);
 
-template <int DIR, bool EXTRA>
-static ChanKernel chan_kernel_of(uint32_t vec, uint32_t f)
+template <int DIR, bool EXTRA, int VEC>
+static ChanKernel chan_kernel_of(uint32_t f, bool dense)
 {
-  if (vec == 4) {
-    if (f == 4) return bn_chan_kernel<DIR, 4, 4, EXTRA>;
-    if (f == 8) return bn_chan_kernel<DIR, 4, 8, EXTRA>;
-    if (f == 16) return bn_chan_kernel<DIR, 4, 16, EXTRA>;
-    if constexpr (DIR == 0 && !EXTRA) return bn_chan_kernel<DIR, 4, 32, EXTRA>;
-  } else {
-    if (f == 4) return bn_chan_kernel<DIR, 1, 4, EXTRA>;
-    if (f == 8) return bn_chan_kernel<DIR, 1, 8, EXTRA>;
-    if (f == 16) return bn_chan_kernel<DIR, 1, 16, EXTRA>;
-    if constexpr (DIR == 0 && !EXTRA) return bn_chan_kernel<DIR, 1, 32, EXTRA>;
-  }
+  if (f == 4) return dense ? bn_chan_kernel<DIR, VEC, 4, EXTRA, true> : bn_chan_kernel<DIR, VEC, 4, EXTRA, false>;
+  if (f == 8) return dense ? bn_chan_kernel<DIR, VEC, 8, EXTRA, true> : bn_chan_kernel<DIR, VEC, 8, EXTRA, false>;
+  if (f == 16) return bn_chan_kernel<DIR, VEC, 16, EXTRA, false>;
+  if constexpr (DIR == 0 && !EXTRA) return bn_chan_kernel<DIR, VEC, 32, EXTRA, false>;
   return nullptr;
+}
+template <int DIR, bool EXTRA>
+static ChanKernel chan_kernel_of(const ChanGeom &g, bool dense)
+{
+  return g.vec == 4 ? chan_kernel_of<DIR, EXTRA, 4>(g.floats, dense) : chan_kernel_of<DIR, EXTRA, 1>(g.floats, dense);
+}
+
+// Whether the grid is one wave of blocks with fewer registers, and more than one with 64.
+static bool chan_dense(const ChanGeom &g, uint32_t blocks, uint32_t threads)
+{
+  if (g.floats > 8) return false;
+  const uint32_t sms = sm_count(), few = g.floats == 4 ? 48u : 56u;
+  return blocks > 65536 / (64 * threads) * sms && blocks <= 65536 / (few * threads) * sms;
 }
 
 static bool chan_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, bool aligned, ChanGeom &g)
@@ -375,13 +391,15 @@ int launch_chan(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)
   ChanGeom g;
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
   if (!chan_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, extra, aligned, g)) return ANODE_E_LAUNCH;
-  ChanKernel k = dir == 0 ? (extra ? chan_kernel_of<0, true>(g.vec, g.floats) : chan_kernel_of<0, false>(g.vec, g.floats))
-                          : (extra ? chan_kernel_of<1, true>(g.vec, g.floats) : chan_kernel_of<1, false>(g.vec, g.floats));
-  if (!k) return ANODE_E_LAUNCH;
   const bool solo = g.threads == 32;
+  const uint32_t blocks = solo ? ceil_div_u32(a.plan.C, kChanWarpTeams) : a.plan.C * g.cluster, threads = solo ? 32 * kChanWarpTeams : g.threads;
+  const bool dense = chan_dense(g, blocks, threads);
+  ChanKernel k = dir == 0 ? (extra ? chan_kernel_of<0, true>(g, dense) : chan_kernel_of<0, false>(g, dense))
+                          : (extra ? chan_kernel_of<1, true>(g, dense) : chan_kernel_of<1, false>(g, dense));
+  if (!k) return ANODE_E_LAUNCH;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(solo ? ceil_div_u32(a.plan.C, kChanWarpTeams) : a.plan.C * g.cluster);
-  cfg.blockDim = dim3(solo ? 32 * kChanWarpTeams : g.threads);
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
   cfg.stream = stream;
   // The launch may overlap the tail of the kernel before it on the stream; every block waits for that kernel's
   // results (griddepcontrol.wait) before it touches memory.
