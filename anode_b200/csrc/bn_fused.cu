@@ -91,8 +91,8 @@ struct ShapeInfo {
   uint64_t tiled_bytes, static_bytes, part_bytes;      // see fill_shape_info
   bool band_ok[2][2];            // the streaming kernel's form for the largest layers, likewise
   BandGeom band[2][2];
-  bool masked_ok[2][2];          // the streaming kernel's masked form, likewise
-  StreamGeom masked[2][2];
+  bool stream_ok[2][2], masked_ok[2][2];      // the streaming kernel and its masked form, likewise (one of them at most)
+  StreamGeom stream[2][2];
   bool long_ok[2][2];            // its counterpart for long rows, likewise
   LongGeom long_rows[2][2];
 };
@@ -473,9 +473,18 @@ static void fill_shape_info(ShapeInfo &s)
   }
   for (int dir = 0; dir < 2; ++dir)
     for (int ex = 0; ex < 2; ++ex) {
-      s.masked_ok[dir][ex] = masked_plan(s.dim0, s.C, s.N, dir, ex != 0, s.masked[dir][ex]);
+      s.stream_ok[dir][ex] = stream_plan(s.dim0, s.C, s.N, dir, ex != 0, s.stream[dir][ex]);
+      s.masked_ok[dir][ex] = !s.stream_ok[dir][ex] && masked_plan(s.dim0, s.C, s.N, dir, ex != 0, s.stream[dir][ex]);
       s.long_ok[dir][ex] = long_plan(s.dim0, s.C, s.N, dir, ex != 0, s.long_rows[dir][ex]);
     }
+}
+
+bool stream_geom_of(const FusedArgs &a, int dir, StreamGeom &g)
+{
+  const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
+  const ShapeInfo &s = shape_info(a.plan.dim0, a.plan.C, a.plan.N);
+  if (s.stream_ok[dir][extra]) g = s.stream[dir][extra];
+  return s.stream_ok[dir][extra];
 }
 
 bool masked_geom_of(const FusedArgs &a, int dir, StreamGeom &g)
@@ -483,7 +492,7 @@ bool masked_geom_of(const FusedArgs &a, int dir, StreamGeom &g)
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
   if (a.mode != MODE_FUSED || a.world > 1) return false;
   const ShapeInfo &s = shape_info(a.plan.dim0, a.plan.C, a.plan.N);
-  if (s.masked_ok[dir][extra]) g = s.masked[dir][extra];
+  if (s.masked_ok[dir][extra]) g = s.stream[dir][extra];
   return s.masked_ok[dir][extra];
 }
 
@@ -569,19 +578,20 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
   return resident_applies(a, dir, aligned) ? ANODE_KERNEL_RESIDENT : -1;
 }
 
-// Rows without an aligned run of channels, on one GPU: where the streaming kernel's masked form is launched in the place of the kernel
-// that pick_kernel_kind names.  Us there and here, forward, backward, residual forward and backward:
-//  - the plain kernel everywhere (figures at the head of bn_stream.cu);
-//  - the register-resident kernel, which loads such rows float by float, from these sizes and twenty samples on: [1084,111,18], 2.2 M,
-//    9.7, 16.6, 16.3, 29.7 and 8.6, 11.3, 10.4, 13.4; [270,490,49] 22.9, 34.9, 34.8, 61.1 and 15.8, 22.6, 19.6, 30.1; [356,2022,25] 59, 84, 85, 157
-//    and 35, 56, 46, 80; but [67,706,37], 1.75 M, 5.2, 8.1, 7.6, 15.7 and 6.6, 8.9, 8.4, 10.2, [802,67,19], 1.0 M, 4.5, 5.5, 5.0, 7.2 and 6.6,
-//    8.1, 7.8, 9.3, and few samples, [16,2017,151] 17.5, 22.2, 22.6, 39.7 and 22.4, 23.8, 25.1, 32.9;
-//  - the tiled kernel, which copies a row at a time, on rows below 200 floats: [604,18,221] 16.4, 20.5, 18.5, 25.6 and 9.3, 11.7, 10.6, 14.8,
-//    [1826,159,179] 128, 246, 213, - and 118, 186, 153, -, [1403,355,131] forward 191 and 143; but [1594,54,227] 54, 81, 77, 101 and 58, 80, 69, 107;
-//    on longer ones in small layers, where the tiled kernel's launch costs ten us: [947,13,350] 19.5, 25.0, 22.6, 27.5 and 13.3, 22.7, 20.1,
-//    30.6, but [2147,15,254], 8.2 M, 27.5, 42.0, 39.0, 49.4 and 29.2, 46.1, 42.6, 63.5.
+// Odd rows, on one GPU: where the streaming kernel, or its masked form for rows without an aligned run of channels, is launched in the
+// place of the kernel that pick_kernel_kind names.  Us there and here, forward, backward, residual forward and backward:
+//  - the plain kernel everywhere (masked; figures at the head of bn_stream.cu);
+//  - the register-resident kernel, which loads such rows float by float, from these sizes and twenty samples on.  Masked: [270,490,49]
+//    22.9, 34.9, 34.8, 61.1 and 15.8, 22.6, 19.6, 30.1, [356,2022,25] 59, 84, 85, 157 and 35, 56, 46, 80; but [67,706,37], 1.75 M, 5.2, 8.1, 7.6,
+//    15.7 and 6.6, 8.9, 8.4, 10.2, [802,67,19], 1.0 M, 4.5, 5.5, 5.0, 7.2 and 6.6, 8.1, 7.8, 9.3, and few samples, [16,2017,151] 17.5, 22.2,
+//    22.6, 39.7 and 22.4, 23.8, 25.1, 32.9.  Aligned runs: [188,356,39], 2.6 M, 11.5, 11.1, 14.8, 31.7 and 6.3, 9.1, 8.3, 12.0, [2604,86,14]
+//    12.8, 16.3, 19.4, 36.0 and 11.0, 15.0, 13.2, 21.1, but [2311,68,14], 2.2 M, 6.7, 9.8, 10.6, 20.6 and 8.4, 10.1, 9.6, 13.2;
+//  - the tiled kernel, which copies a row at a time, masked, on rows below 200 floats: [604,18,221] 16.4, 20.5, 18.5, 25.6 and 9.3, 11.7,
+//    10.6, 14.8, [1826,159,179] 128, 246, 213, - and 118, 186, 153, -, [1403,355,131] forward 191 and 143; but [1594,54,227] 54, 81, 77, 101 and
+//    58, 80, 69, 107; on longer ones in small layers, where the tiled kernel's launch costs ten us: [947,13,350] 19.5, 25.0, 22.6, 27.5 and 13.3,
+//    22.7, 20.1, 30.6, but [2147,15,254], 8.2 M, 27.5, 42.0, 39.0, 49.4 and 29.2, 46.1, 42.6, 63.5.
 constexpr uint32_t kMaskedSamples = 20, kMaskedShortRow = 200;
-constexpr uint64_t kMaskedChan[2][2] = {{2100000, 1900000}, {1900000, 1100000}};        // [direction][residual]
+constexpr uint64_t kMaskedChan[2][2] = {{2300000, 2100000}, {2300000, 1100000}};        // [direction][residual]
 constexpr uint64_t kMaskedTiled[2][2] = {{8000000, 5000000}, {4500000, 2500000}};
 static bool masked_takes(const FusedArgs &a, int dir, int kind, StreamGeom &g)
 {
@@ -590,21 +600,23 @@ static bool masked_takes(const FusedArgs &a, int dir, int kind, StreamGeom &g)
   if (a.plan.dim0 % 4 == 0) return false;
   if (kind == ANODE_KERNEL_REGISTER && (a.plan.N < kMaskedSamples || elements < kMaskedChan[dir][extra])) return false;
   if (kind == ANODE_KERNEL_TILED && a.plan.dim0 >= kMaskedShortRow && (a.plan.N < kMaskedSamples || elements > kMaskedTiled[dir][extra])) return false;
-  return masked_geom_of(a, dir, g);
+  return (kind == ANODE_KERNEL_REGISTER && stream_geom_of(a, dir, g)) || masked_geom_of(a, dir, g);
 }
 
 // Rows of 250 floats and more, on one GPU: where the kernel for long rows (bn_long.cu) is launched in the place of the one that
 // pick_kernel_kind names.  Us there and here, forward, backward, residual forward and backward:
 //  - the tiled kernel where its launch (twelve us and the layer's bytes) is more than the estimate of the other: [1,3,64,64,64] 12.5,
 //    12.4, -, - and 6.0, 7.9, -, -, [1,11,99716] -, 13.8, 13.2, 13.0 and -, 7.2, 6.7, 9.2, [3,19,75580], 4.3 M, 16.6, 18.0, 17.7, 26.4 and 10.3, 15.2,
-//    15.1, 19.4; but [1,4,1630016], 6.5 M, 19.4, 25.2, 22.3, 31.8 and 28.6, 47.6, 47.3, 58.0.  By that rule 0.8 per cent are lost against the
-//    better of the two over 439 passes of 0.3 to 20 M elements;
+//    15.1, 19.4; but [1,4,1630016], 6.5 M, 19.4, 25.2, 22.3, 31.8 and 28.6, 47.6, 47.3, 58.0.  By that rule (and no margin) 0.8 per cent are lost
+//    against the better of the two over 439 passes of 0.3 to 20 M elements;
 //  - the register-resident kernel on ragged rows, which it loads float by float, from these sizes or channels on: [8,217,2678] 18.5, 29.8,
 //    30.9, 52.6 and 12.7, 16.1, 14.5, 20.6, [2,5,19011] 3.8, 5.2, 5.2, 6.9 and 5.1, 4.1, 4.5, 4.6, [9,4,12887] forward 8.1 and 5.5, but
-//    [10,119,1502], 1.8 M, 5.4, 8.5, 8.0 and 7.9, 10.0, 9.8; and on aligned ones in the residual epilogue: [6,276,2060], 3.4 M, 11.7, 16.9 and 10.8,
+//    [10,119,1502], 1.8 M, 5.4, 8.5, 8.0 and 7.9, 10.0, 9.8, and where the clusters take a second wave, [71,25,577] backward 7.1 and 8.9,
+//    [3,1023,366] residual backward 8.0 and 11.3; and on aligned ones in the residual epilogue: [6,276,2060], 3.4 M, 11.7, 16.9 and 10.8,
 //    15.7, [7,331,1108], 2.6 M, backward 12.9 and 10.5.
-constexpr uint32_t kLongRow = 250;
+constexpr uint32_t kLongRow = 250, kLongFewChannels = 128, kLongOneWave = 20;
 constexpr uint64_t kLongTiledMost = 12000000;
+constexpr uint64_t kLongManyChannels = 2400000;
 constexpr uint64_t kLongChan[2][2] = {{3300000, 1800000}, {1800000, 700000}};           // [direction][residual]
 constexpr uint64_t kLongChannel[2][2] = {{64 << 10, 32 << 10}, {32 << 10, 24 << 10}};
 constexpr uint64_t kLongChanAligned[2][2] = {{~0ull, 3000000}, {~0ull, 2400000}};
@@ -614,10 +626,12 @@ static bool long_takes(const FusedArgs &a, int dir, int kind, LongGeom &g)
   const uint64_t channel = (uint64_t)a.plan.dim0 * a.plan.N, elements = channel * a.plan.C;
   if (a.plan.dim0 < kLongRow) return false;
   if (kind == ANODE_KERNEL_TILED)
-    return elements <= kLongTiledMost && long_geom_of(a, dir, g) && g.cost * 1.05f < 12.0f + (float)elements * (dir == 0 ? (extra ? 12 : 8) : extra ? 20 : 12) * 1.6e-7f;
+    return elements <= kLongTiledMost && long_geom_of(a, dir, g) && g.cost * 1.12f < 12.0f + (float)elements * (dir == 0 ? (extra ? 12 : 8) : extra ? 20 : 12) * 1.6e-7f;
   if (kind != ANODE_KERNEL_REGISTER) return false;
-  return (a.plan.dim0 % 4 == 0 ? elements >= kLongChanAligned[dir][extra] : elements >= kLongChan[dir][extra] || channel >= kLongChannel[dir][extra]) &&
-         long_geom_of(a, dir, g);
+  const uint32_t C = a.plan.C;
+  return (a.plan.dim0 % 4 == 0 ? elements >= kLongChanAligned[dir][extra]
+                               : (elements >= kLongChan[dir][extra] && (C <= kLongFewChannels || elements >= kLongManyChannels)) ||
+                                     (channel >= kLongChannel[dir][extra] && C <= kLongOneWave)) && long_geom_of(a, dir, g);
 }
 
 // Launches the one of those two that takes the call, if any.

@@ -115,6 +115,8 @@ bool stream_applies(const FusedArgs &a, int dir, bool aligned);
 uint32_t stream_cluster(const FusedArgs &a, int dir, bool aligned, uint32_t &blocks);
 bool stream_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok);
 int launch_stream(FusedArgs &a, int dir, cudaStream_t stream);
+bool stream_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, StreamGeom &g);      // geometry of a shape, and of a prepared call
+bool stream_geom_of(const FusedArgs &a, int dir, StreamGeom &g);
 // its masked form for rows without an aligned run: the geometry of a shape, and of a prepared call on aligned tensors
 bool masked_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, StreamGeom &g);
 bool masked_geom_of(const FusedArgs &a, int dir, StreamGeom &g);

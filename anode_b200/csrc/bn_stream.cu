@@ -383,44 +383,73 @@ static bool stream_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool ext
   return true;
 }
 
+// Estimated us of units of `cb` channels and clusters of `cl` blocks: a fixed part per wave of blocks (clusters of 8 and 16 fill 85 and
+// 78 per cent of the device's places), and the larger of a thread's chain of batches and the bytes moved, where the cache lines that
+// two runs share come twice, what exceeds L2 between the two walks comes again, and idle threads leave bandwidth unused.  The
+// figures are fitted to 570 launches of the masked form, 60 shapes (16 to 480 floats a row, 3 to 1500 channels, 0.6 to 120 M elements, four
+// directions) with up to 30 units and clusters each: what is chosen by it is 3 per cent above the best of them on average.
+static double stream_cost(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, bool masked, uint32_t cb, uint32_t cl, uint32_t groups, uint32_t L4)
+{
+  const uint32_t wave = kStreamBlocks * sm_count(), run = cb * dim0, rows = ceil_div_u32(N, cl), used = groups < rows ? groups : rows;
+  const double bytes = 4.0 * dim0 * C * N * (dir == 0 ? (extra ? 3 : 2) : extra ? 5 : 3);
+  const double sample = (dir == 0 && !extra ? 1.5 : 2.0) / (dir == 0 ? (extra ? 4 : 8) : extra && masked ? 3 : 4);      // us per sample of a thread
+  const double window = 77e6, rate = 5.15e6;      // bytes that L2 keeps; bytes per us
+  const uint64_t blocks = (uint64_t)ceil_div_u32(C, cb) * cl, places = cl == 16 ? wave * 25 / 32 : cl == 8 ? wave * 17 / 20 : cl == 4 ? wave * 15 / 16 : wave;
+  const double waves = (double)((blocks + places - 1) / places), resident = (double)(blocks < places ? blocks : places);
+  const double over = 4.0 * run * N * (dir == 1 ? 2 : 1) / cl * resident / window - 1;
+  const double again = (dir == 1 ? 0.5 : 0.17) * (over < 0 ? 0 : over > 1 ? 1 : over), lanes = resident * used * L4 / ((double)wave * kStreamThreads);
+  const double moved = bytes * (1 + 9.0 / run) * (1 + again) / rate * (0.9 + 0.1 / lanes);
+  const double chain = waves * ceil_div_u32(rows, used) * sample;
+  return 0.6 + waves * (3.0 + 0.024 * cl) + pow(pow(moved, 2.5) + pow(chain, 2.5), 0.4);
+}
+
+static void stream_set(StreamGeom &g, uint32_t C, uint32_t N, uint32_t cb, uint32_t cl, uint32_t groups, uint32_t L4)
+{
+  g.cb = cb; g.units = ceil_div_u32(C, cb); g.cluster = cl; g.rows = ceil_div_u32(N, cl);
+  g.groups = groups < g.rows ? groups : g.rows;
+  g.threads = (g.groups * L4 + 31) / 32 * 32;
+}
+
+// The geometry that is launched: stream_geom's, or the one of the least estimated time where that is this much less.  Us so and with
+// stream_geom's alone, forward, backward, residual forward and backward: [3865,36,18] 8.9, 11.7, 10.7, 15.4 and 11.0, 17.4, 16.9, 23.3, [1148,44,80]
+// 9.4, 14.6, 11.7, 19.3 and 13.4, 21.2, 18.0, 25.6, [20,1998,102] 9.7, 13.8, 11.4, 18.7 and 14.0, 16.6, 16.6, 19.6, [148,750,38] 9.4, 15.1, 12.6, 20.4 and
+// 19.9, 26.4, 23.1, 30.0; 5 to 9 per cent less over 120 shapes.  (Without the margin some were slower, [1217,108,87] 23.5 and 27.4.)
+constexpr double kStreamOther = 0.85;
+bool stream_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, StreamGeom &g)
+{
+  if (!stream_geom(dim0, C, N, dir, extra, g)) return false;
+  const uint32_t q = dim0 % 4 == 0 ? 1 : dim0 % 2 == 0 ? 2 : 4;
+  double best = kStreamOther * stream_cost(dim0, C, N, dir, extra, false, g.cb, g.cluster, g.groups, g.cb * dim0 / 4);
+  for (uint32_t cb = q; cb <= C && cb <= kStreamChannels && cb * dim0 <= 4 * kStreamThreads; cb += q) {
+    const uint32_t L4 = cb * dim0 / 4, groups = kStreamThreads / L4 < N ? kStreamThreads / L4 : N;
+    if (cb * dim0 < 32 && cb + q <= C) continue;
+    for (uint32_t cl = 1; cl <= 16 && cl * cb <= kStreamRecords && (cl == 1 || N / cl >= groups * 2); cl *= 2) {
+      const double cost = stream_cost(dim0, C, N, dir, extra, false, cb, cl, groups, L4);
+      if (cost < best) { best = cost; stream_set(g, C, N, cb, cl, groups, L4); }
+    }
+  }
+  return true;
+}
+
 // The masked form (RAG): runs of any channels.  The samples of a thread lie a multiple of four floats apart, so the groups of a
 // block are an even number or a multiple of four where C*dim0 asks for it (unless a thread has one sample anyway), and rows are
-// no longer than leaves place for those.
-// Unit and cluster are those of the least estimated time: a fixed part per wave of blocks (clusters of 8 and 16 fill 85 and 78 per
-// cent of the device's places), and the larger of a thread's chain of batches and the bytes moved, where the cache lines that two
-// runs share come twice, what exceeds L2 between the two walks comes again, and idle threads leave bandwidth unused.  The
-// figures are fitted to 570 launches of 60 shapes (16 to 480 floats a row, 3 to 1500 channels, 0.6 to 120 M elements, four
-// directions) with up to 30 units and clusters each: what is chosen is 3 per cent above the best of them on average; the least
-// idle threads and the aligned form's clusters, as chosen there, were 11 per cent slower over 70 other shapes, a third at 3 to 10 channels.
+// no longer than leaves place for those.  (The least idle threads and the aligned form's clusters, as chosen by stream_geom, were 11 per
+// cent slower over 70 shapes, a third at 3 to 10 channels.)
 bool masked_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, StreamGeom &g)
 {
-  const uint32_t rs = C * dim0, m = rs % 4 == 0 ? 1u : rs % 2 == 0 ? 2u : 4u, wave = kStreamBlocks * sm_count();
+  const uint32_t rs = C * dim0, m = rs % 4 == 0 ? 1u : rs % 2 == 0 ? 2u : 4u;
   StreamGeom aligned;
   if (dim0 < 4 || stream_geom(dim0, C, N, dir, extra, aligned)) return false;
-  const double bytes = 4.0 * dim0 * C * N * (dir == 0 ? (extra ? 3 : 2) : extra ? 5 : 3);
-  const double batch_us = (dir == 0 && !extra ? 1.5 : 2.0) / (dir == 0 ? (extra ? 4 : 8) : extra ? 3 : 4);      // per sample of a thread
-  const double window = 77e6, rate = 5.15e6;      // bytes that L2 keeps; bytes per us
   double best = 0;
   for (uint32_t cb = 1; cb <= C && cb <= kStreamChannels && (cb * dim0 + 6) / 4 <= kStreamThreads; ++cb) {
-    const uint32_t run = cb * dim0, L4 = (run + 6) / 4, units = ceil_div_u32(C, cb);
-    if (run < 16 && cb < C) continue;
+    const uint32_t L4 = (cb * dim0 + 6) / 4;
+    if (cb * dim0 < 16 && cb < C) continue;
     uint32_t groups = kStreamThreads / L4;
     groups = groups >= N ? N : groups / m * m;
     if (groups == 0) break;
     for (uint32_t cl = 1; cl <= 16 && cl * cb <= kStreamRecords && (cl == 1 || N / cl >= groups * 2); cl *= 2) {
-      const uint64_t blocks = (uint64_t)units * cl, places = cl == 16 ? wave * 25 / 32 : cl == 8 ? wave * 17 / 20 : cl == 4 ? wave * 15 / 16 : wave;
-      const double waves = (double)((blocks + places - 1) / places), resident = (double)(blocks < places ? blocks : places);
-      const uint32_t rows = ceil_div_u32(N, cl), used = groups < rows ? groups : rows;
-      const double over = 4.0 * run * N * (dir == 1 ? 2 : 1) / cl * resident / window - 1;
-      const double again = (dir == 1 ? 0.5 : 0.17) * (over < 0 ? 0 : over > 1 ? 1 : over), lanes = resident * used * L4 / ((double)wave * kStreamThreads);
-      const double moved = bytes * (1 + 9.0 / run) * (1 + again) / rate * (0.9 + 0.1 / lanes);
-      const double chain = waves * ceil_div_u32(rows, used) * batch_us;
-      const double cost = 0.6 + waves * (3.0 + 0.024 * cl) + pow(pow(moved, 2.5) + pow(chain, 2.5), 0.4);
-      if (best == 0 || cost < best) {
-        best = cost; g.cost = (float)cost;
-        g.cb = cb; g.units = units; g.cluster = cl; g.rows = rows; g.groups = used;
-        g.threads = (used * L4 + 31) / 32 * 32;
-      }
+      const double cost = stream_cost(dim0, C, N, dir, extra, true, cb, cl, groups, L4);
+      if (best == 0 || cost < best) { best = cost; g.cost = (float)cost; stream_set(g, C, N, cb, cl, groups, L4); }
     }
   }
   g.inv_count = 1.0 / ((double)dim0 * (double)N);
@@ -484,7 +513,7 @@ bool stream_preferred(const FusedArgs &a, int dir, bool aligned, bool tiled_ok)
 int launch_stream(FusedArgs &a, int dir, cudaStream_t stream)
 {
   StreamGeom g;
-  const bool masked = !stream_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, stream_extra(a, dir), g);
+  const bool masked = !stream_geom_of(a, dir, g);
   if (masked && !masked_geom_of(a, dir, g)) return ANODE_E_LAUNCH;
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
   // dres may be stored before x is read again only where it is not x itself
@@ -504,7 +533,7 @@ extern "C" int anode_gpu_batch_norm_stream_geometry(uint32_t dim0, uint32_t dim1
   using namespace anode_b200;
   if (!out || (dir != 0 && dir != 1) || check_dims(dim0, dim1, dim2)) return ANODE_E_DIMS;
   StreamGeom g{};
-  const bool ok = stream_geom(dim0, dim1, dim2, dir, false, g);
+  const bool ok = stream_plan(dim0, dim1, dim2, dir, false, g);
   const uint32_t v[7] = {ok ? 1u : 0u, g.cb, g.units, g.cluster, g.rows, g.groups, g.threads};
   for (int i = 0; i < 7; ++i) out[i] = v[i];
   return ANODE_OK;

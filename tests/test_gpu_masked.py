@@ -147,7 +147,7 @@ def test_it_serves_what_the_plain_kernel_is_named_for(shape):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("shape,named,launched", [
-    ((1084, 111, 1, 18), ["register"] * 4, ["stream"] * 4), ((67, 706, 1, 37), ["register"] * 4, ["register"] * 3 + ["stream"]),
+    ((1384, 111, 1, 18), ["register"] * 4, ["stream"] * 4), ((67, 706, 1, 37), ["register"] * 4, ["register"] * 3 + ["stream"]),
     ((16, 2017, 1, 151), ["register"] * 4, ["register"] * 4), ((604, 18, 13, 17), ["tiled"] * 4, ["stream"] * 4),
     ((4294, 15, 1, 254), ["tiled"] * 4, ["tiled"] * 4), ((1841, 15, 1, 165), ["tiled"] * 3 + ["plain"], ["stream"] * 4)])
 def test_where_it_is_launched(shape, named, launched):
