@@ -740,14 +740,8 @@ __global__ void __launch_bounds__(kRingThreads, 1) bn_ring_kernel(const FusedArg
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (TMEM && g.keep_slots && warp == 0) { __syncwarp(); tmem_alloc(&ctl->tmem); tmem_fence_before(); }
-  // the producer, which set up the barriers, goes ahead to its first copies
-  if (warp == kConsumers / 32) {
-    __syncwarp();
-    asm volatile("barrier.cta.arrive 1, %0;" ::"n"(kRingThreads) : "memory");
-  } else {
-    asm volatile("barrier.cta.sync 1, %0;" ::"n"(kRingThreads) : "memory");
-    if (TMEM && g.keep_slots) tmem_fence_after();
-  }
+  __syncthreads();
+  if (TMEM && g.keep_slots) tmem_fence_after();
 
   Sched sc; sc.init(a);
   // the two warps that use the tagged words each see to it that ctl->parity is there for them (in shared memory: a register more and
