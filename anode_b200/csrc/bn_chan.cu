@@ -255,7 +255,7 @@ static ChanKernel chan_kernel_of(const ChanGeom &g, bool dense)
 // Whether the grid is one wave of blocks with fewer registers, and more than one with 64.
 static bool chan_dense(const ChanGeom &g, uint32_t blocks, uint32_t threads)
 {
-  if (g.floats > 8) return false;
+  if (g.floats > 8 || blocks < 256) return false;      // (a wave is more than that)
   const uint32_t sms = sm_count(), few = g.floats == 4 ? 48u : 56u;
   return blocks > 65536 / (64 * threads) * sms && blocks <= 65536 / (few * threads) * sms;
 }
@@ -269,7 +269,8 @@ static bool chan_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra
   g.d0v = dim0 / g.vec; g.total = (uint32_t)total;
   // floats per thread: as few as leave the whole problem on the device at once (about 1024 threads per SM)
   uint32_t f = 4;
-  while (f < fmax && ((uint64_t)C * total * g.vec > (uint64_t)f * sm_count() * 1024 ||
+  const uint32_t most = sm_count() * 1024;
+  while (f < fmax && ((uint64_t)C * total * g.vec > (uint64_t)f * most ||
                       total > (uint64_t)kChanThreads * kChanCluster * (f / g.vec))) f *= 2;
   const uint32_t e = f / g.vec;
   const uint32_t need = (uint32_t)((total + e - 1) / e);             // threads of the team

@@ -297,11 +297,16 @@ bool ring_plan_for(uint32_t dim0, uint32_t C, uint32_t N, bool aligned, int dir,
 
 // Plan of the warp-specialised kernel for a prepared call, or false when it does not serve it.  Ragged rows and the
 // residual epilogue are one-launch, one-GPU forms.
-static bool ring_plan_of(const FusedArgs &a, int dir, bool aligned, Plan &p, RingGeom &g)
+static bool ring_serves(const FusedArgs &a, int dir, bool aligned)
 {
   const bool extra = a.res || a.ymask || a.dres;
-  if ((extra || a.plan.dim0 % 4 != 0) && (a.mode != MODE_FUSED || a.world > 1)) return false;
-  return ring_plan_for(a.plan.dim0, a.plan.C, a.plan.N, aligned, dir, extra, p, g) && p.ws_bytes <= a.ws_capacity;
+  if (!aligned || ((extra || a.plan.dim0 % 4 != 0) && (a.mode != MODE_FUSED || a.world > 1))) return false;
+  const ShapeInfo &s = shape_info(a.plan.dim0, a.plan.C, a.plan.N);
+  return s.ring_ok[dir][extra] && s.ring_plan[dir][extra].ws_bytes <= a.ws_capacity;
+}
+static bool ring_plan_of(const FusedArgs &a, int dir, bool aligned, Plan &p, RingGeom &g)
+{
+  return ring_serves(a, dir, aligned) && ring_plan_for(a.plan.dim0, a.plan.C, a.plan.N, aligned, dir, a.res || a.ymask || a.dres, p, g);
 }
 
 // Bytes of a part up to the end of that plan's words; 0 when the kernel does not serve the call.
@@ -544,8 +549,8 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
 {
   const bool extra = a.res || a.ymask || a.dres;        // residual epilogue
   const bool plain_ok = !(a.mode == MODE_FUSED && a.world > 1);
-  Plan rp; RingGeom g; StreamGeom mg;
-  const bool tiled_ok = ring_plan_of(a, dir, aligned, rp, g) && (kernel_choice() != ANODE_KERNEL_AUTO || tiled_preferred(a, dir));
+  StreamGeom mg;
+  const bool tiled_ok = ring_serves(a, dir, aligned) && (kernel_choice() != ANODE_KERNEL_AUTO || tiled_preferred(a, dir));
   switch (kernel_choice()) {
     case ANODE_KERNEL_TILED: if (tiled_ok) return ANODE_KERNEL_TILED; break;
     case ANODE_KERNEL_CLUSTER: if (segres_applies(a, dir, aligned)) return ANODE_KERNEL_CLUSTER; break;
@@ -752,8 +757,9 @@ int prepare_fwd(FusedArgs &a, uint32_t dim0, uint32_t dim1, uint32_t dim2, float
   if (!aligned4(x) || !aligned4(y)) return ANODE_E_ALIGN;
   if (!ws || !aligned16(ws)) return ANODE_E_WORKSPACE;
   a = FusedArgs{};
-  a.plan = plan_for(dim0, dim1, dim2, aligned16(x) && aligned16(y));
-  const uint64_t part = workspace_part_bytes(dim0, dim1, dim2);
+  const ShapeInfo &shape = shape_info(dim0, dim1, dim2);
+  a.plan = shape.plan[aligned16(x) && aligned16(y) ? 1 : 0];
+  const uint64_t part = shape.part_bytes;
   if (ws_bytes < part) return ANODE_E_WORKSPACE;              // forward uses the first part only
   a.ws_capacity = part;
   a.status = static_cast<uint32_t *>(ws);
@@ -778,8 +784,9 @@ int prepare_bwd(FusedArgs &a, uint32_t dim0, uint32_t dim1, uint32_t dim2, int r
   if (!aligned4(x) || !aligned4(dy) || !aligned4(dx)) return ANODE_E_ALIGN;
   if (!ws || !aligned16(ws)) return ANODE_E_WORKSPACE;
   a = FusedArgs{};
-  a.plan = plan_for(dim0, dim1, dim2, aligned16(x) && aligned16(dy) && aligned16(dx));
-  const uint64_t part = workspace_part_bytes(dim0, dim1, dim2);
+  const ShapeInfo &shape = shape_info(dim0, dim1, dim2);
+  a.plan = shape.plan[aligned16(x) && aligned16(dy) && aligned16(dx) ? 1 : 0];
+  const uint64_t part = shape.part_bytes;
   if (ws_bytes < 2 * part) return ANODE_E_WORKSPACE;
   a.ws_capacity = part;
   a.status = static_cast<uint32_t *>(ws);
@@ -841,7 +848,7 @@ extern "C" int anode_gpu_batch_norm_relu_fused_fwd_3d1_packed_f32(
   const int rc = prepare_fwd(a, dim0, dim1, dim2, epsilon, avg_rate, relu, x, gamma, beta, y, mean, var,
                              run_mean, run_var, workspace, workspace_bytes);
   if (rc) return rc;
-  if (workspace_bytes < anode_gpu_batch_norm_fused_workspace_bytes(dim0, dim1, dim2)) return ANODE_E_WORKSPACE;
+  if (workspace_bytes < 2 * a.ws_capacity) return ANODE_E_WORKSPACE;
   return launch_best(a, 0, aligned16(x) && aligned16(y), stream);
 }
 
@@ -871,7 +878,7 @@ extern "C" int anode_gpu_batch_norm_act_fused_fwd_3d1_packed_f32(
   const int rc = prepare_fwd(a, dim0, dim1, dim2, epsilon, avg_rate, 1, x, gamma, beta, y, mean, var,
                              run_mean, run_var, workspace, workspace_bytes);
   if (rc) return rc;
-  if (workspace_bytes < anode_gpu_batch_norm_fused_workspace_bytes(dim0, dim1, dim2)) return ANODE_E_WORKSPACE;
+  if (workspace_bytes < 2 * a.ws_capacity) return ANODE_E_WORKSPACE;
   a.neg_slope = neg_slope;
   return launch_best(a, 0, aligned16(x) && aligned16(y), stream);
 }
@@ -909,7 +916,7 @@ extern "C" int anode_gpu_batch_norm_add_act_fused_fwd_3d1_packed_f32(
   const int rc = prepare_fwd(a, dim0, dim1, dim2, epsilon, avg_rate, 1, x, gamma, beta, y, mean, var,
                              run_mean, run_var, workspace, workspace_bytes);
   if (rc) return rc;
-  if (workspace_bytes < anode_gpu_batch_norm_fused_workspace_bytes(dim0, dim1, dim2)) return ANODE_E_WORKSPACE;
+  if (workspace_bytes < 2 * a.ws_capacity) return ANODE_E_WORKSPACE;
   a.neg_slope = neg_slope;
   a.res = residual;
   if (!aligned16(residual)) a.plan = plan_for(dim0, dim1, dim2, false);      // scalar path
