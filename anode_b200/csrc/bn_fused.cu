@@ -91,10 +91,11 @@ struct ShapeInfo {
   uint64_t tiled_bytes, static_bytes, part_bytes;      // see fill_shape_info
   bool band_ok[2][2];            // the streaming kernel's form for the largest layers, likewise
   BandGeom band[2][2];
-  bool stream_ok[2][2], masked_ok[2][2];      // the streaming kernel and its masked form, likewise (one of them at most)
-  StreamGeom stream[2][2];
-  bool long_ok[2][2];            // its counterpart for long rows, likewise
-  LongGeom long_rows[2][2];
+  // the streaming kernel and its masked form (one of them at most), and its counterpart for long rows, likewise: searched for when a
+  // call first asks for them (0 not yet, 1 no, 2 yes), since most shapes never do and a search takes some ten microseconds
+  mutable uint8_t stream_ok[2][2], masked_ok[2][2], long_ok[2][2];
+  mutable StreamGeom stream[2][2];
+  mutable LongGeom long_rows[2][2];
 };
 constexpr uint32_t kShapeCache = 64;      // entries per thread, direct mapped
 
@@ -477,19 +478,17 @@ static void fill_shape_info(ShapeInfo &s)
     if (at > s.part_bytes) s.part_bytes = at;
   }
   for (int dir = 0; dir < 2; ++dir)
-    for (int ex = 0; ex < 2; ++ex) {
-      s.stream_ok[dir][ex] = stream_plan(s.dim0, s.C, s.N, dir, ex != 0, s.stream[dir][ex]);
-      s.masked_ok[dir][ex] = !s.stream_ok[dir][ex] && masked_plan(s.dim0, s.C, s.N, dir, ex != 0, s.stream[dir][ex]);
-      s.long_ok[dir][ex] = long_plan(s.dim0, s.C, s.N, dir, ex != 0, s.long_rows[dir][ex]);
-    }
+    for (int ex = 0; ex < 2; ++ex) s.stream_ok[dir][ex] = s.masked_ok[dir][ex] = s.long_ok[dir][ex] = 0;
 }
 
 bool stream_geom_of(const FusedArgs &a, int dir, StreamGeom &g)
 {
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
   const ShapeInfo &s = shape_info(a.plan.dim0, a.plan.C, a.plan.N);
-  if (s.stream_ok[dir][extra]) g = s.stream[dir][extra];
-  return s.stream_ok[dir][extra];
+  uint8_t &ok = s.stream_ok[dir][extra];
+  if (!ok) ok = stream_plan(s.dim0, s.C, s.N, dir, extra, s.stream[dir][extra]) ? 2 : 1;
+  if (ok == 2) g = s.stream[dir][extra];
+  return ok == 2;
 }
 
 bool masked_geom_of(const FusedArgs &a, int dir, StreamGeom &g)
@@ -497,8 +496,10 @@ bool masked_geom_of(const FusedArgs &a, int dir, StreamGeom &g)
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
   if (a.mode != MODE_FUSED || a.world > 1) return false;
   const ShapeInfo &s = shape_info(a.plan.dim0, a.plan.C, a.plan.N);
-  if (s.masked_ok[dir][extra]) g = s.stream[dir][extra];
-  return s.masked_ok[dir][extra];
+  uint8_t &ok = s.masked_ok[dir][extra];
+  if (!ok) ok = masked_plan(s.dim0, s.C, s.N, dir, extra, s.stream[dir][extra]) ? 2 : 1;
+  if (ok == 2) g = s.stream[dir][extra];
+  return ok == 2;
 }
 
 bool band_geom_of(const FusedArgs &a, int dir, BandGeom &g)
@@ -515,8 +516,10 @@ bool long_geom_of(const FusedArgs &a, int dir, LongGeom &g)
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
   if (a.mode != MODE_FUSED || a.world > 1) return false;
   const ShapeInfo &s = shape_info(a.plan.dim0, a.plan.C, a.plan.N);
-  if (s.long_ok[dir][extra]) g = s.long_rows[dir][extra];
-  return s.long_ok[dir][extra];
+  uint8_t &ok = s.long_ok[dir][extra];
+  if (!ok) ok = long_plan(s.dim0, s.C, s.N, dir, extra, s.long_rows[dir][extra]) ? 2 : 1;
+  if (ok == 2) g = s.long_rows[dir][extra];
+  return ok == 2;
 }
 
 // Bytes of a part taken by the tile-plan kernels (plain, warp-specialised, cluster); the records of the

@@ -403,6 +403,9 @@ static double stream_cost(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool e
   return 0.6 + waves * (3.0 + 0.024 * cl) + pow(pow(moved, 2.5) + pow(chain, 2.5), 0.4);
 }
 
+// The next number of channels to look at: all up to eight steps of q, then an eighth more each time.
+static uint32_t next_unit(uint32_t cb, uint32_t q) { return cb + (cb / 8 > q ? cb / 8 / q * q : q); }
+
 static void stream_set(StreamGeom &g, uint32_t C, uint32_t N, uint32_t cb, uint32_t cl, uint32_t groups, uint32_t L4)
 {
   g.cb = cb; g.units = ceil_div_u32(C, cb); g.cluster = cl; g.rows = ceil_div_u32(N, cl);
@@ -420,7 +423,7 @@ bool stream_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, Str
   if (!stream_geom(dim0, C, N, dir, extra, g)) return false;
   const uint32_t q = dim0 % 4 == 0 ? 1 : dim0 % 2 == 0 ? 2 : 4;
   double best = kStreamOther * stream_cost(dim0, C, N, dir, extra, false, g.cb, g.cluster, g.groups, g.cb * dim0 / 4);
-  for (uint32_t cb = q; cb <= C && cb <= kStreamChannels && cb * dim0 <= 4 * kStreamThreads; cb += q) {
+  for (uint32_t cb = q; cb <= C && cb <= kStreamChannels && cb * dim0 <= 4 * kStreamThreads; cb = next_unit(cb, q)) {
     const uint32_t L4 = cb * dim0 / 4, groups = kStreamThreads / L4 < N ? kStreamThreads / L4 : N;
     if (cb * dim0 < 32 && cb + q <= C) continue;
     for (uint32_t cl = 1; cl <= 16 && cl * cb <= kStreamRecords && (cl == 1 || N / cl >= groups * 2); cl *= 2) {
@@ -441,7 +444,7 @@ bool masked_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, Str
   StreamGeom aligned;
   if (dim0 < 4 || stream_geom(dim0, C, N, dir, extra, aligned)) return false;
   double best = 0;
-  for (uint32_t cb = 1; cb <= C && cb <= kStreamChannels && (cb * dim0 + 6) / 4 <= kStreamThreads; ++cb) {
+  for (uint32_t cb = 1; cb <= C && cb <= kStreamChannels && (cb * dim0 + 6) / 4 <= kStreamThreads; cb = next_unit(cb, 1)) {
     const uint32_t L4 = (cb * dim0 + 6) / 4;
     if (cb * dim0 < 16 && cb < C) continue;
     uint32_t groups = kStreamThreads / L4;
