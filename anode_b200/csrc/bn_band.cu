@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
           }
           return q;
         };
-        auto one = [&](const Quad &e, const Quad &z, const Quad &old) {
+        auto one = [&](const Quad &e, const Quad &z, [[maybe_unused]] const Quad &old) {
           Quad o;
           o.a = fma2(scale.a, z.a, fma2(cB.a, e.a, cC.a)); o.b = fma2(scale.b, z.b, fma2(cB.b, e.b, cC.b));
           if (there()) {
@@ -323,19 +323,33 @@ __global__ void __launch_bounds__(kBandThreads, 1) bn_band_kernel(const FusedArg
           next();
         };
         uint32_t i = 0;
-        Quad o0 = olds(0), o1 = olds(1), o2 = olds(2), o3 = olds(3);
-        for (; i + 2 <= g.vpt; i += 2, tm += 16) {
-          Quad e0, z0, e1, z1;
-          tmem_ld(tm, e0, z0, e1, z1);
-          const Quad n0 = olds(i + 4), n1 = olds(i + 5);
-          one(e0, z0, o0); one(e1, z1, o1);
-          o0 = o2; o1 = o3; o2 = n0; o3 = n1;
-          __syncwarp();
-        }
-        if (i < g.vpt) {
-          Quad e0, z0;
-          tmem_ld(tm, e0, z0);
-          one(e0, z0, o0);
+        if constexpr (ADDS) {
+          Quad o0 = olds(0), o1 = olds(1), o2 = olds(2), o3 = olds(3);
+          for (; i + 2 <= g.vpt; i += 2, tm += 16) {
+            Quad e0, z0, e1, z1;
+            tmem_ld(tm, e0, z0, e1, z1);
+            const Quad n0 = olds(i + 4), n1 = olds(i + 5);
+            one(e0, z0, o0); one(e1, z1, o1);
+            o0 = o2; o1 = o3; o2 = n0; o3 = n1;
+            __syncwarp();
+          }
+          if (i < g.vpt) {
+            Quad e0, z0;
+            tmem_ld(tm, e0, z0);
+            one(e0, z0, o0);
+          }
+        } else {
+          for (; i + 2 <= g.vpt; i += 2, tm += 16) {
+            Quad e0, z0, e1, z1;
+            tmem_ld(tm, e0, z0, e1, z1);
+            one(e0, z0, e0); one(e1, z1, e1);
+            __syncwarp();
+          }
+          if (i < g.vpt) {
+            Quad e0, z0;
+            tmem_ld(tm, e0, z0);
+            one(e0, z0, e0);
+          }
         }
       }
       __syncwarp();
