@@ -593,13 +593,14 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
 //    22.9, 34.9, 34.8, 61.1 and 15.8, 22.6, 19.6, 30.1, [356,2022,25] 59, 84, 85, 157 and 35, 56, 46, 80; but [67,706,37], 1.75 M, 5.2, 8.1, 7.6,
 //    15.7 and 6.6, 8.9, 8.4, 10.2, [802,67,19], 1.0 M, 4.5, 5.5, 5.0, 7.2 and 6.6, 8.1, 7.8, 9.3, and few samples, [16,2017,151] 17.5, 22.2,
 //    22.6, 39.7 and 22.4, 23.8, 25.1, 32.9.  Aligned runs: [188,356,39], 2.6 M, 11.5, 11.1, 14.8, 31.7 and 6.3, 9.1, 8.3, 12.0, [2604,86,14]
-//    12.8, 16.3, 19.4, 36.0 and 11.0, 15.0, 13.2, 21.1, but [2311,68,14], 2.2 M, 6.7, 9.8, 10.6, 20.6 and 8.4, 10.1, 9.6, 13.2;
+//    12.8, 16.3, 19.4, 36.0 and 11.0, 15.0, 13.2, 21.1, but [2311,68,14], 2.2 M, 6.7, 9.8, 10.6, 20.6 and 8.4, 10.1, 9.6,
+//    13.2, and forward [30,298,258], 2.3 M, 7.3 and 7.9;
 //  - the tiled kernel, which copies a row at a time, masked, on rows below 200 floats: [604,18,221] 16.4, 20.5, 18.5, 25.6 and 9.3, 11.7,
 //    10.6, 14.8, [1826,159,179] 128, 246, 213, - and 118, 186, 153, -, [1403,355,131] forward 191 and 143; but [1594,54,227] 54, 81, 77, 101 and
 //    58, 80, 69, 107; on longer ones in small layers, where the tiled kernel's launch costs ten us: [947,13,350] 19.5, 25.0, 22.6, 27.5 and 13.3,
 //    22.7, 20.1, 30.6, but [2147,15,254], 8.2 M, 27.5, 42.0, 39.0, 49.4 and 29.2, 46.1, 42.6, 63.5.
 constexpr uint32_t kMaskedSamples = 20, kMaskedShortRow = 200;
-constexpr uint64_t kMaskedChan[2][2] = {{2300000, 2100000}, {2300000, 1100000}};        // [direction][residual]
+constexpr uint64_t kMaskedChan[2][2] = {{2500000, 2100000}, {2300000, 1100000}};        // [direction][residual]
 constexpr uint64_t kMaskedTiled[2][2] = {{8000000, 5000000}, {4500000, 2500000}};
 static bool masked_takes(const FusedArgs &a, int dir, int kind, StreamGeom &g)
 {
@@ -625,6 +626,7 @@ static bool masked_takes(const FusedArgs &a, int dir, int kind, StreamGeom &g)
 constexpr uint32_t kLongRow = 250, kLongFewChannels = 128, kLongOneWave = 20;
 constexpr uint64_t kLongTiledMost = 12000000;
 constexpr uint64_t kLongManyChannels = 2400000;
+constexpr uint32_t kLongChannelsAligned = 600;      // ([20,558,564] 19.5, 29.4 and 16.4, 28.6, but [11,1404,420] 15.6, 25.6 and 22.5, 28.7)
 constexpr uint64_t kLongChan[2][2] = {{3300000, 1800000}, {1800000, 700000}};           // [direction][residual]
 constexpr uint64_t kLongChannel[2][2] = {{64 << 10, 32 << 10}, {32 << 10, 24 << 10}};
 constexpr uint64_t kLongChanAligned[2][2] = {{~0ull, 3000000}, {~0ull, 2400000}};
@@ -637,7 +639,7 @@ static bool long_takes(const FusedArgs &a, int dir, int kind, LongGeom &g)
     return elements <= kLongTiledMost && long_geom_of(a, dir, g) && g.cost * 1.12f < 12.0f + (float)elements * (dir == 0 ? (extra ? 12 : 8) : extra ? 20 : 12) * 1.6e-7f;
   if (kind != ANODE_KERNEL_REGISTER) return false;
   const uint32_t C = a.plan.C;
-  return (a.plan.dim0 % 4 == 0 ? elements >= kLongChanAligned[dir][extra]
+  return (a.plan.dim0 % 4 == 0 ? elements >= kLongChanAligned[dir][extra] && C <= kLongChannelsAligned
                                : (elements >= kLongChan[dir][extra] && (C <= kLongFewChannels || elements >= kLongManyChannels)) ||
                                      (channel >= kLongChannel[dir][extra] && C <= kLongOneWave)) && long_geom_of(a, dir, g);
 }
