@@ -258,10 +258,11 @@ static bool chan_dense(const ChanGeom &g, uint32_t blocks, uint32_t threads)
 {
   if (g.floats > 8 || blocks < 128) return false;      // (a wave is more than that)
   const uint32_t sms = sm_count(), few = g.floats == 4 ? 48u : 56u;
-  // (the SMs of a cluster lie together: clusters of four fill 94 per cent of the places, of eight 85)
+  // (the SMs of a cluster lie together: clusters of four fill 94 per cent of the places, of eight 90: 256 blocks fit where
+  // 296 would, 288 do not)
   auto places = [&](uint32_t registers) {
     const uint32_t n = 65536 / (registers * threads) * sms;
-    return g.cluster == 8 ? n * 17 / 20 : g.cluster == 4 ? n * 15 / 16 : n;
+    return g.cluster == 8 ? n * 9 / 10 : g.cluster == 4 ? n * 15 / 16 : n;
   };
   return blocks > places(64) && blocks <= places(few);
 }
