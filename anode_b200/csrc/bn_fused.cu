@@ -621,15 +621,17 @@ static bool masked_takes(const FusedArgs &a, int dir, int kind, StreamGeom &g)
 //  - the register-resident kernel on ragged rows, which it loads float by float, from these sizes or channels on: [8,217,2678] 18.5, 29.8,
 //    30.9, 52.6 and 12.7, 16.1, 14.5, 20.6, [2,5,19011] 3.8, 5.2, 5.2, 6.9 and 5.1, 4.1, 4.5, 4.6, [9,4,12887] forward 8.1 and 5.5, but
 //    [10,119,1502], 1.8 M, 5.4, 8.5, 8.0 and 7.9, 10.0, 9.8, and where the clusters take a second wave, [71,25,577] backward 7.1 and 8.9,
-//    [3,1023,366] residual backward 8.0 and 11.3; and on aligned ones in the residual epilogue: [6,276,2060], 3.4 M, 11.7, 16.9 and 10.8,
-//    15.7, [7,331,1108], 2.6 M, backward 12.9 and 10.5.
+//    [3,1023,366] residual backward 8.0 and 11.3; and on aligned ones in the residual epilogue, where one block or two hold a channel: [35,183,1292],
+//    8.3 M, 28.3, 40.8 and 23.6, 35.8, [82,110,440], 4.0 M, 14.8, 21.1 and 13.6, 18.5, [7,331,1108], 2.6 M, backward 12.9 and 10.5; but forward
+//    [12,316,1032], 3.9 M, 13.2 and 15.2, [18,380,464], 3.2 M, 10.5 and 12.0, and more channels, [2,512,4096] 10.8, 16.0 and 11.4, 19.4, [11,1404,420]
+//    15.6, 25.6 and 22.5, 28.7.
 constexpr uint32_t kLongRow = 250, kLongFewChannels = 128, kLongOneWave = 20;
 constexpr uint64_t kLongTiledMost = 12000000;
 constexpr uint64_t kLongManyChannels = 2400000;
-constexpr uint32_t kLongChannelsAligned = 600;      // ([20,558,564] 19.5, 29.4 and 16.4, 28.6, but [11,1404,420] 15.6, 25.6 and 22.5, 28.7)
+constexpr uint32_t kLongChannelsAligned = 450;
 constexpr uint64_t kLongChan[2][2] = {{3300000, 1800000}, {1800000, 700000}};           // [direction][residual]
 constexpr uint64_t kLongChannel[2][2] = {{64 << 10, 32 << 10}, {32 << 10, 24 << 10}};
-constexpr uint64_t kLongChanAligned[2][2] = {{~0ull, 3000000}, {~0ull, 2400000}};
+constexpr uint64_t kLongChanAligned[2][2] = {{~0ull, 3950000}, {~0ull, 2400000}};
 static bool long_takes(const FusedArgs &a, int dir, int kind, LongGeom &g)
 {
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
