@@ -103,6 +103,7 @@ SIGNATURES = {
     "anode_gpu_batch_norm_tiled_keep": (c_int, _D + [c_int, c_int, u32, u32, ctypes.POINTER(u32)]),
     "anode_gpu_batch_norm_tiled_last_piece": (u32, _D + [c_int, c_int]),
     "anode_gpu_batch_norm_fused_serving_kernel": (c_int, _D + [c_int] * 4),
+    "anode_gpu_batch_norm_fused_launched_kernel": (c_int, _D + [c_int] * 3),
     "anode_gpu_batch_norm_fused_last_kernel": (c_int, []),
     "anode_gpu_batch_norm_fused_kernel_kind": (c_int, _D + [c_int]),
     "anode_gpu_batch_norm_add_act_fused_kernel_kind": (c_int, _D + [c_int]),

@@ -646,18 +646,26 @@ static bool long_takes(const FusedArgs &a, int dir, int kind, LongGeom &g)
                                      (channel >= kLongChannel[dir][extra] && C <= kLongOneWave)) && long_geom_of(a, dir, g);
 }
 
-// Launches the one of those two that takes the call, if any.
-static int launch_instead(FusedArgs &a, int dir, int kind, bool aligned, cudaStream_t stream)
+// Which of those two takes the call from `kind`: STREAM, LONG (and its geometry), or -1.  Where both do, the one of the smaller estimate.
+static int pick_instead(const FusedArgs &a, int dir, int kind, bool aligned, LongGeom &lg)
 {
   if (!aligned || a.mode != MODE_FUSED || a.world > 1 ||
       (kind != ANODE_KERNEL_REGISTER && kind != ANODE_KERNEL_TILED && kind != ANODE_KERNEL_PLAIN)) return -1;
-  StreamGeom sg; LongGeom lg;
   const int choice = kernel_choice();
-  bool masked = choice == ANODE_KERNEL_AUTO && masked_takes(a, dir, kind, sg);
-  bool rows = choice == ANODE_KERNEL_AUTO ? long_takes(a, dir, kind, lg) : choice == ANODE_KERNEL_LONG && long_geom_of(a, dir, lg);
-  if (masked && rows) (lg.cost < sg.cost ? masked : rows) = false;
-  if (masked && launch_stream(a, dir, stream) == ANODE_OK) return ANODE_KERNEL_STREAM;
-  if (rows && launch_long(a, lg, dir, stream) == ANODE_OK) return ANODE_KERNEL_LONG;
+  if (choice != ANODE_KERNEL_AUTO) return choice == ANODE_KERNEL_LONG && long_geom_of(a, dir, lg) ? ANODE_KERNEL_LONG : -1;
+  StreamGeom sg;
+  const bool masked = masked_takes(a, dir, kind, sg), rows = long_takes(a, dir, kind, lg);
+  if (masked && rows) return lg.cost < sg.cost ? ANODE_KERNEL_LONG : ANODE_KERNEL_STREAM;
+  return masked ? ANODE_KERNEL_STREAM : rows ? ANODE_KERNEL_LONG : -1;
+}
+
+// Launches it; -1 where there is none, or the device refuses its clusters.
+static int launch_instead(FusedArgs &a, int dir, int kind, bool aligned, cudaStream_t stream)
+{
+  LongGeom lg;
+  const int k = pick_instead(a, dir, kind, aligned, lg);
+  if (k == ANODE_KERNEL_STREAM && launch_stream(a, dir, stream) == ANODE_OK) return k;
+  if (k == ANODE_KERNEL_LONG && launch_long(a, lg, dir, stream) == ANODE_OK) return k;
   return -1;
 }
 
@@ -982,6 +990,17 @@ extern "C" int anode_gpu_batch_norm_fused_serving_kernel(uint32_t dim0, uint32_t
   if (check_dims(dim0, dim1, dim2) || (dir != 0 && dir != 1)) return ANODE_E_DIMS;
   const int k = pick_kernel_kind(probe_call(dim0, dim1, dim2, dir, residual != 0, aligned != 0, world), dir, aligned != 0);
   return k < 0 ? ANODE_KERNEL_AUTO : k;
+}
+
+extern "C" int anode_gpu_batch_norm_fused_launched_kernel(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual, int aligned)
+{
+  if (check_dims(dim0, dim1, dim2) || (dir != 0 && dir != 1)) return ANODE_E_DIMS;
+  const FusedArgs a = probe_call(dim0, dim1, dim2, dir, residual != 0, aligned != 0, 1);
+  const int kind = pick_kernel_kind(a, dir, aligned != 0);
+  LongGeom lg; BandGeom bg;
+  const int instead = pick_instead(a, dir, kind, aligned != 0, lg);
+  if (instead >= 0) return instead;
+  return kind == ANODE_KERNEL_STREAM && kernel_choice() != ANODE_KERNEL_STREAM && band_geom_of(a, dir, bg) ? ANODE_KERNEL_BAND : kind;
 }
 
 extern "C" int anode_gpu_batch_norm_fused_last_kernel(void) { return t_last_kernel; }

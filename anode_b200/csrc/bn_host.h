@@ -21,7 +21,7 @@ struct StreamGeom {
   uint32_t cb, units;        // channels per unit
   uint32_t cluster, rows;    // blocks per unit, samples per block
   uint32_t groups, threads;  // sample groups of a block: thread = group * vectors per run + vector
-  float cost;                // masked form: estimated us
+  float cost;                // estimated us (of a prepared call's geometry)
   double inv_count;
 };
 

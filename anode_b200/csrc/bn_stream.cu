@@ -413,6 +413,12 @@ static void stream_set(StreamGeom &g, uint32_t C, uint32_t N, uint32_t cb, uint3
   g.threads = (g.groups * L4 + 31) / 32 * 32;
 }
 
+// What runs of aligned channels take of that estimate: 0.83, 0.70, 0.73 and 0.82 (forward, residual forward, backward, residual backward;
+// medians over 37 to 57 shapes of 250 to 510 floats a row, which the kernel for long rows serves, too).  The smaller estimate of the two is
+// launched: residual forward, backward and residual backward are 0.5, 2 and 0.7 per cent above the better one on average, always this kernel
+// would be 12, 20 and 11.  (Without the factor [99,58,506] residual forward went to long rows, 15.4 us and here 12.1.)
+constexpr double kStreamAligned = 0.72;
+
 // The geometry that is launched: stream_geom's, or the one of the least estimated time where that is this much less.  Us so and with
 // stream_geom's alone, forward, backward, residual forward and backward: [3865,36,18] 8.9, 11.7, 10.7, 15.4 and 11.0, 17.4, 16.9, 23.3, [1148,44,80]
 // 9.4, 14.6, 11.7, 19.3 and 13.4, 21.2, 18.0, 25.6, [20,1998,102] 9.7, 13.8, 11.4, 18.7 and 14.0, 16.6, 16.6, 19.6, [148,750,38] 9.4, 15.1, 12.6, 20.4 and
@@ -422,13 +428,15 @@ bool stream_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, Str
 {
   if (!stream_geom(dim0, C, N, dir, extra, g)) return false;
   const uint32_t q = dim0 % 4 == 0 ? 1 : dim0 % 2 == 0 ? 2 : 4;
-  double best = kStreamOther * stream_cost(dim0, C, N, dir, extra, false, g.cb, g.cluster, g.groups, g.cb * dim0 / 4);
+  const double first = stream_cost(dim0, C, N, dir, extra, false, g.cb, g.cluster, g.groups, g.cb * dim0 / 4);
+  double best = kStreamOther * first;
+  g.cost = (float)(kStreamAligned * first);
   for (uint32_t cb = q; cb <= C && cb <= kStreamChannels && cb * dim0 <= 4 * kStreamThreads; cb = next_unit(cb, q)) {
     const uint32_t L4 = cb * dim0 / 4, groups = kStreamThreads / L4 < N ? kStreamThreads / L4 : N;
     if (cb * dim0 < 32 && cb + q <= C) continue;
     for (uint32_t cl = 1; cl <= 16 && cl * cb <= kStreamRecords && (cl == 1 || N / cl >= groups * 2); cl *= 2) {
       const double cost = stream_cost(dim0, C, N, dir, extra, false, cb, cl, groups, L4);
-      if (cost < best) { best = cost; stream_set(g, C, N, cb, cl, groups, L4); }
+      if (cost < best) { best = cost; g.cost = (float)(kStreamAligned * cost); stream_set(g, C, N, cb, cl, groups, L4); }
     }
   }
   return true;

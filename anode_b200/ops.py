@@ -333,8 +333,8 @@ def set_kernel(name):
 
 
 def serving_kernel(shape, dir, residual=False, aligned=True, world=1):
-    """Name, in KERNELS, of the kernel that a fused call on a [N, C, *spatial] shape launches, or whose place one of its
-    counterparts takes (anode_gpu_batch_norm_fused_serving_kernel); None where a synchronized call takes three."""
+    """Name, in KERNELS, of the kernel that serves a fused call on a [N, C, *spatial] shape; one of its counterparts may be launched in
+    its place, see launched_kernel (anode_gpu_batch_norm_fused_serving_kernel); None where a synchronized call takes three."""
     d0 = 1
     for s in shape[2:]:
         d0 *= int(s)
@@ -342,6 +342,17 @@ def serving_kernel(shape, dir, residual=False, aligned=True, world=1):
     if k < 0:
         raise AnodeError(k, "anode_gpu_batch_norm_fused_serving_kernel")
     return {v: n for n, v in KERNELS.items()}[k] if k else None
+
+
+def launched_kernel(shape, dir, residual=False, aligned=True):
+    """Name, in KERNELS or FORMS, of the kernel that a fused call on one GPU launches (anode_gpu_batch_norm_fused_launched_kernel)."""
+    d0 = 1
+    for s in shape[2:]:
+        d0 *= int(s)
+    k = _lib.load().anode_gpu_batch_norm_fused_launched_kernel(d0, int(shape[1]), int(shape[0]), dir, int(residual), int(aligned))
+    if k < 0:
+        raise AnodeError(k, "anode_gpu_batch_norm_fused_launched_kernel")
+    return {v: n for n, v in {**KERNELS, **FORMS}.items()}[k]
 
 
 def last_kernel():

@@ -198,8 +198,9 @@ void anode_gpu_positive_clip_flat_map_bwd_f32(
  *             REGISTER where it is the faster one.  Queries by shape name those.
  * anode_gpu_batch_norm_fused_set_kernel makes another choice process-wide: that kernel is used wherever it
  * applies, elsewhere one of the first four by the shape.  Meant for tests and measurements; which kernel a
- * call launches is answered by anode_gpu_batch_norm_fused_serving_kernel, which one the last call launched by
- * anode_gpu_batch_norm_fused_last_kernel (anode_routines_gpu_diag.h). */
+ * call is served by is answered by anode_gpu_batch_norm_fused_serving_kernel, which one it launches by
+ * anode_gpu_batch_norm_fused_launched_kernel, which one the last call launched by anode_gpu_batch_norm_fused_last_kernel
+ * (anode_routines_gpu_diag.h). */
 #define ANODE_KERNEL_AUTO      0
 #define ANODE_KERNEL_TILED     1
 #define ANODE_KERNEL_CLUSTER   2

@@ -12,13 +12,17 @@
 extern "C" {
 #endif
 
-/* Kernel that direction `dir` (0 forward, 1 backward) of a fused call launches, with a workspace of the full size:
- * an ANODE_KERNEL_* value of anode_routines_gpu.h.  residual: the residual-epilogue calls; aligned: every tensor on a
+/* Kernel that serves direction `dir` (0 forward, 1 backward) of a fused call, with a workspace of the full size: an ANODE_KERNEL_*
+ * value of anode_routines_gpu.h.  STREAM and LONG may be launched in the place of PLAIN, REGISTER or TILED, and BAND in the place of
+ * STREAM; anode_gpu_batch_norm_fused_launched_kernel tells.  residual: the residual-epilogue calls; aligned: every tensor on a
  * 16-byte boundary; world: ranks of a synchronized call whose communicator has an exchange buffer (1: a call on one
  * GPU).  ANODE_KERNEL_AUTO (0): a synchronized call that no kernel with the exchange inside serves (a reduce, an
  * exchange and an apply kernel are launched). */
 int anode_gpu_batch_norm_fused_serving_kernel(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual,
                                               int aligned, int world);
+
+/* Kernel that such a call on one GPU launches first; another one only where the device refuses its clusters. */
+int anode_gpu_batch_norm_fused_launched_kernel(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual, int aligned);
 
 /* ANODE_KERNEL_* value of the kernel that this thread's last fused call launched, in one launch or with the exchange apart, BAND and
  * STREAM told apart; -1 before the first one. */
@@ -26,7 +30,7 @@ int anode_gpu_batch_norm_fused_last_kernel(void);
 
 /* Family, among the first four ANODE_KERNEL_* values, that the shape of a plain fused call on 16-byte aligned tensors
  * belongs to.  (The REGISTER and STREAM kernels and the TILED kernel's ragged rows count as the family whose shapes they
- * take over on one GPU; for the kernel that is launched ask anode_gpu_batch_norm_fused_serving_kernel.) */
+ * take over on one GPU; for the kernel that is launched ask anode_gpu_batch_norm_fused_launched_kernel.) */
 int anode_gpu_batch_norm_fused_kernel_kind(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir);
 
 /* The same for the residual-epilogue calls (anode_gpu_batch_norm_add_act_fused_*). */
