@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(kLongThreads, kLongBlocks) bn_long_kernel(cons
 bool long_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, LongGeom &g)
 {
   if (dim0 < 16 || C > 0xfffffu) return false;
-  g.per_row = dim0 % 4 ? (dim0 + 6) / 4 : dim0 / 4;
+  g.per_row = dim0 % 4 ? (uint32_t)((dim0 + 6ull) / 4) : dim0 / 4;
   const uint64_t total = (uint64_t)g.per_row * N;
   if (total > 0x3fffffffu) return false;
   g.total = (uint32_t)total;

@@ -452,7 +452,7 @@ bool masked_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, Str
   StreamGeom aligned;
   if (dim0 < 4 || stream_geom(dim0, C, N, dir, extra, aligned)) return false;
   double best = 0;
-  for (uint32_t cb = 1; cb <= C && cb <= kStreamChannels && (cb * dim0 + 6) / 4 <= kStreamThreads; cb = next_unit(cb, 1)) {
+  for (uint32_t cb = 1; cb <= C && cb <= kStreamChannels && ((uint64_t)cb * dim0 + 6) / 4 <= kStreamThreads; cb = next_unit(cb, 1)) {
     const uint32_t L4 = (cb * dim0 + 6) / 4;
     if (cb * dim0 < 16 && cb < C) continue;
     uint32_t groups = kStreamThreads / L4;
