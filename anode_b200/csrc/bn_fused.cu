@@ -586,46 +586,66 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
   return resident_applies(a, dir, aligned) ? ANODE_KERNEL_RESIDENT : -1;
 }
 
+// Us of the kernels that the two below take calls from.  The tiled kernel: its launch and agreement, the layer's bytes, and of ragged rows a
+// copy for each and tensor; seven per cent off over 968 passes of 0.2 to 46 M elements, from memory.  The plain kernel: its agreement, 1.75 to
+// 2 TB/s, and what a row's ends cost; 15 per cent off over 438 passes of 0.4 to 150 M elements.
+static float takes_from_us(const FusedArgs &a, int dir, bool extra, int kind)
+{
+  const float rows = (float)a.plan.C * (float)a.plan.N, bytes = 4.0f * rows * (float)a.plan.dim0 * (dir == 0 ? (extra ? 3.0f : 2.0f) : extra ? 5.0f : 3.0f);
+  if (kind == ANODE_KERNEL_PLAIN) return dir == 0 ? 13.0f + bytes * 5.7e-7f + rows * 4e-5f : 10.0f + bytes * 5e-7f + rows * 4e-5f;
+  return 11.0f + bytes * 1.35e-7f + (a.plan.dim0 % 4 == 0 ? 0.0f : rows * (dir == 1 ? 5e-4f : extra ? 4.3e-4f : 2.2e-4f));
+}
+
 // Odd rows, on one GPU: where the streaming kernel, or its masked form for rows without an aligned run of channels, is launched in the
 // place of the kernel that pick_kernel_kind names.  Us there and here, forward, backward, residual forward and backward:
-//  - the plain kernel everywhere (masked; figures at the head of bn_stream.cu);
 //  - the register-resident kernel, which loads such rows float by float, from these sizes and twenty samples on.  Masked: [270,490,49]
 //    22.9, 34.9, 34.8, 61.1 and 15.8, 22.6, 19.6, 30.1, [356,2022,25] 59, 84, 85, 157 and 35, 56, 46, 80; but [67,706,37], 1.75 M, 5.2, 8.1, 7.6,
 //    15.7 and 6.6, 8.9, 8.4, 10.2, [802,67,19], 1.0 M, 4.5, 5.5, 5.0, 7.2 and 6.6, 8.1, 7.8, 9.3, and few samples, [16,2017,151] 17.5, 22.2,
 //    22.6, 39.7 and 22.4, 23.8, 25.1, 32.9.  Aligned runs: [188,356,39], 2.6 M, 11.5, 11.1, 14.8, 31.7 and 6.3, 9.1, 8.3, 12.0, [2604,86,14]
 //    12.8, 16.3, 19.4, 36.0 and 11.0, 15.0, 13.2, 21.1, but [2311,68,14], 2.2 M, 6.7, 9.8, 10.6, 20.6 and 8.4, 10.1, 9.6,
 //    13.2, and forward [30,298,258], 2.3 M, 7.3 and 7.9;
-//  - the tiled kernel, which copies a row at a time, masked, on rows below 200 floats: [604,18,221] 16.4, 20.5, 18.5, 25.6 and 9.3, 11.7,
-//    10.6, 14.8, [1826,159,179] 128, 246, 213, - and 118, 186, 153, -, [1403,355,131] forward 191 and 143; but [1594,54,227] 54, 81, 77, 101 and
-//    58, 80, 69, 107; on longer ones in small layers, where the tiled kernel's launch costs ten us: [947,13,350] 19.5, 25.0, 22.6, 27.5 and 13.3,
-//    22.7, 20.1, 30.6, but [2147,15,254], 8.2 M, 27.5, 42.0, 39.0, 49.4 and 29.2, 46.1, 42.6, 63.5.
+//  - the plain and the tiled kernel (which copies a row at a time), masked, where its estimate with these margins is below theirs
+//    (takes_from_us): clusters of few channels leave the device empty and walk their samples for long.  Plain: figures at the head of
+//    bn_stream.cu, but [97106,1,81] forward 57 and 144, [93078,1,146] backward 92 and 575, [130265,1,47] residual forward 61 and 254,
+//    [154066,1,113] residual backward 151 and 972; of 438 such passes 306 are taken, 0.62 of the time, eight of them slower by more than a
+//    twentieth, and what is left out would take 1.83 times as long here.  Tiled: [604,18,221] 16.4, 20.5, 18.5, 25.6 and 9.3, 11.7, 10.6, 14.8,
+//    [1826,159,179] 128, 246, 213, - and 118, 186, 153, -, [1403,355,131] forward 191 and 143, [947,13,350] forward 19.5 and 13.3, residual forward 22.6
+//    and 20.1; but [110600,1,165] forward 63 and 496, [2705,2,818] backward 21.9 and 96.9, residual forward 17.9 and 88.1.  On rows of 200 floats and
+//    more only in small layers, where the tiled kernel's launch costs ten us: [1594,54,227] 54, 81, 77, 101 and 58, 80, 69, 107, [2147,15,254], 8.2 M, 27.5,
+//    42.0, 39.0, 49.4 and 29.2, 46.1, 42.6, 63.5.
 constexpr uint32_t kMaskedSamples = 20, kMaskedShortRow = 200;
 constexpr uint64_t kMaskedChan[2][2] = {{2500000, 2100000}, {2300000, 1100000}};        // [direction][residual]
 constexpr uint64_t kMaskedTiled[2][2] = {{8000000, 5000000}, {4500000, 2500000}};
+constexpr float kMaskedMargin[2][2] = {{1.3f, 1.1f}, {1.15f, 1.1f}};
 static bool masked_takes(const FusedArgs &a, int dir, int kind, StreamGeom &g)
 {
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
   const uint64_t elements = (uint64_t)a.plan.dim0 * a.plan.C * a.plan.N;
   if (a.plan.dim0 % 4 == 0) return false;
-  if (kind == ANODE_KERNEL_REGISTER && (a.plan.N < kMaskedSamples || elements < kMaskedChan[dir][extra])) return false;
+  if (kind == ANODE_KERNEL_REGISTER)
+    return a.plan.N >= kMaskedSamples && elements >= kMaskedChan[dir][extra] && (stream_geom_of(a, dir, g) || masked_geom_of(a, dir, g));
   if (kind == ANODE_KERNEL_TILED && a.plan.dim0 >= kMaskedShortRow && (a.plan.N < kMaskedSamples || elements > kMaskedTiled[dir][extra])) return false;
-  return (kind == ANODE_KERNEL_REGISTER && stream_geom_of(a, dir, g)) || masked_geom_of(a, dir, g);
+  return masked_geom_of(a, dir, g) && g.cost * kMaskedMargin[dir][extra] < takes_from_us(a, dir, extra, kind);
 }
 
 // Rows of 250 floats and more, on one GPU: where the kernel for long rows (bn_long.cu) is launched in the place of the one that
 // pick_kernel_kind names.  Us there and here, forward, backward, residual forward and backward:
-//  - the tiled kernel where its launch (twelve us and the layer's bytes) is more than the estimate of the other: [1,3,64,64,64] 12.5,
-//    12.4, -, - and 6.0, 7.9, -, -, [1,11,99716] -, 13.8, 13.2, 13.0 and -, 7.2, 6.7, 9.2, [3,19,75580], 4.3 M, 16.6, 18.0, 17.7, 26.4 and 10.3, 15.2,
-//    15.1, 19.4; but [1,4,1630016], 6.5 M, 19.4, 25.2, 22.3, 31.8 and 28.6, 47.6, 47.3, 58.0.  By that rule (and no margin) 0.8 per cent are lost
-//    against the better of the two over 439 passes of 0.3 to 20 M elements;
+//  - the tiled kernel where its time (takes_from_us) is a tenth more than the estimate of the other (of aligned rows' residual backward, which
+//    the estimate has a little high, a twentieth less): [1,3,64,64,64] 12.5, 12.4, -, - and 6.0, 7.9, -, -, [1,11,99716] -, 13.8, 13.2, 13.0 and
+//    -, 7.2, 6.7, 9.2; but [1,4,1630016], 6.5 M, 19.4, 25.2, 22.3, 31.8 and 28.6, 47.6, 47.3, 58.0, [392,12,1225] 20.2, -, 19.7, - and 22.3, -,
+//    27.7, -, [151,64,1098] forward 26.2 and 31.7, [972,11,365] backward 19.9 and 25.2.  Of 866 passes 634 are taken, 0.75 of the time, 15 of
+//    them slower by more than a twentieth, and what is left out would take 1.05 times as long here;
 //  - the register-resident kernel on ragged rows, which it loads float by float, from these sizes or channels on: [8,217,2678] 18.5, 29.8,
 //    30.9, 52.6 and 12.7, 16.1, 14.5, 20.6, [2,5,19011] 3.8, 5.2, 5.2, 6.9 and 5.1, 4.1, 4.5, 4.6, [9,4,12887] forward 8.1 and 5.5, but
 //    [10,119,1502], 1.8 M, 5.4, 8.5, 8.0 and 7.9, 10.0, 9.8, and where the clusters take a second wave, [71,25,577] backward 7.1 and 8.9,
-//    [3,1023,366] residual backward 8.0 and 11.3; and on aligned ones in the residual epilogue, where one block or two hold a channel: [35,183,1292],
-//    8.3 M, 28.3, 40.8 and 23.6, 35.8, [82,110,440], 4.0 M, 14.8, 21.1 and 13.6, 18.5, [7,331,1108], 2.6 M, backward 12.9 and 10.5; but forward
-//    [12,316,1032], 3.9 M, 13.2 and 15.2, [18,380,464], 3.2 M, 10.5 and 12.0, and more channels, [2,512,4096] 10.8, 16.0 and 11.4, 19.4, [11,1404,420]
+//    [3,1023,366] residual backward 8.0 and 11.3; in three waves and more what each block walks has to make up for them (kLongManyWaves),
+//    [4,2048,435] 12.4, 16.1, 16.4 and 27.4, 21.6, 24.8, [1,1024,8190] forward 24.6 and 26.4, but [1,923,8710] 28.3 and 25.9;
+//  - and the same on aligned ones in the residual epilogue, where one block or two hold a channel: [35,183,1292], 8.3 M, 28.3, 40.8 and
+//    23.6, 35.8, [82,110,440], 4.0 M, 14.8, 21.1 and 13.6, 18.5, [7,331,1108], 2.6 M, backward 12.9 and 10.5; but forward [12,316,1032],
+//    3.9 M, 13.2 and 15.2, [18,380,464], 3.2 M, 10.5 and 12.0, and more channels, [2,512,4096] 10.8, 16.0 and 11.4, 19.4, [11,1404,420]
 //    15.6, 25.6 and 22.5, 28.7.
 constexpr uint32_t kLongRow = 250, kLongFewChannels = 128, kLongOneWave = 20;
+constexpr uint64_t kLongManyWaves[2][2] = {{8500, 4000}, {2000, 0}};                   // floats of a channel: [direction][residual]
 constexpr uint64_t kLongTiledMost = 12000000;
 constexpr uint64_t kLongManyChannels = 2400000;
 constexpr uint32_t kLongChannelsAligned = 450;
@@ -638,9 +658,10 @@ static bool long_takes(const FusedArgs &a, int dir, int kind, LongGeom &g)
   const uint64_t channel = (uint64_t)a.plan.dim0 * a.plan.N, elements = channel * a.plan.C;
   if (a.plan.dim0 < kLongRow) return false;
   if (kind == ANODE_KERNEL_TILED)
-    return elements <= kLongTiledMost && long_geom_of(a, dir, g) && g.cost * 1.12f < 12.0f + (float)elements * (dir == 0 ? (extra ? 12 : 8) : extra ? 20 : 12) * 1.6e-7f;
+    return elements <= kLongTiledMost && long_geom_of(a, dir, g) && g.alone * (dir == 1 && extra && a.plan.dim0 % 4 == 0 ? 0.95f : 1.1f) < takes_from_us(a, dir, extra, kind);
   if (kind != ANODE_KERNEL_REGISTER) return false;
   const uint32_t C = a.plan.C;
+  if (a.plan.dim0 % 4 != 0 && C > 2 * kLongBlocks * sm_count() && channel < kLongManyWaves[dir][extra]) return false;
   return (a.plan.dim0 % 4 == 0 ? elements >= kLongChanAligned[dir][extra] && C <= kLongChannelsAligned
                                : (elements >= kLongChan[dir][extra] && (C <= kLongFewChannels || elements >= kLongManyChannels)) ||
                                      (channel >= kLongChannel[dir][extra] && C <= kLongOneWave)) && long_geom_of(a, dir, g);

@@ -25,12 +25,13 @@ struct StreamGeom {
   double inv_count;
 };
 
-// Geometry of its counterpart for long rows (bn_long.cu)
+// Geometry of its counterpart for long rows (bn_long.cu), and its blocks per SM
+constexpr uint32_t kLongBlocks = 3;
 struct LongGeom {
   uint32_t cluster, stride;         // blocks per channel, distance between a thread's vectors
   uint32_t per_row, total;          // vectors per row and per channel
   uint32_t step_rows, step_col;     // a step of `stride` vectors
-  float cost;                       // estimated us
+  float cost, alone;                // estimated us: among clusters and beside the streaming kernel, and beside other kernels
   double inv_count;
 };
 

@@ -13,7 +13,7 @@
 // costs 0.23 us of a thread forward, 0.4 backward, ragged ones 1.6 times that for their place and lanes).  The tiled kernel, which
 // these layers had, is launched cooperatively and agrees over the whole grid, some ten us a launch whatever the size.  Forward /
 // backward, us, there and here: [4,4,42672] 12.9 / 12.4 and 6.0 / 6.7, [1,4,254072] 14.4 / 13.9 and 6.2 / 8.5, [227,8,1116] 16.5 / 14.8 and
-// 7.6 / 10.3, [3,19,75580] 16.6 / 18.0 and 10.3 / 15.2; ragged rows on the register-resident kernel, [8,217,2678] 18.5 / 29.8 and 12.7 / 16.1.
+// 7.6 / 10.3; ragged rows on the register-resident kernel, [8,217,2678] 18.5 / 29.8 and 12.7 / 16.1.
 //
 // Reference kernels this replaces: routines_gpu/batch_norm.cu:24-57, 125-163, 314-336 (forward), :181-206, 240-280,
 // 354-376, 408-444, 476-515 (backward), flat_map.cu:172-194 (ReLU).
@@ -24,7 +24,7 @@
 
 namespace anode_b200 {
 
-constexpr uint32_t kLongThreads = 256, kLongBlocks = 3, kLongCluster = 16;
+constexpr uint32_t kLongThreads = 256, kLongCluster = 16;
 
 template <int DIR, bool EXTRA, bool RAG>
 __global__ void __launch_bounds__(kLongThreads, kLongBlocks) bn_long_kernel(const FusedArgs a, const LongGeom g)
@@ -270,7 +270,9 @@ __global__ void __launch_bounds__(kLongThreads, kLongBlocks) bn_long_kernel(cons
 // ---- host side -------------------------------------------------------------------------------
 
 // The cluster of the least estimated time, as for the streaming kernel's masked form (masked_plan); the figures are fitted to 155 shapes
-// of 0.3 to 23 M elements in four directions, from which the estimate is off by ten per cent on average.
+// of 0.3 to 23 M elements in four directions, from which the estimate is off by ten per cent on average.  `alone` is the estimate where it
+// is held against another kernel's time: ragged vectors take 1.7 times as long, forward 2.1 (fitted to 782 launches from memory and as
+// many from L2, from which it is off by nine per cent; without those factors, by 12 and 13 on ragged rows, and 20 too low).
 bool long_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, LongGeom &g)
 {
   if (dim0 < 16 || C > 0xfffffu) return false;
@@ -281,6 +283,7 @@ bool long_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, LongG
   const uint32_t wave = kLongBlocks * sm_count();
   const double bytes = 4.0 * dim0 * C * N * (dir == 0 ? (extra ? 3 : 2) : extra ? 5 : 3);
   const double each = dir == 0 ? (extra ? 0.32 : 0.225) : 0.41;      // us per vector of a thread
+  const double ragged = dim0 % 4 == 0 ? 1.0 : dir == 0 && !extra ? 2.1 : 1.7;
   double best = 0;
   for (uint32_t cl = 1; cl <= kLongCluster; cl *= 2) {
     const uint64_t blocks = (uint64_t)C * cl, places = cl == 16 ? wave * 25 / 32 : cl == 8 ? wave * 17 / 20 : cl == 4 ? wave * 15 / 16 : wave;
@@ -289,8 +292,11 @@ bool long_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, LongG
     const double over = 4.0 * dim0 * N * (dir == 1 ? 2 : 1) / cl * resident / 77e6 - 1;
     const double again = (dir == 1 ? 0.5 : 0.17) * (over < 0 ? 0 : over > 1 ? 1 : over), lanes = resident / wave;
     const double moved = bytes * (1 + again) / 5.15e6 * (0.9 + 0.1 / lanes), chain = waves * walk * each;
-    const double cost = 0.5 + waves * (2.4 + 0.024 * cl) + pow(pow(moved, 2.5) + pow(chain, 2.5), 0.4);
-    if (best == 0 || cost < best) { best = cost; g.cost = (float)cost; g.cluster = cl; }
+    const double fixed = 0.5 + waves * (2.4 + 0.024 * cl), cost = fixed + pow(pow(moved, 2.5) + pow(chain, 2.5), 0.4);
+    if (best == 0 || cost < best) {
+      best = cost; g.cost = (float)cost; g.cluster = cl;
+      g.alone = (float)(fixed + pow(pow(moved, 2.5) + pow(chain * ragged, 2.5), 0.4));
+    }
   }
   g.stride = g.cluster * kLongThreads;
   g.step_rows = g.stride / g.per_row; g.step_col = g.stride - g.step_rows * g.per_row;
