@@ -96,6 +96,7 @@ SIGNATURES = {
         (c_int, _D + [c_int, u32, u32, u32, u32, u32, ctypes.POINTER(ctypes.c_uint64)]),
     "anode_gpu_batch_norm_segres_geometry": (c_int, _D + [c_int, ctypes.POINTER(u32)]),
     "anode_gpu_batch_norm_stream_geometry": (c_int, _D + [c_int, ctypes.POINTER(u32)]),
+    "anode_gpu_batch_norm_register_form": (c_int, _D + [c_int, c_int, ctypes.POINTER(u32)]),
     "anode_gpu_batch_norm_long_geometry": (c_int, _D + [c_int, c_int, ctypes.POINTER(u32)]),
     "anode_gpu_batch_norm_stream_masked_geometry": (c_int, _D + [c_int, c_int, ctypes.POINTER(u32)]),
     "anode_gpu_batch_norm_band_geometry": (c_int, _D + [c_int, c_int, ctypes.POINTER(u32)]),

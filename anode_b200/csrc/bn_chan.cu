@@ -15,6 +15,8 @@
 //
 // Reference kernels this replaces: routines_gpu/batch_norm.cu:24-57, 125-163, 314-336 (forward), :181-206, 240-280,
 // 354-376, 408-444, 476-515 (backward), flat_map.cu:172-194 (ReLU).
+#include <atomic>
+
 #include "bn_device.cuh"
 #include "bn_host.h"
 
@@ -24,10 +26,9 @@ constexpr uint32_t kChanThreads = 512;       // most threads of a block
 constexpr uint32_t kChanCluster = 8;         // most blocks of a team (the portable cluster size)
 constexpr uint32_t kChanWarpTeams = 4;       // one-warp teams per block
 
-// Threads that two blocks of an SM are compiled for: 64 registers each, or for teams of a few floats a thread 48 or 56, where blocks that
-// do not divide an SM's 1024 threads would leave a second wave (chan_dense).  Us with 64 and so, forward, [225,56,80] 6.4 and 4.3, [3,239,1451]
-// 6.0 and 4.3, [6,278,354] 5.5 and 3.8, residual backward [19,1970,65] 23.4 and 15.6; but with one wave either way backward [451,21,48] 3.6 and
-// 4.3, [108,84,29] 3.6 and 4.3.
+// Threads that two blocks of an SM are compiled for: 64 registers each at most, or for teams of a few floats a thread 48 or 56, where blocks
+// that do not divide an SM's 1024 threads would leave a second wave (chan_dense).  Us with 64 and so, forward, [225,56,80] 6.4 and 4.3,
+// [3,239,1451] 6.0 and 4.3, [6,278,354] 5.5 and 3.8; but with one wave either way backward [451,21,48] 3.6 and 4.3, [108,84,29] 3.6 and 4.3.
 constexpr uint32_t chan_bound(int floats, bool dense) { return !dense ? kChanThreads : floats == 4 ? 640u : 576u; }
 
 struct ChanGeom {
@@ -252,19 +253,55 @@ static ChanKernel chan_kernel_of(const ChanGeom &g, bool dense)
   return g.vec == 4 ? chan_kernel_of<DIR, EXTRA, 4>(g.floats, dense) : chan_kernel_of<DIR, EXTRA, 1>(g.floats, dense);
 }
 
-// Whether the grid is one wave of blocks with fewer registers, and more than one with 64 ([1265,36,9], 36 clusters of eight: forward
-// 6.2 -> 4.3 us, residual forward 6.7 -> 4.7).
-static bool chan_dense(const ChanGeom &g, uint32_t blocks, uint32_t threads)
+static ChanKernel chan_kernel_of(const ChanGeom &g, int dir, bool extra, bool dense)
+{
+  return dir == 0 ? (extra ? chan_kernel_of<0, true>(g, dense) : chan_kernel_of<0, false>(g, dense))
+                  : (extra ? chan_kernel_of<1, true>(g, dense) : chan_kernel_of<1, false>(g, dense));
+}
+
+// Blocks of a form that an SM holds, 0 where the device does not say: asked for once per form and block size.  The register counts are the
+// compiler's: the backward form of four floats in 16-byte loads has 56 without the bound, not 64, and of 48 registers an SM holds 40 warps, not 42.
+static uint32_t chan_resident(const ChanGeom &g, int dir, bool extra, bool dense, uint32_t threads)
+{
+  static std::atomic<uint8_t> kept[2][2][2][2][2][kChanThreads / 32 + 1];      // one more than the answer
+  std::atomic<uint8_t> &k = kept[dir][extra][g.vec == 4][g.floats == 8][dense][threads / 32];
+  uint8_t n = k.load(std::memory_order_relaxed);
+  if (!n) {
+    int blocks = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, chan_kernel_of(g, dir, extra, dense), (int)threads, 0) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return 0;
+    }
+    k.store(n = (uint8_t)(blocks + 1), std::memory_order_relaxed);
+  }
+  return n - 1u;
+}
+
+// Whether the grid is one wave of blocks in the form of fewer registers, and more than one in the other ([1265,36,9], 36 clusters of eight:
+// forward 6.4 and 4.7 us, residual forward 6.9 and 5.1; a twentieth more blocks than fit gain, too, [2,1938,10,14] forward 4.9 and 4.6).  Of 48
+// registers in the place of 56, with one wave either way, backward [16,899,6,6] takes 4.1 and 3.9, [10,912,8,8] 4.0 and 3.9; but residual
+// backward [94,224,4,6] 4.8 and 4.9, [136,469,2,4], from L2, 3.4 and 3.5: there as if the ordinary form had 64.
+static bool chan_dense(const ChanGeom &g, int dir, bool extra, uint32_t blocks, uint32_t threads)
 {
   if (g.floats > 8 || blocks < 128) return false;      // (a wave is more than that)
-  const uint32_t sms = sm_count(), few = g.floats == 4 ? 48u : 56u;
   // (the SMs of a cluster lie together: clusters of four fill 94 per cent of the places, of eight 90: 256 blocks fit where
   // 296 would, 288 do not)
-  auto places = [&](uint32_t registers) {
-    const uint32_t n = 65536 / (registers * threads) * sms;
+  auto places = [&](bool dense) {
+    uint32_t n = chan_resident(g, dir, extra, dense, threads);
+    if (!dense && dir == 1 && extra && n > 1024 / threads) n = 1024 / threads;
+    n *= sm_count();
     return g.cluster == 8 ? n * 9 / 10 : g.cluster == 4 ? n * 15 / 16 : n;
   };
-  return blocks > places(64) && blocks <= places(few);
+  const uint32_t ordinary = places(false);
+  return ordinary && blocks > ordinary && blocks <= places(true) * 21 / 20;
+}
+
+// blocks of the grid and threads of a block
+static void chan_grid(const ChanGeom &g, uint32_t C, uint32_t &blocks, uint32_t &threads)
+{
+  const bool solo = g.threads == 32;
+  blocks = solo ? ceil_div_u32(C, kChanWarpTeams) : C * g.cluster;
+  threads = solo ? 32 * kChanWarpTeams : g.threads;
 }
 
 static bool chan_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, bool aligned, ChanGeom &g)
@@ -399,11 +436,9 @@ int launch_chan(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)
   ChanGeom g;
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;
   if (!chan_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, extra, aligned, g)) return ANODE_E_LAUNCH;
-  const bool solo = g.threads == 32;
-  const uint32_t blocks = solo ? ceil_div_u32(a.plan.C, kChanWarpTeams) : a.plan.C * g.cluster, threads = solo ? 32 * kChanWarpTeams : g.threads;
-  const bool dense = chan_dense(g, blocks, threads);
-  ChanKernel k = dir == 0 ? (extra ? chan_kernel_of<0, true>(g, dense) : chan_kernel_of<0, false>(g, dense))
-                          : (extra ? chan_kernel_of<1, true>(g, dense) : chan_kernel_of<1, false>(g, dense));
+  uint32_t blocks, threads;
+  chan_grid(g, a.plan.C, blocks, threads);
+  ChanKernel k = chan_kernel_of(g, dir, extra, chan_dense(g, dir, extra, blocks, threads));
   if (!k) return ANODE_E_LAUNCH;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
@@ -422,3 +457,20 @@ int launch_chan(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)
 }
 
 }  // namespace anode_b200
+
+// ---- diagnostics: the form launched for a shape, of aligned tensors ------------------------------
+extern "C" int anode_gpu_batch_norm_register_form(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual, uint32_t *out)
+{
+  using namespace anode_b200;
+  if (!out || (dir != 0 && dir != 1) || check_dims(dim0, dim1, dim2)) return ANODE_E_DIMS;
+  for (int i = 0; i < 8; ++i) out[i] = 0;
+  ChanGeom g;
+  const bool extra = residual != 0;
+  if (!chan_geom(dim0, dim1, dim2, dir, extra, true, g)) return ANODE_OK;
+  uint32_t blocks, threads;
+  chan_grid(g, dim1, blocks, threads);
+  out[0] = 1; out[1] = g.floats; out[2] = g.cluster; out[3] = blocks; out[4] = threads;
+  if (g.floats <= 8) for (int dense = 0; dense < 2; ++dense) out[5 + dense] = chan_resident(g, dir, extra, dense != 0, threads);
+  out[7] = chan_dense(g, dir, extra, blocks, threads);
+  return ANODE_OK;
+}

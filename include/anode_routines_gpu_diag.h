@@ -66,6 +66,11 @@ int anode_gpu_batch_norm_stream_masked_geometry(uint32_t dim0, uint32_t dim1, ui
  * vectors, vectors per row and per channel, rows and columns of such a distance. */
 int anode_gpu_batch_norm_long_geometry(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual, uint32_t *out);
 
+/* Launch of the register-resident kernel for a shape of aligned tensors.  out (8 values): applies, floats of a thread, blocks of a
+ * team, blocks of the grid, threads of a block, blocks that an SM holds of the ordinary form and of the one of fewer registers
+ * (teams of four or eight floats a thread; 0 otherwise, and where there is no device), whether the latter is launched. */
+int anode_gpu_batch_norm_register_form(uint32_t dim0, uint32_t dim1, uint32_t dim2, int dir, int residual, uint32_t *out);
+
 /* Geometry of the band kernel, the streaming kernel's form for large layers.  out (16 values): taken by a call with a workspace
  * of the full size (zeros behind a 0: the kernel cannot take the shape at all), channels per unit, units, sample groups of a tile,
  * samples per thread, samples of a tile, tiles per unit, blocks, steps between a tile's two visits, boxes per band, vectors of
