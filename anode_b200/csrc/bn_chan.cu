@@ -49,8 +49,8 @@ __device__ __forceinline__ void st_cluster_f4(void *p, uint32_t rank, float4 v)
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(remote), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 
-// F: floats a thread holds per tensor
-template <int DIR, int VEC, int F, bool EXTRA, bool DENSE>
+// F: floats a thread holds per tensor; ADDS: the output is added to (the forms without it that do so, too: kLate)
+template <int DIR, int VEC, int F, bool EXTRA, bool DENSE, bool ADDS>
 __global__ void __launch_bounds__(chan_bound(F, DENSE), 2) bn_chan_kernel(const FusedArgs a, const ChanGeom g)
 {
   constexpr int E = F / VEC;
@@ -81,7 +81,15 @@ __global__ void __launch_bounds__(chan_bound(F, DENSE), 2) bn_chan_kernel(const 
   else if (owner) { if (a.run_mean) rm = a.run_mean[c]; if (a.run_var) rv = a.run_var[c]; }
   const float slope = a.neg_slope;      // activation: t * (t > 0 ? 1 : slope)
 
+  // Accumulating writes: what they add to is loaded with the inputs where a thread has four floats of it, else brought to L2 with them and
+  // loaded ahead of the first write ([100,300,7,7] 14.6 us where each load waited for the store before it, and 8.9 so; [2,2048,14,108] 22.7
+  // and 19.1).  In forms of their own: assigning calls have nothing of it to check ([16,899,6,6] 3.9 us and 3.8, [108,84,29] 4.2 and 3.7).
+  // Sixteen single floats more would spill, so they are brought to L2 only, and the residual epilogue has three tensors already: there each
+  // load waits (kLate; in forms of their own those are 4 per cent slower, [184,1311,8,8] 79 and 83).
+  constexpr bool kEarly = ADDS && F == 4, kLate = DIR == 1 && (EXTRA || (VEC == 1 && F == 16));
+  static_assert(!ADDS || (DIR == 1 && !kLate), "no such form");
   Pack<VEC> vx[E], ve[(DIR == 1 || EXTRA) ? E : 1];       // ve: dy, later dz (backward) or the residual (forward)
+  Pack<VEC> old[ADDS ? E : 1];
   {
     uint32_t off = off0, col = col0;
     Pack<VEC> vm[(DIR == 1 && EXTRA) ? E : 1];            // the saved output, which carries the mask
@@ -93,7 +101,8 @@ __global__ void __launch_bounds__(chan_bound(F, DENSE), 2) bn_chan_kernel(const 
       if (k < cnt) {
         vx[k] = Pack<VEC>::load(a.x + off);
         if (DIR == 1) ve[k] = Pack<VEC>::load(a.dy + off);
-        if (DIR == 1 && !EXTRA && a.accumulate) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.out + off));      // (added to below)
+        if (kEarly) old[k] = Pack<VEC>::load(a.out + off);
+        else if (ADDS || (kLate && !EXTRA && a.accumulate)) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.out + off));
         if (DIR == 0 && EXTRA) ve[k] = Pack<VEC>::load(a.res + off);
         if (DIR == 1 && EXTRA) vm[k] = Pack<VEC>::load(a.ymask + off);
       }
@@ -195,13 +204,7 @@ __global__ void __launch_bounds__(chan_bound(F, DENSE), 2) bn_chan_kernel(const 
 
   // ---- apply
   uint32_t off = off0, col = col0;
-  // accumulating writes: what they add to was brought to L2 with the inputs and is loaded ahead of the first of them ([100,300,7,7]
-  // 14.6 us where each load waited for the store before it, and 8.9 so; [2,2048,14,108] 22.7 and 19.1)
-  // (sixteen single floats more would spill, and in the residual epilogue, three tensors already, the place for them costs the assigning
-  // form loads in flight: [41,643,136] 17.7 us and 22.5, [82,246,124] 13.8 and 17.1)
-  constexpr bool kAhead = DIR == 1 && !EXTRA && (VEC == 4 || F < 16);
-  Pack<VEC> old[kAhead ? E : 1];
-  if (kAhead && a.accumulate) {
+  if (ADDS && !kEarly) {
     uint32_t at = off0, to = col0;
 #pragma unroll
     for (int k = 0; k < E; ++k) {
@@ -214,7 +217,7 @@ __global__ void __launch_bounds__(chan_bound(F, DENSE), 2) bn_chan_kernel(const 
   for (int k = 0; k < E; ++k) {
     if (k < cnt) {
       Pack<VEC> o;
-      if (DIR == 1 && !kAhead && a.accumulate) old[0] = Pack<VEC>::load(a.out + off);
+      if (kLate && a.accumulate) o = Pack<VEC>::load(a.out + off);
 #pragma unroll
       for (int i = 0; i < VEC; ++i) {
         if (DIR == 0) {
@@ -223,7 +226,7 @@ __global__ void __launch_bounds__(chan_bound(F, DENSE), 2) bn_chan_kernel(const 
           o.v[i] = yb * (yb > 0.0f ? 1.0f : slope);
         } else {
           const float dx = fmaf(scale, ve[k].v[i], fmaf(cB, vx[k].v[i], cC));
-          o.v[i] = a.accumulate ? old[kAhead ? k : 0].v[i] + dx : dx;
+          o.v[i] = ADDS ? old[ADDS ? k : 0].v[i] + dx : kLate && a.accumulate ? o.v[i] + dx : dx;
         }
       }
       o.put(a.out + off);
@@ -238,37 +241,36 @@ __global__ void __launch_bounds__(chan_bound(F, DENSE), 2) bn_chan_kernel(const 
 
 typedef void (*ChanKernel)(const FusedArgs, const ChanGeom);
 
-template <int DIR, bool EXTRA, int VEC>
+template <int DIR, bool EXTRA, bool ADDS, int VEC>
 static ChanKernel chan_kernel_of(uint32_t f, bool dense)
 {
-  if (f == 4) return dense ? bn_chan_kernel<DIR, VEC, 4, EXTRA, true> : bn_chan_kernel<DIR, VEC, 4, EXTRA, false>;
-  if (f == 8) return dense ? bn_chan_kernel<DIR, VEC, 8, EXTRA, true> : bn_chan_kernel<DIR, VEC, 8, EXTRA, false>;
-  if (f == 16) return bn_chan_kernel<DIR, VEC, 16, EXTRA, false>;
-  if constexpr (DIR == 0 && !EXTRA) return bn_chan_kernel<DIR, VEC, 32, EXTRA, false>;
+  if (f == 4) return dense ? bn_chan_kernel<DIR, VEC, 4, EXTRA, true, ADDS> : bn_chan_kernel<DIR, VEC, 4, EXTRA, false, ADDS>;
+  if (f == 8) return dense ? bn_chan_kernel<DIR, VEC, 8, EXTRA, true, ADDS> : bn_chan_kernel<DIR, VEC, 8, EXTRA, false, ADDS>;
+  if (f == 16) return bn_chan_kernel<DIR, VEC, 16, EXTRA, false, ADDS && VEC == 4>;
+  if constexpr (DIR == 0 && !EXTRA) return bn_chan_kernel<DIR, VEC, 32, EXTRA, false, ADDS>;
   return nullptr;
 }
-template <int DIR, bool EXTRA>
+template <int DIR, bool EXTRA, bool ADDS = false>
 static ChanKernel chan_kernel_of(const ChanGeom &g, bool dense)
 {
-  return g.vec == 4 ? chan_kernel_of<DIR, EXTRA, 4>(g.floats, dense) : chan_kernel_of<DIR, EXTRA, 1>(g.floats, dense);
+  return g.vec == 4 ? chan_kernel_of<DIR, EXTRA, ADDS, 4>(g.floats, dense) : chan_kernel_of<DIR, EXTRA, ADDS, 1>(g.floats, dense);
 }
-
-static ChanKernel chan_kernel_of(const ChanGeom &g, int dir, bool extra, bool dense)
+static ChanKernel chan_kernel_of(const ChanGeom &g, int dir, bool extra, bool adds, bool dense)
 {
-  return dir == 0 ? (extra ? chan_kernel_of<0, true>(g, dense) : chan_kernel_of<0, false>(g, dense))
-                  : (extra ? chan_kernel_of<1, true>(g, dense) : chan_kernel_of<1, false>(g, dense));
+  if (dir == 0) return extra ? chan_kernel_of<0, true>(g, dense) : chan_kernel_of<0, false>(g, dense);
+  return extra ? chan_kernel_of<1, true>(g, dense) : adds ? chan_kernel_of<1, false, true>(g, dense) : chan_kernel_of<1, false>(g, dense);
 }
 
 // Blocks of a form that an SM holds, 0 where the device does not say: asked for once per form and block size.  The register counts are the
 // compiler's: the backward form of four floats in 16-byte loads has 56 without the bound, not 64, and of 48 registers an SM holds 40 warps, not 42.
-static uint32_t chan_resident(const ChanGeom &g, int dir, bool extra, bool dense, uint32_t threads)
+static uint32_t chan_resident(const ChanGeom &g, int dir, bool extra, bool adds, bool dense, uint32_t threads)
 {
-  static std::atomic<uint8_t> kept[2][2][2][2][2][kChanThreads / 32 + 1];      // one more than the answer
-  std::atomic<uint8_t> &k = kept[dir][extra][g.vec == 4][g.floats == 8][dense][threads / 32];
+  static std::atomic<uint8_t> kept[2][2][2][2][2][2][kChanThreads / 32 + 1];      // one more than the answer
+  std::atomic<uint8_t> &k = kept[dir][extra][adds][g.vec == 4][g.floats == 8][dense][threads / 32];
   uint8_t n = k.load(std::memory_order_relaxed);
   if (!n) {
     int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, chan_kernel_of(g, dir, extra, dense), (int)threads, 0) != cudaSuccess) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, chan_kernel_of(g, dir, extra, adds, dense), (int)threads, 0) != cudaSuccess) {
       (void)cudaGetLastError();
       return 0;
     }
@@ -281,13 +283,13 @@ static uint32_t chan_resident(const ChanGeom &g, int dir, bool extra, bool dense
 // forward 6.4 and 4.7 us, residual forward 6.9 and 5.1; a twentieth more blocks than fit gain, too, [2,1938,10,14] forward 4.9 and 4.6).  Of 48
 // registers in the place of 56, with one wave either way, backward [16,899,6,6] takes 4.1 and 3.9, [10,912,8,8] 4.0 and 3.9; but residual
 // backward [94,224,4,6] 4.8 and 4.9, [136,469,2,4], from L2, 3.4 and 3.5: there as if the ordinary form had 64.
-static bool chan_dense(const ChanGeom &g, int dir, bool extra, uint32_t blocks, uint32_t threads)
+static bool chan_dense(const ChanGeom &g, int dir, bool extra, bool adds, uint32_t blocks, uint32_t threads)
 {
   if (g.floats > 8 || blocks < 128) return false;      // (a wave is more than that)
   // (the SMs of a cluster lie together: clusters of four fill 94 per cent of the places, of eight 90: 256 blocks fit where
   // 296 would, 288 do not)
   auto places = [&](bool dense) {
-    uint32_t n = chan_resident(g, dir, extra, dense, threads);
+    uint32_t n = chan_resident(g, dir, extra, adds, dense, threads);
     if (!dense && dir == 1 && extra && n > 1024 / threads) n = 1024 / threads;
     n *= sm_count();
     return g.cluster == 8 ? n * 9 / 10 : g.cluster == 4 ? n * 15 / 16 : n;
@@ -438,7 +440,8 @@ int launch_chan(FusedArgs &a, int dir, bool aligned, cudaStream_t stream)
   if (!chan_geom(a.plan.dim0, a.plan.C, a.plan.N, dir, extra, aligned, g)) return ANODE_E_LAUNCH;
   uint32_t blocks, threads;
   chan_grid(g, a.plan.C, blocks, threads);
-  ChanKernel k = chan_kernel_of(g, dir, extra, chan_dense(g, dir, extra, blocks, threads));
+  const bool adds = dir == 1 && a.accumulate;
+  ChanKernel k = chan_kernel_of(g, dir, extra, adds, chan_dense(g, dir, extra, adds, blocks, threads));
   if (!k) return ANODE_E_LAUNCH;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
@@ -470,7 +473,7 @@ extern "C" int anode_gpu_batch_norm_register_form(uint32_t dim0, uint32_t dim1, 
   uint32_t blocks, threads;
   chan_grid(g, dim1, blocks, threads);
   out[0] = 1; out[1] = g.floats; out[2] = g.cluster; out[3] = blocks; out[4] = threads;
-  if (g.floats <= 8) for (int dense = 0; dense < 2; ++dense) out[5 + dense] = chan_resident(g, dir, extra, dense != 0, threads);
-  out[7] = chan_dense(g, dir, extra, blocks, threads);
+  if (g.floats <= 8) for (int dense = 0; dense < 2; ++dense) out[5 + dense] = chan_resident(g, dir, extra, false, dense != 0, threads);
+  out[7] = chan_dense(g, dir, extra, false, blocks, threads);
   return ANODE_OK;
 }
