@@ -29,7 +29,9 @@ constexpr uint64_t kInferCut = 1500000;   // floats of a single sample from whic
 // averages of a training step, the activations of the layer below).
 // N samples, `step` floats apart, of C channels of `len` floats, `row` floats apart (a single sample's rows may be cut into pieces that
 // take the place of samples, see the launch).
-template <int VEC>
+// PLACE: a thread's place from its row, else from its column, as long as nothing is cut ([1,3,5000011], whose threads have one float each, 73.4 us
+// and 70.6; but 16-byte loads, [64,512,7,7] 3.9 and 4.0).
+template <int VEC, bool PLACE>
 __global__ void __launch_bounds__(kInferThreads) bn_infer_kernel(uint32_t len, uint32_t C, uint32_t N, uint32_t row, uint32_t step, float neg_slope,
                                                                  const float *x, const float *mean, const float *var,
                                                                  const float *gamma, const float *beta, float *y)
@@ -42,7 +44,7 @@ __global__ void __launch_bounds__(kInferThreads) bn_infer_kernel(uint32_t len, u
   // this thread's samples: blockIdx.y, + gridDim.y, ...; `left` of the batch from the next one on
   uint32_t left = N - blockIdx.y;
   const size_t down = (size_t)gridDim.y * step;
-  size_t at = (size_t)blockIdx.y * step + (size_t)c * row + off;
+  size_t at = (size_t)blockIdx.y * step + (PLACE ? (size_t)c * row + off : (size_t)col);
   Pack<VEC> p[kInferFlight];
   auto load = [&] {
 #pragma unroll
@@ -97,8 +99,10 @@ extern "C" int anode_gpu_batch_norm_act_infer_3d1_packed_f32(
   if (!x || !y || !mean || !var) return ANODE_E_NULL;
   if (!aligned4(x) || !aligned4(y)) return ANODE_E_ALIGN;
   const bool vec = aligned16(x) && aligned16(y) && (uint64_t)dim1 * dim0 % 4 == 0;
-  // A single sample leaves a thread one load: its rows are cut into pieces, which take the place of samples ([1,515,64,64,64] 227 us, in
-  // four @A@, [1,16,96,96,96] 25.4 and @B@, [1,132,128,128] 4.6 and @C@).  Not small ones, where the launch is the time.
+  // A single sample leaves a thread one load: its rows are cut into pieces, which take the place of samples (us in one piece, and in four,
+  // from memory: [1,515,64,64,64] 236.5 and 157.1, [1,16,96,96,96] 26.9 and 18.6, [1,132,128,128] 6.05 and 4.6, [1,92,128,128] 4.5 and 3.6).
+  // The line is not drawn by measurements: some smaller ones would gain, too, [1,91,128,128] 4.6 and 3.7, [1,256,56,56] 3.7 and 2.9, while
+  // [1,700,31,33], in three, stays at 2.9.
   uint32_t len = dim0, samples = dim2, step = dim1 * dim0;
   if (dim2 == 1 && (uint64_t)dim1 * dim0 >= kInferCut && (!vec || dim0 % 4 == 0)) {
     const uint32_t lanes = vec ? 4u : 1u;
@@ -133,8 +137,8 @@ extern "C" int anode_gpu_batch_norm_act_infer_3d1_packed_f32(
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg_.attrs = attr; cfg_.numAttrs = 1;
-  const cudaError_t e = vec ? cudaLaunchKernelEx(&cfg_, bn_infer_kernel<4>, len, dim1, dim2, dim0, step, neg_slope, x, mean, var, gamma, beta, y)
-                            : cudaLaunchKernelEx(&cfg_, bn_infer_kernel<1>, len, dim1, dim2, dim0, step, neg_slope, x, mean, var, gamma, beta, y);
+  const auto kernel = vec ? bn_infer_kernel<4, true> : len != dim0 ? bn_infer_kernel<1, true> : bn_infer_kernel<1, false>;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg_, kernel, len, dim1, dim2, dim0, step, neg_slope, x, mean, var, gamma, beta, y);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return ANODE_E_LAUNCH; }
   return ANODE_OK;
 }
