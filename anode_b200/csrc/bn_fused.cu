@@ -658,7 +658,7 @@ static bool long_takes(const FusedArgs &a, int dir, int kind, LongGeom &g)
   const uint64_t channel = (uint64_t)a.plan.dim0 * a.plan.N, elements = channel * a.plan.C;
   if (a.plan.dim0 < kLongRow) return false;
   if (kind == ANODE_KERNEL_TILED)
-    return elements <= kLongTiledMost && long_geom_of(a, dir, g) && g.alone * (dir == 1 && extra && a.plan.dim0 % 4 == 0 ? 0.95f : 1.1f) < takes_from_us(a, dir, extra, kind);
+    return elements <= kLongTiledMost && long_geom_of(a, dir, g) && g.cost * (dir == 1 && extra && a.plan.dim0 % 4 == 0 ? 0.95f : 1.1f) < takes_from_us(a, dir, extra, kind);
   if (kind != ANODE_KERNEL_REGISTER) return false;
   const uint32_t C = a.plan.C;
   if (a.plan.dim0 % 4 != 0 && C > 2 * kLongBlocks * sm_count() && channel < kLongManyWaves[dir][extra]) return false;

@@ -31,7 +31,7 @@ struct LongGeom {
   uint32_t cluster, stride;         // blocks per channel, distance between a thread's vectors
   uint32_t per_row, total;          // vectors per row and per channel
   uint32_t step_rows, step_col;     // a step of `stride` vectors
-  float cost, alone;                // estimated us: among clusters and beside the streaming kernel, and beside other kernels
+  float cost;                       // estimated us
   double inv_count;
 };
 

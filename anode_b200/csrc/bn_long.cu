@@ -270,9 +270,9 @@ __global__ void __launch_bounds__(kLongThreads, kLongBlocks) bn_long_kernel(cons
 // ---- host side -------------------------------------------------------------------------------
 
 // The cluster of the least estimated time, as for the streaming kernel's masked form (masked_plan); the figures are fitted to 155 shapes
-// of 0.3 to 23 M elements in four directions, from which the estimate is off by ten per cent on average.  `alone` is the estimate where it
-// is held against another kernel's time: ragged vectors take 1.7 times as long, forward 2.1 (fitted to 782 launches from memory and as
-// many from L2, from which it is off by nine per cent; without those factors, by 12 and 13 on ragged rows, and 20 too low).
+// of 0.3 to 23 M elements in four directions, from which the estimate is off by ten per cent on average.  In the geometry's cost, which is
+// held against other kernels' times, ragged vectors take 1.7 times as long, forward 2.1 (fitted to 782 launches from memory and as many
+// from L2, from which it is off by nine per cent; without those factors, by 12 and 13 on ragged rows, and 20 too low).
 bool long_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, LongGeom &g)
 {
   if (dim0 < 16 || C > 0xfffffu) return false;
@@ -294,8 +294,8 @@ bool long_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, LongG
     const double moved = bytes * (1 + again) / 5.15e6 * (0.9 + 0.1 / lanes), chain = waves * walk * each;
     const double fixed = 0.5 + waves * (2.4 + 0.024 * cl), cost = fixed + pow(pow(moved, 2.5) + pow(chain, 2.5), 0.4);
     if (best == 0 || cost < best) {
-      best = cost; g.cost = (float)cost; g.cluster = cl;
-      g.alone = (float)(fixed + pow(pow(moved, 2.5) + pow(chain * ragged, 2.5), 0.4));
+      best = cost; g.cluster = cl;
+      g.cost = (float)(fixed + pow(pow(moved, 2.5) + pow(chain * ragged, 2.5), 0.4));
     }
   }
   g.stride = g.cluster * kLongThreads;

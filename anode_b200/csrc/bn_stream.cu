@@ -388,14 +388,17 @@ static bool stream_geom(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool ext
 // two runs share come twice, what exceeds L2 between the two walks comes again, and idle threads leave bandwidth unused.  The
 // figures are fitted to 570 launches of the masked form, 60 shapes (16 to 480 floats a row, 3 to 1500 channels, 0.6 to 120 M elements, four
 // directions) with up to 30 units and clusters each: what is chosen by it is 3 per cent above the best of them on average.
-static double stream_cost(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, bool masked, uint32_t cb, uint32_t cl, uint32_t groups, uint32_t L4)
+// (parts: a last wave counts as much of one as it fills.)
+static double stream_cost(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, bool masked, uint32_t cb, uint32_t cl, uint32_t groups, uint32_t L4,
+                          bool parts = false)
 {
   const uint32_t wave = kStreamBlocks * sm_count(), run = cb * dim0, rows = ceil_div_u32(N, cl), used = groups < rows ? groups : rows;
   const double bytes = 4.0 * dim0 * C * N * (dir == 0 ? (extra ? 3 : 2) : extra ? 5 : 3);
   const double sample = (dir == 0 && !extra ? 1.5 : 2.0) / (dir == 0 ? (extra ? 4 : 8) : extra && masked ? 3 : 4);      // us per sample of a thread
   const double window = 77e6, rate = 5.15e6;      // bytes that L2 keeps; bytes per us
   const uint64_t blocks = (uint64_t)ceil_div_u32(C, cb) * cl, places = cl == 16 ? wave * 25 / 32 : cl == 8 ? wave * 17 / 20 : cl == 4 ? wave * 15 / 16 : wave;
-  const double waves = (double)((blocks + places - 1) / places), resident = (double)(blocks < places ? blocks : places);
+  const double waves = parts && blocks > places ? (double)blocks / places : (double)((blocks + places - 1) / places);
+  const double resident = (double)(blocks < places ? blocks : places);
   const double over = 4.0 * run * N * (dir == 1 ? 2 : 1) / cl * resident / window - 1;
   const double again = (dir == 1 ? 0.5 : 0.17) * (over < 0 ? 0 : over > 1 ? 1 : over), lanes = resident * used * L4 / ((double)wave * kStreamThreads);
   const double moved = bytes * (1 + 9.0 / run) * (1 + again) / rate * (0.9 + 0.1 / lanes);
@@ -413,11 +416,12 @@ static void stream_set(StreamGeom &g, uint32_t C, uint32_t N, uint32_t cb, uint3
   g.threads = (g.groups * L4 + 31) / 32 * 32;
 }
 
-// What runs of aligned channels take of that estimate: 0.83, 0.70, 0.73 and 0.82 (forward, residual forward, backward, residual backward;
-// medians over 37 to 57 shapes of 250 to 510 floats a row, which the kernel for long rows serves, too).  The smaller estimate of the two is
-// launched: residual forward, backward and residual backward are 0.5, 2 and 0.7 per cent above the better one on average, always this kernel
-// would be 12, 20 and 11.  (Without the factor [99,58,506] residual forward went to long rows, 15.4 us and here 12.1.)
-constexpr double kStreamAligned = 0.72;
+// What the estimate of runs of aligned channels, with the last wave in parts, is multiplied by where it is held against the kernel for long
+// rows (long_plan).  The smaller one of the two is launched: of 450 passes of 250 to 510 floats a row, forward, residual forward, backward and
+// residual backward are 2.9, 0.8, 0.4 and 1.0 per cent above the better one (121 to 161 each, of forward passes 7), always this kernel would be
+// 22, 4.5, 5.6 and 3.0; of 241 passes without such runs, with whole waves and no factor, 1.7, 3.2, 2.0 and 0.8, and 1.8, 5.0, 9.2 and 6.6.
+// [207,54,262] backward 13.8 us here and 18.0, [169,32,254] residual backward 10.4 and 11.0.
+constexpr double kStreamAligned = 0.87;
 
 // The geometry that is launched: stream_geom's, or the one of the least estimated time where that is this much less.  Us so and with
 // stream_geom's alone, forward, backward, residual forward and backward: [3865,36,18] 8.9, 11.7, 10.7, 15.4 and 11.0, 17.4, 16.9, 23.3, [1148,44,80]
@@ -428,17 +432,16 @@ bool stream_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, Str
 {
   if (!stream_geom(dim0, C, N, dir, extra, g)) return false;
   const uint32_t q = dim0 % 4 == 0 ? 1 : dim0 % 2 == 0 ? 2 : 4;
-  const double first = stream_cost(dim0, C, N, dir, extra, false, g.cb, g.cluster, g.groups, g.cb * dim0 / 4);
-  double best = kStreamOther * first;
-  g.cost = (float)(kStreamAligned * first);
+  double best = kStreamOther * stream_cost(dim0, C, N, dir, extra, false, g.cb, g.cluster, g.groups, g.cb * dim0 / 4);
   for (uint32_t cb = q; cb <= C && cb <= kStreamChannels && cb * dim0 <= 4 * kStreamThreads; cb = next_unit(cb, q)) {
     const uint32_t L4 = cb * dim0 / 4, groups = kStreamThreads / L4 < N ? kStreamThreads / L4 : N;
     if (cb * dim0 < 32 && cb + q <= C) continue;
     for (uint32_t cl = 1; cl <= 16 && cl * cb <= kStreamRecords && (cl == 1 || N / cl >= groups * 2); cl *= 2) {
       const double cost = stream_cost(dim0, C, N, dir, extra, false, cb, cl, groups, L4);
-      if (cost < best) { best = cost; g.cost = (float)(kStreamAligned * cost); stream_set(g, C, N, cb, cl, groups, L4); }
+      if (cost < best) { best = cost; stream_set(g, C, N, cb, cl, groups, L4); }
     }
   }
+  g.cost = (float)(kStreamAligned * stream_cost(dim0, C, N, dir, extra, false, g.cb, g.cluster, g.groups, g.cb * dim0 / 4, true));
   return true;
 }
 
@@ -467,7 +470,7 @@ bool masked_plan(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra, Str
   return best != 0;
 }
 
-// Whether the grid is one wave of blocks, all resident, that fills the device: nothing of a second wave to pay for.
+// Whether stream_geom's grid is one wave of blocks, all resident, that fills the device: nothing of a second wave to pay for.
 bool stream_one_wave(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra)
 {
   StreamGeom g;
@@ -476,9 +479,11 @@ bool stream_one_wave(uint32_t dim0, uint32_t C, uint32_t N, int dir, bool extra)
   return g.cluster <= 4 && blocks * 20 >= wave * 17 && blocks <= (g.cluster == 4 ? wave * 15 / 16 : wave);
 }
 
+// The rules that choose between this kernel and the others, here and in chan_preferred and band_plan, look at stream_geom's geometry, on
+// which their lines were drawn; what is launched in its place (stream_plan) is estimated to be the faster one, so they err to this side only.
 static bool stream_extra(const FusedArgs &a, int dir) { return (dir == 0 ? a.res : a.ymask) != nullptr; }
 
-// Blocks of a cluster, and of the grid, for this call; 0 where the kernel does not apply.
+// Blocks of a cluster, and of the grid, in stream_geom's geometry for this call; 0 where the kernel does not apply.
 uint32_t stream_cluster(const FusedArgs &a, int dir, bool aligned, uint32_t &blocks)
 {
   StreamGeom g;

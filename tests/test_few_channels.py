@@ -25,3 +25,11 @@ def test_stays_with_the_kernel_named_for_it(shape, call, named):
 def test_goes_where_it_is_faster(shape, call, launched):
     from anode_b200 import ops
     assert ops.launched_kernel(shape, call[0], residual=call[1]) == launched
+
+
+@pytest.mark.parametrize("shape,call,launched", [
+    ((207, 54, 1, 262), BWD, "stream"), ((169, 32, 1, 254), BWD_RES, "stream"), ((22, 450, 1, 262), FWD_RES, "stream"), ((156, 32, 1, 262), BWD_RES, "long"),
+    ((270, 20, 1, 470), FWD, "long")])
+def test_the_smaller_estimate_of_the_two(shape, call, launched):
+    from anode_b200 import ops
+    assert ops.launched_kernel(shape, call[0], residual=call[1]) == launched
