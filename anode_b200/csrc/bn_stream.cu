@@ -420,7 +420,7 @@ static void stream_set(StreamGeom &g, uint32_t C, uint32_t N, uint32_t cb, uint3
 // rows (long_plan).  The smaller one of the two is launched: of 450 passes of 250 to 510 floats a row, forward, residual forward, backward and
 // residual backward are 2.9, 0.8, 0.4 and 1.0 per cent above the better one (121 to 161 each, of forward passes 7), always this kernel would be
 // 22, 4.5, 5.6 and 3.0; of 241 passes without such runs, with whole waves and no factor, 1.7, 3.2, 2.0 and 0.8, and 1.8, 5.0, 9.2 and 6.6.
-// [207,54,262] backward 13.8 us here and 18.0, [169,32,254] residual backward 10.4 and 11.0.
+// [207,54,262] backward 13.8 us here and 18.0, [169,32,254] residual backward 10.4 and 11.0, [197,44,270] backward 16.3 and 11.0.
 constexpr double kStreamAligned = 0.87;
 
 // The geometry that is launched: stream_geom's, or the one of the least estimated time where that is this much less.  Us so and with

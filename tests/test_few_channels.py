@@ -29,7 +29,7 @@ def test_goes_where_it_is_faster(shape, call, launched):
 
 @pytest.mark.parametrize("shape,call,launched", [
     ((207, 54, 1, 262), BWD, "stream"), ((169, 32, 1, 254), BWD_RES, "stream"), ((22, 450, 1, 262), FWD_RES, "stream"), ((156, 32, 1, 262), BWD_RES, "long"),
-    ((270, 20, 1, 470), FWD, "long")])
+    ((496, 20, 1, 253), FWD, "long"), ((197, 44, 1, 270), BWD, "long"), ((183, 46, 1, 350), FWD_RES, "long")])
 def test_the_smaller_estimate_of_the_two(shape, call, launched):
     from anode_b200 import ops
     assert ops.launched_kernel(shape, call[0], residual=call[1]) == launched
