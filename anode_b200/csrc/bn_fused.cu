@@ -607,8 +607,9 @@ static float takes_from_us(const FusedArgs &a, int dir, bool extra, int kind)
 //  - the plain and the tiled kernel (which copies a row at a time), masked, where its estimate with these margins is below theirs
 //    (takes_from_us): clusters of few channels leave the device empty and walk their samples for long.  Plain: figures at the head of
 //    bn_stream.cu, but [97106,1,81] forward 57 and 144, [93078,1,146] backward 92 and 575, [130265,1,47] residual forward 61 and 254,
-//    [154066,1,113] residual backward 151 and 972; of 438 such passes 306 are taken, 0.62 of the time, eight of them slower by more than a
-//    twentieth, and what is left out would take 1.83 times as long here.  Tiled: [604,18,221] 16.4, 20.5, 18.5, 25.6 and 9.3, 11.7, 10.6, 14.8,
+//    [154066,1,113] residual backward 151 and 972; of 452 such passes 326 are taken, 0.62 of the time, nine of them slower by more than a
+//    twentieth (with margins of 1.3, 1.15, 1.1 and 1.1 [4096,3,7,7] backward was left out, 17.9 and 13.2; with a tenth less three are slower by
+//    1.2 to 1.3), and what is left out would take 1.89 times as long here.  Tiled: [604,18,221] 16.4, 20.5, 18.5, 25.6 and 9.3, 11.7, 10.6, 14.8,
 //    [1826,159,179] 128, 246, 213, - and 118, 186, 153, -, [1403,355,131] forward 191 and 143, [947,13,350] forward 19.5 and 13.3, residual forward 22.6
 //    and 20.1; but [110600,1,165] forward 63 and 496, [2705,2,818] backward 21.9 and 96.9, residual forward 17.9 and 88.1.  On rows of 200 floats and
 //    more only in small layers, where the tiled kernel's launch costs ten us: [1594,54,227] 54, 81, 77, 101 and 58, 80, 69, 107, [2147,15,254], 8.2 M, 27.5,
@@ -616,7 +617,7 @@ static float takes_from_us(const FusedArgs &a, int dir, bool extra, int kind)
 constexpr uint32_t kMaskedSamples = 20, kMaskedShortRow = 200;
 constexpr uint64_t kMaskedChan[2][2] = {{2500000, 2100000}, {2300000, 1100000}};        // [direction][residual]
 constexpr uint64_t kMaskedTiled[2][2] = {{8000000, 5000000}, {4500000, 2500000}};
-constexpr float kMaskedMargin[2][2] = {{1.3f, 1.1f}, {1.15f, 1.1f}};
+constexpr float kMaskedMargin[2][2] = {{1.2f, 1.05f}, {1.05f, 1.05f}};
 static bool masked_takes(const FusedArgs &a, int dir, int kind, StreamGeom &g)
 {
   const bool extra = (dir == 0 ? a.res : a.ymask) != nullptr;

@@ -20,7 +20,7 @@ def test_stays_with_the_kernel_named_for_it(shape, call, named):
 
 
 @pytest.mark.parametrize("shape,call,launched", [
-    ((2374, 147, 1, 83), BWD_RES, "stream"), ((4160, 7, 1, 33), FWD, "stream"), ((1403, 355, 1, 131), FWD, "stream"), ((1826, 159, 1, 179), BWD, "stream"),
+    ((4096, 3, 7, 7), BWD, "stream"), ((2374, 147, 1, 83), BWD_RES, "stream"), ((4160, 7, 1, 33), FWD, "stream"), ((1403, 355, 1, 131), FWD, "stream"), ((1826, 159, 1, 179), BWD, "stream"),
     ((1, 3, 1, 262144), FWD, "long"), ((41, 6, 64, 64), BWD, "long"), ((3, 512, 1, 2003), BWD_RES, "long"), ((3, 1023, 1, 1467), BWD_RES, "long")])
 def test_goes_where_it_is_faster(shape, call, launched):
     from anode_b200 import ops
