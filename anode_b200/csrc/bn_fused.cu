@@ -588,10 +588,12 @@ int pick_kernel_kind(const FusedArgs &a, int dir, bool aligned)
 
 // Us of the kernels that the two below take calls from.  The tiled kernel: its launch and agreement, the layer's bytes, and of ragged rows a
 // copy for each and tensor; seven per cent off over 968 passes of 0.2 to 46 M elements, from memory.  The plain kernel: its agreement, 1.75 to
-// 2 TB/s, and what a row's ends cost; 15 per cent off over 438 passes of 0.4 to 150 M elements.
+// 2 TB/s, and what a row's ends cost; 15 per cent off over 438 passes of 0.4 to 150 M elements.  From 256 floats a row on it takes them one by
+// one: 18 per cent off over 260 passes of 0.3 to 40 M elements.
 static float takes_from_us(const FusedArgs &a, int dir, bool extra, int kind)
 {
   const float rows = (float)a.plan.C * (float)a.plan.N, bytes = 4.0f * rows * (float)a.plan.dim0 * (dir == 0 ? (extra ? 3.0f : 2.0f) : extra ? 5.0f : 3.0f);
+  if (kind == ANODE_KERNEL_PLAIN && a.plan.dim0 >= 256) return dir == 0 ? 21.0f + bytes * 3.6e-7f + rows * 1e-3f : 17.0f + bytes * 3.6e-7f + rows * 2e-3f;
   if (kind == ANODE_KERNEL_PLAIN) return dir == 0 ? 13.0f + bytes * 5.7e-7f + rows * 4e-5f : 10.0f + bytes * 5e-7f + rows * 4e-5f;
   return 11.0f + bytes * 1.35e-7f + (a.plan.dim0 % 4 == 0 ? 0.0f : rows * (dir == 1 ? 5e-4f : extra ? 4.3e-4f : 2.2e-4f));
 }
@@ -631,22 +633,25 @@ static bool masked_takes(const FusedArgs &a, int dir, int kind, StreamGeom &g)
 
 // Rows of 250 floats and more, on one GPU: where the kernel for long rows (bn_long.cu) is launched in the place of the one that
 // pick_kernel_kind names.  Us there and here, forward, backward, residual forward and backward:
-//  - the tiled kernel where its time (takes_from_us) is a tenth more than the estimate of the other (of aligned rows' residual backward, which
-//    the estimate has a little high, a twentieth less): [1,3,64,64,64] 12.5, 12.4, -, - and 6.0, 7.9, -, -, [1,11,99716] -, 13.8, 13.2, 13.0 and
-//    -, 7.2, 6.7, 9.2; but [1,4,1630016], 6.5 M, 19.4, 25.2, 22.3, 31.8 and 28.6, 47.6, 47.3, 58.0, [392,12,1225] 20.2, -, 19.7, - and 22.3, -,
-//    27.7, -, [151,64,1098] forward 26.2 and 31.7, [972,11,365] backward 19.9 and 25.2.  Of 866 passes 634 are taken, 0.75 of the time, 15 of
-//    them slower by more than a twentieth, and what is left out would take 1.05 times as long here;
+//  - the tiled kernel where its time (takes_from_us), with what kLongAhead adds, is more than the estimate of the other: [1,3,64,64,64] 12.5,
+//    12.4, -, - and 6.0, 7.9, -, -, [1,11,99716] -, 13.8, 13.2, 13.0 and -, 7.2, 6.7, 9.2; but [1,4,1630016], 6.5 M, 19.4, 25.2, 22.3, 31.8 and
+//    28.6, 47.6, 47.3, 58.0, [392,12,1225] residual forward 19.7 and 27.7, [33,25,6426] backward 23.1 and 27.9.
+//    kLongAhead is from forward and backward passes of a layer in turn on a stream, where a forward pass on the tiled kernel costs more than
+//    the same pass over and over ([32,42,7480], forward and backward, 48.8 us, forward here 44.7; over the 351 of 8000 such pairs for which
+//    these rules and those without estimates of the other kernels launch something else, 0.87 of the time, and 0.86 of that without this kernel);
 //  - the register-resident kernel on ragged rows, which it loads float by float, from these sizes or channels on: [8,217,2678] 18.5, 29.8,
 //    30.9, 52.6 and 12.7, 16.1, 14.5, 20.6, [2,5,19011] 3.8, 5.2, 5.2, 6.9 and 5.1, 4.1, 4.5, 4.6, [9,4,12887] forward 8.1 and 5.5, but
 //    [10,119,1502], 1.8 M, 5.4, 8.5, 8.0 and 7.9, 10.0, 9.8, and where the clusters take a second wave, [71,25,577] backward 7.1 and 8.9,
 //    [3,1023,366] residual backward 8.0 and 11.3; in three waves and more what each block walks has to make up for them (kLongManyWaves),
-//    [4,2048,435] 12.4, 16.1, 16.4 and 27.4, 21.6, 24.8, [1,1024,8190] forward 24.6 and 26.4, but [1,923,8710] 28.3 and 25.9;
+//    [4,2048,435] 12.4, 16.1, 16.4 and 27.4, 21.6, 24.8, [1,1024,8190] forward 24.6 and 26.4, but [1,923,8710] 28.3 and 25.9 (the lines are from
+//    forward and backward in turn: [2,2048,1078] 38.7 and 49.9, [3,1926,1381] 61.4 and 61.1, [5,1173,999] 45.0 and 42.4, [3,1199,2091] 52.7 and 45.9);
 //  - and the same on aligned ones in the residual epilogue, where one block or two hold a channel: [35,183,1292], 8.3 M, 28.3, 40.8 and
 //    23.6, 35.8, [82,110,440], 4.0 M, 14.8, 21.1 and 13.6, 18.5, [7,331,1108], 2.6 M, backward 12.9 and 10.5; but forward [12,316,1032],
 //    3.9 M, 13.2 and 15.2, [18,380,464], 3.2 M, 10.5 and 12.0, and more channels, [2,512,4096] 10.8, 16.0 and 11.4, 19.4, [11,1404,420]
 //    15.6, 25.6 and 22.5, 28.7.
 constexpr uint32_t kLongRow = 250, kLongFewChannels = 128, kLongOneWave = 20;
-constexpr uint64_t kLongManyWaves[2][2] = {{8500, 4000}, {2000, 0}};                   // floats of a channel: [direction][residual]
+constexpr float kLongAhead[2][2][2] = {{{1.5f, 3.0f}, {1.0f, -1.0f}}, {{-1.5f, -0.5f}, {1.0f, 0.5f}}};      // us: [direction][residual][ragged]
+constexpr uint64_t kLongManyWaves[2][2] = {{4250, 2850}, {2000, 0}};                   // floats of a channel: [direction][residual]
 constexpr uint64_t kLongTiledMost = 12000000;
 constexpr uint64_t kLongManyChannels = 2400000;
 constexpr uint32_t kLongChannelsAligned = 450;
@@ -659,7 +664,7 @@ static bool long_takes(const FusedArgs &a, int dir, int kind, LongGeom &g)
   const uint64_t channel = (uint64_t)a.plan.dim0 * a.plan.N, elements = channel * a.plan.C;
   if (a.plan.dim0 < kLongRow) return false;
   if (kind == ANODE_KERNEL_TILED)
-    return elements <= kLongTiledMost && long_geom_of(a, dir, g) && g.cost * (dir == 1 && extra && a.plan.dim0 % 4 == 0 ? 0.95f : 1.1f) < takes_from_us(a, dir, extra, kind);
+    return elements <= kLongTiledMost && long_geom_of(a, dir, g) && g.cost < takes_from_us(a, dir, extra, kind) + kLongAhead[dir][extra][a.plan.dim0 % 4 != 0];
   if (kind != ANODE_KERNEL_REGISTER) return false;
   const uint32_t C = a.plan.C;
   if (a.plan.dim0 % 4 != 0 && C > 2 * kLongBlocks * sm_count() && channel < kLongManyWaves[dir][extra]) return false;
