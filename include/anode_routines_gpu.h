@@ -189,8 +189,8 @@ void anode_gpu_positive_clip_flat_map_bwd_f32(
  *   REGISTER  channels held in the registers of a warp, a block or a cluster (small layers, any alignment;
  *             one GPU);
  *   STREAM    clusters that walk a block of channels twice (layers of short rows; one GPU); its masked form takes runs of
- *             channels that begin anywhere, in the place of PLAIN and, where it is the faster one, of REGISTER and TILED: queries by
- *             shape name those;
+ *             channels that begin anywhere, in the place of PLAIN, REGISTER and TILED where it is the faster one: queries by shape
+ *             name those;
  *   BAND      its form for the largest of them, where the call has a workspace: one walk, with the tiles in tensor memory
  *             between reduction and normalization.  Queries by shape count it as STREAM.  It is launched cooperatively and takes
  *             the whole device, so other streams' kernels run before or after it, not beside it.
